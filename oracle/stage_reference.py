@@ -35,7 +35,7 @@ def _sha(path: str) -> str:
 def stage(source: str = DEFAULT_SOURCE, dest: str = DEST) -> bool:
     """Copy the files when `source` exists; returns whether oracle/_ref/ is populated afterwards."""
     manifest = os.path.join(dest, "MANIFEST.json")
-    if not os.path.isdir(source):
+    if not os.path.exists(os.path.join(source, FILES[0])):      # no checkout, or an empty directory in its place
         return os.path.exists(manifest)
     sums = {}
     for rel in FILES:

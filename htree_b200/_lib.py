@@ -18,6 +18,8 @@ FWD_FUSED = 4
 FWD_TILED = 8
 PARENTS_U16 = 16
 FWD_NO_PIPELINE = 128
+FWD_INFERENCE = 256
+PLAN_BACKWARD, PLAN_PARENTS = 1, 2
 BWD_KEEP_ACCUM = 32
 BWD_NO_FOLD = 64
 
@@ -32,6 +34,11 @@ SYMBOLS = (
     "htree_b200_rotate_keys",
     "htree_b200_block_values",
     "htree_b200_block_keys",
+    "htree_b200_operand_block_bytes",
+    "htree_b200_prepare",
+    "htree_b200_attend",
+    "htree_b200_plan",
+    "htree_b200_run_forward",
     "htree_b200_forward",
     "htree_b200_level_forward",
     "htree_b200_merge_to_global",
@@ -48,6 +55,12 @@ class HtreeShape(ctypes.Structure):
     _fields_ = [(n, ctypes.c_int32) for n in
                 ("B", "T", "H", "H_kv", "K", "V", "compression_rate", "top_k", "max_top_nodes", "dtype", "T_q",
                  "t_offset")]
+
+
+class HtreePlan(ctypes.Structure):
+    _fields_ = ([("bytes", ctypes.c_int64)] +
+                [(n, ctypes.c_int64 * MAX_LEVELS) for n in ("layers_k", "layers_v", "layers_k_rot", "blocks", "blocks_bwd", "parents")] +
+                [("nodes", ctypes.c_int32 * MAX_LEVELS), ("levels", ctypes.c_int32), ("reserved", ctypes.c_int32)])
 
 
 class HtreeTypedGrads(ctypes.Structure):
@@ -96,6 +109,17 @@ def lib() -> ctypes.CDLL:
         L.htree_b200_forward.restype = ctypes.c_int
         L.htree_b200_forward.argtypes = [ctypes.POINTER(HtreeShape), vp, vp, vp, vp, vp, vp, vp, vp, vp, vp, i32, f32, vp, vp, vp, vp,
                                          ctypes.POINTER(HtreeTrace), vp, u32, vp]
+        L.htree_b200_operand_block_bytes.restype = ctypes.c_int64
+        L.htree_b200_operand_block_bytes.argtypes = [ctypes.POINTER(HtreeShape), i32, i32]
+        L.htree_b200_prepare.restype = ctypes.c_int
+        L.htree_b200_prepare.argtypes = [ctypes.POINTER(HtreeShape), vp, vp, vp, vp, vp, i32, vp, vp, vp]
+        L.htree_b200_attend.restype = ctypes.c_int
+        L.htree_b200_attend.argtypes = [ctypes.POINTER(HtreeShape), vp, vp, vp, vp, vp, vp, vp, vp, i32, f32, vp, vp, vp, vp, vp, u32, vp]
+        L.htree_b200_plan.restype = ctypes.c_int
+        L.htree_b200_plan.argtypes = [ctypes.POINTER(HtreeShape), u32, ctypes.POINTER(HtreePlan)]
+        L.htree_b200_run_forward.restype = ctypes.c_int
+        L.htree_b200_run_forward.argtypes = [ctypes.POINTER(HtreeShape), ctypes.POINTER(HtreePlan), vp, vp, vp, vp, vp, vp, i32, f32, vp,
+                                             vp, vp, vp, vp, vp, u32, vp]
         L.htree_b200_level_forward.restype = ctypes.c_int
         L.htree_b200_level_forward.argtypes = [ctypes.POINTER(HtreeShape), i32, i32, vp, vp, vp, vp, vp, vp, i32, f32, vp, vp, vp, vp,
                                                vp, vp]

@@ -1,0 +1,368 @@
+// Forward accumulation: softmax(S) V over everything the selections leave to accumulate, all tree levels in one launch, one
+// warp per (batch, query position, KV head) group.  Replaces the accumulation halves of htree_select_accumulate_gqa_kernel and
+// htree_bottom_accumulate_gqa_kernel together with htree_merge_to_global_kernel and htree_final_normalize_kernel
+// (src/parallel.py:248-867); reads the parent lists that a selection launch wrote.
+//
+// Products, operand blocks and chunk numbering: tform.cuh.  Per chunk of 16 positions a warp copies the operand block(s) and
+// one rotary-table row into its ring in shared memory (two bulk copies, issued NSTG - 1 chunks ahead), forms
+// S^T = K' q^ (one query rotation per chunk), P^T, and O^T += V^T P^T.
+#include "tform.cuh"
+
+namespace htree {
+
+template <int D, bool X3>
+constexpr int acc_stages() { return D == 128 ? 2 : 3; }
+
+// Registers: 168 per thread (12 warps per SM) hold a group of 16 heads of 128; what the kernel needs beyond that is room for
+// the rings, two slots of 8448 bytes per warp at 128-wide heads.
+constexpr int kAccWarps = 4;
+template <int D, bool X3, int NH>
+constexpr int acc_min_blocks() { return (X3 && D == 128) ? 2 : (D == 128 || (X3 && D == 64 && NH == 2)) ? 3 : 4; }
+
+template <typename T, int D, bool X3, int NH, int CR, bool SPLIT>
+__global__ void __launch_bounds__(SPLIT ? 256 : kAccWarps * 32, SPLIT ? 1 : acc_min_blocks<D, X3, NH>())
+acc_mma_kernel(const __grid_constant__ AttnParams p) {
+    using C = TForm<D, X3, CR>;
+    using F = Frag<typename std::conditional<X3, __half, T>::type>;   // type of the values and probabilities
+    constexpr int MT = C::MT, PPC = C::PPC;
+    using Ring = ChunkRing<acc_stages<D, X3>(), C::SLOT>;
+    constexpr int NSTG = acc_stages<D, X3>();
+    extern __shared__ __align__(128) unsigned char smem_raw[];
+
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, g = lane >> 2, r = lane & 3;
+    const int W = blockDim.x >> 5;
+    const int tl = SPLIT ? (int)blockIdx.x : (int)(blockIdx.x * W + warp);
+    if (!SPLIT && tl >= p.Tq) return;
+    const int t = p.t0 + tl;
+    const int b = blockIdx.y / p.Hkv, hk = blockIdx.y % p.Hkv;
+    const int G = p.G, TK = p.TK, L = p.L;
+    const int first = SPLIT ? warp : 0, step = SPLIT ? W : 1;         // this warp's chunks of every level
+
+    // per warp: ring, parent list, kept-candidate bits
+    const size_t per_warp = (Ring::kBytes + sizeof(int32_t) * TK + sizeof(uint32_t) * ((TK * CR + 31) / 32) + 127) & ~size_t(127);
+    unsigned char* wbase = smem_raw + warp * per_warp;
+    Ring ring;
+    ring.init(wbase, lane);
+    int32_t* par = reinterpret_cast<int32_t*>(wbase + Ring::kBytes);
+    uint32_t* selw = reinterpret_cast<uint32_t*>(par + TK);
+
+    const int64_t hbase = ((int64_t)b * p.Tq + tl) * p.H + (int64_t)hk * G;
+    const int64_t qidx = ((int64_t)b * p.Tq + tl) * p.Hkv + hk;
+
+    QueryRegs<T, D, X3, NH> q;
+    load_query<T, D, X3, NH>(reinterpret_cast<const T*>(p.q) + hbase * D, G, g, r, p.scale, q);
+
+    float O[NH][MT][4];
+#pragma unroll
+    for (int h = 0; h < NH; ++h)
+#pragma unroll
+        for (int i = 0; i < MT; ++i) O[h][i][0] = O[h][i][1] = O[h][i][2] = O[h][i][3] = 0.f;
+    // Online softmax with a lazily moved reference: probabilities are taken relative to m_run, which moves (and the
+    // accumulators are rescaled) only when a score exceeds it by more than kLazyMax.  m_run is common to the lanes that share
+    // a head; m_true (the maximum that goes to gmax) and s_run are per lane until the end.
+    constexpr float kLazyMax = 8.f;
+    constexpr float kNone = -1.0e30f;
+    float m_run[NH][2], m_true[NH][2], s_run[NH][2], m_run2[NH][2];
+#pragma unroll
+    for (int h = 0; h < NH; ++h)
+#pragma unroll
+        for (int e = 0; e < 2; ++e) { m_run[h][e] = m_true[h][e] = kNone; m_run2[h][e] = kNone * kLog2e; s_run[h][e] = 0.f; }
+
+    for (int l = L - 1; l >= 0; --l) {
+        const int Nl = p.ln[l];
+        __syncwarp();
+        int np = 0;
+        for (int i = lane; i < TK; i += 32) { const int x = load_parent(p, l, qidx * TK + i); par[i] = x; np += x >= 0; }
+        np = __reduce_add_sync(0xffffffffu, np);
+        const int rc = (int)(((int64_t)t / p.lpow[l]) % CR);
+        const int nc = (np - 1) * CR + rc + 1, rp = nc - 1;
+        if (l > 0 && nc <= TK) continue;                              // every candidate is kept: nothing to accumulate
+        if (np <= 0) continue;
+        const int nchunk = (np + PPC - 1) / PPC;
+        if (l > 0) {
+            // positions the next level kept, from its list (both lists ascending)
+            for (int i = lane; i < (nc + 31) / 32; i += 32) selw[i] = 0u;
+            __syncwarp();
+            for (int i = lane; i < TK; i += 32) {
+                const int node = load_parent(p, l - 1, qidx * TK + i);
+                if (node < 0) continue;
+                const int parent = node / CR;
+                int lo = 0, hi = np;
+                while (lo < hi) { const int mid = (lo + hi) >> 1; if (par[mid] < parent) lo = mid + 1; else hi = mid; }
+                if (lo < np && par[lo] == parent) {
+                    const int j = lo * CR + node % CR;
+                    atomicOr(&selw[j >> 5], 1u << (j & 31));
+                }
+            }
+        }
+        __syncwarp();
+
+        const int nblk = (Nl + CR - 1) / CR;
+        const int64_t bstride = (int64_t)p.Hkv * C::BLOCK;
+        const unsigned char* blk = reinterpret_cast<const unsigned char*>(p.blk[l]) + ((int64_t)b * nblk * p.Hkv + hk) * C::BLOCK;
+        const unsigned char* tab = reinterpret_cast<const unsigned char*>(p.tab) + (int64_t)(rp - 16 * first) * C::TAB;   // of the next issue
+        auto issue = [&](int c) {                                     // chunk c of this level
+            if (lane == 0) {
+                ring.expect(C::SLOT);
+                int p0 = par[c * PPC];
+                if ((unsigned)p0 >= (unsigned)nblk) { if (p.status) atomicOr(p.status, 4); p0 = 0; }
+                if constexpr (CR == 16) {
+                    ring.copy(0, blk + p0 * bstride, C::DATA);
+                } else {
+                    int p1 = c * PPC + 1 < np ? par[c * PPC + 1] : p0;    // past the end of the list: masked, any finite block
+                    if ((unsigned)p1 >= (unsigned)nblk) { if (p.status) atomicOr(p.status, 4); p1 = 0; }
+                    ring.copy(0, blk + p0 * bstride, C::DATA / 2);
+                    ring.copy(C::DATA / 2, blk + p1 * bstride + C::PL * C::PART, C::DATA / 2);
+                }
+                ring.copy(C::DATA, tab, C::TAB);
+            }
+            tab -= (int64_t)16 * C::TAB * step;
+            ring.issued();
+        };
+        int next = first;
+#pragma unroll 1
+        for (int s = 0; s < NSTG - 1 && next < nchunk; ++s, next += step) issue(next);
+#pragma unroll 1
+        for (int c = first; c < nchunk; c += step) {
+            __syncwarp();                                             // everybody is done with the slot that is refilled now
+            if (next < nchunk) { issue(next); next += step; }
+            uint32_t mask = 0xffffu;
+            if (l > 0) mask &= ~(selw[c >> 1] >> ((16 * c) & 31));
+            if (16 * c + 15 > rp) mask &= (2u << (rp - 16 * c)) - 1u;
+            uint32_t slot;
+            if (!ring.wait(slot)) { if (lane == 0 && p.status) atomicOr(p.status, 16); ring.drain(); return; }
+            if (mask == 0) continue;
+            const LaneBase<D, X3, CR> lb(slot, lane);
+            float S[NH][4];
+            score_t<T, D, X3, NH, CR>(lb, slot + C::DATA, r, q, S);
+            if (mask != 0xffffu) {
+                const bool c0 = (mask >> g) & 1, c1 = (mask >> (g + 8)) & 1;
+#pragma unroll
+                for (int h = 0; h < NH; ++h) {
+                    S[h][0] = c0 ? S[h][0] : -INFINITY; S[h][1] = c0 ? S[h][1] : -INFINITY;
+                    S[h][2] = c1 ? S[h][2] : -INFINITY; S[h][3] = c1 ? S[h][3] : -INFINITY;
+                }
+            }
+            bool move = false;
+            float mx[NH][2];
+#pragma unroll
+            for (int h = 0; h < NH; ++h)
+#pragma unroll
+                for (int e = 0; e < 2; ++e) {
+                    mx[h][e] = fmaxf(S[h][e], S[h][2 + e]);
+                    m_true[h][e] = fmaxf(m_true[h][e], mx[h][e]);
+                    move = move || mx[h][e] > m_run[h][e] + kLazyMax;
+                }
+            if (__any_sync(0xffffffffu, move)) {
+#pragma unroll
+                for (int h = 0; h < NH; ++h)
+#pragma unroll
+                    for (int e = 0; e < 2; ++e) {
+                        float m = mx[h][e];
+                        m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, 4));
+                        m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, 8));
+                        m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, 16));
+                        const float n = fmaxf(m_run[h][e], m);
+                        const float f = X3 ? __expf(m_run[h][e] - n) : ex2_approx(m_run2[h][e] - n * kLog2e);
+                        m_run[h][e] = n; m_run2[h][e] = n * kLog2e;
+                        s_run[h][e] *= f;
+#pragma unroll
+                        for (int i = 0; i < MT; ++i) { O[h][i][e] *= f; O[h][i][2 + e] *= f; }
+                    }
+            }
+            uint32_t pb[NH][2], pl[X3 ? NH : 1][2];
+#pragma unroll
+            for (int h = 0; h < NH; ++h) {
+                float P[4];
+#pragma unroll
+                for (int i = 0; i < 4; ++i) {
+                    // fp32 storage keeps the plain difference (an exponent re-based by log2 e rounds at 1e-6 relative)
+                    P[i] = X3 ? __expf(S[h][i] - m_run[h][i & 1]) : ex2_approx(fmaf(S[h][i], kLog2e, -m_run2[h][i & 1]));
+                }
+                s_run[h][0] += P[0] + P[2];
+                s_run[h][1] += P[1] + P[3];
+                if constexpr (X3) {
+                    uint32_t h0, l0, h1, l1;
+                    split_half2(P[0], P[1], h0, l0); split_half2(P[2], P[3], h1, l1);
+                    pb[h][0] = movmatrix_trans(h0); pb[h][1] = movmatrix_trans(h1);
+                    pl[X3 ? h : 0][0] = movmatrix_trans(l0); pl[X3 ? h : 0][1] = movmatrix_trans(l1);
+                } else {
+                    pb[h][0] = movmatrix_trans(F::pack(P[0], P[1])); pb[h][1] = movmatrix_trans(F::pack(P[2], P[3]));
+                }
+            }
+#pragma unroll
+            for (int i = 0; i < MT; ++i) {
+                uint32_t va[4];
+                value_frag<D, X3, CR>(lb, 0, i, va);
+                if constexpr (X3) {
+                    // summed from zero and then added with a round-to-nearest fp32 add: the tensor core's own accumulation
+                    // truncates, and over the ~10^3 chunks of a query that bias would reach 1e-4 relative
+                    uint32_t vl[4];
+                    value_frag<D, X3, CR>(lb, 1, i, vl);
+#pragma unroll
+                    for (int h = 0; h < NH; ++h) {
+                        float acc[4];
+                        mma_zero<__half>(acc, va, pl[X3 ? h : 0][0], pl[X3 ? h : 0][1]);
+                        F::mma(acc, vl[0], vl[1], vl[2], vl[3], pb[h][0], pb[h][1]);
+                        F::mma(acc, va[0], va[1], va[2], va[3], pb[h][0], pb[h][1]);
+#pragma unroll
+                        for (int u = 0; u < 4; ++u) O[h][i][u] += acc[u];
+                    }
+                } else {
+#pragma unroll
+                    for (int h = 0; h < NH; ++h) F::mma(O[h][i], va[0], va[1], va[2], va[3], pb[h][0], pb[h][1]);
+                }
+            }
+        }
+    }
+
+    // ---- totals over the lanes of a head ----
+#pragma unroll
+    for (int h = 0; h < NH; ++h)
+#pragma unroll
+        for (int e = 0; e < 2; ++e)
+#pragma unroll
+            for (int o = 4; o < 32; o <<= 1) {
+                s_run[h][e] += __shfl_xor_sync(0xffffffffu, s_run[h][e], o);
+                m_true[h][e] = fmaxf(m_true[h][e], __shfl_xor_sync(0xffffffffu, m_true[h][e], o));
+            }
+    if constexpr (SPLIT) {
+        // merge the warps' partial states (few queries: a group's chunks are spread over the warps of a block)
+        __syncthreads();                                              // all rings are idle: their memory is free
+        float* st = reinterpret_cast<float*>(smem_raw + W * per_warp);          // [W][3][16]: m_run, m_true, s
+        float* po = reinterpret_cast<float*>(wbase);                  // this warp's O, [16 heads][D]
+        if (g == 0) {
+#pragma unroll
+            for (int h = 0; h < NH; ++h)
+#pragma unroll
+                for (int e = 0; e < 2; ++e) {
+                    const int head = 8 * h + 2 * r + e;
+                    st[(warp * 3 + 0) * 16 + head] = m_run[h][e]; st[(warp * 3 + 1) * 16 + head] = m_true[h][e]; st[(warp * 3 + 2) * 16 + head] = s_run[h][e];
+                }
+        }
+        __syncthreads();
+#pragma unroll
+        for (int h = 0; h < NH; ++h)
+#pragma unroll
+            for (int e = 0; e < 2; ++e) {
+                const int head = 8 * h + 2 * r + e;
+                float m = kNone;
+                for (int w = 0; w < W; ++w) m = fmaxf(m, st[w * 48 + head]);
+                const float f = __expf(m_run[h][e] - m);
+#pragma unroll
+                for (int i = 0; i < MT; ++i) {
+                    po[head * D + C::VB * g + 2 * i] = O[h][i][e] * f;
+                    po[head * D + C::VB * g + 2 * i + 1] = O[h][i][2 + e] * f;
+                }
+            }
+        __syncthreads();
+        for (int i = threadIdx.x; i < G * D; i += blockDim.x) {
+            const int head = i / D;
+            float m = kNone, s = 0.f, o = 0.f;
+            for (int w = 0; w < W; ++w) m = fmaxf(m, st[w * 48 + head]);
+            for (int w = 0; w < W; ++w) {
+                s += st[w * 48 + 32 + head] * __expf(st[w * 48 + head] - m);
+                o += reinterpret_cast<const float*>(smem_raw + w * per_warp)[i];
+            }
+            reinterpret_cast<T*>(p.out)[hbase * D + i] = from_f<T>(o / s);
+            if (i % D == 0) {
+                float mt = kNone;
+                for (int w = 0; w < W; ++w) mt = fmaxf(mt, st[w * 48 + 16 + head]);
+                p.gmax[hbase + head] = mt; p.gsum[hbase + head] = s * __expf(m - mt);
+            }
+        }
+        return;
+    }
+#pragma unroll
+    for (int h = 0; h < NH; ++h)
+#pragma unroll
+        for (int e = 0; e < 2; ++e) {
+            const int head = 8 * h + 2 * r + e;
+            if (head >= G) continue;
+            const float inv = 1.f / s_run[h][e];
+            T* orow = reinterpret_cast<T*>(p.out) + (hbase + head) * D + C::VB * g;
+            if constexpr (sizeof(T) == 4) {
+#pragma unroll
+                for (int i = 0; i < MT / 2; ++i)
+                    reinterpret_cast<float4*>(orow)[i] = make_float4(O[h][2 * i][e] * inv, O[h][2 * i][2 + e] * inv, O[h][2 * i + 1][e] * inv, O[h][2 * i + 1][2 + e] * inv);
+            } else {
+                uint32_t w[MT];
+#pragma unroll
+                for (int i = 0; i < MT; ++i) w[i] = Frag<typename std::conditional<sizeof(T) == 4, __half, T>::type>::pack(O[h][i][e] * inv, O[h][i][2 + e] * inv);
+                if constexpr (MT >= 4) {
+#pragma unroll
+                    for (int i = 0; i < MT / 4; ++i) reinterpret_cast<uint4*>(orow)[i] = make_uint4(w[4 * i], w[4 * i + 1], w[4 * i + 2], w[4 * i + 3]);
+                } else {
+                    *reinterpret_cast<uint2*>(orow) = make_uint2(w[0], w[1]);
+                }
+            }
+            if (g == 0) { p.gmax[hbase + head] = m_true[h][e]; p.gsum[hbase + head] = s_run[h][e] * __expf(m_run[h][e] - m_true[h][e]); }
+        }
+}
+
+template <typename T, int D, bool X3, int NH, int CR>
+static int launch_acc_cr(const AttnParams& p, cudaStream_t st) {
+    using C = TForm<D, X3, CR>;
+    using Ring = ChunkRing<acc_stages<D, X3>(), C::SLOT>;
+    const size_t per_warp = (Ring::kBytes + sizeof(int32_t) * p.TK + sizeof(uint32_t) * ((p.TK * CR + 31) / 32) + 127) & ~size_t(127);
+    const size_t limit = 227 * 1024;
+    // Few groups: one block of 8 warps per group.  Below two groups per SM the chip has room for all their warps at once, and
+    // a single warp's walk over its chunks (about 1 us each) would be the whole time of the call.  Calls whose state the
+    // backward reads (they keep their selections) always take one warp per group: a query's result then does not depend on
+    // how many queries share the call.
+    const int64_t groups = (int64_t)p.Tq * p.B * p.Hkv;
+    const size_t split_smem = 8 * per_warp + 8 * 48 * sizeof(float);
+    if ((p.flags & kFlagSplitOk) && groups <= 2 * 148 && split_smem <= limit) {
+        auto* k = acc_mma_kernel<T, D, X3, NH, CR, true>;
+        const cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)split_smem);
+        if (e != cudaSuccess) return (int)e;
+        k<<<dim3(p.Tq, p.B * p.Hkv), 256, split_smem, st>>>(p);
+        note_launch();
+        return (int)cudaGetLastError();
+    }
+    // warps per block: as many resident warps as registers allow, fewer where long parent lists leave no room for the rings
+    const int max_warps = kAccWarps * acc_min_blocks<D, X3, NH>();
+    int W = 1, best = 0;
+    for (int w = kAccWarps; w >= 1; --w) {
+        if (w == 3) continue;
+        int blocks = (int)(228 * 1024 / (w * per_warp + 1024));
+        if (blocks * w > max_warps) blocks = max_warps / w;
+        if (blocks > 0 && blocks * w > best) { best = blocks * w; W = w; }
+    }
+    if (best == 0 || W * per_warp > limit) return HTREE_E_UNSUPPORTED;
+    auto* k = acc_mma_kernel<T, D, X3, NH, CR, false>;
+    const cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)(W * per_warp));
+    if (e != cudaSuccess) return (int)e;
+    k<<<dim3((p.Tq + W - 1) / W, p.B * p.Hkv), W * 32, W * per_warp, st>>>(p);
+    note_launch();
+    return (int)cudaGetLastError();
+}
+
+template <typename T, int D, bool X3>
+static int launch_acc_t(const AttnParams& p, cudaStream_t st) {
+    if (p.CR == 16) return p.G <= 8 ? launch_acc_cr<T, D, X3, 1, 16>(p, st) : launch_acc_cr<T, D, X3, 2, 16>(p, st);
+    return p.G <= 8 ? launch_acc_cr<T, D, X3, 1, 8>(p, st) : launch_acc_cr<T, D, X3, 2, 8>(p, st);
+}
+template <typename T>
+static int launch_acc_d(const AttnParams& p, cudaStream_t st) {
+    constexpr bool F32 = std::is_same<T, float>::value;
+    return p.K == 128 ? launch_acc_t<T, 128, F32>(p, st) : p.K == 64 ? launch_acc_t<T, 64, F32>(p, st) : launch_acc_t<T, 32, true>(p, st);
+}
+
+// The per-warp parent list, kept bits and ring must fit one warp into an SM's shared memory.
+bool acc_mma_supported(const AttnParams& p, int dtype) {
+    if (!pack_supported(dtype, p.K, p.V, p.CR) || p.G > 16 || !p.tab) return false;
+    for (int l = 0; l < p.L; ++l) if (!p.blk[l]) return false;
+    const size_t slot = (pack_split(dtype, p.K) ? 2 : 1) * (size_t)p.K * 64 + 4 * p.K;
+    return 3 * slot + 512 + 4 * (size_t)p.TK + (size_t)p.TK * p.CR / 8 <= 227 * 1024;
+}
+
+int launch_acc_mma(const AttnParams& p, int dtype, cudaStream_t st) {
+    switch (dtype) {
+        case HTREE_F32: return launch_acc_d<float>(p, st);
+        case HTREE_BF16: return launch_acc_d<__nv_bfloat16>(p, st);
+        default: return launch_acc_d<__half>(p, st);
+    }
+}
+
+}  // namespace htree

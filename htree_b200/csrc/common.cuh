@@ -21,6 +21,9 @@ struct AttnParams {
     const void* lkr[HTREE_MAX_LEVELS];   // keys pre-rotated by their child index (16-bit storage types only), or NULL
     const void* lvb[HTREE_MAX_LEVELS];   // values re-laid-out per parent block for the P.V fragments (tree.cu), or NULL
     const void* lkb[HTREE_MAX_LEVELS];   // pre-rotated keys per parent block in fragment-major order (tree.cu), or NULL
+    const void* blk[HTREE_MAX_LEVELS];   // operand blocks of the transposed kernels (tform.cuh), or NULL
+    const void* vkblk[HTREE_MAX_LEVELS]; // their backward part, or NULL
+    const void* tab;                     // rotary table of the transposed kernels, rows [cos | sin]: IEEE half times scale, or fp32 (split-half)
     int32_t ln[HTREE_MAX_LEVELS];   // N_l
     int64_t lpow[HTREE_MAX_LEVELS]; // CR^l
     const float* cosc;
@@ -126,6 +129,18 @@ __device__ __forceinline__ void store_parent(const AttnParams& p, int l, int64_t
     if (p.flags & HTREE_PARENTS_U16) reinterpret_cast<uint16_t*>(p.parents[l])[idx] = v < 0 ? (uint16_t)0xFFFFu : (uint16_t)v;
     else p.parents[l][idx] = v;
 }
+
+constexpr uint32_t kFlagSplitOk = 1u << 30;   // internal: a forward whose selections are not kept for a backward
+
+// transposed tensor-core kernels (operands.cu, acc_mma.cu)
+bool pack_supported(int dtype, int K, int V, int CR);
+bool pack_split(int dtype, int D);                       // split-half operands?
+size_t pack_block_bytes(int D, bool x3, int CR);         // bytes of one forward block
+int launch_pack_blocks(const HtreeShape& s, int L, const int32_t* ln, void* const* lk, void* const* lv, void* const* blk,
+                       void* const* vkblk, void* const* krot, bool pool, const float* cosc, const float* sinc, cudaStream_t st);
+bool select_mma_supported(const AttnParams& p, int dtype);
+bool acc_mma_supported(const AttnParams& p, int dtype);
+int launch_acc_mma(const AttnParams& p, int dtype, cudaStream_t st);
 
 // launchers implemented in the .cu files (return cudaError_t as int)
 int launch_tree_build(const HtreeShape& s, int L, const int32_t* ln, void* const* lk, void* const* lv, cudaStream_t st);

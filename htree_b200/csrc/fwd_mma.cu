@@ -705,6 +705,15 @@ static int launch_mma_td(const AttnParams& p, cudaStream_t st) {
     return (p.cosh != nullptr && p.sinh != nullptr) ? launch_mma_tdr<T, D, true>(p, st) : launch_mma_tdr<T, D, false>(p, st);
 }
 
+// The selection kernel alone (K' rows of the upper levels; nothing of the leaf level is read).
+bool select_mma_supported(const AttnParams& p, int dtype) {
+    if (dtype != HTREE_BF16 && dtype != HTREE_F16 && dtype != HTREE_F32) return false;
+    if (p.K != 64 && (p.K != 128 || dtype == HTREE_F32)) return false;
+    if (p.G > 16 || (p.CR != 16 && p.CR != 8)) return false;
+    for (int l = 1; l < p.L; ++l) if (!p.lkr[l]) return false;
+    return mma_smem_per_warp(p.TK, p.CR) * MW <= 200 * 1024;
+}
+
 bool fwd_mma_supported(const AttnParams& p, int dtype) {
     if (dtype != HTREE_BF16 && dtype != HTREE_F16 && dtype != HTREE_F32) return false;
     if (p.K != p.V || (p.K != 64 && p.K != 128)) return false;

@@ -1,0 +1,302 @@
+// Shared pieces of the transposed tensor-core kernels (forward accumulation, backward): one warp owns one (batch, query
+// position, KV head) group and walks its candidates in chunks of 16 positions (the children of one parent with 16 children
+// per parent, of two consecutive parents with 8).
+//
+// Every product puts the candidates (or the head dimension) on the M = 16 side of mma.sync.m16n8k16 and the query HEADS on
+// the N = 8 side: S^T = K' q^, O^T += V^T P^T.  A group of at most 8 heads then needs half the instructions of the
+// heads-on-M form, whose other 8 rows would be padding; 9..16 heads are two halves (NH = 2) that share every A fragment, at
+// the instruction count of the heads-on-M form.
+//
+// Operand blocks (written by pack_blocks_kernel, read here as whole blocks by asynchronous bulk copies): per parent and KV
+// head the children's pre-rotated keys K' and values in the order in which the lanes consume them as A fragments, so that a
+// fragment is one conflict-free 16-byte shared load.  With lane = 4g + r, KS = D/16, PPT = D/8, VB = D/8:
+//   16 children   K [ks][lane] = { K'[g][lo], K'[8+g][lo], K'[g][hi], K'[8+g][hi] },  lo = dims PPT*r + 2ks + {0,1}, hi = lo + D/2
+//                 V [i][lane]  = { b0(2i), b0(2i+1), b1(2i), b1(2i+1) },  bj(w) = { V[8j+2r][VB*g+w], V[8j+2r+1][VB*g+w] }
+//                 block = [K | V]; 16 bytes are the four registers of one A fragment in their order (an LDS.128 whose
+//                 registers had to be swapped cost 4 moves per fragment, a quarter of the loop's instructions)
+//    8 children   K [ks][lo, hi][lane] and V [w][lane], 4 bytes each: 8x8 matrices that ldmatrix gathers from two parents
+//                 block = [K even | V | K odd]: a parent in an odd slot of the query's list holds positions 8..15 of its
+//                 chunk, so its keys are also stored rotated by 8 more positions; a chunk then has ONE query rotation for
+//                 its 16 positions and full M tiles, as with 16 children
+//   split-half (fp32 storage, and every storage type with 32-wide heads): each part is a hi plane followed by a lo plane.
+#pragma once
+#include "mma_common.cuh"
+
+namespace htree {
+
+template <int D, bool X3, int CR>
+struct TForm {
+    static constexpr int KS = D / 16, HALF = D / 2, PPT = HALF / 4, VB = D / 8, MT = D / 16;
+    static constexpr int PL = X3 ? 2 : 1;                                  // planes
+    static constexpr int PART = D * 2 * CR;                                // bytes of one plane of one part of a block
+    static constexpr int BLOCK = PL * PART * (CR == 16 ? 2 : 3);           // bytes of a block in global memory
+    static constexpr int DATA = PL * D * 64;                               // bytes of a chunk in shared memory
+    static constexpr int TAB = X3 ? D * 4 : D * 2;                         // one row of the rotary table: [cos | sin]
+    static constexpr int SLOT = DATA + TAB;
+    static constexpr int PPC = 16 / CR;                                    // parents per chunk
+    // part offsets in a slot: 16 children [K | V]; 8 children [K even | V even | V odd | K odd]
+    static constexpr int V_OFF = PL * PART;
+    static constexpr int V2_OFF = 2 * PL * PART, K2_OFF = 3 * PL * PART;   // 8 children only
+};
+
+// Shared-memory addresses of a chunk slot that differ by lane, as 32-bit shared addresses.
+template <int D, bool X3, int CR>
+struct LaneBase {
+    uint32_t k, v;      // 16 children: slot + 16 * lane (v unused); 8 children: ldmatrix row addresses of the key and value matrices
+    __device__ __forceinline__ LaneBase(uint32_t slot, int lane) {
+        using C = TForm<D, X3, CR>;
+        if constexpr (CR == 16) {
+            k = slot + 16 * lane; v = 0;
+        } else {
+            const int j = lane >> 3, row = lane & 7;
+            k = slot + ((j & 1) ? C::K2_OFF : 0) + (j >> 1) * 128 + row * 16;
+            v = slot + ((j >> 1) ? C::V2_OFF : C::V_OFF) + (j & 1) * 128 + row * 16;
+        }
+    }
+};
+__device__ __forceinline__ void lds_frag(uint32_t addr, uint32_t (&a)[4]) {
+    asm volatile("ld.shared.v4.b32 {%0,%1,%2,%3}, [%4];\n" : "=r"(a[0]), "=r"(a[1]), "=r"(a[2]), "=r"(a[3]) : "r"(addr));
+}
+__device__ __forceinline__ void ldmatrix_frag(uint32_t addr, uint32_t (&a)[4]) {
+    asm volatile("ldmatrix.sync.aligned.m8n8.x4.shared.b16 {%0,%1,%2,%3}, [%4];\n" : "=r"(a[0]), "=r"(a[1]), "=r"(a[2]), "=r"(a[3]) : "r"(addr));
+}
+__device__ __forceinline__ uint4 lds_u4(uint32_t addr) {
+    uint4 x;
+    asm volatile("ld.shared.v4.b32 {%0,%1,%2,%3}, [%4];\n" : "=r"(x.x), "=r"(x.y), "=r"(x.z), "=r"(x.w) : "r"(addr));
+    return x;
+}
+// A fragments of k-step ks of the key part (plane pl)
+template <int D, bool X3, int CR>
+__device__ __forceinline__ void key_frag(const LaneBase<D, X3, CR>& s, int pl, int ks, uint32_t (&a)[4]) {
+    using C = TForm<D, X3, CR>;
+    if constexpr (CR == 16) lds_frag(s.k + pl * C::PART + ks * 512, a);
+    else ldmatrix_frag(s.k + pl * C::PART + ks * 256, a);
+}
+// A fragments of output tile i of the value part: dims VB*g + 2i (row g) and VB*g + 2i + 1 (row g + 8)
+template <int D, bool X3, int CR>
+__device__ __forceinline__ void value_frag(const LaneBase<D, X3, CR>& s, int pl, int i, uint32_t (&a)[4]) {
+    using C = TForm<D, X3, CR>;
+    if constexpr (CR == 16) lds_frag(s.k + C::V_OFF + pl * C::PART + i * 512, a);
+    else ldmatrix_frag(s.v + pl * C::PART + i * 256, a);
+}
+// d = A B with a zero accumulator (no registers to clear)
+template <typename T> __device__ __forceinline__ void mma_zero(float (&c)[4], const uint32_t (&a)[4], uint32_t b0, uint32_t b1);
+template <> __device__ __forceinline__ void mma_zero<__half>(float (&c)[4], const uint32_t (&a)[4], uint32_t b0, uint32_t b1) {
+    asm volatile("mma.sync.aligned.m16n8k16.row.col.f32.f16.f16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%10,%10,%10,%10};\n"
+                 : "=f"(c[0]), "=f"(c[1]), "=f"(c[2]), "=f"(c[3])
+                 : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1), "f"(0.f));
+}
+template <> __device__ __forceinline__ void mma_zero<__nv_bfloat16>(float (&c)[4], const uint32_t (&a)[4], uint32_t b0, uint32_t b1) {
+    asm volatile("mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%10,%10,%10,%10};\n"
+                 : "=f"(c[0]), "=f"(c[1]), "=f"(c[2]), "=f"(c[3])
+                 : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1), "f"(0.f));
+}
+
+// The query heads of a group as B fragments of the score product: lane (g, r) holds dims PPT*r + [0, PPT) of both halves of
+// head 8h + g.  16-bit path: IEEE half pairs; split-half path: fp32 values, already multiplied by the softmax scale.
+template <typename T, int D, bool X3, int NH>
+struct QueryRegs {
+    static constexpr int N = X3 ? D / 8 : D / 16;
+    uint32_t v[NH][2][N];
+};
+
+template <typename T, int D>
+__device__ __forceinline__ void load_row_piece_f32(const T* p, bool on, float (&o)[D / 8]) {
+#pragma unroll
+    for (int i = 0; i < D / 8; i += 4) {
+        float x[4] = {0.f, 0.f, 0.f, 0.f};
+        if (on) load4<T>(p + i, x);
+#pragma unroll
+        for (int u = 0; u < 4; ++u) o[i + u] = x[u];
+    }
+}
+
+template <typename T, int D, bool X3, int NH>
+__device__ __forceinline__ void load_query(const T* base, int G, int g, int r, float scale, QueryRegs<T, D, X3, NH>& q) {
+    constexpr int HALF = D / 2, PPT = HALF / 4;
+#pragma unroll
+    for (int h = 0; h < NH; ++h) {
+        const int head = 8 * h + g;
+        const bool on = head < G;
+#pragma unroll
+        for (int hf = 0; hf < 2; ++hf) {
+            const T* p = base + (int64_t)head * D + hf * HALF + PPT * r;
+            if constexpr (X3) {
+                float x[D / 8];
+                load_row_piece_f32<T, D>(p, on, x);
+#pragma unroll
+                for (int i = 0; i < D / 8; ++i) q.v[h][hf][i] = __float_as_uint(x[i] * scale);
+            } else {
+                ldg_vec<PPT / 8>(p, on, q.v[h][hf]);
+                if (!std::is_same<T, __half>::value) {
+#pragma unroll
+                    for (int i = 0; i < D / 16; ++i) {
+                        const float2 f = Frag<__nv_bfloat16>::unpack(q.v[h][hf][i]);
+                        q.v[h][hf][i] = Frag<__half>::pack(fminf(fmaxf(f.x, -65504.f), 65504.f), fminf(fmaxf(f.y, -65504.f), 65504.f));
+                    }
+                }
+            }
+        }
+    }
+}
+
+// B fragments of k-step ks: the query rotated by the chunk's distance.  `tab` is the chunk's table row in shared memory.
+template <int D>
+struct TabRegs16 {
+    uint32_t c[D / 16], s[D / 16];
+};
+template <int D>
+__device__ __forceinline__ void load_tab16(uint32_t tab, int r, TabRegs16<D>& t) {
+    constexpr int HALF = D / 2, PPT = HALF / 4, KS = D / 16;
+#pragma unroll
+    for (int i = 0; i < KS / 4; ++i) {
+        const uint4 c4 = lds_u4(tab + 2 * (PPT * r) + 16 * i);
+        const uint4 s4 = lds_u4(tab + 2 * HALF + 2 * (PPT * r) + 16 * i);
+        t.c[4 * i] = c4.x; t.c[4 * i + 1] = c4.y; t.c[4 * i + 2] = c4.z; t.c[4 * i + 3] = c4.w;
+        t.s[4 * i] = s4.x; t.s[4 * i + 1] = s4.y; t.s[4 * i + 2] = s4.z; t.s[4 * i + 3] = s4.w;
+    }
+}
+__device__ __forceinline__ __half2 as_h2(uint32_t x) { return *reinterpret_cast<const __half2*>(&x); }
+__device__ __forceinline__ uint32_t as_u32(__half2 x) { return *reinterpret_cast<const uint32_t*>(&x); }
+// (lo, hi) rotated by (c, s): lo*c - hi*s, lo*s + hi*c
+__device__ __forceinline__ void rotate_h2(uint32_t lo, uint32_t hi, uint32_t c, uint32_t s, uint32_t& x, uint32_t& y) {
+    x = as_u32(__hfma2(as_h2(lo), as_h2(c), __hneg2(__hmul2(as_h2(hi), as_h2(s)))));
+    y = as_u32(__hfma2(as_h2(hi), as_h2(c), __hmul2(as_h2(lo), as_h2(s))));
+}
+
+// S^T of one chunk: S[h] = C fragment, rows = children g and g + 8, columns = heads 8h + 2r, 8h + 2r + 1.
+template <typename T, int D, int NH, int CR>
+__device__ __forceinline__ void score16(const LaneBase<D, false, CR>& s, uint32_t tab, int r, const QueryRegs<T, D, false, NH>& q, float (&S)[NH][4]) {
+    using FS = Frag<__half>;
+    constexpr int KS = D / 16;
+    TabRegs16<D> t;
+    load_tab16<D>(tab, r, t);
+    float U[NH][4];
+#pragma unroll
+    for (int ks = 0; ks < KS; ++ks) {
+        uint32_t a[4];
+        key_frag<D, false, CR>(s, 0, ks, a);
+#pragma unroll
+        for (int h = 0; h < NH; ++h) {
+            uint32_t b0, b1;
+            rotate_h2(q.v[h][0][ks], q.v[h][1][ks], t.c[ks], t.s[ks], b0, b1);
+            if (ks < 2) mma_zero<__half>(ks ? U[h] : S[h], a, b0, b1);         // two accumulation chains
+            else FS::mma((ks & 1) ? U[h] : S[h], a[0], a[1], a[2], a[3], b0, b1);
+        }
+    }
+#pragma unroll
+    for (int h = 0; h < NH; ++h)
+#pragma unroll
+        for (int i = 0; i < 4; ++i) S[h][i] += U[h][i];
+}
+
+// Split-half form (see mma_common.cuh for why the leading product of every k-step is summed with ordinary fp32 adds).
+// KEEP: the rotated query's hi / lo fragments are returned as well.
+template <typename T, int D, int NH, int CR>
+__device__ __forceinline__ void score_x3(const LaneBase<D, true, CR>& s, uint32_t tab, int r, const QueryRegs<T, D, true, NH>& q, float (&S)[NH][4]) {
+    using FS = Frag<__half>;
+    constexpr int KS = D / 16, HALF = D / 2, PPT = HALF / 4;
+    tab += 4 * PPT * r;
+    float B[NH][4], C[NH][4];
+#pragma unroll
+    for (int kp = 0; kp < KS / 2; ++kp) {
+        const uint4 c4 = lds_u4(tab + 16 * kp), s4 = lds_u4(tab + 4 * HALF + 16 * kp);
+        const float cs[4] = {__uint_as_float(c4.x), __uint_as_float(c4.y), __uint_as_float(c4.z), __uint_as_float(c4.w)};
+        const float sn[4] = {__uint_as_float(s4.x), __uint_as_float(s4.y), __uint_as_float(s4.z), __uint_as_float(s4.w)};
+#pragma unroll
+        for (int u = 0; u < 2; ++u) {
+            const int ks = 2 * kp + u;
+            uint32_t ah[4], al[4];
+            key_frag<D, true, CR>(s, 0, ks, ah);
+            key_frag<D, true, CR>(s, 1, ks, al);
+            const float2 c2 = make_float2(cs[2 * u], cs[2 * u + 1]), s2 = make_float2(sn[2 * u], sn[2 * u + 1]);
+            const float2 n2 = make_float2(-s2.x, -s2.y);
+#pragma unroll
+            for (int h = 0; h < NH; ++h) {
+                const float2 lo = make_float2(__uint_as_float(q.v[h][0][2 * ks]), __uint_as_float(q.v[h][0][2 * ks + 1]));
+                const float2 hi = make_float2(__uint_as_float(q.v[h][1][2 * ks]), __uint_as_float(q.v[h][1][2 * ks + 1]));
+                float2 x, y;
+                rotate_pairs_f32(lo, hi, c2, s2, n2, x, y);
+                uint32_t b0h, b0l, b1h, b1l;
+                split_half2(x.x, x.y, b0h, b0l);
+                split_half2(y.x, y.y, b1h, b1l);
+                if (ks == 0) {
+                    mma_zero<__half>(S[h], ah, b0h, b1h);
+                    mma_zero<__half>(B[h], al, b0h, b1h);
+                    mma_zero<__half>(C[h], ah, b0l, b1l);
+                } else {
+                    float t[4];
+                    mma_zero<__half>(t, ah, b0h, b1h);
+                    FS::mma(B[h], al[0], al[1], al[2], al[3], b0h, b1h);
+                    FS::mma(C[h], ah[0], ah[1], ah[2], ah[3], b0l, b1l);
+#pragma unroll
+                    for (int i = 0; i < 4; ++i) S[h][i] += t[i];
+                }
+            }
+        }
+    }
+#pragma unroll
+    for (int h = 0; h < NH; ++h)
+#pragma unroll
+        for (int i = 0; i < 4; ++i) S[h][i] += B[h][i] + C[h][i];
+}
+
+template <typename T, int D, bool X3, int NH, int CR>
+__device__ __forceinline__ void score_t(const LaneBase<D, X3, CR>& s, uint32_t tab, int r, const QueryRegs<T, D, X3, NH>& q, float (&S)[NH][4]) {
+    if constexpr (X3) score_x3<T, D, NH, CR>(s, tab, r, q, S);
+    else score16<T, D, NH, CR>(s, tab, r, q, S);
+}
+
+// One warp's ring of chunk slots in shared memory, filled by bulk copies the warp issues itself.  Waits are bounded; after
+// one ran out the caller flags status bit 16 and leaves through drain().
+template <int NSTG, int SLOT>
+struct ChunkRing {
+    uint32_t base;                 // 32-bit shared address: NSTG * SLOT bytes, then NSTG barriers
+    uint32_t is = 0, cs = 0;       // stage the next issue / the next wait uses
+    uint32_t parity = 0;           // phase parity of the next wait
+    uint32_t flying = 0;
+    static constexpr size_t kBytes = (size_t)NSTG * SLOT + 128;
+    static constexpr int kWaitCap = 1 << 16;
+
+    __device__ __forceinline__ void init(unsigned char* b, int lane) {
+        base = smem_u32(b);
+        if (lane == 0) {
+            for (int i = 0; i < NSTG; ++i) mbar_init(reinterpret_cast<uint64_t*>(b + (size_t)NSTG * SLOT) + i, 1);
+            fence_barrier_init();
+        }
+        __syncwarp();
+    }
+    __device__ __forceinline__ uint32_t bar(uint32_t stage) const { return base + NSTG * SLOT + 8 * stage; }
+    __device__ __forceinline__ void expect(uint32_t bytes) const {
+        asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;\n" ::"r"(bar(is)), "r"(bytes) : "memory");
+    }
+    __device__ __forceinline__ void copy(uint32_t off, const void* src, uint32_t bytes) const {
+        asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];\n" ::"r"(base + is * SLOT + off),
+                     "l"(src), "r"(bytes), "r"(bar(is))
+                     : "memory");
+    }
+    __device__ __forceinline__ void issued() { is = is + 1 == NSTG ? 0 : is + 1; ++flying; }
+    __device__ __forceinline__ bool wait_stage(uint32_t stage, uint32_t par) const {
+        for (int it = 0; it < kWaitCap; ++it) {
+            uint32_t ok;
+            asm volatile("{\n.reg .pred p;\nmbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\nselp.u32 %0, 1, 0, p;\n}\n"
+                         : "=r"(ok) : "r"(bar(stage)), "r"(par) : "memory");
+            if (ok) return true;
+        }
+        return false;
+    }
+    // waits for the oldest chunk; its slot is `slot` until the next issue after the next __syncwarp
+    __device__ __forceinline__ bool wait(uint32_t& slot) {
+        slot = base + cs * SLOT;
+        const bool ok = wait_stage(cs, parity);
+        if (++cs == NSTG) { cs = 0; parity ^= 1; }
+        --flying;
+        return ok;
+    }
+    __device__ __forceinline__ void drain() {
+        uint32_t slot;
+        while (flying) wait(slot);
+    }
+};
+
+}  // namespace htree

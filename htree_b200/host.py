@@ -184,8 +184,9 @@ def _by_units(q, k, v, dO, outs, dev, streams, compression_rate, max_top_nodes, 
                     kv_ready = torch.cuda.Event(); kv_ready.record(s_in)
                 with torch.cuda.stream(s_run):
                     s_run.wait_event(kv_ready)
-                    layers = ops.build_tree(k_d, v_d, compression_rate, max_top_nodes, rope_base)
-                held([k_d, v_d] + [x for lv in layers if lv is not None for x in lv])
+                    layers = ops.build_operands(k_d, v_d, compression_rate, max_top_nodes, rope_base, backward=bwd)
+                held([k_d, v_d] + [x for lv in layers if lv is not None for x in lv if x is not None] +
+                     list(getattr(layers[3], "blocks_bwd", None) or []))
                 acc = {}
                 windows = windows_edge if b * H_kv + hk in (0, n_units - 1) else windows_all
                 for wi, (t0, t1) in enumerate(windows):

@@ -40,7 +40,7 @@ SAVE_SELECTIONS_FOR_BACKWARD = True
 SELECTION_STORAGE = "int32"
 
 # Largest temporary the forward may allocate for handing selections from its selection kernel to its accumulation
-# kernel when the caller does not keep them (see htree_forward); above it the fused single-kernel forward runs.
+# kernel when the caller does not keep them (see htree_forward); above it the queries run window by window.
 SPLIT_FORWARD_MAX_BYTES = 4 << 30
 
 
@@ -108,6 +108,24 @@ def rope_cache_half(k_dim: int, cache_size: int, rope_base: float, scale: float,
         c, s = rope_cache(k_dim, cache_size, rope_base, device)
         hit = ((c * float(scale)).to(torch.float16).contiguous(), (s * float(scale)).to(torch.float16).contiguous())
         _rope_half[key] = hit
+    return hit
+
+
+_rope_rows: Dict[Tuple, torch.Tensor] = {}
+
+
+def rope_rows(k_dim: int, cache_size: int, rope_base: float, scale: Optional[float], device) -> torch.Tensor:
+    """The rotary table of the transposed tensor-core kernels: rows [cos | sin] of width k_dim, float16 multiplied by
+    `scale`, or plain fp32 when scale is None (split-half kernels)."""
+    key = (k_dim, cache_size, rope_base, scale, device)
+    hit = _rope_rows.get(key)
+    if hit is None:
+        c, s = rope_cache(k_dim, cache_size, rope_base, device)
+        if scale is None:
+            hit = torch.cat([c, s], dim=1).contiguous()
+        else:
+            hit = torch.cat([(c * float(scale)).to(torch.float16), (s * float(scale)).to(torch.float16)], dim=1).contiguous()
+        _rope_rows[key] = hit
     return hit
 
 
@@ -210,12 +228,157 @@ def build_tree(k: torch.Tensor, v: torch.Tensor, compression_rate: int, max_top_
 
 
 class OperandBlocks(list):
-    """The blocked values of every level (the list itself) together with the blocked keys of every level (`.keys`, or
-    None where the pipelined kernels do not apply): the per-parent operand copies of the tensor-core forward."""
+    """Per-parent operand copies of every level.  As written by build_tree(rope_base=...) and block_values: the blocked values
+    (the list itself) and the blocked keys (`.keys`, or None).  As written by build_operands and kept in a forward's context:
+    the combined key/value blocks the transposed kernels read (the list itself, also `.keys` and `.blocks`) and, when a
+    backward follows, its part (`.blocks_bwd`)."""
 
-    def __init__(self, values, keys=None):
+    def __init__(self, values, keys=None, blocks=None, blocks_bwd=None):
         super().__init__(values)
         self.keys = keys
+        self.blocks = blocks
+        self.blocks_bwd = blocks_bwd
+
+
+def _transposed(dtype, K: int, V: int, G: int, compression_rate: int) -> bool:
+    """Shapes with transposed tensor-core kernels (any storage type)."""
+    return K == V and K in (32, 64, 128) and int(compression_rate) in (8, 16) and G <= 16
+
+
+def _split(dtype, K: int) -> bool:
+    """Operands carried as hi + lo half planes: fp32 storage, and 32-wide heads in every storage type."""
+    return dtype == torch.float32 or K == 32
+
+
+def _selects_on_tensor_cores(dtype, K: int) -> bool:
+    return K == 64 or (K == 128 and dtype != torch.float32)
+
+
+_plans: Dict[Tuple, Tuple] = {}
+
+
+def _plan(shape: "_lib.HtreeShape", flags: int) -> "_lib.HtreePlan":
+    """Workspace layout of a forward (htree_b200_plan), kept per shape."""
+    key = (shape.B, shape.T, shape.H, shape.H_kv, shape.K, shape.compression_rate, shape.top_k, shape.max_top_nodes, shape.dtype,
+           shape.T_q, flags)
+    plan = _plans.get(key)
+    if plan is None:
+        plan = _lib.HtreePlan()
+        _lib.check(_lib.lib().htree_b200_plan(ctypes.byref(shape), flags, ctypes.byref(plan)), "plan")
+        if len(_plans) >= 512:       # layouts are cheap to redo: callers with ever-changing lengths do not grow this for ever
+            _plans.clear()
+        _plans[key] = plan
+    return plan
+
+
+def _carve(ws: torch.Tensor, offset: int, shape, dtype) -> torch.Tensor:
+    n = dtype.itemsize
+    for x in shape:
+        n *= x
+    return ws[offset:offset + n].view(dtype).view(shape)
+
+
+class _Workspace:
+    """One buffer with everything a forward derived from k and v, and views of its parts in the reference's layouts."""
+
+    def __init__(self, ws, plan, k, v, cr):
+        self.ws, self.plan, self.k, self.v, self.cr = ws, plan, k, v, cr
+
+    def _levels(self, offsets, first, D, dtype, lead=()):
+        B, _, H_kv, _ = self.k.shape
+        out = [first] if first is not None else []
+        for l in range(len(out), self.plan.levels):
+            out.append(_carve(self.ws, offsets[l], tuple(lead) + (B, self.plan.nodes[l], H_kv, D), dtype) if offsets[l] >= 0 else None)
+        return out
+
+    def layers_k(self):
+        return self._levels(self.plan.layers_k, self.k, self.k.shape[3], self.k.dtype)
+
+    def layers_v(self):
+        return self._levels(self.plan.layers_v, self.v, self.v.shape[3], self.v.dtype)
+
+    def layers_k_rot(self):
+        if not _selects_on_tensor_cores(self.k.dtype, self.k.shape[3]):
+            return None
+        return self._levels(self.plan.layers_k_rot, None, self.k.shape[3], torch.float16, (2,) if self.k.dtype == torch.float32 else ())
+
+    def blocks(self):
+        L, p = self.plan.levels, self.plan
+        ends = [self._block_bytes(l) for l in range(L)]
+        fwd = [self.ws[p.blocks[l]:p.blocks[l] + ends[l][0]] for l in range(L)]
+        bwd = [self.ws[p.blocks_bwd[l]:p.blocks_bwd[l] + ends[l][1]] for l in range(L)] if p.blocks_bwd[0] >= 0 else None
+        return OperandBlocks(fwd, keys=fwd, blocks=fwd, blocks_bwd=bwd)
+
+    def _block_bytes(self, l):
+        B, _, H_kv, K = self.k.shape
+        n = B * ((self.plan.nodes[l] + self.cr - 1) // self.cr) * H_kv * (2 if _split(self.k.dtype, K) else 1) * K * 2 * self.cr
+        return n * (2 if self.cr == 16 else 3), n
+
+
+class BwdContext(dict):
+    """The forward's context: the reference's keys (bwd_ctx of src/parallel.py:1139-1159).  Views of the tree levels and operand
+    copies are made when they are asked for."""
+
+    _LAZY = ("layers_k", "layers_v", "layers_k_rot", "layers_v_blk", "rope_half")
+    workspace: Optional[_Workspace] = None
+
+    def __missing__(self, key):
+        if key == "rope_half":
+            ws = self.workspace
+            ok = ws is not None and _selects_on_tensor_cores(ws.k.dtype, ws.k.shape[3])
+            val = rope_cache_half(ws.k.shape[3], self["cos_cache"].shape[0], self["rope_base"], self["scale"], ws.k.device) if ok else None
+        elif key in self._LAZY and self.workspace is not None:
+            val = self.workspace.blocks() if key == "layers_v_blk" else getattr(self.workspace, key)()
+        else:
+            raise KeyError(key)
+        self[key] = val
+        return val
+
+    def get(self, key, default=None):
+        try:
+            return self[key]
+        except KeyError:
+            return default
+
+    def __contains__(self, key):
+        return super().__contains__(key) or key in self._LAZY
+
+    def drop_tree(self):
+        """Forget everything derived from k and v (a backward then rebuilds it)."""
+        self.workspace = None
+        for key in ("layers_k", "layers_v", "layers_k_rot", "layers_v_blk"):
+            self[key] = None
+
+
+def build_operands(k: torch.Tensor, v: torch.Tensor, compression_rate: int, max_top_nodes: int, rope_base: float,
+                   layers=None, backward: bool = False):
+    """(layers_k, layers_v, layers_k_rot, OperandBlocks) in the form the transposed tensor-core kernels read, for a forward with
+    `_layers`; from k, v alone, or from existing levels `layers` = (layers_k, layers_v).  None in the last two places for
+    shapes without such kernels."""
+    k = k.contiguous(); v = v.contiguous()
+    B, T, H_kv, K = k.shape
+    if not _transposed(k.dtype, K, v.shape[-1], 1, compression_rate):
+        lk, lv = (list(layers[0]), list(layers[1])) if layers is not None else build_tree(k, v, compression_rate, max_top_nodes)
+        return lk, lv, None, None
+    cr = int(compression_rate)
+    sizes = _lib.level_sizes(T, cr, max_top_nodes)
+    shape = _lib.HtreeShape(B, T, H_kv, H_kv, K, K, cr, sizes[-1], int(max_top_nodes), _DTYPES[k.dtype])
+    dev = k.device
+    if layers is None:
+        lk = [k] + [torch.empty(B, n, H_kv, K, dtype=k.dtype, device=dev) for n in sizes[1:]]
+        lv = [v] + [torch.empty(B, n, H_kv, K, dtype=v.dtype, device=dev) for n in sizes[1:]]
+    else:
+        lk, lv = list(layers[0]), list(layers[1])
+    n_blk = lambda l, bwd: int(_lib.lib().htree_b200_operand_block_bytes(ctypes.byref(shape), l, bwd))
+    blocks = [torch.empty(n_blk(l, 0), dtype=torch.uint8, device=dev) for l in range(len(sizes))]
+    bwd = [torch.empty(n_blk(l, 1), dtype=torch.uint8, device=dev) for l in range(len(sizes))] if backward else None
+    lkr = [_rotated_like(x) if l or backward else None for l, x in enumerate(lk)] if _selects_on_tensor_cores(k.dtype, K) else None
+    cos_c, sin_c = rope_cache(K, 16, rope_base, dev)
+    with torch.cuda.device(dev):
+        _lib.check(_lib.lib().htree_b200_prepare(ctypes.byref(shape), _ptrs(lk), _ptrs(lv), _ptrs(blocks), _ptrs(bwd) if bwd else None,
+                                                 _ptrs(lkr) if lkr else None, int(layers is None), cos_c.data_ptr(), sin_c.data_ptr(),
+                                                 _stream()), "prepare")
+    return lk, lv, lkr, OperandBlocks(blocks, keys=blocks, blocks=blocks, blocks_bwd=bwd)
 
 
 def _pipelined(dtype, K: int, compression_rate: int) -> bool:
@@ -337,6 +500,9 @@ def htree_forward(
     with a third element — {"num_layers", "num_groups", "layers": {l: LayerTrace}} — when `return_trace` is set
     (the shape of htree_forward_naive's trace, src/naive.py:225-234).
 
+    `_fused` bounds the temporaries of a call that keeps no selections (windows of queries, see SPLIT_FORWARD_MAX_BYTES);
+    `_no_pipeline` is accepted and has no effect (there is one accumulation kernel); `_tiled` concerns the generic kernels.
+
     Sequence sharding: with `_q_offset` = t0, q holds only the query positions t0 .. t0+q.shape[1]-1 while k, v (or the
     prebuilt tree `_layers` = (layers_k, layers_v)) cover the whole sequence; outputs have q's length."""
     shape = _validate(q, k, v, compression_rate, max_top_nodes, top_k_per_layer, _q_offset)
@@ -345,69 +511,38 @@ def htree_forward(
     if scale is None:
         scale = K ** -0.5
     q = q.contiguous(); k = k.contiguous(); v = v.contiguous()
+    if (not (_force_generic or return_trace) and _transposed(q.dtype, K, V, H // H_kv, compression_rate) and q.data_ptr() % 32 == 0
+            and k.data_ptr() % 16 == 0 and v.data_ptr() % 16 == 0):
+        return _forward_transposed(shape, q, k, v, scale, rope_base, _save_for_backward, _save_parents, _layers, _fused)
     dev = q.device
     if _layers is not None:
         layers_k, layers_v = _layers[0], _layers[1]
-        layers_kr = _layers[2] if len(_layers) > 2 else None
-        layers_vb = _layers[3] if len(_layers) > 3 else None
-        if layers_kr is not None and layers_vb is None:
-            layers_vb = block_values(layers_v, compression_rate, max_top_nodes, layers_kr)
     else:
-        layers_k, layers_v, layers_kr, layers_vb = build_tree(k, v, compression_rate, max_top_nodes, rope_base)
-    if layers_vb is None:
-        layers_kr = None          # the tensor-core forward needs both operand copies
+        layers_k, layers_v = build_tree(k, v, compression_rate, max_top_nodes)
     L = len(layers_k)
     cos_cache, sin_cache = rope_cache(K, top_k_per_layer * compression_rate + 1024, rope_base, dev)
     out = torch.empty(B, T, H, V, dtype=q.dtype, device=dev)
     gmax = torch.empty(B, T, H, dtype=torch.float32, device=dev)
     gsum = torch.empty(B, T, H, dtype=torch.float32, device=dev)
     want_parents = (_save_for_backward and _save_parents) or return_trace
-    # The tensor-core forward is faster as selection kernel + accumulation kernel, which hand the selections over in
-    # buffers of L * B * T * H_kv * top_k ids (cfg3: 805 MB as int32; 2.1 GB per level at the reference's default top_k of
-    # 512 with the same shape).  A caller who does not keep the selections gets them only as temporaries, in int32
-    # whatever SELECTION_STORAGE says, and only up to SPLIT_FORWARD_MAX_BYTES: beyond it the single fused kernel runs,
-    # which needs no buffers and gives identical results.
-    split_forward = layers_kr is not None and not (_force_generic or return_trace or _fused)
-    if want_parents:
-        pdt = _parents_dtype(layers_k, top_k_per_layer)
-    else:
-        pdt = torch.int32
-        if split_forward and L * B * q.shape[1] * H_kv * top_k_per_layer * 4 > SPLIT_FORWARD_MAX_BYTES:
-            split_forward = False
-    parents = [torch.empty(B, q.shape[1], H_kv, top_k_per_layer, dtype=pdt, device=dev) for _ in range(L)] \
-        if (want_parents or split_forward) else None
+    parents = [torch.empty(B, q.shape[1], H_kv, top_k_per_layer, dtype=_parents_dtype(layers_k, top_k_per_layer), device=dev)
+               for _ in range(L)] if want_parents else None
     trace = tr = None
     if return_trace:
         tr = (torch.empty(L, B, T, H, dtype=torch.float32, device=dev),
               torch.empty(L, B, T, H, dtype=torch.float32, device=dev),
               torch.empty(L, B, T, H, V, dtype=torch.float32, device=dev))
         trace = _lib.HtreeTrace(tr[0].data_ptr(), tr[1].data_ptr(), tr[2].data_ptr())
-    flags = _lib.FWD_GENERIC if (_force_generic or return_trace) else (_lib.FWD_FUSED if _fused else 0)
-    if _tiled:
-        flags |= _lib.FWD_TILED
-    if _no_pipeline:
-        flags |= _lib.FWD_NO_PIPELINE
-    flags |= _parents_flag(parents)
-    half_tables = rope_cache_half(K, cos_cache.shape[0], rope_base, scale, dev) if layers_kr is not None else None
-    _run_forward(shape, q, layers_k, layers_v, cos_cache, sin_cache, scale, out, gmax, gsum, parents, trace, flags,
-                 layers_kr, half_tables, layers_vb)
+    flags = _lib.FWD_GENERIC | (_lib.FWD_TILED if _tiled else 0) | _parents_flag(parents)
+    _run_forward(shape, q, layers_k, layers_v, cos_cache, sin_cache, scale, out, gmax, gsum, parents, trace, flags)
     if not (_save_for_backward or return_trace):
         return out
     result = [out]
     if _save_for_backward:
-        G = H // H_kv
         result.append(dict(
-            global_max=gmax, global_sum=gsum,
+            _context_fields(gmax, gsum, cos_cache, sin_cache, L, shape, rope_base, scale),
             per_layer_parents={l: parents[l] for l in range(L)} if (_save_parents and want_parents) else None,
-            layers_k=layers_k, layers_v=layers_v, layers_k_rot=layers_kr, layers_v_blk=layers_vb,
-            cos_cache=cos_cache, sin_cache=sin_cache,
-            rope_half=half_tables,
-            num_layers=L, rope_base=rope_base,
-            compression_rate=compression_rate, top_k_per_layer=top_k_per_layer, max_top_nodes=max_top_nodes,
-            scale=scale, NUM_GROUPS=G,
-            # tuning constants of the reference's Triton kernels; kept so that code reading them keeps working
-            G_PAD=max(16, 1 << (G - 1).bit_length()), TILE_P=4, DROP_BLOCK=64,
-        ))
+            layers_k=layers_k, layers_v=layers_v, layers_k_rot=None, layers_v_blk=None, rope_half=None))
     if return_trace:
         check_status(dev)
         layers = {l: LayerTrace(l, decode_parents(parents[l - 1]) if l > 0 else None, tr[0][l], tr[1][l], tr[2][l])
@@ -415,6 +550,121 @@ def htree_forward(
         result.append({"num_layers": L, "num_groups": H // H_kv, "selection_mode": "parallel_importance",
                        "layers": layers})
     return tuple(result)
+
+
+def _context_fields(gmax, gsum, cos_cache, sin_cache, L, shape, rope_base, scale) -> dict:
+    G = shape.H // shape.H_kv
+    return dict(global_max=gmax, global_sum=gsum, cos_cache=cos_cache, sin_cache=sin_cache, num_layers=L, rope_base=rope_base,
+                compression_rate=shape.compression_rate, top_k_per_layer=shape.top_k, max_top_nodes=shape.max_top_nodes, scale=scale,
+                NUM_GROUPS=G,
+                # tuning constants of the reference's Triton kernels; kept so that code reading them keeps working
+                G_PAD=max(16, 1 << (G - 1).bit_length()), TILE_P=4, DROP_BLOCK=64)
+
+
+def _forward_transposed(shape, q, k, v, scale, rope_base, save, save_parents, given_layers, windows):
+    """The forward on the transposed tensor-core kernels: operand preparation, selection, accumulation."""
+    B, Tq, H, K = q.shape
+    H_kv, TK, CR = shape.H_kv, shape.top_k, shape.compression_rate
+    dev, dtype = q.device, q.dtype
+    n_pos = TK * CR + 1024
+    cos_cache, sin_cache = rope_cache(K, n_pos, rope_base, dev)
+    table = rope_rows(K, n_pos, rope_base, None if _split(dtype, K) else scale, dev)
+    keep = save and save_parents
+    # Callers that do not keep the selections get them only as temporaries (int32 whatever SELECTION_STORAGE says), and only up
+    # to SPLIT_FORWARD_MAX_BYTES at a time: beyond it the queries run window by window over the same tree, with the same results.
+    plan = _plan(shape, _lib.PLAN_BACKWARD if save else 0)
+    L = plan.levels
+    out = torch.empty(B, Tq, H, K, dtype=dtype, device=dev)
+    stats = torch.empty(2, B, Tq, H, dtype=torch.float32, device=dev)
+    per_query = L * H_kv * TK * 4
+    if not keep and (windows or B * Tq * per_query > SPLIT_FORWARD_MAX_BYTES):
+        layers = _operand_layers(k, v, shape, rope_base, given_layers, save)
+        _forward_windows(shape, q, layers, cos_cache, sin_cache, table, scale, out, stats[0], stats[1], per_query)
+        parents = ws = None
+    else:
+        pdt = torch.int32
+        if keep:
+            pdt = _parents_dtype_of(plan, TK)
+        parents = torch.empty(L, B, Tq, H_kv, TK, dtype=pdt, device=dev)
+        flags = (0 if save or given_layers is not None else _lib.FWD_INFERENCE) | (_lib.PARENTS_U16 if pdt == torch.int16 else 0)
+        p0, step = parents.data_ptr(), B * Tq * H_kv * TK * pdt.itemsize
+        pptr = _lib.ptr_array([p0 + l * step for l in range(L)])
+        gmax_ptr = stats.data_ptr()
+        gsum_ptr = gmax_ptr + B * Tq * H * 4
+        with torch.cuda.device(dev):
+            if given_layers is None:
+                ws = torch.empty(plan.bytes, dtype=torch.uint8, device=dev)
+                rc = _lib.lib().htree_b200_run_forward(
+                    ctypes.byref(shape), ctypes.byref(plan), q.data_ptr(), k.data_ptr(), v.data_ptr(), cos_cache.data_ptr(),
+                    sin_cache.data_ptr(), table.data_ptr(), n_pos, scale, ws.data_ptr(), out.data_ptr(), gmax_ptr, gsum_ptr, pptr,
+                    _status(dev).data_ptr(), flags, _stream())
+                layers = None
+            else:
+                ws = None
+                layers = _operand_layers(k, v, shape, rope_base, given_layers, save)
+                rc = _attend(shape, q, layers, cos_cache, sin_cache, table, scale, out.data_ptr(), gmax_ptr, gsum_ptr, pptr, flags)
+        _lib.check(rc, "forward")
+    if not save:
+        return out
+    ctx = BwdContext(_context_fields(stats[0], stats[1], cos_cache, sin_cache, L, shape, rope_base, scale))
+    ctx["per_layer_parents"] = dict(enumerate(parents.unbind(0))) if keep else None
+    if ws is not None:
+        ctx.workspace = _Workspace(ws, plan, k, v, CR)
+    else:
+        ctx.update(layers_k=layers[0], layers_v=layers[1], layers_k_rot=layers[2], layers_v_blk=layers[3])
+        ctx["rope_half"] = rope_cache_half(K, n_pos, rope_base, scale, dev) if _selects_on_tensor_cores(dtype, K) else None
+    return out, ctx
+
+
+def _parents_dtype_of(plan, top_k: int):
+    if SELECTION_STORAGE == "int32":
+        return torch.int32
+    if SELECTION_STORAGE != "uint16":
+        raise ValueError(f"SELECTION_STORAGE must be 'int32' or 'uint16', not {SELECTION_STORAGE!r}")
+    if top_k > 65535 or any(plan.nodes[l] > 65535 for l in range(1, plan.levels)):
+        raise ValueError("SELECTION_STORAGE='uint16' needs pooled levels of at most 65535 nodes")
+    return torch.int16
+
+
+def _operand_layers(k, v, shape, rope_base, given, backward):
+    """(layers_k, layers_v, layers_k_rot, OperandBlocks) for the transposed kernels, from the caller's levels where given."""
+    if given is None:
+        return build_operands(k, v, shape.compression_rate, shape.max_top_nodes, rope_base, backward=backward)
+    if len(given) > 3 and getattr(given[3], "blocks", None) is not None and (not backward or given[3].blocks_bwd is not None):
+        return given
+    return build_operands(given[0][0], given[1][0], shape.compression_rate, shape.max_top_nodes, rope_base, layers=given, backward=backward)
+
+
+def _attend(shape, q, layers, cos_cache, sin_cache, table, scale, out_ptr, gmax_ptr, gsum_ptr, pptr, flags) -> int:
+    return _lib.lib().htree_b200_attend(
+        ctypes.byref(shape), q.data_ptr(), _ptrs(layers[0]), _ptrs(layers[1]), _ptrs(layers[2]) if layers[2] is not None else None,
+        _ptrs(layers[3].blocks), cos_cache.data_ptr(), sin_cache.data_ptr(), table.data_ptr(), cos_cache.shape[0], float(scale),
+        out_ptr, gmax_ptr, gsum_ptr, pptr, _status(q.device).data_ptr(), flags, _stream())
+
+
+def _forward_windows(shape, q, layers, cos_cache, sin_cache, table, scale, out, gmax, gsum, per_query):
+    """The forward over windows of query positions, one batch element at a time, whose selections fit
+    SPLIT_FORWARD_MAX_BYTES."""
+    B, Tq, H, K = q.shape
+    L = len(layers[0])
+    step = max(1, min(Tq, SPLIT_FORWARD_MAX_BYTES // per_query))
+    parents = torch.empty(L, step, shape.H_kv, shape.top_k, dtype=torch.int32, device=q.device)
+    pptr = _ptrs(parents.unbind(0))
+    t_offset = shape.t_offset
+    with torch.cuda.device(q.device):
+        for b in range(B):
+            one = [[x[b:b + 1] for x in layers[0]], [x[b:b + 1] for x in layers[1]],
+                   [None if x is None else (x[:, b:b + 1] if x.dim() == 5 else x[b:b + 1]) for x in layers[2]] if layers[2] is not None else None]
+            blocks = OperandBlocks([])
+            blocks.blocks = [x.view(B, -1)[b] for x in layers[3].blocks]
+            if one[2] is not None and q.dtype == torch.float32 and B > 1:      # the hi and lo planes of one element
+                one[2] = [None if x is None else x.contiguous() for x in one[2]]
+            for a in range(0, Tq, step):
+                n = min(step, Tq - a)
+                w = _lib.HtreeShape(1, shape.T, shape.H, shape.H_kv, shape.K, shape.V, shape.compression_rate, shape.top_k,
+                                    shape.max_top_nodes, shape.dtype, n, t_offset + a)
+                _lib.check(_attend(w, q[b:b + 1, a:a + n], one + [blocks], cos_cache, sin_cache, table, scale, out[b, a:].data_ptr(),
+                                   gmax[b, a:].data_ptr(), gsum[b, a:].data_ptr(), pptr, 0), "forward")
 
 
 def recompute_parents(q, layers_k, layers_v, cos_cache, sin_cache, compression_rate, top_k_per_layer,
@@ -523,16 +773,20 @@ class HTreeFunction(torch.autograd.Function):
         ctx.save_for_backward(q, k, v, output, bwd_ctx["global_max"], bwd_ctx["global_sum"])
         ctx.bwd_ctx = bwd_ctx
         if not save:   # like the reference: drop the pooled levels and rebuild them in backward
-            bwd_ctx["layers_k"] = bwd_ctx["layers_v"] = bwd_ctx["layers_k_rot"] = bwd_ctx["layers_v_blk"] = None
+            if isinstance(bwd_ctx, BwdContext):
+                bwd_ctx.drop_tree()
+            else:
+                bwd_ctx["layers_k"] = bwd_ctx["layers_v"] = bwd_ctx["layers_k_rot"] = bwd_ctx["layers_v_blk"] = None
         return output
 
     @staticmethod
     def backward(ctx, dO):
         q, k, v, output, gmax, gsum = ctx.saved_tensors
-        c = dict(ctx.bwd_ctx)
+        c = ctx.bwd_ctx
         if c["layers_k"] is None:
-            c["layers_k"], c["layers_v"], c["layers_k_rot"], c["layers_v_blk"] = build_tree(
-                k, v, c["compression_rate"], c["max_top_nodes"], c["rope_base"])
+            c = dict(c)
+            c["layers_k"], c["layers_v"], c["layers_k_rot"], c["layers_v_blk"] = build_operands(
+                k, v, c["compression_rate"], c["max_top_nodes"], c["rope_base"], backward=True)
         dq, dk, dv = htree_backward(dO.to(q.dtype), q, output, c, _typed=True)    # gradients come back in the input dtype
         return dq, dk, dv, None, None, None, None, None
 
@@ -553,7 +807,7 @@ htree_forward_triton_autograd = htree_forward_autograd   # drop-in name of the r
 
 __all__ = [
     "decode_parents", "HTREE_SCORE_NEG_INF", "HTREE_SCORE_VALID_THRESHOLD", "LayerTrace", "build_tree", "rope_cache",
-    "rotate_keys", "block_values",
+    "rotate_keys", "block_values", "build_operands",
     "htree_forward", "htree_backward", "recompute_parents", "HTreeFunction", "HTreeTritonFunction",
     "htree_forward_autograd", "htree_forward_triton_autograd", "check_status",
 ]

@@ -58,6 +58,9 @@ extern "C" {
 #define HTREE_FWD_FUSED 4u       /* tensor-core forward: keep selection and accumulation in ONE kernel even when parent
                                     buffers are provided (default then: a selection kernel followed by an accumulation kernel) */
 
+#define HTREE_FWD_INFERENCE 256u /* htree_b200_attend: no backward follows, so calls of few queries may spread a query over
+                                    several warps (whose sums are then merged: last-bit differences between call sizes) */
+
 /* backward flags: a backward may be run as several calls over consecutive query windows (HtreeShape.T_q / t_offset) that share
  * the dk_levels / dv_levels accumulators, e.g. to overlap transfers of q, dO, out and dq with the kernels.  The first call
  * passes HTREE_BWD_NO_FOLD, calls in the middle HTREE_BWD_KEEP_ACCUM | HTREE_BWD_NO_FOLD, the last one HTREE_BWD_KEEP_ACCUM;
@@ -178,6 +181,51 @@ int htree_b200_forward(const HtreeShape* shape, const void* q, void* const* laye
                        const void* sin_half, int32_t n_pos, float scale, void* out,
                        float* gmax, float* gsum, int32_t* const* parents, const HtreeTrace* trace, int32_t* status,
                        uint32_t flags, void* stream);
+
+/* The forward in two calls, for H/H_kv <= 16, K == V in {32, 64, 128}, compression_rate 8 or 16 and any storage type (others:
+ * htree_b200_forward).  Same reference kernels as htree_b200_build_tree and htree_b200_forward; no counterpart of the split.
+ * htree_b200_prepare reads every level's rows once and writes, level by level,
+ *   layers_k[l+1], layers_v[l+1]  the pooled levels (with `pool` != 0; else they are inputs that exist already)
+ *   blocks[l]      operand blocks of the forward, htree_b200_operand_block_bytes(shape, l, 0) bytes, 16-byte aligned
+ *   blocks_bwd     NULL, or L pointers to the backward's part, htree_b200_operand_block_bytes(shape, l, 1) bytes
+ *   layers_k_rot   NULL, or L pointers (each may be NULL) that receive K' rows as htree_b200_rotate_keys writes them
+ * htree_b200_attend then selects (with layers_k_rot of the pooled levels: the tensor-core selection kernel; without, or for
+ * shapes that has no form of, the fp32-arithmetic kernel on layers_k) and accumulates.
+ *   table          [n_pos, K] rows [cos(K/2) | sin(K/2)]: fp32 for fp32 storage and for K = 32, else IEEE half multiplied by scale
+ *   parents        L pointers, written by the selection and read by the accumulation (required)
+ *   q              32-byte aligned */
+int64_t htree_b200_operand_block_bytes(const HtreeShape* shape, int32_t level, int32_t backward);
+int htree_b200_prepare(const HtreeShape* shape, void* const* layers_k, void* const* layers_v, void* const* blocks,
+                       void* const* blocks_bwd, void* const* layers_k_rot, int32_t pool, const float* cos_cache,
+                       const float* sin_cache, void* stream);
+int htree_b200_attend(const HtreeShape* shape, const void* q, void* const* layers_k, void* const* layers_v, void* const* layers_k_rot,
+                      void* const* blocks, const float* cos_cache, const float* sin_cache, const void* table, int32_t n_pos,
+                      float scale, void* out, float* gmax, float* gsum, int32_t* const* parents, int32_t* status, uint32_t flags,
+                      void* stream);
+
+/* Both calls as one, for callers that keep a workspace: htree_b200_plan lays out everything a forward derives from its inputs
+ * in one buffer of plan->bytes bytes (offsets; -1 = not part of it), htree_b200_run_forward fills it and runs the forward.
+ * HTREE_PLAN_BACKWARD adds what a backward reads (blocks_bwd, K' of the leaves), HTREE_PLAN_PARENTS buffers for the
+ * selections (int32) for callers that do not pass their own. */
+#define HTREE_PLAN_BACKWARD 1u
+#define HTREE_PLAN_PARENTS 2u
+typedef struct HtreePlan {
+    int64_t bytes;
+    int64_t layers_k[HTREE_MAX_LEVELS];      /* level 0: -1 (the inputs) */
+    int64_t layers_v[HTREE_MAX_LEVELS];
+    int64_t layers_k_rot[HTREE_MAX_LEVELS];
+    int64_t blocks[HTREE_MAX_LEVELS];
+    int64_t blocks_bwd[HTREE_MAX_LEVELS];
+    int64_t parents[HTREE_MAX_LEVELS];
+    int32_t nodes[HTREE_MAX_LEVELS];
+    int32_t levels;
+    int32_t reserved;
+} HtreePlan;
+int htree_b200_plan(const HtreeShape* shape, uint32_t flags, HtreePlan* plan);
+int htree_b200_run_forward(const HtreeShape* shape, const HtreePlan* plan, const void* q, const void* k, const void* v,
+                           const float* cos_cache, const float* sin_cache, const void* table, int32_t n_pos, float scale,
+                           void* workspace, void* out, float* gmax, float* gsum, int32_t* const* parents, int32_t* status,
+                           uint32_t flags, void* stream);
 
 /* One tree level at a time (the call surface the reference's parity harness uses, correctness_test.py:168-347):
  * htree_b200_level_forward replaces one launch of htree_select_accumulate_gqa_kernel (level > 0; src/parallel.py:537-867)

@@ -39,6 +39,8 @@ SYMBOLS = (
     "htree_b200_attend",
     "htree_b200_plan",
     "htree_b200_run_forward",
+    "htree_b200_backward_plan",
+    "htree_b200_run_backward",
     "htree_b200_forward",
     "htree_b200_level_forward",
     "htree_b200_merge_to_global",
@@ -120,6 +122,11 @@ def lib() -> ctypes.CDLL:
         L.htree_b200_run_forward.restype = ctypes.c_int
         L.htree_b200_run_forward.argtypes = [ctypes.POINTER(HtreeShape), ctypes.POINTER(HtreePlan), vp, vp, vp, vp, vp, vp, i32, f32, vp,
                                              vp, vp, vp, vp, vp, u32, vp]
+        L.htree_b200_backward_plan.restype = ctypes.c_int
+        L.htree_b200_backward_plan.argtypes = [ctypes.POINTER(HtreeShape), ctypes.c_int64, vp, vp]
+        L.htree_b200_run_backward.restype = ctypes.c_int
+        L.htree_b200_run_backward.argtypes = [ctypes.POINTER(HtreeShape), vp, vp, vp, vp, vp, vp, i32, f32, vp, vp, vp, vp, vp, vp, vp,
+                                              ctypes.c_int64, vp, vp, vp, i32, vp, u32, vp]
         L.htree_b200_level_forward.restype = ctypes.c_int
         L.htree_b200_level_forward.argtypes = [ctypes.POINTER(HtreeShape), i32, i32, vp, vp, vp, vp, vp, vp, i32, f32, vp, vp, vp, vp,
                                                vp, vp]

@@ -112,9 +112,10 @@ acc_mma_kernel(const __grid_constant__ AttnParams p) {
                     int p1 = c * PPC + 1 < np ? par[c * PPC + 1] : p0;    // past the end of the list: masked, any finite block
                     if ((unsigned)p1 >= (unsigned)nblk) { if (p.status) atomicOr(p.status, 4); p1 = 0; }
                     ring.copy(0, blk + p0 * bstride, C::DATA / 2);
-                    ring.copy(C::DATA / 2, blk + p1 * bstride + C::PL * C::PART, C::DATA / 2);
+                    ring.copy(C::DATA / 2, blk + p1 * bstride + C::ODD, C::DATA / 2);
                 }
                 ring.copy(C::DATA, tab, C::TAB);
+                if constexpr (C::DUAL) ring.copy(C::DATA + C::TAB, rp - 16 * c >= 8 ? tab - 8 * C::TAB : tab, C::TAB);
             }
             tab -= (int64_t)16 * C::TAB * step;
             ring.issued();

@@ -2,7 +2,7 @@
 #include <atomic>
 #include <cstring>
 
-#include "common.cuh"
+#include "bwd_tform.cuh"
 
 namespace htree {
 
@@ -67,6 +67,79 @@ static int fill_params(AttnParams& p, const HtreeShape* s, int L, const int32_t*
     p.CR = s->compression_rate; p.TK = s->top_k; p.L = L; p.G = s->H / s->H_kv; p.n_pos = n_pos;
     p.Tq = s->T_q > 0 ? s->T_q : s->T; p.t0 = s->t_offset;
     p.scale = scale; p.flags = flags;
+    return 0;
+}
+
+// Windows, launches and buffers of the two-pass backward for a shape and a scratch size.
+struct BwdLayout {
+    BwdParams bp;
+    int64_t acc_bytes, scratch_bytes, zero_bytes;
+    int64_t acck[HTREE_MAX_LEVELS], accv[HTREE_MAX_LEVELS], gk[HTREE_MAX_LEVELS], gv[HTREE_MAX_LEVELS];
+    int64_t o_qb, o_dob, o_stp, o_sts, o_rank, o_cnt, o_base, o_entries, o_items, o_nitems;
+    int total, per_launch;
+};
+
+static int bwd_layout(const HtreeShape* s, int L, const int32_t* ln, int64_t budget, BwdLayout& y) {
+    std::memset(&y, 0, sizeof(y));
+    const int CR = s->compression_rate, TK = s->top_k, D = s->K, G = s->H / s->H_kv;
+    if (!pack_supported(s->dtype, s->K, s->V, CR) || G > 16 || (int64_t)TK * CR > 131072) return HTREE_E_UNSUPPORTED;
+    const bool x3 = pack_split(s->dtype, D);
+    const int NH = G > 8 ? 2 : 1, Tq = s->T_q > 0 ? s->T_q : s->T;
+    BwdParams& bp = y.bp;
+    auto up = [](int64_t x) { return (x + 255) & ~int64_t(255); };
+    int64_t at = 0, MV = 0, NK = 0;
+    for (int l = L - 1; l >= 0; --l) {
+        const int64_t nblk = (ln[l] + CR - 1) / CR, np = nblk < TK ? nblk : TK;
+        const bool used = l == 0 || np * CR > TK;      // does any query accumulate here?
+        bp.voff[l] = used ? (int32_t)MV : -1;
+        bp.koff[l] = (int32_t)NK;
+        if (used) { MV += np; NK += nblk; }
+        const int64_t blocks = (int64_t)s->B * nblk * s->H_kv;
+        y.acck[l] = at; at += up(blocks * D * CR * 4);
+        y.accv[l] = at; at += up(blocks * D * CR * 4);
+    }
+    y.zero_bytes = at;
+    for (int l = 1; l < L; ++l) {
+        const int64_t bytes = up((int64_t)s->B * ln[l] * s->H_kv * D * 4);
+        y.gk[l] = at; at += bytes;
+        y.gv[l] = at; at += bytes;
+    }
+    y.acc_bytes = at;
+    const int64_t qb = (int64_t)NH * D * 16 * (x3 ? 2 : 1), sb = (int64_t)NH * (CR / 8) * 128 * (x3 ? 2 : 1);
+    const int64_t units = (int64_t)s->B * s->H_kv;
+    // A window's blocked queries (4 KB each at 16 heads of 128) should stay in the L2 while its parents gather them: 8192 queries
+    // are 33 MB; longer windows mean longer visit lists and fewer reductions.
+    int64_t subq = 0, bytes = 0;
+    for (int64_t most = 8192; most >= 16; most >>= 1) {
+        const int64_t nw = (Tq + most - 1) / most;
+        subq = (Tq + nw - 1) / nw;
+        const int64_t visits = subq * MV;
+        bytes = up(subq * qb) * 2 + up(visits * sb) * 2 + up(visits * 4) + up(visits * 8) + 2 * up(NK * 4) + up((visits / 8 + NK) * 16) + 256;
+        if (bytes <= budget && visits < (int64_t(1) << 31)) { bp.nw = (int32_t)nw; break; }
+    }
+    if (bp.nw == 0) return HTREE_E_SCRATCH;
+    bp.subq = (int32_t)subq; bp.MV = (int32_t)MV; bp.NK = (int32_t)NK;
+    y.total = (int)(units * bp.nw);
+    int64_t per = budget / bytes;
+    if (per > 32767 / subq) per = 32767 / subq;
+    if (per * subq * MV >= (int64_t(1) << 31)) per = ((int64_t(1) << 31) - 1) / (subq * MV);
+    if (per > y.total) per = y.total;
+    if (per < 1) per = 1;
+    const int64_t launches = (y.total + per - 1) / per;
+    per = (y.total + launches - 1) / launches;
+    y.per_launch = (int)per;
+    // items long enough to pay for their reduction (64 visits: 128 bytes of it a visit), short enough to fill the chip
+    int64_t seg = per * subq * MV / (148 * 16 * 3);
+    bp.seg = (int32_t)(seg < 8 ? 8 : seg > 64 ? 64 : seg);
+    bp.cap = (int32_t)(subq * MV / bp.seg + NK);
+    at = 0;
+    auto take = [&](int64_t n) { const int64_t o = at; at += up(n); return o; };
+    y.o_qb = take(per * subq * qb); y.o_dob = take(per * subq * qb);
+    y.o_stp = take(per * subq * MV * sb); y.o_sts = take(per * subq * MV * sb);
+    y.o_rank = take(per * subq * MV * 4); y.o_entries = take(per * subq * MV * 8);
+    y.o_cnt = take(per * NK * 4); y.o_base = take(per * NK * 4);
+    y.o_items = take(per * bp.cap * (int64_t)sizeof(BwdItem)); y.o_nitems = take(per * 4);
+    y.scratch_bytes = at;
     return 0;
 }
 
@@ -411,6 +484,75 @@ int htree_b200_copy_rows(void* dst, int64_t dpitch, const void* src, int64_t spi
     if (width <= 0 || height <= 0 || dpitch < width || spitch < width) return HTREE_E_SHAPE;
     return (int)cudaMemcpy2DAsync(dst, (size_t)dpitch, src, (size_t)spitch, (size_t)width, (size_t)height, cudaMemcpyDefault,
                                   (cudaStream_t)stream);
+}
+
+int htree_b200_backward_plan(const HtreeShape* shape, int64_t budget, int64_t* acc_bytes, int64_t* scratch_bytes) {
+    if (!acc_bytes || !scratch_bytes) return HTREE_E_NULL;
+    int32_t ln[HTREE_MAX_LEVELS];
+    const int L = check_shape(shape, ln);
+    if (L < 0) return L;
+    BwdLayout y;
+    const int rc = bwd_layout(shape, L, ln, budget, y);
+    if (rc) return rc;
+    *acc_bytes = y.acc_bytes; *scratch_bytes = y.scratch_bytes;
+    return 0;
+}
+
+int htree_b200_run_backward(const HtreeShape* shape, const void* q, void* const* blocks, void* const* blocks_bwd,
+                            const float* cos_cache, const float* sin_cache, const void* table, int32_t n_pos, float scale,
+                            const void* out, const void* dO, const float* gmax, const float* gsum, int32_t* const* parents,
+                            void* acc, void* scratch, int64_t budget, void* dq, void* dk, void* dv, int32_t typed, int32_t* status,
+                            uint32_t flags, void* stream) {
+    int32_t ln[HTREE_MAX_LEVELS];
+    const int L = check_shape(shape, ln);
+    if (L < 0) return L;
+    if (!q || !blocks || !blocks_bwd || !cos_cache || !sin_cache || !table || !out || !dO || !gmax || !gsum || !parents || !acc || !scratch || !dq)
+        return HTREE_E_NULL;
+    if (!(flags & HTREE_BWD_NO_FOLD) && (!dk || !dv)) return HTREE_E_NULL;
+    const bool windowed = shape->T_q != 0 && (shape->T_q != shape->T || shape->t_offset != 0);
+    if (windowed && !(flags & (HTREE_BWD_KEEP_ACCUM | HTREE_BWD_NO_FOLD))) return HTREE_E_WINDOW;
+    if ((int64_t)n_pos < (int64_t)shape->top_k * shape->compression_rate) return HTREE_E_ROPE;
+    if (!aligned32(q) || !aligned32(out) || !aligned32(dO) || !aligned16(table) || !aligned16(acc) || !aligned16(scratch) || !aligned16(dq) ||
+        !aligned16(dk) || !aligned16(dv) || !aligned16(cos_cache) || !aligned16(sin_cache))
+        return HTREE_E_ALIGN;
+    BwdLayout y;
+    int rc = bwd_layout(shape, L, ln, budget, y);
+    if (rc) return rc;
+    BwdParams& bp = y.bp;
+    // the levels themselves are not read: the block pointers stand in for them in the common checks
+    rc = fill_params(bp.a, shape, L, ln, q, blocks, blocks, cos_cache, sin_cache, n_pos, scale, parents, status, flags);
+    if (rc) return rc;
+    AttnParams& p = bp.a;
+    unsigned char *ab = static_cast<unsigned char*>(acc), *sb = static_cast<unsigned char*>(scratch);
+    float *gk[HTREE_MAX_LEVELS], *gv[HTREE_MAX_LEVELS];
+    for (int l = 0; l < L; ++l) {
+        if (!parents[l] || !blocks_bwd[l]) return HTREE_E_NULL;
+        if (!aligned16(blocks_bwd[l])) return HTREE_E_ALIGN;
+        p.blk[l] = blocks[l]; p.vkblk[l] = blocks_bwd[l];
+        bp.acck[l] = reinterpret_cast<float*>(ab + y.acck[l]); bp.accv[l] = reinterpret_cast<float*>(ab + y.accv[l]);
+        gk[l] = reinterpret_cast<float*>(ab + y.gk[l]); gv[l] = reinterpret_cast<float*>(ab + y.gv[l]);
+    }
+    p.tab = table; p.out = const_cast<void*>(out); p.dO = dO; p.gmax = const_cast<float*>(gmax); p.gsum = const_cast<float*>(gsum);
+    p.dq = typed ? nullptr : static_cast<float*>(dq); p.dq_typed = typed ? dq : nullptr;
+    bp.qb = sb + y.o_qb; bp.dob = sb + y.o_dob; bp.stp = sb + y.o_stp; bp.sts = sb + y.o_sts;
+    bp.rank = reinterpret_cast<int32_t*>(sb + y.o_rank); bp.entries = reinterpret_cast<uint2*>(sb + y.o_entries);
+    bp.cnt = reinterpret_cast<int32_t*>(sb + y.o_cnt); bp.base = reinterpret_cast<int32_t*>(sb + y.o_base);
+    bp.items = reinterpret_cast<BwdItem*>(sb + y.o_items); bp.nitems = reinterpret_cast<int32_t*>(sb + y.o_nitems);
+    cudaStream_t st = (cudaStream_t)stream;
+    if (!(flags & HTREE_BWD_KEEP_ACCUM)) {
+        const cudaError_t e = cudaMemsetAsync(acc, 0, (size_t)y.zero_bytes, st);
+        if (e != cudaSuccess) return (int)e;
+    }
+    for (int s0 = 0; s0 < y.total; s0 += y.per_launch) {
+        bp.sub0 = s0; bp.nsub = y.total - s0 < y.per_launch ? y.total - s0 : y.per_launch;
+        const cudaError_t e = cudaMemsetAsync(bp.cnt, 0, (size_t)bp.nsub * bp.NK * sizeof(int32_t), st);
+        if (e != cudaSuccess) return (int)e;
+        rc = launch_bwd_dq(bp, shape->dtype, st);
+        if (rc == 0) rc = launch_bwd_dkv(bp, shape->dtype, st);
+        if (rc) return rc;
+    }
+    if (flags & HTREE_BWD_NO_FOLD) return 0;
+    return launch_bwd_fold(bp, shape->dtype, gk, gv, dk, dv, typed != 0, st);
 }
 
 int htree_b200_backward(const HtreeShape* shape, const void* q, void* const* layers_k, void* const* layers_v,

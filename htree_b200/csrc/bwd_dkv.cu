@@ -1,0 +1,385 @@
+// Parent-stationary pass of the backward (bwd_tform.cuh): the counting sort of the visits by parent, dK and dV, and the
+// mean-pool gradient.  Replaces htree_bwd_dkv_bottom/upper_kernel and htree_bwd_tree_backward_kernel (src/backward.py:443-841).
+#include "bwd_tform.cuh"
+
+namespace htree {
+
+// One block per window: exclusive prefix sums of the parents' visit counts, and the window's work items (pieces of at most
+// `seg` visits of one parent), in parent order.
+__global__ void __launch_bounds__(1024) bwd_scan_kernel(const __grid_constant__ BwdParams bp) {
+    __shared__ int2 wsum[32];
+    const int sub = blockIdx.x, tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    const int32_t* cnt = bp.cnt + (int64_t)sub * bp.NK;
+    int32_t* base = bp.base + (int64_t)sub * bp.NK;
+    BwdItem* items = bp.items + (int64_t)sub * bp.cap;
+    const int per = (bp.NK + 1023) / 1024, k0 = tid * per, k1 = min(bp.NK, k0 + per);
+    int2 s = make_int2(0, 0);
+    for (int k = k0; k < k1; ++k) { const int c = cnt[k]; s.x += c; s.y += (c + bp.seg - 1) / bp.seg; }
+    int2 inc = s;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+        const int x = __shfl_up_sync(0xffffffffu, inc.x, o), y = __shfl_up_sync(0xffffffffu, inc.y, o);
+        if (lane >= o) { inc.x += x; inc.y += y; }
+    }
+    if (lane == 31) wsum[warp] = inc;
+    __syncthreads();
+    int2 before = make_int2(inc.x - s.x, inc.y - s.y);
+    int total = 0;
+    for (int w = 0; w < 32; ++w) {
+        if (w < warp) { before.x += wsum[w].x; before.y += wsum[w].y; }
+        total += wsum[w].y;
+    }
+    for (int k = k0; k < k1; ++k) {
+        const int c = cnt[k];
+        base[k] = before.x;
+        for (int o = 0; o < c; o += bp.seg) items[before.y++] = BwdItem{k, before.x + o, min(bp.seg, c - o), 0};
+        before.x += c;
+    }
+    if (tid == 0) bp.nitems[sub] = total;
+}
+
+// One warp per group: every visit's entry goes to its place in its parent's list.
+__global__ void __launch_bounds__(256) bwd_fill_kernel(const __grid_constant__ BwdParams bp) {
+    const AttnParams& p = bp.a;
+    const int lane = threadIdx.x & 31, qi = (int)((blockIdx.x * blockDim.x + threadIdx.x) >> 5);
+    const int sub = bp.sub0 + blockIdx.y, unit = sub / bp.nw;
+    const int tl = (sub % bp.nw) * bp.subq + qi;
+    if (qi >= bp.subq || tl >= p.Tq) return;
+    const int b = unit / p.Hkv, hk = unit % p.Hkv, TK = p.TK, CR = p.CR;
+    const int64_t grp = (int64_t)blockIdx.y * bp.subq + qi;
+    const int64_t qidx = ((int64_t)b * p.Tq + tl) * p.Hkv + hk;
+    const int t = p.t0 + tl;
+    uint2* entries = bp.entries + (int64_t)blockIdx.y * bp.subq * bp.MV;
+    for (int l = p.L - 1; l >= 0; --l) {
+        if (bp.voff[l] < 0) continue;
+        int np = 0;
+        for (int i = lane; i < TK; i += 32) np += load_parent(p, l, qidx * TK + i) >= 0;
+        np = __reduce_add_sync(0xffffffffu, np);
+        const int rp = (np - 1) * CR + (int)(((int64_t)t / p.lpow[l]) % CR);
+        if (np <= 0 || (l > 0 && rp + 1 <= TK)) continue;
+        const int nblk = (p.ln[l] + CR - 1) / CR;
+        const int32_t* base = bp.base + (int64_t)blockIdx.y * bp.NK + bp.koff[l];
+        const int32_t* cnt = bp.cnt + (int64_t)blockIdx.y * bp.NK + bp.koff[l];
+        for (int i = lane; i < np; i += 32) {
+            int x = load_parent(p, l, qidx * TK + i);
+            if ((unsigned)x >= (unsigned)nblk) x = 0;
+            const int64_t v = grp * bp.MV + bp.voff[l] + i;
+            const int rank = bp.rank[v];     // written by the first pass, except where that gave up (status 16)
+            if ((unsigned)rank < (unsigned)cnt[x]) entries[base[x] + rank] = make_uint2((uint32_t)v, (uint32_t)grp | ((uint32_t)(rp - CR * i) << 15));
+        }
+    }
+}
+
+// dK' (KEYS) or dV of one item: dX^T[dims x children] += A[dims x heads] B[heads x children] over its visits, 16 rows (heads) a
+// step: one visit of up to 16 heads, or two visits of up to 8.  A = the blocked queries rotated by the visit's distance, or the
+// blocked output gradients; B = dS or P as the first pass left them.  One warp per item, operands through the warp's ring.
+// The two gradients are separate launches: each gathers from one blocked tensor only (a window of it stays in L2) and its
+// accumulator is 64 registers, which leaves room for 16 and more warps per SM.
+template <int D, bool X3>
+constexpr int dkv_stages() { return X3 ? 2 : 3; }
+template <int D, bool X3>
+constexpr int dkv_min_blocks() { return X3 ? (D == 128 ? 2 : 3) : D == 128 ? 3 : 4; }
+
+template <typename T, int D, bool X3, int NH, int CR, bool KEYS>
+__global__ void __launch_bounds__(128, dkv_min_blocks<D, X3>()) bwd_dkv_kernel(const __grid_constant__ BwdParams bp) {
+    using BF = BForm<D, X3, NH, CR>;
+    using C = TForm<D, X3, CR>;
+    using FT = typename std::conditional<X3 || KEYS, __half, T>::type;      // operand type of the products
+    using F = Frag<FT>;
+    constexpr int KS = BF::KS, NT = BF::NT, QB = BF::QB, SB = BF::SB, PPT = C::PPT, HALF = C::HALF;
+    constexpr int TAB = KEYS ? C::TAB : 0;
+    constexpr int SLOT = 2 * QB + 2 * SB + 2 * TAB, NSTG = dkv_stages<D, X3>();
+    constexpr int PLANE = NT * 128;                                         // bytes from the hi to the lo words of a record
+    using Ring = ChunkRing<NSTG, SLOT>;
+    extern __shared__ __align__(128) unsigned char smem_raw[];
+    const AttnParams& p = bp.a;
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, g = lane >> 2;
+    const int it = blockIdx.x * (blockDim.x >> 5) + warp, ls = blockIdx.y;
+    if (it >= bp.nitems[ls]) return;
+    const BwdItem item = bp.items[(int64_t)ls * bp.cap + it];
+    Ring ring;
+    ring.init(smem_raw + (size_t)warp * Ring::kBytes, lane);
+    const uint2* entries = bp.entries + (int64_t)ls * bp.subq * bp.MV + item.start;
+    const unsigned char* qsrc = KEYS ? bp.qb : bp.dob;
+    const unsigned char* ssrc = KEYS ? bp.sts : bp.stp;
+    const unsigned char* tab = reinterpret_cast<const unsigned char*>(p.tab);
+    constexpr int VPS = NH == 2 ? 1 : 2;                                    // visits per step
+    const int len = item.len, steps = (len + VPS - 1) / VPS;
+
+    float acc[KS][NT][4];
+#pragma unroll
+    for (int i = 0; i < KS; ++i)
+#pragma unroll
+        for (int n = 0; n < NT; ++n) acc[i][n][0] = acc[i][n][1] = acc[i][n][2] = acc[i][n][3] = 0.f;
+
+    uint2 cur = entries[min(lane, len - 1)], nxt = entries[min(32 + lane, len - 1)];
+    auto issue = [&](int s) {
+        const int e0 = s * VPS;
+        if (e0 && (e0 & 31) == 0) { cur = nxt; nxt = entries[min(e0 + 32 + lane, len - 1)]; }
+        const int e1 = min(e0 + VPS - 1, len - 1);
+        uint2 a, b;
+        a.x = __shfl_sync(0xffffffffu, cur.x, e0 & 31); a.y = __shfl_sync(0xffffffffu, cur.y, e0 & 31);
+        b.x = a.x; b.y = a.y;
+        if (VPS == 2) { b.x = __shfl_sync(0xffffffffu, cur.x, e1 & 31); b.y = __shfl_sync(0xffffffffu, cur.y, e1 & 31); }
+        if (lane == 0) ring.expect(NH == 2 ? 2 * QB + 2 * SB + TAB : SLOT);
+        __syncwarp();
+        // lanes 0..5 issue one copy each: operand, record and table row of the two halves
+        const uint2 mine = (VPS == 2 && (lane & 1)) ? b : a;
+        const unsigned char* src; uint32_t off, bytes;
+        if (lane < 2) { src = qsrc + (int64_t)(mine.y & 0x7fffu) * (NH * QB); off = lane * QB; bytes = NH * QB; }
+        else if (lane < 4) { src = ssrc + (int64_t)mine.x * (NH * SB); off = 2 * QB + (lane & 1) * SB; bytes = NH * SB; }
+        else { src = tab + (int64_t)(mine.y >> 15) * C::TAB; off = 2 * QB + 2 * SB + (lane & 1) * TAB; bytes = TAB; }
+        if (lane < (KEYS ? 6 : 4) && (VPS == 2 || !(lane & 1))) ring.copy(off, src, bytes);
+        ring.issued();
+    };
+    int next = 0;
+#pragma unroll 1
+    for (; next < NSTG - 1 && next < steps; ++next) issue(next);
+#pragma unroll 1
+    for (int s = 0; s < steps; ++s) {
+        __syncwarp();
+        if (next < steps) { issue(next); ++next; }
+        uint32_t slot;
+        if (!ring.wait(slot)) { if (lane == 0 && p.status) atomicOr(p.status, 16); ring.drain(); return; }
+        const bool lone = VPS == 2 && 2 * s + 1 >= len;
+        const uint32_t ra = slot + 2 * QB, rb = ra + SB;
+        uint32_t bw[NT][2], bl[X3 ? NT : 1][2];
+        auto lds32 = [](uint32_t a) { uint32_t x; asm volatile("ld.shared.b32 %0, [%1];" : "=r"(x) : "r"(a)); return x; };
+        auto lds64 = [](uint32_t a, uint32_t& x, uint32_t& y) { asm volatile("ld.shared.v2.b32 {%0,%1}, [%2];" : "=r"(x), "=r"(y) : "r"(a)); };
+#pragma unroll
+        for (int pl = 0; pl < (X3 ? 2 : 1); ++pl) {
+#pragma unroll
+            for (int n = 0; n < NT; ++n) {
+                const uint32_t o = pl * PLANE + lane * (4 * NT) + 4 * n;
+                const uint32_t x = lds32(ra + o), y = lone ? 0u : lds32(rb + o);
+                if (pl == 0) { bw[n][0] = x; bw[n][1] = y; } else { bl[X3 ? n : 0][0] = x; bl[X3 ? n : 0][1] = y; }
+            }
+        }
+        if constexpr (KEYS && !X3) {
+            const uint32_t sel = (g & 1) ? 0x3232u : 0x1010u;
+            const uint32_t ta = slot + 2 * QB + 2 * SB + 2 * PPT * (g >> 1), tb = VPS == 2 ? ta + TAB : ta;
+#pragma unroll
+            for (int k4 = 0; k4 < KS; k4 += 4) {
+                const uint4 ca4 = lds_u4(ta + 4 * k4), sa4 = lds_u4(ta + 2 * HALF + 4 * k4);
+                const uint4 cb4 = VPS == 2 ? lds_u4(tb + 4 * k4) : ca4, sb4 = VPS == 2 ? lds_u4(tb + 2 * HALF + 4 * k4) : sa4;
+                const uint32_t ca[4] = {ca4.x, ca4.y, ca4.z, ca4.w}, sa[4] = {sa4.x, sa4.y, sa4.z, sa4.w};
+                const uint32_t cb[4] = {cb4.x, cb4.y, cb4.z, cb4.w}, sb[4] = {sb4.x, sb4.y, sb4.z, sb4.w};
+#pragma unroll
+                for (int u = 0; u < 4; ++u) {
+                    const int i = k4 + u;
+                    uint32_t la, ha, lb, hb, a[4];
+                    lds64(slot + i * 256 + lane * 8, la, ha);
+                    lds64(slot + QB + i * 256 + lane * 8, lb, hb);
+                    const uint32_t c0 = __byte_perm(ca[u], ca[u], sel), s0 = __byte_perm(sa[u], sa[u], sel);
+                    const uint32_t n0 = neg_h2(s0);
+                    rotate_h2(la, ha, c0, s0, n0, a[0], a[1]);
+                    if constexpr (VPS == 2) {
+                        const uint32_t c1 = __byte_perm(cb[u], cb[u], sel), s1 = __byte_perm(sb[u], sb[u], sel);
+                        rotate_h2(lb, hb, c1, s1, neg_h2(s1), a[2], a[3]);
+                    } else {
+                        rotate_h2(lb, hb, c0, s0, n0, a[2], a[3]);
+                    }
+#pragma unroll
+                    for (int n = 0; n < NT; ++n) F::mma(acc[i][n], a[0], a[1], a[2], a[3], bw[n][0], bw[n][1]);
+                }
+            }
+        } else if constexpr (!X3) {
+#pragma unroll
+            for (int i = 0; i < KS; ++i) {
+                uint32_t a[4];
+                lds64(slot + i * 256 + lane * 8, a[0], a[1]);
+                lds64(slot + QB + i * 256 + lane * 8, a[2], a[3]);
+#pragma unroll
+                for (int n = 0; n < NT; ++n) F::mma(acc[i][n], a[0], a[1], a[2], a[3], bw[n][0], bw[n][1]);
+            }
+        } else {
+#pragma unroll
+            for (int i = 0; i < KS; ++i) {
+                uint32_t ah[4], al[4];
+                if constexpr (KEYS) {
+#pragma unroll
+                    for (int v = 0; v < 2; ++v) {
+                        const uint4 x = lds_u4(slot + v * QB + i * 512 + lane * 16);
+                        const uint32_t t4 = slot + 2 * QB + 2 * SB + (VPS == 2 ? v : 0) * TAB + 4 * (PPT * (g >> 1) + 2 * i + (g & 1));
+                        const float cs = __uint_as_float(lds32(t4)), sn = __uint_as_float(lds32(t4 + 4 * HALF));
+                        float2 u, w;
+                        rotate_pairs_f32(make_float2(__uint_as_float(x.x), __uint_as_float(x.y)), make_float2(__uint_as_float(x.z), __uint_as_float(x.w)),
+                                         make_float2(cs, cs), make_float2(sn, sn), make_float2(-sn, -sn), u, w);
+                        split_half2(u.x, u.y, ah[2 * v], al[2 * v]);
+                        split_half2(w.x, w.y, ah[2 * v + 1], al[2 * v + 1]);
+                    }
+                } else {
+#pragma unroll
+                    for (int v = 0; v < 2; ++v) {
+                        lds64(slot + v * QB + i * 256 + lane * 8, ah[2 * v], ah[2 * v + 1]);
+                        lds64(slot + v * QB + D * 16 + i * 256 + lane * 8, al[2 * v], al[2 * v + 1]);
+                    }
+                }
+#pragma unroll
+                for (int n = 0; n < NT; ++n) {
+                    float t[4];
+                    mma_zero<__half>(t, al, bw[n][0], bw[n][1]);
+                    F::mma(t, ah[0], ah[1], ah[2], ah[3], bl[X3 ? n : 0][0], bl[X3 ? n : 0][1]);
+                    F::mma(t, ah[0], ah[1], ah[2], ah[3], bw[n][0], bw[n][1]);
+#pragma unroll
+                    for (int u = 0; u < 4; ++u) acc[i][n][u] += t[u];
+                }
+            }
+        }
+    }
+
+    int l = 0;
+    while (l + 1 < p.L && (bp.voff[l] < 0 || item.key < bp.koff[l] || item.key >= bp.koff[l] + (p.ln[l] + CR - 1) / CR)) ++l;
+    const int unit = (bp.sub0 + ls) / bp.nw, b = unit / p.Hkv, hk = unit % p.Hkv;
+    const int nblk = (p.ln[l] + CR - 1) / CR;
+    float* dst = (KEYS ? bp.acck[l] : bp.accv[l]) + (((int64_t)b * nblk + (item.key - bp.koff[l])) * p.Hkv + hk) * BF::ACC + 4 * lane;
+#pragma unroll
+    for (int i = 0; i < KS; ++i)
+#pragma unroll
+        for (int n = 0; n < NT; ++n) red_add_v4(dst + (i * NT + n) * 128, acc[i][n][0], acc[i][n][1], acc[i][n][2], acc[i][n][3]);
+}
+
+// Level by level from the top: accumulators to rows (dK' rotated back by the child index), plus the share of the pooled
+// parent's gradient (src/backward.py:787-841).  blockIdx.y: 0 = dK, 1 = dV; one warp per parent block.
+struct FoldArgs {
+    const float* acc[2];
+    const float* up[2];      // the level above, rows in fp32, or NULL at the top
+    void* out[2];            // this level's rows: fp32, or the storage type (typed)
+    const float* cosc;
+    const float* sinc;
+    int64_t total;           // blocks
+    int32_t N, Nup, NBLK, Hkv, typed;
+};
+template <typename TO, int D, int CR>
+__global__ void __launch_bounds__(128) bwd_fold_kernel(const __grid_constant__ FoldArgs f) {
+    constexpr int KS = D / 16, NT = CR / 8, HALF = D / 2, PPT = HALF / 4;
+    __shared__ float sm[4][CR][D + 4];
+    const int which = blockIdx.y, warp = threadIdx.x >> 5, lane = threadIdx.x & 31, g = lane >> 2, r = lane & 3;
+    const int64_t blk = (int64_t)blockIdx.x * 4 + warp;
+    if (blk >= f.total) return;
+    const int h = (int)(blk % f.Hkv), pb = (int)((blk / f.Hkv) % f.NBLK);
+    const int64_t b = blk / ((int64_t)f.Hkv * f.NBLK);
+    const float4* a = reinterpret_cast<const float4*>(f.acc[which]) + blk * (D * CR / 4);
+#pragma unroll
+    for (int i = 0; i < KS; ++i) {
+        const int x = PPT * (g >> 1) + 2 * i + (g & 1);
+#pragma unroll
+        for (int n = 0; n < NT; ++n) {
+            const float4 v = __ldcs(a + (i * NT + n) * 32 + lane);
+            const int c = 8 * n + 2 * r;
+            float lo[2] = {v.x, v.y}, hi[2] = {v.z, v.w};
+#pragma unroll
+            for (int e = 0; e < 2; ++e) {
+                float u = lo[e], w = hi[e];
+                if (which == 0) {
+                    const float cs = __ldg(f.cosc + (c + e) * HALF + x), sn = __ldg(f.sinc + (c + e) * HALF + x);
+                    u = lo[e] * cs + hi[e] * sn;
+                    w = hi[e] * cs - lo[e] * sn;
+                }
+                sm[warp][c + e][x] = u;
+                sm[warp][c + e][x + HALF] = w;
+            }
+        }
+    }
+    __syncwarp();
+    const int cnt = min(CR, f.N - pb * CR);
+    const float4* up = f.up[which] ? reinterpret_cast<const float4*>(f.up[which] + ((b * f.Nup + pb) * f.Hkv + h) * (int64_t)D) : nullptr;
+    constexpr int V4 = D / 4;
+    for (int i = lane; i < cnt * V4; i += 32) {
+        const int c = i / V4, col = i % V4;
+        float4 x = *reinterpret_cast<const float4*>(&sm[warp][c][4 * col]);
+        if (up) {
+            const float4 u = __ldg(up + col);
+            const float n = (float)cnt;
+            x.x += u.x / n; x.y += u.y / n; x.z += u.z / n; x.w += u.w / n;
+        }
+        const int64_t row = ((b * f.N + pb * CR + c) * f.Hkv + h) * (int64_t)D + 4 * col;
+        if (!f.typed || sizeof(TO) == 4) {
+            *reinterpret_cast<float4*>(reinterpret_cast<float*>(f.out[which]) + row) = x;
+        } else {
+            TO o[4] = {from_f<TO>(x.x), from_f<TO>(x.y), from_f<TO>(x.z), from_f<TO>(x.w)};
+            *reinterpret_cast<uint2*>(reinterpret_cast<TO*>(f.out[which]) + row) = *reinterpret_cast<const uint2*>(o);
+        }
+    }
+}
+
+template <typename T, int D, bool X3, int NH, int CR, bool KEYS>
+static int launch_dkv_one(const BwdParams& bp, cudaStream_t st) {
+    using BF = BForm<D, X3, NH, CR>;
+    constexpr int SLOT = 2 * BF::QB + 2 * BF::SB + (KEYS ? 2 * TForm<D, X3, CR>::TAB : 0);
+    using Ring = ChunkRing<dkv_stages<D, X3>(), SLOT>;
+    const size_t smem = 4 * Ring::kBytes;
+    auto* k = bwd_dkv_kernel<T, D, X3, NH, CR, KEYS>;
+    const cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    if (e != cudaSuccess) return (int)e;
+    k<<<dim3((bp.cap + 3) / 4, bp.nsub), 128, smem, st>>>(bp);
+    note_launch();
+    return (int)cudaGetLastError();
+}
+template <typename T, int D, bool X3, int NH, int CR>
+static int launch_dkv_cr(const BwdParams& bp, cudaStream_t st) {
+    const int rc = launch_dkv_one<T, D, X3, NH, CR, true>(bp, st);
+    return rc ? rc : launch_dkv_one<T, D, X3, NH, CR, false>(bp, st);
+}
+template <typename T, int D, bool X3>
+static int launch_dkv_t(const BwdParams& bp, cudaStream_t st) {
+    if (bp.a.CR == 16) return bp.a.G <= 8 ? launch_dkv_cr<T, D, X3, 1, 16>(bp, st) : launch_dkv_cr<T, D, X3, 2, 16>(bp, st);
+    return bp.a.G <= 8 ? launch_dkv_cr<T, D, X3, 1, 8>(bp, st) : launch_dkv_cr<T, D, X3, 2, 8>(bp, st);
+}
+template <typename T>
+static int launch_dkv_d(const BwdParams& bp, cudaStream_t st) {
+    constexpr bool F32 = std::is_same<T, float>::value;
+    return bp.a.K == 128 ? launch_dkv_t<T, 128, F32>(bp, st) : bp.a.K == 64 ? launch_dkv_t<T, 64, F32>(bp, st) : launch_dkv_t<T, 32, true>(bp, st);
+}
+
+int launch_bwd_dkv(const BwdParams& bp, int dtype, cudaStream_t st) {
+    bwd_scan_kernel<<<bp.nsub, 1024, 0, st>>>(bp);
+    note_launch();
+    bwd_fill_kernel<<<dim3((bp.subq + 7) / 8, bp.nsub), 256, 0, st>>>(bp);
+    note_launch();
+    const cudaError_t e = cudaGetLastError();
+    if (e != cudaSuccess) return (int)e;
+    switch (dtype) {
+        case HTREE_F32: return launch_dkv_d<float>(bp, st);
+        case HTREE_BF16: return launch_dkv_d<__nv_bfloat16>(bp, st);
+        default: return launch_dkv_d<__half>(bp, st);
+    }
+}
+
+template <typename TO>
+static void launch_fold_t(const FoldArgs& f, int D, int CR, cudaStream_t st) {
+    const dim3 grid((unsigned)((f.total + 3) / 4), 2);
+    if (CR == 16) {
+        if (D == 128) bwd_fold_kernel<TO, 128, 16><<<grid, 128, 0, st>>>(f);
+        else if (D == 64) bwd_fold_kernel<TO, 64, 16><<<grid, 128, 0, st>>>(f);
+        else bwd_fold_kernel<TO, 32, 16><<<grid, 128, 0, st>>>(f);
+    } else {
+        if (D == 128) bwd_fold_kernel<TO, 128, 8><<<grid, 128, 0, st>>>(f);
+        else if (D == 64) bwd_fold_kernel<TO, 64, 8><<<grid, 128, 0, st>>>(f);
+        else bwd_fold_kernel<TO, 32, 8><<<grid, 128, 0, st>>>(f);
+    }
+}
+
+// gk[l], gv[l]: rows of level l in fp32 (l >= 1: scratch); level 0 goes to dk, dv in fp32 or, typed, the storage type.
+int launch_bwd_fold(const BwdParams& bp, int dtype, float* const* gk, float* const* gv, void* dk, void* dv, bool typed, cudaStream_t st) {
+    const AttnParams& p = bp.a;
+    for (int l = p.L - 1; l >= 0; --l) {
+        FoldArgs f;
+        f.acc[0] = bp.acck[l]; f.acc[1] = bp.accv[l];
+        f.up[0] = l + 1 < p.L ? gk[l + 1] : nullptr; f.up[1] = l + 1 < p.L ? gv[l + 1] : nullptr;
+        f.out[0] = l ? (void*)gk[l] : dk; f.out[1] = l ? (void*)gv[l] : dv;
+        f.cosc = p.cosc; f.sinc = p.sinc;
+        f.N = p.ln[l]; f.Nup = l + 1 < p.L ? p.ln[l + 1] : 0; f.NBLK = (p.ln[l] + p.CR - 1) / p.CR; f.Hkv = p.Hkv;
+        f.total = (int64_t)p.B * f.NBLK * p.Hkv;
+        f.typed = l == 0 && typed;
+        if (dtype == HTREE_BF16) launch_fold_t<__nv_bfloat16>(f, p.K, p.CR, st);
+        else if (dtype == HTREE_F16) launch_fold_t<__half>(f, p.K, p.CR, st);
+        else launch_fold_t<float>(f, p.K, p.CR, st);
+        note_launch();
+        const cudaError_t e = cudaGetLastError();
+        if (e != cudaSuccess) return (int)e;
+    }
+    return 0;
+}
+
+}  // namespace htree

@@ -1,0 +1,432 @@
+// Query-stationary pass of the backward: dq, and P and dS of every visit for the parent-stationary pass (bwd_tform.cuh).
+// One warp per (batch, query position, KV head) group, all levels in one launch.  Replaces
+// htree_bwd_preprocess_delta_kernel, htree_bwd_build_parent_mask_kernel and htree_bwd_dq_bottom/upper_kernel
+// (src/backward.py:45-436); arithmetic of src/naive.py:333-384 with the forward's scores, bit for bit.  Per chunk:
+//   dP^T = V dO^T,  S^T = K' q^,  P = exp(S - gmax) / gsum,  dS = P (dP - D),  dq^T += K~^T dS^T
+// with K~ = scale R(-distance) K' rotated back into the query's frame in registers, its fragments transposed by the load.
+#include "bwd_tform.cuh"
+
+namespace htree {
+
+template <int D, bool X3>
+constexpr int dq_stages() { return D == 128 ? 2 : 3; }
+// Warps per block and blocks per SM: registers first.  The ring takes nearly all of the SM's L1, so anything that spills is
+// re-read from L2 in every chunk: with 180 bytes of spills, groups of 16 heads of 128 spent 4.6 of 9.4 cycles per instruction
+// waiting for it.  Those run as blocks of one warp (24 to 32 bytes of spills at 12 warps per SM; the compiler keeps 150 in larger
+// blocks): 64K positions, 4 KV heads 53 -> 31.6 ms, against 33.3 ms for 8 warps per SM with nothing spilled.
+template <int D, bool X3, int NH>
+constexpr int dq_warps() { return D == 128 && !X3 && NH == 2 ? 1 : 4; }
+template <int D, bool X3, int NH>
+constexpr int dq_min_blocks() { return (D == 128 && (X3 || NH == 2)) ? (X3 ? 2 : 12) : (X3 && NH == 2) ? 2 : 3; }
+
+// ring, parent list, kept-candidate bits, two pointers
+template <typename Ring>
+__host__ __device__ inline size_t dq_warp_bytes(int TK, int CR) {
+    return (Ring::kBytes + sizeof(int32_t) * TK + sizeof(uint32_t) * ((TK * CR + 31) / 32) + 16 + 127) & ~size_t(127);
+}
+
+template <typename T, int D, bool X3, int NH, int CR>
+__global__ void __launch_bounds__(dq_warps<D, X3, NH>() * 32, dq_min_blocks<D, X3, NH>()) bwd_dq_kernel(const __grid_constant__ BwdParams bp) {
+    using C = TForm<D, X3, CR>;
+    using BF = BForm<D, X3, NH, CR>;
+    using F = Frag<typename std::conditional<X3, __half, T>::type>;
+    using FT = typename std::conditional<X3, __half, T>::type;
+    using FS = Frag<__half>;
+    constexpr int KS = C::KS, PPT = C::PPT, PPC = C::PPC, HALF = C::HALF;
+    constexpr int NSTG = dq_stages<D, X3>();
+    using Ring = ChunkRing<NSTG, C::SLOT>;
+    extern __shared__ __align__(128) unsigned char smem_raw[];
+    const AttnParams& p = bp.a;
+
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, g = lane >> 2, r = lane & 3;
+    const int W = blockDim.x >> 5;
+    const int qi = blockIdx.x * W + warp;
+    const int sub = bp.sub0 + blockIdx.y, unit = sub / bp.nw;
+    const int tl = (sub % bp.nw) * bp.subq + qi;
+    if (qi >= bp.subq || tl >= p.Tq) return;
+    const int t = p.t0 + tl;
+    const int b = unit / p.Hkv, hk = unit % p.Hkv;
+    const int G = p.G, TK = p.TK, L = p.L;
+    const int grp = blockIdx.y * bp.subq + qi;
+
+    const size_t per_warp = dq_warp_bytes<Ring>(TK, CR);
+    unsigned char* wbase = smem_raw + warp * per_warp;
+    Ring ring;
+    ring.init(wbase, lane);
+    int32_t* par = reinterpret_cast<int32_t*>(wbase + Ring::kBytes);
+    uint32_t* selw = reinterpret_cast<uint32_t*>(par + TK);
+    // what only the issuing lane needs, once per chunk, lives in shared memory: this level's key and value blocks
+    const unsigned char* volatile* src = reinterpret_cast<const unsigned char* volatile*>(wbase + per_warp - 16);
+
+    const int64_t hbase = ((int64_t)b * p.Tq + tl) * p.H + (int64_t)hk * G;
+    const int64_t qidx = ((int64_t)b * p.Tq + tl) * p.Hkv + hk;
+
+    QueryRegs<T, D, X3, NH> q;
+    load_query<T, D, X3, NH>(reinterpret_cast<const T*>(p.q) + hbase * D, G, g, r, p.scale, q);
+    uint32_t dO[NH][2][KS], dOl[X3 ? NH : 1][2][X3 ? KS : 1];
+    float Drow[NH][2], lse[NH][2], ginv[NH][2];
+#pragma unroll
+    for (int h = 0; h < NH; ++h) {
+        const int head = 8 * h + g;
+        const bool on = head < G;
+        float sum = 0.f;
+#pragma unroll
+        for (int hf = 0; hf < 2; ++hf) {
+            const int64_t off = (hbase + head) * D + hf * HALF + PPT * r;
+            if constexpr (X3) {
+                float x[D / 8], o[D / 8];
+                load_row_piece_f32<T, D>(reinterpret_cast<const T*>(p.dO) + off, on, x);
+                load_row_piece_f32<T, D>(reinterpret_cast<const T*>(p.out) + off, on, o);
+#pragma unroll
+                for (int i = 0; i < D / 16; ++i) {
+                    sum += x[2 * i] * o[2 * i] + x[2 * i + 1] * o[2 * i + 1];
+                    split_half2(x[2 * i], x[2 * i + 1], dO[h][hf][i], dOl[X3 ? h : 0][hf][X3 ? i : 0]);
+                }
+            } else {
+                uint32_t o[KS];
+                ldg_vec<PPT / 8>(reinterpret_cast<const T*>(p.dO) + off, on, dO[h][hf]);
+                ldg_vec<PPT / 8>(reinterpret_cast<const T*>(p.out) + off, on, o);
+#pragma unroll
+                for (int i = 0; i < KS; ++i) {
+                    const float2 x = F::unpack(dO[h][hf][i]), y = F::unpack(o[i]);
+                    sum += x.x * y.x + x.y * y.y;
+                }
+            }
+        }
+        sum += __shfl_xor_sync(0xffffffffu, sum, 1);
+        sum += __shfl_xor_sync(0xffffffffu, sum, 2);
+#pragma unroll
+        for (int e = 0; e < 2; ++e) {
+            const int hd = 8 * h + 2 * r + e;
+            Drow[h][e] = __shfl_sync(0xffffffffu, sum, 4 * (2 * r + e));
+            const float gm = hd < G ? p.gmax[hbase + hd] : 0.f, gs = hd < G ? p.gsum[hbase + hd] : 1.f;
+            // 16-bit: P = 2^(S log2 e - lse); split-half: exp(S - gmax) * ginv (an exponent re-based by log2 e rounds at 1e-6)
+            lse[h][e] = X3 ? gm : (hd < G ? gm * kLog2e + __log2f(gs) : INFINITY);
+            ginv[h][e] = hd < G ? 1.f / gs : 0.f;
+        }
+    }
+
+    // ---- blocked copies of q and dO for the parent-stationary pass: pairs of heads per word, [half][i][lane]{lo, hi} with
+    //      dims x(i, g) = PPT*(g/2) + 2i + (g & 1) (and + D/2) and heads 2r, 2r + 1 ----
+#pragma unroll
+    for (int h = 0; h < NH; ++h) {
+        unsigned char* dst = bp.dob + ((int64_t)grp * NH + h) * BF::QB;
+#pragma unroll
+        for (int i = 0; i < KS; ++i) {
+            *reinterpret_cast<uint2*>(dst + i * 256 + lane * 8) = make_uint2(movmatrix_trans(dO[h][0][i]), movmatrix_trans(dO[h][1][i]));
+            if constexpr (X3)
+                *reinterpret_cast<uint2*>(dst + D * 16 + i * 256 + lane * 8) =
+                    make_uint2(movmatrix_trans(dOl[X3 ? h : 0][0][X3 ? i : 0]), movmatrix_trans(dOl[X3 ? h : 0][1][X3 ? i : 0]));
+        }
+        unsigned char* qd = bp.qb + ((int64_t)grp * NH + h) * BF::QB;
+        if constexpr (X3) {
+            // fp32: 16 bytes per lane and tile {lo(2r), lo(2r+1), hi(2r), hi(2r+1)}; this lane has head g, dims PPT*r + j
+#pragma unroll
+            for (int hf = 0; hf < 2; ++hf)
+#pragma unroll
+                for (int j = 0; j < PPT; ++j)
+                    reinterpret_cast<uint32_t*>(qd)[((j >> 1) * 32 + 4 * (2 * r + (j & 1)) + (g >> 1)) * 4 + 2 * hf + (g & 1)] = q.v[h][hf][j];
+        } else {
+#pragma unroll
+            for (int i = 0; i < KS; ++i)
+                *reinterpret_cast<uint2*>(qd + i * 256 + lane * 8) = make_uint2(movmatrix_trans(q.v[h][0][i]), movmatrix_trans(q.v[h][1][i]));
+        }
+    }
+
+    float dq[NH][KS][4];      // dq^T: dims x(ks, g) (elements 0, 1) and + D/2 (2, 3), heads 2r, 2r + 1
+#pragma unroll
+    for (int h = 0; h < NH; ++h)
+#pragma unroll
+        for (int i = 0; i < KS; ++i) dq[h][i][0] = dq[h][i][1] = dq[h][i][2] = dq[h][i][3] = 0.f;
+
+    for (int l = L - 1; l >= 0; --l) {
+        if (bp.voff[l] < 0) continue;
+        const int Nl = p.ln[l];
+        const int nblk = (Nl + CR - 1) / CR;
+        __syncwarp();
+        int np = 0;
+        for (int i = lane; i < TK; i += 32) { const int x = load_parent(p, l, qidx * TK + i); par[i] = x; np += x >= 0; }
+        np = __reduce_add_sync(0xffffffffu, np);
+        const int rc = (int)(((int64_t)t / p.lpow[l]) % CR);
+        const int nc = (np - 1) * CR + rc + 1, rp = nc - 1;
+        if (np <= 0 || (l > 0 && nc <= TK)) continue;
+        const int nchunk = (np + PPC - 1) / PPC;
+        __syncwarp();
+        // this visit's place in its parent's list
+        int32_t* cnt = bp.cnt + (int64_t)blockIdx.y * bp.NK + bp.koff[l];
+        for (int i = lane; i < np; i += 32) {
+            const int x = (unsigned)par[i] < (unsigned)nblk ? par[i] : 0;
+            bp.rank[(int64_t)grp * bp.MV + bp.voff[l] + i] = atomicAdd(cnt + x, 1);
+        }
+        if (l > 0) {
+            for (int i = lane; i < (nc + 31) / 32; i += 32) selw[i] = 0u;
+            __syncwarp();
+            for (int i = lane; i < TK; i += 32) {
+                const int node = load_parent(p, l - 1, qidx * TK + i);
+                if (node < 0) continue;
+                const int parent = node / CR;
+                int lo = 0, hi = np;
+                while (lo < hi) { const int mid = (lo + hi) >> 1; if (par[mid] < parent) lo = mid + 1; else hi = mid; }
+                if (lo < np && par[lo] == parent) {
+                    const int j = lo * CR + node % CR;
+                    atomicOr(&selw[j >> 5], 1u << (j & 31));
+                }
+            }
+        }
+        if (lane == 0) {
+            const int64_t blk0 = (int64_t)b * nblk * p.Hkv + hk;
+            src[0] = reinterpret_cast<const unsigned char*>(p.blk[l]) + blk0 * C::BLOCK;
+            src[1] = reinterpret_cast<const unsigned char*>(p.vkblk[l]) + blk0 * (C::PL * C::PART);
+        }
+        __syncwarp();
+
+        auto issue = [&](int c) {
+            if (lane == 0) {
+                constexpr int PB = C::PL * C::PART;
+                ring.expect(C::SLOT);
+                int p0 = par[c * PPC];
+                if ((unsigned)p0 >= (unsigned)nblk) { if (p.status) atomicOr(p.status, 8); p0 = 0; }
+                const int64_t kstride = (int64_t)p.Hkv * C::BLOCK, vstride = (int64_t)p.Hkv * (C::PL * C::PART);
+                const unsigned char *kblk = src[0], *vblk = src[1];
+                ring.copy(0, kblk + p0 * kstride, PB);
+                ring.copy(C::V_OFF, vblk + p0 * vstride, PB);
+                if constexpr (CR == 8) {
+                    int p1 = c * PPC + 1 < np ? par[c * PPC + 1] : p0;
+                    if ((unsigned)p1 >= (unsigned)nblk) { if (p.status) atomicOr(p.status, 8); p1 = 0; }
+                    ring.copy(C::K2_OFF, kblk + p1 * kstride + 2 * C::ODD, PB);
+                    ring.copy(C::V2_OFF, vblk + p1 * vstride, PB);
+                }
+                const unsigned char* tab = reinterpret_cast<const unsigned char*>(p.tab) + (int64_t)(rp - 16 * c) * C::TAB;
+                ring.copy(C::DATA, tab, C::TAB);
+                if constexpr (C::DUAL) ring.copy(C::DATA + C::TAB, rp - 16 * c >= 8 ? tab - 8 * C::TAB : tab, C::TAB);
+            }
+            ring.issued();
+        };
+        int next = 0;
+#pragma unroll 1
+        for (; next < NSTG - 1 && next < nchunk; ++next) issue(next);
+        const int visit0 = grp * bp.MV + bp.voff[l];
+#pragma unroll 1
+        for (int c = 0; c < nchunk; ++c) {
+            __syncwarp();
+            if (next < nchunk) { issue(next); ++next; }
+            uint32_t mask = 0xffffu;
+            if (l > 0) mask &= ~(selw[c >> 1] >> ((16 * c) & 31));
+            if (16 * c + 15 > rp) mask &= (2u << (rp - 16 * c)) - 1u;
+            uint32_t slot;
+            if (!ring.wait(slot)) { if (lane == 0 && p.status) atomicOr(p.status, 16); ring.drain(); return; }
+            const LaneBase<D, X3, CR> lb(slot, lane);
+            const uint32_t tabs = slot + C::DATA;
+
+            uint32_t pw[NH][2], sw[NH][2], pwl[X3 ? NH : 1][2], swl[X3 ? NH : 1][2];   // P^T, dS^T: word w = child g + 8w, heads 2r, 2r+1
+            if (mask == 0) {
+#pragma unroll
+                for (int h = 0; h < NH; ++h)
+#pragma unroll
+                    for (int w = 0; w < 2; ++w) {
+                        pw[h][w] = sw[h][w] = 0u;
+                        if constexpr (X3) pwl[X3 ? h : 0][w] = swl[X3 ? h : 0][w] = 0u;
+                    }
+            } else {
+                float dP[NH][4];
+#pragma unroll
+                for (int ks = 0; ks < KS; ++ks) {
+                    uint32_t a[4], al[4];
+                    vk_frag<D, X3, CR>(lb, 0, ks, a);
+                    if constexpr (X3) vk_frag<D, X3, CR>(lb, 1, ks, al);
+#pragma unroll
+                    for (int h = 0; h < NH; ++h) {
+                        if (ks == 0) mma_zero<FT>(dP[h], a, dO[h][0][0], dO[h][1][0]);
+                        else F::mma(dP[h], a[0], a[1], a[2], a[3], dO[h][0][ks], dO[h][1][ks]);
+                        if constexpr (X3) {
+                            F::mma(dP[h], al[0], al[1], al[2], al[3], dO[h][0][ks], dO[h][1][ks]);
+                            F::mma(dP[h], a[0], a[1], a[2], a[3], dOl[X3 ? h : 0][0][X3 ? ks : 0], dOl[X3 ? h : 0][1][X3 ? ks : 0]);
+                        }
+                    }
+                }
+                float S[NH][4];
+                score_t<T, D, X3, NH, CR>(lb, tabs, r, q, S);
+                const bool c0 = (mask >> g) & 1, c1 = (mask >> (g + 8)) & 1;
+                uint32_t db[NH][2], dbl[X3 ? NH : 1][2];       // dS^T as B fragments (children x heads)
+#pragma unroll
+                for (int h = 0; h < NH; ++h) {
+                    float P[4], dS[4];
+#pragma unroll
+                    for (int i = 0; i < 4; ++i) {
+                        P[i] = X3 ? __expf(S[h][i] - lse[h][i & 1]) * ginv[h][i & 1] : ex2_approx(fmaf(S[h][i], kLog2e, -lse[h][i & 1]));
+                        P[i] = (i < 2 ? c0 : c1) ? P[i] : 0.f;
+                        dS[i] = P[i] * (dP[h][i] - Drow[h][i & 1]);
+                    }
+                    if constexpr (X3) {
+                        split_half2(P[0], P[1], pw[h][0], pwl[X3 ? h : 0][0]); split_half2(P[2], P[3], pw[h][1], pwl[X3 ? h : 0][1]);
+                        split_half2(dS[0], dS[1], sw[h][0], swl[X3 ? h : 0][0]); split_half2(dS[2], dS[3], sw[h][1], swl[X3 ? h : 0][1]);
+                        dbl[X3 ? h : 0][0] = movmatrix_trans(swl[X3 ? h : 0][0]); dbl[X3 ? h : 0][1] = movmatrix_trans(swl[X3 ? h : 0][1]);
+                    } else {
+                        pw[h][0] = F::pack(P[0], P[1]); pw[h][1] = F::pack(P[2], P[3]);
+                        sw[h][0] = FS::pack(dS[0], dS[1]); sw[h][1] = FS::pack(dS[2], dS[3]);
+                    }
+                    db[h][0] = movmatrix_trans(sw[h][0]); db[h][1] = movmatrix_trans(sw[h][1]);
+                }
+                // dq^T += K~^T dS^T: transposed key fragments (rows x(ks, g)), rotated back by the chunk's distance
+                if constexpr (!X3) {
+                    const uint32_t sel = (g & 1) ? 0x3232u : 0x1010u;
+                    const uint32_t tb = tabs + 2 * PPT * (g >> 1);
+#pragma unroll
+                    for (int k4 = 0; k4 < KS; k4 += 4) {
+                        const uint4 c4 = lds_u4(tb + 4 * k4), s4 = lds_u4(tb + 2 * HALF + 4 * k4);
+                        const uint32_t cw[4] = {c4.x, c4.y, c4.z, c4.w}, snw[4] = {s4.x, s4.y, s4.z, s4.w};
+                        uint32_t cv[4], snv[4];                  // the odd parent's distance
+                        if constexpr (C::DUAL) {
+                            const uint4 d4 = lds_u4(tb + C::TAB + 4 * k4), t4 = lds_u4(tb + C::TAB + 2 * HALF + 4 * k4);
+                            cv[0] = d4.x; cv[1] = d4.y; cv[2] = d4.z; cv[3] = d4.w;
+                            snv[0] = t4.x; snv[1] = t4.y; snv[2] = t4.z; snv[3] = t4.w;
+                        }
+#pragma unroll
+                        for (int u = 0; u < 4; ++u) {
+                            const int ks = k4 + u;
+                            uint32_t m[4], a[4];
+                            key_frag_trans<D, X3, CR>(lb, 0, ks, m);
+                            const uint32_t cc = __byte_perm(cw[u], cw[u], sel), ss = __byte_perm(snw[u], snw[u], sel);
+                            const uint32_t ns = neg_h2(ss);                    // inverse rotation
+                            rotate_h2(m[0], m[2], cc, ns, ss, a[0], a[1]);
+                            if constexpr (C::DUAL) {
+                                const uint32_t c2 = __byte_perm(cv[u], cv[u], sel), s2 = __byte_perm(snv[u], snv[u], sel);
+                                rotate_h2(m[1], m[3], c2, neg_h2(s2), s2, a[2], a[3]);
+                            } else {
+                                rotate_h2(m[1], m[3], cc, ns, ss, a[2], a[3]);
+                            }
+#pragma unroll
+                            for (int h = 0; h < NH; ++h) FS::mma(dq[h][ks], a[0], a[1], a[2], a[3], db[h][0], db[h][1]);
+                        }
+                    }
+                } else {
+#pragma unroll
+                    for (int ks = 0; ks < KS; ++ks) {
+                        uint32_t mh[4], ml[4], ah[4], al[4];
+                        key_frag_trans<D, X3, CR>(lb, 0, ks, mh);
+                        key_frag_trans<D, X3, CR>(lb, 1, ks, ml);
+                        float cs, sn;
+                        const uint32_t tb = tabs + 4 * (PPT * (g >> 1) + 2 * ks + (g & 1));
+                        asm volatile("ld.shared.f32 %0, [%1];" : "=f"(cs) : "r"(tb));
+                        asm volatile("ld.shared.f32 %0, [%1];" : "=f"(sn) : "r"(tb + 4 * HALF));
+                        float2 x[4];
+#pragma unroll
+                        for (int m = 0; m < 4; ++m) {
+                            const float2 hi = FS::unpack(mh[m]), lo = FS::unpack(ml[m]);
+                            x[m] = make_float2(hi.x + lo.x, hi.y + lo.y);
+                        }
+                        const float2 c2 = make_float2(cs, cs), s2 = make_float2(sn, sn), n2 = make_float2(-sn, -sn);
+#pragma unroll
+                        for (int tile = 0; tile < 2; ++tile) {
+                            const float2 u = ffma2(x[2 + tile], s2, fmul2(x[tile], c2)), w = ffma2(x[tile], n2, fmul2(x[2 + tile], c2));
+                            split_half2(u.x, u.y, ah[2 * tile], al[2 * tile]);
+                            split_half2(w.x, w.y, ah[2 * tile + 1], al[2 * tile + 1]);
+                        }
+#pragma unroll
+                        for (int h = 0; h < NH; ++h) {
+                            // from zero, then a round-to-nearest fp32 add (the tensor core's accumulation truncates)
+                            float acc[4];
+                            mma_zero<__half>(acc, ah, dbl[X3 ? h : 0][0], dbl[X3 ? h : 0][1]);
+                            FS::mma(acc, al[0], al[1], al[2], al[3], db[h][0], db[h][1]);
+                            FS::mma(acc, ah[0], ah[1], ah[2], ah[3], db[h][0], db[h][1]);
+#pragma unroll
+                            for (int i = 0; i < 4; ++i) dq[h][ks][i] += acc[i];
+                        }
+                    }
+                }
+            }
+            // ---- leave P and dS behind, one record per visit ----
+#pragma unroll
+            for (int h = 0; h < NH; ++h) {
+                if constexpr (CR == 16) {
+                    const int64_t o = ((int64_t)(visit0 + c) * NH + h) * BF::SB + lane * 8;
+                    *reinterpret_cast<uint2*>(bp.stp + o) = make_uint2(pw[h][0], pw[h][1]);
+                    *reinterpret_cast<uint2*>(bp.sts + o) = make_uint2(sw[h][0], sw[h][1]);
+                    if constexpr (X3) {
+                        *reinterpret_cast<uint2*>(bp.stp + o + 256) = make_uint2(pwl[X3 ? h : 0][0], pwl[X3 ? h : 0][1]);
+                        *reinterpret_cast<uint2*>(bp.sts + o + 256) = make_uint2(swl[X3 ? h : 0][0], swl[X3 ? h : 0][1]);
+                    }
+                } else {
+#pragma unroll
+                    for (int w = 0; w < 2; ++w) {
+                        if (2 * c + w < np) {
+                            const int64_t o = ((int64_t)(visit0 + 2 * c + w) * NH + h) * BF::SB + lane * 4;
+                            *reinterpret_cast<uint32_t*>(bp.stp + o) = pw[h][w];
+                            *reinterpret_cast<uint32_t*>(bp.sts + o) = sw[h][w];
+                            if constexpr (X3) {
+                                *reinterpret_cast<uint32_t*>(bp.stp + o + 128) = pwl[X3 ? h : 0][w];
+                                *reinterpret_cast<uint32_t*>(bp.sts + o + 128) = swl[X3 ? h : 0][w];
+                            }
+                        }
+                    }
+                }
+            }
+        }
+    }
+
+    // ---- dq through shared memory (the ring is idle), rows written whole: fp32, or rounded once to the storage type ----
+    __syncwarp();
+    float* sm = reinterpret_cast<float*>(wbase);
+    const float post = X3 ? p.scale : 1.f;           // 16-bit: the scale is in the tables
+#pragma unroll
+    for (int h = 0; h < NH; ++h)
+#pragma unroll
+        for (int ks = 0; ks < KS; ++ks)
+#pragma unroll
+            for (int i = 0; i < 4; ++i)
+                sm[(8 * h + 2 * r + (i & 1)) * D + (i >> 1) * HALF + PPT * (g >> 1) + 2 * ks + (g & 1)] = dq[h][ks][i] * post;
+    __syncwarp();
+    for (int i = lane; i < G * D / 4; i += 32) {
+        const float4 x = reinterpret_cast<const float4*>(sm)[i];
+        if (p.dq_typed == nullptr) {
+            reinterpret_cast<float4*>(p.dq + hbase * D)[i] = x;
+        } else if constexpr (sizeof(T) == 4) {
+            reinterpret_cast<float4*>(reinterpret_cast<float*>(p.dq_typed) + hbase * D)[i] = x;
+        } else {
+            using FP = Frag<typename std::conditional<sizeof(T) == 4, __half, T>::type>;
+            reinterpret_cast<uint2*>(reinterpret_cast<T*>(p.dq_typed) + hbase * D)[i] = make_uint2(FP::pack(x.x, x.y), FP::pack(x.z, x.w));
+        }
+    }
+}
+
+template <typename T, int D, bool X3, int NH, int CR>
+static int launch_dq_cr(const BwdParams& bp, cudaStream_t st) {
+    using C = TForm<D, X3, CR>;
+    using Ring = ChunkRing<dq_stages<D, X3>(), C::SLOT>;
+    const int TK = bp.a.TK;
+    const size_t per_warp = dq_warp_bytes<Ring>(TK, CR);
+    constexpr int max_w = dq_warps<D, X3, NH>(), max_warps = max_w * dq_min_blocks<D, X3, NH>();
+    int W = 1, best = 0;
+    for (int w = max_w; w >= 1; w >>= 1) {
+        int blocks = (int)(228 * 1024 / (w * per_warp + 1024));
+        if (blocks * w > max_warps) blocks = max_warps / w;
+        if (blocks > 0 && blocks * w > best) { best = blocks * w; W = w; }
+    }
+    if (best == 0 || W * per_warp > 227 * 1024) return HTREE_E_UNSUPPORTED;
+    auto* k = bwd_dq_kernel<T, D, X3, NH, CR>;
+    const cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)(W * per_warp));
+    if (e != cudaSuccess) return (int)e;
+    k<<<dim3((bp.subq + W - 1) / W, bp.nsub), W * 32, W * per_warp, st>>>(bp);
+    note_launch();
+    return (int)cudaGetLastError();
+}
+
+template <typename T, int D, bool X3>
+static int launch_dq_t(const BwdParams& bp, cudaStream_t st) {
+    if (bp.a.CR == 16) return bp.a.G <= 8 ? launch_dq_cr<T, D, X3, 1, 16>(bp, st) : launch_dq_cr<T, D, X3, 2, 16>(bp, st);
+    return bp.a.G <= 8 ? launch_dq_cr<T, D, X3, 1, 8>(bp, st) : launch_dq_cr<T, D, X3, 2, 8>(bp, st);
+}
+template <typename T>
+static int launch_dq_d(const BwdParams& bp, cudaStream_t st) {
+    constexpr bool F32 = std::is_same<T, float>::value;
+    return bp.a.K == 128 ? launch_dq_t<T, 128, F32>(bp, st) : bp.a.K == 64 ? launch_dq_t<T, 64, F32>(bp, st) : launch_dq_t<T, 32, true>(bp, st);
+}
+int launch_bwd_dq(const BwdParams& bp, int dtype, cudaStream_t st) {
+    switch (dtype) {
+        case HTREE_F32: return launch_dq_d<float>(bp, st);
+        case HTREE_BF16: return launch_dq_d<__nv_bfloat16>(bp, st);
+        default: return launch_dq_d<__half>(bp, st);
+    }
+}
+
+}  // namespace htree

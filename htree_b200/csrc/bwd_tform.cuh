@@ -1,0 +1,51 @@
+// Parameters and layouts shared by the kernels of the two-pass backward (bwd_dq.cu, bwd_dkv.cu).
+//
+// The query-stationary pass (bwd_dq.cu) forms S, P, dP, dS of every accumulated chunk and sums dq in registers.  Pushing dK
+// and dV from there costs one fp32 reduction of CR rows per visit (a query's visit to a parent), 16 KB each at 128-wide heads,
+// and runs at the L2's reduction rate whatever the arithmetic does.  So it only leaves P and dS behind, in the storage
+// precision of the products that consume them (1 KB a visit for 16 heads), and the parent-stationary pass (bwd_dkv.cu) walks the
+// visits of one parent with dK, dV in registers: it fetches the queries (4 KB) and that kilobyte, and reduces once per 64 or so
+// visits.  The order of a parent's visits comes from a counting sort (ranks taken by the first pass, one scan, one fill).
+//
+// Work is cut into windows of `subq` queries of one (batch, KV head) unit, small enough for a window's blocked queries to stay
+// in L2 while its parents gather from them, and into launches of `nsub` windows, whose P and dS fit the caller's buffer.
+#pragma once
+#include "tform.cuh"
+
+namespace htree {
+
+struct BwdItem { int32_t key, start, len, pad; };     // a piece of one parent's visit list
+
+struct BwdParams {
+    AttnParams a;
+    int32_t sub0, nsub, subq, nw;            // windows of this launch: [sub0, sub0 + nsub) of units * nw
+    int32_t MV, NK, seg, cap;                // visit slots per query, parents per unit over all levels, longest item, items per window
+    int32_t voff[HTREE_MAX_LEVELS];          // first visit slot of a level, -1: the level accumulates nothing
+    int32_t koff[HTREE_MAX_LEVELS];          // first parent of a level among the NK
+    unsigned char* qb;                       // blocked queries [group][half]
+    unsigned char* dob;                      // blocked output gradients [group][half]
+    unsigned char* stp;                      // P  [group * MV + visit][half]
+    unsigned char* sts;                      // dS
+    int32_t* rank;                           // [group * MV + visit]
+    int32_t* cnt;                            // [nsub][NK]
+    int32_t* base;                           // [nsub][NK]
+    uint2* entries;                          // [nsub][subq * MV]
+    BwdItem* items;                          // [nsub][cap]
+    int32_t* nitems;                         // [nsub]
+    float* acck[HTREE_MAX_LEVELS];           // dK', dV of every level in accumulator order, [block][i][child tile][lane][4]
+    float* accv[HTREE_MAX_LEVELS];
+};
+
+int launch_bwd_dq(const BwdParams& bp, int dtype, cudaStream_t st);
+int launch_bwd_dkv(const BwdParams& bp, int dtype, cudaStream_t st);
+int launch_bwd_fold(const BwdParams& bp, int dtype, float* const* gk, float* const* gv, void* dk, void* dv, bool typed, cudaStream_t st);
+
+template <int D, bool X3, int NH, int CR>
+struct BForm {
+    static constexpr int KS = D / 16, NT = CR / 8;
+    static constexpr int QB = D * 16 * (X3 ? 2 : 1);        // bytes of 8 heads of blocked queries (split-half: fp32) or gradients
+    static constexpr int SB = NT * 128 * (X3 ? 2 : 1);      // bytes of P or dS of 8 heads of one visit
+    static constexpr int ACC = D * CR;                      // floats of one parent's accumulator
+};
+
+}  // namespace htree

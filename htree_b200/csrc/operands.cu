@@ -98,8 +98,8 @@ __global__ void __launch_bounds__(128) pack_blocks_kernel(const __grid_constant_
     // ---- keys: rotate by the position inside the chunk ----
     uint32_t kw[2][2][PPT / 2], kl[2][2][X3 ? PPT / 2 : 1];   // [tile or version][half][pair of pairs]
 #pragma unroll
-    for (int tl = 0; tl < 2; ++tl) {
-        const int child = CR == 16 ? 8 * tl + g : g;          // 8 children: tl = 1 is the version for odd slots
+    for (int tl = 0; tl < (C::DUAL ? 1 : 2); ++tl) {
+        const int child = CR == 16 ? 8 * tl + g : g;          // 8 children, split-half: tl = 1 is the version for odd slots
         const bool on = child < cnt;
         float lo[PPT], hi[PPT], x[PPT], y[PPT];
         load_piece<T, PPT>(ks_ + child * rs + PPT * r, on, lo);
@@ -140,12 +140,14 @@ __global__ void __launch_bounds__(128) pack_blocks_kernel(const __grid_constant_
     for (int pl = 0; pl < C::PL; ++pl) {
         auto K = [&](int tl, int hf, int i) { return (X3 && pl) ? kl[tl][hf][X3 ? i : 0] : kw[tl][hf][i]; };
         if constexpr (CR == 16) {
-            uint4* d = reinterpret_cast<uint4*>(dst + pl * C::PART);
+            uint32_t* d = reinterpret_cast<uint32_t*>(dst + pl * C::PART);
 #pragma unroll
-            for (int ks = 0; ks < KS; ++ks) d[ks * 32 + lane] = make_uint4(K(0, 0, ks), K(1, 0, ks), K(0, 1, ks), K(1, 1, ks));
+            for (int ks = 0; ks < KS; ++ks)
+#pragma unroll
+                for (int m = 0; m < 4; ++m) d[(4 * ks + m) * 32 + lane] = K(m & 1, m >> 1, ks);
         } else {
 #pragma unroll
-            for (int vv = 0; vv < 2; ++vv) {      // even-slot version first, odd-slot version after the values
+            for (int vv = 0; vv < (C::DUAL ? 1 : 2); ++vv) {      // even-slot version first, odd-slot version after the values
                 uint32_t* d = reinterpret_cast<uint32_t*>(dst + (vv ? 2 * C::PL * C::PART : 0) + pl * C::PART);
 #pragma unroll
                 for (int ks = 0; ks < KS; ++ks) { d[(2 * ks) * 32 + lane] = K(vv, 0, ks); d[(2 * ks + 1) * 32 + lane] = K(vv, 1, ks); }
@@ -240,9 +242,11 @@ __global__ void __launch_bounds__(128) pack_blocks_kernel(const __grid_constant_
         for (int pl = 0; pl < C::PL; ++pl) {
             auto R = [&](int tl, int hf, int i) { return (X3 && pl) ? rl[X3 ? tl : 0][hf][X3 ? i : 0] : rw[tl][hf][i]; };
             if constexpr (CR == 16) {
-                uint4* d = reinterpret_cast<uint4*>(vd + pl * C::PART);
+                uint32_t* d = reinterpret_cast<uint32_t*>(vd + pl * C::PART);
 #pragma unroll
-                for (int ks = 0; ks < KS; ++ks) d[ks * 32 + lane] = make_uint4(R(0, 0, ks), R(NB - 1, 0, ks), R(0, 1, ks), R(NB - 1, 1, ks));
+                for (int ks = 0; ks < KS; ++ks)
+#pragma unroll
+                    for (int m = 0; m < 4; ++m) d[(4 * ks + m) * 32 + lane] = R((NB - 1) * (m & 1), m >> 1, ks);
             } else {
                 uint32_t* d = reinterpret_cast<uint32_t*>(vd + pl * C::PART);
 #pragma unroll
@@ -252,7 +256,7 @@ __global__ void __launch_bounds__(128) pack_blocks_kernel(const __grid_constant_
     }
 }
 
-size_t pack_block_bytes(int D, bool x3, int CR) { return (size_t)(x3 ? 2 : 1) * D * 2 * CR * (CR == 16 ? 2 : 3); }
+size_t pack_block_bytes(int D, bool x3, int CR) { return (size_t)(x3 ? 2 : 1) * D * 2 * CR * (CR == 16 || !x3 ? 2 : 3); }
 
 bool pack_supported(int dtype, int K, int V, int CR) {
     (void)dtype;

@@ -10,14 +10,19 @@
 // Operand blocks (written by pack_blocks_kernel, read here as whole blocks by asynchronous bulk copies): per parent and KV
 // head the children's pre-rotated keys K' and values in the order in which the lanes consume them as A fragments, so that a
 // fragment is one conflict-free 16-byte shared load.  With lane = 4g + r, KS = D/16, PPT = D/8, VB = D/8:
-//   16 children   K [ks][lane] = { K'[g][lo], K'[8+g][lo], K'[g][hi], K'[8+g][hi] },  lo = dims PPT*r + 2ks + {0,1}, hi = lo + D/2
-//                 V [i][lane]  = { b0(2i), b0(2i+1), b1(2i), b1(2i+1) },  bj(w) = { V[8j+2r][VB*g+w], V[8j+2r+1][VB*g+w] }
-//                 block = [K | V]; 16 bytes are the four registers of one A fragment in their order (an LDS.128 whose
-//                 registers had to be swapped cost 4 moves per fragment, a quarter of the loop's instructions)
-//    8 children   K [ks][lo, hi][lane] and V [w][lane], 4 bytes each: 8x8 matrices that ldmatrix gathers from two parents
-//                 block = [K even | V | K odd]: a parent in an odd slot of the query's list holds positions 8..15 of its
-//                 chunk, so its keys are also stored rotated by 8 more positions; a chunk then has ONE query rotation for
-//                 its 16 positions and full M tiles, as with 16 children
+//   K    8x8 matrices [ks][m][lane] of 4-byte words, m = lo / hi dims (8 children), or children 0-7 lo, 8-15 lo, 0-7 hi, 8-15 hi
+//        (16 children); word of lane (g, r) = K'[child g][lo], lo = dims PPT*r + 2ks + {0,1}, hi = lo + D/2.  ldmatrix gives the
+//        A fragments of S^T = K' q^, ldmatrix.trans those of dq^T = K~^T dS^T
+//   V    16 children: [i][lane] = { b0(2i), b0(2i+1), b1(2i), b1(2i+1) },  8 children: [w][lane] = b0(w),
+//        bj(w) = { V[8j+2r][VB*g+w], V[8j+2r+1][VB*g+w] }
+//        A fragments land in four consecutive registers in their order: a 16-byte load whose registers had to be swapped cost
+//        4 moves per fragment, a quarter of the loop's instructions.
+//   16 children   block = [K | V]
+//    8 children   block = [K | V]; a chunk's two parents have distances 8 apart and the query is rotated for each.
+//    8 children, split-half   block = [K even | V | K odd]: keys also stored rotated by 8 more positions, for parents in odd slots
+//                 of the query's list, which hold positions 8..15 of their chunk: one query rotation per chunk.  (16-bit storage
+//                 does not: a score's rounding is the rounding of these half-precision operands, 2^-11 |q||k|, and with scores of
+//                 70 another choice of operands moves probabilities by a percent.)
 //   split-half (fp32 storage, and every storage type with 32-wide heads): each part is a hi plane followed by a lo plane.
 #pragma once
 #include "mma_common.cuh"
@@ -29,28 +34,32 @@ struct TForm {
     static constexpr int KS = D / 16, HALF = D / 2, PPT = HALF / 4, VB = D / 8, MT = D / 16;
     static constexpr int PL = X3 ? 2 : 1;                                  // planes
     static constexpr int PART = D * 2 * CR;                                // bytes of one plane of one part of a block
-    static constexpr int BLOCK = PL * PART * (CR == 16 ? 2 : 3);           // bytes of a block in global memory
+    static constexpr bool DUAL = CR == 8 && !X3;                           // two query rotations per chunk
+    static constexpr int BLOCK = PL * PART * (CR == 16 || DUAL ? 2 : 3);   // bytes of a block in global memory
+    static constexpr int ODD = DUAL ? 0 : PL * PART;                       // where an odd parent's copy starts in its block
+    static constexpr int NTAB = DUAL ? 2 : 1;
     static constexpr int DATA = PL * D * 64;                               // bytes of a chunk in shared memory
     static constexpr int TAB = X3 ? D * 4 : D * 2;                         // one row of the rotary table: [cos | sin]
-    static constexpr int SLOT = DATA + TAB;
+    static constexpr int SLOT = DATA + NTAB * TAB;
     static constexpr int PPC = 16 / CR;                                    // parents per chunk
-    // part offsets in a slot: 16 children [K | V]; 8 children [K even | V even | V odd | K odd]
+    // part offsets in a slot: 16 children [K | V]; 8 children [K even | V even | K odd | V odd], split-half [.. | V odd | K odd]
     static constexpr int V_OFF = PL * PART;
-    static constexpr int V2_OFF = 2 * PL * PART, K2_OFF = 3 * PL * PART;   // 8 children only
+    static constexpr int V2_OFF = (DUAL ? 3 : 2) * PL * PART, K2_OFF = (DUAL ? 2 : 3) * PL * PART;
 };
 
 // Shared-memory addresses of a chunk slot that differ by lane, as 32-bit shared addresses.
 template <int D, bool X3, int CR>
 struct LaneBase {
-    uint32_t k, v;      // 16 children: slot + 16 * lane (v unused); 8 children: ldmatrix row addresses of the key and value matrices
+    uint32_t k, v, vk;   // ldmatrix rows of the key part; value part (16 children: 16-byte pieces, 8: ldmatrix rows); values in key order
     __device__ __forceinline__ LaneBase(uint32_t slot, int lane) {
         using C = TForm<D, X3, CR>;
         if constexpr (CR == 16) {
-            k = slot + 16 * lane; v = 0;
+            k = slot + 16 * lane; v = k + C::V_OFF; vk = v;
         } else {
             const int j = lane >> 3, row = lane & 7;
             k = slot + ((j & 1) ? C::K2_OFF : 0) + (j >> 1) * 128 + row * 16;
             v = slot + ((j >> 1) ? C::V2_OFF : C::V_OFF) + (j & 1) * 128 + row * 16;
+            vk = slot + ((j & 1) ? C::V2_OFF : C::V_OFF) + (j >> 1) * 128 + row * 16;
         }
     }
 };
@@ -59,6 +68,9 @@ __device__ __forceinline__ void lds_frag(uint32_t addr, uint32_t (&a)[4]) {
 }
 __device__ __forceinline__ void ldmatrix_frag(uint32_t addr, uint32_t (&a)[4]) {
     asm volatile("ldmatrix.sync.aligned.m8n8.x4.shared.b16 {%0,%1,%2,%3}, [%4];\n" : "=r"(a[0]), "=r"(a[1]), "=r"(a[2]), "=r"(a[3]) : "r"(addr));
+}
+__device__ __forceinline__ void ldmatrix_trans_frag(uint32_t addr, uint32_t (&a)[4]) {
+    asm volatile("ldmatrix.sync.aligned.m8n8.x4.trans.shared.b16 {%0,%1,%2,%3}, [%4];\n" : "=r"(a[0]), "=r"(a[1]), "=r"(a[2]), "=r"(a[3]) : "r"(addr));
 }
 __device__ __forceinline__ uint4 lds_u4(uint32_t addr) {
     uint4 x;
@@ -69,14 +81,24 @@ __device__ __forceinline__ uint4 lds_u4(uint32_t addr) {
 template <int D, bool X3, int CR>
 __device__ __forceinline__ void key_frag(const LaneBase<D, X3, CR>& s, int pl, int ks, uint32_t (&a)[4]) {
     using C = TForm<D, X3, CR>;
-    if constexpr (CR == 16) lds_frag(s.k + pl * C::PART + ks * 512, a);
-    else ldmatrix_frag(s.k + pl * C::PART + ks * 256, a);
+    ldmatrix_frag(s.k + pl * C::PART + ks * (CR * 32), a);
+}
+// the same matrices transposed: { children 0-7 lo, 8-15 lo, 0-7 hi, 8-15 hi }, lane (g, r) = { K'[2r][x], K'[2r+1][x] } (+ 8 children),
+// x = lo or hi dim PPT*(g/2) + 2ks + (g & 1)
+template <int D, bool X3, int CR>
+__device__ __forceinline__ void key_frag_trans(const LaneBase<D, X3, CR>& s, int pl, int ks, uint32_t (&a)[4]) {
+    ldmatrix_trans_frag(s.k + pl * TForm<D, X3, CR>::PART + ks * (CR * 32), a);
+}
+// A fragments of k-step ks of the values in key order (backward slots)
+template <int D, bool X3, int CR>
+__device__ __forceinline__ void vk_frag(const LaneBase<D, X3, CR>& s, int pl, int ks, uint32_t (&a)[4]) {
+    ldmatrix_frag(s.vk + pl * TForm<D, X3, CR>::PART + ks * (CR * 32), a);
 }
 // A fragments of output tile i of the value part: dims VB*g + 2i (row g) and VB*g + 2i + 1 (row g + 8)
 template <int D, bool X3, int CR>
 __device__ __forceinline__ void value_frag(const LaneBase<D, X3, CR>& s, int pl, int i, uint32_t (&a)[4]) {
     using C = TForm<D, X3, CR>;
-    if constexpr (CR == 16) lds_frag(s.k + C::V_OFF + pl * C::PART + i * 512, a);
+    if constexpr (CR == 16) lds_frag(s.v + pl * C::PART + i * 512, a);
     else ldmatrix_frag(s.v + pl * C::PART + i * 256, a);
 }
 // d = A B with a zero accumulator (no registers to clear)
@@ -141,26 +163,12 @@ __device__ __forceinline__ void load_query(const T* base, int G, int g, int r, f
 }
 
 // B fragments of k-step ks: the query rotated by the chunk's distance.  `tab` is the chunk's table row in shared memory.
-template <int D>
-struct TabRegs16 {
-    uint32_t c[D / 16], s[D / 16];
-};
-template <int D>
-__device__ __forceinline__ void load_tab16(uint32_t tab, int r, TabRegs16<D>& t) {
-    constexpr int HALF = D / 2, PPT = HALF / 4, KS = D / 16;
-#pragma unroll
-    for (int i = 0; i < KS / 4; ++i) {
-        const uint4 c4 = lds_u4(tab + 2 * (PPT * r) + 16 * i);
-        const uint4 s4 = lds_u4(tab + 2 * HALF + 2 * (PPT * r) + 16 * i);
-        t.c[4 * i] = c4.x; t.c[4 * i + 1] = c4.y; t.c[4 * i + 2] = c4.z; t.c[4 * i + 3] = c4.w;
-        t.s[4 * i] = s4.x; t.s[4 * i + 1] = s4.y; t.s[4 * i + 2] = s4.z; t.s[4 * i + 3] = s4.w;
-    }
-}
 __device__ __forceinline__ __half2 as_h2(uint32_t x) { return *reinterpret_cast<const __half2*>(&x); }
 __device__ __forceinline__ uint32_t as_u32(__half2 x) { return *reinterpret_cast<const uint32_t*>(&x); }
-// (lo, hi) rotated by (c, s): lo*c - hi*s, lo*s + hi*c
-__device__ __forceinline__ void rotate_h2(uint32_t lo, uint32_t hi, uint32_t c, uint32_t s, uint32_t& x, uint32_t& y) {
-    x = as_u32(__hfma2(as_h2(lo), as_h2(c), __hneg2(__hmul2(as_h2(hi), as_h2(s)))));
+__device__ __forceinline__ uint32_t neg_h2(uint32_t x) { return x ^ 0x80008000u; }
+// (lo, hi) rotated by (c, s), ns = -s: lo*c - hi*s, lo*s + hi*c, four packed instructions
+__device__ __forceinline__ void rotate_h2(uint32_t lo, uint32_t hi, uint32_t c, uint32_t s, uint32_t ns, uint32_t& x, uint32_t& y) {
+    x = as_u32(__hfma2(as_h2(lo), as_h2(c), __hmul2(as_h2(hi), as_h2(ns))));
     y = as_u32(__hfma2(as_h2(hi), as_h2(c), __hmul2(as_h2(lo), as_h2(s))));
 }
 
@@ -169,25 +177,50 @@ template <typename T, int D, int NH, int CR>
 __device__ __forceinline__ void score16(const LaneBase<D, false, CR>& s, uint32_t tab, int r, const QueryRegs<T, D, false, NH>& q, float (&S)[NH][4]) {
     using FS = Frag<__half>;
     constexpr int KS = D / 16;
-    TabRegs16<D> t;
-    load_tab16<D>(tab, r, t);
-    float U[NH][4];
+    constexpr int HALF = D / 2, PPT = HALF / 4;
+    constexpr bool DUAL = TForm<D, false, CR>::DUAL;
+    constexpr bool TWO = NH == 1 && !DUAL;     // two accumulation chains per half; two halves or two parents are two chains anyway
+    tab += 2 * (PPT * r);
+    float U[TWO || DUAL ? NH : 1][4];          // second chain, or the odd parent's scores
 #pragma unroll
-    for (int ks = 0; ks < KS; ++ks) {
-        uint32_t a[4];
-        key_frag<D, false, CR>(s, 0, ks, a);
+    for (int k4 = 0; k4 < KS; k4 += 4) {
+        const uint4 c4 = lds_u4(tab + 4 * k4), s4 = lds_u4(tab + 2 * HALF + 4 * k4);
+        const uint32_t c[4] = {c4.x, c4.y, c4.z, c4.w}, sn[4] = {s4.x, s4.y, s4.z, s4.w};
+        uint32_t c2[4], sn2[4];
+        if constexpr (DUAL) {
+            const uint4 d4 = lds_u4(tab + 2 * D + 4 * k4), t4 = lds_u4(tab + 2 * D + 2 * HALF + 4 * k4);
+            c2[0] = d4.x; c2[1] = d4.y; c2[2] = d4.z; c2[3] = d4.w;
+            sn2[0] = t4.x; sn2[1] = t4.y; sn2[2] = t4.z; sn2[3] = t4.w;
+        }
 #pragma unroll
-        for (int h = 0; h < NH; ++h) {
-            uint32_t b0, b1;
-            rotate_h2(q.v[h][0][ks], q.v[h][1][ks], t.c[ks], t.s[ks], b0, b1);
-            if (ks < 2) mma_zero<__half>(ks ? U[h] : S[h], a, b0, b1);         // two accumulation chains
-            else FS::mma((ks & 1) ? U[h] : S[h], a[0], a[1], a[2], a[3], b0, b1);
+        for (int u = 0; u < 4; ++u) {
+            const int ks = k4 + u;
+            uint32_t a[4];
+            key_frag<D, false, CR>(s, 0, ks, a);
+            const uint32_t ns = neg_h2(sn[u]);
+#pragma unroll
+            for (int h = 0; h < NH; ++h) {
+                uint32_t b0, b1;
+                rotate_h2(q.v[h][0][ks], q.v[h][1][ks], c[u], sn[u], ns, b0, b1);
+                float (&acc)[4] = TWO && (ks & 1) ? U[TWO ? h : 0] : S[h];
+                if (ks < (TWO ? 2 : 1)) mma_zero<__half>(acc, a, b0, b1);
+                else FS::mma(acc, a[0], a[1], a[2], a[3], b0, b1);
+                if constexpr (DUAL) {
+                    rotate_h2(q.v[h][0][ks], q.v[h][1][ks], c2[u], sn2[u], neg_h2(sn2[u]), b0, b1);
+                    if (ks == 0) mma_zero<__half>(U[DUAL ? h : 0], a, b0, b1);
+                    else FS::mma(U[DUAL ? h : 0], a[0], a[1], a[2], a[3], b0, b1);
+                }
+            }
         }
     }
 #pragma unroll
-    for (int h = 0; h < NH; ++h)
+    for (int h = 0; h < NH; ++h) {
+        if constexpr (DUAL) { S[h][2] = U[DUAL ? h : 0][2]; S[h][3] = U[DUAL ? h : 0][3]; }     // rows 8..15 are the odd parent's children
+        else if constexpr (TWO) {
 #pragma unroll
-        for (int i = 0; i < 4; ++i) S[h][i] += U[h][i];
+            for (int i = 0; i < 4; ++i) S[h][i] += U[TWO ? h : 0][i];
+        }
+    }
 }
 
 // Split-half form (see mma_common.cuh for why the leading product of every k-step is summed with ordinary fp32 adds).

@@ -225,6 +225,6 @@ def _by_units(q, k, v, dO, outs, dev, streams, compression_rate, max_top_nodes, 
                                 _copy_unit(outs[3][b:b + 1, :, hk:hk + 1], dv, s_out)
                     held([q_d, o] + ([dO_d, dq] if bwd else []) + ([dk, dv] if bwd and last else []))
                 if bwd:
-                    held([x for lst in (acc["dk"], acc["dv"]) for x in lst])
+                    held([x for part in acc.values() for x in (part if isinstance(part, list) else [part])])
     s_out.synchronize(); s_run.synchronize(); s_in.synchronize()
     return tuple(outs)

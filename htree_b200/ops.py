@@ -44,6 +44,11 @@ SELECTION_STORAGE = "int32"
 SPLIT_FORWARD_MAX_BYTES = 4 << 30
 
 
+# Scratch of the two-pass backward (htree_b200_run_backward): P and dS of the queries of one launch.  Larger means fewer
+# launches; a shape that does not fit at all takes the one-pass backward, which needs none.
+BACKWARD_MAX_BYTES = 4 << 30
+
+
 def _parents_dtype(layers_k, top_k: int):
     if SELECTION_STORAGE == "int32":
         return torch.int32
@@ -312,7 +317,7 @@ class _Workspace:
     def _block_bytes(self, l):
         B, _, H_kv, K = self.k.shape
         n = B * ((self.plan.nodes[l] + self.cr - 1) // self.cr) * H_kv * (2 if _split(self.k.dtype, K) else 1) * K * 2 * self.cr
-        return n * (2 if self.cr == 16 else 3), n
+        return n * (2 if self.cr == 16 or not _split(self.k.dtype, K) else 3), n
 
 
 class BwdContext(dict):
@@ -683,6 +688,79 @@ def recompute_parents(q, layers_k, layers_v, cos_cache, sin_cache, compression_r
     return {l: parents[l] for l in range(L)}
 
 
+_DO_DTYPE = ("dO has dtype {} but q has {}: pass the output gradient in the operator's storage type (cast it explicitly if the loss "
+             "of precision is acceptable)")
+_bwd_plans: Dict[Tuple, Optional[Tuple[int, int]]] = {}
+
+
+def _backward_operands(q, ctx):
+    """(blocks pointers, blocks_bwd pointers, T, H_kv) of a context with the transposed kernels' operands, else None."""
+    ws = getattr(ctx, "workspace", None)
+    if ws is not None and not dict.__contains__(ctx, "layers_k"):
+        p, base = ws.plan, ws.ws.data_ptr()
+        if p.blocks_bwd[0] < 0:
+            return None
+        L = range(p.levels)
+        return ([base + p.blocks[l] for l in L], [base + p.blocks_bwd[l] for l in L], ws.k.shape[1], ws.k.shape[2])
+    blk = ctx.get("layers_v_blk")
+    if getattr(blk, "blocks_bwd", None) is None:
+        return None
+    k = ctx["layers_k"][0]
+    return ([x.data_ptr() for x in blk.blocks], [x.data_ptr() for x in blk.blocks_bwd], k.shape[1], k.shape[2])
+
+
+def _backward_two_pass(dO, q, output, ctx, operands, typed, window):
+    """The backward on the two-pass kernels; None where their scratch does not fit BACKWARD_MAX_BYTES or an operand is not
+    32-byte aligned (the one-pass backward then runs)."""
+    B, Tq, H, K = q.shape
+    blocks, blocks_bwd, T, H_kv = operands
+    if (q.data_ptr() | dO.data_ptr() | output.data_ptr()) % 32:
+        return None
+    CR, TK, MTN = int(ctx["compression_rate"]), int(ctx["top_k_per_layer"]), int(ctx["max_top_nodes"])
+    budget = BACKWARD_MAX_BYTES
+    key = (B, T, H, H_kv, K, CR, TK, MTN, q.dtype, Tq, budget)
+    shape = _lib.HtreeShape(B, T, H, H_kv, K, K, CR, TK, MTN, _DTYPES[q.dtype], 0 if window is None else Tq,
+                            0 if window is None else int(window["t0"]))
+    if key not in _bwd_plans:
+        a, s = ctypes.c_int64(), ctypes.c_int64()
+        rc = _lib.lib().htree_b200_backward_plan(ctypes.byref(shape), budget, ctypes.byref(a), ctypes.byref(s))
+        if len(_bwd_plans) >= 512:
+            _bwd_plans.clear()
+        _bwd_plans[key] = (a.value, s.value) if rc == 0 else None
+    plan = _bwd_plans[key]
+    if plan is None or window is not None and not window["first"] and "two_pass" not in window["acc"]:
+        return None
+    dev, dtype = q.device, q.dtype
+    parents = ctx.get("per_layer_parents")
+    if parents is None:
+        parents = recompute_parents(q, ctx["layers_k"], ctx["layers_v"], ctx["cos_cache"], ctx["sin_cache"], CR, TK, MTN, ctx["scale"],
+                                    ctx.get("layers_k_rot"))
+    n_pos = ctx["cos_cache"].shape[0]
+    table = rope_rows(K, n_pos, ctx["rope_base"], None if _split(dtype, K) else ctx["scale"], dev)
+    if window is None:
+        acc, flags, final = torch.empty(plan[0], dtype=torch.uint8, device=dev), 0, True
+    else:
+        if window["first"]:
+            window["acc"]["two_pass"] = torch.empty(plan[0], dtype=torch.uint8, device=dev)
+        acc, final = window["acc"]["two_pass"], window["last"]
+        flags = (0 if window["first"] else _lib.BWD_KEEP_ACCUM) | (0 if final else _lib.BWD_NO_FOLD)
+    scratch = torch.empty(plan[1], dtype=torch.uint8, device=dev)
+    gdt = dtype if typed else torch.float32
+    dq = torch.empty(B, Tq, H, K, dtype=gdt, device=dev)
+    dk, dv = (torch.empty(B, T, H_kv, K, dtype=gdt, device=dev) for _ in range(2)) if final else (None, None)
+    L = len(blocks)
+    pl = [parents[l] for l in range(L)]
+    with torch.cuda.device(dev):
+        rc = _lib.lib().htree_b200_run_backward(
+            ctypes.byref(shape), q.data_ptr(), _lib.ptr_array(blocks), _lib.ptr_array(blocks_bwd), ctx["cos_cache"].data_ptr(),
+            ctx["sin_cache"].data_ptr(), table.data_ptr(), n_pos, float(ctx["scale"]), output.data_ptr(), dO.data_ptr(),
+            ctx["global_max"].data_ptr(), ctx["global_sum"].data_ptr(), _ptrs(pl), acc.data_ptr(), scratch.data_ptr(), budget,
+            dq.data_ptr(), dk.data_ptr() if final else None, dv.data_ptr() if final else None, int(typed), _status(dev).data_ptr(),
+            flags | _parents_flag(pl), _stream())
+    _lib.check(rc, "backward")
+    return dq, dk, dv
+
+
 def htree_backward(dO: torch.Tensor, q: torch.Tensor, output: torch.Tensor, bwd_ctx: dict, _force_generic: bool = False,
                    _typed: bool = False, _window: Optional[dict] = None):
     """Backward given the forward context; returns fp32 (dq, dk, dv) with the shapes of q, k, v
@@ -700,6 +778,13 @@ def htree_backward(dO: torch.Tensor, q: torch.Tensor, output: torch.Tensor, bwd_
     window (a forward called with `_q_offset`); dq is returned for the window, dk and dv only with the last window
     (None before)."""
     B, T, H, K = q.shape
+    two_pass = None if _force_generic else _backward_operands(q, bwd_ctx)
+    if two_pass is not None:
+        if dO.dtype != q.dtype:
+            raise ValueError(_DO_DTYPE.format(dO.dtype, q.dtype))
+        res = _backward_two_pass(dO.contiguous(), q.contiguous(), output.contiguous(), bwd_ctx, two_pass, _typed, _window)
+        if res is not None:
+            return res
     layers_k, layers_v = bwd_ctx["layers_k"], bwd_ctx["layers_v"]
     H_kv, V = layers_k[0].shape[2], layers_v[0].shape[-1]
     L = bwd_ctx["num_layers"]
@@ -711,8 +796,7 @@ def htree_backward(dO: torch.Tensor, q: torch.Tensor, output: torch.Tensor, bwd_
     dev = q.device
     q = q.contiguous()
     if dO.dtype != q.dtype:
-        raise ValueError(f"dO has dtype {dO.dtype} but q has {q.dtype}: pass the output gradient in the operator's storage "
-                         "type (cast it explicitly if the loss of precision is acceptable)")
+        raise ValueError(_DO_DTYPE.format(dO.dtype, q.dtype))
     dO = dO.contiguous()
     output = output.contiguous()
     parents = bwd_ctx.get("per_layer_parents")
@@ -783,7 +867,7 @@ class HTreeFunction(torch.autograd.Function):
     def backward(ctx, dO):
         q, k, v, output, gmax, gsum = ctx.saved_tensors
         c = ctx.bwd_ctx
-        if c["layers_k"] is None:
+        if getattr(c, "workspace", None) is None and c["layers_k"] is None:
             c = dict(c)
             c["layers_k"], c["layers_v"], c["layers_k_rot"], c["layers_v_blk"] = build_operands(
                 k, v, c["compression_rate"], c["max_top_nodes"], c["rope_base"], backward=True)

@@ -279,6 +279,21 @@ int htree_b200_backward(const HtreeShape* shape, const void* q, void* const* lay
                         float* const* dk_levels, float* const* dv_levels, const HtreeTypedGrads* typed, int32_t* status,
                         uint32_t flags, void* stream);
 
+/* The backward in two passes over a scratch buffer (shapes of htree_b200_prepare): a query-stationary pass computes dq and leaves
+ * P and dS of every visit (a query's visit to a parent) in `scratch`, a parent-stationary pass sums dK and dV from them.
+ * Same reference kernels and results as htree_b200_backward, and the same query windows (HTREE_BWD_KEEP_ACCUM,
+ * HTREE_BWD_NO_FOLD; `acc` is what the calls of one backward share).
+ *   budget    bytes the scratch may take; htree_b200_backward_plan returns how many of them, and of `acc`, are used
+ *             (HTREE_E_SCRATCH: too little even for the smallest launch; HTREE_E_UNSUPPORTED: not a shape of this path)
+ *   dq, dk, dv  fp32, or with typed != 0 the storage type (dk, dv may be NULL with HTREE_BWD_NO_FOLD)
+ *   q, out, dO 32-byte aligned, everything else 16-byte */
+int htree_b200_backward_plan(const HtreeShape* shape, int64_t budget, int64_t* acc_bytes, int64_t* scratch_bytes);
+int htree_b200_run_backward(const HtreeShape* shape, const void* q, void* const* blocks, void* const* blocks_bwd,
+                            const float* cos_cache, const float* sin_cache, const void* table, int32_t n_pos, float scale,
+                            const void* out, const void* dO, const float* gmax, const float* gsum, int32_t* const* parents,
+                            void* acc, void* scratch, int64_t budget, void* dq, void* dk, void* dv, int32_t typed, int32_t* status,
+                            uint32_t flags, void* stream);
+
 /* Backward without caller-provided scratch.  No counterpart in the reference (its backward allocates its level
  * buffers with torch, src/backward.py:979-981); it exists for callers that cannot allocate device memory around
  * the call: a host program that reaches this library through a plain FFI and holds only the tensors its framework

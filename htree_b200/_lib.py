@@ -61,7 +61,7 @@ class HtreeShape(ctypes.Structure):
 
 class HtreePlan(ctypes.Structure):
     _fields_ = ([("bytes", ctypes.c_int64)] +
-                [(n, ctypes.c_int64 * MAX_LEVELS) for n in ("layers_k", "layers_v", "layers_k_rot", "blocks", "blocks_bwd", "parents")] +
+                [(n, ctypes.c_int64 * MAX_LEVELS) for n in ("layers_k", "layers_v", "blocks", "blocks_bwd", "parents")] +
                 [("nodes", ctypes.c_int32 * MAX_LEVELS), ("levels", ctypes.c_int32), ("reserved", ctypes.c_int32)])
 
 
@@ -114,13 +114,13 @@ def lib() -> ctypes.CDLL:
         L.htree_b200_operand_block_bytes.restype = ctypes.c_int64
         L.htree_b200_operand_block_bytes.argtypes = [ctypes.POINTER(HtreeShape), i32, i32]
         L.htree_b200_prepare.restype = ctypes.c_int
-        L.htree_b200_prepare.argtypes = [ctypes.POINTER(HtreeShape), vp, vp, vp, vp, vp, i32, vp, vp, vp]
+        L.htree_b200_prepare.argtypes = [ctypes.POINTER(HtreeShape), vp, vp, vp, vp, i32, vp, vp, vp]
         L.htree_b200_attend.restype = ctypes.c_int
         L.htree_b200_attend.argtypes = [ctypes.POINTER(HtreeShape), vp, vp, vp, vp, vp, vp, vp, vp, i32, f32, vp, vp, vp, vp, vp, u32, vp]
         L.htree_b200_plan.restype = ctypes.c_int
         L.htree_b200_plan.argtypes = [ctypes.POINTER(HtreeShape), u32, ctypes.POINTER(HtreePlan)]
         L.htree_b200_run_forward.restype = ctypes.c_int
-        L.htree_b200_run_forward.argtypes = [ctypes.POINTER(HtreeShape), ctypes.POINTER(HtreePlan), vp, vp, vp, vp, vp, vp, i32, f32, vp,
+        L.htree_b200_run_forward.argtypes = [ctypes.POINTER(HtreeShape), ctypes.POINTER(HtreePlan), vp, vp, vp, vp, vp, vp, vp, i32, f32, vp,
                                              vp, vp, vp, vp, vp, u32, vp]
         L.htree_b200_backward_plan.restype = ctypes.c_int
         L.htree_b200_backward_plan.argtypes = [ctypes.POINTER(HtreeShape), ctypes.c_int64, vp, vp]

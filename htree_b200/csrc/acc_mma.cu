@@ -4,7 +4,7 @@
 // (src/parallel.py:248-867); reads the parent lists that a selection launch wrote.
 //
 // Products, operand blocks and chunk numbering: tform.cuh.  Per chunk of 16 positions a warp copies the operand block(s) and
-// one rotary-table row into its ring in shared memory (two bulk copies, issued NSTG - 1 chunks ahead), forms
+// one rotary-table row into its ring in shared memory (asynchronously, NSTG - 1 chunks ahead), forms
 // S^T = K' q^ (one query rotation per chunk), P^T, and O^T += V^T P^T.
 #include "tform.cuh"
 
@@ -23,9 +23,10 @@ template <typename T, int D, bool X3, int NH, int CR, bool SPLIT>
 __global__ void __launch_bounds__(SPLIT ? 256 : kAccWarps * 32, SPLIT ? 1 : acc_min_blocks<D, X3, NH>())
 acc_mma_kernel(const __grid_constant__ AttnParams p) {
     using C = TForm<D, X3, CR>;
-    using F = Frag<typename std::conditional<X3, __half, T>::type>;   // type of the values and probabilities
+    using FT = typename std::conditional<X3, __half, T>::type;        // type of the values and probabilities
+    using F = Frag<FT>;
     constexpr int MT = C::MT, PPC = C::PPC;
-    using Ring = ChunkRing<acc_stages<D, X3>(), C::SLOT>;
+    using Ring = WarpRing<acc_stages<D, X3>(), C::SLOT>;
     constexpr int NSTG = acc_stages<D, X3>();
     extern __shared__ __align__(128) unsigned char smem_raw[];
 
@@ -42,7 +43,7 @@ acc_mma_kernel(const __grid_constant__ AttnParams p) {
     const size_t per_warp = (Ring::kBytes + sizeof(int32_t) * TK + sizeof(uint32_t) * ((TK * CR + 31) / 32) + 127) & ~size_t(127);
     unsigned char* wbase = smem_raw + warp * per_warp;
     Ring ring;
-    ring.init(wbase, lane);
+    ring.init(wbase);
     int32_t* par = reinterpret_cast<int32_t*>(wbase + Ring::kBytes);
     uint32_t* selw = reinterpret_cast<uint32_t*>(par + TK);
 
@@ -100,38 +101,39 @@ acc_mma_kernel(const __grid_constant__ AttnParams p) {
         const int nblk = (Nl + CR - 1) / CR;
         const int64_t bstride = (int64_t)p.Hkv * C::BLOCK;
         const unsigned char* blk = reinterpret_cast<const unsigned char*>(p.blk[l]) + ((int64_t)b * nblk * p.Hkv + hk) * C::BLOCK;
-        const unsigned char* tab = reinterpret_cast<const unsigned char*>(p.tab) + (int64_t)(rp - 16 * first) * C::TAB;   // of the next issue
-        auto issue = [&](int c) {                                     // chunk c of this level
-            if (lane == 0) {
-                ring.expect(C::SLOT);
-                int p0 = par[c * PPC];
-                if ((unsigned)p0 >= (unsigned)nblk) { if (p.status) atomicOr(p.status, 4); p0 = 0; }
-                if constexpr (CR == 16) {
-                    ring.copy(0, blk + p0 * bstride, C::DATA);
-                } else {
-                    int p1 = c * PPC + 1 < np ? par[c * PPC + 1] : p0;    // past the end of the list: masked, any finite block
-                    if ((unsigned)p1 >= (unsigned)nblk) { if (p.status) atomicOr(p.status, 4); p1 = 0; }
-                    ring.copy(0, blk + p0 * bstride, C::DATA / 2);
-                    ring.copy(C::DATA / 2, blk + p1 * bstride + C::ODD, C::DATA / 2);
-                }
-                ring.copy(C::DATA, tab, C::TAB);
-                if constexpr (C::DUAL) ring.copy(C::DATA + C::TAB, rp - 16 * c >= 8 ? tab - 8 * C::TAB : tab, C::TAB);
+        const unsigned char* tab = reinterpret_cast<const unsigned char*>(p.tab);
+        auto fill = [&](int c) {                                      // chunk c of this level
+            int p0 = par[c * PPC];
+            if ((unsigned)p0 >= (unsigned)nblk) { if (p.status) atomicOr(p.status, 4); p0 = 0; }
+            if constexpr (CR == 16) {
+                ring.template copy<C::DATA>(0, blk + p0 * bstride, lane);
+            } else {
+                int p1 = c * PPC + 1 < np ? par[c * PPC + 1] : p0;    // past the end of the list: masked, any finite block
+                if ((unsigned)p1 >= (unsigned)nblk) { if (p.status) atomicOr(p.status, 4); p1 = 0; }
+                ring.template copy<C::DATA / 2>(0, blk + p0 * bstride, lane);
+                ring.template copy<C::DATA / 2>(C::DATA / 2, blk + p1 * bstride + C::ODD, lane);
             }
-            tab -= (int64_t)16 * C::TAB * step;
-            ring.issued();
+            const unsigned char* row = tab + (int64_t)(rp - 16 * c) * C::TAB;
+            ring.template copy<C::TAB>(C::DATA, row, lane);
+            if constexpr (C::DUAL) ring.template copy<C::TAB>(C::DATA + C::TAB, rp - 16 * c >= 8 ? row - 8 * C::TAB : row, lane);
         };
+        ring.start();
         int next = first;
 #pragma unroll 1
-        for (int s = 0; s < NSTG - 1 && next < nchunk; ++s, next += step) issue(next);
+        for (int s = 0; s < NSTG - 1; ++s, next += step) {
+            if (next < nchunk) fill(next);
+            ring.commit();
+        }
 #pragma unroll 1
         for (int c = first; c < nchunk; c += step) {
             __syncwarp();                                             // everybody is done with the slot that is refilled now
-            if (next < nchunk) { issue(next); next += step; }
+            if (next < nchunk) fill(next);
+            ring.commit();
+            next += step;
             uint32_t mask = 0xffffu;
             if (l > 0) mask &= ~(selw[c >> 1] >> ((16 * c) & 31));
             if (16 * c + 15 > rp) mask &= (2u << (rp - 16 * c)) - 1u;
-            uint32_t slot;
-            if (!ring.wait(slot)) { if (lane == 0 && p.status) atomicOr(p.status, 16); ring.drain(); return; }
+            const uint32_t slot = ring.wait();
             if (mask == 0) continue;
             const LaneBase<D, X3, CR> lb(slot, lane);
             float S[NH][4];
@@ -185,10 +187,10 @@ acc_mma_kernel(const __grid_constant__ AttnParams p) {
                 if constexpr (X3) {
                     uint32_t h0, l0, h1, l1;
                     split_half2(P[0], P[1], h0, l0); split_half2(P[2], P[3], h1, l1);
-                    pb[h][0] = movmatrix_trans(h0); pb[h][1] = movmatrix_trans(h1);
-                    pl[X3 ? h : 0][0] = movmatrix_trans(l0); pl[X3 ? h : 0][1] = movmatrix_trans(l1);
+                    pb[h][0] = movm(h0); pb[h][1] = movm(h1);
+                    pl[X3 ? h : 0][0] = movm(l0); pl[X3 ? h : 0][1] = movm(l1);
                 } else {
-                    pb[h][0] = movmatrix_trans(F::pack(P[0], P[1])); pb[h][1] = movmatrix_trans(F::pack(P[2], P[3]));
+                    pb[h][0] = movm(F::pack(P[0], P[1])); pb[h][1] = movm(F::pack(P[2], P[3]));
                 }
             }
 #pragma unroll
@@ -204,14 +206,14 @@ acc_mma_kernel(const __grid_constant__ AttnParams p) {
                     for (int h = 0; h < NH; ++h) {
                         float acc[4];
                         mma_zero<__half>(acc, va, pl[X3 ? h : 0][0], pl[X3 ? h : 0][1]);
-                        F::mma(acc, vl[0], vl[1], vl[2], vl[3], pb[h][0], pb[h][1]);
-                        F::mma(acc, va[0], va[1], va[2], va[3], pb[h][0], pb[h][1]);
+                        mma_acc<FT>(acc, vl, pb[h][0], pb[h][1]);
+                        mma_acc<FT>(acc, va, pb[h][0], pb[h][1]);
 #pragma unroll
                         for (int u = 0; u < 4; ++u) O[h][i][u] += acc[u];
                     }
                 } else {
 #pragma unroll
-                    for (int h = 0; h < NH; ++h) F::mma(O[h][i], va[0], va[1], va[2], va[3], pb[h][0], pb[h][1]);
+                    for (int h = 0; h < NH; ++h) mma_acc<FT>(O[h][i], va, pb[h][0], pb[h][1]);
                 }
             }
         }
@@ -229,6 +231,7 @@ acc_mma_kernel(const __grid_constant__ AttnParams p) {
             }
     if constexpr (SPLIT) {
         // merge the warps' partial states (few queries: a group's chunks are spread over the warps of a block)
+        ring.idle();
         __syncthreads();                                              // all rings are idle: their memory is free
         float* st = reinterpret_cast<float*>(smem_raw + W * per_warp);          // [W][3][16]: m_run, m_true, s
         float* po = reinterpret_cast<float*>(wbase);                  // this warp's O, [16 heads][D]
@@ -304,7 +307,7 @@ acc_mma_kernel(const __grid_constant__ AttnParams p) {
 template <typename T, int D, bool X3, int NH, int CR>
 static int launch_acc_cr(const AttnParams& p, cudaStream_t st) {
     using C = TForm<D, X3, CR>;
-    using Ring = ChunkRing<acc_stages<D, X3>(), C::SLOT>;
+    using Ring = WarpRing<acc_stages<D, X3>(), C::SLOT>;
     const size_t per_warp = (Ring::kBytes + sizeof(int32_t) * p.TK + sizeof(uint32_t) * ((p.TK * CR + 31) / 32) + 127) & ~size_t(127);
     const size_t limit = 227 * 1024;
     // Few groups: one block of 8 warps per group.  Below two groups per SM the chip has room for all their warps at once, and

@@ -246,52 +246,46 @@ int64_t htree_b200_operand_block_bytes(const HtreeShape* shape, int32_t level, i
 }
 
 int htree_b200_prepare(const HtreeShape* shape, void* const* layers_k, void* const* layers_v, void* const* blocks,
-                       void* const* blocks_bwd, void* const* layers_k_rot, int32_t pool, const float* cos_cache,
-                       const float* sin_cache, void* stream) {
+                       void* const* blocks_bwd, int32_t pool, const float* cos_cache, const float* sin_cache, void* stream) {
     int32_t ln[HTREE_MAX_LEVELS];
     const int L = check_shape(shape, ln, false);
     if (L < 0) return L;
     if (!layers_k || !layers_v || !blocks || !cos_cache || !sin_cache) return HTREE_E_NULL;
     if (!pack_supported(shape->dtype, shape->K, shape->V, shape->compression_rate)) return HTREE_E_UNSUPPORTED;
-    if (layers_k_rot && (shape->K == 32 || (shape->dtype == HTREE_F32 && shape->K != 64))) return HTREE_E_UNSUPPORTED;
     if (!aligned16(cos_cache) || !aligned16(sin_cache)) return HTREE_E_ALIGN;
     for (int l = 0; l < L; ++l) {
         if (!layers_k[l] || !layers_v[l] || !blocks[l] || (blocks_bwd && !blocks_bwd[l])) return HTREE_E_NULL;
-        if (!aligned16(layers_k[l]) || !aligned16(layers_v[l]) || !aligned16(blocks[l]) || (blocks_bwd && !aligned16(blocks_bwd[l])) ||
-            (layers_k_rot && layers_k_rot[l] && !aligned16(layers_k_rot[l])))
+        if (!aligned16(layers_k[l]) || !aligned16(layers_v[l]) || !aligned16(blocks[l]) || (blocks_bwd && !aligned16(blocks_bwd[l])))
             return HTREE_E_ALIGN;
     }
-    return launch_pack_blocks(*shape, L, ln, layers_k, layers_v, blocks, blocks_bwd, layers_k_rot, pool != 0, cos_cache, sin_cache,
+    return launch_pack_blocks(*shape, L, ln, layers_k, layers_v, blocks, blocks_bwd, pool != 0, cos_cache, sin_cache,
                               (cudaStream_t)stream);
 }
 
-int htree_b200_attend(const HtreeShape* shape, const void* q, void* const* layers_k, void* const* layers_v, void* const* layers_k_rot,
-                      void* const* blocks, const float* cos_cache, const float* sin_cache, const void* table, int32_t n_pos,
-                      float scale, void* out, float* gmax, float* gsum, int32_t* const* parents, int32_t* status, uint32_t flags,
-                      void* stream) {
+int htree_b200_attend(const HtreeShape* shape, const void* q, void* const* layers_k, void* const* layers_v, void* const* blocks,
+                      const float* cos_cache, const float* sin_cache, const void* table, const void* table_f32, int32_t n_pos, float scale,
+                      void* out, float* gmax, float* gsum, int32_t* const* parents, int32_t* status, uint32_t flags, void* stream) {
     int32_t ln[HTREE_MAX_LEVELS];
     const int L = check_shape(shape, ln);
     if (L < 0) return L;
     AttnParams p;
     int rc = fill_params(p, shape, L, ln, q, layers_k, layers_v, cos_cache, sin_cache, n_pos, scale, parents, status, flags);
     if (rc) return rc;
-    if (!out || !gmax || !gsum || !blocks || !table || !parents) return HTREE_E_NULL;
-    if (!aligned16(out) || !aligned16(table)) return HTREE_E_ALIGN;
-    p.out = out; p.gmax = gmax; p.gsum = gsum; p.tab = table;
+    const bool select_only = (flags & HTREE_FWD_SELECT_ONLY) != 0;
+    if (!blocks || !table || !table_f32 || !parents || (!select_only && (!out || !gmax || !gsum))) return HTREE_E_NULL;
+    if (!aligned16(out) || !aligned16(table) || !aligned16(table_f32) || !aligned32(q)) return HTREE_E_ALIGN;
+    p.out = out; p.gmax = gmax; p.gsum = gsum; p.tab = table; p.tab32 = table_f32;
     for (int l = 0; l < L; ++l) {
         if (!parents[l] || !blocks[l]) return HTREE_E_NULL;
         if (!aligned16(blocks[l])) return HTREE_E_ALIGN;
         p.blk[l] = blocks[l];
     }
-    if (!aligned32(q)) return HTREE_E_ALIGN;
     if (!acc_mma_supported(p, shape->dtype)) return HTREE_E_UNSUPPORTED;
     p.flags = flags | HTREE_FWD_SELECT_ONLY;
-    bool fast = layers_k_rot != nullptr && aligned32(cos_cache) && aligned32(sin_cache);
-    for (int l = 1; l < L && fast; ++l) { p.lkr[l] = layers_k_rot[l]; fast = layers_k_rot[l] && aligned32(layers_k_rot[l]); }
-    rc = fast && select_mma_supported(p, shape->dtype) ? launch_fwd_mma(p, shape->dtype, (cudaStream_t)stream)
-                                                       : launch_fwd_generic(p, shape->dtype, (cudaStream_t)stream);
-    if (rc) return rc;
-    p.flags = (flags & ~HTREE_FWD_SELECT_ONLY) | ((flags & HTREE_FWD_INFERENCE) ? kFlagSplitOk : 0u);
+    rc = select_blk_supported(p, shape->dtype) ? launch_select_blk(p, shape->dtype, (cudaStream_t)stream)
+                                               : launch_fwd_generic(p, shape->dtype, (cudaStream_t)stream);
+    if (rc || select_only) return rc;
+    p.flags = flags | ((flags & HTREE_FWD_INFERENCE) ? kFlagSplitOk : 0u);
     return launch_acc_mma(p, shape->dtype, (cudaStream_t)stream);
 }
 
@@ -304,7 +298,6 @@ int htree_b200_plan(const HtreeShape* shape, uint32_t flags, HtreePlan* plan) {
     if (!pack_supported(shape->dtype, shape->K, shape->V, shape->compression_rate) || shape->H / shape->H_kv > 16) return HTREE_E_UNSUPPORTED;
     const int es = esize(shape->dtype), CR = shape->compression_rate;
     const bool x3 = pack_split(shape->dtype, shape->K);
-    const bool rot = shape->K == 64 || (shape->K == 128 && shape->dtype != HTREE_F32);   // shapes with a tensor-core selection kernel
     const int64_t Tq = shape->T_q > 0 ? shape->T_q : shape->T;
     int64_t at = 0;
     auto take = [&](int64_t bytes) { const int64_t o = at; at += (bytes + 255) & ~int64_t(255); return o; };
@@ -314,7 +307,6 @@ int htree_b200_plan(const HtreeShape* shape, uint32_t flags, HtreePlan* plan) {
         plan->nodes[l] = ln[l];
         plan->layers_k[l] = l ? take(rows * shape->K * es) : -1;
         plan->layers_v[l] = l ? take(rows * shape->V * es) : -1;
-        plan->layers_k_rot[l] = rot && (l || (flags & HTREE_PLAN_BACKWARD)) ? take(rows * shape->K * (x3 ? 4 : 2)) : -1;
         plan->blocks[l] = take(blocks * (int64_t)pack_block_bytes(shape->K, x3, CR));
         plan->blocks_bwd[l] = flags & HTREE_PLAN_BACKWARD ? take(blocks * (x3 ? 2 : 1) * shape->K * 2 * CR) : -1;
         plan->parents[l] = flags & HTREE_PLAN_PARENTS ? take((int64_t)shape->B * Tq * shape->H_kv * shape->top_k * 4) : -1;
@@ -324,27 +316,25 @@ int htree_b200_plan(const HtreeShape* shape, uint32_t flags, HtreePlan* plan) {
 }
 
 int htree_b200_run_forward(const HtreeShape* shape, const HtreePlan* plan, const void* q, const void* k, const void* v,
-                           const float* cos_cache, const float* sin_cache, const void* table, int32_t n_pos, float scale,
-                           void* workspace, void* out, float* gmax, float* gsum, int32_t* const* parents, int32_t* status,
+                           const float* cos_cache, const float* sin_cache, const void* table, const void* table_f32, int32_t n_pos,
+                           float scale, void* workspace, void* out, float* gmax, float* gsum, int32_t* const* parents, int32_t* status,
                            uint32_t flags, void* stream) {
     if (!shape || !plan || !k || !v || !workspace) return HTREE_E_NULL;
     if (plan->levels <= 0 || plan->levels > HTREE_MAX_LEVELS) return HTREE_E_LEVELS;
-    void *lk[HTREE_MAX_LEVELS], *lv[HTREE_MAX_LEVELS], *lr[HTREE_MAX_LEVELS], *bl[HTREE_MAX_LEVELS], *bb[HTREE_MAX_LEVELS];
+    void *lk[HTREE_MAX_LEVELS], *lv[HTREE_MAX_LEVELS], *bl[HTREE_MAX_LEVELS], *bb[HTREE_MAX_LEVELS];
     int32_t* par[HTREE_MAX_LEVELS];
     unsigned char* w = static_cast<unsigned char*>(workspace);
     auto at = [&](int64_t o) { return o < 0 ? nullptr : w + o; };
     for (int l = 0; l < plan->levels; ++l) {
         lk[l] = l ? (void*)at(plan->layers_k[l]) : const_cast<void*>(k);
         lv[l] = l ? (void*)at(plan->layers_v[l]) : const_cast<void*>(v);
-        lr[l] = at(plan->layers_k_rot[l]); bl[l] = at(plan->blocks[l]); bb[l] = at(plan->blocks_bwd[l]);
+        bl[l] = at(plan->blocks[l]); bb[l] = at(plan->blocks_bwd[l]);
         par[l] = parents ? parents[l] : reinterpret_cast<int32_t*>(at(plan->parents[l]));
     }
-    const bool rot = plan->levels > 1 ? plan->layers_k_rot[1] >= 0 : plan->layers_k_rot[0] >= 0;
-    const int rc = htree_b200_prepare(shape, lk, lv, bl, plan->blocks_bwd[0] >= 0 ? bb : nullptr, rot ? lr : nullptr, 1, cos_cache,
-                                      sin_cache, stream);
+    const int rc = htree_b200_prepare(shape, lk, lv, bl, plan->blocks_bwd[0] >= 0 ? bb : nullptr, 1, cos_cache, sin_cache, stream);
     if (rc) return rc;
-    return htree_b200_attend(shape, q, lk, lv, rot ? lr : nullptr, bl, cos_cache, sin_cache, table, n_pos, scale, out, gmax, gsum, par,
-                             status, flags, stream);
+    return htree_b200_attend(shape, q, lk, lv, bl, cos_cache, sin_cache, table, table_f32, n_pos, scale, out, gmax, gsum, par, status, flags,
+                             stream);
 }
 
 int htree_b200_block_keys(const HtreeShape* shape, void* const* layers_k_rot, void* const* layers_k_blk, void* stream) {

@@ -59,13 +59,11 @@ __global__ void __launch_bounds__(256) bwd_fill_kernel(const __grid_constant__ B
         if (np <= 0 || (l > 0 && rp + 1 <= TK)) continue;
         const int nblk = (p.ln[l] + CR - 1) / CR;
         const int32_t* base = bp.base + (int64_t)blockIdx.y * bp.NK + bp.koff[l];
-        const int32_t* cnt = bp.cnt + (int64_t)blockIdx.y * bp.NK + bp.koff[l];
         for (int i = lane; i < np; i += 32) {
             int x = load_parent(p, l, qidx * TK + i);
             if ((unsigned)x >= (unsigned)nblk) x = 0;
             const int64_t v = grp * bp.MV + bp.voff[l] + i;
-            const int rank = bp.rank[v];     // written by the first pass, except where that gave up (status 16)
-            if ((unsigned)rank < (unsigned)cnt[x]) entries[base[x] + rank] = make_uint2((uint32_t)v, (uint32_t)grp | ((uint32_t)(rp - CR * i) << 15));
+            entries[base[x] + bp.rank[v]] = make_uint2((uint32_t)v, (uint32_t)grp | ((uint32_t)(rp - CR * i) << 15));
         }
     }
 }
@@ -90,7 +88,7 @@ __global__ void __launch_bounds__(128, dkv_min_blocks<D, X3>()) bwd_dkv_kernel(c
     constexpr int TAB = KEYS ? C::TAB : 0;
     constexpr int SLOT = 2 * QB + 2 * SB + 2 * TAB, NSTG = dkv_stages<D, X3>();
     constexpr int PLANE = NT * 128;                                         // bytes from the hi to the lo words of a record
-    using Ring = ChunkRing<NSTG, SLOT>;
+    using Ring = WarpRing<NSTG, SLOT>;
     extern __shared__ __align__(128) unsigned char smem_raw[];
     const AttnParams& p = bp.a;
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, g = lane >> 2;
@@ -98,7 +96,7 @@ __global__ void __launch_bounds__(128, dkv_min_blocks<D, X3>()) bwd_dkv_kernel(c
     if (it >= bp.nitems[ls]) return;
     const BwdItem item = bp.items[(int64_t)ls * bp.cap + it];
     Ring ring;
-    ring.init(smem_raw + (size_t)warp * Ring::kBytes, lane);
+    ring.init(smem_raw + (size_t)warp * Ring::kBytes);
     const uint2* entries = bp.entries + (int64_t)ls * bp.subq * bp.MV + item.start;
     const unsigned char* qsrc = KEYS ? bp.qb : bp.dob;
     const unsigned char* ssrc = KEYS ? bp.sts : bp.stp;
@@ -113,39 +111,39 @@ __global__ void __launch_bounds__(128, dkv_min_blocks<D, X3>()) bwd_dkv_kernel(c
         for (int n = 0; n < NT; ++n) acc[i][n][0] = acc[i][n][1] = acc[i][n][2] = acc[i][n][3] = 0.f;
 
     uint2 cur = entries[min(lane, len - 1)], nxt = entries[min(32 + lane, len - 1)];
-    auto issue = [&](int s) {
+    auto fill = [&](int s) {                       // operand, record and table row of the step's one or two visits
         const int e0 = s * VPS;
         if (e0 && (e0 & 31) == 0) { cur = nxt; nxt = entries[min(e0 + 32 + lane, len - 1)]; }
-        const int e1 = min(e0 + VPS - 1, len - 1);
-        uint2 a, b;
-        a.x = __shfl_sync(0xffffffffu, cur.x, e0 & 31); a.y = __shfl_sync(0xffffffffu, cur.y, e0 & 31);
-        b.x = a.x; b.y = a.y;
-        if (VPS == 2) { b.x = __shfl_sync(0xffffffffu, cur.x, e1 & 31); b.y = __shfl_sync(0xffffffffu, cur.y, e1 & 31); }
-        if (lane == 0) ring.expect(NH == 2 ? 2 * QB + 2 * SB + TAB : SLOT);
-        __syncwarp();
-        // lanes 0..5 issue one copy each: operand, record and table row of the two halves
-        const uint2 mine = (VPS == 2 && (lane & 1)) ? b : a;
-        const unsigned char* src; uint32_t off, bytes;
-        if (lane < 2) { src = qsrc + (int64_t)(mine.y & 0x7fffu) * (NH * QB); off = lane * QB; bytes = NH * QB; }
-        else if (lane < 4) { src = ssrc + (int64_t)mine.x * (NH * SB); off = 2 * QB + (lane & 1) * SB; bytes = NH * SB; }
-        else { src = tab + (int64_t)(mine.y >> 15) * C::TAB; off = 2 * QB + 2 * SB + (lane & 1) * TAB; bytes = TAB; }
-        if (lane < (KEYS ? 6 : 4) && (VPS == 2 || !(lane & 1))) ring.copy(off, src, bytes);
-        ring.issued();
+        const uint32_t ax = __shfl_sync(0xffffffffu, cur.x, e0 & 31), ay = __shfl_sync(0xffffffffu, cur.y, e0 & 31);
+        ring.template copy<NH * QB>(0, qsrc + (int64_t)(ay & 0x7fffu) * (NH * QB), lane);
+        ring.template copy<NH * SB>(2 * QB, ssrc + (int64_t)ax * (NH * SB), lane);
+        if constexpr (KEYS) ring.template copy<TAB>(2 * QB + 2 * SB, tab + (int64_t)(ay >> 15) * C::TAB, lane);
+        if constexpr (VPS == 2) {
+            const int e1 = min(e0 + 1, len - 1);
+            const uint32_t bx = __shfl_sync(0xffffffffu, cur.x, e1 & 31), by = __shfl_sync(0xffffffffu, cur.y, e1 & 31);
+            ring.template copy<QB>(QB, qsrc + (int64_t)(by & 0x7fffu) * QB, lane);
+            ring.template copy<SB>(2 * QB + SB, ssrc + (int64_t)bx * SB, lane);
+            if constexpr (KEYS) ring.template copy<TAB>(2 * QB + 2 * SB + TAB, tab + (int64_t)(by >> 15) * C::TAB, lane);
+        }
     };
     int next = 0;
 #pragma unroll 1
-    for (; next < NSTG - 1 && next < steps; ++next) issue(next);
+    for (; next < NSTG - 1; ++next) {
+        if (next < steps) fill(next);
+        ring.commit();
+    }
 #pragma unroll 1
     for (int s = 0; s < steps; ++s) {
         __syncwarp();
-        if (next < steps) { issue(next); ++next; }
-        uint32_t slot;
-        if (!ring.wait(slot)) { if (lane == 0 && p.status) atomicOr(p.status, 16); ring.drain(); return; }
+        if (next < steps) fill(next);
+        ring.commit();
+        ++next;
+        const uint32_t slot = ring.wait();
         const bool lone = VPS == 2 && 2 * s + 1 >= len;
         const uint32_t ra = slot + 2 * QB, rb = ra + SB;
         uint32_t bw[NT][2], bl[X3 ? NT : 1][2];
-        auto lds32 = [](uint32_t a) { uint32_t x; asm volatile("ld.shared.b32 %0, [%1];" : "=r"(x) : "r"(a)); return x; };
-        auto lds64 = [](uint32_t a, uint32_t& x, uint32_t& y) { asm volatile("ld.shared.v2.b32 {%0,%1}, [%2];" : "=r"(x), "=r"(y) : "r"(a)); };
+        auto lds32 = [](uint32_t a) { uint32_t x; asm("ld.shared.b32 %0, [%1];" : "=r"(x) : "r"(a)); return x; };
+        auto lds64 = [](uint32_t a, uint32_t& x, uint32_t& y) { asm("ld.shared.v2.b32 {%0,%1}, [%2];" : "=r"(x), "=r"(y) : "r"(a)); };
 #pragma unroll
         for (int pl = 0; pl < (X3 ? 2 : 1); ++pl) {
 #pragma unroll
@@ -180,7 +178,7 @@ __global__ void __launch_bounds__(128, dkv_min_blocks<D, X3>()) bwd_dkv_kernel(c
                         rotate_h2(lb, hb, c0, s0, n0, a[2], a[3]);
                     }
 #pragma unroll
-                    for (int n = 0; n < NT; ++n) F::mma(acc[i][n], a[0], a[1], a[2], a[3], bw[n][0], bw[n][1]);
+                    for (int n = 0; n < NT; ++n) mma_acc<FT>(acc[i][n], a, bw[n][0], bw[n][1]);
                 }
             }
         } else if constexpr (!X3) {
@@ -190,7 +188,7 @@ __global__ void __launch_bounds__(128, dkv_min_blocks<D, X3>()) bwd_dkv_kernel(c
                 lds64(slot + i * 256 + lane * 8, a[0], a[1]);
                 lds64(slot + QB + i * 256 + lane * 8, a[2], a[3]);
 #pragma unroll
-                for (int n = 0; n < NT; ++n) F::mma(acc[i][n], a[0], a[1], a[2], a[3], bw[n][0], bw[n][1]);
+                for (int n = 0; n < NT; ++n) mma_acc<FT>(acc[i][n], a, bw[n][0], bw[n][1]);
             }
         } else {
 #pragma unroll
@@ -219,8 +217,8 @@ __global__ void __launch_bounds__(128, dkv_min_blocks<D, X3>()) bwd_dkv_kernel(c
                 for (int n = 0; n < NT; ++n) {
                     float t[4];
                     mma_zero<__half>(t, al, bw[n][0], bw[n][1]);
-                    F::mma(t, ah[0], ah[1], ah[2], ah[3], bl[X3 ? n : 0][0], bl[X3 ? n : 0][1]);
-                    F::mma(t, ah[0], ah[1], ah[2], ah[3], bw[n][0], bw[n][1]);
+                    mma_acc<FT>(t, ah, bl[X3 ? n : 0][0], bl[X3 ? n : 0][1]);
+                    mma_acc<FT>(t, ah, bw[n][0], bw[n][1]);
 #pragma unroll
                     for (int u = 0; u < 4; ++u) acc[i][n][u] += t[u];
                 }
@@ -307,7 +305,7 @@ template <typename T, int D, bool X3, int NH, int CR, bool KEYS>
 static int launch_dkv_one(const BwdParams& bp, cudaStream_t st) {
     using BF = BForm<D, X3, NH, CR>;
     constexpr int SLOT = 2 * BF::QB + 2 * BF::SB + (KEYS ? 2 * TForm<D, X3, CR>::TAB : 0);
-    using Ring = ChunkRing<dkv_stages<D, X3>(), SLOT>;
+    using Ring = WarpRing<dkv_stages<D, X3>(), SLOT>;
     const size_t smem = 4 * Ring::kBytes;
     auto* k = bwd_dkv_kernel<T, D, X3, NH, CR, KEYS>;
     const cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);

@@ -19,10 +19,10 @@ constexpr int dq_warps() { return D == 128 && !X3 && NH == 2 ? 1 : 4; }
 template <int D, bool X3, int NH>
 constexpr int dq_min_blocks() { return (D == 128 && (X3 || NH == 2)) ? (X3 ? 2 : 12) : (X3 && NH == 2) ? 2 : 3; }
 
-// ring, parent list, kept-candidate bits, two pointers
+// ring, parent list, kept-candidate bits
 template <typename Ring>
 __host__ __device__ inline size_t dq_warp_bytes(int TK, int CR) {
-    return (Ring::kBytes + sizeof(int32_t) * TK + sizeof(uint32_t) * ((TK * CR + 31) / 32) + 16 + 127) & ~size_t(127);
+    return (Ring::kBytes + sizeof(int32_t) * TK + sizeof(uint32_t) * ((TK * CR + 31) / 32) + 127) & ~size_t(127);
 }
 
 template <typename T, int D, bool X3, int NH, int CR>
@@ -34,7 +34,7 @@ __global__ void __launch_bounds__(dq_warps<D, X3, NH>() * 32, dq_min_blocks<D, X
     using FS = Frag<__half>;
     constexpr int KS = C::KS, PPT = C::PPT, PPC = C::PPC, HALF = C::HALF;
     constexpr int NSTG = dq_stages<D, X3>();
-    using Ring = ChunkRing<NSTG, C::SLOT>;
+    using Ring = WarpRing<NSTG, C::SLOT>;
     extern __shared__ __align__(128) unsigned char smem_raw[];
     const AttnParams& p = bp.a;
 
@@ -52,12 +52,9 @@ __global__ void __launch_bounds__(dq_warps<D, X3, NH>() * 32, dq_min_blocks<D, X
     const size_t per_warp = dq_warp_bytes<Ring>(TK, CR);
     unsigned char* wbase = smem_raw + warp * per_warp;
     Ring ring;
-    ring.init(wbase, lane);
+    ring.init(wbase);
     int32_t* par = reinterpret_cast<int32_t*>(wbase + Ring::kBytes);
     uint32_t* selw = reinterpret_cast<uint32_t*>(par + TK);
-    // what only the issuing lane needs, once per chunk, lives in shared memory: this level's key and value blocks
-    const unsigned char* volatile* src = reinterpret_cast<const unsigned char* volatile*>(wbase + per_warp - 16);
-
     const int64_t hbase = ((int64_t)b * p.Tq + tl) * p.H + (int64_t)hk * G;
     const int64_t qidx = ((int64_t)b * p.Tq + tl) * p.Hkv + hk;
 
@@ -113,10 +110,10 @@ __global__ void __launch_bounds__(dq_warps<D, X3, NH>() * 32, dq_min_blocks<D, X
         unsigned char* dst = bp.dob + ((int64_t)grp * NH + h) * BF::QB;
 #pragma unroll
         for (int i = 0; i < KS; ++i) {
-            *reinterpret_cast<uint2*>(dst + i * 256 + lane * 8) = make_uint2(movmatrix_trans(dO[h][0][i]), movmatrix_trans(dO[h][1][i]));
+            *reinterpret_cast<uint2*>(dst + i * 256 + lane * 8) = make_uint2(movm(dO[h][0][i]), movm(dO[h][1][i]));
             if constexpr (X3)
                 *reinterpret_cast<uint2*>(dst + D * 16 + i * 256 + lane * 8) =
-                    make_uint2(movmatrix_trans(dOl[X3 ? h : 0][0][X3 ? i : 0]), movmatrix_trans(dOl[X3 ? h : 0][1][X3 ? i : 0]));
+                    make_uint2(movm(dOl[X3 ? h : 0][0][X3 ? i : 0]), movm(dOl[X3 ? h : 0][1][X3 ? i : 0]));
         }
         unsigned char* qd = bp.qb + ((int64_t)grp * NH + h) * BF::QB;
         if constexpr (X3) {
@@ -129,7 +126,7 @@ __global__ void __launch_bounds__(dq_warps<D, X3, NH>() * 32, dq_min_blocks<D, X
         } else {
 #pragma unroll
             for (int i = 0; i < KS; ++i)
-                *reinterpret_cast<uint2*>(qd + i * 256 + lane * 8) = make_uint2(movmatrix_trans(q.v[h][0][i]), movmatrix_trans(q.v[h][1][i]));
+                *reinterpret_cast<uint2*>(qd + i * 256 + lane * 8) = make_uint2(movm(q.v[h][0][i]), movm(q.v[h][1][i]));
         }
     }
 
@@ -173,48 +170,46 @@ __global__ void __launch_bounds__(dq_warps<D, X3, NH>() * 32, dq_min_blocks<D, X
                 }
             }
         }
-        if (lane == 0) {
-            const int64_t blk0 = (int64_t)b * nblk * p.Hkv + hk;
-            src[0] = reinterpret_cast<const unsigned char*>(p.blk[l]) + blk0 * C::BLOCK;
-            src[1] = reinterpret_cast<const unsigned char*>(p.vkblk[l]) + blk0 * (C::PL * C::PART);
-        }
         __syncwarp();
 
-        auto issue = [&](int c) {
-            if (lane == 0) {
-                constexpr int PB = C::PL * C::PART;
-                ring.expect(C::SLOT);
-                int p0 = par[c * PPC];
-                if ((unsigned)p0 >= (unsigned)nblk) { if (p.status) atomicOr(p.status, 8); p0 = 0; }
-                const int64_t kstride = (int64_t)p.Hkv * C::BLOCK, vstride = (int64_t)p.Hkv * (C::PL * C::PART);
-                const unsigned char *kblk = src[0], *vblk = src[1];
-                ring.copy(0, kblk + p0 * kstride, PB);
-                ring.copy(C::V_OFF, vblk + p0 * vstride, PB);
-                if constexpr (CR == 8) {
-                    int p1 = c * PPC + 1 < np ? par[c * PPC + 1] : p0;
-                    if ((unsigned)p1 >= (unsigned)nblk) { if (p.status) atomicOr(p.status, 8); p1 = 0; }
-                    ring.copy(C::K2_OFF, kblk + p1 * kstride + 2 * C::ODD, PB);
-                    ring.copy(C::V2_OFF, vblk + p1 * vstride, PB);
-                }
-                const unsigned char* tab = reinterpret_cast<const unsigned char*>(p.tab) + (int64_t)(rp - 16 * c) * C::TAB;
-                ring.copy(C::DATA, tab, C::TAB);
-                if constexpr (C::DUAL) ring.copy(C::DATA + C::TAB, rp - 16 * c >= 8 ? tab - 8 * C::TAB : tab, C::TAB);
+        const int64_t blk0 = (int64_t)b * nblk * p.Hkv + hk;
+        const unsigned char* kblk = reinterpret_cast<const unsigned char*>(p.blk[l]) + blk0 * C::BLOCK;
+        const unsigned char* vblk = reinterpret_cast<const unsigned char*>(p.vkblk[l]) + blk0 * (C::PL * C::PART);
+        auto fill = [&](int c) {
+            constexpr int PB = C::PL * C::PART;
+            const int64_t kstride = (int64_t)p.Hkv * C::BLOCK, vstride = (int64_t)p.Hkv * PB;
+            int p0 = par[c * PPC];
+            if ((unsigned)p0 >= (unsigned)nblk) { if (p.status) atomicOr(p.status, 8); p0 = 0; }
+            ring.template copy<PB>(0, kblk + p0 * kstride, lane);
+            ring.template copy<PB>(C::V_OFF, vblk + p0 * vstride, lane);
+            if constexpr (CR == 8) {
+                int p1 = c * PPC + 1 < np ? par[c * PPC + 1] : p0;
+                if ((unsigned)p1 >= (unsigned)nblk) { if (p.status) atomicOr(p.status, 8); p1 = 0; }
+                ring.template copy<PB>(C::K2_OFF, kblk + p1 * kstride + 2 * C::ODD, lane);
+                ring.template copy<PB>(C::V2_OFF, vblk + p1 * vstride, lane);
             }
-            ring.issued();
+            const unsigned char* row = reinterpret_cast<const unsigned char*>(p.tab) + (int64_t)(rp - 16 * c) * C::TAB;
+            ring.template copy<C::TAB>(C::DATA, row, lane);
+            if constexpr (C::DUAL) ring.template copy<C::TAB>(C::DATA + C::TAB, rp - 16 * c >= 8 ? row - 8 * C::TAB : row, lane);
         };
+        ring.start();
         int next = 0;
 #pragma unroll 1
-        for (; next < NSTG - 1 && next < nchunk; ++next) issue(next);
+        for (; next < NSTG - 1; ++next) {
+            if (next < nchunk) fill(next);
+            ring.commit();
+        }
         const int visit0 = grp * bp.MV + bp.voff[l];
 #pragma unroll 1
         for (int c = 0; c < nchunk; ++c) {
             __syncwarp();
-            if (next < nchunk) { issue(next); ++next; }
+            if (next < nchunk) fill(next);
+            ring.commit();
+            ++next;
             uint32_t mask = 0xffffu;
             if (l > 0) mask &= ~(selw[c >> 1] >> ((16 * c) & 31));
             if (16 * c + 15 > rp) mask &= (2u << (rp - 16 * c)) - 1u;
-            uint32_t slot;
-            if (!ring.wait(slot)) { if (lane == 0 && p.status) atomicOr(p.status, 16); ring.drain(); return; }
+            const uint32_t slot = ring.wait();
             const LaneBase<D, X3, CR> lb(slot, lane);
             const uint32_t tabs = slot + C::DATA;
 
@@ -237,10 +232,10 @@ __global__ void __launch_bounds__(dq_warps<D, X3, NH>() * 32, dq_min_blocks<D, X
 #pragma unroll
                     for (int h = 0; h < NH; ++h) {
                         if (ks == 0) mma_zero<FT>(dP[h], a, dO[h][0][0], dO[h][1][0]);
-                        else F::mma(dP[h], a[0], a[1], a[2], a[3], dO[h][0][ks], dO[h][1][ks]);
+                        else mma_acc<FT>(dP[h], a, dO[h][0][ks], dO[h][1][ks]);
                         if constexpr (X3) {
-                            F::mma(dP[h], al[0], al[1], al[2], al[3], dO[h][0][ks], dO[h][1][ks]);
-                            F::mma(dP[h], a[0], a[1], a[2], a[3], dOl[X3 ? h : 0][0][X3 ? ks : 0], dOl[X3 ? h : 0][1][X3 ? ks : 0]);
+                            mma_acc<FT>(dP[h], al, dO[h][0][ks], dO[h][1][ks]);
+                            mma_acc<FT>(dP[h], a, dOl[X3 ? h : 0][0][X3 ? ks : 0], dOl[X3 ? h : 0][1][X3 ? ks : 0]);
                         }
                     }
                 }
@@ -260,12 +255,12 @@ __global__ void __launch_bounds__(dq_warps<D, X3, NH>() * 32, dq_min_blocks<D, X
                     if constexpr (X3) {
                         split_half2(P[0], P[1], pw[h][0], pwl[X3 ? h : 0][0]); split_half2(P[2], P[3], pw[h][1], pwl[X3 ? h : 0][1]);
                         split_half2(dS[0], dS[1], sw[h][0], swl[X3 ? h : 0][0]); split_half2(dS[2], dS[3], sw[h][1], swl[X3 ? h : 0][1]);
-                        dbl[X3 ? h : 0][0] = movmatrix_trans(swl[X3 ? h : 0][0]); dbl[X3 ? h : 0][1] = movmatrix_trans(swl[X3 ? h : 0][1]);
+                        dbl[X3 ? h : 0][0] = movm(swl[X3 ? h : 0][0]); dbl[X3 ? h : 0][1] = movm(swl[X3 ? h : 0][1]);
                     } else {
                         pw[h][0] = F::pack(P[0], P[1]); pw[h][1] = F::pack(P[2], P[3]);
                         sw[h][0] = FS::pack(dS[0], dS[1]); sw[h][1] = FS::pack(dS[2], dS[3]);
                     }
-                    db[h][0] = movmatrix_trans(sw[h][0]); db[h][1] = movmatrix_trans(sw[h][1]);
+                    db[h][0] = movm(sw[h][0]); db[h][1] = movm(sw[h][1]);
                 }
                 // dq^T += K~^T dS^T: transposed key fragments (rows x(ks, g)), rotated back by the chunk's distance
                 if constexpr (!X3) {
@@ -296,7 +291,7 @@ __global__ void __launch_bounds__(dq_warps<D, X3, NH>() * 32, dq_min_blocks<D, X
                                 rotate_h2(m[1], m[3], cc, ns, ss, a[2], a[3]);
                             }
 #pragma unroll
-                            for (int h = 0; h < NH; ++h) FS::mma(dq[h][ks], a[0], a[1], a[2], a[3], db[h][0], db[h][1]);
+                            for (int h = 0; h < NH; ++h) mma_acc<__half>(dq[h][ks], a, db[h][0], db[h][1]);
                         }
                     }
                 } else {
@@ -307,8 +302,8 @@ __global__ void __launch_bounds__(dq_warps<D, X3, NH>() * 32, dq_min_blocks<D, X
                         key_frag_trans<D, X3, CR>(lb, 1, ks, ml);
                         float cs, sn;
                         const uint32_t tb = tabs + 4 * (PPT * (g >> 1) + 2 * ks + (g & 1));
-                        asm volatile("ld.shared.f32 %0, [%1];" : "=f"(cs) : "r"(tb));
-                        asm volatile("ld.shared.f32 %0, [%1];" : "=f"(sn) : "r"(tb + 4 * HALF));
+                        asm("ld.shared.f32 %0, [%1];" : "=f"(cs) : "r"(tb));
+                        asm("ld.shared.f32 %0, [%1];" : "=f"(sn) : "r"(tb + 4 * HALF));
                         float2 x[4];
 #pragma unroll
                         for (int m = 0; m < 4; ++m) {
@@ -327,8 +322,8 @@ __global__ void __launch_bounds__(dq_warps<D, X3, NH>() * 32, dq_min_blocks<D, X
                             // from zero, then a round-to-nearest fp32 add (the tensor core's accumulation truncates)
                             float acc[4];
                             mma_zero<__half>(acc, ah, dbl[X3 ? h : 0][0], dbl[X3 ? h : 0][1]);
-                            FS::mma(acc, al[0], al[1], al[2], al[3], db[h][0], db[h][1]);
-                            FS::mma(acc, ah[0], ah[1], ah[2], ah[3], db[h][0], db[h][1]);
+                            mma_acc<__half>(acc, al, db[h][0], db[h][1]);
+                            mma_acc<__half>(acc, ah, db[h][0], db[h][1]);
 #pragma unroll
                             for (int i = 0; i < 4; ++i) dq[h][ks][i] += acc[i];
                         }
@@ -364,6 +359,7 @@ __global__ void __launch_bounds__(dq_warps<D, X3, NH>() * 32, dq_min_blocks<D, X
         }
     }
 
+    ring.idle();
     // ---- dq through shared memory (the ring is idle), rows written whole: fp32, or rounded once to the storage type ----
     __syncwarp();
     float* sm = reinterpret_cast<float*>(wbase);
@@ -392,7 +388,7 @@ __global__ void __launch_bounds__(dq_warps<D, X3, NH>() * 32, dq_min_blocks<D, X
 template <typename T, int D, bool X3, int NH, int CR>
 static int launch_dq_cr(const BwdParams& bp, cudaStream_t st) {
     using C = TForm<D, X3, CR>;
-    using Ring = ChunkRing<dq_stages<D, X3>(), C::SLOT>;
+    using Ring = WarpRing<dq_stages<D, X3>(), C::SLOT>;
     const int TK = bp.a.TK;
     const size_t per_warp = dq_warp_bytes<Ring>(TK, CR);
     constexpr int max_w = dq_warps<D, X3, NH>(), max_warps = max_w * dq_min_blocks<D, X3, NH>();

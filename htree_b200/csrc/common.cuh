@@ -24,6 +24,7 @@ struct AttnParams {
     const void* blk[HTREE_MAX_LEVELS];   // operand blocks of the transposed kernels (tform.cuh), or NULL
     const void* vkblk[HTREE_MAX_LEVELS]; // their backward part, or NULL
     const void* tab;                     // rotary table of the transposed kernels, rows [cos | sin]: IEEE half times scale, or fp32 (split-half)
+    const void* tab32;                   // fp32 rows [cos | sin] for the selection kernel
     int32_t ln[HTREE_MAX_LEVELS];   // N_l
     int64_t lpow[HTREE_MAX_LEVELS]; // CR^l
     const float* cosc;
@@ -137,7 +138,9 @@ bool pack_supported(int dtype, int K, int V, int CR);
 bool pack_split(int dtype, int D);                       // split-half operands?
 size_t pack_block_bytes(int D, bool x3, int CR);         // bytes of one forward block
 int launch_pack_blocks(const HtreeShape& s, int L, const int32_t* ln, void* const* lk, void* const* lv, void* const* blk,
-                       void* const* vkblk, void* const* krot, bool pool, const float* cosc, const float* sinc, cudaStream_t st);
+                       void* const* vkblk, bool pool, const float* cosc, const float* sinc, cudaStream_t st);
+bool select_blk_supported(const AttnParams& p, int dtype);
+int launch_select_blk(const AttnParams& p, int dtype, cudaStream_t st);
 bool select_mma_supported(const AttnParams& p, int dtype);
 bool acc_mma_supported(const AttnParams& p, int dtype);
 int launch_acc_mma(const AttnParams& p, int dtype, cudaStream_t st);

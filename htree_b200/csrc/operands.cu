@@ -1,7 +1,6 @@
 // Operand preparation of the transposed tensor-core kernels: one warp per (batch, parent, KV head) reads the parent's
 // children once and writes everything that is derived from them: the parent's own pooled row (the next level), the operand
-// blocks of the forward and of the backward (layouts in tform.cuh), and, where wanted, the row-major K' that the selection
-// kernel gathers from.  One launch per level.  HBM / L2 streaming: per 16-bit block of 16 children and 128-wide heads it
+// blocks of the forward and of the backward (layouts in tform.cuh).  One launch per level.  HBM / L2 streaming: per 16-bit block of 16 children and 128-wide heads it
 // reads 8 KB and writes 8.5 KB (12.5 KB with the backward's part); the launches it replaces (pooling, rotation, two blockings
 // per level) read the same rows four times and cost a launch each, which is what short sequences spent their time on.
 #include "tform.cuh"
@@ -13,13 +12,11 @@ struct PackArgs {
     const void* v;
     void* blk;          // forward blocks
     void* vkblk;        // backward: values as A fragments of dP^T, or NULL
-    void* krot;         // row-major K', or NULL
     void* pk;           // pooled rows of the next level, or NULL
     void* pv;
     const float* cosc;
     const float* sinc;
     int64_t total;      // B * NBLK * Hkv
-    int64_t plane;      // split-half K' rows: elements between the planes
     int32_t N, NBLK, Hkv;
 };
 
@@ -119,22 +116,6 @@ __global__ void __launch_bounds__(128) pack_blocks_kernel(const __grid_constant_
         }
         to_half_words<X3, PPT>(x, kw[tl][0], kl[tl][0]);
         to_half_words<X3, PPT>(y, kw[tl][1], kl[tl][1]);
-        if (a.krot && on && (CR == 16 || tl == 0)) {
-            // row-major K' (64-wide rows keep a lane's low and high 8 pairs side by side)
-            __half* kr = reinterpret_cast<__half*>(a.krot) + base + child * rs;
-            const int o0 = D == 64 ? 2 * PPT * r : PPT * r, o1 = D == 64 ? o0 + PPT : HALF + PPT * r;
-            if constexpr (PPT >= 8) {
-#pragma unroll
-                for (int i = 0; i < PPT / 8; ++i) {
-                    *reinterpret_cast<uint4*>(kr + o0 + 8 * i) = make_uint4(kw[tl][0][4 * i], kw[tl][0][4 * i + 1], kw[tl][0][4 * i + 2], kw[tl][0][4 * i + 3]);
-                    *reinterpret_cast<uint4*>(kr + o1 + 8 * i) = make_uint4(kw[tl][1][4 * i], kw[tl][1][4 * i + 1], kw[tl][1][4 * i + 2], kw[tl][1][4 * i + 3]);
-                    if constexpr (X3) {
-                        *reinterpret_cast<uint4*>(kr + a.plane + o0 + 8 * i) = make_uint4(kl[tl][0][4 * i], kl[tl][0][4 * i + 1], kl[tl][0][4 * i + 2], kl[tl][0][4 * i + 3]);
-                        *reinterpret_cast<uint4*>(kr + a.plane + o1 + 8 * i) = make_uint4(kl[tl][1][4 * i], kl[tl][1][4 * i + 1], kl[tl][1][4 * i + 2], kl[tl][1][4 * i + 3]);
-                    }
-                }
-            }
-        }
     }
 #pragma unroll
     for (int pl = 0; pl < C::PL; ++pl) {
@@ -278,17 +259,16 @@ static void launch_pack_d(const PackArgs& a, int D, int CR, cudaStream_t st) {
     else launch_pack_t<T, 32, true>(a, CR, st);
 }
 
-// blk[l] of every level, and, per pointer given, the pooled levels lk[l + 1] / lv[l + 1], the row-major K' krot[l] and vkblk[l].
+// blk[l] of every level, and, where asked for, the pooled levels lk[l + 1] / lv[l + 1] and vkblk[l].
 int launch_pack_blocks(const HtreeShape& s, int L, const int32_t* ln, void* const* lk, void* const* lv, void* const* blk,
-                       void* const* vkblk, void* const* krot, bool pool, const float* cosc, const float* sinc, cudaStream_t st) {
+                       void* const* vkblk, bool pool, const float* cosc, const float* sinc, cudaStream_t st) {
     for (int l = 0; l < L; ++l) {
         PackArgs a;
-        a.k = lk[l]; a.v = lv[l]; a.blk = blk[l]; a.vkblk = vkblk ? vkblk[l] : nullptr; a.krot = krot ? krot[l] : nullptr;
+        a.k = lk[l]; a.v = lv[l]; a.blk = blk[l]; a.vkblk = vkblk ? vkblk[l] : nullptr;
         a.pk = pool && l + 1 < L ? lk[l + 1] : nullptr; a.pv = pool && l + 1 < L ? lv[l + 1] : nullptr;
         a.cosc = cosc; a.sinc = sinc;
         a.N = ln[l]; a.Hkv = s.H_kv; a.NBLK = (ln[l] + s.compression_rate - 1) / s.compression_rate;
         a.total = (int64_t)s.B * a.NBLK * s.H_kv;
-        a.plane = (int64_t)s.B * ln[l] * s.H_kv * s.K;
         switch (s.dtype) {
             case HTREE_F32: launch_pack_d<float>(a, s.K, s.compression_rate, st); break;
             case HTREE_BF16: launch_pack_d<__nv_bfloat16>(a, s.K, s.compression_rate, st); break;

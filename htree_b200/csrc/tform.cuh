@@ -64,17 +64,17 @@ struct LaneBase {
     }
 };
 __device__ __forceinline__ void lds_frag(uint32_t addr, uint32_t (&a)[4]) {
-    asm volatile("ld.shared.v4.b32 {%0,%1,%2,%3}, [%4];\n" : "=r"(a[0]), "=r"(a[1]), "=r"(a[2]), "=r"(a[3]) : "r"(addr));
+    asm("ld.shared.v4.b32 {%0,%1,%2,%3}, [%4];\n" : "=r"(a[0]), "=r"(a[1]), "=r"(a[2]), "=r"(a[3]) : "r"(addr));
 }
 __device__ __forceinline__ void ldmatrix_frag(uint32_t addr, uint32_t (&a)[4]) {
-    asm volatile("ldmatrix.sync.aligned.m8n8.x4.shared.b16 {%0,%1,%2,%3}, [%4];\n" : "=r"(a[0]), "=r"(a[1]), "=r"(a[2]), "=r"(a[3]) : "r"(addr));
+    asm("ldmatrix.sync.aligned.m8n8.x4.shared.b16 {%0,%1,%2,%3}, [%4];\n" : "=r"(a[0]), "=r"(a[1]), "=r"(a[2]), "=r"(a[3]) : "r"(addr));
 }
 __device__ __forceinline__ void ldmatrix_trans_frag(uint32_t addr, uint32_t (&a)[4]) {
-    asm volatile("ldmatrix.sync.aligned.m8n8.x4.trans.shared.b16 {%0,%1,%2,%3}, [%4];\n" : "=r"(a[0]), "=r"(a[1]), "=r"(a[2]), "=r"(a[3]) : "r"(addr));
+    asm("ldmatrix.sync.aligned.m8n8.x4.trans.shared.b16 {%0,%1,%2,%3}, [%4];\n" : "=r"(a[0]), "=r"(a[1]), "=r"(a[2]), "=r"(a[3]) : "r"(addr));
 }
 __device__ __forceinline__ uint4 lds_u4(uint32_t addr) {
     uint4 x;
-    asm volatile("ld.shared.v4.b32 {%0,%1,%2,%3}, [%4];\n" : "=r"(x.x), "=r"(x.y), "=r"(x.z), "=r"(x.w) : "r"(addr));
+    asm("ld.shared.v4.b32 {%0,%1,%2,%3}, [%4];\n" : "=r"(x.x), "=r"(x.y), "=r"(x.z), "=r"(x.w) : "r"(addr));
     return x;
 }
 // A fragments of k-step ks of the key part (plane pl)
@@ -101,15 +101,33 @@ __device__ __forceinline__ void value_frag(const LaneBase<D, X3, CR>& s, int pl,
     if constexpr (CR == 16) lds_frag(s.v + pl * C::PART + i * 512, a);
     else ldmatrix_frag(s.v + pl * C::PART + i * 256, a);
 }
+// The loads from a slot and the products below are not volatile, so that the compiler may overlap one step's loads and
+// rotations with another's products; what orders the loads after the slot's wait is the slot address, which comes out of it.
+template <typename T> __device__ __forceinline__ void mma_acc(float (&c)[4], const uint32_t (&a)[4], uint32_t b0, uint32_t b1);
+template <> __device__ __forceinline__ void mma_acc<__half>(float (&c)[4], const uint32_t (&a)[4], uint32_t b0, uint32_t b1) {
+    asm("mma.sync.aligned.m16n8k16.row.col.f32.f16.f16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};\n"
+        : "+f"(c[0]), "+f"(c[1]), "+f"(c[2]), "+f"(c[3])
+        : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1));
+}
+template <> __device__ __forceinline__ void mma_acc<__nv_bfloat16>(float (&c)[4], const uint32_t (&a)[4], uint32_t b0, uint32_t b1) {
+    asm("mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};\n"
+        : "+f"(c[0]), "+f"(c[1]), "+f"(c[2]), "+f"(c[3])
+        : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1));
+}
+__device__ __forceinline__ uint32_t movm(uint32_t a) {
+    uint32_t d;
+    asm("movmatrix.sync.aligned.m8n8.trans.b16 %0, %1;\n" : "=r"(d) : "r"(a));
+    return d;
+}
 // d = A B with a zero accumulator (no registers to clear)
 template <typename T> __device__ __forceinline__ void mma_zero(float (&c)[4], const uint32_t (&a)[4], uint32_t b0, uint32_t b1);
 template <> __device__ __forceinline__ void mma_zero<__half>(float (&c)[4], const uint32_t (&a)[4], uint32_t b0, uint32_t b1) {
-    asm volatile("mma.sync.aligned.m16n8k16.row.col.f32.f16.f16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%10,%10,%10,%10};\n"
+    asm("mma.sync.aligned.m16n8k16.row.col.f32.f16.f16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%10,%10,%10,%10};\n"
                  : "=f"(c[0]), "=f"(c[1]), "=f"(c[2]), "=f"(c[3])
                  : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1), "f"(0.f));
 }
 template <> __device__ __forceinline__ void mma_zero<__nv_bfloat16>(float (&c)[4], const uint32_t (&a)[4], uint32_t b0, uint32_t b1) {
-    asm volatile("mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%10,%10,%10,%10};\n"
+    asm("mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%10,%10,%10,%10};\n"
                  : "=f"(c[0]), "=f"(c[1]), "=f"(c[2]), "=f"(c[3])
                  : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1), "f"(0.f));
 }
@@ -204,11 +222,11 @@ __device__ __forceinline__ void score16(const LaneBase<D, false, CR>& s, uint32_
                 rotate_h2(q.v[h][0][ks], q.v[h][1][ks], c[u], sn[u], ns, b0, b1);
                 float (&acc)[4] = TWO && (ks & 1) ? U[TWO ? h : 0] : S[h];
                 if (ks < (TWO ? 2 : 1)) mma_zero<__half>(acc, a, b0, b1);
-                else FS::mma(acc, a[0], a[1], a[2], a[3], b0, b1);
+                else mma_acc<__half>(acc, a, b0, b1);
                 if constexpr (DUAL) {
                     rotate_h2(q.v[h][0][ks], q.v[h][1][ks], c2[u], sn2[u], neg_h2(sn2[u]), b0, b1);
                     if (ks == 0) mma_zero<__half>(U[DUAL ? h : 0], a, b0, b1);
-                    else FS::mma(U[DUAL ? h : 0], a[0], a[1], a[2], a[3], b0, b1);
+                    else mma_acc<__half>(U[DUAL ? h : 0], a, b0, b1);
                 }
             }
         }
@@ -260,8 +278,8 @@ __device__ __forceinline__ void score_x3(const LaneBase<D, true, CR>& s, uint32_
                 } else {
                     float t[4];
                     mma_zero<__half>(t, ah, b0h, b1h);
-                    FS::mma(B[h], al[0], al[1], al[2], al[3], b0h, b1h);
-                    FS::mma(C[h], ah[0], ah[1], ah[2], ah[3], b0l, b1l);
+                    mma_acc<__half>(B[h], al, b0h, b1h);
+                    mma_acc<__half>(C[h], ah, b0l, b1l);
 #pragma unroll
                     for (int i = 0; i < 4; ++i) S[h][i] += t[i];
                 }
@@ -280,56 +298,46 @@ __device__ __forceinline__ void score_t(const LaneBase<D, X3, CR>& s, uint32_t t
     else score16<T, D, NH, CR>(s, tab, r, q, S);
 }
 
-// One warp's ring of chunk slots in shared memory, filled by bulk copies the warp issues itself.  Waits are bounded; after
-// one ran out the caller flags status bit 16 and leaves through drain().
+// One warp's ring of chunk slots in shared memory, filled NSTG - 1 chunks ahead by 16-byte asynchronous copies of all lanes
+// (cp.async): one instruction per 512 bytes, no barrier object and no single-lane section.  With one bulk copy per operand,
+// issued by one lane and completing on an mbarrier, the single-lane section (addresses into uniform registers, barrier
+// arithmetic) cost 14 % of the selection kernel.
 template <int NSTG, int SLOT>
-struct ChunkRing {
-    uint32_t base;                 // 32-bit shared address: NSTG * SLOT bytes, then NSTG barriers
-    uint32_t is = 0, cs = 0;       // stage the next issue / the next wait uses
-    uint32_t parity = 0;           // phase parity of the next wait
-    uint32_t flying = 0;
-    static constexpr size_t kBytes = (size_t)NSTG * SLOT + 128;
-    static constexpr int kWaitCap = 1 << 16;
+struct WarpRing {
+    uint32_t base;                 // 32-bit shared address of NSTG * SLOT bytes
+    uint32_t is = 0, cs = 0;       // stage the next fill / the next use takes
+    static constexpr size_t kBytes = ((size_t)NSTG * SLOT + 127) & ~size_t(127);
 
-    __device__ __forceinline__ void init(unsigned char* b, int lane) {
-        base = smem_u32(b);
-        if (lane == 0) {
-            for (int i = 0; i < NSTG; ++i) mbar_init(reinterpret_cast<uint64_t*>(b + (size_t)NSTG * SLOT) + i, 1);
-            fence_barrier_init();
+    __device__ __forceinline__ void init(unsigned char* b) { base = smem_u32(b); }
+    __device__ __forceinline__ void start() { is = cs = 0; }       // before the first fill of a walk; nothing is in flight
+    // BYTES (a multiple of 16) from `src` to offset OFF of the stage being filled
+    template <int BYTES>
+    __device__ __forceinline__ void copy(uint32_t off, const void* src, int lane) const {
+        const uint32_t dst = base + is * SLOT + off + 16 * lane;
+        const unsigned char* s = static_cast<const unsigned char*>(src) + 16 * lane;
+#pragma unroll
+        for (int i = 0; i < BYTES / 512; ++i)
+            asm volatile("cp.async.cg.shared.global [%0], [%1], 16;\n" ::"r"(dst + 512 * i), "l"(s + 512 * i) : "memory");
+        if constexpr (BYTES % 512 != 0) {
+            if (lane < (BYTES % 512) / 16)
+                asm volatile("cp.async.cg.shared.global [%0], [%1], 16;\n" ::"r"(dst + BYTES / 512 * 512), "l"(s + BYTES / 512 * 512) : "memory");
         }
+    }
+    // closes one fill (an empty one where nothing is left to fetch: fills and uses are counted alike)
+    __device__ __forceinline__ void commit() {
+        asm volatile("cp.async.commit_group;\n" ::: "memory");
+        is = is + 1 == NSTG ? 0 : is + 1;
+    }
+    // the oldest fill, complete and visible to every lane
+    __device__ __forceinline__ uint32_t wait() {
+        asm volatile("cp.async.wait_group %0;\n" ::"n"(NSTG - 1) : "memory");
         __syncwarp();
+        uint32_t slot = base + cs * SLOT;
+        asm volatile("" : "+r"(slot)::"memory");
+        cs = cs + 1 == NSTG ? 0 : cs + 1;
+        return slot;
     }
-    __device__ __forceinline__ uint32_t bar(uint32_t stage) const { return base + NSTG * SLOT + 8 * stage; }
-    __device__ __forceinline__ void expect(uint32_t bytes) const {
-        asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;\n" ::"r"(bar(is)), "r"(bytes) : "memory");
-    }
-    __device__ __forceinline__ void copy(uint32_t off, const void* src, uint32_t bytes) const {
-        asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];\n" ::"r"(base + is * SLOT + off),
-                     "l"(src), "r"(bytes), "r"(bar(is))
-                     : "memory");
-    }
-    __device__ __forceinline__ void issued() { is = is + 1 == NSTG ? 0 : is + 1; ++flying; }
-    __device__ __forceinline__ bool wait_stage(uint32_t stage, uint32_t par) const {
-        for (int it = 0; it < kWaitCap; ++it) {
-            uint32_t ok;
-            asm volatile("{\n.reg .pred p;\nmbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\nselp.u32 %0, 1, 0, p;\n}\n"
-                         : "=r"(ok) : "r"(bar(stage)), "r"(par) : "memory");
-            if (ok) return true;
-        }
-        return false;
-    }
-    // waits for the oldest chunk; its slot is `slot` until the next issue after the next __syncwarp
-    __device__ __forceinline__ bool wait(uint32_t& slot) {
-        slot = base + cs * SLOT;
-        const bool ok = wait_stage(cs, parity);
-        if (++cs == NSTG) { cs = 0; parity ^= 1; }
-        --flying;
-        return ok;
-    }
-    __device__ __forceinline__ void drain() {
-        uint32_t slot;
-        while (flying) wait(slot);
-    }
+    __device__ __forceinline__ void idle() const { asm volatile("cp.async.wait_all;\n" ::: "memory"); }
 };
 
 }  // namespace htree

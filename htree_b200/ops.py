@@ -134,6 +134,19 @@ def rope_rows(k_dim: int, cache_size: int, rope_base: float, scale: Optional[flo
     return hit
 
 
+def rope_rows_select(k_dim: int, cache_size: int, rope_base: float, device) -> torch.Tensor:
+    """The rotary table of the selection kernel: fp32 rows [cos | sin | -sin], each part ordered [k-step pair][r][4] over the pairs
+    (k_dim/8)*r + 4*(k-step pair) + {0..3} that lane r of a quad rotates."""
+    key = (k_dim, cache_size, rope_base, "select", device)
+    hit = _rope_rows.get(key)
+    if hit is None:
+        c, s = rope_cache(k_dim, cache_size, rope_base, device)
+        perm = torch.arange(k_dim // 2).view(4, -1, 4).transpose(0, 1).reshape(-1).to(device)
+        hit = torch.cat([c[:, perm], s[:, perm], -s[:, perm]], dim=1).contiguous()
+        _rope_rows[key] = hit
+    return hit
+
+
 def _status(device) -> torch.Tensor:
     device = torch.device(device)
     w = _status_words.get(device)
@@ -302,11 +315,6 @@ class _Workspace:
     def layers_v(self):
         return self._levels(self.plan.layers_v, self.v, self.v.shape[3], self.v.dtype)
 
-    def layers_k_rot(self):
-        if not _selects_on_tensor_cores(self.k.dtype, self.k.shape[3]):
-            return None
-        return self._levels(self.plan.layers_k_rot, None, self.k.shape[3], torch.float16, (2,) if self.k.dtype == torch.float32 else ())
-
     def blocks(self):
         L, p = self.plan.levels, self.plan
         ends = [self._block_bytes(l) for l in range(L)]
@@ -329,9 +337,13 @@ class BwdContext(dict):
 
     def __missing__(self, key):
         if key == "rope_half":
-            ws = self.workspace
-            ok = ws is not None and _selects_on_tensor_cores(ws.k.dtype, ws.k.shape[3])
-            val = rope_cache_half(ws.k.shape[3], self["cos_cache"].shape[0], self["rope_base"], self["scale"], ws.k.device) if ok else None
+            k = self.workspace.k if self.workspace is not None else (self["layers_k"] or [None])[0]
+            ok = k is not None and _selects_on_tensor_cores(k.dtype, k.shape[3])
+            val = rope_cache_half(k.shape[3], self["cos_cache"].shape[0], self["rope_base"], self["scale"], k.device) if ok else None
+        elif key == "layers_k_rot":      # the row-major K' that the one-kernel forms read; the transposed kernels do not
+            lk = self["layers_k"]
+            ok = lk is not None and _selects_on_tensor_cores(lk[0].dtype, lk[0].shape[3])
+            val = rotate_keys(lk, self["compression_rate"], self["max_top_nodes"], self["rope_base"]) if ok else None
         elif key in self._LAZY and self.workspace is not None:
             val = self.workspace.blocks() if key == "layers_v_blk" else getattr(self.workspace, key)()
         else:
@@ -352,12 +364,12 @@ class BwdContext(dict):
         """Forget everything derived from k and v (a backward then rebuilds it)."""
         self.workspace = None
         for key in ("layers_k", "layers_v", "layers_k_rot", "layers_v_blk"):
-            self[key] = None
+            dict.__setitem__(self, key, None)
 
 
 def build_operands(k: torch.Tensor, v: torch.Tensor, compression_rate: int, max_top_nodes: int, rope_base: float,
                    layers=None, backward: bool = False):
-    """(layers_k, layers_v, layers_k_rot, OperandBlocks) in the form the transposed tensor-core kernels read, for a forward with
+    """(layers_k, layers_v, None, OperandBlocks) in the form the transposed tensor-core kernels read, for a forward with
     `_layers`; from k, v alone, or from existing levels `layers` = (layers_k, layers_v).  None in the last two places for
     shapes without such kernels."""
     k = k.contiguous(); v = v.contiguous()
@@ -377,13 +389,12 @@ def build_operands(k: torch.Tensor, v: torch.Tensor, compression_rate: int, max_
     n_blk = lambda l, bwd: int(_lib.lib().htree_b200_operand_block_bytes(ctypes.byref(shape), l, bwd))
     blocks = [torch.empty(n_blk(l, 0), dtype=torch.uint8, device=dev) for l in range(len(sizes))]
     bwd = [torch.empty(n_blk(l, 1), dtype=torch.uint8, device=dev) for l in range(len(sizes))] if backward else None
-    lkr = [_rotated_like(x) if l or backward else None for l, x in enumerate(lk)] if _selects_on_tensor_cores(k.dtype, K) else None
     cos_c, sin_c = rope_cache(K, 16, rope_base, dev)
     with torch.cuda.device(dev):
         _lib.check(_lib.lib().htree_b200_prepare(ctypes.byref(shape), _ptrs(lk), _ptrs(lv), _ptrs(blocks), _ptrs(bwd) if bwd else None,
-                                                 _ptrs(lkr) if lkr else None, int(layers is None), cos_c.data_ptr(), sin_c.data_ptr(),
+                                                 int(layers is None), cos_c.data_ptr(), sin_c.data_ptr(),
                                                  _stream()), "prepare")
-    return lk, lv, lkr, OperandBlocks(blocks, keys=blocks, blocks=blocks, blocks_bwd=bwd)
+    return lk, lv, None, OperandBlocks(blocks, keys=blocks, blocks=blocks, blocks_bwd=bwd)
 
 
 def _pipelined(dtype, K: int, compression_rate: int) -> bool:
@@ -573,6 +584,7 @@ def _forward_transposed(shape, q, k, v, scale, rope_base, save, save_parents, gi
     dev, dtype = q.device, q.dtype
     n_pos = TK * CR + 1024
     cos_cache, sin_cache = rope_cache(K, n_pos, rope_base, dev)
+    table32 = rope_rows_select(K, n_pos, rope_base, dev)
     table = rope_rows(K, n_pos, rope_base, None if _split(dtype, K) else scale, dev)
     keep = save and save_parents
     # Callers that do not keep the selections get them only as temporaries (int32 whatever SELECTION_STORAGE says), and only up
@@ -584,7 +596,7 @@ def _forward_transposed(shape, q, k, v, scale, rope_base, save, save_parents, gi
     per_query = L * H_kv * TK * 4
     if not keep and (windows or B * Tq * per_query > SPLIT_FORWARD_MAX_BYTES):
         layers = _operand_layers(k, v, shape, rope_base, given_layers, save)
-        _forward_windows(shape, q, layers, cos_cache, sin_cache, table, scale, out, stats[0], stats[1], per_query)
+        _forward_windows(shape, q, layers, cos_cache, sin_cache, (table, table32), scale, out, stats[0], stats[1], per_query)
         parents = ws = None
     else:
         pdt = torch.int32
@@ -601,13 +613,13 @@ def _forward_transposed(shape, q, k, v, scale, rope_base, save, save_parents, gi
                 ws = torch.empty(plan.bytes, dtype=torch.uint8, device=dev)
                 rc = _lib.lib().htree_b200_run_forward(
                     ctypes.byref(shape), ctypes.byref(plan), q.data_ptr(), k.data_ptr(), v.data_ptr(), cos_cache.data_ptr(),
-                    sin_cache.data_ptr(), table.data_ptr(), n_pos, scale, ws.data_ptr(), out.data_ptr(), gmax_ptr, gsum_ptr, pptr,
+                    sin_cache.data_ptr(), table.data_ptr(), table32.data_ptr(), n_pos, scale, ws.data_ptr(), out.data_ptr(), gmax_ptr, gsum_ptr, pptr,
                     _status(dev).data_ptr(), flags, _stream())
                 layers = None
             else:
                 ws = None
                 layers = _operand_layers(k, v, shape, rope_base, given_layers, save)
-                rc = _attend(shape, q, layers, cos_cache, sin_cache, table, scale, out.data_ptr(), gmax_ptr, gsum_ptr, pptr, flags)
+                rc = _attend(shape, q, layers, cos_cache, sin_cache, (table, table32), scale, out.data_ptr(), gmax_ptr, gsum_ptr, pptr, flags)
         _lib.check(rc, "forward")
     if not save:
         return out
@@ -616,8 +628,7 @@ def _forward_transposed(shape, q, k, v, scale, rope_base, save, save_parents, gi
     if ws is not None:
         ctx.workspace = _Workspace(ws, plan, k, v, CR)
     else:
-        ctx.update(layers_k=layers[0], layers_v=layers[1], layers_k_rot=layers[2], layers_v_blk=layers[3])
-        ctx["rope_half"] = rope_cache_half(K, n_pos, rope_base, scale, dev) if _selects_on_tensor_cores(dtype, K) else None
+        ctx.update(layers_k=layers[0], layers_v=layers[1], layers_v_blk=layers[3])
     return out, ctx
 
 
@@ -640,14 +651,14 @@ def _operand_layers(k, v, shape, rope_base, given, backward):
     return build_operands(given[0][0], given[1][0], shape.compression_rate, shape.max_top_nodes, rope_base, layers=given, backward=backward)
 
 
-def _attend(shape, q, layers, cos_cache, sin_cache, table, scale, out_ptr, gmax_ptr, gsum_ptr, pptr, flags) -> int:
+def _attend(shape, q, layers, cos_cache, sin_cache, tables, scale, out_ptr, gmax_ptr, gsum_ptr, pptr, flags) -> int:
     return _lib.lib().htree_b200_attend(
-        ctypes.byref(shape), q.data_ptr(), _ptrs(layers[0]), _ptrs(layers[1]), _ptrs(layers[2]) if layers[2] is not None else None,
-        _ptrs(layers[3].blocks), cos_cache.data_ptr(), sin_cache.data_ptr(), table.data_ptr(), cos_cache.shape[0], float(scale),
+        ctypes.byref(shape), q.data_ptr(), _ptrs(layers[0]), _ptrs(layers[1]), _ptrs(layers[3].blocks),
+        cos_cache.data_ptr(), sin_cache.data_ptr(), tables[0].data_ptr(), tables[1].data_ptr(), cos_cache.shape[0], float(scale),
         out_ptr, gmax_ptr, gsum_ptr, pptr, _status(q.device).data_ptr(), flags, _stream())
 
 
-def _forward_windows(shape, q, layers, cos_cache, sin_cache, table, scale, out, gmax, gsum, per_query):
+def _forward_windows(shape, q, layers, cos_cache, sin_cache, tables, scale, out, gmax, gsum, per_query):
     """The forward over windows of query positions, one batch element at a time, whose selections fit
     SPLIT_FORWARD_MAX_BYTES."""
     B, Tq, H, K = q.shape
@@ -658,22 +669,20 @@ def _forward_windows(shape, q, layers, cos_cache, sin_cache, table, scale, out, 
     t_offset = shape.t_offset
     with torch.cuda.device(q.device):
         for b in range(B):
-            one = [[x[b:b + 1] for x in layers[0]], [x[b:b + 1] for x in layers[1]],
-                   [None if x is None else (x[:, b:b + 1] if x.dim() == 5 else x[b:b + 1]) for x in layers[2]] if layers[2] is not None else None]
             blocks = OperandBlocks([])
             blocks.blocks = [x.view(B, -1)[b] for x in layers[3].blocks]
-            if one[2] is not None and q.dtype == torch.float32 and B > 1:      # the hi and lo planes of one element
-                one[2] = [None if x is None else x.contiguous() for x in one[2]]
+            one = [[x[b:b + 1] for x in layers[0]], [x[b:b + 1] for x in layers[1]], None, blocks]
             for a in range(0, Tq, step):
                 n = min(step, Tq - a)
                 w = _lib.HtreeShape(1, shape.T, shape.H, shape.H_kv, shape.K, shape.V, shape.compression_rate, shape.top_k,
                                     shape.max_top_nodes, shape.dtype, n, t_offset + a)
-                _lib.check(_attend(w, q[b:b + 1, a:a + n], one + [blocks], cos_cache, sin_cache, table, scale, out[b, a:].data_ptr(),
+                _lib.check(_attend(w, q[b:b + 1, a:a + n], one, cos_cache, sin_cache, tables, scale, out[b, a:].data_ptr(),
                                    gmax[b, a:].data_ptr(), gsum[b, a:].data_ptr(), pptr, 0), "forward")
 
 
 def recompute_parents(q, layers_k, layers_v, cos_cache, sin_cache, compression_rate, top_k_per_layer,
-                      max_top_nodes, scale, layers_k_rot=None, _force_generic=False, layers_v_blk=None) -> Dict[int, torch.Tensor]:
+                      max_top_nodes, scale, layers_k_rot=None, _force_generic=False, layers_v_blk=None,
+                      rope_base: Optional[float] = None) -> Dict[int, torch.Tensor]:
     """Selection-only replay of the forward (the reference's _recompute_parents, src/backward.py:881-934)."""
     B, T, H, K = q.shape
     H_kv, V = layers_k[0].shape[2], layers_v[0].shape[-1]
@@ -682,6 +691,13 @@ def recompute_parents(q, layers_k, layers_v, cos_cache, sin_cache, compression_r
     L = len(layers_k)
     parents = [torch.empty(B, T, H_kv, top_k_per_layer, dtype=_parents_dtype(layers_k, top_k_per_layer), device=q.device)
                for _ in range(L)]
+    if rope_base is not None and getattr(layers_v_blk, "blocks", None) is not None and not _force_generic and q.is_contiguous() and q.data_ptr() % 32 == 0:
+        rows = rope_rows_select(K, cos_cache.shape[0], rope_base, q.device)
+        tables = (rows, rows)                            # the selection reads the second only
+        with torch.cuda.device(q.device):
+            _lib.check(_attend(shape, q, (layers_k, layers_v, None, layers_v_blk), cos_cache, sin_cache, tables, scale, None, None, None,
+                               _ptrs(parents), _lib.FWD_SELECT_ONLY | _parents_flag(parents)), "select")
+        return {l: parents[l] for l in range(L)}
     _run_forward(shape, q.contiguous(), layers_k, layers_v, cos_cache, sin_cache, scale, None, None, None, parents,
                  None, _lib.FWD_SELECT_ONLY | (_lib.FWD_GENERIC if _force_generic else 0) | _parents_flag(parents),
                  layers_k_rot, None, layers_v_blk)
@@ -734,7 +750,7 @@ def _backward_two_pass(dO, q, output, ctx, operands, typed, window):
     parents = ctx.get("per_layer_parents")
     if parents is None:
         parents = recompute_parents(q, ctx["layers_k"], ctx["layers_v"], ctx["cos_cache"], ctx["sin_cache"], CR, TK, MTN, ctx["scale"],
-                                    ctx.get("layers_k_rot"))
+                                    layers_v_blk=ctx["layers_v_blk"], rope_base=ctx["rope_base"])
     n_pos = ctx["cos_cache"].shape[0]
     table = rope_rows(K, n_pos, ctx["rope_base"], None if _split(dtype, K) else ctx["scale"], dev)
     if window is None:

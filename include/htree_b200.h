@@ -188,24 +188,22 @@ int htree_b200_forward(const HtreeShape* shape, const void* q, void* const* laye
  *   layers_k[l+1], layers_v[l+1]  the pooled levels (with `pool` != 0; else they are inputs that exist already)
  *   blocks[l]      operand blocks of the forward, htree_b200_operand_block_bytes(shape, l, 0) bytes, 16-byte aligned
  *   blocks_bwd     NULL, or L pointers to the backward's part, htree_b200_operand_block_bytes(shape, l, 1) bytes
- *   layers_k_rot   NULL, or L pointers (each may be NULL) that receive K' rows as htree_b200_rotate_keys writes them
- * htree_b200_attend then selects (with layers_k_rot of the pooled levels: the tensor-core selection kernel; without, or for
- * shapes that has no form of, the fp32-arithmetic kernel on layers_k) and accumulates.
+ * htree_b200_attend then selects (on the tensor cores for K = 64 and for 16-bit K = 128, else with fp32 arithmetic on layers_k) and
+ * accumulates; with HTREE_FWD_SELECT_ONLY it stops after the selection (out, gmax, gsum may be NULL).
  *   table          [n_pos, K] rows [cos(K/2) | sin(K/2)]: fp32 for fp32 storage and for K = 32, else IEEE half multiplied by scale
+ *   table_f32      [n_pos, 3K/2] fp32 rows [cos | sin | -sin], each part ordered [i][r][4] over the pairs (K/8)*r + 4*i + {0..3}
  *   parents        L pointers, written by the selection and read by the accumulation (required)
  *   q              32-byte aligned */
 int64_t htree_b200_operand_block_bytes(const HtreeShape* shape, int32_t level, int32_t backward);
 int htree_b200_prepare(const HtreeShape* shape, void* const* layers_k, void* const* layers_v, void* const* blocks,
-                       void* const* blocks_bwd, void* const* layers_k_rot, int32_t pool, const float* cos_cache,
-                       const float* sin_cache, void* stream);
-int htree_b200_attend(const HtreeShape* shape, const void* q, void* const* layers_k, void* const* layers_v, void* const* layers_k_rot,
-                      void* const* blocks, const float* cos_cache, const float* sin_cache, const void* table, int32_t n_pos,
-                      float scale, void* out, float* gmax, float* gsum, int32_t* const* parents, int32_t* status, uint32_t flags,
-                      void* stream);
+                       void* const* blocks_bwd, int32_t pool, const float* cos_cache, const float* sin_cache, void* stream);
+int htree_b200_attend(const HtreeShape* shape, const void* q, void* const* layers_k, void* const* layers_v, void* const* blocks,
+                      const float* cos_cache, const float* sin_cache, const void* table, const void* table_f32, int32_t n_pos, float scale,
+                      void* out, float* gmax, float* gsum, int32_t* const* parents, int32_t* status, uint32_t flags, void* stream);
 
 /* Both calls as one, for callers that keep a workspace: htree_b200_plan lays out everything a forward derives from its inputs
  * in one buffer of plan->bytes bytes (offsets; -1 = not part of it), htree_b200_run_forward fills it and runs the forward.
- * HTREE_PLAN_BACKWARD adds what a backward reads (blocks_bwd, K' of the leaves), HTREE_PLAN_PARENTS buffers for the
+ * HTREE_PLAN_BACKWARD adds what a backward reads (blocks_bwd), HTREE_PLAN_PARENTS buffers for the
  * selections (int32) for callers that do not pass their own. */
 #define HTREE_PLAN_BACKWARD 1u
 #define HTREE_PLAN_PARENTS 2u
@@ -213,7 +211,6 @@ typedef struct HtreePlan {
     int64_t bytes;
     int64_t layers_k[HTREE_MAX_LEVELS];      /* level 0: -1 (the inputs) */
     int64_t layers_v[HTREE_MAX_LEVELS];
-    int64_t layers_k_rot[HTREE_MAX_LEVELS];
     int64_t blocks[HTREE_MAX_LEVELS];
     int64_t blocks_bwd[HTREE_MAX_LEVELS];
     int64_t parents[HTREE_MAX_LEVELS];
@@ -223,8 +220,8 @@ typedef struct HtreePlan {
 } HtreePlan;
 int htree_b200_plan(const HtreeShape* shape, uint32_t flags, HtreePlan* plan);
 int htree_b200_run_forward(const HtreeShape* shape, const HtreePlan* plan, const void* q, const void* k, const void* v,
-                           const float* cos_cache, const float* sin_cache, const void* table, int32_t n_pos, float scale,
-                           void* workspace, void* out, float* gmax, float* gsum, int32_t* const* parents, int32_t* status,
+                           const float* cos_cache, const float* sin_cache, const void* table, const void* table_f32, int32_t n_pos,
+                           float scale, void* workspace, void* out, float* gmax, float* gsum, int32_t* const* parents, int32_t* status,
                            uint32_t flags, void* stream);
 
 /* One tree level at a time (the call surface the reference's parity harness uses, correctness_test.py:168-347):

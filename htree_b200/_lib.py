@@ -172,4 +172,9 @@ def level_sizes(T: int, compression_rate: int, max_top_nodes: int):
 
 def ptr_array(ptrs):
     """A C array of void* from a list of integer addresses (None -> NULL)."""
-    return (ctypes.c_void_p * len(ptrs))(*[ctypes.c_void_p(p) if p else None for p in ptrs])
+    return (ctypes.c_void_p * len(ptrs))(*ptrs)
+
+
+def address_array(first: int, step: int, n: int):
+    """A C array of the n addresses first, first + step, ..."""
+    return (ctypes.c_void_p * n)(*range(first, first + step * n, step)) if step else ptr_array([first] * n)

@@ -318,7 +318,8 @@ static int launch_acc_cr(const AttnParams& p, cudaStream_t st) {
     const size_t split_smem = 8 * per_warp + 8 * 48 * sizeof(float);
     if ((p.flags & kFlagSplitOk) && groups <= 2 * 148 && split_smem <= limit) {
         auto* k = acc_mma_kernel<T, D, X3, NH, CR, true>;
-        const cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)split_smem);
+        static SmemLimit shared;
+        const cudaError_t e = shared.raise((const void*)k, split_smem);
         if (e != cudaSuccess) return (int)e;
         k<<<dim3(p.Tq, p.B * p.Hkv), 256, split_smem, st>>>(p);
         note_launch();
@@ -335,7 +336,8 @@ static int launch_acc_cr(const AttnParams& p, cudaStream_t st) {
     }
     if (best == 0 || W * per_warp > limit) return HTREE_E_UNSUPPORTED;
     auto* k = acc_mma_kernel<T, D, X3, NH, CR, false>;
-    const cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)(W * per_warp));
+    static SmemLimit shared;
+        const cudaError_t e = shared.raise((const void*)k, W * per_warp);
     if (e != cudaSuccess) return (int)e;
     k<<<dim3((p.Tq + W - 1) / W, p.B * p.Hkv), W * 32, W * per_warp, st>>>(p);
     note_launch();

@@ -308,7 +308,8 @@ static int launch_dkv_one(const BwdParams& bp, cudaStream_t st) {
     using Ring = WarpRing<dkv_stages<D, X3>(), SLOT>;
     const size_t smem = 4 * Ring::kBytes;
     auto* k = bwd_dkv_kernel<T, D, X3, NH, CR, KEYS>;
-    const cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    static SmemLimit shared;
+        const cudaError_t e = shared.raise((const void*)k, smem);
     if (e != cudaSuccess) return (int)e;
     k<<<dim3((bp.cap + 3) / 4, bp.nsub), 128, smem, st>>>(bp);
     note_launch();

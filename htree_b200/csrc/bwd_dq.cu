@@ -400,7 +400,8 @@ static int launch_dq_cr(const BwdParams& bp, cudaStream_t st) {
     }
     if (best == 0 || W * per_warp > 227 * 1024) return HTREE_E_UNSUPPORTED;
     auto* k = bwd_dq_kernel<T, D, X3, NH, CR>;
-    const cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)(W * per_warp));
+    static SmemLimit shared;
+        const cudaError_t e = shared.raise((const void*)k, W * per_warp);
     if (e != cudaSuccess) return (int)e;
     k<<<dim3((bp.subq + W - 1) / W, bp.nsub), W * 32, W * per_warp, st>>>(bp);
     note_launch();

@@ -5,6 +5,9 @@
 #include <cuda_runtime.h>
 #include <stdint.h>
 
+#include <atomic>
+#include <mutex>
+
 #include "../../include/htree_b200.h"
 
 namespace htree {
@@ -130,6 +133,26 @@ __device__ __forceinline__ void store_parent(const AttnParams& p, int l, int64_t
     if (p.flags & HTREE_PARENTS_U16) reinterpret_cast<uint16_t*>(p.parents[l])[idx] = v < 0 ? (uint16_t)0xFFFFu : (uint16_t)v;
     else p.parents[l][idx] = v;
 }
+
+// A kernel's dynamic shared-memory limit per device, raised when a launch needs more than any before it (setting the attribute
+// on every launch costs as much as a third of the launch).  One object per kernel.
+class SmemLimit {
+    std::mutex m_;
+    std::atomic<size_t> have_[64] = {};
+
+  public:
+    cudaError_t raise(const void* kernel, size_t bytes) {
+        int dev = 0;
+        cudaError_t e = cudaGetDevice(&dev);
+        if (e != cudaSuccess) return e;
+        if (dev < 64 && have_[dev].load(std::memory_order_acquire) >= bytes) return cudaSuccess;
+        std::lock_guard<std::mutex> lock(m_);
+        if (dev < 64 && have_[dev].load(std::memory_order_relaxed) >= bytes) return cudaSuccess;
+        e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
+        if (e == cudaSuccess && dev < 64) have_[dev].store(bytes, std::memory_order_release);
+        return e;
+    }
+};
 
 constexpr uint32_t kFlagSplitOk = 1u << 30;   // internal: a forward whose selections are not kept for a backward
 

@@ -370,7 +370,8 @@ static int launch_select_cr(const AttnParams& p, cudaStream_t st) {
     const size_t split_smem = kSelSplitWarps * Ring::kBytes + scratch;
     if ((groups <= 2 * 148 || p.TK * CR > 1024) && p.TK * CR <= kSelSplitKeys && split_smem <= limit) {
         auto* k = select_mma_kernel<T, D, X3, NH, CR, true>;
-        const cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)split_smem);
+        static SmemLimit shared;
+        const cudaError_t e = shared.raise((const void*)k, split_smem);
         if (e != cudaSuccess) return (int)e;
         k<<<dim3(p.Tq, p.B * p.Hkv), kSelSplitWarps * 32, split_smem, st>>>(p);
         note_launch();
@@ -386,7 +387,8 @@ static int launch_select_cr(const AttnParams& p, cudaStream_t st) {
     }
     if (best == 0 || W * per_warp > limit) return HTREE_E_UNSUPPORTED;
     auto* k = select_mma_kernel<T, D, X3, NH, CR, false>;
-    const cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)(W * per_warp));
+    static SmemLimit shared;
+        const cudaError_t e = shared.raise((const void*)k, W * per_warp);
     if (e != cudaSuccess) return (int)e;
     k<<<dim3((p.Tq + W - 1) / W, p.B * p.Hkv), W * 32, W * per_warp, st>>>(p);
     note_launch();

@@ -177,7 +177,43 @@ def check_status(device=None) -> None:
 
 
 def _stream() -> int:
-    return torch.cuda.current_stream().cuda_stream
+    return torch._C._cuda_getCurrentRawStream(torch._C._cuda_getDevice())
+
+
+class _on_device:
+    """torch.cuda.device for the common case that the tensors' device is the current one (a tenth of its cost)."""
+
+    __slots__ = ("index", "guard")
+
+    def __init__(self, index: int):
+        self.index, self.guard = index, None
+
+    def __enter__(self):
+        if torch._C._cuda_getDevice() != self.index:
+            self.guard = torch.cuda.device(self.index)
+            self.guard.__enter__()
+
+    def __exit__(self, *exc):
+        if self.guard is not None:
+            self.guard.__exit__(*exc)
+
+
+_table_sets: Dict[Tuple, Tuple] = {}
+
+
+def _tables(k_dim: int, n_pos: int, rope_base: float, scale: float, split: bool, index: int):
+    """(cos, sin, rows of the transposed kernels, rows of the selection kernel, status word) of one configuration and the
+    addresses of the five: what a call would otherwise look up one by one."""
+    key = (k_dim, n_pos, rope_base, scale, split, index)
+    hit = _table_sets.get(key)
+    if hit is None:
+        dev = torch.device("cuda", index)
+        ts = rope_cache(k_dim, n_pos, rope_base, dev) + (rope_rows(k_dim, n_pos, rope_base, None if split else scale, dev),
+                                                         rope_rows_select(k_dim, n_pos, rope_base, dev), _status(dev))
+        if len(_table_sets) >= 256:
+            _table_sets.clear()
+        hit = _table_sets[key] = ts + tuple(t.data_ptr() for t in ts)
+    return hit
 
 
 def _validate(q, k, v, compression_rate, max_top_nodes, top_k_per_layer, q_offset=None):
@@ -234,7 +270,7 @@ def build_tree(k: torch.Tensor, v: torch.Tensor, compression_rate: int, max_top_
         cos_c = sin_c = None
         if want_rot:
             cos_c, sin_c = rope_cache(K, max(int(compression_rate), 16), rope_base, k.device)
-        with torch.cuda.device(k.device):
+        with _on_device(k.get_device()):
             _lib.check(_lib.lib().htree_b200_build_tree(
                 ctypes.byref(shape), _ptrs(layers_k), _ptrs(layers_v), _ptrs(layers_kr) if want_rot else None,
                 _ptrs(layers_kb) if want_kblk else None, _ptrs(layers_vb) if want_blk else None,
@@ -282,7 +318,7 @@ def _plan(shape: "_lib.HtreeShape", flags: int) -> "_lib.HtreePlan":
     plan = _plans.get(key)
     if plan is None:
         plan = _lib.HtreePlan()
-        _lib.check(_lib.lib().htree_b200_plan(ctypes.byref(shape), flags, ctypes.byref(plan)), "plan")
+        _lib.check(_lib.lib().htree_b200_plan(shape, flags, plan), "plan")
         if len(_plans) >= 512:       # layouts are cheap to redo: callers with ever-changing lengths do not grow this for ever
             _plans.clear()
         _plans[key] = plan
@@ -332,11 +368,14 @@ class BwdContext(dict):
     """The forward's context: the reference's keys (bwd_ctx of src/parallel.py:1139-1159).  Views of the tree levels and operand
     copies are made when they are asked for."""
 
-    _LAZY = ("layers_k", "layers_v", "layers_k_rot", "layers_v_blk", "rope_half")
+    _LAZY = ("layers_k", "layers_v", "layers_k_rot", "layers_v_blk", "rope_half", "per_layer_parents")
     workspace: Optional[_Workspace] = None
+    parents: Optional[torch.Tensor] = None         # the kept selections of all levels, [L, B, T_q, H_kv, top_k]
 
     def __missing__(self, key):
-        if key == "rope_half":
+        if key == "per_layer_parents" and self.parents is not None:
+            val = dict(enumerate(self.parents.unbind(0)))
+        elif key == "rope_half":
             k = self.workspace.k if self.workspace is not None else (self["layers_k"] or [None])[0]
             ok = k is not None and _selects_on_tensor_cores(k.dtype, k.shape[3])
             val = rope_cache_half(k.shape[3], self["cos_cache"].shape[0], self["rope_base"], self["scale"], k.device) if ok else None
@@ -390,7 +429,7 @@ def build_operands(k: torch.Tensor, v: torch.Tensor, compression_rate: int, max_
     blocks = [torch.empty(n_blk(l, 0), dtype=torch.uint8, device=dev) for l in range(len(sizes))]
     bwd = [torch.empty(n_blk(l, 1), dtype=torch.uint8, device=dev) for l in range(len(sizes))] if backward else None
     cos_c, sin_c = rope_cache(K, 16, rope_base, dev)
-    with torch.cuda.device(dev):
+    with _on_device(torch.device(dev).index):
         _lib.check(_lib.lib().htree_b200_prepare(ctypes.byref(shape), _ptrs(lk), _ptrs(lv), _ptrs(blocks), _ptrs(bwd) if bwd else None,
                                                  int(layers is None), cos_c.data_ptr(), sin_c.data_ptr(),
                                                  _stream()), "prepare")
@@ -419,7 +458,7 @@ def build_tree_into(k: torch.Tensor, v: torch.Tensor, out_k, out_v, compression_
     if len(sizes) == 1:
         return
     shape = _lib.HtreeShape(B, T, H_kv, H_kv, K, V, int(compression_rate), 1, int(max_top_nodes), _DTYPES[k.dtype])
-    with torch.cuda.device(k.device):
+    with _on_device(k.get_device()):
         _lib.check(_lib.lib().htree_b200_build_tree(ctypes.byref(shape), _ptrs(layers_k), _ptrs(layers_v), None, None, None, None,
                                                     None, _stream()), "build_tree")
 
@@ -461,7 +500,7 @@ def block_values(layers_v, compression_rate: int, max_top_nodes: int, layers_k_r
     out = [_blocked_like(x, compression_rate) for x in layers_v]
     shape = _lib.HtreeShape(B, T, H_kv, H_kv, V, V, int(compression_rate), 1, int(max_top_nodes), _DTYPES[v.dtype])
     keys = None
-    with torch.cuda.device(v.device):
+    with _on_device(v.get_device()):
         _lib.check(_lib.lib().htree_b200_block_values(ctypes.byref(shape), _ptrs(layers_v), _ptrs(out), _stream()), "block_values")
         if layers_k_rot is not None and _pipelined(v.dtype, layers_k_rot[0].shape[-1], compression_rate):
             keys = [_blocked_like(x, compression_rate) for x in layers_k_rot]
@@ -479,7 +518,7 @@ def rotate_keys(layers_k, compression_rate: int, max_top_nodes: int, rope_base: 
     out = [_rotated_like(x) for x in layers_k]
     shape = _lib.HtreeShape(B, T, H_kv, H_kv, K, K, int(compression_rate), 1, int(max_top_nodes), _DTYPES[k.dtype])
     cos_c, sin_c = rope_cache(K, max(int(compression_rate), 16), rope_base, k.device)
-    with torch.cuda.device(k.device):
+    with _on_device(k.get_device()):
         _lib.check(_lib.lib().htree_b200_rotate_keys(ctypes.byref(shape), _ptrs(layers_k), _ptrs(out),
                                                      cos_c.data_ptr(), sin_c.data_ptr(), _stream()), "rotate_keys")
     return out
@@ -487,7 +526,7 @@ def rotate_keys(layers_k, compression_rate: int, max_top_nodes: int, rope_base: 
 
 def _run_forward(shape, q, layers_k, layers_v, cos_cache, sin_cache, scale, out, gmax, gsum, parents, trace, flags,
                  layers_kr=None, half_tables=None, layers_vb=None):
-    with torch.cuda.device(q.device):
+    with _on_device(q.get_device()):
         rc = _lib.lib().htree_b200_forward(
             ctypes.byref(shape), q.data_ptr(), _ptrs(layers_k), _ptrs(layers_v),
             _ptrs(layers_kr) if layers_kr is not None else None,
@@ -581,50 +620,48 @@ def _forward_transposed(shape, q, k, v, scale, rope_base, save, save_parents, gi
     """The forward on the transposed tensor-core kernels: operand preparation, selection, accumulation."""
     B, Tq, H, K = q.shape
     H_kv, TK, CR = shape.H_kv, shape.top_k, shape.compression_rate
-    dev, dtype = q.device, q.dtype
+    dev, dtype, index = q.device, q.dtype, q.get_device()
     n_pos = TK * CR + 1024
-    cos_cache, sin_cache = rope_cache(K, n_pos, rope_base, dev)
-    table32 = rope_rows_select(K, n_pos, rope_base, dev)
-    table = rope_rows(K, n_pos, rope_base, None if _split(dtype, K) else scale, dev)
+    cos_cache, sin_cache, table, table32, _, cos_ptr, sin_ptr, tab_ptr, tab32_ptr, status_ptr = _tables(
+        K, n_pos, rope_base, scale, _split(dtype, K), index)
     keep = save and save_parents
     # Callers that do not keep the selections get them only as temporaries (int32 whatever SELECTION_STORAGE says), and only up
     # to SPLIT_FORWARD_MAX_BYTES at a time: beyond it the queries run window by window over the same tree, with the same results.
     plan = _plan(shape, _lib.PLAN_BACKWARD if save else 0)
     L = plan.levels
-    out = torch.empty(B, Tq, H, K, dtype=dtype, device=dev)
-    stats = torch.empty(2, B, Tq, H, dtype=torch.float32, device=dev)
+    out = torch.empty_like(q)
+    stats = torch.empty((2, B, Tq, H), dtype=torch.float32, device=dev)
     per_query = L * H_kv * TK * 4
+    ws = layers = parents = None
     if not keep and (windows or B * Tq * per_query > SPLIT_FORWARD_MAX_BYTES):
         layers = _operand_layers(k, v, shape, rope_base, given_layers, save)
         _forward_windows(shape, q, layers, cos_cache, sin_cache, (table, table32), scale, out, stats[0], stats[1], per_query)
-        parents = ws = None
     else:
-        pdt = torch.int32
-        if keep:
-            pdt = _parents_dtype_of(plan, TK)
-        parents = torch.empty(L, B, Tq, H_kv, TK, dtype=pdt, device=dev)
+        pdt = _parents_dtype_of(plan, TK) if keep else torch.int32
+        parents = torch.empty((L, B, Tq, H_kv, TK), dtype=pdt, device=dev)
         flags = (0 if save or given_layers is not None else _lib.FWD_INFERENCE) | (_lib.PARENTS_U16 if pdt == torch.int16 else 0)
-        p0, step = parents.data_ptr(), B * Tq * H_kv * TK * pdt.itemsize
-        pptr = _lib.ptr_array([p0 + l * step for l in range(L)])
+        pptr = _lib.address_array(parents.data_ptr(), B * Tq * H_kv * TK * pdt.itemsize, L)
         gmax_ptr = stats.data_ptr()
         gsum_ptr = gmax_ptr + B * Tq * H * 4
-        with torch.cuda.device(dev):
+        with _on_device(index):
             if given_layers is None:
                 ws = torch.empty(plan.bytes, dtype=torch.uint8, device=dev)
                 rc = _lib.lib().htree_b200_run_forward(
-                    ctypes.byref(shape), ctypes.byref(plan), q.data_ptr(), k.data_ptr(), v.data_ptr(), cos_cache.data_ptr(),
-                    sin_cache.data_ptr(), table.data_ptr(), table32.data_ptr(), n_pos, scale, ws.data_ptr(), out.data_ptr(), gmax_ptr, gsum_ptr, pptr,
-                    _status(dev).data_ptr(), flags, _stream())
-                layers = None
+                    shape, plan, q.data_ptr(), k.data_ptr(), v.data_ptr(), cos_ptr, sin_ptr, tab_ptr, tab32_ptr, n_pos, scale,
+                    ws.data_ptr(), out.data_ptr(), gmax_ptr, gsum_ptr, pptr, status_ptr, flags,
+                    torch._C._cuda_getCurrentRawStream(index))
             else:
-                ws = None
                 layers = _operand_layers(k, v, shape, rope_base, given_layers, save)
                 rc = _attend(shape, q, layers, cos_cache, sin_cache, (table, table32), scale, out.data_ptr(), gmax_ptr, gsum_ptr, pptr, flags)
-        _lib.check(rc, "forward")
+        if rc:
+            _lib.check(rc, "forward")
     if not save:
         return out
     ctx = BwdContext(_context_fields(stats[0], stats[1], cos_cache, sin_cache, L, shape, rope_base, scale))
-    ctx["per_layer_parents"] = dict(enumerate(parents.unbind(0))) if keep else None
+    if keep:
+        ctx.parents = parents
+    else:
+        ctx["per_layer_parents"] = None
     if ws is not None:
         ctx.workspace = _Workspace(ws, plan, k, v, CR)
     else:
@@ -667,7 +704,7 @@ def _forward_windows(shape, q, layers, cos_cache, sin_cache, tables, scale, out,
     parents = torch.empty(L, step, shape.H_kv, shape.top_k, dtype=torch.int32, device=q.device)
     pptr = _ptrs(parents.unbind(0))
     t_offset = shape.t_offset
-    with torch.cuda.device(q.device):
+    with _on_device(q.get_device()):
         for b in range(B):
             blocks = OperandBlocks([])
             blocks.blocks = [x.view(B, -1)[b] for x in layers[3].blocks]
@@ -694,7 +731,7 @@ def recompute_parents(q, layers_k, layers_v, cos_cache, sin_cache, compression_r
     if rope_base is not None and getattr(layers_v_blk, "blocks", None) is not None and not _force_generic and q.is_contiguous() and q.data_ptr() % 32 == 0:
         rows = rope_rows_select(K, cos_cache.shape[0], rope_base, q.device)
         tables = (rows, rows)                            # the selection reads the second only
-        with torch.cuda.device(q.device):
+        with _on_device(q.get_device()):
             _lib.check(_attend(shape, q, (layers_k, layers_v, None, layers_v_blk), cos_cache, sin_cache, tables, scale, None, None, None,
                                _ptrs(parents), _lib.FWD_SELECT_ONLY | _parents_flag(parents)), "select")
         return {l: parents[l] for l in range(L)}
@@ -739,41 +776,53 @@ def _backward_two_pass(dO, q, output, ctx, operands, typed, window):
                             0 if window is None else int(window["t0"]))
     if key not in _bwd_plans:
         a, s = ctypes.c_int64(), ctypes.c_int64()
-        rc = _lib.lib().htree_b200_backward_plan(ctypes.byref(shape), budget, ctypes.byref(a), ctypes.byref(s))
+        rc = _lib.lib().htree_b200_backward_plan(shape, budget, ctypes.byref(a), ctypes.byref(s))
         if len(_bwd_plans) >= 512:
             _bwd_plans.clear()
-        _bwd_plans[key] = (a.value, s.value) if rc == 0 else None
+        _bwd_plans[key] = ((a.value + 255) // 256 * 256, s.value) if rc == 0 else None
     plan = _bwd_plans[key]
     if plan is None or window is not None and not window["first"] and "two_pass" not in window["acc"]:
         return None
-    dev, dtype = q.device, q.dtype
-    parents = ctx.get("per_layer_parents")
-    if parents is None:
-        parents = recompute_parents(q, ctx["layers_k"], ctx["layers_v"], ctx["cos_cache"], ctx["sin_cache"], CR, TK, MTN, ctx["scale"],
-                                    layers_v_blk=ctx["layers_v_blk"], rope_base=ctx["rope_base"])
-    n_pos = ctx["cos_cache"].shape[0]
-    table = rope_rows(K, n_pos, ctx["rope_base"], None if _split(dtype, K) else ctx["scale"], dev)
+    dev, dtype, index = q.device, q.dtype, q.get_device()
+    L = len(blocks)
+    kept = getattr(ctx, "parents", None)
+    if kept is not None and not dict.__contains__(ctx, "per_layer_parents"):
+        pptr = _lib.address_array(kept.data_ptr(), kept.stride(0) * kept.element_size(), L)
+        pflag = _lib.PARENTS_U16 if kept.dtype == torch.int16 else 0
+    else:
+        parents = ctx.get("per_layer_parents")
+        if parents is None:
+            parents = recompute_parents(q, ctx["layers_k"], ctx["layers_v"], ctx["cos_cache"], ctx["sin_cache"], CR, TK, MTN, ctx["scale"],
+                                        layers_v_blk=ctx["layers_v_blk"], rope_base=ctx["rope_base"])
+        kept = [parents[l] for l in range(L)]
+        pptr, pflag = _ptrs(kept), _parents_flag(kept)
+    n_pos, scale = ctx["cos_cache"].shape[0], float(ctx["scale"])
+    t = _tables(K, n_pos, ctx["rope_base"], scale, _split(dtype, K), index)
     if window is None:
-        acc, flags, final = torch.empty(plan[0], dtype=torch.uint8, device=dev), 0, True
+        scratch = torch.empty(plan[0] + plan[1], dtype=torch.uint8, device=dev)
+        acc_ptr, flags, final = scratch.data_ptr(), 0, True
+        scratch_ptr = acc_ptr + plan[0]
     else:
         if window["first"]:
             window["acc"]["two_pass"] = torch.empty(plan[0], dtype=torch.uint8, device=dev)
-        acc, final = window["acc"]["two_pass"], window["last"]
+        acc_ptr, final = window["acc"]["two_pass"].data_ptr(), window["last"]
         flags = (0 if window["first"] else _lib.BWD_KEEP_ACCUM) | (0 if final else _lib.BWD_NO_FOLD)
-    scratch = torch.empty(plan[1], dtype=torch.uint8, device=dev)
+        scratch = torch.empty(plan[1], dtype=torch.uint8, device=dev)
+        scratch_ptr = scratch.data_ptr()
     gdt = dtype if typed else torch.float32
-    dq = torch.empty(B, Tq, H, K, dtype=gdt, device=dev)
-    dk, dv = (torch.empty(B, T, H_kv, K, dtype=gdt, device=dev) for _ in range(2)) if final else (None, None)
-    L = len(blocks)
-    pl = [parents[l] for l in range(L)]
-    with torch.cuda.device(dev):
+    dq = torch.empty((B, Tq, H, K), dtype=gdt, device=dev)
+    dk = dv = None
+    if final:
+        dk = torch.empty((B, T, H_kv, K), dtype=gdt, device=dev)
+        dv = torch.empty((B, T, H_kv, K), dtype=gdt, device=dev)
+    with _on_device(index):
         rc = _lib.lib().htree_b200_run_backward(
-            ctypes.byref(shape), q.data_ptr(), _lib.ptr_array(blocks), _lib.ptr_array(blocks_bwd), ctx["cos_cache"].data_ptr(),
-            ctx["sin_cache"].data_ptr(), table.data_ptr(), n_pos, float(ctx["scale"]), output.data_ptr(), dO.data_ptr(),
-            ctx["global_max"].data_ptr(), ctx["global_sum"].data_ptr(), _ptrs(pl), acc.data_ptr(), scratch.data_ptr(), budget,
-            dq.data_ptr(), dk.data_ptr() if final else None, dv.data_ptr() if final else None, int(typed), _status(dev).data_ptr(),
-            flags | _parents_flag(pl), _stream())
-    _lib.check(rc, "backward")
+            shape, q.data_ptr(), _lib.ptr_array(blocks), _lib.ptr_array(blocks_bwd), t[5], t[6], t[7], n_pos, scale, output.data_ptr(),
+            dO.data_ptr(), ctx["global_max"].data_ptr(), ctx["global_sum"].data_ptr(), pptr, acc_ptr, scratch_ptr, budget, dq.data_ptr(),
+            dk.data_ptr() if final else None, dv.data_ptr() if final else None, 1 if typed else 0, t[9], flags | pflag,
+            torch._C._cuda_getCurrentRawStream(index))
+    if rc:
+        _lib.check(rc, "backward")
     return dq, dk, dv
 
 
@@ -843,7 +892,7 @@ def htree_backward(dO: torch.Tensor, q: torch.Tensor, output: torch.Tensor, bwd_
         typed = _lib.HtreeTypedGrads(dq.data_ptr(), dk_t.data_ptr(), dv_t.data_ptr())
     else:
         dq = torch.empty(B, T, H, K, dtype=torch.float32, device=dev)
-    with torch.cuda.device(dev):
+    with _on_device(torch.device(dev).index):
         rc = _lib.lib().htree_b200_backward(
             ctypes.byref(shape), q.data_ptr(), _ptrs(layers_k), _ptrs(layers_v),
             _ptrs(layers_kr) if layers_kr is not None else None, cos_cache.data_ptr(), sin_cache.data_ptr(),

@@ -149,6 +149,28 @@ def lib() -> ctypes.CDLL:
     return _lib
 
 
+_glue = None
+
+
+def glue():
+    """The torch-side call path (csrc/torch_glue.cpp).  False where another build of the library was asked for by path: the
+    extension is linked to the one beside it."""
+    global _glue
+    if _glue is None:
+        lib()
+        if os.environ.get("HTREE_B200_LIB"):
+            _glue = False
+        else:
+            import importlib.util
+            path = os.path.join(_HERE, "_torch_glue.so")
+            if not os.path.exists(path):
+                raise RuntimeError(f"{path} is missing: build it with `python -m htree_b200.build`")
+            spec = importlib.util.spec_from_file_location("_torch_glue", path)
+            _glue = importlib.util.module_from_spec(spec)
+            spec.loader.exec_module(_glue)
+    return _glue
+
+
 def launch_count() -> int:
     return int(lib().htree_b200_launch_count())
 

@@ -16,6 +16,7 @@ HERE = os.path.dirname(os.path.abspath(__file__))
 CSRC = os.path.join(HERE, "csrc")
 LIB = os.path.join(HERE, "libhtree_b200.so")
 PROBES_LIB = os.path.join(HERE, "libhtree_b200_probes.so")    # measurement aids of the benchmark (csrc/bench/), not the operator
+GLUE_LIB = os.path.join(HERE, "_torch_glue.so")               # Python extension: the torch-side call path
 OBJ_DIR = os.path.join(HERE, "build")
 ARCH = ["-gencode", "arch=compute_100a,code=sm_100a"]
 FLAGS = ["-O3", "-std=c++17", "-lineinfo", "-Xcompiler", "-fPIC", "--expt-relaxed-constexpr", "-Xptxas", "-v"]
@@ -72,7 +73,27 @@ def build(force: bool = False, verbose: bool = False, defines=(), out: str = LIB
             raise RuntimeError(f"link failed:\n{r.stdout}\n{r.stderr}")
     if out == LIB:
         build_probes(force)
+        build_glue(force)
     return LIB_
+
+
+def build_glue(force: bool = False) -> str:
+    """The torch-side call path (csrc/torch_glue.cpp) as a Python extension next to the library, which it links."""
+    src = os.path.join(CSRC, "torch_glue.cpp")
+    header = os.path.join(HERE, "..", "include", "htree_b200.h")
+    if force or _stale(GLUE_LIB, [src, header]):
+        import sysconfig
+        import torch
+        from torch.utils import cpp_extension as ce
+        inc = [f"-isystem{p}" for p in [*ce.include_paths(), sysconfig.get_paths()["include"], "/usr/local/cuda/include"]]
+        libs = [f"-L{p}" for p in ce.library_paths()] + ["-L/usr/local/cuda/lib64"]
+        cmd = ["g++", "-O2", "-std=c++17", "-fPIC", "-shared", "-DTORCH_EXTENSION_NAME=_torch_glue", "-DTORCH_API_INCLUDE_EXTENSION_H",
+               f"-D_GLIBCXX_USE_CXX11_ABI={int(torch._C._GLIBCXX_USE_CXX11_ABI)}", *inc, src, "-o", GLUE_LIB, *libs, "-lc10", "-lc10_cuda",
+               "-ltorch_cpu", "-ltorch", "-ltorch_python", f"-L{HERE}", "-lhtree_b200", "-Wl,-rpath,$ORIGIN"]
+        r = subprocess.run(cmd, capture_output=True, text=True)
+        if r.returncode != 0:
+            raise RuntimeError(f"g++ failed on {src}:\n{r.stdout}\n{r.stderr}")
+    return GLUE_LIB
 
 
 def build_probes(force: bool = False) -> str:

@@ -568,6 +568,13 @@ def htree_forward(
     q = q.contiguous(); k = k.contiguous(); v = v.contiguous()
     if (not (_force_generic or return_trace) and _transposed(q.dtype, K, V, H // H_kv, compression_rate) and q.data_ptr() % 32 == 0
             and k.data_ptr() % 16 == 0 and v.data_ptr() % 16 == 0):
+        if not (_save_for_backward or _fused or _layers is not None) and _lib.glue():
+            n_pos = top_k_per_layer * compression_rate + 1024
+            out = _lib.glue().plain_forward(q, k, v, _tables(K, n_pos, rope_base, scale, _split(q.dtype, K), q.get_device())[:5],
+                                            compression_rate, max_top_nodes, top_k_per_layer, scale,
+                                            -1 if _q_offset is None else _q_offset, SPLIT_FORWARD_MAX_BYTES)
+            if out is not None:
+                return out
         return _forward_transposed(shape, q, k, v, scale, rope_base, _save_for_backward, _save_parents, _layers, _fused)
     dev = q.device
     if _layers is not None:
@@ -948,6 +955,16 @@ def htree_forward_autograd(q, k, v, compression_rate: int = 16, max_top_nodes: i
     """Differentiable forward (signature of htree_forward_triton_autograd, src/backward.py:1196-1208)."""
     if scale is None:
         scale = q.shape[-1] ** -0.5
+    if SAVE_SELECTIONS_FOR_BACKWARD and SELECTION_STORAGE == "int32" and q.dim() == 4 and _lib.glue():
+        q = q.contiguous(); k = k.contiguous(); v = v.contiguous()
+        _validate(q, k, v, compression_rate, max_top_nodes, top_k_per_layer)
+        K = q.shape[3]
+        if _transposed(q.dtype, K, v.shape[3], q.shape[2] // k.shape[2], compression_rate):
+            out = _lib.glue().autograd_forward(
+                q, k, v, _tables(K, top_k_per_layer * compression_rate + 1024, rope_base, scale, _split(q.dtype, K), q.get_device())[:5],
+                compression_rate, max_top_nodes, top_k_per_layer, scale, BACKWARD_MAX_BYTES)
+            if out is not None:
+                return out
     return HTreeFunction.apply(q.contiguous(), k.contiguous(), v.contiguous(), compression_rate, max_top_nodes,
                                top_k_per_layer, scale, rope_base)
 

@@ -11,7 +11,7 @@
 namespace htree {
 
 template <int D, bool X3>
-constexpr int acc_stages() { return D == 128 ? 2 : 3; }
+constexpr int acc_stages() { return D * (X3 ? 2 : 1) >= 128 ? 2 : 3; }     // slots of 8 KB: warps matter more than depth
 
 // Registers: 168 per thread (12 warps per SM) hold a group of 16 heads of 128; what the kernel needs beyond that is room for
 // the rings, two slots of 8448 bytes per warp at 128-wide heads.
@@ -275,8 +275,7 @@ acc_mma_kernel(const __grid_constant__ AttnParams p) {
                 p.gmax[hbase + head] = mt; p.gsum[hbase + head] = s * __expf(m - mt);
             }
         }
-        return;
-    }
+    } else {
 #pragma unroll
     for (int h = 0; h < NH; ++h)
 #pragma unroll
@@ -302,6 +301,7 @@ acc_mma_kernel(const __grid_constant__ AttnParams p) {
             }
             if (g == 0) { p.gmax[hbase + head] = m_true[h][e]; p.gsum[hbase + head] = s_run[h][e] * __expf(m_run[h][e] - m_true[h][e]); }
         }
+    }
 }
 
 template <typename T, int D, bool X3, int NH, int CR>

@@ -258,13 +258,15 @@ int htree_b200_prepare(const HtreeShape* shape, void* const* layers_k, void* con
         if (!aligned16(layers_k[l]) || !aligned16(layers_v[l]) || !aligned16(blocks[l]) || (blocks_bwd && !aligned16(blocks_bwd[l])))
             return HTREE_E_ALIGN;
     }
-    return launch_pack_blocks(*shape, L, ln, layers_k, layers_v, blocks, blocks_bwd, pool != 0, cos_cache, sin_cache,
+    return launch_pack_blocks(*shape, 0, L, ln, layers_k, layers_v, blocks, blocks_bwd, pool != 0, cos_cache, sin_cache,
                               (cudaStream_t)stream);
 }
 
-int htree_b200_attend(const HtreeShape* shape, const void* q, void* const* layers_k, void* const* layers_v, void* const* blocks,
-                      const float* cos_cache, const float* sin_cache, const void* table, const void* table_f32, int32_t n_pos, float scale,
-                      void* out, float* gmax, float* gsum, int32_t* const* parents, int32_t* status, uint32_t flags, void* stream) {
+// `pack_leaves`: the leaf blocks are still to be packed, those that the selections name
+static int attend(const HtreeShape* shape, const void* q, void* const* layers_k, void* const* layers_v, void* const* blocks,
+                  const float* cos_cache, const float* sin_cache, const void* table, const void* table_f32, int32_t n_pos, float scale,
+                  void* out, float* gmax, float* gsum, int32_t* const* parents, int32_t* status, uint32_t flags, bool pack_leaves,
+                  void* stream) {
     int32_t ln[HTREE_MAX_LEVELS];
     const int L = check_shape(shape, ln);
     if (L < 0) return L;
@@ -285,8 +287,19 @@ int htree_b200_attend(const HtreeShape* shape, const void* q, void* const* layer
     rc = select_blk_supported(p, shape->dtype) ? launch_select_blk(p, shape->dtype, (cudaStream_t)stream)
                                                : launch_fwd_generic(p, shape->dtype, (cudaStream_t)stream);
     if (rc || select_only) return rc;
+    if (pack_leaves) {
+        rc = launch_pack_listed(*shape, p.Tq, layers_k[0], layers_v[0], blocks[0], parents[0], cos_cache, sin_cache, (cudaStream_t)stream);
+        if (rc) return rc;
+    }
     p.flags = flags | ((flags & HTREE_FWD_INFERENCE) ? kFlagSplitOk : 0u);
     return launch_acc_mma(p, shape->dtype, (cudaStream_t)stream);
+}
+
+int htree_b200_attend(const HtreeShape* shape, const void* q, void* const* layers_k, void* const* layers_v, void* const* blocks,
+                      const float* cos_cache, const float* sin_cache, const void* table, const void* table_f32, int32_t n_pos, float scale,
+                      void* out, float* gmax, float* gsum, int32_t* const* parents, int32_t* status, uint32_t flags, void* stream) {
+    return attend(shape, q, layers_k, layers_v, blocks, cos_cache, sin_cache, table, table_f32, n_pos, scale, out, gmax, gsum, parents,
+                  status, flags, false, stream);
 }
 
 int htree_b200_plan(const HtreeShape* shape, uint32_t flags, HtreePlan* plan) {
@@ -331,10 +344,26 @@ int htree_b200_run_forward(const HtreeShape* shape, const HtreePlan* plan, const
         bl[l] = at(plan->blocks[l]); bb[l] = at(plan->blocks_bwd[l]);
         par[l] = parents ? parents[l] : reinterpret_cast<int32_t*>(at(plan->parents[l]));
     }
-    const int rc = htree_b200_prepare(shape, lk, lv, bl, plan->blocks_bwd[0] >= 0 ? bb : nullptr, 1, cos_cache, sin_cache, stream);
+    // A window of few queries against a long sequence reads a small part of the leaves' blocks: when the selections can name at most
+    // half of them, the leaves are only pooled (read once, a sixteenth or an eighth written) and the named blocks packed afterwards.
+    // The blocks of all leaves are twice the bytes to move and were a third of a call with one new query against 16K positions.
+    const int32_t Tq = shape->T_q > 0 ? shape->T_q : shape->T;
+    const int64_t nblk = (shape->T + shape->compression_rate - 1) / shape->compression_rate;
+    int rc;
+    const bool few = (flags & HTREE_FWD_INFERENCE) && plan->levels > 1 && 2 * (int64_t)Tq * shape->top_k <= nblk;
+    if (few) {
+        int32_t ln[HTREE_MAX_LEVELS];
+        const int L = check_shape(shape, ln);
+        if (L < 0) return L;
+        if (L != plan->levels || !cos_cache || !sin_cache) return HTREE_E_NULL;
+        if (!aligned16(k) || !aligned16(v) || !aligned16(workspace) || !aligned16(cos_cache) || !aligned16(sin_cache)) return HTREE_E_ALIGN;
+        rc = launch_tree_build(*shape, 2, ln, lk, lv, (cudaStream_t)stream);
+        if (rc == 0) rc = launch_pack_blocks(*shape, 1, L, ln, lk, lv, bl, nullptr, true, cos_cache, sin_cache, (cudaStream_t)stream);
+    } else {
+        rc = htree_b200_prepare(shape, lk, lv, bl, plan->blocks_bwd[0] >= 0 ? bb : nullptr, 1, cos_cache, sin_cache, stream);
+    }
     if (rc) return rc;
-    return htree_b200_attend(shape, q, lk, lv, bl, cos_cache, sin_cache, table, table_f32, n_pos, scale, out, gmax, gsum, par, status, flags,
-                             stream);
+    return attend(shape, q, lk, lv, bl, cos_cache, sin_cache, table, table_f32, n_pos, scale, out, gmax, gsum, par, status, flags, few, stream);
 }
 
 int htree_b200_block_keys(const HtreeShape* shape, void* const* layers_k_rot, void* const* layers_k_blk, void* stream) {

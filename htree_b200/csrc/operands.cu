@@ -16,7 +16,9 @@ struct PackArgs {
     void* pv;
     const float* cosc;
     const float* sinc;
-    int64_t total;      // B * NBLK * Hkv
+    const int32_t* list;    // NULL, or parents [B, Tq, Hkv, TK]: only the blocks they name are packed
+    int64_t total;      // B * NBLK * Hkv blocks, or list entries
+    int32_t Tq, TK;
     int32_t N, NBLK, Hkv;
 };
 
@@ -79,9 +81,15 @@ template <typename T, int D, bool X3, int CR>
 __global__ void __launch_bounds__(128) pack_blocks_kernel(const __grid_constant__ PackArgs a) {
     using C = TForm<D, X3, CR>;
     constexpr int HALF = C::HALF, PPT = C::PPT, KS = C::KS, VB = C::VB;
-    const int64_t blk = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
+    int64_t blk = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
     if (blk >= a.total) return;
     const int lane = threadIdx.x & 31, g = lane >> 2, r = lane & 3;
+    if (a.list) {
+        const int node = a.list[blk];
+        if ((unsigned)node >= (unsigned)a.NBLK) return;
+        const int64_t grp = blk / a.TK;
+        blk = ((grp / ((int64_t)a.Hkv * a.Tq)) * a.NBLK + node) * a.Hkv + grp % a.Hkv;
+    }
     const int h = (int)(blk % a.Hkv);
     const int p = (int)((blk / a.Hkv) % a.NBLK);
     const int64_t b = blk / ((int64_t)a.Hkv * a.NBLK);
@@ -259,26 +267,44 @@ static void launch_pack_d(const PackArgs& a, int D, int CR, cudaStream_t st) {
     else launch_pack_t<T, 32, true>(a, CR, st);
 }
 
-// blk[l] of every level, and, where asked for, the pooled levels lk[l + 1] / lv[l + 1] and vkblk[l].
-int launch_pack_blocks(const HtreeShape& s, int L, const int32_t* ln, void* const* lk, void* const* lv, void* const* blk,
+static int launch_pack(const PackArgs& a, const HtreeShape& s, cudaStream_t st) {
+    switch (s.dtype) {
+        case HTREE_F32: launch_pack_d<float>(a, s.K, s.compression_rate, st); break;
+        case HTREE_BF16: launch_pack_d<__nv_bfloat16>(a, s.K, s.compression_rate, st); break;
+        default: launch_pack_d<__half>(a, s.K, s.compression_rate, st); break;
+    }
+    note_launch();
+    return (int)cudaGetLastError();
+}
+
+static PackArgs pack_args(const HtreeShape& s, int N, const void* k, const void* v, void* blk, const float* cosc, const float* sinc) {
+    PackArgs a{};
+    a.k = k; a.v = v; a.blk = blk; a.cosc = cosc; a.sinc = sinc;
+    a.N = N; a.Hkv = s.H_kv; a.NBLK = (N + s.compression_rate - 1) / s.compression_rate;
+    a.total = (int64_t)s.B * a.NBLK * s.H_kv;
+    return a;
+}
+
+// blk[l] of the levels from `first` up, and, where asked for, the pooled levels lk[l + 1] / lv[l + 1] and vkblk[l].
+int launch_pack_blocks(const HtreeShape& s, int first, int L, const int32_t* ln, void* const* lk, void* const* lv, void* const* blk,
                        void* const* vkblk, bool pool, const float* cosc, const float* sinc, cudaStream_t st) {
-    for (int l = 0; l < L; ++l) {
-        PackArgs a;
-        a.k = lk[l]; a.v = lv[l]; a.blk = blk[l]; a.vkblk = vkblk ? vkblk[l] : nullptr;
+    for (int l = first; l < L; ++l) {
+        PackArgs a = pack_args(s, ln[l], lk[l], lv[l], blk[l], cosc, sinc);
+        a.vkblk = vkblk ? vkblk[l] : nullptr;
         a.pk = pool && l + 1 < L ? lk[l + 1] : nullptr; a.pv = pool && l + 1 < L ? lv[l + 1] : nullptr;
-        a.cosc = cosc; a.sinc = sinc;
-        a.N = ln[l]; a.Hkv = s.H_kv; a.NBLK = (ln[l] + s.compression_rate - 1) / s.compression_rate;
-        a.total = (int64_t)s.B * a.NBLK * s.H_kv;
-        switch (s.dtype) {
-            case HTREE_F32: launch_pack_d<float>(a, s.K, s.compression_rate, st); break;
-            case HTREE_BF16: launch_pack_d<__nv_bfloat16>(a, s.K, s.compression_rate, st); break;
-            default: launch_pack_d<__half>(a, s.K, s.compression_rate, st); break;
-        }
-        note_launch();
-        const cudaError_t e = cudaGetLastError();
-        if (e != cudaSuccess) return (int)e;
+        const int rc = launch_pack(a, s, st);
+        if (rc) return rc;
     }
     return 0;
+}
+
+// The leaf blocks that the parent lists of level 0 name, [B, Tq, H_kv, top_k] (a block named twice is written twice, alike).
+int launch_pack_listed(const HtreeShape& s, int Tq, const void* k, const void* v, void* blk, const int32_t* parents, const float* cosc,
+                       const float* sinc, cudaStream_t st) {
+    PackArgs a = pack_args(s, s.T, k, v, blk, cosc, sinc);
+    a.list = parents; a.Tq = Tq; a.TK = s.top_k;
+    a.total = (int64_t)s.B * Tq * s.H_kv * s.top_k;
+    return launch_pack(a, s, st);
 }
 
 }  // namespace htree

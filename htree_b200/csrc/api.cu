@@ -137,7 +137,7 @@ static int bwd_layout(const HtreeShape* s, int L, const int32_t* ln, int64_t bud
     y.o_qb = take(per * subq * qb); y.o_dob = take(per * subq * qb);
     y.o_stp = take(per * subq * MV * sb); y.o_sts = take(per * subq * MV * sb);
     y.o_rank = take(per * subq * MV * 4); y.o_entries = take(per * subq * MV * 8);
-    y.o_cnt = take(per * NK * 4); y.o_base = take(per * NK * 4);
+    y.o_cnt = take(per * NK * 4); y.o_base = take(per * NK * 8);
     y.o_items = take(per * bp.cap * (int64_t)sizeof(BwdItem)); y.o_nitems = take(per * 4);
     y.scratch_bytes = at;
     return 0;
@@ -555,7 +555,7 @@ int htree_b200_run_backward(const HtreeShape* shape, const void* q, void* const*
     p.dq = typed ? nullptr : static_cast<float*>(dq); p.dq_typed = typed ? dq : nullptr;
     bp.qb = sb + y.o_qb; bp.dob = sb + y.o_dob; bp.stp = sb + y.o_stp; bp.sts = sb + y.o_sts;
     bp.rank = reinterpret_cast<int32_t*>(sb + y.o_rank); bp.entries = reinterpret_cast<uint2*>(sb + y.o_entries);
-    bp.cnt = reinterpret_cast<int32_t*>(sb + y.o_cnt); bp.base = reinterpret_cast<int32_t*>(sb + y.o_base);
+    bp.cnt = reinterpret_cast<int32_t*>(sb + y.o_cnt); bp.base = reinterpret_cast<int2*>(sb + y.o_base);
     bp.items = reinterpret_cast<BwdItem*>(sb + y.o_items); bp.nitems = reinterpret_cast<int32_t*>(sb + y.o_nitems);
     cudaStream_t st = (cudaStream_t)stream;
     if (!(flags & HTREE_BWD_KEEP_ACCUM)) {

@@ -28,7 +28,7 @@ struct BwdParams {
     unsigned char* sts;                      // dS
     int32_t* rank;                           // [group * MV + visit]
     int32_t* cnt;                            // [nsub][NK]
-    int32_t* base;                           // [nsub][NK]
+    int2* base;                              // [nsub][NK]: first entry, first item
     uint2* entries;                          // [nsub][subq * MV]
     BwdItem* items;                          // [nsub][cap]
     int32_t* nitems;                         // [nsub]

@@ -77,8 +77,10 @@ __global__ void __launch_bounds__(256) bwd_fill_kernel(const __grid_constant__ B
 // blocked output gradients; B = dS or P as the first pass left them.  One warp per item, operands through the warp's ring.
 // The two gradients are separate launches: each gathers from one blocked tensor only (a window of it stays in L2) and its
 // accumulator is 64 registers, which leaves room for 16 and more warps per SM.
-template <int D, bool X3>
-constexpr int dkv_stages() { return X3 ? 2 : 3; }
+// Ring depth: three slots; two where that lets more blocks share an SM and they are the faster choice: split-half, and the keys of
+// groups of 9 to 16 heads of 128 (65536 positions, 64 heads: 13.2 -> 12.4 ms; with 8 heads a group three slots keep a lead of 1%).
+template <int D, bool X3, int NH, bool KEYS>
+constexpr int dkv_stages() { return X3 || (KEYS && D == 128 && NH == 2) ? 2 : 3; }
 template <int D, bool X3>
 constexpr int dkv_min_blocks() { return X3 ? (D == 128 ? 2 : 3) : D == 128 ? 3 : 4; }
 
@@ -90,7 +92,7 @@ __global__ void __launch_bounds__(128, dkv_min_blocks<D, X3>()) bwd_dkv_kernel(c
     using F = Frag<FT>;
     constexpr int KS = BF::KS, NT = BF::NT, QB = BF::QB, SB = BF::SB, PPT = C::PPT, HALF = C::HALF;
     constexpr int TAB = KEYS ? C::TAB : 0;
-    constexpr int SLOT = 2 * QB + 2 * SB + 2 * TAB, NSTG = dkv_stages<D, X3>();
+    constexpr int SLOT = 2 * QB + 2 * SB + 2 * TAB, NSTG = dkv_stages<D, X3, NH, KEYS>();
     constexpr int PLANE = NT * 128;                                         // bytes from the hi to the lo words of a record
     using Ring = WarpRing<NSTG, SLOT>;
     extern __shared__ __align__(128) unsigned char smem_raw[];
@@ -309,7 +311,7 @@ template <typename T, int D, bool X3, int NH, int CR, bool KEYS>
 static int launch_dkv_one(const BwdParams& bp, cudaStream_t st) {
     using BF = BForm<D, X3, NH, CR>;
     constexpr int SLOT = 2 * BF::QB + 2 * BF::SB + (KEYS ? 2 * TForm<D, X3, CR>::TAB : 0);
-    using Ring = WarpRing<dkv_stages<D, X3>(), SLOT>;
+    using Ring = WarpRing<dkv_stages<D, X3, NH, KEYS>(), SLOT>;
     const size_t smem = 4 * Ring::kBytes;
     auto* k = bwd_dkv_kernel<T, D, X3, NH, CR, KEYS>;
     static SmemLimit shared;

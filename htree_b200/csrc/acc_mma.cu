@@ -32,8 +32,9 @@ acc_mma_kernel(const __grid_constant__ AttnParams p) {
 
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, g = lane >> 2, r = lane & 3;
     const int W = blockDim.x >> 5;
-    const int tl = SPLIT ? (int)blockIdx.x : (int)(blockIdx.x * W + warp);
-    if (!SPLIT && tl >= p.Tq) return;
+    const int from_end = SPLIT ? (int)blockIdx.x : (int)(blockIdx.x * W + warp);
+    if (!SPLIT && from_end >= p.Tq) return;
+    const int tl = p.Tq - 1 - from_end;                               // the longest walks first: they would be the tail of a short call
     const int t = p.t0 + tl;
     const int b = blockIdx.y / p.Hkv, hk = blockIdx.y % p.Hkv;
     const int G = p.G, TK = p.TK, L = p.L;
@@ -80,22 +81,6 @@ acc_mma_kernel(const __grid_constant__ AttnParams p) {
         if (l > 0 && nc <= TK) continue;                              // every candidate is kept: nothing to accumulate
         if (np <= 0) continue;
         const int nchunk = (np + PPC - 1) / PPC;
-        if (l > 0) {
-            // positions the next level kept, from its list (both lists ascending)
-            for (int i = lane; i < (nc + 31) / 32; i += 32) selw[i] = 0u;
-            __syncwarp();
-            for (int i = lane; i < TK; i += 32) {
-                const int node = load_parent(p, l - 1, qidx * TK + i);
-                if (node < 0) continue;
-                const int parent = node / CR;
-                int lo = 0, hi = np;
-                while (lo < hi) { const int mid = (lo + hi) >> 1; if (par[mid] < parent) lo = mid + 1; else hi = mid; }
-                if (lo < np && par[lo] == parent) {
-                    const int j = lo * CR + node % CR;
-                    atomicOr(&selw[j >> 5], 1u << (j & 31));
-                }
-            }
-        }
         __syncwarp();
 
         const int nblk = (Nl + CR - 1) / CR;
@@ -123,6 +108,22 @@ acc_mma_kernel(const __grid_constant__ AttnParams p) {
         for (int s = 0; s < NSTG - 1; ++s, next += step) {
             if (next < nchunk) fill(next);
             ring.commit();
+        }
+        if (l > 0) {
+            // positions the next level kept, from its list (both lists ascending); found while the first blocks are on their way
+            for (int i = lane; i < (nc + 31) / 32; i += 32) selw[i] = 0u;
+            __syncwarp();
+            for (int i = lane; i < TK; i += 32) {
+                const int node = load_parent(p, l - 1, qidx * TK + i);
+                if (node < 0) continue;
+                const int parent = node / CR;
+                int lo = 0, hi = np;
+                while (lo < hi) { const int mid = (lo + hi) >> 1; if (par[mid] < parent) lo = mid + 1; else hi = mid; }
+                if (lo < np && par[lo] == parent) {
+                    const int j = lo * CR + node % CR;
+                    atomicOr(&selw[j >> 5], 1u << (j & 31));
+                }
+            }
         }
 #pragma unroll 1
         for (int c = first; c < nchunk; c += step) {

@@ -41,7 +41,7 @@ __global__ void __launch_bounds__(dq_warps<D, X3, NH>() * 32, dq_min_blocks<D, X
 
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, g = lane >> 2, r = lane & 3;
     const int W = blockDim.x >> 5;
-    const int qi = blockIdx.x * W + warp;
+    const int qi = (int)(gridDim.x - 1 - blockIdx.x) * W + warp;      // the longest walks first: they would be the tail of the launch
     const int sub = bp.sub0 + blockIdx.y, unit = sub / bp.nw;
     const int tl = (sub % bp.nw) * bp.subq + qi;
     if (qi >= bp.subq || tl >= p.Tq) return;
@@ -150,29 +150,6 @@ __global__ void __launch_bounds__(dq_warps<D, X3, NH>() * 32, dq_min_blocks<D, X
         if (np <= 0 || (l > 0 && nc <= TK)) continue;
         const int nchunk = (np + PPC - 1) / PPC;
         __syncwarp();
-        // this visit's place in its parent's list
-        int32_t* cnt = bp.cnt + (int64_t)blockIdx.y * bp.NK + bp.koff[l];
-        for (int i = lane; i < np; i += 32) {
-            const int x = (unsigned)par[i] < (unsigned)nblk ? par[i] : 0;
-            bp.rank[(int64_t)grp * bp.MV + bp.voff[l] + i] = atomicAdd(cnt + x, 1);
-        }
-        if (l > 0) {
-            for (int i = lane; i < (nc + 31) / 32; i += 32) selw[i] = 0u;
-            __syncwarp();
-            for (int i = lane; i < TK; i += 32) {
-                const int node = load_parent(p, l - 1, qidx * TK + i);
-                if (node < 0) continue;
-                const int parent = node / CR;
-                int lo = 0, hi = np;
-                while (lo < hi) { const int mid = (lo + hi) >> 1; if (par[mid] < parent) lo = mid + 1; else hi = mid; }
-                if (lo < np && par[lo] == parent) {
-                    const int j = lo * CR + node % CR;
-                    atomicOr(&selw[j >> 5], 1u << (j & 31));
-                }
-            }
-        }
-        __syncwarp();
-
         const int64_t blk0 = (int64_t)b * nblk * p.Hkv + hk;
         const unsigned char* kblk = reinterpret_cast<const unsigned char*>(p.blk[l]) + blk0 * C::BLOCK;
         const unsigned char* vblk = reinterpret_cast<const unsigned char*>(p.vkblk[l]) + blk0 * (C::PL * C::PART);
@@ -199,6 +176,27 @@ __global__ void __launch_bounds__(dq_warps<D, X3, NH>() * 32, dq_min_blocks<D, X
         for (; next < NSTG - 1; ++next) {
             if (next < nchunk) fill(next);
             ring.commit();
+        }
+        // this visit's place in its parent's list
+        int32_t* cnt = bp.cnt + (int64_t)blockIdx.y * bp.NK + bp.koff[l];
+        for (int i = lane; i < np; i += 32) {
+            const int x = (unsigned)par[i] < (unsigned)nblk ? par[i] : 0;
+            bp.rank[(int64_t)grp * bp.MV + bp.voff[l] + i] = atomicAdd(cnt + x, 1);
+        }
+        if (l > 0) {
+            for (int i = lane; i < (nc + 31) / 32; i += 32) selw[i] = 0u;
+            __syncwarp();
+            for (int i = lane; i < TK; i += 32) {
+                const int node = load_parent(p, l - 1, qidx * TK + i);
+                if (node < 0) continue;
+                const int parent = node / CR;
+                int lo = 0, hi = np;
+                while (lo < hi) { const int mid = (lo + hi) >> 1; if (par[mid] < parent) lo = mid + 1; else hi = mid; }
+                if (lo < np && par[lo] == parent) {
+                    const int j = lo * CR + node % CR;
+                    atomicOr(&selw[j >> 5], 1u << (j & 31));
+                }
+            }
         }
         const int visit0 = grp * bp.MV + bp.voff[l];
 #pragma unroll 1

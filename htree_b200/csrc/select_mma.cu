@@ -16,11 +16,11 @@ struct SelForm {
     static constexpr int DATA = PPC * KPART, TAB = D * 6, SLOT = DATA + PPC * TAB;
     // a table row is [cos | sin | -sin] in fp32, each part ordered [k-step pair][r][4]: the four lanes of a quad read 64 consecutive
     // bytes (rows in natural order cost 8 wavefronts a load, a third of the kernel's shared-memory traffic)
-#ifndef SEL_NSTG
-#define SEL_NSTG (SLOT > 4096 ? 2 : 3)
-#endif
-    static constexpr int NSTG = SEL_NSTG;
+    static constexpr int NSTG = SLOT > 4096 ? 2 : 3;
 };
+// Queries up to here take the longest walks first, so that these are not the tail of the call; in longer ones nearly all walks
+// have full length and the forward order was 2% faster (16384 to 65536 positions).
+constexpr int kSelReverse = 8192;
 constexpr int kSelSplitWarps = 8, kSelSplitKeys = 32 * 32 * kSelSplitWarps;      // SPLIT keeps 32 keys per thread
 
 // shared memory besides the rings: importances, chunk maxima, two parent lists, counters
@@ -117,8 +117,9 @@ select_mma_kernel(const __grid_constant__ AttnParams p) {
 
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, g = lane >> 2, r = lane & 3;
     const int W = blockDim.x >> 5;
-    const int tl = SPLIT ? (int)blockIdx.x : (int)(blockIdx.x * W + warp);
-    if (!SPLIT && tl >= p.Tq) return;
+    const int at = SPLIT ? (int)blockIdx.x : (int)(blockIdx.x * W + warp);
+    if (!SPLIT && at >= p.Tq) return;
+    const int tl = p.Tq <= kSelReverse ? p.Tq - 1 - at : at;
     const int t = p.t0 + tl;
     const int b = blockIdx.y / p.Hkv, hk = blockIdx.y % p.Hkv;
     const int G = p.G, TK = p.TK, L = p.L, maxc = TK * CR;

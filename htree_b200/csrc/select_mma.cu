@@ -241,13 +241,17 @@ select_mma_kernel(const __grid_constant__ AttnParams p) {
             float M = -INFINITY;
             for (int a = lane; a < np; a += 32) M = fmaxf(M, cmax[a]);
             M = warp_max(M);
+            if constexpr (SPLIT) __syncthreads();           // every warp has read the maxima before they become factors
             // Exact Top-K: search for the TK-th largest key (non-negative floats order like their bit patterns) by counting the keys
             // at or above a probe, in the bracket that the smallest and the largest key span.  The next probe is where the logit of the
             // count, interpolated over the bit patterns, reaches TK, every fourth one the middle: 5 to 8 counts where bisecting the
             // 31 bits takes 13 to 21.
             uint32_t* key = reinterpret_cast<uint32_t*>(imp);
+            __syncwarp();
+            for (int a = SPLIT ? (int)threadIdx.x : lane; a < np; a += nthr) cmax[a] = __expf(cmax[a] - M);
+            sync();
             auto value = [&](int j) {
-                const float v = imp[j] * __expf(cmax[j / CR] - M);
+                const float v = imp[j] * cmax[j / CR];
                 return __float_as_uint(j == rp ? kForcedImportance : v);
             };
             const bool in_regs = SPLIT || maxc <= 1024;

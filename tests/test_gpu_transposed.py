@@ -1,0 +1,90 @@
+"""The kernels that put candidates on the matrix rows and heads on the columns (operand blocks, selection, accumulation, the
+two-pass backward) against the kernels that gather rows, at the sizes where they can go wrong: one position, one position
+more or less than a block of children, ragged lengths, 1 / 8 / 9 / 16 heads per group, both branchings, every head size and type."""
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+DEV = "cuda"
+BF, HF, FP = torch.bfloat16, torch.float16, torch.float32
+
+
+def _inputs(dt, B, T, Hkv, G, D, clustered=False):
+    g = torch.Generator(device=DEV).manual_seed(T * 131 + G * 7 + D)
+    q, k, v, dO = (torch.randn(B, T, h, D, device=DEV, dtype=dt, generator=g) for h in (Hkv * G, Hkv, Hkv, Hkv * G))
+    if clustered:
+        k = (k.float() + 3 * torch.randn(B, T, Hkv, 4, device=DEV, generator=g) @ torch.randn(4, D, device=DEV, generator=g)).to(dt)
+    return q, k, v, dO
+
+
+def _rel(a, b):
+    return ((a.float() - b.float()).norm() / b.float().norm().clamp_min(1e-20)).item()
+
+
+@pytest.mark.parametrize("dt,D,CR,G,B,T,TK,MTN", [
+    (BF, 128, 16, 16, 1, 1, 16, 64), (BF, 128, 16, 9, 2, 257, 16, 64), (BF, 128, 16, 8, 1, 3001, 32, 128),
+    (HF, 128, 8, 16, 1, 1777, 16, 64), (HF, 64, 8, 1, 2, 255, 16, 64), (BF, 64, 16, 16, 1, 1777, 512, 8192),
+    (FP, 64, 8, 8, 1, 1777, 16, 64), (FP, 64, 16, 9, 1, 17, 16, 64), (FP, 128, 16, 4, 1, 3001, 32, 64), (FP, 128, 8, 16, 1, 500, 16, 64),
+    (HF, 32, 16, 4, 1, 3001, 512, 512), (BF, 32, 8, 12, 1, 1777, 16, 64), (FP, 32, 16, 1, 2, 16, 16, 64)])
+def test_forward_and_backward(dt, D, CR, G, B, T, TK, MTN, monkeypatch):
+    import htree_b200 as ht
+    from htree_b200 import ops
+    q, k, v, dO = _inputs(dt, B, T, 2, G, D)
+    out, ctx = ht.htree_forward(q, k, v, CR, MTN, TK, _save_for_backward=True)
+    assert ctx["layers_v_blk"] is not None, "these sizes are meant to take the operand blocks"
+    ref, rctx = ht.htree_forward(q, k, v, CR, MTN, TK, _save_for_backward=True, _force_generic=True)
+    alone = ht.htree_forward(q, k, v, CR, MTN, TK)      # inference splits a group over eight warps where there are few groups
+    assert torch.equal(alone, out) if B * T * 2 > 296 else _rel(alone, out) < (2e-6 if dt == FP else 4e-3)
+    # outputs where the selections agree (16-bit scores have half-precision operands: a few near-ties fall the other way)
+    exact = dt == FP or D == 32
+    same = torch.stack([(ctx["per_layer_parents"][l] == rctx["per_layer_parents"][l]).all(-1) for l in range(ctx["num_layers"])]).all(0)
+    assert same.float().mean().item() >= (1.0 if exact else 0.98)
+    rows = same.repeat_interleave(G, -1)
+    assert _rel(out[rows], ref[rows]) < (1e-5 if dt == FP else 4e-3)
+    # gradients from the same saved state
+    ours, gen = ht.htree_backward(dO, q, out, ctx), ht.htree_backward(dO, q, out, ctx, _force_generic=True)
+    for a, b in zip(ours, gen):
+        # (one position attends to itself alone: P = 1 and dq, dk are zero up to rounding)
+        assert (a - b).abs().max().item() < 1e-2 if T == 1 else _rel(a, b) < (1e-5 if exact else 3e-3)
+    # several windows of queries instead of one
+    monkeypatch.setattr(ops, "BACKWARD_MAX_BYTES", 1 << 22)
+    parts = ht.htree_backward(dO, q, out, ctx)
+    assert torch.equal(parts[0], ours[0])
+    assert T == 1 or max(_rel(a, b) for a, b in zip(parts[1:], ours[1:])) < 1e-5
+    torch.cuda.synchronize()
+    ops.check_status()
+
+
+@pytest.mark.parametrize("dt,D,CR,G,B,T,TK,MTN,clustered", [
+    (BF, 128, 16, 16, 1, 140, 16, 64, False),      # fewer than 296 groups: eight warps a group
+    (BF, 128, 16, 16, 1, 12000, 512, 2048, False), # lists too long for one warp
+    (BF, 128, 16, 12, 1, 9001, 32, 256, True), (HF, 128, 8, 8, 1, 9001, 32, 128, False), (BF, 64, 8, 4, 1, 5000, 64, 64, True),
+    (HF, 64, 16, 9, 2, 1777, 16, 64, False), (FP, 64, 8, 1, 1, 1777, 16, 64, False), (FP, 64, 16, 16, 1, 5000, 64, 64, True)])
+def test_selections_bit_identical(dt, D, CR, G, B, T, TK, MTN, clustered):
+    import htree_b200 as ht
+    from htree_b200 import ops
+    q, k, v, _ = _inputs(dt, B, T, 2, G, D, clustered)
+    _, ctx = ht.htree_forward(q, k, v, CR, MTN, TK, _save_for_backward=True)
+    gathered = ops.recompute_parents(q, ctx["layers_k"], ctx["layers_v"], ctx["cos_cache"], ctx["sin_cache"], CR, TK, MTN, ctx["scale"], ctx["layers_k_rot"])
+    for l, want in gathered.items():
+        assert torch.equal(ctx["per_layer_parents"][l], want), f"level {l}"
+    w = min(5, T)
+    _, cw = ht.htree_forward(q[:, T - w:].contiguous(), k, v, CR, MTN, TK, _q_offset=T - w, _save_for_backward=True)
+    for l, want in gathered.items():
+        assert torch.equal(cw["per_layer_parents"][l], want[:, T - w:]), f"level {l}, last positions alone"
+    torch.cuda.synchronize()
+    ops.check_status()
+
+
+@pytest.mark.parametrize("dt,D,CR,G,T,TK,MTN,W", [
+    (BF, 128, 16, 16, 20000, 64, 64, 1), (HF, 64, 16, 8, 9001, 16, 64, 17), (FP, 64, 8, 8, 9001, 32, 128, 3), (HF, 32, 16, 4, 9001, 16, 64, 1),
+    (BF, 128, 16, 16, 4000, 16, 64, 125), (BF, 128, 16, 16, 4000, 16, 64, 8)])      # either side of 2 * W * TK = parents
+def test_few_queries(dt, D, CR, G, T, TK, MTN, W):
+    import htree_b200 as ht
+    from htree_b200 import ops
+    q, k, v, _ = _inputs(dt, 1, T, 2, G, D)
+    full = ht.htree_forward(q, k, v, CR, MTN, TK)
+    part = ht.htree_forward(q[:, T - W:].contiguous(), k, v, CR, MTN, TK, _q_offset=T - W)
+    assert _rel(part, full[:, T - W:]) < (2e-6 if dt == FP else 4e-3)
+    torch.cuda.synchronize()
+    ops.check_status()

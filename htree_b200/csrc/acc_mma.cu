@@ -147,22 +147,30 @@ acc_mma_kernel(const __grid_constant__ AttnParams p) {
                     S[h][2] = c1 ? S[h][2] : -INFINITY; S[h][3] = c1 ? S[h][3] : -INFINITY;
                 }
             }
-            bool move = false;
-            float mx[NH][2];
+            // exponents relative to the reference; fp32 storage keeps the plain difference (an exponent re-based by log2 e rounds
+            // at 1e-6 relative)
+            float ex[NH][4];
+            auto exponents = [&]() {
+#pragma unroll
+                for (int h = 0; h < NH; ++h)
+#pragma unroll
+                    for (int i = 0; i < 4; ++i) ex[h][i] = X3 ? S[h][i] - m_run[h][i & 1] : fmaf(S[h][i], kLog2e, -m_run2[h][i & 1]);
+            };
+            exponents();
+            float top = ex[0][0];
 #pragma unroll
             for (int h = 0; h < NH; ++h)
 #pragma unroll
                 for (int e = 0; e < 2; ++e) {
-                    mx[h][e] = fmaxf(S[h][e], S[h][2 + e]);
-                    m_true[h][e] = fmaxf(m_true[h][e], mx[h][e]);
-                    move = move || mx[h][e] > m_run[h][e] + kLazyMax;
+                    top = fmaxf(top, fmaxf(ex[h][e], ex[h][2 + e]));
+                    m_true[h][e] = fmaxf(m_true[h][e], fmaxf(S[h][e], S[h][2 + e]));
                 }
-            if (__any_sync(0xffffffffu, move)) {
+            if (__any_sync(0xffffffffu, top > (X3 ? kLazyMax : kLazyMax * kLog2e))) {
 #pragma unroll
                 for (int h = 0; h < NH; ++h)
 #pragma unroll
                     for (int e = 0; e < 2; ++e) {
-                        float m = mx[h][e];
+                        float m = fmaxf(S[h][e], S[h][2 + e]);
                         m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, 4));
                         m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, 8));
                         m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, 16));
@@ -173,16 +181,14 @@ acc_mma_kernel(const __grid_constant__ AttnParams p) {
 #pragma unroll
                         for (int i = 0; i < MT; ++i) { O[h][i][e] *= f; O[h][i][2 + e] *= f; }
                     }
+                exponents();
             }
             uint32_t pb[NH][2], pl[X3 ? NH : 1][2];
 #pragma unroll
             for (int h = 0; h < NH; ++h) {
                 float P[4];
 #pragma unroll
-                for (int i = 0; i < 4; ++i) {
-                    // fp32 storage keeps the plain difference (an exponent re-based by log2 e rounds at 1e-6 relative)
-                    P[i] = X3 ? __expf(S[h][i] - m_run[h][i & 1]) : ex2_approx(fmaf(S[h][i], kLog2e, -m_run2[h][i & 1]));
-                }
+                for (int i = 0; i < 4; ++i) P[i] = X3 ? __expf(ex[h][i]) : ex2_approx(ex[h][i]);
                 s_run[h][0] += P[0] + P[2];
                 s_run[h][1] += P[1] + P[3];
                 if constexpr (X3) {

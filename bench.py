@@ -531,7 +531,7 @@ def main():
 
         def select_only():
             return hops.recompute_parents(q, fctx["layers_k"], fctx["layers_v"], fctx["cos_cache"], fctx["sin_cache"], CR, TK, MTN,
-                                          fctx["scale"], fctx["layers_k_rot"])
+                                          fctx["scale"], layers_v_blk=fctx["layers_v_blk"], rope_base=10000.0)
 
         select_only()
         torch.cuda.synchronize()
@@ -545,14 +545,14 @@ def main():
         del fctx
         torch.cuda.empty_cache()
 
-    # ---- streaming kernels: mean-pool tree build + key pre-rotation, timed alone (inputs larger than L2) ----
+    # ---- streaming kernel: mean-pool tree and operand blocks of every level, timed alone (inputs larger than L2) ----
     sa = torch.cuda.Event(enable_timing=True); sb = torch.cuda.Event(enable_timing=True)
-    hops.build_tree(k, v, CR, MTN, 10000.0)
+    hops.build_operands(k, v, CR, MTN, 10000.0, backward=bool(bwd))
     torch.cuda.synchronize()
     n_tb = 10
     sa.record()
     for _ in range(n_tb):
-        hops.build_tree(k, v, CR, MTN, 10000.0)
+        hops.build_operands(k, v, CR, MTN, 10000.0, backward=bool(bwd))
     sb.record()
     torch.cuda.synchronize()
     tree_ms = sa.elapsed_time(sb) / n_tb
@@ -685,18 +685,17 @@ def main():
                 "backward_tflops": (cm["flops_bwd"] / world / (bwd_ms * 1e-3) / 1e12) if bwd else None,
                 "forward_requested_gather_gbs": cm["gather_bytes_fwd"] / world / (fwd_ms * 1e-3) / 1e9,
                 "forward_compulsory_hbm_frac": cm["bytes_fwd"] / world / (fwd_ms * 1e-3) / 1e9 / pk["hbm_gbs"]}
-    # what actually bounds the two attention kernels: gathered rows per second (forward) and bytes of fp32 reductions
-    # into the dK/dV level buffers per second (backward: 2 * D floats per accumulated row), against ceilings measured now
+    # what bounds the kernels: whole operand blocks gathered from L2 by the two forward launches and the backward's first
+    # pass, and the visit records that pass leaves for the second, against the gather ceiling measured now
     limits = measure_limits(dev)
     if "l2_gather_gbs" in limits:
         limits["forward_gather_gbs"] = roofline["forward_requested_gather_gbs"]
         limits["forward_gather_frac"] = limits["forward_gather_gbs"] / limits["l2_gather_gbs"]
     if sel_ms is not None and "l2_gather_gbs" in limits and es_bytes(c) == 2 and D == 128 and CR == 16:
-        # bytes the two kernels actually move from L2 per launch: the selection kernel gathers a chunk's pre-rotated keys
-        # and reads its two fp32 table rows; the pipelined accumulation kernel copies a chunk's blocked keys, blocked
-        # values and two packed-half table rows into shared memory
+        # bytes per chunk: the selection copies the keys of one parent's block and a row of the fp32 rotary table (three
+        # parts), the accumulation keys, values and a row of the half-precision table
         acc_ms = fwd_ms - tree_ms - sel_ms
-        sel_bytes = cm["selection_chunks"] / world * (CR * D * 2 + 2 * (D // 2) * 4)
+        sel_bytes = cm["selection_chunks"] / world * (CR * D * 2 + 3 * (D // 2) * 4)
         acc_bytes = cm["accumulation_chunks"] / world * (2 * CR * D * 2 + 2 * (D // 2) * 2)
         limits["selection_kernel_ms"] = sel_ms
         limits["accumulation_kernel_ms"] = acc_ms
@@ -704,21 +703,25 @@ def main():
         limits["accumulation_kernel_l2_gbs"] = acc_bytes / (acc_ms * 1e-3) / 1e9
         limits["selection_kernel_l2_frac"] = limits["selection_kernel_l2_gbs"] / limits["l2_gather_gbs"]
         limits["accumulation_kernel_l2_frac"] = limits["accumulation_kernel_l2_gbs"] / limits["l2_gather_gbs"]
-    if bwd and "l2_reduction_gbs" in limits:
-        red_bytes = cm["accumulated_rows"] * 2 * D * 4 / world
-        limits["backward_reduction_gbs"] = red_bytes / (bwd_ms * 1e-3) / 1e9
-        limits["backward_reduction_frac"] = limits["backward_reduction_gbs"] / limits["l2_reduction_gbs"]
+    if bwd and "l2_gather_gbs" in limits and es_bytes(c) == 2 and D == 128 and CR == 16:
+        # per chunk: the first pass copies key and value blocks and a table row and writes a record of P and one of dS; the
+        # second reads both back with the query's blocked heads, its output gradient and a table row
+        record, heads = CR * (8 if H // Hkv <= 8 else 16) * 2, (8 if H // Hkv <= 8 else 16) * D * 2
+        per_chunk = (2 * CR * D * 2 + D * 2 + 2 * record) + (2 * record + 2 * heads + D * 2)
+        limits["backward_l2_gbs"] = cm["accumulation_chunks"] / world * per_chunk / (bwd_ms * 1e-3) / 1e9
+        limits["backward_l2_frac"] = limits["backward_l2_gbs"] / limits["l2_gather_gbs"]
     es = 4 if c["dtype"] == "float32" else 2
     lv_sizes = cm["levels"]
     n_rows = B * Hkv if (seq_mode or world == 1) else len(units)
-    tree_bytes = es * n_rows * 2 * D * sum(lv_sizes[i] + lv_sizes[i + 1] for i in range(len(lv_sizes) - 1))     # pool K and V
-    if es == 2:
-        copies = 1 + (1 if D in (64, 128) and CR in (8, 16) else 0) + (1 if D == 128 and CR == 16 else 0)     # K -> K', V -> V^, K' -> K'^
-        tree_bytes += copies * 2 * 2 * n_rows * D * sum(lv_sizes)                                                # each: read + write of every level
-    streaming = {"kernels": "tree_build_kernel + rotate_keys / block_values / block_keys kernels (all levels, rank 0)", "ms": tree_ms,
+    # every level is read once (K and V), pooled rows are written, and each level's operand blocks: keys and values in half
+    # precision or as hi + lo half pairs, with eight children split-half keys twice, and the values once more for a backward
+    pairs = es == 4 or D == 32
+    block_bytes = 2 * D * (2 if pairs else 1) * ((3 if pairs and CR == 8 else 2) + (1 if bwd else 0))
+    tree_bytes = n_rows * (2 * es * D * (sum(lv_sizes) + sum(lv_sizes[1:])) + block_bytes * sum(lv_sizes))
+    streaming = {"kernels": "pack_blocks_kernel (pooling, rotation and operand blocks of all levels, rank 0)", "ms": tree_ms,
                  "algorithmic_bytes": tree_bytes, "achieved": tree_bytes / (tree_ms * 1e-3) / 1e9, "unit": "GB/s",
                  "peak": pk["hbm_gbs"], "frac": tree_bytes / (tree_ms * 1e-3) / 1e9 / pk["hbm_gbs"],
-                 "note": "CUDA events around 10 back-to-back builds, includes launch gaps between the per-level kernels"}
+                 "note": "CUDA events around 10 back-to-back builds, includes allocations and launch gaps between the per-level kernels"}
     line = {"metric": metric, "value": B * T / (ms_step * 1e-3), "unit": "tokens/s", "n_gpus": world,
             "steps": args.steps, "warmup": max(3, args.warmup), "ms_per_step": ms_step, "higher_is_better": True,
             "scaling": "strong", "vs_baseline": None, "dtype": "bf16" if c["dtype"] == "bfloat16" else c["dtype"],

@@ -21,11 +21,25 @@ struct SelForm {
 // Queries up to here take the longest walks first, so that these are not the tail of the call; in longer ones nearly all walks
 // have full length and the forward order was 2% faster (16384 to 65536 positions).
 constexpr int kSelReverse = 8192;
+// Above this many candidates a group gets a whole block: their importances (16 KB for 4096) leave room for few warps per SM where
+// each has its own, below it the block-wide Top-K costs more in barriers than it gives.  128-wide heads, one warp against eight:
+// 2500 candidates 2.20 / 2.91 ms (40000 positions, 16 heads), 5000 candidates 11.3 / 9.3 ms (80000 positions).
+constexpr int kSelLong = 4096;
 constexpr int kSelSplitWarps = 8, kSelSplitKeys = 32 * 32 * kSelSplitWarps;      // SPLIT keeps 32 keys per thread
 
+// The most candidates a group has on any level that selects: the children of TK parents, or of all there are.
+__host__ __device__ __forceinline__ int sel_max_candidates(const AttnParams& p, int CR) {
+    int most = CR;
+    for (int l = 1; l < p.L; ++l) {
+        const int parents = (p.ln[l] + CR - 1) / CR;
+        const int n = (parents < p.TK ? parents : p.TK) * CR;
+        if (n > most) most = n;
+    }
+    return most;
+}
 // shared memory besides the rings: importances, chunk maxima, two parent lists, counters
-__host__ __device__ inline size_t sel_scratch_bytes(int TK, int CR) {
-    return ((size_t)TK * CR * 4 + (size_t)TK * 4 + 8 * (size_t)TK + 16 + 64 + 127) & ~size_t(127);
+__host__ __device__ inline size_t sel_scratch_bytes(int maxc, int TK, int CR) {
+    return ((size_t)maxc * 4 + (size_t)(maxc / CR) * 4 + 8 * (size_t)TK + 16 + 64 + 127) & ~size_t(127);
 }
 
 template <int D, bool X3, int NH>
@@ -122,19 +136,19 @@ select_mma_kernel(const __grid_constant__ AttnParams p) {
     const int tl = p.Tq <= kSelReverse ? p.Tq - 1 - at : at;
     const int t = p.t0 + tl;
     const int b = blockIdx.y / p.Hkv, hk = blockIdx.y % p.Hkv;
-    const int G = p.G, TK = p.TK, L = p.L, maxc = TK * CR;
+    const int G = p.G, TK = p.TK, L = p.L, maxc = sel_max_candidates(p, CR);
     const int first = SPLIT ? warp : 0, step = SPLIT ? W : 1;
     const int tid = SPLIT ? (int)threadIdx.x : lane, nthr = SPLIT ? kSelSplitWarps * 32 : 32;   // the threads that share a group
     auto sync = [&]() { if constexpr (SPLIT) __syncthreads(); else __syncwarp(); };
 
-    const size_t scratch = sel_scratch_bytes(TK, CR);
+    const size_t scratch = sel_scratch_bytes(maxc, TK, CR);
     unsigned char* wbase = smem_raw + (SPLIT ? warp * Ring::kBytes : warp * (Ring::kBytes + scratch));
     unsigned char* sbase = SPLIT ? smem_raw + W * Ring::kBytes : wbase + Ring::kBytes;
     Ring ring;
     ring.init(wbase);
     float* imp = reinterpret_cast<float*>(sbase);
     float* cmax = imp + maxc;
-    int32_t* par = reinterpret_cast<int32_t*>(cmax + TK);
+    int32_t* par = reinterpret_cast<int32_t*>(cmax + maxc / CR);
     int32_t* nxt = par + TK;
     int* cnt = reinterpret_cast<int*>(nxt + TK);       // SPLIT: three rotating counters
     int* wtot = cnt + 4;                               // SPLIT: one per warp
@@ -367,13 +381,13 @@ template <typename T, int D, bool X3, int NH, int CR>
 static int launch_select_cr(const AttnParams& p, cudaStream_t st) {
     using SF = SelForm<D, X3, CR>;
     using Ring = WarpRing<SF::NSTG, SF::SLOT>;
-    const size_t scratch = sel_scratch_bytes(p.TK, CR), limit = 227 * 1024;
+    const int maxc = sel_max_candidates(p, CR);
+    const size_t scratch = sel_scratch_bytes(maxc, p.TK, CR), limit = 227 * 1024;
     const int64_t groups = (int64_t)p.Tq * p.B * p.Hkv;
     // A block of 8 warps per group where there are few groups (below two per SM a single warp's walk over its chunks is the whole
-    // time of the call), and for long lists: 512 parents of 16 are 32 KB of importances, which one group can have per SM-quarter
-    // but not one warp in sixteen.
+    // time of the call), and for long lists: (above kSelLong).
     const size_t split_smem = kSelSplitWarps * Ring::kBytes + scratch;
-    if ((groups <= 2 * 148 || p.TK * CR > 1024) && p.TK * CR <= kSelSplitKeys && split_smem <= limit) {
+    if ((groups <= 2 * 148 || maxc > kSelLong) && maxc <= kSelSplitKeys && split_smem <= limit) {
         auto* k = select_mma_kernel<T, D, X3, NH, CR, true>;
         static SmemLimit shared;
         const cudaError_t e = shared.raise((const void*)k, split_smem);
@@ -412,7 +426,7 @@ bool select_blk_supported(const AttnParams& p, int dtype) {
     for (int l = 1; l < p.L; ++l) if (!p.blk[l]) return false;
     const bool x3 = dtype == HTREE_F32;
     const size_t ring = 3 * ((x3 ? 2 : 1) * (size_t)p.K * 32 + 8 * p.K) + 128;
-    return ring + sel_scratch_bytes(p.TK, p.CR) <= 227 * 1024;
+    return ring + sel_scratch_bytes(sel_max_candidates(p, p.CR), p.TK, p.CR) <= 227 * 1024;
 }
 
 int launch_select_blk(const AttnParams& p, int dtype, cudaStream_t st) {

@@ -41,12 +41,13 @@ acc_mma_kernel(const __grid_constant__ AttnParams p) {
     const int first = SPLIT ? warp : 0, step = SPLIT ? W : 1;         // this warp's chunks of every level
 
     // per warp: ring, parent list, kept-candidate bits
-    const size_t per_warp = (Ring::kBytes + sizeof(int32_t) * TK + sizeof(uint32_t) * ((TK * CR + 31) / 32) + 127) & ~size_t(127);
+    const WalkLayout lay = walk_layout(p, CR);
+    const size_t per_warp = walk_warp_bytes<Ring>(lay);
     unsigned char* wbase = smem_raw + warp * per_warp;
     Ring ring;
     ring.init(wbase);
-    int32_t* par = reinterpret_cast<int32_t*>(wbase + Ring::kBytes);
-    uint32_t* selw = reinterpret_cast<uint32_t*>(par + TK);
+    const ParentList par{wbase + Ring::kBytes, lay.narrow};
+    uint32_t* selw = reinterpret_cast<uint32_t*>(wbase + Ring::kBytes + lay.list);
 
     const int64_t hbase = ((int64_t)b * p.Tq + tl) * p.H + (int64_t)hk * G;
     const int64_t qidx = ((int64_t)b * p.Tq + tl) * p.Hkv + hk;
@@ -73,9 +74,8 @@ acc_mma_kernel(const __grid_constant__ AttnParams p) {
     for (int l = L - 1; l >= 0; --l) {
         const int Nl = p.ln[l];
         __syncwarp();
-        int np = 0;
-        for (int i = lane; i < TK; i += 32) { const int x = load_parent(p, l, qidx * TK + i); par[i] = x; np += x >= 0; }
-        np = __reduce_add_sync(0xffffffffu, np);
+        const int nblk = (Nl + CR - 1) / CR;
+        const int np = par.load(p, l, qidx * TK, nblk, 4, lane);
         const int rc = (int)(((int64_t)t / p.lpow[l]) % CR);
         const int nc = (np - 1) * CR + rc + 1, rp = nc - 1;
         if (l > 0 && nc <= TK) continue;                              // every candidate is kept: nothing to accumulate
@@ -83,18 +83,15 @@ acc_mma_kernel(const __grid_constant__ AttnParams p) {
         const int nchunk = (np + PPC - 1) / PPC;
         __syncwarp();
 
-        const int nblk = (Nl + CR - 1) / CR;
         const int64_t bstride = (int64_t)p.Hkv * C::BLOCK;
         const unsigned char* blk = reinterpret_cast<const unsigned char*>(p.blk[l]) + ((int64_t)b * nblk * p.Hkv + hk) * C::BLOCK;
         const unsigned char* tab = reinterpret_cast<const unsigned char*>(p.tab);
         auto fill = [&](int c) {                                      // chunk c of this level
-            int p0 = par[c * PPC];
-            if ((unsigned)p0 >= (unsigned)nblk) { if (p.status) atomicOr(p.status, 4); p0 = 0; }
+            const int p0 = par[c * PPC];
             if constexpr (CR == 16) {
                 ring.template copy<C::DATA>(0, blk + p0 * bstride, lane);
             } else {
-                int p1 = c * PPC + 1 < np ? par[c * PPC + 1] : p0;    // past the end of the list: masked, any finite block
-                if ((unsigned)p1 >= (unsigned)nblk) { if (p.status) atomicOr(p.status, 4); p1 = 0; }
+                const int p1 = c * PPC + 1 < np ? par[c * PPC + 1] : p0;  // past the end of the list: masked, any finite block
                 ring.template copy<C::DATA / 2>(0, blk + p0 * bstride, lane);
                 ring.template copy<C::DATA / 2>(C::DATA / 2, blk + p1 * bstride + C::ODD, lane);
             }
@@ -315,7 +312,7 @@ template <typename T, int D, bool X3, int NH, int CR>
 static int launch_acc_cr(const AttnParams& p, cudaStream_t st) {
     using C = TForm<D, X3, CR>;
     using Ring = WarpRing<acc_stages<D, X3>(), C::SLOT>;
-    const size_t per_warp = (Ring::kBytes + sizeof(int32_t) * p.TK + sizeof(uint32_t) * ((p.TK * CR + 31) / 32) + 127) & ~size_t(127);
+    const size_t per_warp = walk_warp_bytes<Ring>(walk_layout(p, CR));
     const size_t limit = 227 * 1024;
     // Few groups: one block of 8 warps per group.  Below two groups per SM the chip has room for all their warps at once, and
     // a single warp's walk over its chunks (about 1 us each) would be the whole time of the call.  Calls whose state the
@@ -367,7 +364,7 @@ bool acc_mma_supported(const AttnParams& p, int dtype) {
     if (!pack_supported(dtype, p.K, p.V, p.CR) || p.G > 16 || !p.tab) return false;
     for (int l = 0; l < p.L; ++l) if (!p.blk[l]) return false;
     const size_t slot = (pack_split(dtype, p.K) ? 2 : 1) * (size_t)p.K * 64 + 4 * p.K;
-    return 3 * slot + 512 + 4 * (size_t)p.TK + (size_t)p.TK * p.CR / 8 <= 227 * 1024;
+    return 3 * slot + 512 + walk_layout(p, p.CR).list + walk_layout(p, p.CR).bits <= 227 * 1024;
 }
 
 int launch_acc_mma(const AttnParams& p, int dtype, cudaStream_t st) {

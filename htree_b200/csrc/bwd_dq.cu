@@ -20,12 +20,6 @@ constexpr int dq_warps() { return D == 128 && !X3 && NH == 2 ? 1 : 4; }
 template <int D, bool X3, int NH>
 constexpr int dq_min_blocks() { return D == 32 && NH == 1 ? 4 : (D == 128 && (X3 || NH == 2)) ? (X3 ? 2 : 12) : (X3 && NH == 2) ? 2 : 3; }
 
-// ring, parent list, kept-candidate bits
-template <typename Ring>
-__host__ __device__ inline size_t dq_warp_bytes(int TK, int CR) {
-    return (Ring::kBytes + sizeof(int32_t) * TK + sizeof(uint32_t) * ((TK * CR + 31) / 32) + 127) & ~size_t(127);
-}
-
 template <typename T, int D, bool X3, int NH, int CR>
 __global__ void __launch_bounds__(dq_warps<D, X3, NH>() * 32, dq_min_blocks<D, X3, NH>()) bwd_dq_kernel(const __grid_constant__ BwdParams bp) {
     using C = TForm<D, X3, CR>;
@@ -50,12 +44,13 @@ __global__ void __launch_bounds__(dq_warps<D, X3, NH>() * 32, dq_min_blocks<D, X
     const int G = p.G, TK = p.TK, L = p.L;
     const int grp = blockIdx.y * bp.subq + qi;
 
-    const size_t per_warp = dq_warp_bytes<Ring>(TK, CR);
+    const WalkLayout lay = walk_layout(p, CR);
+    const size_t per_warp = walk_warp_bytes<Ring>(lay);
     unsigned char* wbase = smem_raw + warp * per_warp;
     Ring ring;
     ring.init(wbase);
-    int32_t* par = reinterpret_cast<int32_t*>(wbase + Ring::kBytes);
-    uint32_t* selw = reinterpret_cast<uint32_t*>(par + TK);
+    const ParentList par{wbase + Ring::kBytes, lay.narrow};
+    uint32_t* selw = reinterpret_cast<uint32_t*>(wbase + Ring::kBytes + lay.list);
     const int64_t hbase = ((int64_t)b * p.Tq + tl) * p.H + (int64_t)hk * G;
     const int64_t qidx = ((int64_t)b * p.Tq + tl) * p.Hkv + hk;
 
@@ -142,9 +137,7 @@ __global__ void __launch_bounds__(dq_warps<D, X3, NH>() * 32, dq_min_blocks<D, X
         const int Nl = p.ln[l];
         const int nblk = (Nl + CR - 1) / CR;
         __syncwarp();
-        int np = 0;
-        for (int i = lane; i < TK; i += 32) { const int x = load_parent(p, l, qidx * TK + i); par[i] = x; np += x >= 0; }
-        np = __reduce_add_sync(0xffffffffu, np);
+        const int np = par.load(p, l, qidx * TK, nblk, 8, lane);
         const int rc = (int)(((int64_t)t / p.lpow[l]) % CR);
         const int nc = (np - 1) * CR + rc + 1, rp = nc - 1;
         if (np <= 0 || (l > 0 && nc <= TK)) continue;
@@ -156,13 +149,11 @@ __global__ void __launch_bounds__(dq_warps<D, X3, NH>() * 32, dq_min_blocks<D, X
         auto fill = [&](int c) {
             constexpr int PB = C::PL * C::PART;
             const int64_t kstride = (int64_t)p.Hkv * C::BLOCK, vstride = (int64_t)p.Hkv * PB;
-            int p0 = par[c * PPC];
-            if ((unsigned)p0 >= (unsigned)nblk) { if (p.status) atomicOr(p.status, 8); p0 = 0; }
+            const int p0 = par[c * PPC];
             ring.template copy<PB>(0, kblk + p0 * kstride, lane);
             ring.template copy<PB>(C::V_OFF, vblk + p0 * vstride, lane);
             if constexpr (CR == 8) {
-                int p1 = c * PPC + 1 < np ? par[c * PPC + 1] : p0;
-                if ((unsigned)p1 >= (unsigned)nblk) { if (p.status) atomicOr(p.status, 8); p1 = 0; }
+                const int p1 = c * PPC + 1 < np ? par[c * PPC + 1] : p0;
                 ring.template copy<PB>(C::K2_OFF, kblk + p1 * kstride + 2 * C::ODD, lane);
                 ring.template copy<PB>(C::V2_OFF, vblk + p1 * vstride, lane);
             }
@@ -180,8 +171,7 @@ __global__ void __launch_bounds__(dq_warps<D, X3, NH>() * 32, dq_min_blocks<D, X
         // this visit's place in its parent's list
         int32_t* cnt = bp.cnt + (int64_t)blockIdx.y * bp.NK + bp.koff[l];
         for (int i = lane; i < np; i += 32) {
-            const int x = (unsigned)par[i] < (unsigned)nblk ? par[i] : 0;
-            bp.rank[(int64_t)grp * bp.MV + bp.voff[l] + i] = atomicAdd(cnt + x, 1);
+            bp.rank[(int64_t)grp * bp.MV + bp.voff[l] + i] = atomicAdd(cnt + par[i], 1);
         }
         if (l > 0) {
             for (int i = lane; i < (nc + 31) / 32; i += 32) selw[i] = 0u;
@@ -388,8 +378,7 @@ template <typename T, int D, bool X3, int NH, int CR>
 static int launch_dq_cr(const BwdParams& bp, cudaStream_t st) {
     using C = TForm<D, X3, CR>;
     using Ring = WarpRing<dq_stages<D, X3>(), C::SLOT>;
-    const int TK = bp.a.TK;
-    const size_t per_warp = dq_warp_bytes<Ring>(TK, CR);
+    const size_t per_warp = walk_warp_bytes<Ring>(walk_layout(bp.a, CR));
     constexpr int max_w = dq_warps<D, X3, NH>(), max_warps = max_w * dq_min_blocks<D, X3, NH>();
     int W = 1, best = 0;
     for (int w = max_w; w >= 1; w >>= 1) {

@@ -340,4 +340,39 @@ struct WarpRing {
     __device__ __forceinline__ void idle() const { asm volatile("cp.async.wait_all;\n" ::: "memory"); }
 };
 
+// A query's parent list of one level in shared memory, 16 bits an entry where every level's parents can be numbered with them
+// (4 KB against 2 KB a warp matter with 512 nodes per layer, where lists and bits decide how many warps share an SM).
+struct ParentList {
+    unsigned char* at;
+    bool narrow;
+    __device__ __forceinline__ int operator[](int i) const {
+        return narrow ? (int)reinterpret_cast<const uint16_t*>(at)[i] : reinterpret_cast<const int32_t*>(at)[i];
+    }
+    // from the selections: returns the number of parents; entries that are no parent of the level become 0 and set `bit`
+    __device__ __forceinline__ int load(const AttnParams& p, int l, int64_t list, int nblk, int bit, int lane) const {
+        int np = 0;
+        for (int i = lane; i < min(p.TK, nblk); i += 32) {
+            int x = load_parent(p, l, list + i);
+            if (x < 0) continue;
+            ++np;
+            if (x >= nblk) { if (p.status) atomicOr(p.status, bit); x = 0; }
+            if (narrow) reinterpret_cast<uint16_t*>(at)[i] = (uint16_t)x; else reinterpret_cast<int32_t*>(at)[i] = x;
+        }
+        return __reduce_add_sync(0xffffffffu, np);
+    }
+};
+// What the walk over a level's candidates keeps per warp beside the ring: the parent list and one bit per candidate of a level
+// that selects.  Both are bounded by the parents that the levels have.
+struct WalkLayout { int list, bits; bool narrow; };      // bytes
+__host__ __device__ __forceinline__ WalkLayout walk_layout(const AttnParams& p, int CR) {
+    const int leaf = (p.ln[0] + CR - 1) / CR, up = p.L > 1 ? (p.ln[1] + CR - 1) / CR : 1;
+    WalkLayout w;
+    w.narrow = leaf <= 65536;
+    w.list = ((leaf < p.TK ? leaf : p.TK) * (w.narrow ? 2 : 4) + 3) & ~3;
+    w.bits = ((up < p.TK ? up : p.TK) * CR + 31) / 32 * 4;
+    return w;
+}
+template <typename Ring>
+__host__ __device__ __forceinline__ size_t walk_warp_bytes(const WalkLayout& w) { return (Ring::kBytes + w.list + w.bits + 127) & ~size_t(127); }
+
 }  // namespace htree

@@ -83,19 +83,19 @@ acc_mma_kernel(const __grid_constant__ AttnParams p) {
         const int nchunk = (np + PPC - 1) / PPC;
         __syncwarp();
 
-        const int64_t bstride = (int64_t)p.Hkv * C::BLOCK;
+        const uint32_t bstride = (uint32_t)p.Hkv * C::BLOCK;                // (a grid has at most 65535 KV heads)
         const unsigned char* blk = reinterpret_cast<const unsigned char*>(p.blk[l]) + ((int64_t)b * nblk * p.Hkv + hk) * C::BLOCK;
         const unsigned char* tab = reinterpret_cast<const unsigned char*>(p.tab);
         auto fill = [&](int c) {                                      // chunk c of this level
             const int p0 = par[c * PPC];
             if constexpr (CR == 16) {
-                ring.template copy<C::DATA>(0, blk + p0 * bstride, lane);
+                ring.template copy<C::DATA>(0, blk + (uint64_t)(uint32_t)p0 * bstride, lane);
             } else {
                 const int p1 = c * PPC + 1 < np ? par[c * PPC + 1] : p0;  // past the end of the list: masked, any finite block
-                ring.template copy<C::DATA / 2>(0, blk + p0 * bstride, lane);
-                ring.template copy<C::DATA / 2>(C::DATA / 2, blk + p1 * bstride + C::ODD, lane);
+                ring.template copy<C::DATA / 2>(0, blk + (uint64_t)(uint32_t)p0 * bstride, lane);
+                ring.template copy<C::DATA / 2>(C::DATA / 2, blk + (uint64_t)(uint32_t)p1 * bstride + C::ODD, lane);
             }
-            const unsigned char* row = tab + (int64_t)(rp - 16 * c) * C::TAB;
+            const unsigned char* row = tab + (uint32_t)(rp - 16 * c) * C::TAB;
             ring.template copy<C::TAB>(C::DATA, row, lane);
             if constexpr (C::DUAL) ring.template copy<C::TAB>(C::DATA + C::TAB, rp - 16 * c >= 8 ? row - 8 * C::TAB : row, lane);
         };

@@ -148,16 +148,16 @@ __global__ void __launch_bounds__(dq_warps<D, X3, NH>() * 32, dq_min_blocks<D, X
         const unsigned char* vblk = reinterpret_cast<const unsigned char*>(p.vkblk[l]) + blk0 * (C::PL * C::PART);
         auto fill = [&](int c) {
             constexpr int PB = C::PL * C::PART;
-            const int64_t kstride = (int64_t)p.Hkv * C::BLOCK, vstride = (int64_t)p.Hkv * PB;
+            const uint32_t kstride = (uint32_t)p.Hkv * C::BLOCK, vstride = (uint32_t)p.Hkv * PB;
             const int p0 = par[c * PPC];
-            ring.template copy<PB>(0, kblk + p0 * kstride, lane);
-            ring.template copy<PB>(C::V_OFF, vblk + p0 * vstride, lane);
+            ring.template copy<PB>(0, kblk + (uint64_t)(uint32_t)p0 * kstride, lane);
+            ring.template copy<PB>(C::V_OFF, vblk + (uint64_t)(uint32_t)p0 * vstride, lane);
             if constexpr (CR == 8) {
                 const int p1 = c * PPC + 1 < np ? par[c * PPC + 1] : p0;
-                ring.template copy<PB>(C::K2_OFF, kblk + p1 * kstride + 2 * C::ODD, lane);
-                ring.template copy<PB>(C::V2_OFF, vblk + p1 * vstride, lane);
+                ring.template copy<PB>(C::K2_OFF, kblk + (uint64_t)(uint32_t)p1 * kstride + 2 * C::ODD, lane);
+                ring.template copy<PB>(C::V2_OFF, vblk + (uint64_t)(uint32_t)p1 * vstride, lane);
             }
-            const unsigned char* row = reinterpret_cast<const unsigned char*>(p.tab) + (int64_t)(rp - 16 * c) * C::TAB;
+            const unsigned char* row = reinterpret_cast<const unsigned char*>(p.tab) + (uint32_t)(rp - 16 * c) * C::TAB;
             ring.template copy<C::TAB>(C::DATA, row, lane);
             if constexpr (C::DUAL) ring.template copy<C::TAB>(C::DATA + C::TAB, rp - 16 * c >= 8 ? row - 8 * C::TAB : row, lane);
         };

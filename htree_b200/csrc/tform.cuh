@@ -305,15 +305,18 @@ __device__ __forceinline__ void score_t(const LaneBase<D, X3, CR>& s, uint32_t t
 template <int NSTG, int SLOT>
 struct WarpRing {
     uint32_t base;                 // 32-bit shared address of NSTG * SLOT bytes
-    uint32_t is = 0, cs = 0;       // stage the next fill / the next use takes
+    uint32_t fill, use;            // addresses of the stages that the next fill / the next use takes
     static constexpr size_t kBytes = ((size_t)NSTG * SLOT + 127) & ~size_t(127);
 
-    __device__ __forceinline__ void init(unsigned char* b) { base = smem_u32(b); }
-    __device__ __forceinline__ void start() { is = cs = 0; }       // before the first fill of a walk; nothing is in flight
+    __device__ __forceinline__ void init(unsigned char* b) { base = smem_u32(b); start(); }
+    __device__ __forceinline__ void start() { fill = use = base; }       // before the first fill of a walk; nothing is in flight
+    __device__ __forceinline__ uint32_t after(uint32_t a) const {
+        return NSTG == 2 ? 2 * base + SLOT - a : a == base + (NSTG - 1) * SLOT ? base : a + SLOT;
+    }
     // BYTES (a multiple of 16) from `src` to offset OFF of the stage being filled
     template <int BYTES>
     __device__ __forceinline__ void copy(uint32_t off, const void* src, int lane) const {
-        const uint32_t dst = base + is * SLOT + off + 16 * lane;
+        const uint32_t dst = fill + off + 16 * lane;
         const unsigned char* s = static_cast<const unsigned char*>(src) + 16 * lane;
 #pragma unroll
         for (int i = 0; i < BYTES / 512; ++i)
@@ -326,15 +329,15 @@ struct WarpRing {
     // closes one fill (an empty one where nothing is left to fetch: fills and uses are counted alike)
     __device__ __forceinline__ void commit() {
         asm volatile("cp.async.commit_group;\n" ::: "memory");
-        is = is + 1 == NSTG ? 0 : is + 1;
+        fill = after(fill);
     }
     // the oldest fill, complete and visible to every lane
     __device__ __forceinline__ uint32_t wait() {
         asm volatile("cp.async.wait_group %0;\n" ::"n"(NSTG - 1) : "memory");
         __syncwarp();
-        uint32_t slot = base + cs * SLOT;
+        uint32_t slot = use;
         asm volatile("" : "+r"(slot)::"memory");
-        cs = cs + 1 == NSTG ? 0 : cs + 1;
+        use = after(use);
         return slot;
     }
     __device__ __forceinline__ void idle() const { asm volatile("cp.async.wait_all;\n" ::: "memory"); }

@@ -28,6 +28,7 @@ struct AttnParams {
     const void* vkblk[HTREE_MAX_LEVELS]; // their backward part, or NULL
     const void* tab;                     // rotary table of the transposed kernels, rows [cos | sin]: IEEE half times scale, or fp32 (split-half)
     const void* tab32;                   // fp32 rows [cos | sin] for the selection kernel
+    int32_t sel_maxc;                    // most candidates of a group on a level that selects (set by the selection's launch)
     int32_t ln[HTREE_MAX_LEVELS];   // N_l
     int64_t lpow[HTREE_MAX_LEVELS]; // CR^l
     const float* cosc;

@@ -28,11 +28,11 @@ constexpr int kSelLong = 4096;
 constexpr int kSelSplitWarps = 8, kSelSplitKeys = 32 * 32 * kSelSplitWarps;      // SPLIT keeps 32 keys per thread
 
 // The most candidates a group has on any level that selects: the children of TK parents, or of all there are.
-__host__ __device__ __forceinline__ int sel_max_candidates(const AttnParams& p, int CR) {
-    int most = CR;
+static int sel_max_candidates(const AttnParams& p) {
+    int most = p.CR;
     for (int l = 1; l < p.L; ++l) {
-        const int parents = (p.ln[l] + CR - 1) / CR;
-        const int n = (parents < p.TK ? parents : p.TK) * CR;
+        const int parents = (p.ln[l] + p.CR - 1) / p.CR;
+        const int n = (parents < p.TK ? parents : p.TK) * p.CR;
         if (n > most) most = n;
     }
     return most;
@@ -136,7 +136,7 @@ select_mma_kernel(const __grid_constant__ AttnParams p) {
     const int tl = p.Tq <= kSelReverse ? p.Tq - 1 - at : at;
     const int t = p.t0 + tl;
     const int b = blockIdx.y / p.Hkv, hk = blockIdx.y % p.Hkv;
-    const int G = p.G, TK = p.TK, L = p.L, maxc = sel_max_candidates(p, CR);
+    const int G = p.G, TK = p.TK, L = p.L, maxc = p.sel_maxc;
     const int first = SPLIT ? warp : 0, step = SPLIT ? W : 1;
     const int tid = SPLIT ? (int)threadIdx.x : lane, nthr = SPLIT ? kSelSplitWarps * 32 : 32;   // the threads that share a group
     auto sync = [&]() { if constexpr (SPLIT) __syncthreads(); else __syncwarp(); };
@@ -190,16 +190,17 @@ select_mma_kernel(const __grid_constant__ AttnParams p) {
         } else {
             const int nchunk = (np + PPC - 1) / PPC;
             const int nblk = (Nl + CR - 1) / CR;
-            const int64_t bstride = (int64_t)p.Hkv * C::BLOCK;
+            const uint32_t bstride = (uint32_t)p.Hkv * C::BLOCK;
             const unsigned char* blk = reinterpret_cast<const unsigned char*>(p.blk[l]) + ((int64_t)b * nblk * p.Hkv + hk) * C::BLOCK;
+            // Every parent here is below nblk and needs no check (one in this loop cost 2 to 9%): lists ascend and none of them passes
+            // the query's own ancestor, position t / lpow[l + 1] of the level above; only a list that ends there has it as its last
+            // parent, and then the candidates stop at t / lpow[l], which is a node of this level for every t < T.
             auto fill = [&](int c) {
 #pragma unroll
                 for (int w = 0; w < PPC; ++w) {
                     const int a = PPC == 1 ? c : min(c * PPC + w, np - 1);     // past the end of the list: masked, any finite block
-                    int pb = par[a];
-                    if ((unsigned)pb >= (unsigned)nblk) { if (p.status) atomicOr(p.status, 4); pb = 0; }
-                    ring.template copy<SF::KPART>(w * SF::KPART, blk + pb * bstride, lane);
-                    ring.template copy<SF::TAB>(SF::DATA + w * SF::TAB, reinterpret_cast<const unsigned char*>(p.tab32) + (int64_t)(rp - CR * a) * SF::TAB, lane);
+                                    ring.template copy<SF::KPART>(w * SF::KPART, blk + (uint64_t)(uint32_t)par[a] * bstride, lane);
+                    ring.template copy<SF::TAB>(SF::DATA + w * SF::TAB, reinterpret_cast<const unsigned char*>(p.tab32) + (uint32_t)(rp - CR * a) * SF::TAB, lane);
                 }
             };
             ring.start();
@@ -378,10 +379,11 @@ select_mma_kernel(const __grid_constant__ AttnParams p) {
 }
 
 template <typename T, int D, bool X3, int NH, int CR>
-static int launch_select_cr(const AttnParams& p, cudaStream_t st) {
+static int launch_select_cr(const AttnParams& in, cudaStream_t st) {
+    AttnParams p = in;
     using SF = SelForm<D, X3, CR>;
     using Ring = WarpRing<SF::NSTG, SF::SLOT>;
-    const int maxc = sel_max_candidates(p, CR);
+    const int maxc = p.sel_maxc = sel_max_candidates(p);
     const size_t scratch = sel_scratch_bytes(maxc, p.TK, CR), limit = 227 * 1024;
     const int64_t groups = (int64_t)p.Tq * p.B * p.Hkv;
     // A block of 8 warps per group where there are few groups (below two per SM a single warp's walk over its chunks is the whole
@@ -426,7 +428,7 @@ bool select_blk_supported(const AttnParams& p, int dtype) {
     for (int l = 1; l < p.L; ++l) if (!p.blk[l]) return false;
     const bool x3 = dtype == HTREE_F32;
     const size_t ring = 3 * ((x3 ? 2 : 1) * (size_t)p.K * 32 + 8 * p.K) + 128;
-    return ring + sel_scratch_bytes(sel_max_candidates(p, p.CR), p.TK, p.CR) <= 227 * 1024;
+    return ring + sel_scratch_bytes(sel_max_candidates(p), p.TK, p.CR) <= 227 * 1024;
 }
 
 int launch_select_blk(const AttnParams& p, int dtype, cudaStream_t st) {

@@ -76,7 +76,7 @@ __global__ void __launch_bounds__(256) bwd_fill_kernel(const __grid_constant__ B
 // step: one visit of up to 16 heads, or two visits of up to 8.  A = the blocked queries rotated by the visit's distance, or the
 // blocked output gradients; B = dS or P as the first pass left them.  One warp per item, operands through the warp's ring.
 // The two gradients are separate launches: each gathers from one blocked tensor only (a window of it stays in L2) and its
-// accumulator is 64 registers, which leaves room for 16 and more warps per SM.
+// accumulator is 64 registers, which leaves room for 12 and more warps per SM.  Bound by that gather: 14 TB/s of a measured 20.
 // Ring depth: three slots; two where that lets more blocks share an SM and they are the faster choice: split-half, and the keys of
 // groups of 9 to 16 heads of 128 (65536 positions, 64 heads: 13.2 -> 12.4 ms; with 8 heads a group three slots keep a lead of 1%).
 template <int D, bool X3, int NH, bool KEYS>
@@ -315,7 +315,7 @@ static int launch_dkv_one(const BwdParams& bp, cudaStream_t st) {
     const size_t smem = 4 * Ring::kBytes;
     auto* k = bwd_dkv_kernel<T, D, X3, NH, CR, KEYS>;
     static SmemLimit shared;
-        const cudaError_t e = shared.raise((const void*)k, smem);
+    const cudaError_t e = shared.raise((const void*)k, smem);
     if (e != cudaSuccess) return (int)e;
     k<<<dim3((bp.cap + 3) / 4, bp.nsub), 128, smem, st>>>(bp);
     note_launch();

@@ -4,6 +4,10 @@
 // (src/backward.py:45-436); arithmetic of src/naive.py:333-384 with the forward's scores, bit for bit.  Per chunk:
 //   dP^T = V dO^T,  S^T = K' q^,  P = exp(S - gmax) / gsum,  dS = P (dP - D),  dq^T += K~^T dS^T
 // with K~ = scale R(-distance) K' rotated back into the query's frame in registers, its fragments transposed by the load.
+//
+// Bound by the latency of those five products in a row at 12 warps per SM (issue 46%, shared-memory pipe 65%, tensor pipe 37%).
+// 4 x 65536 positions, 64 heads of 128: this pass 135 ms and the parent-stationary one 90 ms, where the single kernel with reductions
+// took 360 ms.
 #include "bwd_tform.cuh"
 
 namespace htree {
@@ -389,7 +393,7 @@ static int launch_dq_cr(const BwdParams& bp, cudaStream_t st) {
     if (best == 0 || W * per_warp > 227 * 1024) return HTREE_E_UNSUPPORTED;
     auto* k = bwd_dq_kernel<T, D, X3, NH, CR>;
     static SmemLimit shared;
-        const cudaError_t e = shared.raise((const void*)k, W * per_warp);
+    const cudaError_t e = shared.raise((const void*)k, W * per_warp);
     if (e != cudaSuccess) return (int)e;
     k<<<dim3((bp.subq + W - 1) / W, bp.nsub), W * 32, W * per_warp, st>>>(bp);
     note_launch();

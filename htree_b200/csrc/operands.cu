@@ -1,6 +1,7 @@
 // Operand preparation of the transposed tensor-core kernels: one warp per (batch, parent, KV head) reads the parent's
 // children once and writes everything that is derived from them: the parent's own pooled row (the next level), the operand
-// blocks of the forward and of the backward (layouts in tform.cuh).  One launch per level.  HBM / L2 streaming: per 16-bit block of 16 children and 128-wide heads it
+// blocks of the forward and of the backward (layouts in tform.cuh).  One launch per level.
+// HBM / L2 streaming: per 16-bit block of 16 children and 128-wide heads it
 // reads 8 KB and writes 8.5 KB (12.5 KB with the backward's part); the launches it replaces (pooling, rotation, two blockings
 // per level) read the same rows four times and cost a launch each, which is what short sequences spent their time on.
 #include "tform.cuh"

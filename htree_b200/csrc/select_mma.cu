@@ -5,6 +5,9 @@
 // One warp per (batch, query position, KV head) group; with SPLIT the 8 warps of a block share a group's chunks.  A candidate's
 // importance does not depend on which: every chunk is evaluated alike (the query rotated in fp32 and rounded once to half per
 // parent, two accumulation chains, the chunk's own maximum as reference, heads summed in one fixed tree) and the search is exact.
+//
+// Bound by instruction issue and latency at 12 to 16 warps per SM; of its time the copies are a third, the Top-K search and the
+// rotation a tenth each.  Measured against the kernel that gathers rows: 4 x 65536 positions, 64 heads of 128: 49 -> 43.7 ms.
 #include "tform.cuh"
 
 namespace htree {
@@ -409,7 +412,7 @@ static int launch_select_cr(const AttnParams& in, cudaStream_t st) {
     if (best == 0 || W * per_warp > limit) return HTREE_E_UNSUPPORTED;
     auto* k = select_mma_kernel<T, D, X3, NH, CR, false>;
     static SmemLimit shared;
-        const cudaError_t e = shared.raise((const void*)k, W * per_warp);
+    const cudaError_t e = shared.raise((const void*)k, W * per_warp);
     if (e != cudaSuccess) return (int)e;
     k<<<dim3((p.Tq + W - 1) / W, p.B * p.Hkv), W * 32, W * per_warp, st>>>(p);
     note_launch();

@@ -7,7 +7,7 @@
 // heads-on-M form, whose other 8 rows would be padding; 9..16 heads are two halves (NH = 2) that share every A fragment, at
 // the instruction count of the heads-on-M form.
 //
-// Operand blocks (written by pack_blocks_kernel, read here as whole blocks by asynchronous bulk copies): per parent and KV
+// Operand blocks (written by pack_blocks_kernel, read here as whole blocks by asynchronous copies): per parent and KV
 // head the children's pre-rotated keys K' and values in the order in which the lanes consume them as A fragments, so that a
 // fragment is one conflict-free 16-byte shared load.  With lane = 4g + r, KS = D/16, PPT = D/8, VB = D/8:
 //   K    8x8 matrices [ks][m][lane] of 4-byte words, m = lo / hi dims (8 children), or children 0-7 lo, 8-15 lo, 0-7 hi, 8-15 hi
@@ -344,7 +344,7 @@ struct WarpRing {
 };
 
 // A query's parent list of one level in shared memory, 16 bits an entry where every level's parents can be numbered with them
-// (4 KB against 2 KB a warp matter with 512 nodes per layer, where lists and bits decide how many warps share an SM).
+// (with 512 nodes per layer 1 KB instead of 2 beside 17 KB of ring: lists and bits decide whether 11 or 12 warps share an SM).
 struct ParentList {
     unsigned char* at;
     bool narrow;

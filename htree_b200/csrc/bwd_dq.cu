@@ -356,17 +356,24 @@ __global__ void __launch_bounds__(dq_warps<D, X3, NH>() * 32, dq_min_blocks<D, X
     // ---- dq through shared memory (the ring is idle), rows written whole: fp32, or rounded once to the storage type ----
     __syncwarp();
     float* sm = reinterpret_cast<float*>(wbase);
+    // 128 dims of 16-bit storage: rows and every 16 floats of a row are 4 floats further apart (unpadded, 8 lanes of a store met in
+    // one bank).  With 32 and 64 dims 2 and 4 lanes meet and the padded addresses cost more than they give.
+    constexpr bool PADDED = D == 128 && !X3;
+    constexpr int ROW = D + (PADDED ? D / 4 + 4 : 0);
+    static_assert(8 * NH * ROW * sizeof(float) <= Ring::kBytes, "the rows fit the ring");
     const float post = X3 ? p.scale : 1.f;           // 16-bit: the scale is in the tables
 #pragma unroll
     for (int h = 0; h < NH; ++h)
 #pragma unroll
         for (int ks = 0; ks < KS; ++ks)
 #pragma unroll
-            for (int i = 0; i < 4; ++i)
-                sm[(8 * h + 2 * r + (i & 1)) * D + (i >> 1) * HALF + PPT * (g >> 1) + 2 * ks + (g & 1)] = dq[h][ks][i] * post;
+            for (int i = 0; i < 4; ++i) {
+                if constexpr (PADDED) sm[(8 * h + 2 * r + (i & 1)) * ROW + ((i >> 1) * HALF + PPT * (g >> 1)) / 16 * 20 + 2 * ks + (g & 1)] = dq[h][ks][i] * post;
+                else sm[(8 * h + 2 * r + (i & 1)) * D + (i >> 1) * HALF + PPT * (g >> 1) + 2 * ks + (g & 1)] = dq[h][ks][i] * post;
+            }
     __syncwarp();
     for (int i = lane; i < G * D / 4; i += 32) {
-        const float4 x = reinterpret_cast<const float4*>(sm)[i];
+        const float4 x = reinterpret_cast<const float4*>(sm)[PADDED ? i / (D / 4) * (ROW / 4) + i % (D / 4) / 4 * 5 + i % 4 : i];
         if (p.dq_typed == nullptr) {
             reinterpret_cast<float4*>(p.dq + hbase * D)[i] = x;
         } else if constexpr (sizeof(T) == 4) {

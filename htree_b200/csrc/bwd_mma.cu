@@ -114,9 +114,6 @@ __global__ void HTREE_BWD_BOUNDS bwd_mma_kernel(const __grid_constant__ AttnPara
     for (int i = 0; i < NOT; ++i) { dqa[i][0] = dqa[i][1] = dqa[i][2] = dqa[i][3] = 0.f; }
 
     for (int l = L - 1; l >= 0; --l) {
-#ifdef HTREE_BWD_SKIP_LEVEL   // timing experiments only: leaves out one level's work (results are then incomplete)
-        if (l == HTREE_BWD_SKIP_LEVEL) continue;
-#endif
         const int Nl = p.ln[l];
         const __half* lkr = reinterpret_cast<const __half*>(p.lkr[l]);
         const T* lv = reinterpret_cast<const T*>(p.lv[l]);

@@ -188,9 +188,6 @@ fwd_mma_kernel(const __grid_constant__ AttnParams p) {
             for (int i = 0; i < NSTG; ++i) mbar_init(&bars[i], 1);
             fence_barrier_init();
         }
-#ifdef HTREE_FWD_KNOCK_ALLCOPY
-        for (uint32_t i = lane * 16u; i < (uint32_t)NSTG * SLOT; i += 512u) *reinterpret_cast<uint4*>(ring + i) = make_uint4(0u, 0u, 0u, 0u);
-#endif
         __syncwarp();
     }
     auto pipe_issue = [&](uint32_t n, int a) {       // lane 0: start the copies for the chunk at parent slot a into ring slot n % NSTG
@@ -198,16 +195,6 @@ fwd_mma_kernel(const __grid_constant__ AttnParams p) {
         if (pb < 0 || pb >= blk_count) pb = 0;       // flagged where the chunk is consumed
         const int sl = (int)(n % NSTG);
         unsigned char* dst = ring + (size_t)sl * SLOT;
-#ifdef HTREE_FWD_KNOCK_ALLCOPY   // timing experiments only: no copies and no waits, the kernels compute on a zero-filled ring
-        return;
-#endif
-#ifdef HTREE_FWD_KNOCK_KCOPY   // timing experiments only: upper-level chunks of the accumulation kernel bring their values alone
-        if (MODE == 2 && pipe_level > 0) {
-            mbar_arrive_expect_tx(&bars[sl], 4096u);
-            bulk_copy_g2s(dst + 4096, vblk + (int64_t)pb * blk_stride, 4096u, &bars[sl]);
-            return;
-        }
-#endif
         mbar_arrive_expect_tx(&bars[sl], SLOT);
         bulk_copy_g2s(dst, kblk + (int64_t)pb * blk_stride, 4096u, &bars[sl]);
         if (MODE == 2) bulk_copy_g2s(dst + 4096, vblk + (int64_t)pb * blk_stride, 4096u, &bars[sl]);
@@ -245,9 +232,7 @@ fwd_mma_kernel(const __grid_constant__ AttnParams p) {
             pissued = pn + NSTG;
         }
         const int sl = (int)(pn % NSTG);
-#ifndef HTREE_FWD_KNOCK_ALLCOPY
         if (!mbar_wait_bounded(&bars[sl], (pn / NSTG) & 1u, kPipeWaitCap)) { pipe_abort(); return nullptr; }
-#endif
         ++pn;
         return ring + (size_t)sl * SLOT;
     };
@@ -324,13 +309,6 @@ fwd_mma_kernel(const __grid_constant__ AttnParams p) {
         auto score = [&](int a, float (&S0)[4], float (&S1)[4], bool select) {
             int node0 = par[a] * CR;
             if (node0 < 0 || node0 >= Nl) { if (p.status) atomicOr(p.status, 4); node0 = 0; }
-#ifdef HTREE_FWD_KNOCK_SCORE   // timing experiments only: levels in the kernel's bit mask (selection kernel: bits 0-7,
-            // accumulation kernel: bits 8-15) are not scored; results are wrong
-            if (((kAccumulateKernel ? (HTREE_FWD_KNOCK_SCORE) >> 8 : (HTREE_FWD_KNOCK_SCORE)) >> l) & 1) {
-                S0[0] = S0[1] = S0[2] = S0[3] = S1[0] = S1[1] = S1[2] = S1[3] = 0.f;
-                return;
-            }
-#endif
             if constexpr (PIPE) {
                 // the rotation of a chunk is fixed by the kernel: fp32 tables where the Top-K is decided (selection kernel) or
                 // no packed-half tables were given, packed-half tables otherwise; its table rows are in the slot
@@ -453,9 +431,6 @@ fwd_mma_kernel(const __grid_constant__ AttnParams p) {
         };
 
         if (l > 0 && kAccumulateKernel) {
-#ifdef HTREE_FWD_KNOCK_LEVEL   // timing experiments only: the accumulation kernel leaves out the levels of this bit mask
-            if (((HTREE_FWD_KNOCK_LEVEL) >> l) & 1) continue;
-#endif
             if (nc > TK) {
                 // kept-candidate bit mask from the two sorted lists: the level's parents and the next level's parents
                 for (int i = lane; i < (nc + 31) / 32; i += 32) selw[i] = 0u;

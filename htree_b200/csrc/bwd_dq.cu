@@ -16,7 +16,7 @@ template <int D, bool X3>
 constexpr int dq_stages() { return D * (X3 ? 2 : 1) >= 128 ? 2 : 3; }     // slots of 8 KB: warps matter more than depth
 // Warps per block and blocks per SM: registers first.  The ring takes nearly all of the SM's L1, so anything that spills is
 // re-read from L2 in every chunk: with 180 bytes of spills, groups of 16 heads of 128 spent 4.6 of 9.4 cycles per instruction
-// waiting for it.  Those run as blocks of one warp (24 to 32 bytes of spills at 12 warps per SM; the compiler keeps 150 in larger
+// waiting for it.  Those run as blocks of one warp (at most 20 bytes of spills at 12 warps per SM; the compiler keeps 150 in larger
 // blocks): 64K positions, 4 KV heads 53 -> 31.6 ms, against 33.3 ms for 8 warps per SM with nothing spilled.  32-wide heads fit
 // 16 warps (10.2 -> 9.9 ms at 12000 positions, 512 nodes per layer).
 template <int D, bool X3, int NH>

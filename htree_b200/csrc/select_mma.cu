@@ -320,6 +320,7 @@ select_mma_kernel(const __grid_constant__ AttnParams p) {
                 __syncthreads();
 #pragma unroll
                 for (int w = 0; w < kSelSplitWarps; ++w) { lo = min(lo, (uint32_t)wtot[2 * w]); hi = max(hi, (uint32_t)wtot[2 * w + 1]); }
+                __syncthreads();       // the placement below writes wtot, and where all importances are equal no count comes between
             }
             hi += 1u;
             int c_lo = nc, c_hi = 1;

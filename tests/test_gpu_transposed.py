@@ -57,7 +57,8 @@ def test_forward_and_backward(dt, D, CR, G, B, T, TK, MTN, monkeypatch):
 
 @pytest.mark.parametrize("dt,D,CR,G,B,T,TK,MTN,clustered", [
     (BF, 128, 16, 16, 1, 140, 16, 64, False),      # fewer than 296 groups: eight warps a group
-    (BF, 128, 16, 16, 1, 12000, 512, 2048, False), # lists too long for one warp
+    (BF, 128, 16, 16, 1, 12000, 512, 2048, False), # 752 candidates, more than a level keeps for the last positions only
+    (BF, 128, 16, 16, 1, 72000, 512, 8192, False), # 4512 candidates: lists too long for one warp
     (BF, 128, 16, 12, 1, 9001, 32, 256, True), (HF, 128, 8, 8, 1, 9001, 32, 128, False), (BF, 64, 8, 4, 1, 5000, 64, 64, True),
     (HF, 64, 16, 9, 2, 1777, 16, 64, False), (FP, 64, 8, 1, 1, 1777, 16, 64, False), (FP, 64, 16, 16, 1, 5000, 64, 64, True)])
 def test_selections_bit_identical(dt, D, CR, G, B, T, TK, MTN, clustered):
@@ -86,5 +87,26 @@ def test_few_queries(dt, D, CR, G, T, TK, MTN, W):
     full = ht.htree_forward(q, k, v, CR, MTN, TK)
     part = ht.htree_forward(q[:, T - W:].contiguous(), k, v, CR, MTN, TK, _q_offset=T - W)
     assert _rel(part, full[:, T - W:]) < (2e-6 if dt == FP else 4e-3)
+    torch.cuda.synchronize()
+    ops.check_status()
+
+
+@pytest.mark.parametrize("dt,D,CR,G,T,TK,MTN,W,zero", [
+    (BF, 128, 16, 16, 9001, 32, 128, 3, "q"), (HF, 64, 8, 4, 9001, 64, 64, 40, "k"), (FP, 64, 16, 8, 9001, 32, 64, 2, "q"),
+    (BF, 128, 16, 9, 9001, 32, 128, 400, "k"),      # one warp per group
+    (BF, 128, 16, 4, 72000, 512, 8192, 600, "q")])  # lists above 4096 candidates
+def test_equal_importances(dt, D, CR, G, T, TK, MTN, W, zero):
+    """Every candidate but the forced one equally important: the smallest positions are kept, and no search runs."""
+    import htree_b200 as ht
+    from htree_b200 import ops
+    q, k, v, _ = _inputs(dt, 1, T, 2, G, D)
+    (q if zero == "q" else k).zero_()
+    q = q[:, T - W:].contiguous()
+    lists = []
+    for generic in (False, True):
+        _, ctx = ht.htree_forward(q, k, v, CR, MTN, TK, _q_offset=T - W, _save_for_backward=True, _force_generic=generic)
+        lists.append(ctx["per_layer_parents"])
+    for l in lists[0]:
+        assert torch.equal(lists[0][l], lists[1][l]), f"level {l}"
     torch.cuda.synchronize()
     ops.check_status()

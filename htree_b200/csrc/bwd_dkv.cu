@@ -52,12 +52,12 @@ __global__ void __launch_bounds__(256) bwd_fill_kernel(const __grid_constant__ B
     BwdItem* items = bp.items + (int64_t)blockIdx.y * bp.cap;
     for (int l = p.L - 1; l >= 0; --l) {
         if (bp.voff[l] < 0) continue;
-        int np = 0;
-        for (int i = lane; i < TK; i += 32) np += load_parent(p, l, qidx * TK + i) >= 0;
+        const int nblk = (p.ln[l] + CR - 1) / CR;
+        int np = 0;                                // the parents, counted and bounded as ParentList::load does for the first pass
+        for (int i = lane; i < min(TK, nblk); i += 32) np += load_parent(p, l, qidx * TK + i) >= 0;
         np = __reduce_add_sync(0xffffffffu, np);
         const int rp = (np - 1) * CR + (int)(((int64_t)t / p.lpow[l]) % CR);
         if (np <= 0 || (l > 0 && rp + 1 <= TK)) continue;
-        const int nblk = (p.ln[l] + CR - 1) / CR;
         const int2* base = bp.base + (int64_t)blockIdx.y * bp.NK + bp.koff[l];
         const int32_t* cnt = bp.cnt + (int64_t)blockIdx.y * bp.NK + bp.koff[l];
         for (int i = lane; i < np; i += 32) {

@@ -351,17 +351,21 @@ struct ParentList {
     __device__ __forceinline__ int operator[](int i) const {
         return narrow ? (int)reinterpret_cast<const uint16_t*>(at)[i] : reinterpret_cast<const int32_t*>(at)[i];
     }
-    // from the selections: returns the number of parents; entries that are no parent of the level become 0 and set `bit`
+    // A query's list of one level: returns the number of its parents, looking at no more entries than the level has parents.  Entries
+    // that are no parent of the level become 0 and set `bit`, and so do holes before the last parent: a backward's lists come from
+    // its caller, and a slot left as it was would index blocks and counters with what the shared memory held before.
     __device__ __forceinline__ int load(const AttnParams& p, int l, int64_t list, int nblk, int bit, int lane) const {
-        int np = 0;
+        int np = 0, end = 0;
         for (int i = lane; i < min(p.TK, nblk); i += 32) {
             int x = load_parent(p, l, list + i);
-            if (x < 0) continue;
-            ++np;
+            if (x >= 0) { ++np; end = i + 1; }
             if (x >= nblk) { if (p.status) atomicOr(p.status, bit); x = 0; }
+            x = max(x, 0);
             if (narrow) reinterpret_cast<uint16_t*>(at)[i] = (uint16_t)x; else reinterpret_cast<int32_t*>(at)[i] = x;
         }
-        return __reduce_add_sync(0xffffffffu, np);
+        np = __reduce_add_sync(0xffffffffu, np);
+        if (end > np && p.status) atomicOr(p.status, bit);
+        return np;
     }
 };
 // What the walk over a level's candidates keeps per warp beside the ring: the parent list and one bit per candidate of a level

@@ -110,3 +110,41 @@ def test_equal_importances(dt, D, CR, G, T, TK, MTN, W, zero):
         assert torch.equal(lists[0][l], lists[1][l]), f"level {l}"
     torch.cuda.synchronize()
     ops.check_status()
+
+
+@pytest.mark.parametrize("dt,D,CR,G,T,TK,MTN", [(BF, 128, 16, 16, 3001, 32, 128), (FP, 64, 8, 8, 1777, 16, 64), (HF, 64, 16, 4, 300, 32, 64)])
+@pytest.mark.parametrize("compact", [False, True])
+def test_malformed_parent_lists(dt, D, CR, G, T, TK, MTN, compact, monkeypatch):
+    """A backward whose caller's lists have holes, ids past the end of a level, or more entries than the level has parents reads and
+    writes nothing out of range, reports it, and leaves the other queries' gradients as they are."""
+    import htree_b200 as ht
+    from htree_b200 import ops
+    if compact:
+        monkeypatch.setattr(ops, "SELECTION_STORAGE", "uint16")
+    q, k, v, dO = _inputs(dt, 1, T, 2, G, D)
+    out, ctx = ht.htree_forward(q, k, v, CR, MTN, TK, _save_for_backward=True)
+    want = ht.htree_backward(dO, q, out, ctx)[0]
+    lists = {l: x.clone() for l, x in ctx["per_layer_parents"].items()}
+    for bad in range(3):
+        ctx["per_layer_parents"] = hurt = {l: x.clone() for l, x in lists.items()}
+        rows = torch.arange(T // 2, T, 7, device=DEV)
+        leaf, top = hurt[0], hurt[ctx["num_layers"] - 1]
+        if bad == 0:                                  # holes, the first entry among them
+            leaf[:, rows, 0, 1] = -1
+            leaf[:, rows, 1, 0] = -1
+        elif bad == 1:                                # past the end (the largest 16-bit id where ids are 16-bit)
+            leaf[:, rows, 0, 2] = -2 if compact else 1 << 30
+            top[:, rows, 1, 0] = (T + CR - 1) // CR
+        else:                                         # as many entries as fit, all of one parent, and a list of none
+            leaf[:, rows, 0] = 3
+            leaf[:, rows, 1] = -1
+        got = ht.htree_backward(dO, q, out, ctx)
+        torch.cuda.synchronize()
+        assert all(x.isfinite().all() for x in got)
+        same = torch.ones(T, dtype=torch.bool, device=DEV)
+        same[rows] = False
+        assert torch.equal(got[0][:, same], want[:, same])
+        if bad < 2:
+            with pytest.raises(RuntimeError, match="outside its tree level"):
+                ops.check_status()
+    ops.check_status()

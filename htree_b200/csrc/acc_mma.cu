@@ -224,6 +224,10 @@ acc_mma_kernel(const __grid_constant__ AttnParams p) {
                     for (int h = 0; h < NH; ++h) mma_acc<FT>(O[h][i], va, pb[h][0], pb[h][1]);
                 }
             }
+#pragma unroll
+            for (int h = 0; h < NH; ++h)
+#pragma unroll
+                for (int i = 0; i < MT; ++i) consumed(O[h][i]);
         }
     }
 

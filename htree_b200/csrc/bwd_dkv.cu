@@ -230,6 +230,10 @@ __global__ void __launch_bounds__(128, dkv_min_blocks<D, X3>()) bwd_dkv_kernel(c
                 }
             }
         }
+#pragma unroll
+        for (int i = 0; i < KS; ++i)
+#pragma unroll
+            for (int n = 0; n < NT; ++n) consumed(acc[i][n]);
     }
 
     int l = 0;

@@ -322,6 +322,10 @@ __global__ void __launch_bounds__(dq_warps<D, X3, NH>() * 32, dq_min_blocks<D, X
                         }
                     }
                 }
+#pragma unroll
+                for (int h = 0; h < NH; ++h)
+#pragma unroll
+                    for (int ks = 0; ks < KS; ++ks) consumed(dq[h][ks]);       // (dP and the scores end in the records)
             }
             // ---- leave P and dS behind, one record per visit ----
 #pragma unroll

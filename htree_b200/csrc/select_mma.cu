@@ -251,6 +251,7 @@ select_mma_kernel(const __grid_constant__ AttnParams p) {
                 }
                 e0 += __shfl_xor_sync(0xffffffffu, e0, 1); e1 += __shfl_xor_sync(0xffffffffu, e1, 1);
                 e0 += __shfl_xor_sync(0xffffffffu, e0, 2); e1 += __shfl_xor_sync(0xffffffffu, e1, 2);
+                // (all of the chunk's loads end in these stores, ahead of the copies that refill the slot)
                 if (r < 2 && 16 * c + 8 * r + g < maxc) imp[16 * c + 8 * r + g] = r ? e1 : e0;
                 if (lane < PPC && c * PPC + lane < np) cmax[c * PPC + lane] = lane ? m1 : m0;
             }

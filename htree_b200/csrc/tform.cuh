@@ -102,7 +102,12 @@ __device__ __forceinline__ void value_frag(const LaneBase<D, X3, CR>& s, int pl,
     else ldmatrix_frag(s.v + pl * C::PART + i * 256, a);
 }
 // The loads from a slot and the products below are not volatile, so that the compiler may overlap one step's loads and
-// rotations with another's products; what orders the loads after the slot's wait is the slot address, which comes out of it.
+// rotations with another's products.  What orders the loads after the slot's wait is the slot address, which comes out of it; what
+// orders them before the copies that refill the slot is that everything they went into exists by then: stored to memory, or passed
+// to consumed() at the end of the chunk.  (consumed() is no instruction, and the registers it names are carried to the next chunk.)
+__device__ __forceinline__ void consumed(const float (&x)[4]) {
+    asm volatile("" ::"f"(x[0]), "f"(x[1]), "f"(x[2]), "f"(x[3]) : "memory");
+}
 template <typename T> __device__ __forceinline__ void mma_acc(float (&c)[4], const uint32_t (&a)[4], uint32_t b0, uint32_t b1);
 template <> __device__ __forceinline__ void mma_acc<__half>(float (&c)[4], const uint32_t (&a)[4], uint32_t b0, uint32_t b1) {
     asm("mma.sync.aligned.m16n8k16.row.col.f32.f16.f16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};\n"

@@ -66,14 +66,18 @@ acc_mma_kernel(const __grid_constant__ AttnParams p) {
         for (int i = 0; i < MT; ++i) O[h][i][0] = O[h][i][1] = O[h][i][2] = O[h][i][3] = 0.f;
     // Online softmax with a lazily moved reference: probabilities are taken relative to m_run, which moves (and the
     // accumulators are rescaled) only when a score exceeds it by more than kLazyMax.  m_run is common to the lanes that share
-    // a head; m_true (the maximum that goes to gmax) and s_run are per lane until the end.
+    // a head; m_true (the maximum that goes to gmax) and s_run are per lane until the end.  16-bit storage keeps m_run in units of
+    // log 2 and at whole numbers: two references then differ by a power of two, so that P, which is rounded to the storage type
+    // relative to the reference, rounds alike whichever warp forms it and however many share a group's chunks.  With references
+    // at the scores themselves a query's row differed by 3e-3 (bf16) between calls of few and of many queries.
     constexpr float kLazyMax = 8.f;
     constexpr float kNone = -1.0e30f;
-    float m_run[NH][2], m_true[NH][2], s_run[NH][2], m_run2[NH][2];
+    float m_run[NH][2], m_true[NH][2], s_run[NH][2];
+    auto factor = [](float from, float to) { return X3 ? __expf(from - to) : ex2_approx(from - to); };      // between two references
 #pragma unroll
     for (int h = 0; h < NH; ++h)
 #pragma unroll
-        for (int e = 0; e < 2; ++e) { m_run[h][e] = m_true[h][e] = kNone; m_run2[h][e] = kNone * kLog2e; s_run[h][e] = 0.f; }
+        for (int e = 0; e < 2; ++e) { m_run[h][e] = m_true[h][e] = kNone; s_run[h][e] = 0.f; }
 
     for (int l = L - 1; l >= 0; --l) {
         const int Nl = p.ln[l];
@@ -155,7 +159,7 @@ acc_mma_kernel(const __grid_constant__ AttnParams p) {
 #pragma unroll
                 for (int h = 0; h < NH; ++h)
 #pragma unroll
-                    for (int i = 0; i < 4; ++i) ex[h][i] = X3 ? S[h][i] - m_run[h][i & 1] : fmaf(S[h][i], kLog2e, -m_run2[h][i & 1]);
+                    for (int i = 0; i < 4; ++i) ex[h][i] = X3 ? S[h][i] - m_run[h][i & 1] : fmaf(S[h][i], kLog2e, -m_run[h][i & 1]);
             };
             exponents();
             float top = ex[0][0];
@@ -175,9 +179,9 @@ acc_mma_kernel(const __grid_constant__ AttnParams p) {
                         m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, 4));
                         m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, 8));
                         m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, 16));
-                        const float n = fmaxf(m_run[h][e], m);
-                        const float f = X3 ? __expf(m_run[h][e] - n) : ex2_approx(m_run2[h][e] - n * kLog2e);
-                        m_run[h][e] = n; m_run2[h][e] = n * kLog2e;
+                        const float n = fmaxf(m_run[h][e], X3 ? m : ceilf(m * kLog2e));
+                        const float f = factor(m_run[h][e], n);
+                        m_run[h][e] = n;
                         s_run[h][e] *= f;
 #pragma unroll
                         for (int i = 0; i < MT; ++i) { O[h][i][e] *= f; O[h][i][2 + e] *= f; }
@@ -264,7 +268,7 @@ acc_mma_kernel(const __grid_constant__ AttnParams p) {
                 const int head = 8 * h + 2 * r + e;
                 float m = kNone;
                 for (int w = 0; w < W; ++w) m = fmaxf(m, st[w * 48 + head]);
-                const float f = __expf(m_run[h][e] - m);
+                const float f = factor(m_run[h][e], m);
 #pragma unroll
                 for (int i = 0; i < MT; ++i) {
                     po[head * D + C::VB * g + 2 * i] = O[h][i][e] * f;
@@ -277,14 +281,14 @@ acc_mma_kernel(const __grid_constant__ AttnParams p) {
             float m = kNone, s = 0.f, o = 0.f;
             for (int w = 0; w < W; ++w) m = fmaxf(m, st[w * 48 + head]);
             for (int w = 0; w < W; ++w) {
-                s += st[w * 48 + 32 + head] * __expf(st[w * 48 + head] - m);
+                s += st[w * 48 + 32 + head] * factor(st[w * 48 + head], m);
                 o += reinterpret_cast<const float*>(smem_raw + w * per_warp)[i];
             }
             reinterpret_cast<T*>(p.out)[hbase * D + i] = from_f<T>(o / s);
             if (i % D == 0) {
                 float mt = kNone;
                 for (int w = 0; w < W; ++w) mt = fmaxf(mt, st[w * 48 + 16 + head]);
-                p.gmax[hbase + head] = mt; p.gsum[hbase + head] = s * __expf(m - mt);
+                p.gmax[hbase + head] = mt; p.gsum[hbase + head] = s * (X3 ? __expf(m - mt) : ex2_approx(fmaf(-mt, kLog2e, m)));
             }
         }
     } else {
@@ -311,7 +315,7 @@ acc_mma_kernel(const __grid_constant__ AttnParams p) {
                     *reinterpret_cast<uint2*>(orow) = make_uint2(w[0], w[1]);
                 }
             }
-            if (g == 0) { p.gmax[hbase + head] = m_true[h][e]; p.gsum[hbase + head] = s_run[h][e] * __expf(m_run[h][e] - m_true[h][e]); }
+            if (g == 0) { p.gmax[hbase + head] = m_true[h][e]; p.gsum[hbase + head] = s_run[h][e] * (X3 ? __expf(m_run[h][e] - m_true[h][e]) : ex2_approx(fmaf(-m_true[h][e], kLog2e, m_run[h][e]))); }
         }
     }
 }

@@ -86,7 +86,13 @@ def test_few_queries(dt, D, CR, G, T, TK, MTN, W):
     q, k, v, _ = _inputs(dt, 1, T, 2, G, D)
     full = ht.htree_forward(q, k, v, CR, MTN, TK)
     part = ht.htree_forward(q[:, T - W:].contiguous(), k, v, CR, MTN, TK, _q_offset=T - W)
-    assert _rel(part, full[:, T - W:]) < (2e-6 if dt == FP else 4e-3)
+    # Sums in another order differ by up to 1e-6 relative (the tensor core truncates its fp32 sums).  A 16-bit probability or result
+    # falls on the other side of a rounding boundary with 1e-6 / 2^-8 (bf16; 2^-11: fp16), 1 in 500 at most: 2-norm 2^-8 * sqrt(1/4000)
+    # = 6e-5 (bf16) or 2^-11 * sqrt(1/500) = 2e-5.  Room for three and five times that.
+    want = full[:, T - W:]
+    assert _rel(part, want) < (2e-6 if dt == FP else 2e-4)
+    if dt != FP and D > 32:
+        assert (part != want).float().mean().item() < 1e-2, "rows depend on how many queries share the call"
     torch.cuda.synchronize()
     ops.check_status()
 

@@ -97,15 +97,20 @@ acc_mma_kernel(const __grid_constant__ AttnParams p) {
         auto fill = [&](int c) {                                      // chunk c of this level
             const int p0 = par[c * PPC];
             if constexpr (CR == 16) {
-                ring.template copy<C::DATA>(0, blk + (uint64_t)(uint32_t)p0 * bstride, lane);
+                static_assert(!X3 || C::FACS_OFF == C::DATA, "the factors follow the operands");
+                ring.template copy<C::DATA + (X3 ? 16 : 0)>(0, blk + (uint64_t)(uint32_t)p0 * bstride, lane);
             } else {
                 const int p1 = c * PPC + 1 < np ? par[c * PPC + 1] : p0;  // past the end of the list: masked, any finite block
                 ring.template copy<C::DATA / 2>(0, blk + (uint64_t)(uint32_t)p0 * bstride, lane);
                 ring.template copy<C::DATA / 2>(C::DATA / 2, blk + (uint64_t)(uint32_t)p1 * bstride + C::ODD, lane);
+                if constexpr (X3) {
+                    ring.template copy<16>(C::DATA, blk + (uint64_t)(uint32_t)p0 * bstride + C::FACS_OFF, lane);
+                    ring.template copy<16>(C::DATA + 16, blk + (uint64_t)(uint32_t)p1 * bstride + C::FACS_OFF, lane);
+                }
             }
             const unsigned char* row = tab + (uint32_t)(rp - 16 * c) * C::TAB;
-            ring.template copy<C::TAB>(C::DATA, row, lane);
-            if constexpr (C::DUAL) ring.template copy<C::TAB>(C::DATA + C::TAB, rp - 16 * c >= 8 ? row - 8 * C::TAB : row, lane);
+            ring.template copy<C::TAB>(C::TAB_OFF, row, lane);
+            if constexpr (C::DUAL) ring.template copy<C::TAB>(C::TAB_OFF + C::TAB, rp - 16 * c >= 8 ? row - 8 * C::TAB : row, lane);
         };
         ring.start();
         int next = first;
@@ -143,7 +148,14 @@ acc_mma_kernel(const __grid_constant__ AttnParams p) {
             if (mask == 0) continue;
             const LaneBase<D, X3, CR> lb(slot, lane);
             float S[NH][4];
-            score_t<T, D, X3, NH, CR>(lb, slot + C::DATA, r, q, S);
+            float2 fac[2];
+            chunk_factors<D, X3, CR>(slot, fac);
+            score_t<T, D, X3, NH, CR>(lb, slot, r, q, S);
+            if constexpr (X3) {
+                const float f0 = fac[0].x * q.inv, f1 = fac[1].x * q.inv;
+#pragma unroll
+                for (int h = 0; h < NH; ++h) { S[h][0] *= f0; S[h][1] *= f0; S[h][2] *= f1; S[h][3] *= f1; }
+            }
             if (mask != 0xffffu) {
                 const bool c0 = (mask >> g) & 1, c1 = (mask >> (g + 8)) & 1;
 #pragma unroll
@@ -189,6 +201,8 @@ acc_mma_kernel(const __grid_constant__ AttnParams p) {
                 exponents();
             }
             uint32_t pb[NH][2], pl[X3 ? NH : 1][2];
+            float ratio[2], vfac = fac[0].y;                          // split-half: what brings the block's values back
+            if constexpr (X3 && CR == 8) vfac = common_factor(fac[0].y, fac[1].y, ratio);
 #pragma unroll
             for (int h = 0; h < NH; ++h) {
                 float P[4];
@@ -198,6 +212,7 @@ acc_mma_kernel(const __grid_constant__ AttnParams p) {
                 s_run[h][1] += P[1] + P[3];
                 if constexpr (X3) {
                     uint32_t h0, l0, h1, l1;
+                    if constexpr (CR == 8) { P[0] *= ratio[0]; P[1] *= ratio[0]; P[2] *= ratio[1]; P[3] *= ratio[1]; }
                     split_half2(P[0], P[1], h0, l0); split_half2(P[2], P[3], h1, l1);
                     pb[h][0] = movm(h0); pb[h][1] = movm(h1);
                     pl[X3 ? h : 0][0] = movm(l0); pl[X3 ? h : 0][1] = movm(l1);
@@ -221,7 +236,7 @@ acc_mma_kernel(const __grid_constant__ AttnParams p) {
                         mma_acc<FT>(acc, vl, pb[h][0], pb[h][1]);
                         mma_acc<FT>(acc, va, pb[h][0], pb[h][1]);
 #pragma unroll
-                        for (int u = 0; u < 4; ++u) O[h][i][u] += acc[u];
+                        for (int u = 0; u < 4; ++u) O[h][i][u] = fmaf(acc[u], vfac, O[h][i][u]);
                     }
                 } else {
 #pragma unroll

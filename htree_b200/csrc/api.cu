@@ -75,7 +75,7 @@ struct BwdLayout {
     BwdParams bp;
     int64_t acc_bytes, scratch_bytes, zero_bytes;
     int64_t acck[HTREE_MAX_LEVELS], accv[HTREE_MAX_LEVELS], gk[HTREE_MAX_LEVELS], gv[HTREE_MAX_LEVELS];
-    int64_t o_qb, o_dob, o_stp, o_sts, o_rank, o_cnt, o_base, o_entries, o_items, o_nitems;
+    int64_t o_qb, o_dob, o_stp, o_sts, o_fac, o_rank, o_cnt, o_base, o_entries, o_items, o_nitems;
     int total, per_launch;
 };
 
@@ -114,7 +114,7 @@ static int bwd_layout(const HtreeShape* s, int L, const int32_t* ln, int64_t bud
         const int64_t nw = (Tq + most - 1) / most;
         subq = (Tq + nw - 1) / nw;
         const int64_t visits = subq * MV;
-        bytes = up(subq * qb) * 2 + up(visits * sb) * 2 + up(visits * 4) + up(visits * 8) + 2 * up(NK * 4) + up((visits / 8 + NK) * 16) + 256;
+        bytes = up(subq * qb) * 2 + up(visits * sb) * 2 + up(visits * 4) + (x3 ? up(visits * 16) + up(subq * L * 8) : up(visits * 8)) + 2 * up(NK * 4) + up((visits / 8 + NK) * 16) + 256;
         if (bytes <= budget && visits < (int64_t(1) << 31)) { bp.nw = (int32_t)nw; break; }
     }
     if (bp.nw == 0) return HTREE_E_SCRATCH;
@@ -136,7 +136,8 @@ static int bwd_layout(const HtreeShape* s, int L, const int32_t* ln, int64_t bud
     auto take = [&](int64_t n) { const int64_t o = at; at += up(n); return o; };
     y.o_qb = take(per * subq * qb); y.o_dob = take(per * subq * qb);
     y.o_stp = take(per * subq * MV * sb); y.o_sts = take(per * subq * MV * sb);
-    y.o_rank = take(per * subq * MV * 4); y.o_entries = take(per * subq * MV * 8);
+    y.o_fac = x3 ? take(per * subq * L * 8) : -1;
+    y.o_rank = take(per * subq * MV * 4); y.o_entries = take(per * subq * MV * (int64_t)(x3 ? sizeof(BwdEntry<true>) : sizeof(BwdEntry<false>)));
     y.o_cnt = take(per * NK * 4); y.o_base = take(per * NK * 8);
     y.o_items = take(per * bp.cap * (int64_t)sizeof(BwdItem)); y.o_nitems = take(per * 4);
     y.scratch_bytes = at;
@@ -554,7 +555,8 @@ int htree_b200_run_backward(const HtreeShape* shape, const void* q, void* const*
     p.tab = table; p.out = const_cast<void*>(out); p.dO = dO; p.gmax = const_cast<float*>(gmax); p.gsum = const_cast<float*>(gsum);
     p.dq = typed ? nullptr : static_cast<float*>(dq); p.dq_typed = typed ? dq : nullptr;
     bp.qb = sb + y.o_qb; bp.dob = sb + y.o_dob; bp.stp = sb + y.o_stp; bp.sts = sb + y.o_sts;
-    bp.rank = reinterpret_cast<int32_t*>(sb + y.o_rank); bp.entries = reinterpret_cast<uint2*>(sb + y.o_entries);
+    bp.fac = y.o_fac < 0 ? nullptr : reinterpret_cast<float2*>(sb + y.o_fac);
+    bp.rank = reinterpret_cast<int32_t*>(sb + y.o_rank); bp.entries = sb + y.o_entries;
     bp.cnt = reinterpret_cast<int32_t*>(sb + y.o_cnt); bp.base = reinterpret_cast<int2*>(sb + y.o_base);
     bp.items = reinterpret_cast<BwdItem*>(sb + y.o_items); bp.nitems = reinterpret_cast<int32_t*>(sb + y.o_nitems);
     cudaStream_t st = (cudaStream_t)stream;

@@ -48,7 +48,7 @@ __global__ void __launch_bounds__(256) bwd_fill_kernel(const __grid_constant__ B
     const int64_t grp = (int64_t)blockIdx.y * bp.subq + qi;
     const int64_t qidx = ((int64_t)b * p.Tq + tl) * p.Hkv + hk;
     const int t = p.t0 + tl;
-    uint2* entries = bp.entries + (int64_t)blockIdx.y * bp.subq * bp.MV;
+    const int64_t entry0 = (int64_t)blockIdx.y * bp.subq * bp.MV;
     BwdItem* items = bp.items + (int64_t)blockIdx.y * bp.cap;
     for (int l = p.L - 1; l >= 0; --l) {
         if (bp.voff[l] < 0) continue;
@@ -66,7 +66,13 @@ __global__ void __launch_bounds__(256) bwd_fill_kernel(const __grid_constant__ B
             const int64_t v = grp * bp.MV + bp.voff[l] + i;
             const int2 at = base[x];
             const int rank = bp.rank[v];
-            entries[at.x + rank] = make_uint2((uint32_t)v, (uint32_t)grp | ((uint32_t)(rp - CR * i) << 15));
+            const uint32_t where = (uint32_t)grp | ((uint32_t)(rp - CR * i) << 15);
+            if (bp.fac) {
+                const float2 f = bp.fac[grp * p.L + l];
+                reinterpret_cast<BwdEntry<true>*>(bp.entries)[entry0 + at.x + rank] = BwdEntry<true>{(uint32_t)v, where, f.x, f.y};
+            } else {
+                reinterpret_cast<BwdEntry<false>*>(bp.entries)[entry0 + at.x + rank] = BwdEntry<false>{(uint32_t)v, where};
+            }
             if (rank % bp.seg == 0) items[at.y + rank / bp.seg] = BwdItem{bp.koff[l] + x, at.x + rank, min(bp.seg, cnt[x] - rank), 0};
         }
     }
@@ -81,11 +87,13 @@ __global__ void __launch_bounds__(256) bwd_fill_kernel(const __grid_constant__ B
 // groups of 9 to 16 heads of 128 (65536 positions, 64 heads: 13.2 -> 12.4 ms; with 8 heads a group three slots keep a lead of 1%).
 template <int D, bool X3, int NH, bool KEYS>
 constexpr int dkv_stages() { return X3 || (KEYS && D == 128 && NH == 2) ? 2 : 3; }
-template <int D, bool X3>
-constexpr int dkv_min_blocks() { return X3 ? (D == 128 ? 2 : 3) : D == 128 ? 3 : 4; }
+// Blocks per SM that the registers have to allow: six for the smallest split-half dV accumulators (80 registers; the compiler's 83 and
+// 86 left five).
+template <int D, bool X3, int CR, bool KEYS>
+constexpr int dkv_min_blocks() { return X3 ? (D == 128 ? 2 : !KEYS && (D == 32 || CR == 8) ? 6 : 3) : D == 128 ? 3 : 4; }
 
 template <typename T, int D, bool X3, int NH, int CR, bool KEYS>
-__global__ void __launch_bounds__(128, dkv_min_blocks<D, X3>()) bwd_dkv_kernel(const __grid_constant__ BwdParams bp) {
+__global__ void __launch_bounds__(128, dkv_min_blocks<D, X3, CR, KEYS>()) bwd_dkv_kernel(const __grid_constant__ BwdParams bp) {
     using BF = BForm<D, X3, NH, CR>;
     using C = TForm<D, X3, CR>;
     using FT = typename std::conditional<X3 || KEYS, __half, T>::type;      // operand type of the products
@@ -103,7 +111,8 @@ __global__ void __launch_bounds__(128, dkv_min_blocks<D, X3>()) bwd_dkv_kernel(c
     const BwdItem item = bp.items[(int64_t)ls * bp.cap + it];
     Ring ring;
     ring.init(smem_raw + (size_t)warp * Ring::kBytes);
-    const uint2* entries = bp.entries + (int64_t)ls * bp.subq * bp.MV + item.start;
+    using Entry = BwdEntry<X3>;
+    const Entry* entries = reinterpret_cast<const Entry*>(bp.entries) + (int64_t)ls * bp.subq * bp.MV + item.start;
     const unsigned char* qsrc = KEYS ? bp.qb : bp.dob;
     const unsigned char* ssrc = KEYS ? bp.sts : bp.stp;
     const unsigned char* tab = reinterpret_cast<const unsigned char*>(p.tab);
@@ -116,17 +125,38 @@ __global__ void __launch_bounds__(128, dkv_min_blocks<D, X3>()) bwd_dkv_kernel(c
 #pragma unroll
         for (int n = 0; n < NT; ++n) acc[i][n][0] = acc[i][n][1] = acc[i][n][2] = acc[i][n][3] = 0.f;
 
-    uint2 cur = entries[min(lane, len - 1)], nxt = entries[min(32 + lane, len - 1)];
+    Entry cur = entries[min(lane, len - 1)], nxt = entries[min(32 + lane, len - 1)];
+    static_assert(!X3 || NSTG == 2, "a step's factors are taken when the next one is fetched");
+    float fa = 0.f, fb = 0.f;                      // split-half: the factors of the visits fetched last
+    bool differ = false;                           // do they differ among the 32 of `cur`?
+    auto compare = [&]() {
+        if constexpr (X3) {
+            const float f = KEYS ? cur.fk : cur.fv;
+            fa = fb = __shfl_sync(0xffffffffu, f, 0);
+            differ = __any_sync(0xffffffffu, f != fa);
+        }
+    };
+    compare();
     auto fill = [&](int s) {                       // operand, record and table row of the step's one or two visits
         const int e0 = s * VPS;
-        if (e0 && (e0 & 31) == 0) { cur = nxt; nxt = entries[min(e0 + 32 + lane, len - 1)]; }
-        const uint32_t ax = __shfl_sync(0xffffffffu, cur.x, e0 & 31), ay = __shfl_sync(0xffffffffu, cur.y, e0 & 31);
+        if (e0 && (e0 & 31) == 0) {
+            cur = nxt; nxt = entries[min(e0 + 32 + lane, len - 1)];
+            compare();
+        }
+        if constexpr (X3) {
+            if (differ) {
+                const float f = KEYS ? cur.fk : cur.fv;
+                fa = __shfl_sync(0xffffffffu, f, e0 & 31);
+                if constexpr (VPS == 2) fb = __shfl_sync(0xffffffffu, f, (e0 + 1) & 31);      // (past the end: the last entry again)
+            }
+        }
+        const uint32_t ax = __shfl_sync(0xffffffffu, cur.visit, e0 & 31), ay = __shfl_sync(0xffffffffu, cur.where, e0 & 31);
         ring.template copy<NH * QB>(0, qsrc + (int64_t)(ay & 0x7fffu) * (NH * QB), lane);
         ring.template copy<NH * SB>(2 * QB, ssrc + (int64_t)ax * (NH * SB), lane);
         if constexpr (KEYS) ring.template copy<TAB>(2 * QB + 2 * SB, tab + (int64_t)(ay >> 15) * C::TAB, lane);
         if constexpr (VPS == 2) {
             const int e1 = min(e0 + 1, len - 1);
-            const uint32_t bx = __shfl_sync(0xffffffffu, cur.x, e1 & 31), by = __shfl_sync(0xffffffffu, cur.y, e1 & 31);
+            const uint32_t bx = __shfl_sync(0xffffffffu, cur.visit, e1 & 31), by = __shfl_sync(0xffffffffu, cur.where, e1 & 31);
             ring.template copy<QB>(QB, qsrc + (int64_t)(by & 0x7fffu) * QB, lane);
             ring.template copy<SB>(2 * QB + SB, ssrc + (int64_t)bx * SB, lane);
             if constexpr (KEYS) ring.template copy<TAB>(2 * QB + 2 * SB + TAB, tab + (int64_t)(by >> 15) * C::TAB, lane);
@@ -141,6 +171,7 @@ __global__ void __launch_bounds__(128, dkv_min_blocks<D, X3>()) bwd_dkv_kernel(c
 #pragma unroll 1
     for (int s = 0; s < steps; ++s) {
         __syncwarp();
+        const float f0 = fa, f1 = fb;              // of this step's visits
         if (next < steps) fill(next);
         ring.commit();
         ++next;
@@ -157,6 +188,17 @@ __global__ void __launch_bounds__(128, dkv_min_blocks<D, X3>()) bwd_dkv_kernel(c
                 const uint32_t o = pl * PLANE + lane * (4 * NT) + 4 * n;
                 const uint32_t x = lds32(ra + o), y = lone ? 0u : lds32(rb + o);
                 if (pl == 0) { bw[n][0] = x; bw[n][1] = y; } else { bl[X3 ? n : 0][0] = x; bl[X3 ? n : 0][1] = y; }
+            }
+        }
+        float vfac = f0;                           // what brings this step's products back
+        if (X3 && VPS == 2 && f0 != f1) {          // two visits in one product: to their common factor (a product by a power of two)
+            float ratio[2];
+            vfac = common_factor(fminf(fmaxf(f0, 0x1p-126f), 0x1p126f), fminf(fmaxf(f1, 0x1p-126f), 0x1p126f), ratio);
+            const __half2 r0 = __float2half2_rn(ratio[0]), r1 = __float2half2_rn(ratio[1]);
+#pragma unroll
+            for (int n = 0; n < NT; ++n) {
+                bw[n][0] = as_u32(__hmul2(as_h2(bw[n][0]), r0)); bw[n][1] = as_u32(__hmul2(as_h2(bw[n][1]), r1));
+                bl[X3 ? n : 0][0] = as_u32(__hmul2(as_h2(bl[X3 ? n : 0][0]), r0)); bl[X3 ? n : 0][1] = as_u32(__hmul2(as_h2(bl[X3 ? n : 0][1]), r1));
             }
         }
         if constexpr (KEYS && !X3) {
@@ -226,7 +268,7 @@ __global__ void __launch_bounds__(128, dkv_min_blocks<D, X3>()) bwd_dkv_kernel(c
                     mma_acc<FT>(t, ah, bl[X3 ? n : 0][0], bl[X3 ? n : 0][1]);
                     mma_acc<FT>(t, ah, bw[n][0], bw[n][1]);
 #pragma unroll
-                    for (int u = 0; u < 4; ++u) acc[i][n][u] += t[u];
+                    for (int u = 0; u < 4; ++u) acc[i][n][u] = fmaf(t[u], vfac, acc[i][n][u]);
                 }
             }
         }

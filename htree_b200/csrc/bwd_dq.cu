@@ -62,11 +62,29 @@ __global__ void __launch_bounds__(dq_warps<D, X3, NH>() * 32, dq_min_blocks<D, X
     load_query<T, D, X3, NH>(reinterpret_cast<const T*>(p.q) + hbase * D, G, g, r, p.scale, q);
     uint32_t dO[NH][2][KS], dOl[X3 ? NH : 1][2][X3 ? KS : 1];
     float Drow[NH][2], lse[NH][2], ginv[NH][2];
+    constexpr float kPScale = 16384.f;                  // split-half: P is carried times 2^14
+    float dscale = 1.f, dinv = 1.f;                     // split-half: dO times dscale; dinv = 1 / (dscale kPScale), for P dO and for dS
+    float bound_v = 0.f, bound_d = 0.f;                 // |P (dP - D)| as carried <= bound_v * the value block's factor + bound_d
+    float vtop = 0.f, sscale = 1.f;                     // the largest such factor so far, and the scale of dS that follows from it
+    if constexpr (X3) {
+        float most = 0.f;
+#pragma unroll
+        for (int h = 0; h < NH; ++h)
+#pragma unroll
+            for (int hf = 0; hf < 2; ++hf) {
+                float x[D / 8];
+                load_row_piece_f32<T, D>(reinterpret_cast<const T*>(p.dO) + (hbase + 8 * h + g) * D + hf * HALF + PPT * r, 8 * h + g < G, x);
+#pragma unroll
+                for (int i = 0; i < D / 8; ++i) most = fmaxf(most, fabsf(x[i]));
+            }
+        dscale = range_scale_coarse(redux_max_f32(most, 0xffffffffu));
+        dinv = pow2_inverse(dscale) * (1.f / kPScale);
+    }
 #pragma unroll
     for (int h = 0; h < NH; ++h) {
         const int head = 8 * h + g;
         const bool on = head < G;
-        float sum = 0.f;
+        float sum = 0.f, l1 = 0.f;
 #pragma unroll
         for (int hf = 0; hf < 2; ++hf) {
             const int64_t off = (hbase + head) * D + hf * HALF + PPT * r;
@@ -76,6 +94,8 @@ __global__ void __launch_bounds__(dq_warps<D, X3, NH>() * 32, dq_min_blocks<D, X
                 load_row_piece_f32<T, D>(reinterpret_cast<const T*>(p.out) + off, on, o);
 #pragma unroll
                 for (int i = 0; i < D / 16; ++i) {
+                    x[2 * i] *= dscale; x[2 * i + 1] *= dscale;
+                    l1 += fabsf(x[2 * i]) + fabsf(x[2 * i + 1]);
                     sum += x[2 * i] * o[2 * i] + x[2 * i + 1] * o[2 * i + 1];
                     split_half2(x[2 * i], x[2 * i + 1], dO[h][hf][i], dOl[X3 ? h : 0][hf][X3 ? i : 0]);
                 }
@@ -92,6 +112,12 @@ __global__ void __launch_bounds__(dq_warps<D, X3, NH>() * 32, dq_min_blocks<D, X
         }
         sum += __shfl_xor_sync(0xffffffffu, sum, 1);
         sum += __shfl_xor_sync(0xffffffffu, sum, 2);
+        if constexpr (X3) {
+            l1 += __shfl_xor_sync(0xffffffffu, l1, 1);
+            l1 += __shfl_xor_sync(0xffffffffu, l1, 2);
+            bound_v = fmaxf(bound_v, kPScale * 16384.f * redux_max_f32(l1, 0xffffffffu));      // values are carried below 2^14
+            bound_d = fmaxf(bound_d, kPScale * redux_max_f32(fabsf(sum), 0xffffffffu));
+        }
 #pragma unroll
         for (int e = 0; e < 2; ++e) {
             const int hd = 8 * h + 2 * r + e;
@@ -99,7 +125,7 @@ __global__ void __launch_bounds__(dq_warps<D, X3, NH>() * 32, dq_min_blocks<D, X
             const float gm = hd < G ? p.gmax[hbase + hd] : 0.f, gs = hd < G ? p.gsum[hbase + hd] : 1.f;
             // 16-bit: P = 2^(S log2 e - lse); split-half: exp(S - gmax) * ginv (an exponent re-based by log2 e rounds at 1e-6)
             lse[h][e] = X3 ? gm : (hd < G ? gm * kLog2e + __log2f(gs) : INFINITY);
-            ginv[h][e] = hd < G ? 1.f / gs : 0.f;
+            ginv[h][e] = hd < G ? kPScale / gs : 0.f;
         }
     }
 
@@ -136,6 +162,7 @@ __global__ void __launch_bounds__(dq_warps<D, X3, NH>() * 32, dq_min_blocks<D, X
 #pragma unroll
         for (int i = 0; i < KS; ++i) dq[h][i][0] = dq[h][i][1] = dq[h][i][2] = dq[h][i][3] = 0.f;
 
+    float back = dinv;                                                // split-half: times dS as carried = dS
     for (int l = L - 1; l >= 0; --l) {
         if (bp.voff[l] < 0) continue;
         const int Nl = p.ln[l];
@@ -160,10 +187,12 @@ __global__ void __launch_bounds__(dq_warps<D, X3, NH>() * 32, dq_min_blocks<D, X
                 const int p1 = c * PPC + 1 < np ? par[c * PPC + 1] : p0;
                 ring.template copy<PB>(C::K2_OFF, kblk + (uint64_t)(uint32_t)p1 * kstride + 2 * C::ODD, lane);
                 ring.template copy<PB>(C::V2_OFF, vblk + (uint64_t)(uint32_t)p1 * vstride, lane);
+                if constexpr (X3) ring.template copy<16>(C::DATA + 16, kblk + (uint64_t)(uint32_t)p1 * kstride + C::FACS_OFF, lane);
             }
+            if constexpr (X3) ring.template copy<16>(C::DATA, kblk + (uint64_t)(uint32_t)p0 * kstride + C::FACS_OFF, lane);
             const unsigned char* row = reinterpret_cast<const unsigned char*>(p.tab) + (uint32_t)(rp - 16 * c) * C::TAB;
-            ring.template copy<C::TAB>(C::DATA, row, lane);
-            if constexpr (C::DUAL) ring.template copy<C::TAB>(C::DATA + C::TAB, rp - 16 * c >= 8 ? row - 8 * C::TAB : row, lane);
+            ring.template copy<C::TAB>(C::TAB_OFF, row, lane);
+            if constexpr (C::DUAL) ring.template copy<C::TAB>(C::TAB_OFF + C::TAB, rp - 16 * c >= 8 ? row - 8 * C::TAB : row, lane);
         };
         ring.start();
         int next = 0;
@@ -174,8 +203,22 @@ __global__ void __launch_bounds__(dq_warps<D, X3, NH>() * 32, dq_min_blocks<D, X
         }
         // this visit's place in its parent's list
         int32_t* cnt = bp.cnt + (int64_t)blockIdx.y * bp.NK + bp.koff[l];
+        float v = 0.f;                                                // split-half: the largest factor of the values that will be met
         for (int i = lane; i < np; i += 32) {
             bp.rank[(int64_t)grp * bp.MV + bp.voff[l] + i] = atomicAdd(cnt + par[i], 1);
+            if constexpr (X3) v = fmaxf(v, __ldg(reinterpret_cast<const float*>(kblk + (uint64_t)(uint32_t)par[i] * ((uint32_t)p.Hkv * C::BLOCK) + C::FACS_OFF) + 1));
+        }
+        if constexpr (X3) {
+            // dS's scale follows from a bound, 2^4 to 2^8 above what ordinary data reach at P = 1.  Found per level: per chunk, from the
+            // largest |dS| or from the chunk's own factor, cost the pass 5 to 7% (32-wide heads)
+            v = redux_max_f32(v, 0xffffffffu);
+            if (v > vtop) {
+                const float s = range_scale_coarse(fmaf(bound_v, v, bound_d)), f = s * pow2_inverse(sscale);
+                vtop = v; sscale = s; back = dinv * pow2_inverse(s);
+#pragma unroll
+                for (int h = 0; h < NH; ++h) { Drow[h][0] *= f; Drow[h][1] *= f; }
+            }
+            if (lane == 0) bp.fac[(int64_t)grp * L + l] = make_float2(back * q.inv, dinv);
         }
         if (l > 0) {
             for (int i = lane; i < (nc + 31) / 32; i += 32) selw[i] = 0u;
@@ -204,7 +247,7 @@ __global__ void __launch_bounds__(dq_warps<D, X3, NH>() * 32, dq_min_blocks<D, X
             if (16 * c + 15 > rp) mask &= (2u << (rp - 16 * c)) - 1u;
             const uint32_t slot = ring.wait();
             const LaneBase<D, X3, CR> lb(slot, lane);
-            const uint32_t tabs = slot + C::DATA;
+            const uint32_t tabs = slot + C::TAB_OFF;
 
             uint32_t pw[NH][2], sw[NH][2], pwl[X3 ? NH : 1][2], swl[X3 ? NH : 1][2];   // P^T, dS^T: word w = child g + 8w, heads 2r, 2r+1
             if (mask == 0) {
@@ -233,17 +276,21 @@ __global__ void __launch_bounds__(dq_warps<D, X3, NH>() * 32, dq_min_blocks<D, X
                     }
                 }
                 float S[NH][4];
-                score_t<T, D, X3, NH, CR>(lb, tabs, r, q, S);
+                float2 fac[2];
+                chunk_factors<D, X3, CR>(slot, fac);
+                score_t<T, D, X3, NH, CR>(lb, slot, r, q, S);
+                const float sfac[2] = {fac[0].x * q.inv, fac[1].x * q.inv};
                 const bool c0 = (mask >> g) & 1, c1 = (mask >> (g + 8)) & 1;
                 uint32_t db[NH][2], dbl[X3 ? NH : 1][2];       // dS^T as B fragments (children x heads)
+                if constexpr (X3) { fac[0].y *= sscale; fac[1].y *= sscale; }
 #pragma unroll
                 for (int h = 0; h < NH; ++h) {
                     float P[4], dS[4];
 #pragma unroll
                     for (int i = 0; i < 4; ++i) {
-                        P[i] = X3 ? __expf(S[h][i] - lse[h][i & 1]) * ginv[h][i & 1] : ex2_approx(fmaf(S[h][i], kLog2e, -lse[h][i & 1]));
+                        P[i] = X3 ? __expf(fmaf(S[h][i], sfac[i >> 1], -lse[h][i & 1])) * ginv[h][i & 1] : ex2_approx(fmaf(S[h][i], kLog2e, -lse[h][i & 1]));
                         P[i] = (i < 2 ? c0 : c1) ? P[i] : 0.f;
-                        dS[i] = P[i] * (dP[h][i] - Drow[h][i & 1]);
+                        dS[i] = P[i] * (X3 ? fmaf(dP[h][i], fac[i >> 1].y, -Drow[h][i & 1]) : dP[h][i] - Drow[h][i & 1]);
                     }
                     if constexpr (X3) {
                         split_half2(P[0], P[1], pw[h][0], pwl[X3 ? h : 0][0]); split_half2(P[2], P[3], pw[h][1], pwl[X3 ? h : 0][1]);
@@ -288,6 +335,9 @@ __global__ void __launch_bounds__(dq_warps<D, X3, NH>() * 32, dq_min_blocks<D, X
                         }
                     }
                 } else {
+                    float ratio[2] = {1.f, 1.f}, kfac = fac[0].x;
+                    if constexpr (CR == 8 && C::KSCALED) kfac = common_factor(fac[0].x, fac[1].x, ratio);
+                    kfac *= back;
 #pragma unroll
                     for (int ks = 0; ks < KS; ++ks) {
                         uint32_t mh[4], ml[4], ah[4], al[4];
@@ -303,22 +353,23 @@ __global__ void __launch_bounds__(dq_warps<D, X3, NH>() * 32, dq_min_blocks<D, X
                             const float2 hi = FS::unpack(mh[m]), lo = FS::unpack(ml[m]);
                             x[m] = make_float2(hi.x + lo.x, hi.y + lo.y);
                         }
-                        const float2 c2 = make_float2(cs, cs), s2 = make_float2(sn, sn), n2 = make_float2(-sn, -sn);
 #pragma unroll
                         for (int tile = 0; tile < 2; ++tile) {
+                            const float ct = CR == 8 && C::KSCALED ? cs * ratio[tile] : cs, st = CR == 8 && C::KSCALED ? sn * ratio[tile] : sn;
+                            const float2 c2 = make_float2(ct, ct), s2 = make_float2(st, st), n2 = make_float2(-st, -st);
                             const float2 u = ffma2(x[2 + tile], s2, fmul2(x[tile], c2)), w = ffma2(x[tile], n2, fmul2(x[2 + tile], c2));
                             split_half2(u.x, u.y, ah[2 * tile], al[2 * tile]);
                             split_half2(w.x, w.y, ah[2 * tile + 1], al[2 * tile + 1]);
                         }
 #pragma unroll
                         for (int h = 0; h < NH; ++h) {
-                            // from zero, then a round-to-nearest fp32 add (the tensor core's accumulation truncates)
+                            // from zero, then a round-to-nearest fp32 multiply-add (the tensor core's accumulation truncates)
                             float acc[4];
                             mma_zero<__half>(acc, ah, dbl[X3 ? h : 0][0], dbl[X3 ? h : 0][1]);
                             mma_acc<__half>(acc, al, db[h][0], db[h][1]);
                             mma_acc<__half>(acc, ah, db[h][0], db[h][1]);
 #pragma unroll
-                            for (int i = 0; i < 4; ++i) dq[h][ks][i] += acc[i];
+                            for (int i = 0; i < 4; ++i) dq[h][ks][i] = fmaf(acc[i], kfac, dq[h][ks][i]);
                         }
                     }
                 }

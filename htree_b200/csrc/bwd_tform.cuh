@@ -7,12 +7,21 @@
 // visits of one parent with dK, dV in registers: it fetches the queries (4 KB) and that kilobyte, and reduces once per 64 or so
 // visits.  The order of a parent's visits comes from a counting sort (ranks taken by the first pass, one scan, one fill).
 //
+// Split-half operands are brought to the top of half's range by powers of two (range_scale): the heads and the output gradients of a
+// group by one each, P (at most 1) by 2^14, dS by one per group and level, from a bound on it.  What undoes them is one factor for dK and
+// one for dV, which travel in a visit's entry and are applied where its product joins the fp32 sum: gradients of a mean-reduced loss
+// keep their digits, and a visit does not depend on other groups.
+//
 // Work is cut into windows of `subq` queries of one (batch, KV head) unit, small enough for a window's blocked queries to stay
 // in L2 while its parents gather from them, and into launches of `nsub` windows, whose P and dS fit the caller's buffer.
 #pragma once
 #include "tform.cuh"
 
 namespace htree {
+
+// A visit in its parent's list: visit slot, group | table row << 15, and, split-half, the factors of dK and dV.
+template <bool X3> struct BwdEntry { uint32_t visit, where; };
+template <> struct __align__(16) BwdEntry<true> { uint32_t visit, where; float fk, fv; };
 
 struct BwdItem { int32_t key, start, len, pad; };     // a piece of one parent's visit list
 
@@ -26,10 +35,11 @@ struct BwdParams {
     unsigned char* dob;                      // blocked output gradients [group][half]
     unsigned char* stp;                      // P  [group * MV + visit][half]
     unsigned char* sts;                      // dS
+    float2* fac;                             // split-half: {dK, dV} factors of the visits of a group and level, [group * L + level]; else NULL
     int32_t* rank;                           // [group * MV + visit]
     int32_t* cnt;                            // [nsub][NK]
     int2* base;                              // [nsub][NK]: first entry, first item
-    uint2* entries;                          // [nsub][subq * MV]
+    void* entries;                           // [nsub][subq * MV] Entry
     BwdItem* items;                          // [nsub][cap]
     int32_t* nitems;                         // [nsub]
     float* acck[HTREE_MAX_LEVELS];           // dK', dV of every level in accumulator order, [block][i][child tile][lane][4]

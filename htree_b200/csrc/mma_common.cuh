@@ -402,7 +402,8 @@ __device__ __forceinline__ void load_rows_half(const T* base, int g, int r, cons
 
 // ---------------------------------------------------------------------------------------------------------------
 // fp32 storage on the tensor cores: split-half products.  A value x is carried as hi = half(x) and lo = half(x - hi)
-// (22 significand bits together); a product of two such values is formed as hi*hi + hi*lo + lo*hi by three
+// (22 significand bits together, while |x| is between 2^-2 and 2^16: half ends at 2^-24, so a pair is good to 2^-25 absolute
+// whatever its value, and what is smaller is brought there first, see range_scale); a product of two such values is formed as hi*hi + hi*lo + lo*hi by three
 // mma.sync.m16n8k16 f16 instructions with fp32 accumulation (lo*lo is below fp32 resolution).  This keeps the scores,
 // and with them the Top-K decisions, at fp32 accuracy, which single TF32 / half products (10-11 bits) do not.
 // 64-wide heads only: the fp32 query rows already take 32 registers per thread.
@@ -415,6 +416,20 @@ __device__ __forceinline__ void split_half2(float x0, float x1, uint32_t& hi, ui
     hi = *reinterpret_cast<const uint32_t*>(&h);
     lo = *reinterpret_cast<const uint32_t*>(&l);
 }
+
+// The power of two that brings a largest magnitude m into [2^13, 2^14), so that everything down to 2^-15 of it keeps its 22 bits as a
+// half pair, a rotation (factor sqrt 2) stays in range, and nothing needs clamping.  1 where m is not finite.  Limited to
+// 2^-115 .. 2^126, so that the inverse is a normal number too: for m = 0 it is the smallest one, neutral in a maximum of inverses.
+__device__ __forceinline__ float range_scale(float m) {
+    const int e = __float_as_int(m) >> 23;
+    return e >= 255 ? 1.f : __int_as_float(min(267 - e, 253) << 23);
+}
+// The same in steps of 2^4, into [2^10, 2^14): where factors of different groups meet in one product, most of them are then equal.
+__device__ __forceinline__ float range_scale_coarse(float m) {
+    const int e = __float_as_int(m) >> 23;
+    return e >= 255 ? 1.f : __int_as_float((((min(267 - e, 251) + 1) & ~3) - 1) << 23);      // 127 + 4 n, rounded down
+}
+__device__ __forceinline__ float pow2_inverse(float s) { return __int_as_float((254 << 23) - __float_as_int(s)); }     // of 2^-126 .. 2^126
 
 // fp32 rows g and g+8 of a [heads, D] block: raw[rr][hf][i] = bits of element hf*D/2 + PPT*r + i (zero for rows beyond the group)
 template <int D>

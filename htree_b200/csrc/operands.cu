@@ -101,6 +101,32 @@ __global__ void __launch_bounds__(128) pack_blocks_kernel(const __grid_constant_
     const T* vs_ = reinterpret_cast<const T*>(a.v) + base;
     unsigned char* dst = reinterpret_cast<unsigned char*>(a.blk) + blk * C::BLOCK;
 
+    // ---- split-half: the block's factors, from the largest magnitudes of its rows (read here and, from L1, again below) ----
+    constexpr int NB = CR / 8;
+    float kscale = 1.f, vscale = 1.f;
+    if constexpr (X3) {
+        float km = 0.f, vm = 0.f;
+#pragma unroll
+        for (int tl = 0; tl < NB; ++tl) {
+            const int child = 8 * tl + g;
+#pragma unroll
+            for (int hf = 0; hf < 2; ++hf) {
+                float x[PPT];
+                if constexpr (C::KSCALED) {
+                    load_piece<T, PPT>(ks_ + child * rs + hf * HALF + PPT * r, child < cnt, x);
+#pragma unroll
+                    for (int i = 0; i < PPT; ++i) km = fmaxf(km, fabsf(x[i]));
+                }
+                load_piece<T, PPT>(vs_ + child * rs + hf * HALF + PPT * r, child < cnt, x);
+#pragma unroll
+                for (int i = 0; i < PPT; ++i) vm = fmaxf(vm, fabsf(x[i]));
+            }
+        }
+        if constexpr (C::KSCALED) kscale = range_scale(redux_max_f32(km, 0xffffffffu));
+        vscale = range_scale(redux_max_f32(vm, 0xffffffffu));
+        if (lane == 0) *reinterpret_cast<float2*>(dst + C::FACS_OFF) = make_float2(pow2_inverse(kscale), pow2_inverse(vscale));
+    }
+
     // ---- keys: rotate by the position inside the chunk ----
     uint32_t kw[2][2][PPT / 2], kl[2][2][X3 ? PPT / 2 : 1];   // [tile or version][half][pair of pairs]
 #pragma unroll
@@ -110,6 +136,10 @@ __global__ void __launch_bounds__(128) pack_blocks_kernel(const __grid_constant_
         float lo[PPT], hi[PPT], x[PPT], y[PPT];
         load_piece<T, PPT>(ks_ + child * rs + PPT * r, on, lo);
         load_piece<T, PPT>(ks_ + child * rs + HALF + PPT * r, on, hi);
+        if constexpr (C::KSCALED) {
+#pragma unroll
+            for (int i = 0; i < PPT; ++i) { lo[i] *= kscale; hi[i] *= kscale; }
+        }
         const float4* cp = reinterpret_cast<const float4*>(a.cosc + (8 * tl + g) * HALF + PPT * r);
         const float4* sp = reinterpret_cast<const float4*>(a.sinc + (8 * tl + g) * HALF + PPT * r);
 #pragma unroll
@@ -146,7 +176,6 @@ __global__ void __launch_bounds__(128) pack_blocks_kernel(const __grid_constant_
     }
 
     // ---- values: pairs of children per word ----
-    constexpr int NB = CR / 8;
     uint32_t vw[NB][VB], vl[X3 ? NB : 1][X3 ? VB : 1];
 #pragma unroll
     for (int j = 0; j < NB; ++j) {
@@ -156,7 +185,7 @@ __global__ void __launch_bounds__(128) pack_blocks_kernel(const __grid_constant_
         load_piece<T, VB>(vs_ + (c0 + 1) * rs + VB * g, c0 + 1 < cnt, x1);
 #pragma unroll
         for (int w = 0; w < VB; ++w) {
-            if constexpr (X3) split_half2(clamp_half(x0[w]), clamp_half(x1[w]), vw[j][w], vl[X3 ? j : 0][X3 ? w : 0]);
+            if constexpr (X3) split_half2(clamp_half(x0[w] * vscale), clamp_half(x1[w] * vscale), vw[j][w], vl[X3 ? j : 0][X3 ? w : 0]);
             else vw[j][w] = Frag<T>::pack(x0[w], x1[w]);      // exact: the values are of this type
         }
     }
@@ -223,7 +252,7 @@ __global__ void __launch_bounds__(128) pack_blocks_kernel(const __grid_constant_
                 load_piece<T, PPT>(vs_ + child * rs + hf * HALF + PPT * r, on, x);
 #pragma unroll
                 for (int i = 0; i < PPT / 2; ++i) {
-                    if constexpr (X3) split_half2(clamp_half(x[2 * i]), clamp_half(x[2 * i + 1]), rw[tl][hf][i], rl[X3 ? tl : 0][hf][X3 ? i : 0]);
+                    if constexpr (X3) split_half2(clamp_half(x[2 * i] * vscale), clamp_half(x[2 * i + 1] * vscale), rw[tl][hf][i], rl[X3 ? tl : 0][hf][X3 ? i : 0]);
                     else rw[tl][hf][i] = Frag<T>::pack(x[2 * i], x[2 * i + 1]);
                 }
             }
@@ -246,7 +275,7 @@ __global__ void __launch_bounds__(128) pack_blocks_kernel(const __grid_constant_
     }
 }
 
-size_t pack_block_bytes(int D, bool x3, int CR) { return (size_t)(x3 ? 2 : 1) * D * 2 * CR * (CR == 16 || !x3 ? 2 : 3); }
+size_t pack_block_bytes(int D, bool x3, int CR) { return (size_t)(x3 ? 2 : 1) * D * 2 * CR * (CR == 16 || !x3 ? 2 : 3) + (x3 ? 128 : 0); }
 
 bool pack_supported(int dtype, int K, int V, int CR) {
     (void)dtype;

@@ -23,7 +23,10 @@
 //                 of the query's list, which hold positions 8..15 of their chunk: one query rotation per chunk.  (16-bit storage
 //                 does not: a score's rounding is the rounding of these half-precision operands, 2^-11 |q||k|, and with scores of
 //                 70 another choice of operands moves probabilities by a percent.)
-//   split-half (fp32 storage, and every storage type with 32-wide heads): each part is a hi plane followed by a lo plane.
+//   split-half (fp32 storage, and every storage type with 32-wide heads): each part is a hi plane followed by a lo plane.  The keys
+//                 and the values of a block are multiplied by powers of two that bring their largest magnitudes to the top of half's range
+//                 (range_scale; not the keys of 64-wide heads, whose selection works on the plain ones), and the block ends in a line
+//                 with the inverse factors {keys, values}.  They belong to the block, so that no row depends on other blocks.
 #pragma once
 #include "mma_common.cuh"
 
@@ -35,13 +38,18 @@ struct TForm {
     static constexpr int PL = X3 ? 2 : 1;                                  // planes
     static constexpr int PART = D * 2 * CR;                                // bytes of one plane of one part of a block
     static constexpr bool DUAL = CR == 8 && !X3;                           // two query rotations per chunk
-    static constexpr int BLOCK = PL * PART * (CR == 16 || DUAL ? 2 : 3);   // bytes of a block in global memory
+    static constexpr int FACS = X3 ? 128 : 0;                              // the line of factors (a whole one: blocks stay aligned to lines)
+    static constexpr int BLOCK = PL * PART * (CR == 16 || DUAL ? 2 : 3) + FACS;   // bytes of a block in global memory
+    static constexpr int FACS_OFF = BLOCK - FACS;
+    static constexpr bool KSCALED = X3 && D != 64;                         // are a block's keys multiplied by their factor?
     static constexpr int ODD = DUAL ? 0 : PL * PART;                       // where an odd parent's copy starts in its block
     static constexpr int NTAB = DUAL ? 2 : 1;
     static constexpr int DATA = PL * D * 64;                               // bytes of a chunk in shared memory
     static constexpr int TAB = X3 ? D * 4 : D * 2;                         // one row of the rotary table: [cos | sin]
-    static constexpr int SLOT = DATA + NTAB * TAB;
     static constexpr int PPC = 16 / CR;                                    // parents per chunk
+    // a slot: operands, {key factor, value factor, -, -} per parent, table rows, all at whole lines like their sources
+    static constexpr int TAB_OFF = DATA + (X3 ? 128 : 0);
+    static constexpr int SLOT = TAB_OFF + NTAB * TAB;
     // part offsets in a slot: 16 children [K | V]; 8 children [K even | V even | K odd | V odd], split-half [.. | V odd | K odd]
     static constexpr int V_OFF = PL * PART;
     static constexpr int V2_OFF = (DUAL ? 3 : 2) * PL * PART, K2_OFF = (DUAL ? 2 : 3) * PL * PART;
@@ -71,6 +79,11 @@ __device__ __forceinline__ void ldmatrix_frag(uint32_t addr, uint32_t (&a)[4]) {
 }
 __device__ __forceinline__ void ldmatrix_trans_frag(uint32_t addr, uint32_t (&a)[4]) {
     asm("ldmatrix.sync.aligned.m8n8.x4.trans.shared.b16 {%0,%1,%2,%3}, [%4];\n" : "=r"(a[0]), "=r"(a[1]), "=r"(a[2]), "=r"(a[3]) : "r"(addr));
+}
+__device__ __forceinline__ float2 lds_f2(uint32_t addr) {
+    float2 x;
+    asm("ld.shared.v2.f32 {%0,%1}, [%2];\n" : "=f"(x.x), "=f"(x.y) : "r"(addr));
+    return x;
 }
 __device__ __forceinline__ uint4 lds_u4(uint32_t addr) {
     uint4 x;
@@ -138,11 +151,13 @@ template <> __device__ __forceinline__ void mma_zero<__nv_bfloat16>(float (&c)[4
 }
 
 // The query heads of a group as B fragments of the score product: lane (g, r) holds dims PPT*r + [0, PPT) of both halves of
-// head 8h + g.  16-bit path: IEEE half pairs; split-half path: fp32 values, already multiplied by the softmax scale.
+// head 8h + g.  16-bit path: IEEE half pairs; split-half path: fp32 values, already multiplied by the softmax scale and by the power
+// of two that brings the group's largest one to the top of half's range; `inv` is its inverse.
 template <typename T, int D, bool X3, int NH>
 struct QueryRegs {
     static constexpr int N = X3 ? D / 8 : D / 16;
     uint32_t v[NH][2][N];
+    float inv;
 };
 
 template <typename T, int D>
@@ -159,6 +174,7 @@ __device__ __forceinline__ void load_row_piece_f32(const T* p, bool on, float (&
 template <typename T, int D, bool X3, int NH>
 __device__ __forceinline__ void load_query(const T* base, int G, int g, int r, float scale, QueryRegs<T, D, X3, NH>& q) {
     constexpr int HALF = D / 2, PPT = HALF / 4;
+    float most = 0.f;
 #pragma unroll
     for (int h = 0; h < NH; ++h) {
         const int head = 8 * h + g;
@@ -170,7 +186,7 @@ __device__ __forceinline__ void load_query(const T* base, int G, int g, int r, f
                 float x[D / 8];
                 load_row_piece_f32<T, D>(p, on, x);
 #pragma unroll
-                for (int i = 0; i < D / 8; ++i) q.v[h][hf][i] = __float_as_uint(x[i] * scale);
+                for (int i = 0; i < D / 8; ++i) { q.v[h][hf][i] = __float_as_uint(x[i] * scale); most = fmaxf(most, fabsf(x[i] * scale)); }
             } else {
                 ldg_vec<PPT / 8>(p, on, q.v[h][hf]);
                 if (!std::is_same<T, __half>::value) {
@@ -182,6 +198,16 @@ __device__ __forceinline__ void load_query(const T* base, int G, int g, int r, f
                 }
             }
         }
+    }
+    if constexpr (X3) {
+        const float s = range_scale_coarse(redux_max_f32(most, 0xffffffffu));
+        q.inv = pow2_inverse(s);
+#pragma unroll
+        for (int h = 0; h < NH; ++h)
+#pragma unroll
+            for (int hf = 0; hf < 2; ++hf)
+#pragma unroll
+                for (int i = 0; i < D / 8; ++i) q.v[h][hf][i] = __float_as_uint(__uint_as_float(q.v[h][hf][i]) * s);
     }
 }
 
@@ -297,8 +323,26 @@ __device__ __forceinline__ void score_x3(const LaneBase<D, true, CR>& s, uint32_
         for (int i = 0; i < 4; ++i) S[h][i] += B[h][i] + C[h][i];
 }
 
+// The factors of a chunk's parents, .x of the keys and .y of the values: f[0] of rows 0..7, f[1] of rows 8..15 (one parent: the same).
+template <int D, bool X3, int CR>
+__device__ __forceinline__ void chunk_factors(uint32_t slot, float2 (&f)[2]) {
+    using C = TForm<D, X3, CR>;
+    f[0] = f[1] = make_float2(1.f, 1.f);
+    if constexpr (X3) {
+        f[0] = f[1] = lds_f2(slot + C::DATA);
+        if constexpr (CR == 8) f[1] = lds_f2(slot + C::DATA + 16);
+    }
+}
+// Two parents in one product over children: their common factor (the larger one) and what each parent's rows are multiplied by.
+__device__ __forceinline__ float common_factor(float a, float b, float (&ratio)[2]) {
+    const float f = fmaxf(a, b), inv = pow2_inverse(f);
+    ratio[0] = a * inv; ratio[1] = b * inv;
+    return f;
+}
+// Scores; split-half ones still have to be multiplied by f[row / 8].x * q.inv, a power of two.
 template <typename T, int D, bool X3, int NH, int CR>
-__device__ __forceinline__ void score_t(const LaneBase<D, X3, CR>& s, uint32_t tab, int r, const QueryRegs<T, D, X3, NH>& q, float (&S)[NH][4]) {
+__device__ __forceinline__ void score_t(const LaneBase<D, X3, CR>& s, uint32_t slot, int r, const QueryRegs<T, D, X3, NH>& q, float (&S)[NH][4]) {
+    const uint32_t tab = slot + TForm<D, X3, CR>::TAB_OFF;
     if constexpr (X3) score_x3<T, D, NH, CR>(s, tab, r, q, S);
     else score16<T, D, NH, CR>(s, tab, r, q, S);
 }

@@ -360,8 +360,9 @@ class _Workspace:
 
     def _block_bytes(self, l):
         B, _, H_kv, K = self.k.shape
-        n = B * ((self.plan.nodes[l] + self.cr - 1) // self.cr) * H_kv * (2 if _split(self.k.dtype, K) else 1) * K * 2 * self.cr
-        return n * (2 if self.cr == 16 or not _split(self.k.dtype, K) else 3), n
+        blocks, split = B * ((self.plan.nodes[l] + self.cr - 1) // self.cr) * H_kv, _split(self.k.dtype, K)
+        n = blocks * (2 if split else 1) * K * 2 * self.cr
+        return n * (2 if self.cr == 16 or not split else 3) + (128 * blocks if split else 0), n
 
 
 class BwdContext(dict):

@@ -154,3 +154,49 @@ def test_malformed_parent_lists(dt, D, CR, G, T, TK, MTN, compact, monkeypatch):
             with pytest.raises(RuntimeError, match="outside its tree level"):
                 ops.check_status()
     ops.check_status()
+
+
+def _compare_with_generic(dt, D, CR, G, scales, tol_out, tol_grad):
+    """Outputs and gradients of inputs times `scales` (q, k, v, dO) against the fp32-arithmetic kernels on the same saved state."""
+    import htree_b200 as ht
+    q, k, v, dO = (x * s for x, s in zip(_inputs(dt, 1, 1500, 2, G, D), scales))
+    out, ctx = ht.htree_forward(q, k, v, CR, 64, 32, _save_for_backward=True)
+    ref, rctx = ht.htree_forward(q, k, v, CR, 64, 32, _save_for_backward=True, _force_generic=True)
+    same = torch.stack([(ctx["per_layer_parents"][l] == rctx["per_layer_parents"][l]).all(-1) for l in range(ctx["num_layers"])]).all(0)
+    rows = same.repeat_interleave(G, -1)
+    assert same.float().mean().item() >= 0.98
+    rel = lambda a, b: ((a.double() - b.double()).norm() / b.double().norm()).item()
+    assert rel(out[rows], ref[rows]) < tol_out
+    for name, a, b in zip(("dq", "dk", "dv"), ht.htree_backward(dO, q, out, ctx), ht.htree_backward(dO, q, out, ctx, _force_generic=True)):
+        assert rel(a, b) < tol_grad, (name, scales)
+
+
+@pytest.mark.parametrize("dt,D,CR,G", [(FP, 128, 16, 8), (FP, 128, 8, 16), (FP, 64, 16, 4), (FP, 64, 8, 12), (FP, 32, 16, 4), (BF, 32, 16, 9),
+                                       (BF, 32, 8, 4), (HF, 32, 8, 16)])
+def test_range_of_split_half(dt, D, CR, G):
+    """Half pairs carry fp32 values over a wider range than half's: a mean-reduced loss (dO of 1e-8), small and large values, small
+    queries against large keys.  The tolerances are those of inputs near 1."""
+    scales = [(1, 1, 1, 1), (1, 1, 3e-3, 3e-3)]
+    if dt != HF:
+        scales += [(1, 1, 1, 1e-8), (1, 1, 1, 1e6), (1, 1, 1e-6, 1), (1, 1, 1e6, 1), (1, 1, 1e4, 1e-6)]
+        if D != 64:      # the selection of 64-wide heads reads the keys as they are
+            scales += [(1e-5, 1e5, 1, 1), (1e5, 1e-5, 1, 1)]
+    for s in scales:
+        _compare_with_generic(dt, D, CR, G, s, 1e-5 if dt == FP else 4e-3, 1e-5)
+
+
+@pytest.mark.parametrize("D,CR,G", [(128, 16, 8), (64, 8, 4), (32, 8, 9)])
+def test_range_within_a_call(D, CR, G):
+    """Groups, heads and blocks of very different magnitude in one call: each group and each block has its own scale, so a small
+    gradient or value is as exact as it would be alone."""
+    import htree_b200 as ht
+    q, k, v, dO = _inputs(FP, 1, 1500, 2, G, D)
+    dO[:, ::2] *= 1e-9                       # every other query: visits of both kinds share a parent
+    v[:, 700:, 1] *= 1e-7
+    q[:, 1::3] *= 1e-3
+    out, ctx = ht.htree_forward(q, k, v, CR, 64, 32, _save_for_backward=True)
+    ours, gen = ht.htree_backward(dO, q, out, ctx), ht.htree_backward(dO, q, out, ctx, _force_generic=True)
+    for part in (slice(0, None, 2), slice(1, None, 2)):
+        assert _rel(ours[0][:, part], gen[0][:, part]) < 1e-5
+    for a, b in zip(ours[1:], gen[1:]):
+        assert _rel(a[:, :, 0], b[:, :, 0]) < 1e-5 and _rel(a[:, :, 1], b[:, :, 1]) < 1e-5

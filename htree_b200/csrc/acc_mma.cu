@@ -19,12 +19,12 @@ constexpr int acc_stages() { return D * (X3 ? 2 : 1) >= 128 ? 2 : 3; }     // sl
 
 // Registers: 168 per thread (12 warps per SM) hold a group of 16 heads of 128; what the kernel needs beyond that is room for
 // the rings, two slots of 8448 bytes per warp at 128-wide heads.
-constexpr int kAccWarps = 4;
+constexpr int kAccWarps = 4, kAccSplitWarps = 8;
 template <int D, bool X3, int NH>
 constexpr int acc_min_blocks() { return (X3 && D == 128) ? 2 : (D == 128 || (X3 && D == 64 && NH == 2)) ? 3 : 4; }
 
 template <typename T, int D, bool X3, int NH, int CR, bool SPLIT>
-__global__ void __launch_bounds__(SPLIT ? 256 : kAccWarps * 32, SPLIT ? 1 : acc_min_blocks<D, X3, NH>())
+__global__ void __launch_bounds__((SPLIT ? kAccSplitWarps : kAccWarps) * 32, SPLIT ? 1 : acc_min_blocks<D, X3, NH>())
 acc_mma_kernel(const __grid_constant__ AttnParams p) {
     using C = TForm<D, X3, CR>;
     using FT = typename std::conditional<X3, __half, T>::type;        // type of the values and probabilities
@@ -35,7 +35,7 @@ acc_mma_kernel(const __grid_constant__ AttnParams p) {
     extern __shared__ __align__(128) unsigned char smem_raw[];
 
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, g = lane >> 2, r = lane & 3;
-    const int W = blockDim.x >> 5;
+    const int W = SPLIT ? kAccSplitWarps : blockDim.x >> 5;
     const int from_end = SPLIT ? (int)blockIdx.x : (int)(blockIdx.x * W + warp);
     if (!SPLIT && from_end >= p.Tq) return;
     const int tl = p.Tq - 1 - from_end;                               // the longest walks first: they would be the tail of a short call
@@ -66,18 +66,18 @@ acc_mma_kernel(const __grid_constant__ AttnParams p) {
         for (int i = 0; i < MT; ++i) O[h][i][0] = O[h][i][1] = O[h][i][2] = O[h][i][3] = 0.f;
     // Online softmax with a lazily moved reference: probabilities are taken relative to m_run, which moves (and the
     // accumulators are rescaled) only when a score exceeds it by more than kLazyMax.  m_run is common to the lanes that share
-    // a head; m_true (the maximum that goes to gmax) and s_run are per lane until the end.  16-bit storage keeps m_run in units of
-    // log 2 and at whole numbers: two references then differ by a power of two, so that P, which is rounded to the storage type
-    // relative to the reference, rounds alike whichever warp forms it and however many share a group's chunks.  With references
-    // at the scores themselves a query's row differed by 3e-3 (bf16) between calls of few and of many queries.
+    // a head; m_true (the maximum that goes to gmax) and s_run are per lane until the end.
+    // With SPLIT a chunk's reference is the one that a single warp walking all chunks would have there: P is rounded to the storage type
+    // relative to it, and with references of their own a query's row differed by 3e-3 (bf16) between calls of few and of many
+    // queries.  The warps take their chunks in rounds; a vote says whether any of the round moves the reference, and only then (the
+    // first round, and as often as scores grow by 8) they exchange their maxima and follow the moves in order.
     constexpr float kLazyMax = 8.f;
     constexpr float kNone = -1.0e30f;
-    float m_run[NH][2], m_true[NH][2], s_run[NH][2];
-    auto factor = [](float from, float to) { return X3 ? __expf(from - to) : ex2_approx(from - to); };      // between two references
+    float m_run[NH][2], m_true[NH][2], s_run[NH][2], m_run2[NH][2];
 #pragma unroll
     for (int h = 0; h < NH; ++h)
 #pragma unroll
-        for (int e = 0; e < 2; ++e) { m_run[h][e] = m_true[h][e] = kNone; s_run[h][e] = 0.f; }
+        for (int e = 0; e < 2; ++e) { m_run[h][e] = m_true[h][e] = kNone; m_run2[h][e] = kNone * kLog2e; s_run[h][e] = 0.f; }
 
     for (int l = L - 1; l >= 0; --l) {
         const int Nl = p.ln[l];
@@ -135,20 +135,14 @@ acc_mma_kernel(const __grid_constant__ AttnParams p) {
                 }
             }
         }
-#pragma unroll 1
-        for (int c = first; c < nchunk; c += step) {
-            __syncwarp();                                             // everybody is done with the slot that is refilled now
-            if (next < nchunk) fill(next);
-            ring.commit();
-            next += step;
+        auto chunk_mask = [&](int c) {                                // the chunk's candidates that accumulate
             uint32_t mask = 0xffffu;
             if (l > 0) mask &= ~(selw[c >> 1] >> ((16 * c) & 31));
             if (16 * c + 15 > rp) mask &= (2u << (rp - 16 * c)) - 1u;
-            const uint32_t slot = ring.wait();
-            if (mask == 0) continue;
-            const LaneBase<D, X3, CR> lb(slot, lane);
-            float S[NH][4];
-            float2 fac[2];
+            return mask;
+        };
+        float2 fac[2];
+        auto scores = [&](uint32_t slot, uint32_t mask, const LaneBase<D, X3, CR>& lb, float (&S)[NH][4]) {
             chunk_factors<D, X3, CR>(slot, fac);
             score_t<T, D, X3, NH, CR>(lb, slot, r, q, S);
             if constexpr (X3) {
@@ -164,6 +158,37 @@ acc_mma_kernel(const __grid_constant__ AttnParams p) {
                     S[h][2] = c1 ? S[h][2] : -INFINITY; S[h][3] = c1 ? S[h][3] : -INFINITY;
                 }
             }
+        };
+        auto head_max = [&](float a, float b) {                       // over the lanes of a head
+            float m = fmaxf(a, b);
+            m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, 4));
+            m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, 8));
+            return fmaxf(m, __shfl_xor_sync(0xffffffffu, m, 16));
+        };
+        auto rescale = [&](int h, int e, float n) {                   // the accumulators of a head to another reference
+            const float f = X3 ? __expf(m_run[h][e] - n) : ex2_approx(m_run2[h][e] - n * kLog2e);
+            m_run[h][e] = n; m_run2[h][e] = n * kLog2e;
+            s_run[h][e] *= f;
+#pragma unroll
+            for (int i = 0; i < MT; ++i) { O[h][i][e] *= f; O[h][i][2 + e] *= f; }
+        };
+#pragma unroll 1
+        for (int c = first; c < (SPLIT ? nchunk + first : nchunk); c += step) {      // SPLIT: rounds of W chunks, some of the last missing
+            __syncwarp();                                             // everybody is done with the slot that is refilled now
+            if (next < nchunk) fill(next);
+            ring.commit();
+            next += step;
+            const uint32_t mask = SPLIT && c >= nchunk ? 0u : chunk_mask(c);
+            const uint32_t slot = ring.wait();
+            if (!SPLIT && mask == 0) continue;
+            const LaneBase<D, X3, CR> lb(slot, lane);
+            float S[NH][4];
+            if (!SPLIT || mask != 0) {
+                scores(slot, mask, lb, S);
+            } else {                                                  // nothing to accumulate, but the round goes on
+#pragma unroll
+                for (int h = 0; h < NH; ++h) S[h][0] = S[h][1] = S[h][2] = S[h][3] = -INFINITY;
+            }
             // exponents relative to the reference; fp32 storage keeps the plain difference (an exponent re-based by log2 e rounds
             // at 1e-6 relative)
             float ex[NH][4];
@@ -171,7 +196,7 @@ acc_mma_kernel(const __grid_constant__ AttnParams p) {
 #pragma unroll
                 for (int h = 0; h < NH; ++h)
 #pragma unroll
-                    for (int i = 0; i < 4; ++i) ex[h][i] = X3 ? S[h][i] - m_run[h][i & 1] : fmaf(S[h][i], kLog2e, -m_run[h][i & 1]);
+                    for (int i = 0; i < 4; ++i) ex[h][i] = X3 ? S[h][i] - m_run[h][i & 1] : fmaf(S[h][i], kLog2e, -m_run2[h][i & 1]);
             };
             exponents();
             float top = ex[0][0];
@@ -182,23 +207,69 @@ acc_mma_kernel(const __grid_constant__ AttnParams p) {
                     top = fmaxf(top, fmaxf(ex[h][e], ex[h][2 + e]));
                     m_true[h][e] = fmaxf(m_true[h][e], fmaxf(S[h][e], S[h][2 + e]));
                 }
-            if (__any_sync(0xffffffffu, top > (X3 ? kLazyMax : kLazyMax * kLog2e))) {
+            constexpr float kMove = X3 ? kLazyMax : kLazyMax * kLog2e;
+            float after[SPLIT ? NH : 1][2];                           // the reference behind the round's last chunk
+            bool moved;
+            if constexpr (SPLIT) {
+                moved = __syncthreads_or(top > kMove);
+                if (moved) {
+                    float* st = reinterpret_cast<float*>(smem_raw + W * per_warp);
 #pragma unroll
-                for (int h = 0; h < NH; ++h)
+                    for (int h = 0; h < NH; ++h)
 #pragma unroll
-                    for (int e = 0; e < 2; ++e) {
-                        float m = fmaxf(S[h][e], S[h][2 + e]);
-                        m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, 4));
-                        m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, 8));
-                        m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, 16));
-                        const float n = fmaxf(m_run[h][e], X3 ? m : ceilf(m * kLog2e));
-                        const float f = factor(m_run[h][e], n);
-                        m_run[h][e] = n;
-                        s_run[h][e] *= f;
+                        for (int e = 0; e < 2; ++e) {
+                            const float m = head_max(S[h][e], S[h][2 + e]);
+                            if (g == 0) st[warp * 48 + 8 * h + 2 * r + e] = m;
+                            after[h][e] = m_run[h][e];
+                        }
+                    __syncthreads();                                  // (the vote of the next round orders these reads before its writes)
+                    float m[kAccSplitWarps][NH][2], mine[NH][2];
 #pragma unroll
-                        for (int i = 0; i < MT; ++i) { O[h][i][e] *= f; O[h][i][2 + e] *= f; }
+                    for (int w = 0; w < kAccSplitWarps; ++w)
+#pragma unroll
+                        for (int h = 0; h < NH; ++h) {
+                            const float2 x = *reinterpret_cast<const float2*>(st + w * 48 + 8 * h + 2 * r);
+                            m[w][h][0] = x.x; m[w][h][1] = x.y;
+                        }
+#pragma unroll
+                    for (int w = 0; w < kAccSplitWarps; ++w) {
+                        float t = -INFINITY;
+#pragma unroll
+                        for (int h = 0; h < NH; ++h)
+#pragma unroll
+                            for (int e = 0; e < 2; ++e)
+                                t = fmaxf(t, X3 ? m[w][h][e] - after[h][e] : fmaf(m[w][h][e], kLog2e, -(after[h][e] * kLog2e)));
+                        const bool move = __any_sync(0xffffffffu, t > kMove);
+#pragma unroll
+                        for (int h = 0; h < NH; ++h)
+#pragma unroll
+                            for (int e = 0; e < 2; ++e) {
+                                if (move) after[h][e] = fmaxf(after[h][e], m[w][h][e]);
+                                if (w == warp) mine[h][e] = after[h][e];
+                            }
                     }
-                exponents();
+                    bool later = false;                               // does a later chunk of the round move it again?
+#pragma unroll
+                    for (int h = 0; h < NH; ++h)
+#pragma unroll
+                        for (int e = 0; e < 2; ++e) {
+                            const float n = mask != 0 ? mine[h][e] : after[h][e];
+                            later |= n != after[h][e];
+                            rescale(h, e, n);
+                        }
+                    moved = __any_sync(0xffffffffu, later);
+                    exponents();
+                }
+                if (mask == 0) continue;
+            } else {
+                moved = __any_sync(0xffffffffu, top > kMove);
+                if (moved) {
+#pragma unroll
+                    for (int h = 0; h < NH; ++h)
+#pragma unroll
+                        for (int e = 0; e < 2; ++e) rescale(h, e, fmaxf(m_run[h][e], head_max(S[h][e], S[h][2 + e])));
+                    exponents();
+                }
             }
             uint32_t pb[NH][2], pl[X3 ? NH : 1][2];
             float ratio[2], vfac = fac[0].y;                          // split-half: what brings the block's values back
@@ -243,6 +314,14 @@ acc_mma_kernel(const __grid_constant__ AttnParams p) {
                     for (int h = 0; h < NH; ++h) mma_acc<FT>(O[h][i], va, pb[h][0], pb[h][1]);
                 }
             }
+            if constexpr (SPLIT) {
+                if (moved) {
+#pragma unroll
+                    for (int h = 0; h < NH; ++h)
+#pragma unroll
+                        for (int e = 0; e < 2; ++e) rescale(h, e, after[h][e]);
+                }
+            }
 #pragma unroll
             for (int h = 0; h < NH; ++h)
 #pragma unroll
@@ -283,7 +362,7 @@ acc_mma_kernel(const __grid_constant__ AttnParams p) {
                 const int head = 8 * h + 2 * r + e;
                 float m = kNone;
                 for (int w = 0; w < W; ++w) m = fmaxf(m, st[w * 48 + head]);
-                const float f = factor(m_run[h][e], m);
+                const float f = __expf(m_run[h][e] - m);
 #pragma unroll
                 for (int i = 0; i < MT; ++i) {
                     po[head * D + C::VB * g + 2 * i] = O[h][i][e] * f;
@@ -296,14 +375,14 @@ acc_mma_kernel(const __grid_constant__ AttnParams p) {
             float m = kNone, s = 0.f, o = 0.f;
             for (int w = 0; w < W; ++w) m = fmaxf(m, st[w * 48 + head]);
             for (int w = 0; w < W; ++w) {
-                s += st[w * 48 + 32 + head] * factor(st[w * 48 + head], m);
+                s += st[w * 48 + 32 + head] * __expf(st[w * 48 + head] - m);
                 o += reinterpret_cast<const float*>(smem_raw + w * per_warp)[i];
             }
             reinterpret_cast<T*>(p.out)[hbase * D + i] = from_f<T>(o / s);
             if (i % D == 0) {
                 float mt = kNone;
                 for (int w = 0; w < W; ++w) mt = fmaxf(mt, st[w * 48 + 16 + head]);
-                p.gmax[hbase + head] = mt; p.gsum[hbase + head] = s * (X3 ? __expf(m - mt) : ex2_approx(fmaf(-mt, kLog2e, m)));
+                p.gmax[hbase + head] = mt; p.gsum[hbase + head] = s * __expf(m - mt);
             }
         }
     } else {
@@ -330,7 +409,7 @@ acc_mma_kernel(const __grid_constant__ AttnParams p) {
                     *reinterpret_cast<uint2*>(orow) = make_uint2(w[0], w[1]);
                 }
             }
-            if (g == 0) { p.gmax[hbase + head] = m_true[h][e]; p.gsum[hbase + head] = s_run[h][e] * (X3 ? __expf(m_run[h][e] - m_true[h][e]) : ex2_approx(fmaf(-m_true[h][e], kLog2e, m_run[h][e]))); }
+            if (g == 0) { p.gmax[hbase + head] = m_true[h][e]; p.gsum[hbase + head] = s_run[h][e] * __expf(m_run[h][e] - m_true[h][e]); }
         }
     }
 }
@@ -346,13 +425,13 @@ static int launch_acc_cr(const AttnParams& p, cudaStream_t st) {
     // backward reads (they keep their selections) always take one warp per group: a query's result then does not depend on
     // how many queries share the call.
     const int64_t groups = (int64_t)p.Tq * p.B * p.Hkv;
-    const size_t split_smem = 8 * per_warp + 8 * 48 * sizeof(float);
+    const size_t split_smem = kAccSplitWarps * (per_warp + 48 * sizeof(float));
     if ((p.flags & kFlagSplitOk) && groups <= 2 * 148 && split_smem <= limit) {
         auto* k = acc_mma_kernel<T, D, X3, NH, CR, true>;
         static SmemLimit shared;
         const cudaError_t e = shared.raise((const void*)k, split_smem);
         if (e != cudaSuccess) return (int)e;
-        k<<<dim3(p.Tq, p.B * p.Hkv), 256, split_smem, st>>>(p);
+        k<<<dim3(p.Tq, p.B * p.Hkv), kAccSplitWarps * 32, split_smem, st>>>(p);
         note_launch();
         return (int)cudaGetLastError();
     }

@@ -60,7 +60,7 @@ extern "C" {
 
 #define HTREE_FWD_INFERENCE 256u /* htree_b200_attend: no backward follows, so calls of few queries may spread a query over
                                     several warps, whose sums are then merged: a row differs between call sizes by the
-                                    order of its fp32 sums, and by the rounding of the result that follows from it */
+                                    order of its fp32 sums and by the roundings of its 16-bit values that follow from it */
 
 /* backward flags: a backward may be run as several calls over consecutive query windows (HtreeShape.T_q / t_offset) that share
  * the dk_levels / dv_levels accumulators, e.g. to overlap transfers of q, dO, out and dq with the kernels.  The first call

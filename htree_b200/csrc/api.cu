@@ -138,7 +138,7 @@ static int bwd_layout(const HtreeShape* s, int L, const int32_t* ln, int64_t bud
     y.o_stp = take(per * subq * MV * sb); y.o_sts = take(per * subq * MV * sb);
     y.o_fac = x3 ? take(per * subq * L * 8) : -1;
     y.o_rank = take(per * subq * MV * 4); y.o_entries = take(per * subq * MV * (int64_t)(x3 ? sizeof(BwdEntry<true>) : sizeof(BwdEntry<false>)));
-    y.o_cnt = take(per * NK * 4); y.o_base = take(per * NK * 8);
+    y.o_cnt = take(per * NK * 4 + 4 + units * 4); y.o_base = take(per * NK * 8);
     y.o_items = take(per * bp.cap * (int64_t)sizeof(BwdItem)); y.o_nitems = take(per * 4);
     y.scratch_bytes = at;
     return 0;
@@ -557,18 +557,16 @@ int htree_b200_run_backward(const HtreeShape* shape, const void* q, void* const*
     bp.qb = sb + y.o_qb; bp.dob = sb + y.o_dob; bp.stp = sb + y.o_stp; bp.sts = sb + y.o_sts;
     bp.fac = y.o_fac < 0 ? nullptr : reinterpret_cast<float2*>(sb + y.o_fac);
     bp.rank = reinterpret_cast<int32_t*>(sb + y.o_rank); bp.entries = sb + y.o_entries;
-    bp.cnt = reinterpret_cast<int32_t*>(sb + y.o_cnt); bp.base = reinterpret_cast<int2*>(sb + y.o_base);
+    bp.cnt = reinterpret_cast<int32_t*>(sb + y.o_cnt); bp.range = reinterpret_cast<uint32_t*>(bp.cnt + (int64_t)y.per_launch * bp.NK); bp.base = reinterpret_cast<int2*>(sb + y.o_base);
     bp.items = reinterpret_cast<BwdItem*>(sb + y.o_items); bp.nitems = reinterpret_cast<int32_t*>(sb + y.o_nitems);
     cudaStream_t st = (cudaStream_t)stream;
-    if (!(flags & HTREE_BWD_KEEP_ACCUM)) {
-        const cudaError_t e = cudaMemsetAsync(acc, 0, (size_t)y.zero_bytes, st);
-        if (e != cudaSuccess) return (int)e;
-    }
     for (int s0 = 0; s0 < y.total; s0 += y.per_launch) {
         bp.sub0 = s0; bp.nsub = y.total - s0 < y.per_launch ? y.total - s0 : y.per_launch;
-        const cudaError_t e = cudaMemsetAsync(bp.cnt, 0, (size_t)bp.nsub * bp.NK * sizeof(int32_t), st);
+        // the counters, and ahead of the first launch (which has the most windows) the words of the range behind them
+        const cudaError_t e = cudaMemsetAsync(bp.cnt, 0, (size_t)bp.nsub * bp.NK * sizeof(int32_t) + (s0 == 0 ? (1 + (size_t)shape->B * shape->H_kv) * sizeof(uint32_t) : 0), st);
         if (e != cudaSuccess) return (int)e;
-        rc = launch_bwd_dq(bp, shape->dtype, st);
+        rc = s0 == 0 ? launch_bwd_begin(bp, shape->dtype, acc, flags & HTREE_BWD_KEEP_ACCUM ? 0 : y.zero_bytes, st) : 0;
+        if (rc == 0) rc = launch_bwd_dq(bp, shape->dtype, st);
         if (rc == 0) rc = launch_bwd_dkv(bp, shape->dtype, st);
         if (rc) return rc;
     }

@@ -4,6 +4,65 @@
 
 namespace htree {
 
+// 16-bit storage: what bounds dS (ds_scale), the largest |dO|_1 of a row and the largest value of every unit, of those that are
+// finite.  Streams dO (the first `of_dO` blocks) and the leaves' values (`of_v` blocks a unit; pooled values are means of them) once, and
+// clears the accumulators on the way (a launch of their own cost 2 of the 121 us of a step of 1000 positions).  18 us at 2 x 16384
+// positions, 16 heads of 64; 27 us at 2 x 7777, 32 heads of 128 (5 TB/s).
+struct RangeArgs {
+    const uint4* dO;
+    const uint4* v;              // blocks [b][parent][KV head] of `piece` 16-byte pieces
+    int64_t n_dO;
+    uint4* zero;                 // the accumulators to clear, or n_zero = 0
+    int64_t n_zero;
+    int32_t of_dO, of_v, NBLK, Hkv, piece;
+    uint32_t* range;
+};
+template <typename T, int D>
+__global__ void __launch_bounds__(256) bwd_range_kernel(const __grid_constant__ RangeArgs a) {
+    constexpr int LPR = D / 8, U = 4;              // lanes per row; 16-byte pieces in flight
+    using F = Frag<T>;
+    __shared__ float part[8];
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    for (int64_t i = (int64_t)blockIdx.x * 256 + threadIdx.x; i < a.n_zero; i += (int64_t)gridDim.x * 256) a.zero[i] = make_uint4(0u, 0u, 0u, 0u);
+    const bool values = (int)blockIdx.x >= a.of_dO;
+    const int at = values ? ((int)blockIdx.x - a.of_dO) % a.of_v : (int)blockIdx.x, unit = values ? ((int)blockIdx.x - a.of_dO) / a.of_v : 0;
+    const int64_t n = values ? (int64_t)a.NBLK * a.piece : a.n_dO, step = (int64_t)(values ? a.of_v : a.of_dO) * 8 * 32 * U;
+    const uint4* src = values ? a.v + ((int64_t)(unit / a.Hkv) * a.NBLK * a.Hkv + unit % a.Hkv) * a.piece : a.dO;
+    float most = 0.f;
+    for (int64_t i0 = ((int64_t)at * 8 + warp) * 32 * U; i0 < n; i0 += step) {
+        uint4 x[U];
+#pragma unroll
+        for (int u = 0; u < U; ++u) {
+            const int64_t i = i0 + 32 * u + lane;
+            const uint32_t row = (uint32_t)i / (uint32_t)a.piece;      // (a unit's values are below 2^32 pieces)
+            x[u] = i < n ? __ldg(src + (values ? i + (int64_t)row * a.piece * (a.Hkv - 1) : i)) : make_uint4(0u, 0u, 0u, 0u);
+        }
+#pragma unroll
+        for (int u = 0; u < U; ++u) {
+            const uint32_t w[4] = {x[u].x, x[u].y, x[u].z, x[u].w};
+            float s = 0.f, m = 0.f;
+#pragma unroll
+            for (int k = 0; k < 4; ++k) {
+                const float2 f = F::unpack(w[k]);
+                s += fabsf(f.x) + fabsf(f.y);
+                if (fabsf(f.x) < INFINITY) m = fmaxf(m, fabsf(f.x));
+                if (fabsf(f.y) < INFINITY) m = fmaxf(m, fabsf(f.y));
+            }
+#pragma unroll
+            for (int o = 1; o < LPR; o <<= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
+            if (values) s = m;
+            if (s < INFINITY) most = fmaxf(most, s);
+        }
+    }
+    most = redux_max_f32(most, 0xffffffffu);
+    if (lane == 0) part[warp] = most;
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        for (int w = 1; w < 8; ++w) most = fmaxf(most, part[w]);
+        atomicMax(a.range + (values ? 1 + unit : 0), __float_as_uint(most));
+    }
+}
+
 // One block per window: exclusive prefix sums over the parents of their visits and of their work items (pieces of at most `seg`
 // visits of one parent).  The items themselves are written by the next kernel: one block that wrote them all took 80 us where
 // parents have thousands of visits (12000 positions, 512 nodes per layer).
@@ -282,11 +341,12 @@ __global__ void __launch_bounds__(128, dkv_min_blocks<D, X3, CR, KEYS>()) bwd_dk
     while (l + 1 < p.L && (bp.voff[l] < 0 || item.key < bp.koff[l] || item.key >= bp.koff[l] + (p.ln[l] + CR - 1) / CR)) ++l;
     const int unit = (bp.sub0 + ls) / bp.nw, b = unit / p.Hkv, hk = unit % p.Hkv;
     const int nblk = (p.ln[l] + CR - 1) / CR;
+    const float post = KEYS && !X3 ? pow2_inverse(ds_scale(__ldg(bp.range), __ldg(bp.range + 1 + unit))) : 1.f;
     float* dst = (KEYS ? bp.acck[l] : bp.accv[l]) + (((int64_t)b * nblk + (item.key - bp.koff[l])) * p.Hkv + hk) * BF::ACC + 4 * lane;
 #pragma unroll
     for (int i = 0; i < KS; ++i)
 #pragma unroll
-        for (int n = 0; n < NT; ++n) red_add_v4(dst + (i * NT + n) * 128, acc[i][n][0], acc[i][n][1], acc[i][n][2], acc[i][n][3]);
+        for (int n = 0; n < NT; ++n) red_add_v4(dst + (i * NT + n) * 128, acc[i][n][0] * post, acc[i][n][1] * post, acc[i][n][2] * post, acc[i][n][3] * post);
 }
 
 // Level by level from the top: accumulators to rows (dK' rotated back by the child index), plus the share of the pooled
@@ -381,6 +441,32 @@ template <typename T>
 static int launch_dkv_d(const BwdParams& bp, cudaStream_t st) {
     constexpr bool F32 = std::is_same<T, float>::value;
     return bp.a.K == 128 ? launch_dkv_t<T, 128, F32>(bp, st) : bp.a.K == 64 ? launch_dkv_t<T, 64, F32>(bp, st) : launch_dkv_t<T, 32, true>(bp, st);
+}
+
+template <typename T>
+static void launch_range_t(const BwdParams& bp, void* zero, int64_t zero_bytes, cudaStream_t st) {
+    const AttnParams& p = bp.a;
+    RangeArgs a;
+    a.dO = static_cast<const uint4*>(p.dO); a.v = static_cast<const uint4*>(p.vkblk[0]);
+    a.n_dO = (int64_t)p.B * p.Tq * p.H * p.K / 8; a.piece = p.CR * p.K / 8;
+    a.NBLK = (p.ln[0] + p.CR - 1) / p.CR; a.Hkv = p.Hkv; a.range = bp.range;
+    a.zero = static_cast<uint4*>(zero); a.n_zero = zero_bytes / 16;
+    // 16 KB a block and more; dO fills the chip and the units share it once more
+    auto blocks = [](int64_t pieces, int most) { const int64_t b = (pieces + 1023) / 1024; return (int)(b < most ? b : most); };
+    const int units = p.B * p.Hkv;
+    a.of_dO = blocks(a.n_dO, 148 * 8); a.of_v = blocks((int64_t)a.NBLK * a.piece, units < 148 ? 148 * 8 / units : 8);
+    const unsigned grid = (unsigned)(a.of_dO + units * a.of_v);
+    if (p.K == 128) bwd_range_kernel<T, 128><<<grid, 256, 0, st>>>(a);
+    else bwd_range_kernel<T, 64><<<grid, 256, 0, st>>>(a);
+}
+// Ahead of the first pass, bp.range being zero: clears `zero_bytes` of accumulators (a multiple of 256, or none) and finds the range of
+// 16-bit operands (split ones have factors per group).
+int launch_bwd_begin(const BwdParams& bp, int dtype, void* zero, int64_t zero_bytes, cudaStream_t st) {
+    if (pack_split(dtype, bp.a.K)) return zero_bytes ? (int)cudaMemsetAsync(zero, 0, (size_t)zero_bytes, st) : 0;
+    if (dtype == HTREE_BF16) launch_range_t<__nv_bfloat16>(bp, zero, zero_bytes, st);
+    else launch_range_t<__half>(bp, zero, zero_bytes, st);
+    note_launch();
+    return (int)cudaGetLastError();
 }
 
 int launch_bwd_dkv(const BwdParams& bp, int dtype, cudaStream_t st) {

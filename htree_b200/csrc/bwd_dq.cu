@@ -65,7 +65,7 @@ __global__ void __launch_bounds__(dq_warps<D, X3, NH>() * 32, dq_min_blocks<D, X
     constexpr float kPScale = 16384.f;                  // split-half: P is carried times 2^14
     float dscale = 1.f, dinv = 1.f;                     // split-half: dO times dscale; dinv = 1 / (dscale kPScale), for P dO and for dS
     float bound_v = 0.f, bound_d = 0.f;                 // |P (dP - D)| as carried <= bound_v * the value block's factor + bound_d
-    float vtop = 0.f, sscale = 1.f;                     // the largest such factor so far, and the scale of dS that follows from it
+    float vtop = 0.f, sscale = 1.f;                     // the largest such factor so far; the scale of dS
     if constexpr (X3) {
         float most = 0.f;
 #pragma unroll
@@ -84,7 +84,7 @@ __global__ void __launch_bounds__(dq_warps<D, X3, NH>() * 32, dq_min_blocks<D, X
     for (int h = 0; h < NH; ++h) {
         const int head = 8 * h + g;
         const bool on = head < G;
-        float sum = 0.f, l1 = 0.f;
+        float sum = 0.f, l1 = 0.f;                      // dO . out and |dO|_1 of this lane's head
 #pragma unroll
         for (int hf = 0; hf < 2; ++hf) {
             const int64_t off = (hbase + head) * D + hf * HALF + PPT * r;
@@ -107,14 +107,17 @@ __global__ void __launch_bounds__(dq_warps<D, X3, NH>() * 32, dq_min_blocks<D, X
                 for (int i = 0; i < KS; ++i) {
                     const float2 x = F::unpack(dO[h][hf][i]), y = F::unpack(o[i]);
                     sum += x.x * y.x + x.y * y.y;
+                    l1 += fabsf(x.x) + fabsf(x.y);
                 }
             }
         }
         sum += __shfl_xor_sync(0xffffffffu, sum, 1);
         sum += __shfl_xor_sync(0xffffffffu, sum, 2);
-        if constexpr (X3) {
-            l1 += __shfl_xor_sync(0xffffffffu, l1, 1);
-            l1 += __shfl_xor_sync(0xffffffffu, l1, 2);
+        l1 += __shfl_xor_sync(0xffffffffu, l1, 1);
+        l1 += __shfl_xor_sync(0xffffffffu, l1, 2);
+        if constexpr (!X3) {
+            bound_v = fmaxf(bound_v, redux_max_f32(l1, 0xffffffffu));
+        } else {
             bound_v = fmaxf(bound_v, kPScale * 16384.f * redux_max_f32(l1, 0xffffffffu));      // values are carried below 2^14
             bound_d = fmaxf(bound_d, kPScale * redux_max_f32(fabsf(sum), 0xffffffffu));
         }
@@ -127,6 +130,16 @@ __global__ void __launch_bounds__(dq_warps<D, X3, NH>() * 32, dq_min_blocks<D, X
             lse[h][e] = X3 ? gm : (hd < G ? gm * kLog2e + __log2f(gs) : INFINITY);
             ginv[h][e] = hd < G ? kPScale / gs : 0.f;
         }
+    }
+
+    float rescale = 1.f;                                // 16-bit: from dS as carried for dq to dS as carried in the records
+    if constexpr (!X3) {
+        const uint32_t v = __ldg(bp.range + 1 + unit);
+        const float call = ds_scale(__ldg(bp.range), v);
+        sscale = fmaxf(ds_scale(__float_as_uint(bound_v), v), call);      // (not smaller: sums of the same row may round differently)
+        rescale = call * pow2_inverse(sscale);
+#pragma unroll
+        for (int h = 0; h < NH; ++h) { Drow[h][0] *= sscale; Drow[h][1] *= sscale; }
     }
 
     // ---- blocked copies of q and dO for the parent-stationary pass: pairs of heads per word, [half][i][lane]{lo, hi} with
@@ -290,7 +303,7 @@ __global__ void __launch_bounds__(dq_warps<D, X3, NH>() * 32, dq_min_blocks<D, X
                     for (int i = 0; i < 4; ++i) {
                         P[i] = X3 ? __expf(fmaf(S[h][i], sfac[i >> 1], -lse[h][i & 1])) * ginv[h][i & 1] : ex2_approx(fmaf(S[h][i], kLog2e, -lse[h][i & 1]));
                         P[i] = (i < 2 ? c0 : c1) ? P[i] : 0.f;
-                        dS[i] = P[i] * (X3 ? fmaf(dP[h][i], fac[i >> 1].y, -Drow[h][i & 1]) : dP[h][i] - Drow[h][i & 1]);
+                        dS[i] = P[i] * fmaf(dP[h][i], X3 ? fac[i >> 1].y : sscale, -Drow[h][i & 1]);
                     }
                     if constexpr (X3) {
                         split_half2(P[0], P[1], pw[h][0], pwl[X3 ? h : 0][0]); split_half2(P[2], P[3], pw[h][1], pwl[X3 ? h : 0][1]);
@@ -301,6 +314,9 @@ __global__ void __launch_bounds__(dq_warps<D, X3, NH>() * 32, dq_min_blocks<D, X
                         sw[h][0] = FS::pack(dS[0], dS[1]); sw[h][1] = FS::pack(dS[2], dS[3]);
                     }
                     db[h][0] = movm(sw[h][0]); db[h][1] = movm(sw[h][1]);
+                    if (!X3 && rescale != 1.f) {
+                        sw[h][0] = FS::pack(dS[0] * rescale, dS[1] * rescale); sw[h][1] = FS::pack(dS[2] * rescale, dS[3] * rescale);
+                    }
                 }
                 // dq^T += K~^T dS^T: transposed key fragments (rows x(ks, g)), rotated back by the chunk's distance
                 if constexpr (!X3) {
@@ -416,7 +432,7 @@ __global__ void __launch_bounds__(dq_warps<D, X3, NH>() * 32, dq_min_blocks<D, X
     constexpr bool PADDED = D == 128 && !X3;
     constexpr int ROW = D + (PADDED ? D / 4 + 4 : 0);
     static_assert(8 * NH * ROW * sizeof(float) <= Ring::kBytes, "the rows fit the ring");
-    const float post = X3 ? p.scale : 1.f;           // 16-bit: the scale is in the tables
+    const float post = X3 ? p.scale : pow2_inverse(sscale);           // 16-bit: the softmax scale is in the tables
 #pragma unroll
     for (int h = 0; h < NH; ++h)
 #pragma unroll

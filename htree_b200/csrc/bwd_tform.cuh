@@ -12,6 +12,11 @@
 // one for dV, which travel in a visit's entry and are applied where its product joins the fp32 sum: gradients of a mean-reduced loss
 // keep their digits, and a visit does not depend on other groups.
 //
+// 16-bit operands go as they are, but dS is formed here and is a half, carried times a power of two from what bounds it: the largest
+// |dO|_1 of a row and the largest value of the (batch, KV head) unit (bwd_range_kernel).  For dq the row is one of the group, so that
+// a query's dq does not depend on the others; in a record for dK it is one of the whole call, since the sums over visits run inside
+// the products.  The two are the same wherever the magnitudes of dO differ by less than 2^4.
+//
 // Work is cut into windows of `subq` queries of one (batch, KV head) unit, small enough for a window's blocked queries to stay
 // in L2 while its parents gather from them, and into launches of `nsub` windows, whose P and dS fit the caller's buffer.
 #pragma once
@@ -20,7 +25,7 @@
 namespace htree {
 
 // A visit in its parent's list: visit slot, group | table row << 15, and, split-half, the factors of dK and dV.
-template <bool X3> struct BwdEntry { uint32_t visit, where; };
+template <bool X3> struct __align__(8) BwdEntry { uint32_t visit, where; };
 template <> struct __align__(16) BwdEntry<true> { uint32_t visit, where; float fk, fv; };
 
 struct BwdItem { int32_t key, start, len, pad; };     // a piece of one parent's visit list
@@ -35,6 +40,7 @@ struct BwdParams {
     unsigned char* dob;                      // blocked output gradients [group][half]
     unsigned char* stp;                      // P  [group * MV + visit][half]
     unsigned char* sts;                      // dS
+    uint32_t* range;                         // 16-bit: bits of the largest |dO|_1 of a row, and of every unit's largest |v|; else unused
     float2* fac;                             // split-half: {dK, dV} factors of the visits of a group and level, [group * L + level]; else NULL
     int32_t* rank;                           // [group * MV + visit]
     int32_t* cnt;                            // [nsub][NK]
@@ -46,6 +52,13 @@ struct BwdParams {
     float* accv[HTREE_MAX_LEVELS];
 };
 
+// The power of two that 16-bit dS is carried with, in steps of 2^4: brings |P (dP - D)| <= 2 max|dO|_1 max|v| below 2^15.
+__device__ __forceinline__ float ds_scale(uint32_t dO_l1, uint32_t v) {
+    const int e = 393 - (int)(dO_l1 >> 23) - (int)(v >> 23);
+    return __int_as_float((((min(max(e, 27), 227) + 1) & ~3) - 1) << 23);
+}
+
+int launch_bwd_begin(const BwdParams& bp, int dtype, void* zero, int64_t zero_bytes, cudaStream_t st);
 int launch_bwd_dq(const BwdParams& bp, int dtype, cudaStream_t st);
 int launch_bwd_dkv(const BwdParams& bp, int dtype, cudaStream_t st);
 int launch_bwd_fold(const BwdParams& bp, int dtype, float* const* gk, float* const* gv, void* dk, void* dv, bool typed, cudaStream_t st);

@@ -201,3 +201,28 @@ def test_range_within_a_call(D, CR, G):
         assert _rel(ours[0][:, part], gen[0][:, part]) < 1e-5
     for a, b in zip(ours[1:], gen[1:]):
         assert _rel(a[:, :, 0], b[:, :, 0]) < 1e-5 and _rel(a[:, :, 1], b[:, :, 1]) < 1e-5
+
+
+@pytest.mark.parametrize("dt,D,CR,G", [(BF, 128, 16, 16), (BF, 128, 8, 5), (BF, 64, 16, 9), (BF, 64, 8, 8), (HF, 128, 16, 8), (HF, 64, 8, 16)])
+def test_range_of_16_bit_gradients(dt, D, CR, G):
+    """dS of the 16-bit kernels is a half: gradients keep their digits whatever the loss is divided by and however large the values."""
+    scales = [(1, 1, 1, 1), (1, 1, 3e-3, 3e-3)]
+    if dt == BF:
+        scales += [(1, 1, 1, 1e-8), (1, 1, 1, 1e6), (1, 1, 1e-6, 1), (1, 1, 1e6, 1), (1, 1, 1e4, 1e-6)]
+    for s in scales:
+        _compare_with_generic(dt, D, CR, G, s, 4e-3, 3e-3)
+
+
+@pytest.mark.parametrize("dt,D,T", [(BF, 128, 1), (BF, 64, 333), (HF, 128, 5000)])
+def test_gradient_range_ignores_what_is_not_finite(dt, D, T):
+    """The bound on dS is taken over finite rows: an infinite output gradient spoils its own head's gradient only."""
+    import htree_b200 as ht
+    q, k, v, dO = _inputs(dt, 1, T, 2, 4, D)
+    out, ctx = ht.htree_forward(q, k, v, 16, 64, 32, _save_for_backward=True)
+    want = ht.htree_backward(dO, q, out, ctx)[0]
+    dO[:, -1, 0, 3] = float("inf")
+    got = ht.htree_backward(dO, q, out, ctx)[0]
+    if T > 1:
+        # the other rows have the same bound, or half of it: dS rounds differently where it is subnormal (2^-25 of the bound)
+        assert _rel(got[:, :-1], want[:, :-1]) < 1e-4
+    assert got[:, -1, 4:].isfinite().all()

@@ -41,12 +41,15 @@ from htree_b200 import configs  # noqa: E402
 
 FALLBACK_PEAKS = {"hbm_gbs": 6650.0, "bf16_tflops": 1590.0, "bf16_tflops_sustained": 1400.0}
 
-# DRAM traffic (dram__bytes_read.sum + dram__bytes_write.sum per launch, one ncu capture) of the attention kernels on
-# the default workload at a quarter of the sequence length (B=4, T=16384).  DRAM traffic grows in proportion to the number
-# of (batch, position, kv head) groups, so the bench scales the figure by the ratio of groups.
-NCU_TRAFFIC_BYTES_QUARTER_CFG3 = {"forward": (1.081223e9 + 0.191851e9) + (1.419880e9 + 1.077576e9),   # selection + accumulation
-                                  "backward": 3.929301e9 + 2.410741e9,
-                                  "capture": "kernels as of commit b82f34d"}
+# DRAM traffic (dram__bytes_read.sum + dram__bytes_write.sum, one ncu capture) of a step's attention kernels with the default
+# workload's heads on one batch element of 16384 positions.  The forward's grows with the number of (batch, position, kv head)
+# groups; the backward's is the records of P and dS that its first pass leaves for its second (1 KB written and read back per group
+# and chunk) and grows with the accumulated chunks.
+NCU_TRAFFIC_BYTES = {"T": 16384, "B": 1,
+                     "forward": (0.2708e9 + 0.0363e9) + (0.3468e9 + 0.2333e9),                  # selection + accumulation
+                     "backward": (0.2852e9 + 0.0466e9) + (1.0510e9 + 7.0009e9) + 0.0628e9       # range, first pass, fill
+                                 + (3.7652e9 + 0.0551e9) + (3.7811e9 + 0.0570e9) + 0.0770e9,    # dK, dV, fold
+                     "capture": "profiles/operand_block_kernels_cfg3_eighth.md"}
 
 TDT = {"float32": torch.float32, "bfloat16": torch.bfloat16, "float16": torch.float16}
 
@@ -65,6 +68,14 @@ def peaks():
     p = dict(FALLBACK_PEAKS)
     p["_source"] = "fallback"
     return p
+
+
+def ncu_traffic(c: dict, cm: dict, direction: str) -> float:
+    """DRAM bytes of one direction of a step, from the captured small case of the same heads."""
+    small = configs.cost_model(dict(c, B=NCU_TRAFFIC_BYTES["B"], T=NCU_TRAFFIC_BYTES["T"]))
+    ratio = (cm["accumulation_chunks"] / small["accumulation_chunks"] if direction == "backward"
+             else c["B"] * c["T"] / (NCU_TRAFFIC_BYTES["B"] * NCU_TRAFFIC_BYTES["T"]))
+    return NCU_TRAFFIC_BYTES[direction] * ratio
 
 
 class ClockSampler:
@@ -675,10 +686,9 @@ def main():
     roofline = {"kernel": f"{dominant} attention kernel(s) (all tree levels, one pass per step per rank)",
                 "bound": "tensor", "achieved": achieved, "peak": peak_tf, "unit": "TFLOP/s",
                 "frac": achieved / peak_tf, "peak_source": f"{pk['_source']} bf16 dense, sustained",
-                "traffic": (NCU_TRAFFIC_BYTES_QUARTER_CFG3[dominant] * (B * T * Hkv) / (4 * 16384 * 4) / world
-                            if args.workload == "cfg3" else None),
-                "traffic_source": (f"ncu capture at T=16384 ({NCU_TRAFFIC_BYTES_QUARTER_CFG3['capture']}) scaled by the number "
-                                   "of groups") if args.workload == "cfg3" else None,
+                "traffic": ncu_traffic(c, cm, dominant) / world if args.workload == "cfg3" else None,
+                "traffic_source": (f"ncu capture at B=1, T=16384 ({NCU_TRAFFIC_BYTES['capture']}) scaled by the "
+                                   + ("accumulated chunks" if dominant == "backward" else "number of groups")) if args.workload == "cfg3" else None,
                 "algorithmic_flops_per_launch": dom_flops,
                 "forward_ms": fwd_ms, "backward_ms": bwd_ms,
                 "forward_tflops": cm["flops_fwd"] / world / (fwd_ms * 1e-3) / 1e12,
@@ -716,7 +726,7 @@ def main():
     # every level is read once (K and V), pooled rows are written, and each level's operand blocks: keys and values in half
     # precision or as hi + lo half pairs, with eight children split-half keys twice, and the values once more for a backward
     pairs = es == 4 or D == 32
-    block_bytes = 2 * D * (2 if pairs else 1) * ((3 if pairs and CR == 8 else 2) + (1 if bwd else 0))
+    block_bytes = 2 * D * (2 if pairs else 1) * ((3 if pairs and CR == 8 else 2) + (1 if bwd else 0)) + (128 // CR if pairs else 0)
     tree_bytes = n_rows * (2 * es * D * (sum(lv_sizes) + sum(lv_sizes[1:])) + block_bytes * sum(lv_sizes))
     streaming = {"kernels": "pack_blocks_kernel (pooling, rotation and operand blocks of all levels, rank 0)", "ms": tree_ms,
                  "algorithmic_bytes": tree_bytes, "achieved": tree_bytes / (tree_ms * 1e-3) / 1e9, "unit": "GB/s",

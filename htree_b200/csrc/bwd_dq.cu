@@ -5,8 +5,8 @@
 //   dP^T = V dO^T,  S^T = K' q^,  P = exp(S - gmax) / gsum,  dS = P (dP - D),  dq^T += K~^T dS^T
 // with K~ = scale R(-distance) K' rotated back into the query's frame in registers, its fragments transposed by the load.
 //
-// Bound by the latency of those five products in a row at 12 warps per SM (issue 46%, shared-memory pipe 65%, tensor pipe 37%).
-// 4 x 65536 positions, 64 heads of 128: this pass 135 ms and the parent-stationary one 90 ms, where the single kernel with reductions
+// Bound by the latency of those five products in a row at 12 warps per SM (issue 49%, shared-memory pipe 67%, tensor pipe 38%).
+// 4 x 65536 positions, 64 heads of 128: this pass 137 ms and the parent-stationary one 90 ms, where the single kernel with reductions
 // took 360 ms.
 #include "bwd_tform.cuh"
 

@@ -202,7 +202,7 @@ select_mma_kernel(const __grid_constant__ AttnParams p) {
 #pragma unroll
                 for (int w = 0; w < PPC; ++w) {
                     const int a = PPC == 1 ? c : min(c * PPC + w, np - 1);     // past the end of the list: masked, any finite block
-                                    ring.template copy<SF::KPART>(w * SF::KPART, blk + (uint64_t)(uint32_t)par[a] * bstride, lane);
+                    ring.template copy<SF::KPART>(w * SF::KPART, blk + (uint64_t)(uint32_t)par[a] * bstride, lane);
                     ring.template copy<SF::TAB>(SF::DATA + w * SF::TAB, reinterpret_cast<const unsigned char*>(p.tab32) + (uint32_t)(rp - CR * a) * SF::TAB, lane);
                 }
             };
@@ -392,7 +392,7 @@ static int launch_select_cr(const AttnParams& in, cudaStream_t st) {
     const size_t scratch = sel_scratch_bytes(maxc, p.TK, CR), limit = 227 * 1024;
     const int64_t groups = (int64_t)p.Tq * p.B * p.Hkv;
     // A block of 8 warps per group where there are few groups (below two per SM a single warp's walk over its chunks is the whole
-    // time of the call), and for long lists: (above kSelLong).
+    // time of the call), and for lists above kSelLong.
     const size_t split_smem = kSelSplitWarps * Ring::kBytes + scratch;
     if ((groups <= 2 * 148 || maxc > kSelLong) && maxc <= kSelSplitKeys && split_smem <= limit) {
         auto* k = select_mma_kernel<T, D, X3, NH, CR, true>;

@@ -556,7 +556,8 @@ def htree_forward(
     with a third element — {"num_layers", "num_groups", "layers": {l: LayerTrace}} — when `return_trace` is set
     (the shape of htree_forward_naive's trace, src/naive.py:225-234).
 
-    `_fused` bounds the temporaries of a call that keeps no selections (windows of queries, see SPLIT_FORWARD_MAX_BYTES);
+    `_fused` bounds the temporaries of a call that keeps no selections (windows of queries, see SPLIT_FORWARD_MAX_BYTES; no effect
+    where they are kept);
     `_no_pipeline` is accepted and has no effect (there is one accumulation kernel); `_tiled` concerns the generic kernels.
 
     Sequence sharding: with `_q_offset` = t0, q holds only the query positions t0 .. t0+q.shape[1]-1 while k, v (or the

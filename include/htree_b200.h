@@ -268,6 +268,7 @@ int htree_b200_topk(const float* values, const int32_t* pay1, const int32_t* pay
  *   typed  NULL (the reference's contract: fp32 dq, dk, dv as above), or the three outputs in the storage type: dq is
  *          then not written (it may be NULL), dk_levels[0] / dv_levels[0] still have to be provided as fp32
  *          accumulators but hold no result on return, and the finished gradients are rounded once into typed->dq/dk/dv.
+ * The tensor-core kernel forms dS as an unscaled half: with output gradients far below 1e-3 use htree_b200_run_backward.
  * A shape that no compiled kernel takes is refused with HTREE_E_UNSUPPORTED before anything is queued on the stream.
  */
 int htree_b200_backward(const HtreeShape* shape, const void* q, void* const* layers_k, void* const* layers_v,

@@ -7,31 +7,46 @@
 // one rotary-table row into its ring in shared memory (asynchronously, NSTG - 1 chunks ahead), forms
 // S^T = K' q^ (one query rotation per chunk), P^T, and O^T += V^T P^T.
 //
-// Bound by the L2 gather of the blocks (14.6 to 16.1 of a measured 20 TB/s) and by the latency of a chunk's chain at 12 to 16 warps
-// per SM: without its copies it would take about 80% of its time.  Measured against the kernel that gathers rows with heads on the matrix
+// Bound by the L2 gather of the blocks (14.6 to 17.1 of a measured 20 TB/s) and the shared-memory read pipe (63% busy with 16 heads a
+// group, 76% with 8): without its copies it would take about 80% of its time.  Measured against the kernel that gathers rows with heads on the matrix
 // rows: 4 x 65536 positions, 64 heads of 128: 95 -> 77 ms; 12000 positions, 16 heads of 32, top_k 512: 5.1 ms, FFMA kernel before.
 #include "tform.cuh"
 
 namespace htree {
 
-template <int D, bool X3>
-constexpr int acc_stages() { return D * (X3 ? 2 : 1) >= 128 ? 2 : 3; }     // slots of 8 KB: warps matter more than depth
-
-// Registers: 168 per thread (12 warps per SM) hold a group of 16 heads of 128; what the kernel needs beyond that is room for
-// the rings, two slots of 8448 bytes per warp at 128-wide heads.
+// Registers and rings: 168 per thread (12 warps per SM) hold a group of 16 heads of 128; those of up to 8 heads fit 16 warps, but
+// two slots of 8448 bytes per warp do not.  There a warp has one slot for keys and one for values: the next keys are fetched as soon as
+// the scores are formed, the next values behind the chunk's products, each with half a chunk (of 16 warps) to arrive.
+// One slot against two (us, whole launch): 8 heads of 128, 65536 positions 14790 -> 14510 and 7777 positions 1356 -> 1307; 8 children
+// 1140 -> 1081; fp32 storage, 128-wide heads 386 -> 357 and with 16 heads a group 1031 -> 866; fp32, 64-wide, 8 children 2696 -> 2534.
+// Where the warps are as many either way it costs 1 to 10% (waits and barriers twice per chunk): 16 heads of 128, 64-wide 16-bit
+// heads, 32-wide heads (634 -> 689), fp32 64-wide heads with 16 children (84.5 -> 88.9).
+template <int D, bool X3, int NH, int CR>
+constexpr bool acc_single() { return (D == 128 && (NH == 1 || X3)) || (X3 && D == 64 && NH == 1 && CR == 8); }
+template <int D, bool X3, int NH, int CR>
+constexpr int acc_stages() { return acc_single<D, X3, NH, CR>() ? 1 : D * (X3 ? 2 : 1) >= 128 ? 2 : 3; }     // slots of 8 KB: warps matter more than depth
 constexpr int kAccWarps = 4, kAccSplitWarps = 8;
-template <int D, bool X3, int NH>
-constexpr int acc_min_blocks() { return (X3 && D == 128) ? 2 : (D == 128 || (X3 && D == 64 && NH == 2)) ? 3 : 4; }
+template <int D, bool X3, int NH, int CR>
+constexpr int acc_min_blocks() { return (X3 && D == 128) ? 2 : D == 128 ? (NH == 1 ? 4 : 3) : (X3 && D == 64 && NH == 2) ? 3 : 4; }
+// A warp's rings: keys with their table rows, and values.
+template <int D, bool X3, int NH, int CR>
+struct AccRings {
+    static constexpr int NSTG = acc_stages<D, X3, NH, CR>();
+    using C = TForm<D, X3, CR>;
+    using Keys = WarpRing<NSTG, C::KSLOT + (NSTG > 1 ? C::VSLOT : 0)>;      // (of several stages: with the values)
+    using Values = WarpRing<1, C::VSLOT>;
+    static constexpr size_t kBytes = Keys::kBytes + (NSTG > 1 ? 0 : Values::kBytes);
+};
 
 template <typename T, int D, bool X3, int NH, int CR, bool SPLIT>
-__global__ void __launch_bounds__((SPLIT ? kAccSplitWarps : kAccWarps) * 32, SPLIT ? 1 : acc_min_blocks<D, X3, NH>())
+__global__ void __launch_bounds__((SPLIT ? kAccSplitWarps : kAccWarps) * 32, SPLIT ? 1 : acc_min_blocks<D, X3, NH, CR>())
 acc_mma_kernel(const __grid_constant__ AttnParams p) {
     using C = TForm<D, X3, CR>;
     using FT = typename std::conditional<X3, __half, T>::type;        // type of the values and probabilities
     using F = Frag<FT>;
     constexpr int MT = C::MT, PPC = C::PPC;
-    using Ring = WarpRing<acc_stages<D, X3>(), C::SLOT>;
-    constexpr int NSTG = acc_stages<D, X3>();
+    using Ring = AccRings<D, X3, NH, CR>;
+    constexpr int NSTG = Ring::NSTG;
     extern __shared__ __align__(128) unsigned char smem_raw[];
 
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, g = lane >> 2, r = lane & 3;
@@ -48,8 +63,10 @@ acc_mma_kernel(const __grid_constant__ AttnParams p) {
     const WalkLayout lay = walk_layout(p, CR);
     const size_t per_warp = walk_warp_bytes<Ring>(lay);
     unsigned char* wbase = smem_raw + warp * per_warp;
-    Ring ring;
-    ring.init(wbase);
+    typename Ring::Keys kring;
+    typename Ring::Values vring;
+    kring.init(wbase);
+    vring.init(wbase + Ring::Keys::kBytes);
     const ParentList par{wbase + Ring::kBytes, lay.narrow};
     uint32_t* selw = reinterpret_cast<uint32_t*>(wbase + Ring::kBytes + lay.list);
 
@@ -94,30 +111,34 @@ acc_mma_kernel(const __grid_constant__ AttnParams p) {
         const uint32_t bstride = (uint32_t)p.Hkv * C::BLOCK;                // (a grid has at most 65535 KV heads)
         const unsigned char* blk = reinterpret_cast<const unsigned char*>(p.blk[l]) + ((int64_t)b * nblk * p.Hkv + hk) * C::BLOCK;
         const unsigned char* tab = reinterpret_cast<const unsigned char*>(p.tab);
-        auto fill = [&](int c) {                                      // chunk c of this level
-            const int p0 = par[c * PPC];
-            if constexpr (CR == 16) {
-                static_assert(!X3 || C::FACS_OFF == C::DATA, "the factors follow the operands");
-                ring.template copy<C::DATA + (X3 ? 16 : 0)>(0, blk + (uint64_t)(uint32_t)p0 * bstride, lane);
-            } else {
-                const int p1 = c * PPC + 1 < np ? par[c * PPC + 1] : p0;  // past the end of the list: masked, any finite block
-                ring.template copy<C::DATA / 2>(0, blk + (uint64_t)(uint32_t)p0 * bstride, lane);
-                ring.template copy<C::DATA / 2>(C::DATA / 2, blk + (uint64_t)(uint32_t)p1 * bstride + C::ODD, lane);
-                if constexpr (X3) {
-                    ring.template copy<16>(C::DATA, blk + (uint64_t)(uint32_t)p0 * bstride + C::FACS_OFF, lane);
-                    ring.template copy<16>(C::DATA + 16, blk + (uint64_t)(uint32_t)p1 * bstride + C::FACS_OFF, lane);
-                }
+        int n0 = 0, n1 = 0;                                           // the parents of the chunk whose keys were fetched last
+        auto fill_keys = [&](int c) {                                 // chunk c of this level
+            n0 = par[c * PPC];
+            kring.template copy<C::PB>(0, blk + (uint64_t)(uint32_t)n0 * bstride, lane);
+            if constexpr (X3) kring.template copy<16>(C::DATA, blk + (uint64_t)(uint32_t)n0 * bstride + C::FACS_OFF, lane);
+            if constexpr (CR == 8) {
+                n1 = c * PPC + 1 < np ? par[c * PPC + 1] : n0;        // past the end of the list: masked, any finite block
+                kring.template copy<C::PB>(C::PB, blk + (uint64_t)(uint32_t)n1 * bstride + 2 * C::ODD, lane);
+                if constexpr (X3) kring.template copy<16>(C::DATA + 16, blk + (uint64_t)(uint32_t)n1 * bstride + C::FACS_OFF, lane);
             }
             const unsigned char* row = tab + (uint32_t)(rp - 16 * c) * C::TAB;
-            ring.template copy<C::TAB>(C::TAB_OFF, row, lane);
-            if constexpr (C::DUAL) ring.template copy<C::TAB>(C::TAB_OFF + C::TAB, rp - 16 * c >= 8 ? row - 8 * C::TAB : row, lane);
+            kring.template copy<C::TAB>(C::TAB_OFF, row, lane);
+            if constexpr (C::DUAL) kring.template copy<C::TAB>(C::TAB_OFF + C::TAB, rp - 16 * c >= 8 ? row - 8 * C::TAB : row, lane);
         };
-        ring.start();
+        auto fill_values = [&]() {                                    // of the same chunk
+            const uint32_t at = NSTG > 1 ? kring.fill + C::KSLOT : vring.fill;
+            kring.template copy_to<C::PB>(at, blk + (uint64_t)(uint32_t)n0 * bstride + C::PB, lane);
+            if constexpr (CR == 8) kring.template copy_to<C::PB>(at + C::PB, blk + (uint64_t)(uint32_t)n1 * bstride + C::PB, lane);
+        };
+        kring.start();
+        vring.start();
         int next = first;
 #pragma unroll 1
-        for (int s = 0; s < NSTG - 1; ++s, next += step) {
-            if (next < nchunk) fill(next);
-            ring.commit();
+        for (int s = 0; s < (NSTG == 1 ? 1 : NSTG - 1); ++s, next += step) {
+            if (next < nchunk) fill_keys(next);
+            if constexpr (NSTG == 1) kring.commit();
+            if (next < nchunk) fill_values();
+            if constexpr (NSTG == 1) vring.commit(); else kring.commit();
         }
         if (l > 0) {
             // positions the next level kept, from its list (both lists ascending); found while the first blocks are on their way
@@ -141,7 +162,7 @@ acc_mma_kernel(const __grid_constant__ AttnParams p) {
             if (16 * c + 15 > rp) mask &= (2u << (rp - 16 * c)) - 1u;
             return mask;
         };
-        float2 fac[2];
+        float2 fac[2] = {make_float2(1.f, 1.f), make_float2(1.f, 1.f)};
         auto scores = [&](uint32_t slot, uint32_t mask, const LaneBase<D, X3, CR>& lb, float (&S)[NH][4]) {
             chunk_factors<D, X3, CR>(slot, fac);
             score_t<T, D, X3, NH, CR>(lb, slot, r, q, S);
@@ -174,20 +195,45 @@ acc_mma_kernel(const __grid_constant__ AttnParams p) {
         };
 #pragma unroll 1
         for (int c = first; c < (SPLIT ? nchunk + first : nchunk); c += step) {      // SPLIT: rounds of W chunks, some of the last missing
-            __syncwarp();                                             // everybody is done with the slot that is refilled now
-            if (next < nchunk) fill(next);
-            ring.commit();
-            next += step;
+            if constexpr (NSTG > 1) {
+                __syncwarp();                                         // everybody is done with the slots that are refilled now
+                if (next < nchunk) { fill_keys(next); fill_values(); }
+                kring.commit();
+                next += step;
+            }
             const uint32_t mask = SPLIT && c >= nchunk ? 0u : chunk_mask(c);
-            const uint32_t slot = ring.wait();
-            if (!SPLIT && mask == 0) continue;
-            const LaneBase<D, X3, CR> lb(slot, lane);
+            const uint32_t keys = kring.template wait<NSTG == 1 ? 1 : NSTG - 1>();
+            const LaneBase<D, X3, CR> lb(keys, keys, lane);
             float S[NH][4];
-            if (!SPLIT || mask != 0) {
-                scores(slot, mask, lb, S);
-            } else {                                                  // nothing to accumulate, but the round goes on
+            if (mask != 0) {
+                scores(keys, mask, lb, S);
+            } else {                                                  // nothing to accumulate
 #pragma unroll
                 for (int h = 0; h < NH; ++h) S[h][0] = S[h][1] = S[h][2] = S[h][3] = -INFINITY;
+            }
+            if constexpr (NSTG == 1) {
+#pragma unroll
+                for (int h = 0; h < NH; ++h) consumed(S[h]);
+                if constexpr (X3) asm volatile("" ::"f"(fac[0].x), "f"(fac[0].y), "f"(fac[1].x), "f"(fac[1].y) : "memory");
+                __syncwarp();                                         // everybody is done with the keys
+                if (next < nchunk) fill_keys(next);
+                kring.commit();
+            }
+            auto wait_values = [&]() {                                // (of a chunk fetched as one they are here already)
+                if constexpr (NSTG == 1) return vring.template wait<1>(); else return keys + C::KSLOT;
+            };
+            auto values_done = [&]() {                                // and with the values: the next chunk's follow
+                if constexpr (NSTG == 1) {
+                    __syncwarp();
+                    if (next < nchunk) fill_values();
+                    vring.commit();
+                    next += step;
+                }
+            };
+            if (!SPLIT && mask == 0) {
+                wait_values();
+                values_done();
+                continue;
             }
             // exponents relative to the reference; fp32 storage keeps the plain difference (an exponent re-based by log2 e rounds
             // at 1e-6 relative)
@@ -260,7 +306,11 @@ acc_mma_kernel(const __grid_constant__ AttnParams p) {
                     moved = __any_sync(0xffffffffu, later);
                     exponents();
                 }
-                if (mask == 0) continue;
+                if (mask == 0) {
+                    wait_values();
+                    values_done();
+                    continue;
+                }
             } else {
                 moved = __any_sync(0xffffffffu, top > kMove);
                 if (moved) {
@@ -291,15 +341,17 @@ acc_mma_kernel(const __grid_constant__ AttnParams p) {
                     pb[h][0] = movm(F::pack(P[0], P[1])); pb[h][1] = movm(F::pack(P[2], P[3]));
                 }
             }
+            const uint32_t values = wait_values();
+            const LaneBase<D, X3, CR> lv(values, values, lane);
 #pragma unroll
             for (int i = 0; i < MT; ++i) {
                 uint32_t va[4];
-                value_frag<D, X3, CR>(lb, 0, i, va);
+                value_frag<D, X3, CR>(lv, 0, i, va);
                 if constexpr (X3) {
                     // summed from zero and then added with a round-to-nearest fp32 add: the tensor core's own accumulation
                     // truncates, and over the ~10^3 chunks of a query that bias would reach 1e-4 relative
                     uint32_t vl[4];
-                    value_frag<D, X3, CR>(lb, 1, i, vl);
+                    value_frag<D, X3, CR>(lv, 1, i, vl);
 #pragma unroll
                     for (int h = 0; h < NH; ++h) {
                         float acc[4];
@@ -326,6 +378,7 @@ acc_mma_kernel(const __grid_constant__ AttnParams p) {
             for (int h = 0; h < NH; ++h)
 #pragma unroll
                 for (int i = 0; i < MT; ++i) consumed(O[h][i]);
+            values_done();
         }
     }
 
@@ -341,7 +394,7 @@ acc_mma_kernel(const __grid_constant__ AttnParams p) {
             }
     if constexpr (SPLIT) {
         // merge the warps' partial states (few queries: a group's chunks are spread over the warps of a block)
-        ring.idle();
+        kring.idle();
         __syncthreads();                                              // all rings are idle: their memory is free
         float* st = reinterpret_cast<float*>(smem_raw + W * per_warp);          // [W][3][16]: m_run, m_true, s
         float* po = reinterpret_cast<float*>(wbase);                  // this warp's O, [16 heads][D]
@@ -417,7 +470,7 @@ acc_mma_kernel(const __grid_constant__ AttnParams p) {
 template <typename T, int D, bool X3, int NH, int CR>
 static int launch_acc_cr(const AttnParams& p, cudaStream_t st) {
     using C = TForm<D, X3, CR>;
-    using Ring = WarpRing<acc_stages<D, X3>(), C::SLOT>;
+    using Ring = AccRings<D, X3, NH, CR>;
     const size_t per_warp = walk_warp_bytes<Ring>(walk_layout(p, CR));
     const size_t limit = 227 * 1024;
     // Few groups: one block of 8 warps per group.  Below two groups per SM the chip has room for all their warps at once, and
@@ -436,7 +489,7 @@ static int launch_acc_cr(const AttnParams& p, cudaStream_t st) {
         return (int)cudaGetLastError();
     }
     // warps per block: as many resident warps as registers allow, fewer where long parent lists leave no room for the rings
-    const int max_warps = kAccWarps * acc_min_blocks<D, X3, NH>();
+    const int max_warps = kAccWarps * acc_min_blocks<D, X3, NH, CR>();
     int W = 1, best = 0;
     for (int w = kAccWarps; w >= 1; --w) {
         if (w == 3) continue;

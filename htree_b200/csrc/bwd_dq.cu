@@ -33,7 +33,7 @@ __global__ void __launch_bounds__(dq_warps<D, X3, NH>() * 32, dq_min_blocks<D, X
     using FS = Frag<__half>;
     constexpr int KS = C::KS, PPT = C::PPT, PPC = C::PPC, HALF = C::HALF;
     constexpr int NSTG = dq_stages<D, X3>();
-    using Ring = WarpRing<NSTG, C::SLOT>;
+    using Ring = WarpRing<NSTG, C::KSLOT + C::VSLOT>;
     extern __shared__ __align__(128) unsigned char smem_raw[];
     const AttnParams& p = bp.a;
 
@@ -191,15 +191,15 @@ __global__ void __launch_bounds__(dq_warps<D, X3, NH>() * 32, dq_min_blocks<D, X
         const unsigned char* kblk = reinterpret_cast<const unsigned char*>(p.blk[l]) + blk0 * C::BLOCK;
         const unsigned char* vblk = reinterpret_cast<const unsigned char*>(p.vkblk[l]) + blk0 * (C::PL * C::PART);
         auto fill = [&](int c) {
-            constexpr int PB = C::PL * C::PART;
+            constexpr int PB = C::PB;
             const uint32_t kstride = (uint32_t)p.Hkv * C::BLOCK, vstride = (uint32_t)p.Hkv * PB;
             const int p0 = par[c * PPC];
             ring.template copy<PB>(0, kblk + (uint64_t)(uint32_t)p0 * kstride, lane);
-            ring.template copy<PB>(C::V_OFF, vblk + (uint64_t)(uint32_t)p0 * vstride, lane);
+            ring.template copy<PB>(C::KSLOT, vblk + (uint64_t)(uint32_t)p0 * vstride, lane);
             if constexpr (CR == 8) {
                 const int p1 = c * PPC + 1 < np ? par[c * PPC + 1] : p0;
-                ring.template copy<PB>(C::K2_OFF, kblk + (uint64_t)(uint32_t)p1 * kstride + 2 * C::ODD, lane);
-                ring.template copy<PB>(C::V2_OFF, vblk + (uint64_t)(uint32_t)p1 * vstride, lane);
+                ring.template copy<PB>(C::PB, kblk + (uint64_t)(uint32_t)p1 * kstride + 2 * C::ODD, lane);
+                ring.template copy<PB>(C::KSLOT + C::PB, vblk + (uint64_t)(uint32_t)p1 * vstride, lane);
                 if constexpr (X3) ring.template copy<16>(C::DATA + 16, kblk + (uint64_t)(uint32_t)p1 * kstride + C::FACS_OFF, lane);
             }
             if constexpr (X3) ring.template copy<16>(C::DATA, kblk + (uint64_t)(uint32_t)p0 * kstride + C::FACS_OFF, lane);
@@ -259,7 +259,7 @@ __global__ void __launch_bounds__(dq_warps<D, X3, NH>() * 32, dq_min_blocks<D, X
             if (l > 0) mask &= ~(selw[c >> 1] >> ((16 * c) & 31));
             if (16 * c + 15 > rp) mask &= (2u << (rp - 16 * c)) - 1u;
             const uint32_t slot = ring.wait();
-            const LaneBase<D, X3, CR> lb(slot, lane);
+            const LaneBase<D, X3, CR> lb(slot, slot + C::KSLOT, lane);
             const uint32_t tabs = slot + C::TAB_OFF;
 
             uint32_t pw[NH][2], sw[NH][2], pwl[X3 ? NH : 1][2], swl[X3 ? NH : 1][2];   // P^T, dS^T: word w = child g + 8w, heads 2r, 2r+1
@@ -459,7 +459,7 @@ __global__ void __launch_bounds__(dq_warps<D, X3, NH>() * 32, dq_min_blocks<D, X
 template <typename T, int D, bool X3, int NH, int CR>
 static int launch_dq_cr(const BwdParams& bp, cudaStream_t st) {
     using C = TForm<D, X3, CR>;
-    using Ring = WarpRing<dq_stages<D, X3>(), C::SLOT>;
+    using Ring = WarpRing<dq_stages<D, X3>(), C::KSLOT + C::VSLOT>;
     const size_t per_warp = walk_warp_bytes<Ring>(walk_layout(bp.a, CR));
     constexpr int max_w = dq_warps<D, X3, NH>(), max_warps = max_w * dq_min_blocks<D, X3, NH>();
     int W = 1, best = 0;

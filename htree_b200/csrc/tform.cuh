@@ -44,30 +44,29 @@ struct TForm {
     static constexpr bool KSCALED = X3 && D != 64;                         // are a block's keys multiplied by their factor?
     static constexpr int ODD = DUAL ? 0 : PL * PART;                       // where an odd parent's copy starts in its block
     static constexpr int NTAB = DUAL ? 2 : 1;
-    static constexpr int DATA = PL * D * 64;                               // bytes of a chunk in shared memory
-    static constexpr int TAB = X3 ? D * 4 : D * 2;                         // one row of the rotary table: [cos | sin]
     static constexpr int PPC = 16 / CR;                                    // parents per chunk
-    // a slot: operands, {key factor, value factor, -, -} per parent, table rows, all at whole lines like their sources
+    static constexpr int PB = PL * PART;                                   // bytes of one part of a block
+    static constexpr int DATA = PB * PPC;                                  // bytes of the keys, or of the values, of a chunk in shared memory
+    static constexpr int TAB = X3 ? D * 4 : D * 2;                         // one row of the rotary table: [cos | sin]
+    // a slot of keys: the parents' keys, {key factor, value factor, -, -} per parent, table rows, all at whole lines like their
+    // sources; a slot of values: the parents' values
     static constexpr int TAB_OFF = DATA + (X3 ? 128 : 0);
-    static constexpr int SLOT = TAB_OFF + NTAB * TAB;
-    // part offsets in a slot: 16 children [K | V]; 8 children [K even | V even | K odd | V odd], split-half [.. | V odd | K odd]
-    static constexpr int V_OFF = PL * PART;
-    static constexpr int V2_OFF = (DUAL ? 3 : 2) * PL * PART, K2_OFF = (DUAL ? 2 : 3) * PL * PART;
+    static constexpr int KSLOT = TAB_OFF + NTAB * TAB, VSLOT = DATA;
 };
 
 // Shared-memory addresses of a chunk slot that differ by lane, as 32-bit shared addresses.
 template <int D, bool X3, int CR>
 struct LaneBase {
     uint32_t k, v, vk;   // ldmatrix rows of the key part; value part (16 children: 16-byte pieces, 8: ldmatrix rows); values in key order
-    __device__ __forceinline__ LaneBase(uint32_t slot, int lane) {
+    __device__ __forceinline__ LaneBase(uint32_t keys, uint32_t values, int lane) {
         using C = TForm<D, X3, CR>;
         if constexpr (CR == 16) {
-            k = slot + 16 * lane; v = k + C::V_OFF; vk = v;
+            k = keys + 16 * lane; v = vk = values + 16 * lane;
         } else {
             const int j = lane >> 3, row = lane & 7;
-            k = slot + ((j & 1) ? C::K2_OFF : 0) + (j >> 1) * 128 + row * 16;
-            v = slot + ((j >> 1) ? C::V2_OFF : C::V_OFF) + (j & 1) * 128 + row * 16;
-            vk = slot + ((j & 1) ? C::V2_OFF : C::V_OFF) + (j >> 1) * 128 + row * 16;
+            k = keys + ((j & 1) ? C::PB : 0) + (j >> 1) * 128 + row * 16;
+            v = values + ((j >> 1) ? C::PB : 0) + (j & 1) * 128 + row * 16;
+            vk = values + ((j & 1) ? C::PB : 0) + (j >> 1) * 128 + row * 16;
         }
     }
 };
@@ -360,12 +359,14 @@ struct WarpRing {
     __device__ __forceinline__ void init(unsigned char* b) { base = smem_u32(b); start(); }
     __device__ __forceinline__ void start() { fill = use = base; }       // before the first fill of a walk; nothing is in flight
     __device__ __forceinline__ uint32_t after(uint32_t a) const {
-        return NSTG == 2 ? 2 * base + SLOT - a : a == base + (NSTG - 1) * SLOT ? base : a + SLOT;
+        return NSTG == 1 ? a : NSTG == 2 ? 2 * base + SLOT - a : a == base + (NSTG - 1) * SLOT ? base : a + SLOT;
     }
     // BYTES (a multiple of 16) from `src` to offset OFF of the stage being filled
     template <int BYTES>
-    __device__ __forceinline__ void copy(uint32_t off, const void* src, int lane) const {
-        const uint32_t dst = fill + off + 16 * lane;
+    __device__ __forceinline__ void copy(uint32_t off, const void* src, int lane) const { copy_to<BYTES>(fill + off, src, lane); }
+    template <int BYTES>
+    static __device__ __forceinline__ void copy_to(uint32_t at, const void* src, int lane) {
+        const uint32_t dst = at + 16 * lane;
         const unsigned char* s = static_cast<const unsigned char*>(src) + 16 * lane;
 #pragma unroll
         for (int i = 0; i < BYTES / 512; ++i)
@@ -380,9 +381,10 @@ struct WarpRing {
         asm volatile("cp.async.commit_group;\n" ::: "memory");
         fill = after(fill);
     }
-    // the oldest fill, complete and visible to every lane
+    // the oldest fill, complete and visible to every lane: YOUNGER fills (of any ring of the warp) were closed after it
+    template <int YOUNGER = NSTG - 1>
     __device__ __forceinline__ uint32_t wait() {
-        asm volatile("cp.async.wait_group %0;\n" ::"n"(NSTG - 1) : "memory");
+        asm volatile("cp.async.wait_group %0;\n" ::"n"(YOUNGER) : "memory");
         __syncwarp();
         uint32_t slot = use;
         asm volatile("" : "+r"(slot)::"memory");

@@ -6,8 +6,9 @@
 // importance does not depend on which: every chunk is evaluated alike (the query rotated in fp32 and rounded once to half per
 // parent, two accumulation chains, the chunk's own maximum as reference, heads summed in one fixed tree) and the search is exact.
 //
-// Bound by instruction issue and latency at 12 to 16 warps per SM; of its time the copies are a third, the Top-K search and the
-// rotation a tenth each.  Measured against the kernel that gathers rows: 4 x 65536 positions, 64 heads of 128: 49 -> 43.7 ms.
+// Bound by the shared-memory read pipe (76% busy at 8 heads of 128) and latency at 12 to 16 warps per SM; of its time the copies are a
+// third, the Top-K search and the rotation a tenth each.  Measured against the kernel that gathers rows: 4 x 65536 positions, 64 heads
+// of 128: 49 -> 43.7 ms.
 #include "tform.cuh"
 
 namespace htree {
@@ -16,9 +17,11 @@ template <int D, bool X3, int CR>
 struct SelForm {
     using C = TForm<D, X3, CR>;
     static constexpr int PPC = C::PPC, KPART = C::PL * C::PART;     // keys of one parent (the version without the odd slot's rotation)
-    static constexpr int DATA = PPC * KPART, TAB = D * 6, SLOT = DATA + PPC * TAB;
+    static constexpr int DATA = PPC * KPART, TAB_ROW = D * 6, TAB = D * 4, SLOT = DATA + PPC * TAB;
     // a table row is [cos | sin | -sin] in fp32, each part ordered [k-step pair][r][4]: the four lanes of a quad read 64 consecutive
-    // bytes (rows in natural order cost 8 wavefronts a load, a third of the kernel's shared-memory traffic)
+    // bytes (rows in natural order cost 8 wavefronts a load, a third of the kernel's shared-memory traffic).  A 16-byte load takes 4
+    // wavefronts however many lanes share its words, so the third part is not fetched but formed, one packed multiply for two values:
+    // 16 of 88 wavefronts a chunk and an eighth of the bytes.  8 heads of 128, 65536 positions: 8.08 -> 7.08 ms; 16 heads 1.43 -> 1.38.
     static constexpr int NSTG = SLOT > 4096 ? 2 : 3;
 };
 // Queries up to here take the longest walks first, so that these are not the tail of the call; in longer ones nearly all walks
@@ -62,15 +65,13 @@ __device__ __forceinline__ void select_scores(uint32_t slot, int lane, const flo
     float U[PPC][NH][4], V[PPC][NH][4], B[PPC][NH][4];     // 16-bit: chains of even and odd k-steps (U, V); split-half: hi*hi (U), hi*lo (V), lo*hi (B)
 #pragma unroll
     for (int kp = 0; kp < KS / 2; ++kp) {
-        float cs[PPC][4], sn[PPC][4], ng[PPC][4];
+        float cs[PPC][4], sn[PPC][4];
 #pragma unroll
         for (int w = 0; w < PPC; ++w) {
             const uint4 c4 = lds_u4(tab + w * SF::TAB + 64 * kp), s4 = lds_u4(tab + w * SF::TAB + 4 * HALF + 64 * kp);
-            const uint4 n4 = lds_u4(tab + w * SF::TAB + 8 * HALF + 64 * kp);
             const float tsc = X3 ? scale : 1.f;            // split-half: the scale goes into the table values
             cs[w][0] = __uint_as_float(c4.x) * tsc; cs[w][1] = __uint_as_float(c4.y) * tsc; cs[w][2] = __uint_as_float(c4.z) * tsc; cs[w][3] = __uint_as_float(c4.w) * tsc;
             sn[w][0] = __uint_as_float(s4.x) * tsc; sn[w][1] = __uint_as_float(s4.y) * tsc; sn[w][2] = __uint_as_float(s4.z) * tsc; sn[w][3] = __uint_as_float(s4.w) * tsc;
-            ng[w][0] = __uint_as_float(n4.x) * tsc; ng[w][1] = __uint_as_float(n4.y) * tsc; ng[w][2] = __uint_as_float(n4.z) * tsc; ng[w][3] = __uint_as_float(n4.w) * tsc;
         }
 #pragma unroll
         for (int u = 0; u < 2; ++u) {
@@ -81,7 +82,7 @@ __device__ __forceinline__ void select_scores(uint32_t slot, int lane, const flo
 #pragma unroll
             for (int w = 0; w < PPC; ++w) {
                 const float2 c2 = make_float2(cs[w][2 * u], cs[w][2 * u + 1]), s2 = make_float2(sn[w][2 * u], sn[w][2 * u + 1]);
-                const float2 n2 = make_float2(ng[w][2 * u], ng[w][2 * u + 1]);
+                const float2 n2 = fmul2(s2, make_float2(-1.f, -1.f));
 #pragma unroll
                 for (int h = 0; h < NH; ++h) {
                     float2 x, y;
@@ -203,7 +204,7 @@ select_mma_kernel(const __grid_constant__ AttnParams p) {
                 for (int w = 0; w < PPC; ++w) {
                     const int a = PPC == 1 ? c : min(c * PPC + w, np - 1);     // past the end of the list: masked, any finite block
                     ring.template copy<SF::KPART>(w * SF::KPART, blk + (uint64_t)(uint32_t)par[a] * bstride, lane);
-                    ring.template copy<SF::TAB>(SF::DATA + w * SF::TAB, reinterpret_cast<const unsigned char*>(p.tab32) + (uint32_t)(rp - CR * a) * SF::TAB, lane);
+                    ring.template copy<SF::TAB>(SF::DATA + w * SF::TAB, reinterpret_cast<const unsigned char*>(p.tab32) + (uint32_t)(rp - CR * a) * SF::TAB_ROW, lane);
                 }
             };
             ring.start();
@@ -275,12 +276,22 @@ select_mma_kernel(const __grid_constant__ AttnParams p) {
             };
             const bool in_regs = SPLIT || maxc <= 1024;
             uint32_t kreg[32];
-            if (in_regs) {
+            // over the thread's keys, whole eights of them that hold none left out: levels of few candidates spent more on the search
+            // among 1024 than on their scores (fp16, 7777 positions, top_k 32: 567 -> 517 us)
+            auto each = [&](auto f) {
 #pragma unroll
-                for (int i = 0; i < 32; ++i) {
+                for (int i0 = 0; i0 < 32; i0 += 8) {
+                    if (nthr * i0 < nc) {
+#pragma unroll
+                        for (int i = i0; i < i0 + 8; ++i) f(i);
+                    }
+                }
+            };
+            if (in_regs) {
+                each([&](int i) {
                     const int j = tid + nthr * i;
                     kreg[i] = j < nc ? value(j) : 0u;          // padding is below every probe
-                }
+                });
             } else {
                 for (int j = tid; j < nc; j += nthr) key[j] = value(j);
                 sync();
@@ -289,8 +300,7 @@ select_mma_kernel(const __grid_constant__ AttnParams p) {
             auto count = [&](uint32_t x) {
                 int c = 0;
                 if (in_regs) {
-#pragma unroll
-                    for (int i = 0; i < 32; ++i) c += kreg[i] >= x;
+                    each([&](int i) { c += kreg[i] >= x; });
                 } else {
                     for (int j = tid; j < nc; j += nthr) c += key[j] >= x;
                 }
@@ -307,11 +317,10 @@ select_mma_kernel(const __grid_constant__ AttnParams p) {
             // lo: more than TK keys reach it; hi: fewer do (the forced candidate, the largest by far, is left out of the bracket)
             uint32_t lo = 0xffffffffu, hi = 0u;
             if (in_regs) {
-#pragma unroll
-                for (int i = 0; i < 32; ++i) {
+                each([&](int i) {
                     const int j = tid + nthr * i;
                     if (j < nc && j != rp) { lo = min(lo, kreg[i]); hi = max(hi, kreg[i]); }
-                }
+                });
             } else {
                 for (int j = tid; j < nc; j += nthr) if (j != rp) { lo = min(lo, key[j]); hi = max(hi, key[j]); }
             }
@@ -369,8 +378,7 @@ select_mma_kernel(const __grid_constant__ AttnParams p) {
                 base_eq += tot_eq; base_out += tot_k;
             };
             if (in_regs) {
-#pragma unroll
-                for (int i = 0; i < 32; ++i) if (nthr * i < nc) place(tid + nthr * i, kreg[i]);
+                each([&](int i) { if (nthr * i < nc) place(tid + nthr * i, kreg[i]); });
             } else {
                 for (int j0 = 0; j0 < nc; j0 += nthr) { const int j = j0 + tid; place(j, j < nc ? key[j] : 0u); }
             }

@@ -3,7 +3,8 @@
 // htree_bwd_preprocess_delta_kernel, htree_bwd_build_parent_mask_kernel and htree_bwd_dq_bottom/upper_kernel
 // (src/backward.py:45-436); arithmetic of src/naive.py:333-384 with the forward's scores, bit for bit.  Per chunk:
 //   dP^T = V dO^T,  S^T = K' q^,  P = exp(S - gmax) / gsum,  dS = P (dP - D),  dq^T += K~^T dS^T
-// with K~ = scale R(-distance) K' rotated back into the query's frame in registers, its fragments transposed by the load.
+// with K~ = scale R(-distance) K', its fragments transposed by the load: rotated back into the query's frame in registers, or, split-half,
+// dq^T += R(-distance) (K'^T dS^T), which leaves the keys' planes as they are.
 //
 // Bound by the latency of those five products in a row at 12 warps per SM (issue 49%, shared-memory pipe 67%, tensor pipe 38%).
 // 4 x 65536 positions, 64 heads of 128: this pass 137 ms and the parent-stationary one 90 ms, where the single kernel with reductions
@@ -351,41 +352,48 @@ __global__ void __launch_bounds__(dq_warps<D, X3, NH>() * 32, dq_min_blocks<D, X
                         }
                     }
                 } else {
+                    // Split-half: the keys' planes go into the product as they are, and the chunk's sums are rotated back in fp32 as they
+                    // join dq: 8 multiply-adds a tile and half, where rotating the keys put both planes together and split them again.
+                    // 2 x 16384 positions, 8 heads of 64: 4.55 -> 3.84 ms; 4096 positions, 8 heads of 128: 652 -> 575 us; 32-wide heads
+                    // 1080 -> 914 us; groups of 16 heads within 2% either way.  The same distance from an fp32 evaluation as before.
                     float ratio[2] = {1.f, 1.f}, kfac = fac[0].x;
-                    if constexpr (CR == 8 && C::KSCALED) kfac = common_factor(fac[0].x, fac[1].x, ratio);
+                    if constexpr (CR == 8 && C::KSCALED) {
+                        kfac = common_factor(fac[0].x, fac[1].x, ratio);
+                        if (ratio[0] != ratio[1]) {
+#pragma unroll
+                            for (int h = 0; h < NH; ++h)
+#pragma unroll
+                                for (int w = 0; w < 2; ++w) {
+                                    const __half2 f = __float2half2_rn(ratio[w]);       // (a power of two, at most 1)
+                                    db[h][w] = as_u32(__hmul2(as_h2(db[h][w]), f));
+                                    dbl[X3 ? h : 0][w] = as_u32(__hmul2(as_h2(dbl[X3 ? h : 0][w]), f));
+                                }
+                        }
+                    }
                     kfac *= back;
 #pragma unroll
                     for (int ks = 0; ks < KS; ++ks) {
-                        uint32_t mh[4], ml[4], ah[4], al[4];
+                        uint32_t mh[4], ml[4];
                         key_frag_trans<D, X3, CR>(lb, 0, ks, mh);
                         key_frag_trans<D, X3, CR>(lb, 1, ks, ml);
                         float cs, sn;
                         const uint32_t tb = tabs + 4 * (PPT * (g >> 1) + 2 * ks + (g & 1));
                         asm("ld.shared.f32 %0, [%1];" : "=f"(cs) : "r"(tb));
                         asm("ld.shared.f32 %0, [%1];" : "=f"(sn) : "r"(tb + 4 * HALF));
-                        float2 x[4];
-#pragma unroll
-                        for (int m = 0; m < 4; ++m) {
-                            const float2 hi = FS::unpack(mh[m]), lo = FS::unpack(ml[m]);
-                            x[m] = make_float2(hi.x + lo.x, hi.y + lo.y);
-                        }
-#pragma unroll
-                        for (int tile = 0; tile < 2; ++tile) {
-                            const float ct = CR == 8 && C::KSCALED ? cs * ratio[tile] : cs, st = CR == 8 && C::KSCALED ? sn * ratio[tile] : sn;
-                            const float2 c2 = make_float2(ct, ct), s2 = make_float2(st, st), n2 = make_float2(-st, -st);
-                            const float2 u = ffma2(x[2 + tile], s2, fmul2(x[tile], c2)), w = ffma2(x[tile], n2, fmul2(x[2 + tile], c2));
-                            split_half2(u.x, u.y, ah[2 * tile], al[2 * tile]);
-                            split_half2(w.x, w.y, ah[2 * tile + 1], al[2 * tile + 1]);
-                        }
+                        cs *= kfac; sn *= kfac;
+                        const uint32_t ah[4] = {mh[0], mh[2], mh[1], mh[3]}, al[4] = {ml[0], ml[2], ml[1], ml[3]};
 #pragma unroll
                         for (int h = 0; h < NH; ++h) {
-                            // from zero, then a round-to-nearest fp32 multiply-add (the tensor core's accumulation truncates)
+                            // from zero, then round-to-nearest fp32 multiply-adds (the tensor core's accumulation truncates)
                             float acc[4];
                             mma_zero<__half>(acc, ah, dbl[X3 ? h : 0][0], dbl[X3 ? h : 0][1]);
                             mma_acc<__half>(acc, al, db[h][0], db[h][1]);
                             mma_acc<__half>(acc, ah, db[h][0], db[h][1]);
 #pragma unroll
-                            for (int i = 0; i < 4; ++i) dq[h][ks][i] = fmaf(acc[i], kfac, dq[h][ks][i]);
+                            for (int e = 0; e < 2; ++e) {
+                                dq[h][ks][e] = fmaf(acc[2 + e], sn, fmaf(acc[e], cs, dq[h][ks][e]));
+                                dq[h][ks][2 + e] = fmaf(acc[e], -sn, fmaf(acc[2 + e], cs, dq[h][ks][2 + e]));
+                            }
                         }
                     }
                 }

@@ -9,7 +9,8 @@
 //
 // Bound by the L2 gather of the blocks (14.6 to 17.1 of a measured 20 TB/s) and the shared-memory read pipe (63% busy with 16 heads a
 // group, 76% with 8): without its copies it would take about 80% of its time.  Measured against the kernel that gathers rows with heads on the matrix
-// rows: 4 x 65536 positions, 64 heads of 128: 95 -> 77 ms; 12000 positions, 16 heads of 32, top_k 512: 5.1 ms, FFMA kernel before.
+// rows: 4 x 65536 positions, 64 heads of 128: 95 -> 77 ms.  Groups of at most 4 heads leave half of the 8 columns empty: where queries
+// select many of the same parents two or four of them share a warp (tform.cuh): 12000 positions, 16 heads of 32, top_k 512: 5.06 -> 3.32 ms.
 #include "tform.cuh"
 
 namespace htree {
@@ -29,52 +30,61 @@ constexpr int kAccWarps = 4, kAccSplitWarps = 8;
 template <int D, bool X3, int NH, int CR>
 constexpr int acc_min_blocks() { return (X3 && D == 128) ? 2 : D == 128 ? (NH == 1 ? 4 : 3) : (X3 && D == 64 && NH == 2) ? 3 : 4; }
 // A warp's rings: keys with their table rows, and values.
-template <int D, bool X3, int NH, int CR>
+template <int D, bool X3, int NH, int CR, int PK = 1>
 struct AccRings {
-    static constexpr int NSTG = acc_stages<D, X3, NH, CR>();
-    using C = TForm<D, X3, CR>;
+    // (lists of several queries beside three slots would cost warps: 12000 positions, 512 nodes per layer 3.60 -> 3.32 ms with two)
+    static constexpr int NSTG = PK > 1 && acc_stages<D, X3, NH, CR>() > 2 ? 2 : acc_stages<D, X3, NH, CR>();
+    using C = TForm<D, X3, CR, PK>;
     using Keys = WarpRing<NSTG, C::KSLOT + (NSTG > 1 ? C::VSLOT : 0)>;      // (of several stages: with the values)
     using Values = WarpRing<1, C::VSLOT>;
     static constexpr size_t kBytes = Keys::kBytes + (NSTG > 1 ? 0 : Values::kBytes);
 };
 
-template <typename T, int D, bool X3, int NH, int CR, bool SPLIT>
+template <typename T, int D, bool X3, int NH, int CR, bool SPLIT, int PK>
 __global__ void __launch_bounds__((SPLIT ? kAccSplitWarps : kAccWarps) * 32, SPLIT ? 1 : acc_min_blocks<D, X3, NH, CR>())
 acc_mma_kernel(const __grid_constant__ AttnParams p) {
-    using C = TForm<D, X3, CR>;
+    static_assert(PK == 1 || (NH == 1 && CR == 16 && !SPLIT), "several queries share a warp's 8 columns");
+    using C = TForm<D, X3, CR, PK>;
+    using QC = Cols<PK>;
     using FT = typename std::conditional<X3, __half, T>::type;        // type of the values and probabilities
     using F = Frag<FT>;
     constexpr int MT = C::MT, PPC = C::PPC;
-    using Ring = AccRings<D, X3, NH, CR>;
-    constexpr int NSTG = Ring::NSTG;
+    using Ring = AccRings<D, X3, NH, CR, PK>;
+    constexpr int NSTG = Ring::NSTG, GP = QC::GP;
     extern __shared__ __align__(128) unsigned char smem_raw[];
 
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, g = lane >> 2, r = lane & 3;
     const int W = SPLIT ? kAccSplitWarps : blockDim.x >> 5;
     const int from_end = SPLIT ? (int)blockIdx.x : (int)(blockIdx.x * W + warp);
-    if (!SPLIT && from_end >= p.Tq) return;
-    const int tl = p.Tq - 1 - from_end;                               // the longest walks first: they would be the tail of a short call
-    const int t = p.t0 + tl;
+    const int npack = PK == 1 ? p.Tq : (p.Tq + PK - 1) / PK;
+    if (!SPLIT && from_end >= npack) return;
+    const int tl = (npack - 1 - from_end) * PK;                       // the longest walks first: they would be the tail of a short call
     const int b = blockIdx.y / p.Hkv, hk = blockIdx.y % p.Hkv;
     const int G = p.G, TK = p.TK, L = p.L;
     const int first = SPLIT ? warp : 0, step = SPLIT ? W : 1;         // this warp's chunks of every level
 
     // per warp: ring, parent list, kept-candidate bits
     const WalkLayout lay = walk_layout(p, CR);
-    const size_t per_warp = walk_warp_bytes<Ring>(lay);
+    const size_t per_warp = walk_warp_bytes<Ring, PK>(lay);
     unsigned char* wbase = smem_raw + warp * per_warp;
     typename Ring::Keys kring;
     typename Ring::Values vring;
     kring.init(wbase);
     vring.init(wbase + Ring::Keys::kBytes);
-    const ParentList par{wbase + Ring::kBytes, lay.narrow};
-    uint32_t* selw = reinterpret_cast<uint32_t*>(wbase + Ring::kBytes + lay.list);
+    auto list_of = [&](int j) { return ParentList{wbase + Ring::kBytes + j * lay.list, lay.narrow}; };        // query tl + j
+    auto bits_of = [&](int j) { return reinterpret_cast<uint32_t*>(wbase + Ring::kBytes + PK * lay.list + j * lay.bits); };
+    const ParentList par = list_of(0);
+    uint32_t* selw = bits_of(0);
 
     const int64_t hbase = ((int64_t)b * p.Tq + tl) * p.H + (int64_t)hk * G;
     const int64_t qidx = ((int64_t)b * p.Tq + tl) * p.Hkv + hk;
 
     QueryRegs<T, D, X3, NH> q;
-    load_query<T, D, X3, NH>(reinterpret_cast<const T*>(p.q) + hbase * D, G, g, r, p.scale, q);
+    load_query<T, D, X3, NH, PK>([&](int h) -> const T* {
+        const int j = QC::of_lane(g), head = PK == 1 ? 8 * h + g : g % GP;
+        return head < G && (PK == 1 || tl + j < p.Tq) ? reinterpret_cast<const T*>(p.q) + (hbase + (int64_t)j * p.H + head) * D : nullptr;
+    }, r, p.scale, q);
+    const uint32_t tab_of_lane = PK == 1 ? 0 : QC::of_lane(g) * C::TAB;
 
     float O[NH][MT][4];
 #pragma unroll
@@ -100,20 +110,41 @@ acc_mma_kernel(const __grid_constant__ AttnParams p) {
         const int Nl = p.ln[l];
         __syncwarp();
         const int nblk = (Nl + CR - 1) / CR;
-        const int np = par.load(p, l, qidx * TK, nblk, 4, lane);
-        const int rc = (int)(((int64_t)t / p.lpow[l]) % CR);
-        const int nc = (np - 1) * CR + rc + 1, rp = nc - 1;
-        if (l > 0 && nc <= TK) continue;                              // every candidate is kept: nothing to accumulate
-        if (np <= 0) continue;
-        const int nchunk = (np + PPC - 1) / PPC;
-        __syncwarp();
+        int np, rp, nchunk = 0;
+        UnionWalk<PK> walk;
+        if constexpr (PK == 1) {
+            np = par.load(p, l, qidx * TK, nblk, 4, lane);
+            const int nc = (np - 1) * CR + (int)(((int64_t)(p.t0 + tl) / p.lpow[l]) % CR) + 1;
+            rp = nc - 1;
+            if (l > 0 && nc <= TK) continue;                          // every candidate is kept: nothing to accumulate
+            if (np <= 0) continue;
+            nchunk = (np + PPC - 1) / PPC;
+            __syncwarp();
+        } else {
+            np = rp = 0;                                              // of query lane mod PK
+            for (int j = 0; j < PK; ++j) {
+                if (tl + j >= p.Tq) break;
+                int n = list_of(j).load(p, l, (qidx + (int64_t)j * p.Hkv) * TK, nblk, 4, lane);
+                const int right = (n - 1) * CR + (int)(((int64_t)(p.t0 + tl + j) / p.lpow[l]) % CR);
+                if (l > 0 && right < TK) n = 0;                       // every candidate is kept: nothing to accumulate
+                if (l > 0 && n > 0) {
+                    uint32_t* bits = bits_of(j);
+                    for (int i = lane; i < (right + 32) / 32; i += 32) bits[i] = 0u;
+                    __syncwarp();
+                    mark_kept(p, l, (qidx + (int64_t)j * p.Hkv) * TK, list_of(j), n, CR, bits, lane);
+                }
+                if (lane % PK == j) { np = n; rp = right; }
+            }
+            __syncwarp();
+            walk.start(list_of(lane % PK), l > 0 ? bits_of(lane % PK) : nullptr, np, rp);
+        }
 
         const uint32_t bstride = (uint32_t)p.Hkv * C::BLOCK;                // (a grid has at most 65535 KV heads)
         const unsigned char* blk = reinterpret_cast<const unsigned char*>(p.blk[l]) + ((int64_t)b * nblk * p.Hkv + hk) * C::BLOCK;
         const unsigned char* tab = reinterpret_cast<const unsigned char*>(p.tab);
         int n0 = 0, n1 = 0;                                           // the parents of the chunk whose keys were fetched last
-        auto fill_keys = [&](int c) {                                 // chunk c of this level
-            n0 = par[c * PPC];
+        auto fill_keys = [&](int c) {                                 // chunk c of this level (several queries: of n0, c being this lane's row)
+            if constexpr (PK == 1) n0 = par[c * PPC];
             kring.template copy<C::PB>(0, blk + (uint64_t)(uint32_t)n0 * bstride, lane);
             if constexpr (X3) kring.template copy<16>(C::DATA, blk + (uint64_t)(uint32_t)n0 * bstride + C::FACS_OFF, lane);
             if constexpr (CR == 8) {
@@ -121,6 +152,7 @@ acc_mma_kernel(const __grid_constant__ AttnParams p) {
                 kring.template copy<C::PB>(C::PB, blk + (uint64_t)(uint32_t)n1 * bstride + 2 * C::ODD, lane);
                 if constexpr (X3) kring.template copy<16>(C::DATA + 16, blk + (uint64_t)(uint32_t)n1 * bstride + C::FACS_OFF, lane);
             }
+            if constexpr (PK > 1) { copy_tab_rows<PK, C::TAB>(kring, C::TAB_OFF, tab, c, lane); return; }
             const unsigned char* row = tab + (uint32_t)(rp - 16 * c) * C::TAB;
             kring.template copy<C::TAB>(C::TAB_OFF, row, lane);
             if constexpr (C::DUAL) kring.template copy<C::TAB>(C::TAB_OFF + C::TAB, rp - 16 * c >= 8 ? row - 8 * C::TAB : row, lane);
@@ -132,29 +164,34 @@ acc_mma_kernel(const __grid_constant__ AttnParams p) {
         };
         kring.start();
         vring.start();
+        // several queries: the masks (of this lane's query) of the chunks that are on their way, and whether the chunk behind them exists
+        constexpr int AHEAD = NSTG == 1 ? 1 : NSTG - 1;
+        uint32_t masks[AHEAD];
+        int pending = 0;
+        bool more = true;
         int next = first;
-#pragma unroll 1
-        for (int s = 0; s < (NSTG == 1 ? 1 : NSTG - 1); ++s, next += step) {
-            if (next < nchunk) fill_keys(next);
+        auto fetch_keys = [&](int slot) {
+            if constexpr (PK == 1) {
+                more = next < nchunk;
+                if (more) fill_keys(next);
+            } else {
+                n0 = more ? walk.step() : -1;
+                more = n0 >= 0;
+                masks[slot] = more ? walk.mask() : 0u;
+                if (more) { fill_keys(walk.row()); ++pending; }
+            }
+        };
+#pragma unroll
+        for (int s = 0; s < AHEAD; ++s, next += step) {
+            fetch_keys(s);
             if constexpr (NSTG == 1) kring.commit();
-            if (next < nchunk) fill_values();
+            if (more) fill_values();
             if constexpr (NSTG == 1) vring.commit(); else kring.commit();
         }
-        if (l > 0) {
-            // positions the next level kept, from its list (both lists ascending); found while the first blocks are on their way
-            for (int i = lane; i < (nc + 31) / 32; i += 32) selw[i] = 0u;
+        if (PK == 1 && l > 0) {                                       // found while the first blocks are on their way
+            for (int i = lane; i < (rp + 32) / 32; i += 32) selw[i] = 0u;
             __syncwarp();
-            for (int i = lane; i < TK; i += 32) {
-                const int node = load_parent(p, l - 1, qidx * TK + i);
-                if (node < 0) continue;
-                const int parent = node / CR;
-                int lo = 0, hi = np;
-                while (lo < hi) { const int mid = (lo + hi) >> 1; if (par[mid] < parent) lo = mid + 1; else hi = mid; }
-                if (lo < np && par[lo] == parent) {
-                    const int j = lo * CR + node % CR;
-                    atomicOr(&selw[j >> 5], 1u << (j & 31));
-                }
-            }
+            mark_kept(p, l, qidx * TK, par, np, CR, selw, lane);
         }
         auto chunk_mask = [&](int c) {                                // the chunk's candidates that accumulate
             uint32_t mask = 0xffffu;
@@ -165,7 +202,7 @@ acc_mma_kernel(const __grid_constant__ AttnParams p) {
         float2 fac[2] = {make_float2(1.f, 1.f), make_float2(1.f, 1.f)};
         auto scores = [&](uint32_t slot, uint32_t mask, const LaneBase<D, X3, CR>& lb, float (&S)[NH][4]) {
             chunk_factors<D, X3, CR>(slot, fac);
-            score_t<T, D, X3, NH, CR>(lb, slot, r, q, S);
+            score_t<T, D, X3, NH, CR>(lb, slot, r, q, S, tab_of_lane);
             if constexpr (X3) {
                 const float f0 = fac[0].x * q.inv, f1 = fac[1].x * q.inv;
 #pragma unroll
@@ -194,18 +231,31 @@ acc_mma_kernel(const __grid_constant__ AttnParams p) {
             for (int i = 0; i < MT; ++i) { O[h][i][e] *= f; O[h][i][2 + e] *= f; }
         };
 #pragma unroll 1
-        for (int c = first; c < (SPLIT ? nchunk + first : nchunk); c += step) {      // SPLIT: rounds of W chunks, some of the last missing
+        for (int c = first; PK > 1 ? pending > 0 : c < (SPLIT ? nchunk + first : nchunk); c += step) {      // SPLIT: rounds of W chunks, some of the last missing
+            uint32_t mask;                                            // the chunk's candidates that accumulate
+            bool any;
+            if constexpr (PK > 1) {
+                any = __any_sync(0xffffffffu, masks[0] != 0u);
+                mask = __shfl_sync(0xffffffffu, masks[0], QC::of_pair(r));        // those of the lane's columns
+                --pending;
+#pragma unroll
+                for (int s = 0; s + 1 < AHEAD; ++s) masks[s] = masks[s + 1];
+            }
             if constexpr (NSTG > 1) {
                 __syncwarp();                                         // everybody is done with the slots that are refilled now
-                if (next < nchunk) { fill_keys(next); fill_values(); }
+                fetch_keys(AHEAD - 1);
+                if (more) fill_values();
                 kring.commit();
                 next += step;
             }
-            const uint32_t mask = SPLIT && c >= nchunk ? 0u : chunk_mask(c);
+            if constexpr (PK == 1) {
+                mask = SPLIT && c >= nchunk ? 0u : chunk_mask(c);
+                any = mask != 0u;
+            }
             const uint32_t keys = kring.template wait<NSTG == 1 ? 1 : NSTG - 1>();
             const LaneBase<D, X3, CR> lb(keys, keys, lane);
             float S[NH][4];
-            if (mask != 0) {
+            if (any) {
                 scores(keys, mask, lb, S);
             } else {                                                  // nothing to accumulate
 #pragma unroll
@@ -216,7 +266,7 @@ acc_mma_kernel(const __grid_constant__ AttnParams p) {
                 for (int h = 0; h < NH; ++h) consumed(S[h]);
                 if constexpr (X3) asm volatile("" ::"f"(fac[0].x), "f"(fac[0].y), "f"(fac[1].x), "f"(fac[1].y) : "memory");
                 __syncwarp();                                         // everybody is done with the keys
-                if (next < nchunk) fill_keys(next);
+                fetch_keys(0);
                 kring.commit();
             }
             auto wait_values = [&]() {                                // (of a chunk fetched as one they are here already)
@@ -225,12 +275,12 @@ acc_mma_kernel(const __grid_constant__ AttnParams p) {
             auto values_done = [&]() {                                // and with the values: the next chunk's follow
                 if constexpr (NSTG == 1) {
                     __syncwarp();
-                    if (next < nchunk) fill_values();
+                    if (more) fill_values();
                     vring.commit();
                     next += step;
                 }
             };
-            if (!SPLIT && mask == 0) {
+            if (!SPLIT && !any) {
                 wait_values();
                 values_done();
                 continue;
@@ -299,25 +349,30 @@ acc_mma_kernel(const __grid_constant__ AttnParams p) {
                     for (int h = 0; h < NH; ++h)
 #pragma unroll
                         for (int e = 0; e < 2; ++e) {
-                            const float n = mask != 0 ? mine[h][e] : after[h][e];
+                            const float n = any ? mine[h][e] : after[h][e];
                             later |= n != after[h][e];
                             rescale(h, e, n);
                         }
                     moved = __any_sync(0xffffffffu, later);
                     exponents();
                 }
-                if (mask == 0) {
+                if (!any) {
                     wait_values();
                     values_done();
                     continue;
                 }
             } else {
-                moved = __any_sync(0xffffffffu, top > kMove);
+                const uint32_t over = __ballot_sync(0xffffffffu, top > kMove);
+                moved = over != 0u;
                 if (moved) {
+                    const bool mine = PK == 1 || (over & QC::lanes_of_pair(r)) != 0u;      // a query's reference follows its own scores
 #pragma unroll
                     for (int h = 0; h < NH; ++h)
 #pragma unroll
-                        for (int e = 0; e < 2; ++e) rescale(h, e, fmaxf(m_run[h][e], head_max(S[h][e], S[h][2 + e])));
+                        for (int e = 0; e < 2; ++e) {
+                            const float m = head_max(S[h][e], S[h][2 + e]);
+                            rescale(h, e, mine ? fmaxf(m_run[h][e], m) : m_run[h][e]);
+                        }
                     exponents();
                 }
             }
@@ -443,10 +498,11 @@ acc_mma_kernel(const __grid_constant__ AttnParams p) {
     for (int h = 0; h < NH; ++h)
 #pragma unroll
         for (int e = 0; e < 2; ++e) {
-            const int head = 8 * h + 2 * r + e;
-            if (head >= G) continue;
+            const int j = QC::of_pair(r), head = PK == 1 ? 8 * h + 2 * r + e : (2 * r + e) % GP;
+            if (head >= G || (PK > 1 && tl + j >= p.Tq)) continue;
+            const int64_t at = hbase + (int64_t)j * p.H + head;
             const float inv = 1.f / s_run[h][e];
-            T* orow = reinterpret_cast<T*>(p.out) + (hbase + head) * D + C::VB * g;
+            T* orow = reinterpret_cast<T*>(p.out) + at * D + C::VB * g;
             if constexpr (sizeof(T) == 4) {
 #pragma unroll
                 for (int i = 0; i < MT / 2; ++i)
@@ -462,32 +518,15 @@ acc_mma_kernel(const __grid_constant__ AttnParams p) {
                     *reinterpret_cast<uint2*>(orow) = make_uint2(w[0], w[1]);
                 }
             }
-            if (g == 0) { p.gmax[hbase + head] = m_true[h][e]; p.gsum[hbase + head] = s_run[h][e] * __expf(m_run[h][e] - m_true[h][e]); }
+            if (g == 0) { p.gmax[at] = m_true[h][e]; p.gsum[at] = s_run[h][e] * __expf(m_run[h][e] - m_true[h][e]); }
         }
     }
 }
 
-template <typename T, int D, bool X3, int NH, int CR>
-static int launch_acc_cr(const AttnParams& p, cudaStream_t st) {
-    using C = TForm<D, X3, CR>;
-    using Ring = AccRings<D, X3, NH, CR>;
-    const size_t per_warp = walk_warp_bytes<Ring>(walk_layout(p, CR));
-    const size_t limit = 227 * 1024;
-    // Few groups: one block of 8 warps per group.  Below two groups per SM the chip has room for all their warps at once, and
-    // a single warp's walk over its chunks (about 1 us each) would be the whole time of the call.  Calls whose state the
-    // backward reads (they keep their selections) always take one warp per group: a query's result then does not depend on
-    // how many queries share the call.
-    const int64_t groups = (int64_t)p.Tq * p.B * p.Hkv;
-    const size_t split_smem = kAccSplitWarps * (per_warp + 48 * sizeof(float));
-    if ((p.flags & kFlagSplitOk) && groups <= 2 * 148 && split_smem <= limit) {
-        auto* k = acc_mma_kernel<T, D, X3, NH, CR, true>;
-        static SmemLimit shared;
-        const cudaError_t e = shared.raise((const void*)k, split_smem);
-        if (e != cudaSuccess) return (int)e;
-        k<<<dim3(p.Tq, p.B * p.Hkv), kAccSplitWarps * 32, split_smem, st>>>(p);
-        note_launch();
-        return (int)cudaGetLastError();
-    }
+// One warp per group, or per PK queries.
+template <typename T, int D, bool X3, int NH, int CR, int PK>
+static int launch_acc_warps(const AttnParams& p, cudaStream_t st) {
+    const size_t per_warp = walk_warp_bytes<AccRings<D, X3, NH, CR, PK>, PK>(walk_layout(p, CR));
     // warps per block: as many resident warps as registers allow, fewer where long parent lists leave no room for the rings
     const int max_warps = kAccWarps * acc_min_blocks<D, X3, NH, CR>();
     int W = 1, best = 0;
@@ -497,14 +536,42 @@ static int launch_acc_cr(const AttnParams& p, cudaStream_t st) {
         if (blocks * w > max_warps) blocks = max_warps / w;
         if (blocks > 0 && blocks * w > best) { best = blocks * w; W = w; }
     }
-    if (best == 0 || W * per_warp > limit) return HTREE_E_UNSUPPORTED;
-    auto* k = acc_mma_kernel<T, D, X3, NH, CR, false>;
+    if (best == 0 || W * per_warp > 227 * 1024) return HTREE_E_UNSUPPORTED;
+    auto* k = acc_mma_kernel<T, D, X3, NH, CR, false, PK>;
     static SmemLimit shared;
     const cudaError_t e = shared.raise((const void*)k, W * per_warp);
     if (e != cudaSuccess) return (int)e;
-    k<<<dim3((p.Tq + W - 1) / W, p.B * p.Hkv), W * 32, W * per_warp, st>>>(p);
+    k<<<dim3((p.Tq + PK * W - 1) / (PK * W), p.B * p.Hkv), W * 32, W * per_warp, st>>>(p);
     note_launch();
     return (int)cudaGetLastError();
+}
+
+template <typename T, int D, bool X3, int NH, int CR>
+static int launch_acc_cr(const AttnParams& p, cudaStream_t st) {
+    const size_t per_warp = walk_warp_bytes<AccRings<D, X3, NH, CR>>(walk_layout(p, CR));
+    // Few groups: one block of 8 warps per group.  Below two groups per SM the chip has room for all their warps at once, and
+    // a single warp's walk over its chunks (about 1 us each) would be the whole time of the call.  Calls whose state the
+    // backward reads (they keep their selections) always take one warp per group: a query's result then does not depend on
+    // how many queries share the call.
+    const int64_t groups = (int64_t)p.Tq * p.B * p.Hkv;
+    const size_t split_smem = kAccSplitWarps * (per_warp + 48 * sizeof(float));
+    if ((p.flags & kFlagSplitOk) && groups <= 2 * 148 && split_smem <= 227 * 1024) {
+        auto* k = acc_mma_kernel<T, D, X3, NH, CR, true, 1>;
+        static SmemLimit shared;
+        const cudaError_t e = shared.raise((const void*)k, split_smem);
+        if (e != cudaSuccess) return (int)e;
+        k<<<dim3(p.Tq, p.B * p.Hkv), kAccSplitWarps * 32, split_smem, st>>>(p);
+        note_launch();
+        return (int)cudaGetLastError();
+    }
+    if constexpr (NH == 1 && CR == 16) {
+        const int PK = queries_per_warp(CR, p.G, p.TK, (p.ln[0] + CR - 1) / CR, groups);
+        int rc = HTREE_E_UNSUPPORTED;
+        if (PK == 2) rc = launch_acc_warps<T, D, X3, NH, CR, 2>(p, st);
+        if (PK == 4) rc = launch_acc_warps<T, D, X3, NH, CR, 4>(p, st);
+        if (rc != HTREE_E_UNSUPPORTED) return rc;
+    }
+    return launch_acc_warps<T, D, X3, NH, CR, 1>(p, st);
 }
 
 template <typename T, int D, bool X3>

@@ -75,7 +75,7 @@ struct BwdLayout {
     BwdParams bp;
     int64_t acc_bytes, scratch_bytes, zero_bytes;
     int64_t acck[HTREE_MAX_LEVELS], accv[HTREE_MAX_LEVELS], gk[HTREE_MAX_LEVELS], gv[HTREE_MAX_LEVELS];
-    int64_t o_qb, o_dob, o_stp, o_sts, o_fac, o_rank, o_cnt, o_base, o_entries, o_items, o_nitems;
+    int64_t o_qb, o_dob, o_stp, o_sts, o_fac, o_rank, o_nvis, o_cnt, o_base, o_entries, o_items, o_nitems;
     int total, per_launch;
 };
 
@@ -87,10 +87,13 @@ static int bwd_layout(const HtreeShape* s, int L, const int32_t* ln, int64_t bud
     const int NH = G > 8 ? 2 : 1, Tq = s->T_q > 0 ? s->T_q : s->T;
     BwdParams& bp = y.bp;
     auto up = [](int64_t x) { return (x + 255) & ~int64_t(255); };
+    const int64_t units = (int64_t)s->B * s->H_kv;
+    const int PK = bp.PK = queries_per_warp(CR, G, TK, (ln[0] + CR - 1) / CR, units * Tq);
+    const bool many = PK > 1;
     int64_t at = 0, MV = 0, NK = 0;
     for (int l = L - 1; l >= 0; --l) {
-        const int64_t nblk = (ln[l] + CR - 1) / CR, np = nblk < TK ? nblk : TK;
-        const bool used = l == 0 || np * CR > TK;      // does any query accumulate here?
+        const int64_t nblk = (ln[l] + CR - 1) / CR, one = nblk < TK ? nblk : TK, np = nblk < (int64_t)PK * TK ? nblk : (int64_t)PK * TK;
+        const bool used = l == 0 || one * CR > TK;     // does any query accumulate here?
         bp.voff[l] = used ? (int32_t)MV : -1;
         bp.koff[l] = (int32_t)NK;
         if (used) { MV += np; NK += nblk; }
@@ -106,38 +109,41 @@ static int bwd_layout(const HtreeShape* s, int L, const int32_t* ln, int64_t bud
     }
     y.acc_bytes = at;
     const int64_t qb = (int64_t)NH * D * 16 * (x3 ? 2 : 1), sb = (int64_t)NH * (CR / 8) * 128 * (x3 ? 2 : 1);
-    const int64_t units = (int64_t)s->B * s->H_kv;
+    const int64_t entry = x3 ? (many ? sizeof(BwdEntry<true, true>) : sizeof(BwdEntry<true, false>)) : (many ? sizeof(BwdEntry<false, true>) : sizeof(BwdEntry<false, false>));
     // A window's blocked queries (4 KB each at 16 heads of 128) should stay in the L2 while its parents gather them: 8192 queries
     // are 33 MB; longer windows mean longer visit lists and fewer reductions.
-    int64_t subq = 0, bytes = 0;
+    int64_t subq = 0, ng = 0, bytes = 0;
     for (int64_t most = 8192; most >= 16; most >>= 1) {
         const int64_t nw = (Tq + most - 1) / most;
-        subq = (Tq + nw - 1) / nw;
-        const int64_t visits = subq * MV;
-        bytes = up(subq * qb) * 2 + up(visits * sb) * 2 + up(visits * 4) + (x3 ? up(visits * 16) + up(subq * L * 8) : up(visits * 8)) + 2 * up(NK * 4) + up((visits / 8 + NK) * 16) + 256;
+        subq = ((Tq + nw - 1) / nw + PK - 1) / PK * PK;
+        ng = subq / PK;
+        const int64_t visits = ng * MV;
+        bytes = up(ng * qb) * 2 + up(visits * sb) * 2 + up(visits * (many ? 16 : 4)) + up(visits * entry) + (x3 ? up(ng * L * 8) : 0) + (many ? up(ng * L * 4) : 0) +
+                2 * up(NK * 4) + up((visits / 8 + NK) * 16) + 256;
         if (bytes <= budget && visits < (int64_t(1) << 31)) { bp.nw = (int32_t)nw; break; }
     }
     if (bp.nw == 0) return HTREE_E_SCRATCH;
-    bp.subq = (int32_t)subq; bp.MV = (int32_t)MV; bp.NK = (int32_t)NK;
+    bp.subq = (int32_t)subq; bp.ng = (int32_t)ng; bp.MV = (int32_t)MV; bp.NK = (int32_t)NK;
     y.total = (int)(units * bp.nw);
     int64_t per = budget / bytes;
-    if (per > 32767 / subq) per = 32767 / subq;
-    if (per * subq * MV >= (int64_t(1) << 31)) per = ((int64_t(1) << 31) - 1) / (subq * MV);
+    if (per > 32767 / ng) per = 32767 / ng;
+    if (per * ng * MV >= (int64_t(1) << 31)) per = ((int64_t(1) << 31) - 1) / (ng * MV);
     if (per > y.total) per = y.total;
     if (per < 1) per = 1;
     const int64_t launches = (y.total + per - 1) / per;
     per = (y.total + launches - 1) / launches;
     y.per_launch = (int)per;
     // items long enough to pay for their reduction (64 visits: 128 bytes of it a visit), short enough to fill the chip
-    int64_t seg = per * subq * MV / (148 * 16 * 3);
+    int64_t seg = per * ng * MV / (148 * 16 * 3);
     bp.seg = (int32_t)(seg < 8 ? 8 : seg > 64 ? 64 : seg);
-    bp.cap = (int32_t)(subq * MV / bp.seg + NK);
+    bp.cap = (int32_t)(ng * MV / bp.seg + NK);
     at = 0;
     auto take = [&](int64_t n) { const int64_t o = at; at += up(n); return o; };
-    y.o_qb = take(per * subq * qb); y.o_dob = take(per * subq * qb);
-    y.o_stp = take(per * subq * MV * sb); y.o_sts = take(per * subq * MV * sb);
-    y.o_fac = x3 ? take(per * subq * L * 8) : -1;
-    y.o_rank = take(per * subq * MV * 4); y.o_entries = take(per * subq * MV * (int64_t)(x3 ? sizeof(BwdEntry<true>) : sizeof(BwdEntry<false>)));
+    y.o_qb = take(per * ng * qb); y.o_dob = take(per * ng * qb);
+    y.o_stp = take(per * ng * MV * sb); y.o_sts = take(per * ng * MV * sb);
+    y.o_fac = x3 ? take(per * ng * L * 8) : -1;
+    y.o_nvis = many ? take(per * ng * L * 4) : -1;
+    y.o_rank = take(per * ng * MV * (many ? 16 : 4)); y.o_entries = take(per * ng * MV * entry);
     y.o_cnt = take(per * NK * 4 + 4 + units * 4); y.o_base = take(per * NK * 8);
     y.o_items = take(per * bp.cap * (int64_t)sizeof(BwdItem)); y.o_nitems = take(per * 4);
     y.scratch_bytes = at;
@@ -556,7 +562,8 @@ int htree_b200_run_backward(const HtreeShape* shape, const void* q, void* const*
     p.dq = typed ? nullptr : static_cast<float*>(dq); p.dq_typed = typed ? dq : nullptr;
     bp.qb = sb + y.o_qb; bp.dob = sb + y.o_dob; bp.stp = sb + y.o_stp; bp.sts = sb + y.o_sts;
     bp.fac = y.o_fac < 0 ? nullptr : reinterpret_cast<float2*>(sb + y.o_fac);
-    bp.rank = reinterpret_cast<int32_t*>(sb + y.o_rank); bp.entries = sb + y.o_entries;
+    bp.rank = reinterpret_cast<int32_t*>(sb + y.o_rank); bp.vis = reinterpret_cast<uint4*>(sb + y.o_rank);
+    bp.nvis = y.o_nvis < 0 ? nullptr : reinterpret_cast<int32_t*>(sb + y.o_nvis); bp.entries = sb + y.o_entries;
     bp.cnt = reinterpret_cast<int32_t*>(sb + y.o_cnt); bp.range = reinterpret_cast<uint32_t*>(bp.cnt + (int64_t)y.per_launch * bp.NK); bp.base = reinterpret_cast<int2*>(sb + y.o_base);
     bp.items = reinterpret_cast<BwdItem*>(sb + y.o_items); bp.nitems = reinterpret_cast<int32_t*>(sb + y.o_nitems);
     cudaStream_t st = (cudaStream_t)stream;

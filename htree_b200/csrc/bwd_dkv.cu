@@ -128,11 +128,39 @@ __global__ void __launch_bounds__(256) bwd_fill_kernel(const __grid_constant__ B
             const uint32_t where = (uint32_t)grp | ((uint32_t)(rp - CR * i) << 15);
             if (bp.fac) {
                 const float2 f = bp.fac[grp * p.L + l];
-                reinterpret_cast<BwdEntry<true>*>(bp.entries)[entry0 + at.x + rank] = BwdEntry<true>{(uint32_t)v, where, f.x, f.y};
+                reinterpret_cast<BwdEntry<true, false>*>(bp.entries)[entry0 + at.x + rank] = BwdEntry<true, false>{(uint32_t)v, where, f.x, f.y};
             } else {
-                reinterpret_cast<BwdEntry<false>*>(bp.entries)[entry0 + at.x + rank] = BwdEntry<false>{(uint32_t)v, where};
+                reinterpret_cast<BwdEntry<false, false>*>(bp.entries)[entry0 + at.x + rank] = BwdEntry<false, false>{(uint32_t)v, where};
             }
             if (rank % bp.seg == 0) items[at.y + rank / bp.seg] = BwdItem{bp.koff[l] + x, at.x + rank, min(bp.seg, cnt[x] - rank), 0};
+        }
+    }
+}
+
+// The same for groups of several queries, whose visits the first pass has listed.
+__global__ void __launch_bounds__(256) bwd_fill_many_kernel(const __grid_constant__ BwdParams bp) {
+    const AttnParams& p = bp.a;
+    const int lane = threadIdx.x & 31, gi = (int)((blockIdx.x * blockDim.x + threadIdx.x) >> 5);
+    if (gi >= bp.ng || ((bp.sub0 + (int)blockIdx.y) % bp.nw) * bp.subq + gi * bp.PK >= p.Tq) return;
+    const int64_t grp = (int64_t)blockIdx.y * bp.ng + gi, entry0 = (int64_t)blockIdx.y * bp.ng * bp.MV;
+    BwdItem* items = bp.items + (int64_t)blockIdx.y * bp.cap;
+    for (int l = p.L - 1; l >= 0; --l) {
+        if (bp.voff[l] < 0) continue;
+        const int n = bp.nvis[grp * p.L + l];
+        const int2* base = bp.base + (int64_t)blockIdx.y * bp.NK + bp.koff[l];
+        const int32_t* cnt = bp.cnt + (int64_t)blockIdx.y * bp.NK + bp.koff[l];
+        for (int i = lane; i < n; i += 32) {
+            const int64_t v = grp * bp.MV + bp.voff[l] + i;
+            const uint4 x = bp.vis[v];
+            const int2 at = base[x.x];
+            const int rank = (int)x.y;
+            if (bp.fac) {
+                const float2 f = bp.fac[grp * p.L + l];
+                reinterpret_cast<BwdEntry<true, true>*>(bp.entries)[entry0 + at.x + rank] = BwdEntry<true, true>{(uint32_t)v, (uint32_t)grp, {x.z, x.w}, f.x, f.y, {0.f, 0.f}};
+            } else {
+                reinterpret_cast<BwdEntry<false, true>*>(bp.entries)[entry0 + at.x + rank] = BwdEntry<false, true>{(uint32_t)v, (uint32_t)grp, {x.z, x.w}};
+            }
+            if (rank % bp.seg == 0) items[at.y + rank / bp.seg] = BwdItem{bp.koff[l] + (int)x.x, at.x + rank, min(bp.seg, cnt[x.x] - rank), 0};
         }
     }
 }
@@ -151,7 +179,7 @@ constexpr int dkv_stages() { return X3 || (KEYS && D == 128 && NH == 2) ? 2 : 3;
 template <int D, bool X3, int CR, bool KEYS>
 constexpr int dkv_min_blocks() { return X3 ? (D == 128 ? 2 : !KEYS && (D == 32 || CR == 8) ? 6 : 3) : D == 128 ? 3 : 4; }
 
-template <typename T, int D, bool X3, int NH, int CR, bool KEYS>
+template <typename T, int D, bool X3, int NH, int CR, bool KEYS, int PK>
 __global__ void __launch_bounds__(128, dkv_min_blocks<D, X3, CR, KEYS>()) bwd_dkv_kernel(const __grid_constant__ BwdParams bp) {
     using BF = BForm<D, X3, NH, CR>;
     using C = TForm<D, X3, CR>;
@@ -159,7 +187,8 @@ __global__ void __launch_bounds__(128, dkv_min_blocks<D, X3, CR, KEYS>()) bwd_dk
     using F = Frag<FT>;
     constexpr int KS = BF::KS, NT = BF::NT, QB = BF::QB, SB = BF::SB, PPT = C::PPT, HALF = C::HALF;
     constexpr int TAB = KEYS ? C::TAB : 0;
-    constexpr int SLOT = 2 * QB + 2 * SB + 2 * TAB, NSTG = dkv_stages<D, X3, NH, KEYS>();
+    constexpr int SLOT = 2 * QB + 2 * SB + 2 * PK * TAB, NSTG = dkv_stages<D, X3, NH, KEYS>();
+    const uint32_t tab_of_pair = PK == 1 ? 0 : Cols<PK>::of_pair(threadIdx.x & 3) * TAB;
     constexpr int PLANE = NT * 128;                                         // bytes from the hi to the lo words of a record
     using Ring = WarpRing<NSTG, SLOT>;
     extern __shared__ __align__(128) unsigned char smem_raw[];
@@ -170,8 +199,8 @@ __global__ void __launch_bounds__(128, dkv_min_blocks<D, X3, CR, KEYS>()) bwd_dk
     const BwdItem item = bp.items[(int64_t)ls * bp.cap + it];
     Ring ring;
     ring.init(smem_raw + (size_t)warp * Ring::kBytes);
-    using Entry = BwdEntry<X3>;
-    const Entry* entries = reinterpret_cast<const Entry*>(bp.entries) + (int64_t)ls * bp.subq * bp.MV + item.start;
+    using Entry = BwdEntry<X3, (PK > 1)>;
+    const Entry* entries = reinterpret_cast<const Entry*>(bp.entries) + (int64_t)ls * bp.ng * bp.MV + item.start;
     const unsigned char* qsrc = KEYS ? bp.qb : bp.dob;
     const unsigned char* ssrc = KEYS ? bp.sts : bp.stp;
     const unsigned char* tab = reinterpret_cast<const unsigned char*>(p.tab);
@@ -210,15 +239,24 @@ __global__ void __launch_bounds__(128, dkv_min_blocks<D, X3, CR, KEYS>()) bwd_dk
             }
         }
         const uint32_t ax = __shfl_sync(0xffffffffu, cur.visit, e0 & 31), ay = __shfl_sync(0xffffffffu, cur.where, e0 & 31);
+        auto tab_rows = [&](int e, uint32_t off) {                     // of entry e, a row per query
+            if constexpr (KEYS && PK > 1) {
+                uint32_t w = __shfl_sync(0xffffffffu, cur.rows[0], e & 31);
+                if constexpr (PK > 2) { const uint32_t w1 = __shfl_sync(0xffffffffu, cur.rows[1], e & 31); if (lane & 2) w = w1; }
+                copy_tab_rows<PK, C::TAB>(ring, off, tab, (int)(lane & 1 ? w >> 16 : w & 0xffffu), lane);
+            }
+        };
         ring.template copy<NH * QB>(0, qsrc + (int64_t)(ay & 0x7fffu) * (NH * QB), lane);
         ring.template copy<NH * SB>(2 * QB, ssrc + (int64_t)ax * (NH * SB), lane);
-        if constexpr (KEYS) ring.template copy<TAB>(2 * QB + 2 * SB, tab + (int64_t)(ay >> 15) * C::TAB, lane);
+        if constexpr (KEYS && PK == 1) ring.template copy<TAB>(2 * QB + 2 * SB, tab + (int64_t)(ay >> 15) * C::TAB, lane);
+        tab_rows(e0, 2 * QB + 2 * SB);
         if constexpr (VPS == 2) {
             const int e1 = min(e0 + 1, len - 1);
             const uint32_t bx = __shfl_sync(0xffffffffu, cur.visit, e1 & 31), by = __shfl_sync(0xffffffffu, cur.where, e1 & 31);
             ring.template copy<QB>(QB, qsrc + (int64_t)(by & 0x7fffu) * QB, lane);
             ring.template copy<SB>(2 * QB + SB, ssrc + (int64_t)bx * SB, lane);
-            if constexpr (KEYS) ring.template copy<TAB>(2 * QB + 2 * SB + TAB, tab + (int64_t)(by >> 15) * C::TAB, lane);
+            if constexpr (KEYS && PK == 1) ring.template copy<TAB>(2 * QB + 2 * SB + TAB, tab + (int64_t)(by >> 15) * C::TAB, lane);
+            tab_rows(e1, 2 * QB + 2 * SB + PK * TAB);
         }
     };
     int next = 0;
@@ -262,7 +300,7 @@ __global__ void __launch_bounds__(128, dkv_min_blocks<D, X3, CR, KEYS>()) bwd_dk
         }
         if constexpr (KEYS && !X3) {
             const uint32_t sel = (g & 1) ? 0x3232u : 0x1010u;
-            const uint32_t ta = slot + 2 * QB + 2 * SB + 2 * PPT * (g >> 1), tb = VPS == 2 ? ta + TAB : ta;
+            const uint32_t ta = slot + 2 * QB + 2 * SB + 2 * PPT * (g >> 1) + tab_of_pair, tb = VPS == 2 ? ta + PK * TAB : ta;
 #pragma unroll
             for (int k4 = 0; k4 < KS; k4 += 4) {
                 const uint4 ca4 = lds_u4(ta + 4 * k4), sa4 = lds_u4(ta + 2 * HALF + 4 * k4);
@@ -305,7 +343,7 @@ __global__ void __launch_bounds__(128, dkv_min_blocks<D, X3, CR, KEYS>()) bwd_dk
 #pragma unroll
                     for (int v = 0; v < 2; ++v) {
                         const uint4 x = lds_u4(slot + v * QB + i * 512 + lane * 16);
-                        const uint32_t t4 = slot + 2 * QB + 2 * SB + (VPS == 2 ? v : 0) * TAB + 4 * (PPT * (g >> 1) + 2 * i + (g & 1));
+                        const uint32_t t4 = slot + 2 * QB + 2 * SB + (VPS == 2 ? v : 0) * PK * TAB + tab_of_pair + 4 * (PPT * (g >> 1) + 2 * i + (g & 1));
                         const float cs = __uint_as_float(lds32(t4)), sn = __uint_as_float(lds32(t4 + 4 * HALF));
                         float2 u, w;
                         rotate_pairs_f32(make_float2(__uint_as_float(x.x), __uint_as_float(x.y)), make_float2(__uint_as_float(x.z), __uint_as_float(x.w)),
@@ -413,13 +451,13 @@ __global__ void __launch_bounds__(128) bwd_fold_kernel(const __grid_constant__ F
     }
 }
 
-template <typename T, int D, bool X3, int NH, int CR, bool KEYS>
+template <typename T, int D, bool X3, int NH, int CR, bool KEYS, int PK>
 static int launch_dkv_one(const BwdParams& bp, cudaStream_t st) {
     using BF = BForm<D, X3, NH, CR>;
-    constexpr int SLOT = 2 * BF::QB + 2 * BF::SB + (KEYS ? 2 * TForm<D, X3, CR>::TAB : 0);
+    constexpr int SLOT = 2 * BF::QB + 2 * BF::SB + (KEYS ? 2 * PK * TForm<D, X3, CR>::TAB : 0);
     using Ring = WarpRing<dkv_stages<D, X3, NH, KEYS>(), SLOT>;
     const size_t smem = 4 * Ring::kBytes;
-    auto* k = bwd_dkv_kernel<T, D, X3, NH, CR, KEYS>;
+    auto* k = bwd_dkv_kernel<T, D, X3, NH, CR, KEYS, PK>;
     static SmemLimit shared;
     const cudaError_t e = shared.raise((const void*)k, smem);
     if (e != cudaSuccess) return (int)e;
@@ -429,8 +467,13 @@ static int launch_dkv_one(const BwdParams& bp, cudaStream_t st) {
 }
 template <typename T, int D, bool X3, int NH, int CR>
 static int launch_dkv_cr(const BwdParams& bp, cudaStream_t st) {
-    const int rc = launch_dkv_one<T, D, X3, NH, CR, true>(bp, st);
-    return rc ? rc : launch_dkv_one<T, D, X3, NH, CR, false>(bp, st);
+    int rc;
+    if constexpr (NH == 1 && CR == 16) {
+        if (bp.PK == 2) { rc = launch_dkv_one<T, D, X3, NH, CR, true, 2>(bp, st); return rc ? rc : launch_dkv_one<T, D, X3, NH, CR, false, 2>(bp, st); }
+        if (bp.PK == 4) { rc = launch_dkv_one<T, D, X3, NH, CR, true, 4>(bp, st); return rc ? rc : launch_dkv_one<T, D, X3, NH, CR, false, 2>(bp, st); }
+    }
+    rc = launch_dkv_one<T, D, X3, NH, CR, true, 1>(bp, st);
+    return rc ? rc : launch_dkv_one<T, D, X3, NH, CR, false, 1>(bp, st);
 }
 template <typename T, int D, bool X3>
 static int launch_dkv_t(const BwdParams& bp, cudaStream_t st) {
@@ -472,7 +515,8 @@ int launch_bwd_begin(const BwdParams& bp, int dtype, void* zero, int64_t zero_by
 int launch_bwd_dkv(const BwdParams& bp, int dtype, cudaStream_t st) {
     bwd_scan_kernel<<<bp.nsub, 1024, 0, st>>>(bp);
     note_launch();
-    bwd_fill_kernel<<<dim3((bp.subq + 7) / 8, bp.nsub), 256, 0, st>>>(bp);
+    if (bp.PK > 1) bwd_fill_many_kernel<<<dim3((bp.ng + 7) / 8, bp.nsub), 256, 0, st>>>(bp);
+    else bwd_fill_kernel<<<dim3((bp.subq + 7) / 8, bp.nsub), 256, 0, st>>>(bp);
     note_launch();
     const cudaError_t e = cudaGetLastError();
     if (e != cudaSuccess) return (int)e;

@@ -13,8 +13,8 @@
 
 namespace htree {
 
-template <int D, bool X3>
-constexpr int dq_stages() { return D * (X3 ? 2 : 1) >= 128 ? 2 : 3; }     // slots of 8 KB: warps matter more than depth
+template <int D, bool X3, int PK>
+constexpr int dq_stages() { return D * (X3 ? 2 : 1) >= 128 ? 2 : PK > 1 ? 2 : 3; }     // slots of 8 KB: warps matter more than depth
 // Warps per block and blocks per SM: registers first.  The ring takes nearly all of the SM's L1, so anything that spills is
 // re-read from L2 in every chunk: with 180 bytes of spills, groups of 16 heads of 128 spent 4.6 of 9.4 cycles per instruction
 // waiting for it.  Those run as blocks of one warp (at most 20 bytes of spills at 12 warps per SM; the compiler keeps 150 in larger
@@ -25,42 +25,59 @@ constexpr int dq_warps() { return D == 128 && !X3 && NH == 2 ? 1 : 4; }
 template <int D, bool X3, int NH>
 constexpr int dq_min_blocks() { return D == 32 && NH == 1 ? 4 : (D == 128 && (X3 || NH == 2)) ? (X3 ? 2 : 12) : (X3 && NH == 2) ? 2 : 3; }
 
-template <typename T, int D, bool X3, int NH, int CR>
+// SUMS: 16-bit dq takes R(-distance) (K'^T dS^T) too, whose distance may differ by query.  Calls whose queries could share a warp
+// take it however many there are, so that dq does not depend on that; elsewhere rotating the keys is 4% faster.
+template <typename T, int D, bool X3, int NH, int CR, int PK, bool SUMS>
 __global__ void __launch_bounds__(dq_warps<D, X3, NH>() * 32, dq_min_blocks<D, X3, NH>()) bwd_dq_kernel(const __grid_constant__ BwdParams bp) {
-    using C = TForm<D, X3, CR>;
+    static_assert(PK == 1 || (NH == 1 && CR == 16 && (X3 || SUMS)), "several queries share a warp's 8 columns");
+    using C = TForm<D, X3, CR, PK>;
+    using QC = Cols<PK>;
     using BF = BForm<D, X3, NH, CR>;
     using F = Frag<typename std::conditional<X3, __half, T>::type>;
     using FT = typename std::conditional<X3, __half, T>::type;
     using FS = Frag<__half>;
-    constexpr int KS = C::KS, PPT = C::PPT, PPC = C::PPC, HALF = C::HALF;
-    constexpr int NSTG = dq_stages<D, X3>();
+    constexpr int KS = C::KS, PPT = C::PPT, PPC = C::PPC, HALF = C::HALF, GP = QC::GP;
+    constexpr int NSTG = dq_stages<D, X3, PK>();
     using Ring = WarpRing<NSTG, C::KSLOT + C::VSLOT>;
     extern __shared__ __align__(128) unsigned char smem_raw[];
     const AttnParams& p = bp.a;
 
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, g = lane >> 2, r = lane & 3;
     const int W = blockDim.x >> 5;
-    const int qi = (int)(gridDim.x - 1 - blockIdx.x) * W + warp;      // the longest walks first: they would be the tail of the launch
+    const int gi = (int)(gridDim.x - 1 - blockIdx.x) * W + warp;      // the longest walks first: they would be the tail of the launch
+    const int qi = gi * PK;
     const int sub = bp.sub0 + blockIdx.y, unit = sub / bp.nw;
     const int tl = (sub % bp.nw) * bp.subq + qi;
     if (qi >= bp.subq || tl >= p.Tq) return;
-    const int t = p.t0 + tl;
     const int b = unit / p.Hkv, hk = unit % p.Hkv;
     const int G = p.G, TK = p.TK, L = p.L;
-    const int grp = blockIdx.y * bp.subq + qi;
+    const int grp = blockIdx.y * bp.ng + gi;
 
     const WalkLayout lay = walk_layout(p, CR);
-    const size_t per_warp = walk_warp_bytes<Ring>(lay);
+    const size_t per_warp = walk_warp_bytes<Ring, PK>(lay);
     unsigned char* wbase = smem_raw + warp * per_warp;
     Ring ring;
     ring.init(wbase);
-    const ParentList par{wbase + Ring::kBytes, lay.narrow};
-    uint32_t* selw = reinterpret_cast<uint32_t*>(wbase + Ring::kBytes + lay.list);
+    auto list_of = [&](int j) { return ParentList{wbase + Ring::kBytes + j * lay.list, lay.narrow}; };        // query tl + j
+    auto bits_of = [&](int j) { return reinterpret_cast<uint32_t*>(wbase + Ring::kBytes + PK * lay.list + j * lay.bits); };
+    const ParentList par = list_of(0);
+    uint32_t* selw = bits_of(0);
     const int64_t hbase = ((int64_t)b * p.Tq + tl) * p.H + (int64_t)hk * G;
     const int64_t qidx = ((int64_t)b * p.Tq + tl) * p.Hkv + hk;
 
     QueryRegs<T, D, X3, NH> q;
-    load_query<T, D, X3, NH>(reinterpret_cast<const T*>(p.q) + hbase * D, G, g, r, p.scale, q);
+    // the rows of column 8h + g (operands) and of columns 8h + 2r, + 1 (results), or -1
+    auto row_of_lane = [&](int h) -> int64_t {
+        const int j = QC::of_lane(g), head = PK == 1 ? 8 * h + g : g % GP;
+        return head < G && (PK == 1 || tl + j < p.Tq) ? hbase + (int64_t)j * p.H + head : -1;
+    };
+    auto row_of_pair = [&](int h, int e) -> int64_t {
+        const int j = QC::of_pair(r), head = PK == 1 ? 8 * h + 2 * r + e : (2 * r + e) % GP;
+        return head < G && (PK == 1 || tl + j < p.Tq) ? hbase + (int64_t)j * p.H + head : -1;
+    };
+    const uint32_t tab_of_lane = PK == 1 ? 0 : QC::of_lane(g) * C::TAB, tab_of_pair = PK == 1 ? 0 : QC::of_pair(r) * C::TAB;
+    load_query<T, D, X3, NH, PK>([&](int h) -> const T* { const int64_t at = row_of_lane(h); return at < 0 ? nullptr : reinterpret_cast<const T*>(p.q) + at * D; },
+                                 r, p.scale, q);
     uint32_t dO[NH][2][KS], dOl[X3 ? NH : 1][2][X3 ? KS : 1];
     float Drow[NH][2], lse[NH][2], ginv[NH][2];
     constexpr float kPScale = 16384.f;                  // split-half: P is carried times 2^14
@@ -74,21 +91,21 @@ __global__ void __launch_bounds__(dq_warps<D, X3, NH>() * 32, dq_min_blocks<D, X
 #pragma unroll
             for (int hf = 0; hf < 2; ++hf) {
                 float x[D / 8];
-                load_row_piece_f32<T, D>(reinterpret_cast<const T*>(p.dO) + (hbase + 8 * h + g) * D + hf * HALF + PPT * r, 8 * h + g < G, x);
+                load_row_piece_f32<T, D>(reinterpret_cast<const T*>(p.dO) + row_of_lane(h) * D + hf * HALF + PPT * r, row_of_lane(h) >= 0, x);
 #pragma unroll
                 for (int i = 0; i < D / 8; ++i) most = fmaxf(most, fabsf(x[i]));
             }
-        dscale = range_scale_coarse(redux_max_f32(most, 0xffffffffu));
-        dinv = pow2_inverse(dscale) * (1.f / kPScale);
+        dscale = range_scale_coarse(QC::max_of(most));
+        dinv = QC::for_pair(pow2_inverse(dscale), r) * (1.f / kPScale);
     }
 #pragma unroll
     for (int h = 0; h < NH; ++h) {
-        const int head = 8 * h + g;
-        const bool on = head < G;
+        const int64_t row = row_of_lane(h);
+        const bool on = row >= 0;
         float sum = 0.f, l1 = 0.f;                      // dO . out and |dO|_1 of this lane's head
 #pragma unroll
         for (int hf = 0; hf < 2; ++hf) {
-            const int64_t off = (hbase + head) * D + hf * HALF + PPT * r;
+            const int64_t off = row * D + hf * HALF + PPT * r;
             if constexpr (X3) {
                 float x[D / 8], o[D / 8];
                 load_row_piece_f32<T, D>(reinterpret_cast<const T*>(p.dO) + off, on, x);
@@ -117,22 +134,23 @@ __global__ void __launch_bounds__(dq_warps<D, X3, NH>() * 32, dq_min_blocks<D, X
         l1 += __shfl_xor_sync(0xffffffffu, l1, 1);
         l1 += __shfl_xor_sync(0xffffffffu, l1, 2);
         if constexpr (!X3) {
-            bound_v = fmaxf(bound_v, redux_max_f32(l1, 0xffffffffu));
+            bound_v = fmaxf(bound_v, QC::max_of(l1));
         } else {
-            bound_v = fmaxf(bound_v, kPScale * 16384.f * redux_max_f32(l1, 0xffffffffu));      // values are carried below 2^14
-            bound_d = fmaxf(bound_d, kPScale * redux_max_f32(fabsf(sum), 0xffffffffu));
+            bound_v = fmaxf(bound_v, kPScale * 16384.f * QC::max_of(l1));      // values are carried below 2^14
+            bound_d = fmaxf(bound_d, kPScale * QC::max_of(fabsf(sum)));
         }
 #pragma unroll
         for (int e = 0; e < 2; ++e) {
-            const int hd = 8 * h + 2 * r + e;
+            const int64_t at = row_of_pair(h, e);
             Drow[h][e] = __shfl_sync(0xffffffffu, sum, 4 * (2 * r + e));
-            const float gm = hd < G ? p.gmax[hbase + hd] : 0.f, gs = hd < G ? p.gsum[hbase + hd] : 1.f;
+            const float gm = at >= 0 ? p.gmax[at] : 0.f, gs = at >= 0 ? p.gsum[at] : 1.f;
             // 16-bit: P = 2^(S log2 e - lse); split-half: exp(S - gmax) * ginv (an exponent re-based by log2 e rounds at 1e-6)
-            lse[h][e] = X3 ? gm : (hd < G ? gm * kLog2e + __log2f(gs) : INFINITY);
-            ginv[h][e] = hd < G ? kPScale / gs : 0.f;
+            lse[h][e] = X3 ? gm : (at >= 0 ? gm * kLog2e + __log2f(gs) : INFINITY);
+            ginv[h][e] = at >= 0 ? kPScale / gs : 0.f;
         }
     }
 
+    bound_v = QC::for_pair(bound_v, r); bound_d = QC::for_pair(bound_d, r);
     float rescale = 1.f;                                // 16-bit: from dS as carried for dq to dS as carried in the records
     if constexpr (!X3) {
         const uint32_t v = __ldg(bp.range + 1 + unit);
@@ -182,19 +200,40 @@ __global__ void __launch_bounds__(dq_warps<D, X3, NH>() * 32, dq_min_blocks<D, X
         const int Nl = p.ln[l];
         const int nblk = (Nl + CR - 1) / CR;
         __syncwarp();
-        const int np = par.load(p, l, qidx * TK, nblk, 8, lane);
-        const int rc = (int)(((int64_t)t / p.lpow[l]) % CR);
-        const int nc = (np - 1) * CR + rc + 1, rp = nc - 1;
-        if (np <= 0 || (l > 0 && nc <= TK)) continue;
-        const int nchunk = (np + PPC - 1) / PPC;
-        __syncwarp();
+        int np, rp, nchunk = 0;
+        UnionWalk<PK> walk;
+        if constexpr (PK == 1) {
+            np = par.load(p, l, qidx * TK, nblk, 8, lane);
+            rp = (np - 1) * CR + (int)(((int64_t)(p.t0 + tl) / p.lpow[l]) % CR);
+            if (np <= 0 || (l > 0 && rp + 1 <= TK)) continue;
+            nchunk = (np + PPC - 1) / PPC;
+            __syncwarp();
+        } else {
+            np = rp = 0;                                              // of query lane mod PK
+            for (int j = 0; j < PK; ++j) {
+                if (tl + j >= p.Tq) break;
+                int n = list_of(j).load(p, l, (qidx + (int64_t)j * p.Hkv) * TK, nblk, 8, lane);
+                const int right = (n - 1) * CR + (int)(((int64_t)(p.t0 + tl + j) / p.lpow[l]) % CR);
+                if (l > 0 && right < TK) n = 0;
+                if (l > 0 && n > 0) {
+                    uint32_t* bits = bits_of(j);
+                    for (int i = lane; i < (right + 32) / 32; i += 32) bits[i] = 0u;
+                    __syncwarp();
+                    mark_kept(p, l, (qidx + (int64_t)j * p.Hkv) * TK, list_of(j), n, CR, bits, lane);
+                }
+                if (lane % PK == j) { np = n; rp = right; }
+            }
+            __syncwarp();
+            walk.start(list_of(lane % PK), l > 0 ? bits_of(lane % PK) : nullptr, np, rp);
+        }
         const int64_t blk0 = (int64_t)b * nblk * p.Hkv + hk;
         const unsigned char* kblk = reinterpret_cast<const unsigned char*>(p.blk[l]) + blk0 * C::BLOCK;
         const unsigned char* vblk = reinterpret_cast<const unsigned char*>(p.vkblk[l]) + blk0 * (C::PL * C::PART);
-        auto fill = [&](int c) {
+        const uint32_t kstride = (uint32_t)p.Hkv * C::BLOCK;
+        auto fill = [&](int c, int p0) {                              // chunk c; several queries: of parent p0, c being this lane's row
             constexpr int PB = C::PB;
-            const uint32_t kstride = (uint32_t)p.Hkv * C::BLOCK, vstride = (uint32_t)p.Hkv * PB;
-            const int p0 = par[c * PPC];
+            const uint32_t vstride = (uint32_t)p.Hkv * PB;
+            if constexpr (PK == 1) p0 = par[c * PPC];
             ring.template copy<PB>(0, kblk + (uint64_t)(uint32_t)p0 * kstride, lane);
             ring.template copy<PB>(C::KSLOT, vblk + (uint64_t)(uint32_t)p0 * vstride, lane);
             if constexpr (CR == 8) {
@@ -204,67 +243,109 @@ __global__ void __launch_bounds__(dq_warps<D, X3, NH>() * 32, dq_min_blocks<D, X
                 if constexpr (X3) ring.template copy<16>(C::DATA + 16, kblk + (uint64_t)(uint32_t)p1 * kstride + C::FACS_OFF, lane);
             }
             if constexpr (X3) ring.template copy<16>(C::DATA, kblk + (uint64_t)(uint32_t)p0 * kstride + C::FACS_OFF, lane);
+            if constexpr (PK > 1) { copy_tab_rows<PK, C::TAB>(ring, C::TAB_OFF, p.tab, c, lane); return; }
             const unsigned char* row = reinterpret_cast<const unsigned char*>(p.tab) + (uint32_t)(rp - 16 * c) * C::TAB;
             ring.template copy<C::TAB>(C::TAB_OFF, row, lane);
             if constexpr (C::DUAL) ring.template copy<C::TAB>(C::TAB_OFF + C::TAB, rp - 16 * c >= 8 ? row - 8 * C::TAB : row, lane);
         };
         ring.start();
-        int next = 0;
-#pragma unroll 1
-        for (; next < NSTG - 1; ++next) {
-            if (next < nchunk) fill(next);
-            ring.commit();
-        }
         // this visit's place in its parent's list
         int32_t* cnt = bp.cnt + (int64_t)blockIdx.y * bp.NK + bp.koff[l];
+        const int visit0 = grp * bp.MV + bp.voff[l];
+        constexpr int AHEAD = NSTG - 1;
+        uint32_t masks[AHEAD];                                        // several queries: of the chunks on their way, for this lane's
+        uint4 placed = make_uint4(0u, 0u, 0u, 0u);                    // the visit fetched last (its rank arrives during a chunk)
+        int next = 0, pending = 0;
+        bool more = true;
+        auto fetch = [&](int slot) {
+            if constexpr (PK == 1) {
+                if (next < nchunk) fill(next, 0);
+                ++next;
+            } else {
+                const int parent = more ? walk.step() : -1;
+                more = parent >= 0;
+                masks[slot] = more ? walk.mask() : 0u;
+                if (more) {
+                    const int row = walk.row();
+                    fill(row, parent);
+                    uint32_t rows[2] = {0u, 0u};
+#pragma unroll
+                    for (int j = 0; j < PK; ++j) rows[j >> 1] |= (uint32_t)__shfl_sync(0xffffffffu, row, j) << (16 * (j & 1));
+                    if (lane == 0) {
+                        if (next) bp.vis[visit0 + next - 1] = placed;
+                        placed = make_uint4((uint32_t)parent, (uint32_t)atomicAdd(cnt + parent, 1), rows[0], rows[1]);
+                    }
+                    ++next; ++pending;
+                }
+            }
+            ring.commit();
+        };
+#pragma unroll
+        for (int s = 0; s < AHEAD; ++s) fetch(s);
         float v = 0.f;                                                // split-half: the largest factor of the values that will be met
-        for (int i = lane; i < np; i += 32) {
-            bp.rank[(int64_t)grp * bp.MV + bp.voff[l] + i] = atomicAdd(cnt + par[i], 1);
-            if constexpr (X3) v = fmaxf(v, __ldg(reinterpret_cast<const float*>(kblk + (uint64_t)(uint32_t)par[i] * ((uint32_t)p.Hkv * C::BLOCK) + C::FACS_OFF) + 1));
+        if constexpr (PK == 1) {
+            for (int i = lane; i < np; i += 32) {
+                bp.rank[visit0 + i] = atomicAdd(cnt + par[i], 1);
+                if constexpr (X3) v = fmaxf(v, __ldg(reinterpret_cast<const float*>(kblk + (uint64_t)(uint32_t)par[i] * kstride + C::FACS_OFF) + 1));
+            }
+            if constexpr (X3) v = redux_max_f32(v, 0xffffffffu);
+        } else if constexpr (X3) {
+#pragma unroll
+            for (int j = 0; j < PK; ++j) {
+                const int n = __shfl_sync(0xffffffffu, np, j);
+                float x = 0.f;
+                for (int i = lane; i < n; i += 32) x = fmaxf(x, __ldg(reinterpret_cast<const float*>(kblk + (uint64_t)(uint32_t)list_of(j)[i] * kstride + C::FACS_OFF) + 1));
+                x = redux_max_f32(x, 0xffffffffu);
+                if (QC::of_pair(r) == j) v = x;
+            }
         }
+        float krat = 1.f, vrat = 1.f;                                 // several queries, split-half: to the factors that a record's columns share
         if constexpr (X3) {
             // dS's scale follows from a bound, 2^4 to 2^8 above what ordinary data reach at P = 1.  Found per level: per chunk, from the
             // largest |dS| or from the chunk's own factor, cost the pass 5 to 7% (32-wide heads)
-            v = redux_max_f32(v, 0xffffffffu);
             if (v > vtop) {
                 const float s = range_scale_coarse(fmaf(bound_v, v, bound_d)), f = s * pow2_inverse(sscale);
                 vtop = v; sscale = s; back = dinv * pow2_inverse(s);
 #pragma unroll
                 for (int h = 0; h < NH; ++h) { Drow[h][0] *= f; Drow[h][1] *= f; }
             }
-            if (lane == 0) bp.fac[(int64_t)grp * L + l] = make_float2(back * q.inv, dinv);
-        }
-        if (l > 0) {
-            for (int i = lane; i < (nc + 31) / 32; i += 32) selw[i] = 0u;
-            __syncwarp();
-            for (int i = lane; i < TK; i += 32) {
-                const int node = load_parent(p, l - 1, qidx * TK + i);
-                if (node < 0) continue;
-                const int parent = node / CR;
-                int lo = 0, hi = np;
-                while (lo < hi) { const int mid = (lo + hi) >> 1; if (par[mid] < parent) lo = mid + 1; else hi = mid; }
-                if (lo < np && par[lo] == parent) {
-                    const int j = lo * CR + node % CR;
-                    atomicOr(&selw[j >> 5], 1u << (j & 31));
-                }
+            float fk = back * q.inv, fv = dinv;
+            if constexpr (PK > 1) {
+                const float ck = redux_max_f32(fk, 0xffffffffu), cv = redux_max_f32(fv, 0xffffffffu);
+                krat = fk * pow2_inverse(ck); vrat = fv * pow2_inverse(cv);
+                fk = ck; fv = cv;
             }
+            if (lane == 0) bp.fac[(int64_t)grp * L + l] = make_float2(fk, fv);
         }
-        const int visit0 = grp * bp.MV + bp.voff[l];
-#pragma unroll 1
-        for (int c = 0; c < nchunk; ++c) {
+        if (PK == 1 && l > 0) {
+            for (int i = lane; i < (rp + 32) / 32; i += 32) selw[i] = 0u;
             __syncwarp();
-            if (next < nchunk) fill(next);
-            ring.commit();
-            ++next;
+            mark_kept(p, l, qidx * TK, par, np, CR, selw, lane);
+        }
+#pragma unroll 1
+        for (int c = 0; PK > 1 ? pending > 0 : c < nchunk; ++c) {
             uint32_t mask = 0xffffu;
-            if (l > 0) mask &= ~(selw[c >> 1] >> ((16 * c) & 31));
-            if (16 * c + 15 > rp) mask &= (2u << (rp - 16 * c)) - 1u;
+            bool any;
+            if constexpr (PK > 1) {
+                any = __any_sync(0xffffffffu, masks[0] != 0u);
+                mask = __shfl_sync(0xffffffffu, masks[0], QC::of_pair(r));        // of the lane's columns
+                --pending;
+#pragma unroll
+                for (int s = 0; s + 1 < AHEAD; ++s) masks[s] = masks[s + 1];
+            }
+            __syncwarp();
+            fetch(AHEAD - 1);
+            if constexpr (PK == 1) {
+                if (l > 0) mask &= ~(selw[c >> 1] >> ((16 * c) & 31));
+                if (16 * c + 15 > rp) mask &= (2u << (rp - 16 * c)) - 1u;
+                any = mask != 0u;
+            }
             const uint32_t slot = ring.wait();
             const LaneBase<D, X3, CR> lb(slot, slot + C::KSLOT, lane);
             const uint32_t tabs = slot + C::TAB_OFF;
 
             uint32_t pw[NH][2], sw[NH][2], pwl[X3 ? NH : 1][2], swl[X3 ? NH : 1][2];   // P^T, dS^T: word w = child g + 8w, heads 2r, 2r+1
-            if (mask == 0) {
+            if (!any) {
 #pragma unroll
                 for (int h = 0; h < NH; ++h)
 #pragma unroll
@@ -292,7 +373,7 @@ __global__ void __launch_bounds__(dq_warps<D, X3, NH>() * 32, dq_min_blocks<D, X
                 float S[NH][4];
                 float2 fac[2];
                 chunk_factors<D, X3, CR>(slot, fac);
-                score_t<T, D, X3, NH, CR>(lb, slot, r, q, S);
+                score_t<T, D, X3, NH, CR>(lb, slot, r, q, S, tab_of_lane);
                 const float sfac[2] = {fac[0].x * q.inv, fac[1].x * q.inv};
                 const bool c0 = (mask >> g) & 1, c1 = (mask >> (g + 8)) & 1;
                 uint32_t db[NH][2], dbl[X3 ? NH : 1][2];       // dS^T as B fragments (children x heads)
@@ -315,6 +396,14 @@ __global__ void __launch_bounds__(dq_warps<D, X3, NH>() * 32, dq_min_blocks<D, X
                         sw[h][0] = FS::pack(dS[0], dS[1]); sw[h][1] = FS::pack(dS[2], dS[3]);
                     }
                     db[h][0] = movm(sw[h][0]); db[h][1] = movm(sw[h][1]);
+                    if constexpr (X3 && PK > 1) {
+                        if (krat != 1.f) {
+                            split_half2(dS[0] * krat, dS[1] * krat, sw[h][0], swl[X3 ? h : 0][0]); split_half2(dS[2] * krat, dS[3] * krat, sw[h][1], swl[X3 ? h : 0][1]);
+                        }
+                        if (vrat != 1.f) {
+                            split_half2(P[0] * vrat, P[1] * vrat, pw[h][0], pwl[X3 ? h : 0][0]); split_half2(P[2] * vrat, P[3] * vrat, pw[h][1], pwl[X3 ? h : 0][1]);
+                        }
+                    }
                     if (!X3 && rescale != 1.f) {
                         sw[h][0] = FS::pack(dS[0] * rescale, dS[1] * rescale); sw[h][1] = FS::pack(dS[2] * rescale, dS[3] * rescale);
                     }
@@ -322,7 +411,7 @@ __global__ void __launch_bounds__(dq_warps<D, X3, NH>() * 32, dq_min_blocks<D, X
                 // dq^T += K~^T dS^T: transposed key fragments (rows x(ks, g)), rotated back by the chunk's distance
                 if constexpr (!X3) {
                     const uint32_t sel = (g & 1) ? 0x3232u : 0x1010u;
-                    const uint32_t tb = tabs + 2 * PPT * (g >> 1);
+                    const uint32_t tb = tabs + 2 * PPT * (g >> 1) + tab_of_pair;
 #pragma unroll
                     for (int k4 = 0; k4 < KS; k4 += 4) {
                         const uint4 c4 = lds_u4(tb + 4 * k4), s4 = lds_u4(tb + 2 * HALF + 4 * k4);
@@ -339,6 +428,18 @@ __global__ void __launch_bounds__(dq_warps<D, X3, NH>() * 32, dq_min_blocks<D, X
                             uint32_t m[4], a[4];
                             key_frag_trans<D, X3, CR>(lb, 0, ks, m);
                             const uint32_t cc = __byte_perm(cw[u], cw[u], sel), ss = __byte_perm(snw[u], snw[u], sel);
+                            if constexpr (SUMS) {            // the chunk's sums are rotated, in fp32
+                                const uint32_t am[4] = {m[0], m[2], m[1], m[3]};
+                                const float cf = __low2float(as_h2(cc)), sf = __low2float(as_h2(ss));
+                                float acc[4];
+                                mma_zero<__half>(acc, am, db[0][0], db[0][1]);
+#pragma unroll
+                                for (int e = 0; e < 2; ++e) {
+                                    dq[0][ks][e] = fmaf(acc[2 + e], sf, fmaf(acc[e], cf, dq[0][ks][e]));
+                                    dq[0][ks][2 + e] = fmaf(acc[e], -sf, fmaf(acc[2 + e], cf, dq[0][ks][2 + e]));
+                                }
+                                continue;
+                            }
                             const uint32_t ns = neg_h2(ss);                    // inverse rotation
                             rotate_h2(m[0], m[2], cc, ns, ss, a[0], a[1]);
                             if constexpr (C::DUAL) {
@@ -377,7 +478,7 @@ __global__ void __launch_bounds__(dq_warps<D, X3, NH>() * 32, dq_min_blocks<D, X
                         key_frag_trans<D, X3, CR>(lb, 0, ks, mh);
                         key_frag_trans<D, X3, CR>(lb, 1, ks, ml);
                         float cs, sn;
-                        const uint32_t tb = tabs + 4 * (PPT * (g >> 1) + 2 * ks + (g & 1));
+                        const uint32_t tb = tabs + 4 * (PPT * (g >> 1) + 2 * ks + (g & 1)) + tab_of_pair;
                         asm("ld.shared.f32 %0, [%1];" : "=f"(cs) : "r"(tb));
                         asm("ld.shared.f32 %0, [%1];" : "=f"(sn) : "r"(tb + 4 * HALF));
                         cs *= kfac; sn *= kfac;
@@ -416,7 +517,7 @@ __global__ void __launch_bounds__(dq_warps<D, X3, NH>() * 32, dq_min_blocks<D, X
                 } else {
 #pragma unroll
                     for (int w = 0; w < 2; ++w) {
-                        if (2 * c + w < np) {
+                        if (2 * c + w < np) {      // (PK == 1)
                             const int64_t o = ((int64_t)(visit0 + 2 * c + w) * NH + h) * BF::SB + lane * 4;
                             *reinterpret_cast<uint32_t*>(bp.stp + o) = pw[h][w];
                             *reinterpret_cast<uint32_t*>(bp.sts + o) = sw[h][w];
@@ -427,6 +528,12 @@ __global__ void __launch_bounds__(dq_warps<D, X3, NH>() * 32, dq_min_blocks<D, X
                         }
                     }
                 }
+            }
+        }
+        if constexpr (PK > 1) {
+            if (lane == 0) {
+                if (next) bp.vis[visit0 + next - 1] = placed;
+                bp.nvis[(int64_t)grp * L + l] = next;
             }
         }
     }
@@ -451,24 +558,29 @@ __global__ void __launch_bounds__(dq_warps<D, X3, NH>() * 32, dq_min_blocks<D, X
                 else sm[(8 * h + 2 * r + (i & 1)) * D + (i >> 1) * HALF + PPT * (g >> 1) + 2 * ks + (g & 1)] = dq[h][ks][i] * post;
             }
     __syncwarp();
-    for (int i = lane; i < G * D / 4; i += 32) {
-        const float4 x = reinterpret_cast<const float4*>(sm)[PADDED ? i / (D / 4) * (ROW / 4) + i % (D / 4) / 4 * 5 + i % 4 : i];
-        if (p.dq_typed == nullptr) {
-            reinterpret_cast<float4*>(p.dq + hbase * D)[i] = x;
-        } else if constexpr (sizeof(T) == 4) {
-            reinterpret_cast<float4*>(reinterpret_cast<float*>(p.dq_typed) + hbase * D)[i] = x;
-        } else {
-            using FP = Frag<typename std::conditional<sizeof(T) == 4, __half, T>::type>;
-            reinterpret_cast<uint2*>(reinterpret_cast<T*>(p.dq_typed) + hbase * D)[i] = make_uint2(FP::pack(x.x, x.y), FP::pack(x.z, x.w));
+    for (int j = 0; j < PK; ++j) {                                    // query by query: its G rows are in one piece
+        if (PK > 1 && tl + j >= p.Tq) break;
+        const int64_t first = (hbase + (int64_t)j * p.H) * D;
+        for (int i0 = lane; i0 < G * D / 4; i0 += 32) {
+            const int i = i0 + j * GP * (D / 4);
+            const float4 x = reinterpret_cast<const float4*>(sm)[PADDED ? i / (D / 4) * (ROW / 4) + i % (D / 4) / 4 * 5 + i % 4 : i];
+            if (p.dq_typed == nullptr) {
+                reinterpret_cast<float4*>(p.dq + first)[i0] = x;
+            } else if constexpr (sizeof(T) == 4) {
+                reinterpret_cast<float4*>(reinterpret_cast<float*>(p.dq_typed) + first)[i0] = x;
+            } else {
+                using FP = Frag<typename std::conditional<sizeof(T) == 4, __half, T>::type>;
+                reinterpret_cast<uint2*>(reinterpret_cast<T*>(p.dq_typed) + first)[i0] = make_uint2(FP::pack(x.x, x.y), FP::pack(x.z, x.w));
+            }
         }
     }
 }
 
-template <typename T, int D, bool X3, int NH, int CR>
-static int launch_dq_cr(const BwdParams& bp, cudaStream_t st) {
-    using C = TForm<D, X3, CR>;
-    using Ring = WarpRing<dq_stages<D, X3>(), C::KSLOT + C::VSLOT>;
-    const size_t per_warp = walk_warp_bytes<Ring>(walk_layout(bp.a, CR));
+template <typename T, int D, bool X3, int NH, int CR, int PK, bool SUMS>
+static int launch_dq_warps(const BwdParams& bp, cudaStream_t st) {
+    using C = TForm<D, X3, CR, PK>;
+    using Ring = WarpRing<dq_stages<D, X3, PK>(), C::KSLOT + C::VSLOT>;
+    const size_t per_warp = walk_warp_bytes<Ring, PK>(walk_layout(bp.a, CR));
     constexpr int max_w = dq_warps<D, X3, NH>(), max_warps = max_w * dq_min_blocks<D, X3, NH>();
     int W = 1, best = 0;
     for (int w = max_w; w >= 1; w >>= 1) {
@@ -477,13 +589,22 @@ static int launch_dq_cr(const BwdParams& bp, cudaStream_t st) {
         if (blocks > 0 && blocks * w > best) { best = blocks * w; W = w; }
     }
     if (best == 0 || W * per_warp > 227 * 1024) return HTREE_E_UNSUPPORTED;
-    auto* k = bwd_dq_kernel<T, D, X3, NH, CR>;
+    auto* k = bwd_dq_kernel<T, D, X3, NH, CR, PK, SUMS>;
     static SmemLimit shared;
     const cudaError_t e = shared.raise((const void*)k, W * per_warp);
     if (e != cudaSuccess) return (int)e;
-    k<<<dim3((bp.subq + W - 1) / W, bp.nsub), W * 32, W * per_warp, st>>>(bp);
+    k<<<dim3((bp.ng + W - 1) / W, bp.nsub), W * 32, W * per_warp, st>>>(bp);
     note_launch();
     return (int)cudaGetLastError();
+}
+template <typename T, int D, bool X3, int NH, int CR>
+static int launch_dq_cr(const BwdParams& bp, cudaStream_t st) {
+    if constexpr (NH == 1 && CR == 16) {
+        if (bp.PK == 2) return launch_dq_warps<T, D, X3, NH, CR, 2, !X3>(bp, st);
+        if (bp.PK == 4) return launch_dq_warps<T, D, X3, NH, CR, 4, !X3>(bp, st);
+        if (!X3 && sharing_queries(CR, bp.a.G, bp.a.TK, (bp.a.ln[0] + CR - 1) / CR) > 1) return launch_dq_warps<T, D, X3, NH, CR, 1, !X3>(bp, st);
+    }
+    return launch_dq_warps<T, D, X3, NH, CR, 1, false>(bp, st);
 }
 
 template <typename T, int D, bool X3>

@@ -17,6 +17,10 @@
 // a query's dq does not depend on the others; in a record for dK it is one of the whole call, since the sums over visits run inside
 // the products.  The two are the same wherever the magnitudes of dO differ by less than 2^4.
 //
+// Where several queries share a warp (PK > 1, tform.cuh) they are one group here: eight columns of blocked heads, one record for all who
+// visit a parent, a table row per query.  12000 positions, 16 heads of 32, top_k 512: dq 8.1 -> 6.8 ms, dK and dV 4.4 -> 2.6 ms, half the
+// records.  A query's scales are its own; a record's columns are brought to their largest factor.
+//
 // Work is cut into windows of `subq` queries of one (batch, KV head) unit, small enough for a window's blocked queries to stay
 // in L2 while its parents gather from them, and into launches of `nsub` windows, whose P and dS fit the caller's buffer.
 #pragma once
@@ -24,16 +28,20 @@
 
 namespace htree {
 
-// A visit in its parent's list: visit slot, group | table row << 15, and, split-half, the factors of dK and dV.
-template <bool X3> struct __align__(8) BwdEntry { uint32_t visit, where; };
-template <> struct __align__(16) BwdEntry<true> { uint32_t visit, where; float fk, fv; };
+// A visit in its parent's list: visit slot, group | table row << 15, and, split-half, the factors of dK and dV.  Where several queries
+// share a warp (MANY) a group is PK queries and a visit one of any of them: the group, and a table row per query in 16 bits each.
+template <bool X3, bool MANY> struct __align__(8) BwdEntry { uint32_t visit, where; };
+template <> struct __align__(16) BwdEntry<true, false> { uint32_t visit, where; float fk, fv; };
+template <> struct __align__(16) BwdEntry<false, true> { uint32_t visit, where, rows[2]; };
+template <> struct __align__(16) BwdEntry<true, true> { uint32_t visit, where, rows[2]; float fk, fv, pad[2]; };
 
 struct BwdItem { int32_t key, start, len, pad; };     // a piece of one parent's visit list
 
 struct BwdParams {
     AttnParams a;
     int32_t sub0, nsub, subq, nw;            // windows of this launch: [sub0, sub0 + nsub) of units * nw
-    int32_t MV, NK, seg, cap;                // visit slots per query, parents per unit over all levels, longest item, items per window
+    int32_t MV, NK, seg, cap;                // visit slots per group, parents per unit over all levels, longest item, items per window
+    int32_t PK, ng;                          // queries per group, groups per window (subq / PK)
     int32_t voff[HTREE_MAX_LEVELS];          // first visit slot of a level, -1: the level accumulates nothing
     int32_t koff[HTREE_MAX_LEVELS];          // first parent of a level among the NK
     unsigned char* qb;                       // blocked queries [group][half]
@@ -42,7 +50,9 @@ struct BwdParams {
     unsigned char* sts;                      // dS
     uint32_t* range;                         // 16-bit: bits of the largest |dO|_1 of a row, and of every unit's largest |v|; else unused
     float2* fac;                             // split-half: {dK, dV} factors of the visits of a group and level, [group * L + level]; else NULL
-    int32_t* rank;                           // [group * MV + visit]
+    int32_t* rank;                           // [group * MV + visit], or
+    uint4* vis;                              // MANY: {parent, rank, rows} [group * MV + visit]
+    int32_t* nvis;                           // MANY: visits [group * L + level]
     int32_t* cnt;                            // [nsub][NK]
     int2* base;                              // [nsub][NK]: first entry, first item
     void* entries;                           // [nsub][subq * MV] Entry

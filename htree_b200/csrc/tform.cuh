@@ -32,7 +32,11 @@
 
 namespace htree {
 
-template <int D, bool X3, int CR>
+// Several queries in one warp (PK > 1; groups of at most 4 heads, 16 children): consecutive positions share the 8 columns, GP = 8 / PK
+// of them each.  The warp walks the union of their parent lists; a block that several of them selected is fetched, read and multiplied
+// once, each column rotated by its own query's distance (PK table rows a chunk).  A query that did not select it has P = 0 there,
+// which changes nothing: rows are those of a walk alone, bit for bit.
+template <int D, bool X3, int CR, int PK = 1>
 struct TForm {
     static constexpr int KS = D / 16, HALF = D / 2, PPT = HALF / 4, VB = D / 8, MT = D / 16;
     static constexpr int PL = X3 ? 2 : 1;                                  // planes
@@ -43,7 +47,7 @@ struct TForm {
     static constexpr int FACS_OFF = BLOCK - FACS;
     static constexpr bool KSCALED = X3 && D != 64;                         // are a block's keys multiplied by their factor?
     static constexpr int ODD = DUAL ? 0 : PL * PART;                       // where an odd parent's copy starts in its block
-    static constexpr int NTAB = DUAL ? 2 : 1;
+    static constexpr int NTAB = DUAL ? 2 : PK;
     static constexpr int PPC = 16 / CR;                                    // parents per chunk
     static constexpr int PB = PL * PART;                                   // bytes of one part of a block
     static constexpr int DATA = PB * PPC;                                  // bytes of the keys, or of the values, of a chunk in shared memory
@@ -151,7 +155,7 @@ template <> __device__ __forceinline__ void mma_zero<__nv_bfloat16>(float (&c)[4
 
 // The query heads of a group as B fragments of the score product: lane (g, r) holds dims PPT*r + [0, PPT) of both halves of
 // head 8h + g.  16-bit path: IEEE half pairs; split-half path: fp32 values, already multiplied by the softmax scale and by the power
-// of two that brings the group's largest one to the top of half's range; `inv` is its inverse.
+// of two that brings the query's largest one to the top of half's range; `inv` is its inverse (for the columns 2r, 2r + 1).
 template <typename T, int D, bool X3, int NH>
 struct QueryRegs {
     static constexpr int N = X3 ? D / 8 : D / 16;
@@ -170,17 +174,39 @@ __device__ __forceinline__ void load_row_piece_f32(const T* p, bool on, float (&
     }
 }
 
-template <typename T, int D, bool X3, int NH>
-__device__ __forceinline__ void load_query(const T* base, int G, int g, int r, float scale, QueryRegs<T, D, X3, NH>& q) {
+// Columns of a warp and the queries they belong to.
+template <int PK>
+struct Cols {
+    static constexpr int GP = 8 / PK;                                                       // columns of a query
+    static __device__ __forceinline__ int of_lane(int g) { return PK == 1 ? 0 : g / GP; }       // query of column g (B fragments)
+    static __device__ __forceinline__ int of_pair(int r) { return PK == 1 ? 0 : 2 * r / GP; }   // query of columns 2r, 2r + 1 (C fragments)
+    // over the lanes (g, *) of a query's columns
+    static __device__ __forceinline__ float max_of(float x) {
+        if constexpr (PK == 1) return redux_max_f32(x, 0xffffffffu);
+#pragma unroll
+        for (int o = 1; o < 4 * GP; o <<= 1) x = fmaxf(x, __shfl_xor_sync(0xffffffffu, x, o));
+        return x;
+    }
+    // a value per query held by the lanes (g, *) of its columns, for the lanes (*, r)
+    static __device__ __forceinline__ float for_pair(float x, int r) { return PK == 1 ? x : __shfl_sync(0xffffffffu, x, 4 * GP * of_pair(r)); }
+    // the lanes (*, r) of the query of columns 2r, 2r + 1
+    static __device__ __forceinline__ uint32_t lanes_of_pair(int r) {
+        return PK == 1 ? 0xffffffffu : PK == 2 ? 0x33333333u << (r & 2) : 0x11111111u << r;
+    }
+};
+
+// row(h): the row of column 8h + g, or NULL.
+template <typename T, int D, bool X3, int NH, int PK = 1, typename Row>
+__device__ __forceinline__ void load_query(Row row, int r, float scale, QueryRegs<T, D, X3, NH>& q) {
     constexpr int HALF = D / 2, PPT = HALF / 4;
     float most = 0.f;
 #pragma unroll
     for (int h = 0; h < NH; ++h) {
-        const int head = 8 * h + g;
-        const bool on = head < G;
+        const T* base = row(h);
+        const bool on = base != nullptr;
 #pragma unroll
         for (int hf = 0; hf < 2; ++hf) {
-            const T* p = base + (int64_t)head * D + hf * HALF + PPT * r;
+            const T* p = base + hf * HALF + PPT * r;
             if constexpr (X3) {
                 float x[D / 8];
                 load_row_piece_f32<T, D>(p, on, x);
@@ -199,8 +225,8 @@ __device__ __forceinline__ void load_query(const T* base, int G, int g, int r, f
         }
     }
     if constexpr (X3) {
-        const float s = range_scale_coarse(redux_max_f32(most, 0xffffffffu));
-        q.inv = pow2_inverse(s);
+        const float s = range_scale_coarse(Cols<PK>::max_of(most));
+        q.inv = Cols<PK>::for_pair(pow2_inverse(s), r);
 #pragma unroll
         for (int h = 0; h < NH; ++h)
 #pragma unroll
@@ -340,8 +366,9 @@ __device__ __forceinline__ float common_factor(float a, float b, float (&ratio)[
 }
 // Scores; split-half ones still have to be multiplied by f[row / 8].x * q.inv, a power of two.
 template <typename T, int D, bool X3, int NH, int CR>
-__device__ __forceinline__ void score_t(const LaneBase<D, X3, CR>& s, uint32_t slot, int r, const QueryRegs<T, D, X3, NH>& q, float (&S)[NH][4]) {
-    const uint32_t tab = slot + TForm<D, X3, CR>::TAB_OFF;
+__device__ __forceinline__ void score_t(const LaneBase<D, X3, CR>& s, uint32_t slot, int r, const QueryRegs<T, D, X3, NH>& q, float (&S)[NH][4],
+                                        uint32_t tab_of_lane = 0) {
+    const uint32_t tab = slot + TForm<D, X3, CR>::TAB_OFF + tab_of_lane;
     if constexpr (X3) score_x3<T, D, NH, CR>(s, tab, r, q, S);
     else score16<T, D, NH, CR>(s, tab, r, q, S);
 }
@@ -419,6 +446,49 @@ struct ParentList {
         return np;
     }
 };
+// The union of PK queries' lists (of 16-bit entries), walked in ascending order.  Lane j (mod PK) holds query j's list and place in it.
+template <int PK>
+struct UnionWalk {
+    const uint16_t* list;         // of this lane's query
+    const uint32_t* selw;         // its kept-candidate bits (levels that select), or NULL
+    int np, rp, at;               // its parents, its right-most position, the next entry
+    uint32_t head;                // that entry's parent: read a step ahead
+    int rank;                     // of the step taken last: its rank in this lane's list, or -1
+    __device__ __forceinline__ void start(const ParentList& par, const uint32_t* bits, int n, int right) {
+        list = reinterpret_cast<const uint16_t*>(par.at); selw = bits; np = n; rp = right; at = 0;
+        head = n > 0 ? list[0] : 0xffffffffu;
+    }
+    // the next parent of any list, or -1
+    __device__ __forceinline__ int step() {
+        const uint32_t least = __reduce_min_sync(0xffffffffu, head);
+        const bool mine = head == least && least != 0xffffffffu;
+        rank = mine ? at : -1;
+        if (mine) { ++at; head = at < np ? list[at] : 0xffffffffu; }
+        return (int)least;
+    }
+    __device__ __forceinline__ uint32_t mask() const {               // the step's candidates that accumulate for this lane's query
+        if (rank < 0) return 0u;
+        uint32_t m = 0xffffu;
+        if (selw) m &= ~(selw[rank >> 1] >> ((16 * rank) & 31));
+        if (16 * rank + 15 > rp) m &= (2u << (rp - 16 * rank)) - 1u;
+        return m;
+    }
+    __device__ __forceinline__ int row() const { return rank < 0 ? 0 : rp - 16 * rank; }       // its distance (any row where it has no part)
+};
+// the step's table rows, one after the other
+template <int PK, int TAB, typename Ring>
+__device__ __forceinline__ void copy_tab_rows(const Ring& ring, uint32_t off, const void* tab, int row, int lane) {
+    constexpr int PER = TAB / 16;
+#pragma unroll
+    for (int i = 0; i < PK * PER; i += 32) {
+        const int piece = i + lane;
+        const int of = __shfl_sync(0xffffffffu, row, piece / PER);
+        if (PK * PER >= 32 || piece < PK * PER)
+            asm volatile("cp.async.cg.shared.global [%0], [%1], 16;\n" ::"r"(ring.fill + off + 16 * piece),
+                         "l"(static_cast<const unsigned char*>(tab) + (int64_t)of * TAB + 16 * (piece % PER)) : "memory");
+    }
+}
+
 // What the walk over a level's candidates keeps per warp beside the ring: the parent list and one bit per candidate of a level
 // that selects.  Both are bounded by the parents that the levels have.
 struct WalkLayout { int list, bits; bool narrow; };      // bytes
@@ -430,7 +500,33 @@ __host__ __device__ __forceinline__ WalkLayout walk_layout(const AttnParams& p, 
     w.bits = ((up < p.TK ? up : p.TK) * CR + 31) / 32 * 4;
     return w;
 }
-template <typename Ring>
-__host__ __device__ __forceinline__ size_t walk_warp_bytes(const WalkLayout& w) { return (Ring::kBytes + w.list + w.bits + 127) & ~size_t(127); }
+template <typename Ring, int PK = 1>
+__host__ __device__ __forceinline__ size_t walk_warp_bytes(const WalkLayout& w) { return (Ring::kBytes + PK * (w.list + w.bits) + 127) & ~size_t(127); }
+// one bit per candidate of a level that the next level kept, from its list (both lists ascending); the bits are clear and the list there
+__device__ __forceinline__ void mark_kept(const AttnParams& p, int l, int64_t list, const ParentList& par, int np, int CR, uint32_t* selw, int lane) {
+    for (int i = lane; i < p.TK; i += 32) {
+        const int node = load_parent(p, l - 1, list + i);
+        if (node < 0) continue;
+        const int parent = node / CR;
+        int lo = 0, hi = np;
+        while (lo < hi) { const int mid = (lo + hi) >> 1; if (par[mid] < parent) lo = mid + 1; else hi = mid; }
+        if (lo < np && par[lo] == parent) {
+            const int j = lo * CR + node % CR;
+            atomicOr(&selw[j >> 5], 1u << (j & 31));
+        }
+    }
+}
+// How many queries may share a warp (see the head of this file).  It pays where they select many of the same parents: with TK of n leaf
+// parents selected, PK queries meet n (1 - (1 - TK/n)^PK) of them, or all the same ones while there are no more than TK.  At TK = n/4
+// two queries still meet 12% fewer blocks than one by one; further down a step's extra work (5 to 10%) eats what is saved.
+inline int sharing_queries(int CR, int G, int TK, int leaf_parents) {
+    return CR != 16 || G > 4 || TK * 16 > 65536 || 4 * (int64_t)TK < leaf_parents ? 1 : G > 2 ? 2 : 4;
+}
+// ... and how many do: as long as their warps fill half of the chip's places, since each walks up to PK times as far.  (fp32, 2048 positions
+// of 2 x 4 heads of 64, 2048 warps instead of 4096: 84.7 -> 77.8 us.)
+inline int queries_per_warp(int CR, int G, int TK, int leaf_parents, int64_t groups) {
+    const int PK = sharing_queries(CR, G, TK, leaf_parents);
+    return groups >= (int64_t)PK * 148 * 8 ? PK : 1;
+}
 
 }  // namespace htree

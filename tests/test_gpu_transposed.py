@@ -226,3 +226,36 @@ def test_gradient_range_ignores_what_is_not_finite(dt, D, T):
         # the other rows have the same bound, or half of it: dS rounds differently where it is subnormal (2^-25 of the bound)
         assert _rel(got[:, :-1], want[:, :-1]) < 1e-4
     assert got[:, -1, 4:].isfinite().all()
+
+
+@pytest.mark.parametrize("dt,D,G,T,TK,MTN,Hkv,clustered", [
+    (HF, 32, 4, 3001, 512, 8192, 4, False),      # every query reads everything there is: lists alike
+    (FP, 32, 1, 5003, 512, 512, 2, False), (HF, 32, 2, 3001, 64, 512, 4, True), (BF, 32, 3, 2399, 64, 64, 4, False),
+    (BF, 64, 4, 4001, 64, 256, 2, True), (HF, 64, 1, 3001, 64, 64, 4, False), (FP, 64, 3, 2048, 32, 64, 4, True), (FP, 64, 4, 2049, 32, 64, 4, False),
+    (BF, 128, 4, 2047, 64, 128, 4, True), (HF, 128, 2, 4001, 128, 128, 4, False), (FP, 128, 4, 2049, 64, 64, 4, False)])
+def test_queries_that_share_a_warp(dt, D, G, T, TK, MTN, Hkv, clustered):
+    """Up to four queries of small groups walk the union of their lists in one warp.  Windows of too few queries for that take a warp
+    each: their rows, and dq, are the same bits.  (Odd lengths: the last warp has fewer queries.)"""
+    import htree_b200 as ht
+    from htree_b200 import ops
+    q, k, v, dO = _inputs(dt, 1, T, Hkv, G, D, clustered)
+    dO = dO * (torch.rand(1, T, 1, 1, device=DEV) * 8 - 4).exp2().to(dt)       # neighbours of different size
+    out, ctx = ht.htree_forward(q, k, v, 16, MTN, TK, _save_for_backward=True)
+    ours, want = ht.htree_backward(dO, q, out, ctx), ht.htree_backward(dO, q, out, ctx, _force_generic=True)
+    step, acc, outs, dqs = 1001 // Hkv, {}, [], []
+    cuts = list(range(0, T, step)) + [T]
+    for a, b in zip(cuts, cuts[1:]):
+        qw = q[:, a:b].contiguous()
+        o, c = ht.htree_forward(qw, k, v, 16, MTN, TK, _save_for_backward=True, _q_offset=a)
+        r = ht.htree_backward(dO[:, a:b].contiguous(), qw, o, c, _window=dict(t0=a, first=a == 0, last=b == T, acc=acc))
+        outs.append(o); dqs.append(r[0])
+    assert torch.equal(torch.cat(outs, 1), out), "a row depends on the queries beside it"
+    assert torch.equal(torch.cat(dqs, 1), ours[0]), "dq depends on the queries beside it"
+    # sums in another order: 1e-6 relative; 16-bit dV takes P and dS takes dP in 16 bits, alike on both sides
+    assert _rel(r[1], ours[1]) < 1e-5 and _rel(r[2], ours[2]) < 1e-5
+    exact = dt == FP or D == 32
+    if not clustered:      # (clustered scores reach 70: the half-precision operands of a score move its probability by a percent)
+        for a, b in zip(ours, want):
+            assert _rel(a, b) < (2e-5 if exact else 3e-3)
+    torch.cuda.synchronize()
+    ops.check_status()

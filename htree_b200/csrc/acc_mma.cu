@@ -43,6 +43,7 @@ struct AccRings {
 template <typename T, int D, bool X3, int NH, int CR, bool SPLIT, int PK>
 __global__ void __launch_bounds__((SPLIT ? kAccSplitWarps : kAccWarps) * 32, SPLIT ? 1 : acc_min_blocks<D, X3, NH, CR>())
 acc_mma_kernel(const __grid_constant__ AttnParams p) {
+    chain_enter();
     static_assert(PK == 1 || (NH == 1 && CR == 16 && !SPLIT), "several queries share a warp's 8 columns");
     using C = TForm<D, X3, CR, PK>;
     using QC = Cols<PK>;
@@ -541,9 +542,7 @@ static int launch_acc_warps(const AttnParams& p, cudaStream_t st) {
     static SmemLimit shared;
     const cudaError_t e = shared.raise((const void*)k, W * per_warp);
     if (e != cudaSuccess) return (int)e;
-    k<<<dim3((p.Tq + PK * W - 1) / (PK * W), p.B * p.Hkv), W * 32, W * per_warp, st>>>(p);
-    note_launch();
-    return (int)cudaGetLastError();
+    return launch_chained(k, dim3((p.Tq + PK * W - 1) / (PK * W), p.B * p.Hkv), dim3(W * 32), W * per_warp, st, p);
 }
 
 template <typename T, int D, bool X3, int NH, int CR>
@@ -560,9 +559,7 @@ static int launch_acc_cr(const AttnParams& p, cudaStream_t st) {
         static SmemLimit shared;
         const cudaError_t e = shared.raise((const void*)k, split_smem);
         if (e != cudaSuccess) return (int)e;
-        k<<<dim3(p.Tq, p.B * p.Hkv), kAccSplitWarps * 32, split_smem, st>>>(p);
-        note_launch();
-        return (int)cudaGetLastError();
+        return launch_chained(k, dim3(p.Tq, p.B * p.Hkv), dim3(kAccSplitWarps * 32), split_smem, st, p);
     }
     if constexpr (NH == 1 && CR == 16) {
         const int PK = queries_per_warp(CR, p.G, p.TK, (p.ln[0] + CR - 1) / CR, groups);

@@ -74,10 +74,13 @@ static int fill_params(AttnParams& p, const HtreeShape* s, int L, const int32_t*
 struct BwdLayout {
     BwdParams bp;
     int64_t acc_bytes, scratch_bytes, zero_bytes;
-    int64_t acck[HTREE_MAX_LEVELS], accv[HTREE_MAX_LEVELS], gk[HTREE_MAX_LEVELS], gv[HTREE_MAX_LEVELS];
+    int64_t acck[HTREE_MAX_LEVELS], accv[HTREE_MAX_LEVELS];
     int64_t o_qb, o_dob, o_stp, o_sts, o_fac, o_rank, o_nvis, o_cnt, o_base, o_entries, o_items, o_nitems;
     int total, per_launch;
 };
+
+// the counters of `windows` windows, in whole 16-byte pieces; the words of the range stand behind those of a whole launch
+static int64_t cnt_words(int64_t windows, int64_t NK) { return (windows * NK + 3) & ~int64_t(3); }
 
 static int bwd_layout(const HtreeShape* s, int L, const int32_t* ln, int64_t budget, BwdLayout& y) {
     std::memset(&y, 0, sizeof(y));
@@ -102,11 +105,6 @@ static int bwd_layout(const HtreeShape* s, int L, const int32_t* ln, int64_t bud
         y.accv[l] = at; at += up(blocks * D * CR * 4);
     }
     y.zero_bytes = at;
-    for (int l = 1; l < L; ++l) {
-        const int64_t bytes = up((int64_t)s->B * ln[l] * s->H_kv * D * 4);
-        y.gk[l] = at; at += bytes;
-        y.gv[l] = at; at += bytes;
-    }
     y.acc_bytes = at;
     const int64_t qb = (int64_t)NH * D * 16 * (x3 ? 2 : 1), sb = (int64_t)NH * (CR / 8) * 128 * (x3 ? 2 : 1);
     const int64_t entry = x3 ? (many ? sizeof(BwdEntry<true, true>) : sizeof(BwdEntry<true, false>)) : (many ? sizeof(BwdEntry<false, true>) : sizeof(BwdEntry<false, false>));
@@ -144,7 +142,7 @@ static int bwd_layout(const HtreeShape* s, int L, const int32_t* ln, int64_t bud
     y.o_fac = x3 ? take(per * ng * L * 8) : -1;
     y.o_nvis = many ? take(per * ng * L * 4) : -1;
     y.o_rank = take(per * ng * MV * (many ? 16 : 4)); y.o_entries = take(per * ng * MV * entry);
-    y.o_cnt = take(per * NK * 4 + 4 + units * 4); y.o_base = take(per * NK * 8);
+    y.o_cnt = take(cnt_words(per, NK) * 4 + 4 + units * 4); y.o_base = take(per * NK * 8);
     y.o_items = take(per * bp.cap * (int64_t)sizeof(BwdItem)); y.o_nitems = take(per * 4);
     y.scratch_bytes = at;
     return 0;
@@ -550,13 +548,11 @@ int htree_b200_run_backward(const HtreeShape* shape, const void* q, void* const*
     if (rc) return rc;
     AttnParams& p = bp.a;
     unsigned char *ab = static_cast<unsigned char*>(acc), *sb = static_cast<unsigned char*>(scratch);
-    float *gk[HTREE_MAX_LEVELS], *gv[HTREE_MAX_LEVELS];
     for (int l = 0; l < L; ++l) {
         if (!parents[l] || !blocks_bwd[l]) return HTREE_E_NULL;
         if (!aligned16(blocks_bwd[l])) return HTREE_E_ALIGN;
         p.blk[l] = blocks[l]; p.vkblk[l] = blocks_bwd[l];
         bp.acck[l] = reinterpret_cast<float*>(ab + y.acck[l]); bp.accv[l] = reinterpret_cast<float*>(ab + y.accv[l]);
-        gk[l] = reinterpret_cast<float*>(ab + y.gk[l]); gv[l] = reinterpret_cast<float*>(ab + y.gv[l]);
     }
     p.tab = table; p.out = const_cast<void*>(out); p.dO = dO; p.gmax = const_cast<float*>(gmax); p.gsum = const_cast<float*>(gsum);
     p.dq = typed ? nullptr : static_cast<float*>(dq); p.dq_typed = typed ? dq : nullptr;
@@ -564,21 +560,20 @@ int htree_b200_run_backward(const HtreeShape* shape, const void* q, void* const*
     bp.fac = y.o_fac < 0 ? nullptr : reinterpret_cast<float2*>(sb + y.o_fac);
     bp.rank = reinterpret_cast<int32_t*>(sb + y.o_rank); bp.vis = reinterpret_cast<uint4*>(sb + y.o_rank);
     bp.nvis = y.o_nvis < 0 ? nullptr : reinterpret_cast<int32_t*>(sb + y.o_nvis); bp.entries = sb + y.o_entries;
-    bp.cnt = reinterpret_cast<int32_t*>(sb + y.o_cnt); bp.range = reinterpret_cast<uint32_t*>(bp.cnt + (int64_t)y.per_launch * bp.NK); bp.base = reinterpret_cast<int2*>(sb + y.o_base);
+    bp.cnt = reinterpret_cast<int32_t*>(sb + y.o_cnt); bp.range = reinterpret_cast<uint32_t*>(bp.cnt + cnt_words(y.per_launch, bp.NK)); bp.base = reinterpret_cast<int2*>(sb + y.o_base);
     bp.items = reinterpret_cast<BwdItem*>(sb + y.o_items); bp.nitems = reinterpret_cast<int32_t*>(sb + y.o_nitems);
     cudaStream_t st = (cudaStream_t)stream;
     for (int s0 = 0; s0 < y.total; s0 += y.per_launch) {
         bp.sub0 = s0; bp.nsub = y.total - s0 < y.per_launch ? y.total - s0 : y.per_launch;
         // the counters, and ahead of the first launch (which has the most windows) the words of the range behind them
-        const cudaError_t e = cudaMemsetAsync(bp.cnt, 0, (size_t)bp.nsub * bp.NK * sizeof(int32_t) + (s0 == 0 ? (1 + (size_t)shape->B * shape->H_kv) * sizeof(uint32_t) : 0), st);
-        if (e != cudaSuccess) return (int)e;
-        rc = s0 == 0 ? launch_bwd_begin(bp, shape->dtype, acc, flags & HTREE_BWD_KEEP_ACCUM ? 0 : y.zero_bytes, st) : 0;
+        rc = launch_bwd_clear(bp.cnt, cnt_words(bp.nsub, bp.NK) * 4 + (s0 == 0 ? (1 + (int64_t)shape->B * shape->H_kv) * 4 : 0), st);
+        if (rc == 0 && s0 == 0) rc = launch_bwd_begin(bp, shape->dtype, acc, flags & HTREE_BWD_KEEP_ACCUM ? 0 : y.zero_bytes, st);
         if (rc == 0) rc = launch_bwd_dq(bp, shape->dtype, st);
         if (rc == 0) rc = launch_bwd_dkv(bp, shape->dtype, st);
         if (rc) return rc;
     }
     if (flags & HTREE_BWD_NO_FOLD) return 0;
-    return launch_bwd_fold(bp, shape->dtype, gk, gv, dk, dv, typed != 0, st);
+    return launch_bwd_fold(bp, shape->dtype, dk, dv, typed != 0, st);
 }
 
 int htree_b200_backward(const HtreeShape* shape, const void* q, void* const* layers_k, void* const* layers_v,

@@ -19,6 +19,7 @@ struct RangeArgs {
 };
 template <typename T, int D>
 __global__ void __launch_bounds__(256) bwd_range_kernel(const __grid_constant__ RangeArgs a) {
+    chain_enter();
     constexpr int LPR = D / 8, U = 4;              // lanes per row; 16-byte pieces in flight
     using F = Frag<T>;
     __shared__ float part[8];
@@ -67,6 +68,7 @@ __global__ void __launch_bounds__(256) bwd_range_kernel(const __grid_constant__ 
 // visits of one parent).  The items themselves are written by the next kernel: one block that wrote them all took 80 us where
 // parents have thousands of visits (12000 positions, 512 nodes per layer).
 __global__ void __launch_bounds__(1024) bwd_scan_kernel(const __grid_constant__ BwdParams bp) {
+    chain_enter();
     __shared__ int2 wsum[32];
     const int sub = blockIdx.x, tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const int32_t* cnt = bp.cnt + (int64_t)sub * bp.NK;
@@ -98,6 +100,7 @@ __global__ void __launch_bounds__(1024) bwd_scan_kernel(const __grid_constant__ 
 
 // One warp per group: every visit's entry goes to its place in its parent's list; the first visit of an item writes the item.
 __global__ void __launch_bounds__(256) bwd_fill_kernel(const __grid_constant__ BwdParams bp) {
+    chain_enter();
     const AttnParams& p = bp.a;
     const int lane = threadIdx.x & 31, qi = (int)((blockIdx.x * blockDim.x + threadIdx.x) >> 5);
     const int sub = bp.sub0 + blockIdx.y, unit = sub / bp.nw;
@@ -139,6 +142,7 @@ __global__ void __launch_bounds__(256) bwd_fill_kernel(const __grid_constant__ B
 
 // The same for groups of several queries, whose visits the first pass has listed.
 __global__ void __launch_bounds__(256) bwd_fill_many_kernel(const __grid_constant__ BwdParams bp) {
+    chain_enter();
     const AttnParams& p = bp.a;
     const int lane = threadIdx.x & 31, gi = (int)((blockIdx.x * blockDim.x + threadIdx.x) >> 5);
     if (gi >= bp.ng || ((bp.sub0 + (int)blockIdx.y) % bp.nw) * bp.subq + gi * bp.PK >= p.Tq) return;
@@ -195,8 +199,14 @@ __global__ void __launch_bounds__(128, dkv_min_blocks<D, X3, CR, KEYS>()) bwd_dk
     const AttnParams& p = bp.a;
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, g = lane >> 2;
     const int it = blockIdx.x * (blockDim.x >> 5) + warp, ls = blockIdx.y;
-    if (it >= bp.nitems[ls]) return;
-    const BwdItem item = bp.items[(int64_t)ls * bp.cap + it];
+    // dV needs nothing of dK's launch before it, so it does not wait for it until its own end (what it reads was complete when that launch
+    // began, and let this one be set up; read through L2, since no wait stands before the reads).
+    if constexpr (KEYS) chain_wait();
+    chain_next();
+    auto leave = [&]() { if constexpr (!KEYS) chain_wait(); };
+    if (it >= __ldcg(bp.nitems + ls)) { leave(); return; }
+    const int4 item4 = __ldcg(reinterpret_cast<const int4*>(bp.items + (int64_t)ls * bp.cap + it));
+    const BwdItem item{item4.x, item4.y, item4.z, item4.w};
     Ring ring;
     ring.init(smem_raw + (size_t)warp * Ring::kBytes);
     using Entry = BwdEntry<X3, (PK > 1)>;
@@ -213,7 +223,17 @@ __global__ void __launch_bounds__(128, dkv_min_blocks<D, X3, CR, KEYS>()) bwd_dk
 #pragma unroll
         for (int n = 0; n < NT; ++n) acc[i][n][0] = acc[i][n][1] = acc[i][n][2] = acc[i][n][3] = 0.f;
 
-    Entry cur = entries[min(lane, len - 1)], nxt = entries[min(32 + lane, len - 1)];
+    auto entry = [&](int e) {
+        Entry x;
+        if constexpr (sizeof(Entry) == 8) {
+            *reinterpret_cast<uint2*>(&x) = __ldcg(reinterpret_cast<const uint2*>(entries + min(e, len - 1)));
+        } else {
+#pragma unroll
+            for (int i = 0; i < (int)sizeof(Entry) / 16; ++i) reinterpret_cast<uint4*>(&x)[i] = __ldcg(reinterpret_cast<const uint4*>(entries + min(e, len - 1)) + i);
+        }
+        return x;
+    };
+    Entry cur = entry(lane), nxt = entry(32 + lane);
     static_assert(!X3 || NSTG == 2, "a step's factors are taken when the next one is fetched");
     float fa = 0.f, fb = 0.f;                      // split-half: the factors of the visits fetched last
     bool differ = false;                           // do they differ among the 32 of `cur`?
@@ -228,7 +248,7 @@ __global__ void __launch_bounds__(128, dkv_min_blocks<D, X3, CR, KEYS>()) bwd_dk
     auto fill = [&](int s) {                       // operand, record and table row of the step's one or two visits
         const int e0 = s * VPS;
         if (e0 && (e0 & 31) == 0) {
-            cur = nxt; nxt = entries[min(e0 + 32 + lane, len - 1)];
+            cur = nxt; nxt = entry(e0 + 32 + lane);
             compare();
         }
         if constexpr (X3) {
@@ -385,29 +405,61 @@ __global__ void __launch_bounds__(128, dkv_min_blocks<D, X3, CR, KEYS>()) bwd_dk
     for (int i = 0; i < KS; ++i)
 #pragma unroll
         for (int n = 0; n < NT; ++n) red_add_v4(dst + (i * NT + n) * 128, acc[i][n][0] * post, acc[i][n][1] * post, acc[i][n][2] * post, acc[i][n][3] * post);
+    leave();
 }
 
-// Level by level from the top: accumulators to rows (dK' rotated back by the child index), plus the share of the pooled
-// parent's gradient (src/backward.py:787-841).  blockIdx.y: 0 = dK, 1 = dV; one warp per parent block.
+// Accumulators to the leaves' gradients: dK' rotated back by the child index, plus the mean-pool shares of the ancestors' gradients
+// (src/backward.py:787-841), which every block of leaves sums up for itself from the top: a row of D per level, where a launch per
+// level would wait for the one before.  blockIdx.y: 0 = dK, 1 = dV; one warp per block of leaves.
 struct FoldArgs {
-    const float* acc[2];
-    const float* up[2];      // the level above, rows in fp32, or NULL at the top
-    void* out[2];            // this level's rows: fp32, or the storage type (typed)
+    const float* acc[2][HTREE_MAX_LEVELS];
+    void* out[2];            // leaf rows: fp32, or the storage type (typed)
     const float* cosc;
     const float* sinc;
-    int64_t total;           // blocks
-    int32_t N, Nup, NBLK, Hkv, typed;
+    int64_t total;           // blocks of leaves
+    int32_t N[HTREE_MAX_LEVELS];
+    int32_t L, Hkv, typed;
 };
 template <typename TO, int D, int CR>
 __global__ void __launch_bounds__(128) bwd_fold_kernel(const __grid_constant__ FoldArgs f) {
+    chain_enter();
     constexpr int KS = D / 16, NT = CR / 8, HALF = D / 2, PPT = HALF / 4;
     __shared__ float sm[4][CR][D + 4];
     const int which = blockIdx.y, warp = threadIdx.x >> 5, lane = threadIdx.x & 31, g = lane >> 2, r = lane & 3;
     const int64_t blk = (int64_t)blockIdx.x * 4 + warp;
     if (blk >= f.total) return;
-    const int h = (int)(blk % f.Hkv), pb = (int)((blk / f.Hkv) % f.NBLK);
-    const int64_t b = blk / ((int64_t)f.Hkv * f.NBLK);
-    const float4* a = reinterpret_cast<const float4*>(f.acc[which]) + blk * (D * CR / 4);
+    const int nblk = (f.N[0] + CR - 1) / CR;
+    const int h = (int)(blk % f.Hkv), pb = (int)((blk / f.Hkv) % nblk);
+    const int64_t b = blk / ((int64_t)f.Hkv * nblk);
+
+    // ---- the gradient of the block's own pooled row: lane x holds the pairs x + 32 u (dims x + 32 u and + D/2) ----
+    constexpr int U = HALF > 32 ? HALF / 32 : 1;
+    float ulo[U], uhi[U];
+#pragma unroll
+    for (int u = 0; u < U; ++u) ulo[u] = uhi[u] = 0.f;
+    for (int m = f.L - 1; m > 0; --m) {
+        int n = pb;
+        for (int i = 1; i < m; ++i) n /= CR;
+        const int c = n % CR, cnt = min(CR, f.N[m] - (n - c)), nb = (f.N[m] + CR - 1) / CR;
+        const float* a = f.acc[which][m] + ((b * nb + n / CR) * f.Hkv + h) * (int64_t)(D * CR);
+#pragma unroll
+        for (int u = 0; u < U; ++u) {
+            const int x = lane + 32 * u;
+            if (HALF < 32 && x >= HALF) break;
+            // where the accumulators keep child c, dims x and x + D/2 (see BwdParams)
+            const float* at = a + ((((x % PPT) >> 1) * NT + (c >> 3)) * 32 + 4 * (2 * (x / PPT) + (x & 1)) + ((c & 7) >> 1)) * 4 + (c & 1);
+            float lo = at[0], hi = at[2];
+            if (which == 0) {
+                const float cs = __ldg(f.cosc + c * HALF + x), sn = __ldg(f.sinc + c * HALF + x), y = lo;
+                lo = y * cs + hi * sn;
+                hi = hi * cs - y * sn;
+            }
+            if (m + 1 < f.L) { const float k = (float)cnt; lo += ulo[u] / k; hi += uhi[u] / k; }
+            ulo[u] = lo; uhi[u] = hi;
+        }
+    }
+
+    const float4* a = reinterpret_cast<const float4*>(f.acc[which][0]) + blk * (D * CR / 4);
 #pragma unroll
     for (int i = 0; i < KS; ++i) {
         const int x = PPT * (g >> 1) + 2 * i + (g & 1);
@@ -430,18 +482,23 @@ __global__ void __launch_bounds__(128) bwd_fold_kernel(const __grid_constant__ F
         }
     }
     __syncwarp();
-    const int cnt = min(CR, f.N - pb * CR);
-    const float4* up = f.up[which] ? reinterpret_cast<const float4*>(f.up[which] + ((b * f.Nup + pb) * f.Hkv + h) * (int64_t)D) : nullptr;
+    const int cnt = min(CR, f.N[0] - pb * CR);
+    if (f.L > 1) {
+        const float n = (float)cnt;
+#pragma unroll
+        for (int u = 0; u < U; ++u) {
+            const int x = lane + 32 * u;
+            if (HALF < 32 && x >= HALF) break;
+            const float lo = ulo[u] / n, hi = uhi[u] / n;
+            for (int c = 0; c < cnt; ++c) { sm[warp][c][x] += lo; sm[warp][c][x + HALF] += hi; }
+        }
+        __syncwarp();
+    }
     constexpr int V4 = D / 4;
     for (int i = lane; i < cnt * V4; i += 32) {
         const int c = i / V4, col = i % V4;
-        float4 x = *reinterpret_cast<const float4*>(&sm[warp][c][4 * col]);
-        if (up) {
-            const float4 u = __ldg(up + col);
-            const float n = (float)cnt;
-            x.x += u.x / n; x.y += u.y / n; x.z += u.z / n; x.w += u.w / n;
-        }
-        const int64_t row = ((b * f.N + pb * CR + c) * f.Hkv + h) * (int64_t)D + 4 * col;
+        const float4 x = *reinterpret_cast<const float4*>(&sm[warp][c][4 * col]);
+        const int64_t row = ((b * f.N[0] + pb * CR + c) * f.Hkv + h) * (int64_t)D + 4 * col;
         if (!f.typed || sizeof(TO) == 4) {
             *reinterpret_cast<float4*>(reinterpret_cast<float*>(f.out[which]) + row) = x;
         } else {
@@ -461,9 +518,7 @@ static int launch_dkv_one(const BwdParams& bp, cudaStream_t st) {
     static SmemLimit shared;
     const cudaError_t e = shared.raise((const void*)k, smem);
     if (e != cudaSuccess) return (int)e;
-    k<<<dim3((bp.cap + 3) / 4, bp.nsub), 128, smem, st>>>(bp);
-    note_launch();
-    return (int)cudaGetLastError();
+    return launch_chained(k, dim3((bp.cap + 3) / 4, bp.nsub), dim3(128), smem, st, bp);
 }
 template <typename T, int D, bool X3, int NH, int CR>
 static int launch_dkv_cr(const BwdParams& bp, cudaStream_t st) {
@@ -487,7 +542,7 @@ static int launch_dkv_d(const BwdParams& bp, cudaStream_t st) {
 }
 
 template <typename T>
-static void launch_range_t(const BwdParams& bp, void* zero, int64_t zero_bytes, cudaStream_t st) {
+static int launch_range_t(const BwdParams& bp, void* zero, int64_t zero_bytes, cudaStream_t st) {
     const AttnParams& p = bp.a;
     RangeArgs a;
     a.dO = static_cast<const uint4*>(p.dO); a.v = static_cast<const uint4*>(p.vkblk[0]);
@@ -499,27 +554,30 @@ static void launch_range_t(const BwdParams& bp, void* zero, int64_t zero_bytes, 
     const int units = p.B * p.Hkv;
     a.of_dO = blocks(a.n_dO, 148 * 8); a.of_v = blocks((int64_t)a.NBLK * a.piece, units < 148 ? 148 * 8 / units : 8);
     const unsigned grid = (unsigned)(a.of_dO + units * a.of_v);
-    if (p.K == 128) bwd_range_kernel<T, 128><<<grid, 256, 0, st>>>(a);
-    else bwd_range_kernel<T, 64><<<grid, 256, 0, st>>>(a);
+    return launch_chained(p.K == 128 ? bwd_range_kernel<T, 128> : bwd_range_kernel<T, 64>, dim3(grid), dim3(256), 0, st, a);
+}
+// Zeros, `n` 16-byte pieces (a memset node in the chain would have to end and be waited for like any launch that is not chained).
+__global__ void __launch_bounds__(256) bwd_clear_kernel(uint4* p, int64_t n) {
+    chain_enter();
+    for (int64_t i = (int64_t)blockIdx.x * 256 + threadIdx.x; i < n; i += (int64_t)gridDim.x * 256) p[i] = make_uint4(0u, 0u, 0u, 0u);
+}
+// clears whole 16-byte pieces: `bytes` rounded up
+int launch_bwd_clear(void* p, int64_t bytes, cudaStream_t st) {
+    const int64_t n = (bytes + 15) / 16, blocks = (n + 1023) / 1024;
+    return launch_chained(bwd_clear_kernel, dim3((unsigned)(blocks < 148 * 8 ? blocks : 148 * 8)), dim3(256), 0, st, static_cast<uint4*>(p), n);
 }
 // Ahead of the first pass, bp.range being zero: clears `zero_bytes` of accumulators (a multiple of 256, or none) and finds the range of
 // 16-bit operands (split ones have factors per group).
 int launch_bwd_begin(const BwdParams& bp, int dtype, void* zero, int64_t zero_bytes, cudaStream_t st) {
-    if (pack_split(dtype, bp.a.K)) return zero_bytes ? (int)cudaMemsetAsync(zero, 0, (size_t)zero_bytes, st) : 0;
-    if (dtype == HTREE_BF16) launch_range_t<__nv_bfloat16>(bp, zero, zero_bytes, st);
-    else launch_range_t<__half>(bp, zero, zero_bytes, st);
-    note_launch();
-    return (int)cudaGetLastError();
+    if (pack_split(dtype, bp.a.K)) return zero_bytes ? launch_bwd_clear(zero, zero_bytes, st) : 0;
+    return dtype == HTREE_BF16 ? launch_range_t<__nv_bfloat16>(bp, zero, zero_bytes, st) : launch_range_t<__half>(bp, zero, zero_bytes, st);
 }
 
 int launch_bwd_dkv(const BwdParams& bp, int dtype, cudaStream_t st) {
-    bwd_scan_kernel<<<bp.nsub, 1024, 0, st>>>(bp);
-    note_launch();
-    if (bp.PK > 1) bwd_fill_many_kernel<<<dim3((bp.ng + 7) / 8, bp.nsub), 256, 0, st>>>(bp);
-    else bwd_fill_kernel<<<dim3((bp.subq + 7) / 8, bp.nsub), 256, 0, st>>>(bp);
-    note_launch();
-    const cudaError_t e = cudaGetLastError();
-    if (e != cudaSuccess) return (int)e;
+    int rc = launch_chained(bwd_scan_kernel, dim3(bp.nsub), dim3(1024), 0, st, bp);
+    if (rc == 0) rc = bp.PK > 1 ? launch_chained(bwd_fill_many_kernel, dim3((bp.ng + 7) / 8, bp.nsub), dim3(256), 0, st, bp)
+                                : launch_chained(bwd_fill_kernel, dim3((bp.subq + 7) / 8, bp.nsub), dim3(256), 0, st, bp);
+    if (rc) return rc;
     switch (dtype) {
         case HTREE_F32: return launch_dkv_d<float>(bp, st);
         case HTREE_BF16: return launch_dkv_d<__nv_bfloat16>(bp, st);
@@ -527,40 +585,24 @@ int launch_bwd_dkv(const BwdParams& bp, int dtype, cudaStream_t st) {
     }
 }
 
-template <typename TO>
-static void launch_fold_t(const FoldArgs& f, int D, int CR, cudaStream_t st) {
-    const dim3 grid((unsigned)((f.total + 3) / 4), 2);
-    if (CR == 16) {
-        if (D == 128) bwd_fold_kernel<TO, 128, 16><<<grid, 128, 0, st>>>(f);
-        else if (D == 64) bwd_fold_kernel<TO, 64, 16><<<grid, 128, 0, st>>>(f);
-        else bwd_fold_kernel<TO, 32, 16><<<grid, 128, 0, st>>>(f);
-    } else {
-        if (D == 128) bwd_fold_kernel<TO, 128, 8><<<grid, 128, 0, st>>>(f);
-        else if (D == 64) bwd_fold_kernel<TO, 64, 8><<<grid, 128, 0, st>>>(f);
-        else bwd_fold_kernel<TO, 32, 8><<<grid, 128, 0, st>>>(f);
-    }
+template <typename TO, int CR>
+static int launch_fold_t(const FoldArgs& f, int D, cudaStream_t st) {
+    return launch_chained(D == 128 ? bwd_fold_kernel<TO, 128, CR> : D == 64 ? bwd_fold_kernel<TO, 64, CR> : bwd_fold_kernel<TO, 32, CR>,
+                          dim3((unsigned)((f.total + 3) / 4), 2), dim3(128), 0, st, f);
 }
 
-// gk[l], gv[l]: rows of level l in fp32 (l >= 1: scratch); level 0 goes to dk, dv in fp32 or, typed, the storage type.
-int launch_bwd_fold(const BwdParams& bp, int dtype, float* const* gk, float* const* gv, void* dk, void* dv, bool typed, cudaStream_t st) {
+// dk, dv in fp32 or, typed, the storage type.
+int launch_bwd_fold(const BwdParams& bp, int dtype, void* dk, void* dv, bool typed, cudaStream_t st) {
     const AttnParams& p = bp.a;
-    for (int l = p.L - 1; l >= 0; --l) {
-        FoldArgs f;
-        f.acc[0] = bp.acck[l]; f.acc[1] = bp.accv[l];
-        f.up[0] = l + 1 < p.L ? gk[l + 1] : nullptr; f.up[1] = l + 1 < p.L ? gv[l + 1] : nullptr;
-        f.out[0] = l ? (void*)gk[l] : dk; f.out[1] = l ? (void*)gv[l] : dv;
-        f.cosc = p.cosc; f.sinc = p.sinc;
-        f.N = p.ln[l]; f.Nup = l + 1 < p.L ? p.ln[l + 1] : 0; f.NBLK = (p.ln[l] + p.CR - 1) / p.CR; f.Hkv = p.Hkv;
-        f.total = (int64_t)p.B * f.NBLK * p.Hkv;
-        f.typed = l == 0 && typed;
-        if (dtype == HTREE_BF16) launch_fold_t<__nv_bfloat16>(f, p.K, p.CR, st);
-        else if (dtype == HTREE_F16) launch_fold_t<__half>(f, p.K, p.CR, st);
-        else launch_fold_t<float>(f, p.K, p.CR, st);
-        note_launch();
-        const cudaError_t e = cudaGetLastError();
-        if (e != cudaSuccess) return (int)e;
-    }
-    return 0;
+    FoldArgs f;
+    for (int l = 0; l < p.L; ++l) { f.acc[0][l] = bp.acck[l]; f.acc[1][l] = bp.accv[l]; f.N[l] = p.ln[l]; }
+    f.out[0] = dk; f.out[1] = dv;
+    f.cosc = p.cosc; f.sinc = p.sinc;
+    f.L = p.L; f.Hkv = p.Hkv; f.typed = typed;
+    f.total = (int64_t)p.B * ((p.ln[0] + p.CR - 1) / p.CR) * p.Hkv;
+    if (dtype == HTREE_BF16) return p.CR == 16 ? launch_fold_t<__nv_bfloat16, 16>(f, p.K, st) : launch_fold_t<__nv_bfloat16, 8>(f, p.K, st);
+    if (dtype == HTREE_F16) return p.CR == 16 ? launch_fold_t<__half, 16>(f, p.K, st) : launch_fold_t<__half, 8>(f, p.K, st);
+    return p.CR == 16 ? launch_fold_t<float, 16>(f, p.K, st) : launch_fold_t<float, 8>(f, p.K, st);
 }
 
 }  // namespace htree

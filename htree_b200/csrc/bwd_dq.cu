@@ -29,6 +29,7 @@ constexpr int dq_min_blocks() { return D == 32 && NH == 1 ? 4 : (D == 128 && (X3
 // take it however many there are, so that dq does not depend on that; elsewhere rotating the keys is 4% faster.
 template <typename T, int D, bool X3, int NH, int CR, int PK, bool SUMS>
 __global__ void __launch_bounds__(dq_warps<D, X3, NH>() * 32, dq_min_blocks<D, X3, NH>()) bwd_dq_kernel(const __grid_constant__ BwdParams bp) {
+    chain_enter();
     static_assert(PK == 1 || (NH == 1 && CR == 16 && (X3 || SUMS)), "several queries share a warp's 8 columns");
     using C = TForm<D, X3, CR, PK>;
     using QC = Cols<PK>;
@@ -593,9 +594,7 @@ static int launch_dq_warps(const BwdParams& bp, cudaStream_t st) {
     static SmemLimit shared;
     const cudaError_t e = shared.raise((const void*)k, W * per_warp);
     if (e != cudaSuccess) return (int)e;
-    k<<<dim3((bp.ng + W - 1) / W, bp.nsub), W * 32, W * per_warp, st>>>(bp);
-    note_launch();
-    return (int)cudaGetLastError();
+    return launch_chained(k, dim3((bp.ng + W - 1) / W, bp.nsub), dim3(W * 32), W * per_warp, st, bp);
 }
 template <typename T, int D, bool X3, int NH, int CR>
 static int launch_dq_cr(const BwdParams& bp, cudaStream_t st) {

@@ -71,7 +71,8 @@ __device__ __forceinline__ float ds_scale(uint32_t dO_l1, uint32_t v) {
 int launch_bwd_begin(const BwdParams& bp, int dtype, void* zero, int64_t zero_bytes, cudaStream_t st);
 int launch_bwd_dq(const BwdParams& bp, int dtype, cudaStream_t st);
 int launch_bwd_dkv(const BwdParams& bp, int dtype, cudaStream_t st);
-int launch_bwd_fold(const BwdParams& bp, int dtype, float* const* gk, float* const* gv, void* dk, void* dv, bool typed, cudaStream_t st);
+int launch_bwd_fold(const BwdParams& bp, int dtype, void* dk, void* dv, bool typed, cudaStream_t st);
+int launch_bwd_clear(void* p, int64_t bytes, cudaStream_t st);
 
 template <int D, bool X3, int NH, int CR>
 struct BForm {

@@ -122,6 +122,26 @@ __device__ __forceinline__ int block_scan_flag(bool f, int* wtot, int* total) {
 
 void note_launch(int n = 1);   // diagnostic launch counter (api.cu)
 
+// The operator's launches depend on one another in a chain, and the small ones are as long as the gap between two of them.  A chained
+// launch may be set up while its predecessor still runs (programmatic dependent launch): its first act is to wait until that one has
+// ended and its writes are visible, the second to let the next launch be set up.  Everything behind chain_enter() is ordered as by the
+// stream.  (A step of 1000 positions 118 -> 103 us, a decode call 76 -> 69 us.)
+__device__ __forceinline__ void chain_wait() { asm volatile("griddepcontrol.wait;\n" ::: "memory"); }
+__device__ __forceinline__ void chain_next() { asm volatile("griddepcontrol.launch_dependents;\n" ::: "memory"); }
+__device__ __forceinline__ void chain_enter() { chain_wait(); chain_next(); }
+template <typename... P>
+int launch_chained(void (*kernel)(P...), dim3 grid, dim3 block, size_t smem, cudaStream_t st, const P&... args) {
+    cudaLaunchAttribute at;
+    at.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    at.val.programmaticStreamSerializationAllowed = 1;
+    cudaLaunchConfig_t cfg{};
+    cfg.gridDim = grid; cfg.blockDim = block; cfg.dynamicSmemBytes = smem; cfg.stream = st;
+    cfg.attrs = &at; cfg.numAttrs = 1;
+    const cudaError_t e = cudaLaunchKernelEx(&cfg, kernel, args...);
+    note_launch();
+    return (int)e;
+}
+
 // Parent lists: int32 with -1 for "none" (the reference's layout), or uint16 with 0xFFFF under HTREE_PARENTS_U16.
 __device__ __forceinline__ int load_parent(const AttnParams& p, int l, int64_t idx) {
     if (p.flags & HTREE_PARENTS_U16) {

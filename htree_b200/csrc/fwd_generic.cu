@@ -116,6 +116,7 @@ __device__ __forceinline__ int count_ge(const uint32_t* key, int nc, uint32_t th
 // candidates tile by tile with an online softmax, instead of holding every score of the level.
 template <typename T, int GP, bool TILED>
 __global__ void __launch_bounds__(NT) fwd_generic_kernel(const __grid_constant__ AttnParams p) {
+    chain_enter();
     extern __shared__ __align__(16) unsigned char smem_raw[];
     const int K = p.K, V = p.V, CR = p.CR, TK = p.TK, G = p.G, L = p.L, half = K >> 1;
     const int GPAD = (G + GP - 1) / GP * GP, RS = GPAD + 4, maxc = TK * CR;
@@ -501,15 +502,10 @@ __global__ void __launch_bounds__(NT) fwd_generic_kernel(const __grid_constant__
 template <typename T, bool TILED>
 static int launch_tt(const AttnParams& p, size_t smem, int GP, cudaStream_t st) {
     dim3 grid(p.Tq, p.B * p.Hkv);
-    cudaError_t e;
-#define HT_LAUNCH(GPV)                                                                                                     \
-    e = cudaFuncSetAttribute(fwd_generic_kernel<T, GPV, TILED>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);  \
-    if (e != cudaSuccess) return (int)e;                                                                                   \
-    fwd_generic_kernel<T, GPV, TILED><<<grid, NT, smem, st>>>(p);
-    if (GP == 4) { HT_LAUNCH(4) } else if (GP == 8) { HT_LAUNCH(8) } else { HT_LAUNCH(16) }
-#undef HT_LAUNCH
-    note_launch();
-    return (int)cudaGetLastError();
+    auto* k = GP == 4 ? fwd_generic_kernel<T, 4, TILED> : GP == 8 ? fwd_generic_kernel<T, 8, TILED> : fwd_generic_kernel<T, 16, TILED>;
+    const cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    if (e != cudaSuccess) return (int)e;
+    return launch_chained(k, grid, dim3(NT), smem, st, p);
 }
 
 template <typename T>

@@ -80,6 +80,7 @@ __device__ __forceinline__ void to_half_words(const float (&x)[N], uint32_t (&hi
 
 template <typename T, int D, bool X3, int CR>
 __global__ void __launch_bounds__(128) pack_blocks_kernel(const __grid_constant__ PackArgs a) {
+    chain_enter();
     using C = TForm<D, X3, CR>;
     constexpr int HALF = C::HALF, PPT = C::PPT, KS = C::KS, VB = C::VB;
     int64_t blk = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
@@ -284,27 +285,21 @@ bool pack_supported(int dtype, int K, int V, int CR) {
 bool pack_split(int dtype, int D) { return dtype == HTREE_F32 || D == 32; }
 
 template <typename T, int D, bool X3>
-static void launch_pack_t(const PackArgs& a, int CR, cudaStream_t st) {
-    const unsigned grid = (unsigned)((a.total + 3) / 4);
-    if (CR == 16) pack_blocks_kernel<T, D, X3, 16><<<grid, 128, 0, st>>>(a);
-    else pack_blocks_kernel<T, D, X3, 8><<<grid, 128, 0, st>>>(a);
+static int launch_pack_t(const PackArgs& a, int CR, cudaStream_t st) {
+    return launch_chained(CR == 16 ? pack_blocks_kernel<T, D, X3, 16> : pack_blocks_kernel<T, D, X3, 8>, dim3((unsigned)((a.total + 3) / 4)), dim3(128), 0, st, a);
 }
 template <typename T>
-static void launch_pack_d(const PackArgs& a, int D, int CR, cudaStream_t st) {
+static int launch_pack_d(const PackArgs& a, int D, int CR, cudaStream_t st) {
     constexpr bool F32 = std::is_same<T, float>::value;
-    if (D == 128) launch_pack_t<T, 128, F32>(a, CR, st);
-    else if (D == 64) launch_pack_t<T, 64, F32>(a, CR, st);
-    else launch_pack_t<T, 32, true>(a, CR, st);
+    return D == 128 ? launch_pack_t<T, 128, F32>(a, CR, st) : D == 64 ? launch_pack_t<T, 64, F32>(a, CR, st) : launch_pack_t<T, 32, true>(a, CR, st);
 }
 
 static int launch_pack(const PackArgs& a, const HtreeShape& s, cudaStream_t st) {
     switch (s.dtype) {
-        case HTREE_F32: launch_pack_d<float>(a, s.K, s.compression_rate, st); break;
-        case HTREE_BF16: launch_pack_d<__nv_bfloat16>(a, s.K, s.compression_rate, st); break;
-        default: launch_pack_d<__half>(a, s.K, s.compression_rate, st); break;
+        case HTREE_F32: return launch_pack_d<float>(a, s.K, s.compression_rate, st);
+        case HTREE_BF16: return launch_pack_d<__nv_bfloat16>(a, s.K, s.compression_rate, st);
+        default: return launch_pack_d<__half>(a, s.K, s.compression_rate, st);
     }
-    note_launch();
-    return (int)cudaGetLastError();
 }
 
 static PackArgs pack_args(const HtreeShape& s, int N, const void* k, const void* v, void* blk, const float* cosc, const float* sinc) {

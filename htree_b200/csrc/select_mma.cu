@@ -127,6 +127,7 @@ __device__ __forceinline__ void select_scores(uint32_t slot, int lane, const flo
 template <typename T, int D, bool X3, int NH, int CR, bool SPLIT>
 __global__ void __launch_bounds__(SPLIT ? kSelSplitWarps * 32 : 128, SPLIT ? 2 : sel_min_blocks<D, X3, NH>())
 select_mma_kernel(const __grid_constant__ AttnParams p) {
+    chain_enter();
     using SF = SelForm<D, X3, CR>;
     using C = TForm<D, X3, CR>;
     constexpr int PPC = SF::PPC, NSTG = SF::NSTG, HALF = D / 2, PPT = HALF / 4;
@@ -407,9 +408,7 @@ static int launch_select_cr(const AttnParams& in, cudaStream_t st) {
         static SmemLimit shared;
         const cudaError_t e = shared.raise((const void*)k, split_smem);
         if (e != cudaSuccess) return (int)e;
-        k<<<dim3(p.Tq, p.B * p.Hkv), kSelSplitWarps * 32, split_smem, st>>>(p);
-        note_launch();
-        return (int)cudaGetLastError();
+        return launch_chained(k, dim3(p.Tq, p.B * p.Hkv), dim3(kSelSplitWarps * 32), split_smem, st, p);
     }
     const size_t per_warp = Ring::kBytes + scratch;
     constexpr int max_warps = 4 * sel_min_blocks<D, X3, NH>();
@@ -424,9 +423,7 @@ static int launch_select_cr(const AttnParams& in, cudaStream_t st) {
     static SmemLimit shared;
     const cudaError_t e = shared.raise((const void*)k, W * per_warp);
     if (e != cudaSuccess) return (int)e;
-    k<<<dim3((p.Tq + W - 1) / W, p.B * p.Hkv), W * 32, W * per_warp, st>>>(p);
-    note_launch();
-    return (int)cudaGetLastError();
+    return launch_chained(k, dim3((p.Tq + W - 1) / W, p.B * p.Hkv), dim3(W * 32), W * per_warp, st, p);
 }
 
 template <typename T, int D, bool X3>

@@ -65,6 +65,7 @@ struct BuildArgs {
 // blockIdx.y = 0 pools K, 1 pools V.  UNR = children loaded per unrolled batch.
 template <typename T, int UNR>
 __global__ void __launch_bounds__(256) tree_build_kernel(const __grid_constant__ BuildArgs a) {
+    chain_enter();
     constexpr int VN = Vec16<T>::N;
     const int which = blockIdx.y;
     const int64_t idx = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
@@ -115,11 +116,8 @@ static int build_levels(const HtreeShape& s, int L, const int32_t* ln, void* con
 #ifndef HTREE_BUILD_UNR
 #define HTREE_BUILD_UNR 8   // children loaded per batch: 8 keeps 80 registers and 3 blocks per SM (82 % of HBM peak vs 51 % with 16)
 #endif
-        if (s.compression_rate >= 16) tree_build_kernel<T, HTREE_BUILD_UNR><<<grid, 256, 0, st>>>(a);
-        else tree_build_kernel<T, 8><<<grid, 256, 0, st>>>(a);
-        note_launch();
-        cudaError_t e = cudaGetLastError();
-        if (e != cudaSuccess) return (int)e;
+        const int rc = launch_chained(s.compression_rate >= 16 ? tree_build_kernel<T, HTREE_BUILD_UNR> : tree_build_kernel<T, 8>, grid, dim3(256), 0, st, a);
+        if (rc) return rc;
     }
     return 0;
 }

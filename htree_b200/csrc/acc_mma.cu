@@ -29,11 +29,15 @@ constexpr int acc_stages() { return acc_single<D, X3, NH, CR>() ? 1 : D * (X3 ? 
 constexpr int kAccWarps = 4, kAccSplitWarps = 8;
 template <int D, bool X3, int NH, int CR>
 constexpr int acc_min_blocks() { return (X3 && D == 128) ? 2 : D == 128 ? (NH == 1 ? 4 : 3) : (X3 && D == 64 && NH == 2) ? 3 : 4; }
+// Slots of the warps that share a query: two of 8 KB, three of less, so that two blocks of 64- and 32-wide heads still share an SM (a third
+// slot of 8 KB gave nothing: 28.4 against 29.2 us).
+template <int D, bool X3>
+constexpr int acc_split_stages() { return D * (X3 ? 2 : 1) >= 256 ? 1 : D * (X3 ? 2 : 1) >= 128 ? 2 : 3; }
 // A warp's rings: keys with their table rows, and values.
-template <int D, bool X3, int NH, int CR, int PK = 1>
+template <int D, bool X3, int NH, int CR, int PK = 1, bool SPLIT = false>
 struct AccRings {
     // (lists of several queries beside three slots would cost warps: 12000 positions, 512 nodes per layer 3.60 -> 3.32 ms with two)
-    static constexpr int NSTG = PK > 1 && acc_stages<D, X3, NH, CR>() > 2 ? 2 : acc_stages<D, X3, NH, CR>();
+    static constexpr int NSTG = SPLIT ? acc_split_stages<D, X3>() : PK > 1 && acc_stages<D, X3, NH, CR>() > 2 ? 2 : acc_stages<D, X3, NH, CR>();
     using C = TForm<D, X3, CR, PK>;
     using Keys = WarpRing<NSTG, C::KSLOT + (NSTG > 1 ? C::VSLOT : 0)>;      // (of several stages: with the values)
     using Values = WarpRing<1, C::VSLOT>;
@@ -50,32 +54,38 @@ acc_mma_kernel(const __grid_constant__ AttnParams p) {
     using FT = typename std::conditional<X3, __half, T>::type;        // type of the values and probabilities
     using F = Frag<FT>;
     constexpr int MT = C::MT, PPC = C::PPC;
-    using Ring = AccRings<D, X3, NH, CR, PK>;
+    using Ring = AccRings<D, X3, NH, CR, PK, SPLIT>;
     constexpr int NSTG = Ring::NSTG, GP = QC::GP;
     extern __shared__ __align__(128) unsigned char smem_raw[];
 
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, g = lane >> 2, r = lane & 3;
     const int W = SPLIT ? kAccSplitWarps : blockDim.x >> 5;
-    const int from_end = SPLIT ? (int)blockIdx.x : (int)(blockIdx.x * W + warp);
+    const int CL = SPLIT ? (int)cluster_blocks() : 1, rank = SPLIT ? (int)cluster_rank() : 0;       // the blocks that share a query
+    const int from_end = SPLIT ? (int)blockIdx.x / CL : (int)(blockIdx.x * W + warp);
     const int npack = PK == 1 ? p.Tq : (p.Tq + PK - 1) / PK;
     if (!SPLIT && from_end >= npack) return;
     const int tl = (npack - 1 - from_end) * PK;                       // the longest walks first: they would be the tail of a short call
     const int b = blockIdx.y / p.Hkv, hk = blockIdx.y % p.Hkv;
     const int G = p.G, TK = p.TK, L = p.L;
-    const int first = SPLIT ? warp : 0, step = SPLIT ? W : 1;         // this warp's chunks of every level
+    const int first = SPLIT ? rank * W + warp : 0, step = SPLIT ? CL * W : 1;      // this warp's chunks of every level
 
     // per warp: ring, parent list, kept-candidate bits
     const WalkLayout lay = walk_layout(p, CR);
-    const size_t per_warp = walk_warp_bytes<Ring, PK>(lay);
+    const size_t per_warp = SPLIT ? Ring::kBytes : walk_warp_bytes<Ring, PK>(lay);       // (SPLIT: one list for all)
     unsigned char* wbase = smem_raw + warp * per_warp;
+    unsigned char* lists = SPLIT ? smem_raw + W * per_warp : wbase + Ring::kBytes;
     typename Ring::Keys kring;
     typename Ring::Values vring;
     kring.init(wbase);
     vring.init(wbase + Ring::Keys::kBytes);
-    auto list_of = [&](int j) { return ParentList{wbase + Ring::kBytes + j * lay.list, lay.narrow}; };        // query tl + j
-    auto bits_of = [&](int j) { return reinterpret_cast<uint32_t*>(wbase + Ring::kBytes + PK * lay.list + j * lay.bits); };
+    auto list_of = [&](int j) { return ParentList{lists + j * lay.list, lay.narrow}; };        // query tl + j
+    auto bits_of = [&](int j) { return reinterpret_cast<uint32_t*>(lists + PK * lay.list + j * lay.bits); };
     const ParentList par = list_of(0);
     uint32_t* selw = bits_of(0);
+    float* exchange = reinterpret_cast<float*>(lists + walk_lists_bytes(lay));                  // SPLIT: [W][3][16]
+    uint32_t* votes = reinterpret_cast<uint32_t*>(exchange + 48 * kAccSplitWarps);              // SPLIT: [2][blocks], of even and odd rounds
+    int round = 0;
+    if (CL > 1) cluster_sync();                                       // every block has started: its shared memory may be written
 
     const int64_t hbase = ((int64_t)b * p.Tq + tl) * p.H + (int64_t)hk * G;
     const int64_t qidx = ((int64_t)b * p.Tq + tl) * p.Hkv + hk;
@@ -107,9 +117,10 @@ acc_mma_kernel(const __grid_constant__ AttnParams p) {
 #pragma unroll
         for (int e = 0; e < 2; ++e) { m_run[h][e] = m_true[h][e] = kNone; m_run2[h][e] = kNone * kLog2e; s_run[h][e] = 0.f; }
 
+    auto group_sync = [&]() { if constexpr (SPLIT) __syncthreads(); else __syncwarp(); };       // of the threads that share a list
     for (int l = L - 1; l >= 0; --l) {
         const int Nl = p.ln[l];
-        __syncwarp();
+        group_sync();
         const int nblk = (Nl + CR - 1) / CR;
         int np, rp, nchunk = 0;
         UnionWalk<PK> walk;
@@ -120,7 +131,7 @@ acc_mma_kernel(const __grid_constant__ AttnParams p) {
             if (l > 0 && nc <= TK) continue;                          // every candidate is kept: nothing to accumulate
             if (np <= 0) continue;
             nchunk = (np + PPC - 1) / PPC;
-            __syncwarp();
+            group_sync();                                             // (SPLIT: every warp has written the same list)
         } else {
             np = rp = 0;                                              // of query lane mod PK
             for (int j = 0; j < PK; ++j) {
@@ -132,7 +143,7 @@ acc_mma_kernel(const __grid_constant__ AttnParams p) {
                     uint32_t* bits = bits_of(j);
                     for (int i = lane; i < (right + 32) / 32; i += 32) bits[i] = 0u;
                     __syncwarp();
-                    mark_kept(p, l, (qidx + (int64_t)j * p.Hkv) * TK, list_of(j), n, CR, bits, lane);
+                    mark_kept<32>(p, l, (qidx + (int64_t)j * p.Hkv) * TK, list_of(j), n, CR, bits, lane);
                 }
                 if (lane % PK == j) { np = n; rp = right; }
             }
@@ -190,9 +201,12 @@ acc_mma_kernel(const __grid_constant__ AttnParams p) {
             if constexpr (NSTG == 1) vring.commit(); else kring.commit();
         }
         if (PK == 1 && l > 0) {                                       // found while the first blocks are on their way
-            for (int i = lane; i < (rp + 32) / 32; i += 32) selw[i] = 0u;
-            __syncwarp();
-            mark_kept(p, l, qidx * TK, par, np, CR, selw, lane);
+            constexpr int NT = SPLIT ? kAccSplitWarps * 32 : 32;
+            const int me = SPLIT ? (int)threadIdx.x : lane;
+            for (int i = me; i < (rp + 32) / 32; i += NT) selw[i] = 0u;
+            group_sync();
+            mark_kept<NT>(p, l, qidx * TK, par, np, CR, selw, me);
+            if constexpr (SPLIT) __syncthreads();
         }
         auto chunk_mask = [&](int c) {                                // the chunk's candidates that accumulate
             uint32_t mask = 0xffffu;
@@ -309,8 +323,16 @@ acc_mma_kernel(const __grid_constant__ AttnParams p) {
             bool moved;
             if constexpr (SPLIT) {
                 moved = __syncthreads_or(top > kMove);
+                if (CL > 1) {
+                    uint32_t* v = votes + 8 * (round & 1);
+                    if ((int)threadIdx.x < CL) st_cluster(cluster_addr(v + rank, threadIdx.x), moved);
+                    cluster_sync();
+                    moved = false;
+                    for (int i = 0; i < CL; ++i) moved |= v[i] != 0u;
+                    ++round;
+                }
                 if (moved) {
-                    float* st = reinterpret_cast<float*>(smem_raw + W * per_warp);
+                    float* st = exchange;
 #pragma unroll
                     for (int h = 0; h < NH; ++h)
 #pragma unroll
@@ -319,31 +341,35 @@ acc_mma_kernel(const __grid_constant__ AttnParams p) {
                             if (g == 0) st[warp * 48 + 8 * h + 2 * r + e] = m;
                             after[h][e] = m_run[h][e];
                         }
-                    __syncthreads();                                  // (the vote of the next round orders these reads before its writes)
-                    float m[kAccSplitWarps][NH][2], mine[NH][2];
+                    if (CL > 1) cluster_sync(); else __syncthreads();   // (the vote of the next round orders these reads before its writes)
+                    float mine[NH][2];
+                    for (int blk = 0; blk < CL; ++blk) {
+                        const uint32_t from = cluster_addr(st + 2 * r, blk);
+                        float m[kAccSplitWarps][NH][2];
 #pragma unroll
-                    for (int w = 0; w < kAccSplitWarps; ++w)
+                        for (int w = 0; w < kAccSplitWarps; ++w)
 #pragma unroll
-                        for (int h = 0; h < NH; ++h) {
-                            const float2 x = *reinterpret_cast<const float2*>(st + w * 48 + 8 * h + 2 * r);
-                            m[w][h][0] = x.x; m[w][h][1] = x.y;
-                        }
-#pragma unroll
-                    for (int w = 0; w < kAccSplitWarps; ++w) {
-                        float t = -INFINITY;
-#pragma unroll
-                        for (int h = 0; h < NH; ++h)
-#pragma unroll
-                            for (int e = 0; e < 2; ++e)
-                                t = fmaxf(t, X3 ? m[w][h][e] - after[h][e] : fmaf(m[w][h][e], kLog2e, -(after[h][e] * kLog2e)));
-                        const bool move = __any_sync(0xffffffffu, t > kMove);
-#pragma unroll
-                        for (int h = 0; h < NH; ++h)
-#pragma unroll
-                            for (int e = 0; e < 2; ++e) {
-                                if (move) after[h][e] = fmaxf(after[h][e], m[w][h][e]);
-                                if (w == warp) mine[h][e] = after[h][e];
+                            for (int h = 0; h < NH; ++h) {
+                                const float2 x = ld_cluster2(from + 4 * (w * 48 + 8 * h));
+                                m[w][h][0] = x.x; m[w][h][1] = x.y;
                             }
+#pragma unroll
+                        for (int w = 0; w < kAccSplitWarps; ++w) {
+                            float t = -INFINITY;
+#pragma unroll
+                            for (int h = 0; h < NH; ++h)
+#pragma unroll
+                                for (int e = 0; e < 2; ++e)
+                                    t = fmaxf(t, X3 ? m[w][h][e] - after[h][e] : fmaf(m[w][h][e], kLog2e, -(after[h][e] * kLog2e)));
+                            const bool move = __any_sync(0xffffffffu, t > kMove);
+#pragma unroll
+                            for (int h = 0; h < NH; ++h)
+#pragma unroll
+                                for (int e = 0; e < 2; ++e) {
+                                    if (move) after[h][e] = fmaxf(after[h][e], m[w][h][e]);
+                                    if (w == warp && blk == rank) mine[h][e] = after[h][e];
+                                }
+                        }
                     }
                     bool later = false;                               // does a later chunk of the round move it again?
 #pragma unroll
@@ -449,11 +475,13 @@ acc_mma_kernel(const __grid_constant__ AttnParams p) {
                 m_true[h][e] = fmaxf(m_true[h][e], __shfl_xor_sync(0xffffffffu, m_true[h][e], o));
             }
     if constexpr (SPLIT) {
-        // merge the warps' partial states (few queries: a group's chunks are spread over the warps of a block)
+        // Merge the warps' partial states (few queries: a group's chunks are spread over the warps of a block or of several).  All
+        // followed the same references: their sums add up as they are.
         kring.idle();
-        __syncthreads();                                              // all rings are idle: their memory is free
-        float* st = reinterpret_cast<float*>(smem_raw + W * per_warp);          // [W][3][16]: m_run, m_true, s
-        float* po = reinterpret_cast<float*>(wbase);                  // this warp's O, [16 heads][D]
+        if (CL > 1) cluster_sync(); else __syncthreads();             // all rings are idle: their memory is free, and so is the exchange
+        float* st = exchange;                                         // [W][3][16]: m_run, m_true, s; the block's in [0]
+        float* po = reinterpret_cast<float*>(wbase);                  // this warp's O, [16 heads][D]; the block's in the first warp's
+        float* bo = reinterpret_cast<float*>(smem_raw);
         if (g == 0) {
 #pragma unroll
             for (int h = 0; h < NH; ++h)
@@ -463,37 +491,43 @@ acc_mma_kernel(const __grid_constant__ AttnParams p) {
                     st[(warp * 3 + 0) * 16 + head] = m_run[h][e]; st[(warp * 3 + 1) * 16 + head] = m_true[h][e]; st[(warp * 3 + 2) * 16 + head] = s_run[h][e];
                 }
         }
-        __syncthreads();
 #pragma unroll
         for (int h = 0; h < NH; ++h)
 #pragma unroll
             for (int e = 0; e < 2; ++e) {
                 const int head = 8 * h + 2 * r + e;
-                float m = kNone;
-                for (int w = 0; w < W; ++w) m = fmaxf(m, st[w * 48 + head]);
-                const float f = __expf(m_run[h][e] - m);
 #pragma unroll
                 for (int i = 0; i < MT; ++i) {
-                    po[head * D + C::VB * g + 2 * i] = O[h][i][e] * f;
-                    po[head * D + C::VB * g + 2 * i + 1] = O[h][i][2 + e] * f;
+                    po[head * D + C::VB * g + 2 * i] = O[h][i][e];
+                    po[head * D + C::VB * g + 2 * i + 1] = O[h][i][2 + e];
                 }
             }
         __syncthreads();
         for (int i = threadIdx.x; i < G * D; i += blockDim.x) {
+            float o = bo[i];
+#pragma unroll
+            for (int w = 1; w < kAccSplitWarps; ++w) o += reinterpret_cast<const float*>(smem_raw + w * per_warp)[i];
+            bo[i] = o;
+        }
+        if (threadIdx.x < 8 * NH) {
+            float mt = st[16 + threadIdx.x], s = st[32 + threadIdx.x];
+            for (int w = 1; w < W; ++w) { mt = fmaxf(mt, st[w * 48 + 16 + threadIdx.x]); s += st[w * 48 + 32 + threadIdx.x]; }
+            st[16 + threadIdx.x] = mt; st[32 + threadIdx.x] = s;
+        }
+        if (CL > 1) cluster_sync(); else __syncthreads();
+        const int part = (G * D + CL - 1) / CL;                       // this block's share of the results
+        for (int i = rank * part + (int)threadIdx.x; i < min(G * D, (rank + 1) * part); i += blockDim.x) {
             const int head = i / D;
-            float m = kNone, s = 0.f, o = 0.f;
-            for (int w = 0; w < W; ++w) m = fmaxf(m, st[w * 48 + head]);
-            for (int w = 0; w < W; ++w) {
-                s += st[w * 48 + 32 + head] * __expf(st[w * 48 + head] - m);
-                o += reinterpret_cast<const float*>(smem_raw + w * per_warp)[i];
+            float o = 0.f, s = 0.f, mt = kNone;
+            for (int c = 0; c < CL; ++c) {
+                o += ld_cluster(cluster_addr(bo + i, c));
+                s += ld_cluster(cluster_addr(st + 32 + head, c));
+                mt = fmaxf(mt, ld_cluster(cluster_addr(st + 16 + head, c)));
             }
             reinterpret_cast<T*>(p.out)[hbase * D + i] = from_f<T>(o / s);
-            if (i % D == 0) {
-                float mt = kNone;
-                for (int w = 0; w < W; ++w) mt = fmaxf(mt, st[w * 48 + 16 + head]);
-                p.gmax[hbase + head] = mt; p.gsum[hbase + head] = s * __expf(m - mt);
-            }
+            if (i % D == 0) { p.gmax[hbase + head] = mt; p.gsum[hbase + head] = s * __expf(st[head] - mt); }
         }
+        if (CL > 1) cluster_sync();                                   // nobody leaves while others read from it
     } else {
 #pragma unroll
     for (int h = 0; h < NH; ++h)
@@ -547,19 +581,23 @@ static int launch_acc_warps(const AttnParams& p, cudaStream_t st) {
 
 template <typename T, int D, bool X3, int NH, int CR>
 static int launch_acc_cr(const AttnParams& p, cudaStream_t st) {
-    const size_t per_warp = walk_warp_bytes<AccRings<D, X3, NH, CR>>(walk_layout(p, CR));
     // Few groups: one block of 8 warps per group.  Below two groups per SM the chip has room for all their warps at once, and
     // a single warp's walk over its chunks (about 1 us each) would be the whole time of the call.  Calls whose state the
     // backward reads (they keep their selections) always take one warp per group: a query's result then does not depend on
     // how many queries share the call.
     const int64_t groups = (int64_t)p.Tq * p.B * p.Hkv;
-    const size_t split_smem = kAccSplitWarps * (per_warp + 48 * sizeof(float));
+    const size_t split_smem = kAccSplitWarps * (AccRings<D, X3, NH, CR, 1, true>::kBytes + 48 * sizeof(float)) + 64 + walk_lists_bytes(walk_layout(p, CR));
     if ((p.flags & kFlagSplitOk) && groups <= 2 * 148 && split_smem <= 227 * 1024) {
         auto* k = acc_mma_kernel<T, D, X3, NH, CR, true, 1>;
         static SmemLimit shared;
         const cudaError_t e = shared.raise((const void*)k, split_smem);
         if (e != cudaSuccess) return (int)e;
-        return launch_chained(k, dim3(p.Tq, p.B * p.Hkv), dim3(kAccSplitWarps * 32), split_smem, st, p);
+        // Blocks per group: while each has an SM, and as a level has chunks for their warps.  A round of chunks ends in a barrier of the
+        // cluster, and a walk over 128 chunks was 16 rounds of one block: 4 x 1 queries against 16384 positions, 16 heads of 128, 8 blocks
+        // each: 29 -> 20 us; 5 queries of one head against 512 leaf parents: the call 118 -> 71 us.
+        int CL = 1;
+        while (CL < 8 && 2 * CL * groups <= 148 && 2 * CL * kAccSplitWarps <= (p.TK * CR + 15) / 16) CL *= 2;
+        return launch_chained_clusters(k, CL, dim3(p.Tq * CL, p.B * p.Hkv), dim3(kAccSplitWarps * 32), split_smem, st, p);
     }
     if constexpr (NH == 1 && CR == 16) {
         const int PK = queries_per_warp(CR, p.G, p.TK, (p.ln[0] + CR - 1) / CR, groups);

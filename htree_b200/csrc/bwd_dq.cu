@@ -220,7 +220,7 @@ __global__ void __launch_bounds__(dq_warps<D, X3, NH>() * 32, dq_min_blocks<D, X
                     uint32_t* bits = bits_of(j);
                     for (int i = lane; i < (right + 32) / 32; i += 32) bits[i] = 0u;
                     __syncwarp();
-                    mark_kept(p, l, (qidx + (int64_t)j * p.Hkv) * TK, list_of(j), n, CR, bits, lane);
+                    mark_kept<32>(p, l, (qidx + (int64_t)j * p.Hkv) * TK, list_of(j), n, CR, bits, lane);
                 }
                 if (lane % PK == j) { np = n; rp = right; }
             }
@@ -321,7 +321,7 @@ __global__ void __launch_bounds__(dq_warps<D, X3, NH>() * 32, dq_min_blocks<D, X
         if (PK == 1 && l > 0) {
             for (int i = lane; i < (rp + 32) / 32; i += 32) selw[i] = 0u;
             __syncwarp();
-            mark_kept(p, l, qidx * TK, par, np, CR, selw, lane);
+            mark_kept<32>(p, l, qidx * TK, par, np, CR, selw, lane);
         }
 #pragma unroll 1
         for (int c = 0; PK > 1 ? pending > 0 : c < nchunk; ++c) {

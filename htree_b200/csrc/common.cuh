@@ -125,22 +125,47 @@ void note_launch(int n = 1);   // diagnostic launch counter (api.cu)
 // The operator's launches depend on one another in a chain, and the small ones are as long as the gap between two of them.  A chained
 // launch may be set up while its predecessor still runs (programmatic dependent launch): its first act is to wait until that one has
 // ended and its writes are visible, the second to let the next launch be set up.  Everything behind chain_enter() is ordered as by the
-// stream.  (A step of 1000 positions 118 -> 103 us, a decode call 76 -> 69 us.)
+// stream.  (A decode call 76 -> 69 us, a forward of 2048 positions 117 -> 115, of one level 24.5 -> 19.7.)
 __device__ __forceinline__ void chain_wait() { asm volatile("griddepcontrol.wait;\n" ::: "memory"); }
 __device__ __forceinline__ void chain_next() { asm volatile("griddepcontrol.launch_dependents;\n" ::: "memory"); }
 __device__ __forceinline__ void chain_enter() { chain_wait(); chain_next(); }
 template <typename... P>
-int launch_chained(void (*kernel)(P...), dim3 grid, dim3 block, size_t smem, cudaStream_t st, const P&... args) {
-    cudaLaunchAttribute at;
-    at.id = cudaLaunchAttributeProgrammaticStreamSerialization;
-    at.val.programmaticStreamSerializationAllowed = 1;
+int launch_chained_clusters(void (*kernel)(P...), int cluster, dim3 grid, dim3 block, size_t smem, cudaStream_t st, const P&... args) {
+    cudaLaunchAttribute at[2];
+    at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    at[0].val.programmaticStreamSerializationAllowed = 1;
+    at[1].id = cudaLaunchAttributeClusterDimension;
+    at[1].val.clusterDim.x = cluster; at[1].val.clusterDim.y = at[1].val.clusterDim.z = 1;
     cudaLaunchConfig_t cfg{};
     cfg.gridDim = grid; cfg.blockDim = block; cfg.dynamicSmemBytes = smem; cfg.stream = st;
-    cfg.attrs = &at; cfg.numAttrs = 1;
+    cfg.attrs = at; cfg.numAttrs = cluster > 1 ? 2 : 1;
     const cudaError_t e = cudaLaunchKernelEx(&cfg, kernel, args...);
     note_launch();
     return (int)e;
 }
+template <typename... P>
+int launch_chained(void (*kernel)(P...), dim3 grid, dim3 block, size_t smem, cudaStream_t st, const P&... args) {
+    return launch_chained_clusters(kernel, 1, grid, block, smem, st, args...);
+}
+
+// Blocks of a cluster (along x) that work on one query: rank, barrier and the other blocks' shared memory.
+__device__ __forceinline__ uint32_t cluster_rank() { uint32_t x; asm volatile("mov.u32 %0, %%cluster_ctarank;" : "=r"(x)); return x; }
+__device__ __forceinline__ uint32_t cluster_blocks() { uint32_t x; asm volatile("mov.u32 %0, %%cluster_nctarank;" : "=r"(x)); return x; }
+__device__ __forceinline__ void cluster_sync() {
+    asm volatile("barrier.cluster.arrive.release.aligned;\nbarrier.cluster.wait.acquire.aligned;\n" ::: "memory");
+}
+__device__ __forceinline__ uint32_t cluster_addr(const void* p, uint32_t rank) {         // p, in this block's shared memory, of block `rank`
+    uint32_t a;
+    asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(a) : "r"((uint32_t)__cvta_generic_to_shared(p)), "r"(rank));
+    return a;
+}
+__device__ __forceinline__ float ld_cluster(uint32_t a) { float x; asm volatile("ld.shared::cluster.f32 %0, [%1];" : "=f"(x) : "r"(a) : "memory"); return x; }
+__device__ __forceinline__ float2 ld_cluster2(uint32_t a) {
+    float2 x;
+    asm volatile("ld.shared::cluster.v2.f32 {%0,%1}, [%2];" : "=f"(x.x), "=f"(x.y) : "r"(a) : "memory");
+    return x;
+}
+__device__ __forceinline__ void st_cluster(uint32_t a, uint32_t x) { asm volatile("st.shared::cluster.b32 [%0], %1;" ::"r"(a), "r"(x) : "memory"); }
 
 // Parent lists: int32 with -1 for "none" (the reference's layout), or uint16 with 0xFFFF under HTREE_PARENTS_U16.
 __device__ __forceinline__ int load_parent(const AttnParams& p, int l, int64_t idx) {

@@ -2,7 +2,7 @@
 // selecting half of htree_select_accumulate_gqa_kernel (src/parallel.py:537-867, 1167-1399).  Products, chunks and operand blocks
 // of tform.cuh; writes the parent list that each level consumes.
 //
-// One warp per (batch, query position, KV head) group; with SPLIT the 8 warps of a block share a group's chunks.  A candidate's
+// One warp per (batch, query position, KV head) group; with SPLIT the 8 warps of a block, or of up to 8 blocks, share a group's chunks.  A candidate's
 // importance does not depend on which: every chunk is evaluated alike (the query rotated in fp32 and rounded once to half per
 // parent, two accumulation chains, the chunk's own maximum as reference, heads summed in one fixed tree) and the search is exact.
 //
@@ -136,13 +136,15 @@ select_mma_kernel(const __grid_constant__ AttnParams p) {
 
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, g = lane >> 2, r = lane & 3;
     const int W = blockDim.x >> 5;
-    const int at = SPLIT ? (int)blockIdx.x : (int)(blockIdx.x * W + warp);
+    // SPLIT: the blocks of a cluster score a group's chunks; the first of them finds the Top-K and hands the list to the others
+    const int CL = SPLIT ? (int)cluster_blocks() : 1, rank = SPLIT ? (int)cluster_rank() : 0;
+    const int at = SPLIT ? (int)blockIdx.x / CL : (int)(blockIdx.x * W + warp);
     if (!SPLIT && at >= p.Tq) return;
     const int tl = p.Tq <= kSelReverse ? p.Tq - 1 - at : at;
     const int t = p.t0 + tl;
     const int b = blockIdx.y / p.Hkv, hk = blockIdx.y % p.Hkv;
     const int G = p.G, TK = p.TK, L = p.L, maxc = p.sel_maxc;
-    const int first = SPLIT ? warp : 0, step = SPLIT ? W : 1;
+    const int first = SPLIT ? rank * W + warp : 0, step = SPLIT ? CL * W : 1;
     const int tid = SPLIT ? (int)threadIdx.x : lane, nthr = SPLIT ? kSelSplitWarps * 32 : 32;   // the threads that share a group
     auto sync = [&]() { if constexpr (SPLIT) __syncthreads(); else __syncwarp(); };
 
@@ -158,6 +160,7 @@ select_mma_kernel(const __grid_constant__ AttnParams p) {
     int* cnt = reinterpret_cast<int*>(nxt + TK);       // SPLIT: three rotating counters
     int* wtot = cnt + 4;                               // SPLIT: one per warp
     if (SPLIT && threadIdx.x < 4) cnt[threadIdx.x] = 0;
+    if (CL > 1) cluster_sync();                        // every block has started: its shared memory may be written
 
     const int64_t hbase = ((int64_t)b * p.Tq + tl) * p.H + (int64_t)hk * G;
     const int64_t qidx = ((int64_t)b * p.Tq + tl) * p.Hkv + hk;
@@ -183,7 +186,7 @@ select_mma_kernel(const __grid_constant__ AttnParams p) {
     sync();
 
     for (int l = L - 1; l >= 0; --l) {
-        for (int i = tid; i < TK; i += nthr) store_parent(p, l, qidx * TK + i, par[i]);
+        if (rank == 0) for (int i = tid; i < TK; i += nthr) store_parent(p, l, qidx * TK + i, par[i]);
         if (l == 0) break;
         const int Nl = p.ln[l];
         const int rc = (int)(((int64_t)t / p.lpow[l]) % CR);
@@ -254,10 +257,16 @@ select_mma_kernel(const __grid_constant__ AttnParams p) {
                 e0 += __shfl_xor_sync(0xffffffffu, e0, 1); e1 += __shfl_xor_sync(0xffffffffu, e1, 1);
                 e0 += __shfl_xor_sync(0xffffffffu, e0, 2); e1 += __shfl_xor_sync(0xffffffffu, e1, 2);
                 // (all of the chunk's loads end in these stores, ahead of the copies that refill the slot)
-                if (r < 2 && 16 * c + 8 * r + g < maxc) imp[16 * c + 8 * r + g] = r ? e1 : e0;
-                if (lane < PPC && c * PPC + lane < np) cmax[c * PPC + lane] = lane ? m1 : m0;
+                if (rank == 0) {
+                    if (r < 2 && 16 * c + 8 * r + g < maxc) imp[16 * c + 8 * r + g] = r ? e1 : e0;
+                    if (lane < PPC && c * PPC + lane < np) cmax[c * PPC + lane] = lane ? m1 : m0;
+                } else {
+                    if (r < 2 && 16 * c + 8 * r + g < maxc) st_cluster(cluster_addr(imp + 16 * c + 8 * r + g, 0), __float_as_uint(r ? e1 : e0));
+                    if (lane < PPC && c * PPC + lane < np) st_cluster(cluster_addr(cmax + c * PPC + lane, 0), __float_as_uint(lane ? m1 : m0));
+                }
             }
-            sync();
+            if (CL > 1) cluster_sync(); else sync();
+            if (rank == 0) {
             // common reference maximum (src/naive.py:204-205), right-most candidate forced (src/naive.py:93)
             float M = -INFINITY;
             for (int a = lane; a < np; a += 32) M = fmaxf(M, cmax[a]);
@@ -386,6 +395,16 @@ select_mma_kernel(const __grid_constant__ AttnParams p) {
             for (int i = base_out + tid; i < TK; i += nthr) nxt[i] = -1;
             if (SPLIT && threadIdx.x < 3) cnt[threadIdx.x] = 0;
             np = base_out;
+            if (CL > 1) {                                       // the kept list and its length to the other blocks
+                __syncthreads();
+                for (int i = threadIdx.x; i < TK * (CL - 1); i += nthr) st_cluster(cluster_addr(nxt + i % TK, 1 + i / TK), (uint32_t)nxt[i % TK]);
+                if ((int)threadIdx.x < CL - 1) st_cluster(cluster_addr(cnt + 3, 1 + threadIdx.x), (uint32_t)np);
+            }
+            }
+            if (CL > 1) {
+                cluster_sync();
+                if (rank) np = cnt[3];
+            }
         }
         sync();
         int32_t* tmp = par; par = nxt; nxt = tmp;
@@ -408,7 +427,11 @@ static int launch_select_cr(const AttnParams& in, cudaStream_t st) {
         static SmemLimit shared;
         const cudaError_t e = shared.raise((const void*)k, split_smem);
         if (e != cudaSuccess) return (int)e;
-        return launch_chained(k, dim3(p.Tq, p.B * p.Hkv), dim3(kSelSplitWarps * 32), split_smem, st, p);
+        // Blocks per group, while each has an SM and as a level has chunks for their warps (long lists of many groups: one).  With the
+        // accumulation alone on clusters a decode call took 63.5 us, with both 60.9.
+        int CL = 1;
+        while (CL < 8 && 2 * CL * groups <= 148 && 2 * CL * kSelSplitWarps <= maxc / 16) CL *= 2;
+        return launch_chained_clusters(k, CL, dim3(p.Tq * CL, p.B * p.Hkv), dim3(kSelSplitWarps * 32), split_smem, st, p);
     }
     const size_t per_warp = Ring::kBytes + scratch;
     constexpr int max_warps = 4 * sel_min_blocks<D, X3, NH>();

@@ -502,9 +502,11 @@ __host__ __device__ __forceinline__ WalkLayout walk_layout(const AttnParams& p, 
 }
 template <typename Ring, int PK = 1>
 __host__ __device__ __forceinline__ size_t walk_warp_bytes(const WalkLayout& w) { return (Ring::kBytes + PK * (w.list + w.bits) + 127) & ~size_t(127); }
+__host__ __device__ __forceinline__ size_t walk_lists_bytes(const WalkLayout& w) { return ((size_t)w.list + w.bits + 127) & ~size_t(127); }
 // one bit per candidate of a level that the next level kept, from its list (both lists ascending); the bits are clear and the list there
-__device__ __forceinline__ void mark_kept(const AttnParams& p, int l, int64_t list, const ParentList& par, int np, int CR, uint32_t* selw, int lane) {
-    for (int i = lane; i < p.TK; i += 32) {
+template <int NT>
+__device__ __forceinline__ void mark_kept(const AttnParams& p, int l, int64_t list, const ParentList& par, int np, int CR, uint32_t* selw, int thread) {
+    for (int i = thread; i < p.TK; i += NT) {
         const int node = load_parent(p, l - 1, list + i);
         if (node < 0) continue;
         const int parent = node / CR;

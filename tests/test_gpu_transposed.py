@@ -79,7 +79,11 @@ def test_selections_bit_identical(dt, D, CR, G, B, T, TK, MTN, clustered):
 
 @pytest.mark.parametrize("dt,D,CR,G,T,TK,MTN,W", [
     (BF, 128, 16, 16, 20000, 64, 64, 1), (HF, 64, 16, 8, 9001, 16, 64, 17), (FP, 64, 8, 8, 9001, 32, 128, 3), (HF, 32, 16, 4, 9001, 16, 64, 1),
-    (BF, 128, 16, 16, 4000, 16, 64, 125), (BF, 128, 16, 16, 4000, 16, 64, 8)])      # either side of 2 * W * TK = parents
+    (BF, 128, 16, 16, 4000, 16, 64, 125), (BF, 128, 16, 16, 4000, 16, 64, 8),       # either side of 2 * W * TK = parents
+    # blocks per query: 8, 4, 2 and 1 (by the room on the chip), 2 (by the chunks of a level); long lists; fp32 of 128 dims; 8 children
+    (BF, 128, 16, 16, 20000, 128, 64, 9), (BF, 128, 16, 16, 20000, 128, 64, 18), (BF, 128, 16, 16, 20000, 128, 64, 37),
+    (BF, 128, 16, 16, 20000, 128, 64, 38), (BF, 64, 16, 16, 20000, 16, 64, 2), (HF, 128, 16, 1, 30000, 1024, 2048, 1),
+    (FP, 128, 16, 16, 9001, 128, 128, 5), (BF, 128, 8, 9, 12000, 512, 512, 2)])
 def test_few_queries(dt, D, CR, G, T, TK, MTN, W):
     import htree_b200 as ht
     from htree_b200 import ops

@@ -271,7 +271,7 @@ int htree_b200_prepare(const HtreeShape* shape, void* const* layers_k, void* con
 static int attend(const HtreeShape* shape, const void* q, void* const* layers_k, void* const* layers_v, void* const* blocks,
                   const float* cos_cache, const float* sin_cache, const void* table, const void* table_f32, int32_t n_pos, float scale,
                   void* out, float* gmax, float* gsum, int32_t* const* parents, int32_t* status, uint32_t flags, bool pack_leaves,
-                  void* stream) {
+                  float* top_keys, void* stream) {
     int32_t ln[HTREE_MAX_LEVELS];
     const int L = check_shape(shape, ln);
     if (L < 0) return L;
@@ -289,8 +289,15 @@ static int attend(const HtreeShape* shape, const void* q, void* const* layers_k,
     }
     if (!acc_mma_supported(p, shape->dtype)) return HTREE_E_UNSUPPORTED;
     p.flags = flags | HTREE_FWD_SELECT_ONLY;
-    rc = select_blk_supported(p, shape->dtype) ? launch_select_blk(p, shape->dtype, (cudaStream_t)stream)
-                                               : launch_fwd_generic(p, shape->dtype, (cudaStream_t)stream);
+    if (select_blk_supported(p, shape->dtype)) {
+        rc = launch_select_blk(p, shape->dtype, (cudaStream_t)stream);
+    } else {
+        p.ktop = top_keys;
+        rc = launch_select_top(p, shape->dtype, !fwd_generic_tiled(p), (cudaStream_t)stream);
+        if (rc == 0) p.first_level = L - 2;       // (0: two levels, nothing below selects)
+        if (rc == HTREE_E_UNSUPPORTED || (rc == 0 && L > 2)) rc = launch_fwd_generic(p, shape->dtype, (cudaStream_t)stream);
+        p.first_level = 0;
+    }
     if (rc || select_only) return rc;
     if (pack_leaves) {
         rc = launch_pack_listed(*shape, p.Tq, layers_k[0], layers_v[0], blocks[0], parents[0], cos_cache, sin_cache, (cudaStream_t)stream);
@@ -304,7 +311,7 @@ int htree_b200_attend(const HtreeShape* shape, const void* q, void* const* layer
                       const float* cos_cache, const float* sin_cache, const void* table, const void* table_f32, int32_t n_pos, float scale,
                       void* out, float* gmax, float* gsum, int32_t* const* parents, int32_t* status, uint32_t flags, void* stream) {
     return attend(shape, q, layers_k, layers_v, blocks, cos_cache, sin_cache, table, table_f32, n_pos, scale, out, gmax, gsum, parents,
-                  status, flags, false, stream);
+                  status, flags, false, nullptr, stream);
 }
 
 int htree_b200_plan(const HtreeShape* shape, uint32_t flags, HtreePlan* plan) {
@@ -329,6 +336,7 @@ int htree_b200_plan(const HtreeShape* shape, uint32_t flags, HtreePlan* plan) {
         plan->blocks_bwd[l] = flags & HTREE_PLAN_BACKWARD ? take(blocks * (x3 ? 2 : 1) * shape->K * 2 * CR) : -1;
         plan->parents[l] = flags & HTREE_PLAN_PARENTS ? take((int64_t)shape->B * Tq * shape->H_kv * shape->top_k * 4) : -1;
     }
+    take(top_keys_bytes(*shape, L, ln));       // at the workspace's end
     plan->bytes = at;
     return 0;
 }
@@ -368,7 +376,11 @@ int htree_b200_run_forward(const HtreeShape* shape, const HtreePlan* plan, const
         rc = htree_b200_prepare(shape, lk, lv, bl, plan->blocks_bwd[0] >= 0 ? bb : nullptr, 1, cos_cache, sin_cache, stream);
     }
     if (rc) return rc;
-    return attend(shape, q, lk, lv, bl, cos_cache, sin_cache, table, table_f32, n_pos, scale, out, gmax, gsum, par, status, flags, few, stream);
+    int32_t ln[HTREE_MAX_LEVELS];
+    const int L = check_shape(shape, ln);
+    const int64_t top = L < 0 ? 0 : (top_keys_bytes(*shape, L, ln) + 255) & ~int64_t(255);
+    return attend(shape, q, lk, lv, bl, cos_cache, sin_cache, table, table_f32, n_pos, scale, out, gmax, gsum, par, status, flags, few,
+                  top ? reinterpret_cast<float*>(w + plan->bytes - top) : nullptr, stream);
 }
 
 int htree_b200_block_keys(const HtreeShape* shape, void* const* layers_k_rot, void* const* layers_k_blk, void* stream) {

@@ -27,6 +27,8 @@ struct AttnParams {
     const void* blk[HTREE_MAX_LEVELS];   // operand blocks of the transposed kernels (tform.cuh), or NULL
     const void* vkblk[HTREE_MAX_LEVELS]; // their backward part, or NULL
     const void* tab;                     // rotary table of the transposed kernels, rows [cos | sin]: IEEE half times scale, or fp32 (split-half)
+    float* ktop;                         // rotated keys of the top level (select_top.cu), or NULL
+    int32_t first_level;                 // fwd_generic_kernel: where it starts, the lists of that level given; 0 = the top
     const void* tab32;                   // fp32 rows [cos | sin] for the selection kernel
     int32_t sel_maxc;                    // most candidates of a group on a level that selects (set by the selection's launch)
     int32_t ln[HTREE_MAX_LEVELS];   // N_l
@@ -167,6 +169,37 @@ __device__ __forceinline__ float2 ld_cluster2(uint32_t a) {
 }
 __device__ __forceinline__ void st_cluster(uint32_t a, uint32_t x) { asm volatile("st.shared::cluster.b32 [%0], %1;" ::"r"(a), "r"(x) : "memory"); }
 
+// Exact Top-K over non-negative floats, whose bit patterns order like the values: search for the TK-th largest key by counting the keys at
+// or above a probe, in the bracket [lo, hi) that the smallest and the largest key span (one forced key above hi left out of it).  The next
+// probe is where the logit of the count, interpolated over the bit patterns, reaches TK, every fourth one the middle: 5 to 8 counts where
+// bisecting the 31 bits takes 13 to 21.
+struct TopKBound {
+    uint32_t tau;      // keys above are kept
+    int need;          // and this many of those equal to it, the smallest positions
+    bool exact;        // none equal to it is
+};
+template <typename Count>
+__device__ __forceinline__ TopKBound topk_search(Count count, uint32_t lo, uint32_t hi, int nc, int TK) {
+    int c_lo = nc, c_hi = 1;
+    if (TK == 1) { hi = 0x7f800000u; c_hi = 0; }       // only the forced candidate is kept
+    bool exact = false;
+    auto logit = [&](int c) { return __log2f(__fdividef((float)c - 0.25f, (float)(nc - c) + 0.75f)); };
+    const float want = logit(TK);
+    float f_lo = logit(c_lo), f_hi = logit(c_hi < 1 ? 1 : c_hi);
+    for (int it = 0; hi - lo > 1u; ++it) {
+        uint32_t x = lo + ((hi - lo) >> 1);
+        if ((it & 3) != 3) {
+            const float f = fminf(fmaxf(__fdividef(f_lo - want, f_lo - f_hi), 0.f), 1.f);
+            x = lo + (uint32_t)(f * (float)(hi - lo));
+            x = x <= lo ? lo + 1u : x >= hi ? hi - 1u : x;
+        }
+        const int c = count(x);
+        if (c == TK) { lo = x - 1u; c_hi = TK; exact = true; break; }    // the kept keys are those at or above x
+        if (c > TK) { lo = x; f_lo = logit(c); } else { hi = x; c_hi = c; f_hi = logit(c < 1 ? 1 : c); }
+    }
+    return TopKBound{lo, TK - c_hi, exact};
+}
+
 // Parent lists: int32 with -1 for "none" (the reference's layout), or uint16 with 0xFFFF under HTREE_PARENTS_U16.
 __device__ __forceinline__ int load_parent(const AttnParams& p, int l, int64_t idx) {
     if (p.flags & HTREE_PARENTS_U16) {
@@ -210,6 +243,9 @@ int launch_pack_listed(const HtreeShape& s, int Tq, const void* k, const void* v
                        const float* sinc, cudaStream_t st);
 int launch_pack_blocks(const HtreeShape& s, int first, int L, const int32_t* ln, void* const* lk, void* const* lv, void* const* blk,
                        void* const* vkblk, bool pool, const float* cosc, const float* sinc, cudaStream_t st);
+int64_t top_keys_bytes(const HtreeShape& s, int L, const int32_t* ln);       // select_top.cu
+int launch_select_top(const AttnParams& p, int dtype, bool sums, cudaStream_t st);
+bool fwd_generic_tiled(const AttnParams& p);             // does fwd_generic_kernel take its tiled form?
 bool select_blk_supported(const AttnParams& p, int dtype);
 int launch_select_blk(const AttnParams& p, int dtype, cudaStream_t st);
 bool select_mma_supported(const AttnParams& p, int dtype);

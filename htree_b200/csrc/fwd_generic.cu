@@ -140,6 +140,8 @@ __global__ void __launch_bounds__(NT) fwd_generic_kernel(const __grid_constant__
     int32_t* nxt = m.par + TK;
     if (p.level_mode) {
         for (int i = tid; i < TK; i += NT) par[i] = p.parents_in[qidx * TK + i];
+    } else if (p.first_level) {
+        for (int i = tid; i < TK; i += NT) par[i] = load_parent(p, p.first_level, qidx * TK + i);
     } else {
         int np0 = (int)(((int64_t)t / p.lpow[L - 1]) / CR) + 1;
         if (np0 > TK) np0 = TK;
@@ -148,7 +150,7 @@ __global__ void __launch_bounds__(NT) fwd_generic_kernel(const __grid_constant__
     int slot = 0;
     __syncthreads();
 
-    const int l_hi = p.level_mode ? p.level_index : L - 1, l_lo = p.level_mode ? p.level_index : 0;
+    const int l_hi = p.level_mode ? p.level_index : p.first_level ? p.first_level : L - 1, l_lo = p.level_mode ? p.level_index : 0;
     for (int l = l_hi; l >= l_lo; --l) {
         const int Nl = p.ln[l];
         const int64_t tslot = p.level_mode ? 0 : l;   // slot of this level in the trace arrays
@@ -508,14 +510,18 @@ static int launch_tt(const AttnParams& p, size_t smem, int GP, cudaStream_t st) 
     return launch_chained(k, grid, dim3(NT), smem, st, p);
 }
 
+bool fwd_generic_tiled(const AttnParams& p) {
+    const int GP = p.G <= 4 ? 4 : (p.G <= 8 ? 8 : 16), GPAD = (p.G + GP - 1) / GP * GP;
+    return fwd_smem_layout(p.K, p.V, GPAD, GP, p.TK * p.CR, p.TK, false, nullptr, nullptr) > 227 * 1024 || (p.flags & HTREE_FWD_TILED);
+}
+
 template <typename T>
 static int launch_t(const AttnParams& p, cudaStream_t st) {
     const int G = p.G;
     const int GP = G <= 4 ? 4 : (G <= 8 ? 8 : 16);
     const int GPAD = (G + GP - 1) / GP * GP;
     const size_t limit = 227 * 1024;
-    const size_t full = fwd_smem_layout(p.K, p.V, GPAD, GP, p.TK * p.CR, p.TK, false, nullptr, nullptr);
-    if (full <= limit && !(p.flags & HTREE_FWD_TILED)) return launch_tt<T, false>(p, full, GP, st);
+    if (!fwd_generic_tiled(p)) return launch_tt<T, false>(p, fwd_smem_layout(p.K, p.V, GPAD, GP, p.TK * p.CR, p.TK, false, nullptr, nullptr), GP, st);
     const size_t tiled = fwd_smem_layout(p.K, p.V, GPAD, GP, p.TK * p.CR, p.TK, true, nullptr, nullptr);
     if (tiled > limit) return HTREE_E_UNSUPPORTED;
     return launch_tt<T, true>(p, tiled, GP, st);

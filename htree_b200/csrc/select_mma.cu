@@ -272,10 +272,6 @@ select_mma_kernel(const __grid_constant__ AttnParams p) {
             for (int a = lane; a < np; a += 32) M = fmaxf(M, cmax[a]);
             M = warp_max(M);
             if constexpr (SPLIT) __syncthreads();           // every warp has read the maxima before they become factors
-            // Exact Top-K: search for the TK-th largest key (non-negative floats order like their bit patterns) by counting the keys
-            // at or above a probe, in the bracket that the smallest and the largest key span.  The next probe is where the logit of the
-            // count, interpolated over the bit patterns, reaches TK, every fourth one the middle: 5 to 8 counts where bisecting the
-            // 31 bits takes 13 to 21.
             uint32_t* key = reinterpret_cast<uint32_t*>(imp);
             __syncwarp();
             for (int a = SPLIT ? (int)threadIdx.x : lane; a < np; a += nthr) cmax[a] = __expf(cmax[a] - M);
@@ -324,7 +320,7 @@ select_mma_kernel(const __grid_constant__ AttnParams p) {
                 }
                 return c;
             };
-            // lo: more than TK keys reach it; hi: fewer do (the forced candidate, the largest by far, is left out of the bracket)
+            // the smallest and the largest key (the forced candidate, the largest by far, is left out)
             uint32_t lo = 0xffffffffu, hi = 0u;
             if (in_regs) {
                 each([&](int i) {
@@ -342,26 +338,10 @@ select_mma_kernel(const __grid_constant__ AttnParams p) {
                 for (int w = 0; w < kSelSplitWarps; ++w) { lo = min(lo, (uint32_t)wtot[2 * w]); hi = max(hi, (uint32_t)wtot[2 * w + 1]); }
                 __syncthreads();       // the placement below writes wtot, and where all importances are equal no count comes between
             }
-            hi += 1u;
-            int c_lo = nc, c_hi = 1;
-            if (TK == 1) { hi = 0x7f800000u; c_hi = 0; }       // only the forced candidate is kept
-            bool exact = false;
-            auto logit = [&](int c) { return __log2f(__fdividef((float)c - 0.25f, (float)(nc - c) + 0.75f)); };
-            const float want = logit(TK);
-            float f_lo = logit(c_lo), f_hi = logit(c_hi < 1 ? 1 : c_hi);
-            for (int it = 0; hi - lo > 1u; ++it) {
-                uint32_t x = lo + ((hi - lo) >> 1);
-                if ((it & 3) != 3) {
-                    const float f = fminf(fmaxf(__fdividef(f_lo - want, f_lo - f_hi), 0.f), 1.f);
-                    x = lo + (uint32_t)(f * (float)(hi - lo));
-                    x = x <= lo ? lo + 1u : x >= hi ? hi - 1u : x;
-                }
-                const int c = count(x);
-                if (c == TK) { lo = x - 1u; c_hi = TK; exact = true; break; }    // the kept keys are those at or above x
-                if (c > TK) { lo = x; f_lo = logit(c); } else { hi = x; c_hi = c; f_hi = logit(c < 1 ? 1 : c); }
-            }
-            const uint32_t tau = lo;
-            const int need = TK - c_hi;     // keys equal to tau that are kept: the smallest positions
+            const TopKBound bound = topk_search(count, lo, hi + 1u, nc, TK);
+            const uint32_t tau = bound.tau;
+            const int need = bound.need;
+            const bool exact = bound.exact;
             int base_eq = 0, base_out = 0;
             auto place = [&](int j, uint32_t kx) {
                 const bool gt = j < nc && kx > tau, eq = !exact && j < nc && kx == tau;

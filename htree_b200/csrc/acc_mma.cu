@@ -595,8 +595,11 @@ static int launch_acc_cr(const AttnParams& p, cudaStream_t st) {
         // Blocks per group: while each has an SM, and as a level has chunks for their warps.  A round of chunks ends in a barrier of the
         // cluster, and a walk over 128 chunks was 16 rounds of one block: 4 x 1 queries against 16384 positions, 16 heads of 128, 8 blocks
         // each: 29 -> 20 us; 5 queries of one head against 512 leaf parents: the call 118 -> 71 us.
+        // (Chunks of 4 KB pass so fast that a cluster's barriers have to be shared by four rounds.)
+        constexpr int rounds = TForm<D, X3, CR>::VSLOT >= 4096 ? 1 : 4;
+        const int leaf = (p.ln[0] + CR - 1) / CR, chunks = ((p.TK < leaf ? p.TK : leaf) * CR + 15) / 16;
         int CL = 1;
-        while (CL < 8 && 2 * CL * groups <= 148 && 2 * CL * kAccSplitWarps <= (p.TK * CR + 15) / 16) CL *= 2;
+        while (CL < 8 && 2 * CL * groups <= 148 && 2 * CL * kAccSplitWarps * rounds <= chunks) CL *= 2;
         return launch_chained_clusters(k, CL, dim3(p.Tq * CL, p.B * p.Hkv), dim3(kAccSplitWarps * 32), split_smem, st, p);
     }
     if constexpr (NH == 1 && CR == 16) {

@@ -196,17 +196,12 @@ __global__ void __launch_bounds__(128, dkv_min_blocks<D, X3, CR, KEYS>()) bwd_dk
     constexpr int PLANE = NT * 128;                                         // bytes from the hi to the lo words of a record
     using Ring = WarpRing<NSTG, SLOT>;
     extern __shared__ __align__(128) unsigned char smem_raw[];
+    chain_enter();
     const AttnParams& p = bp.a;
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, g = lane >> 2;
     const int it = blockIdx.x * (blockDim.x >> 5) + warp, ls = blockIdx.y;
-    // dV needs nothing of dK's launch before it, so it does not wait for it until its own end (what it reads was complete when that launch
-    // began, and let this one be set up; read through L2, since no wait stands before the reads).
-    if constexpr (KEYS) chain_wait();
-    chain_next();
-    auto leave = [&]() { if constexpr (!KEYS) chain_wait(); };
-    if (it >= __ldcg(bp.nitems + ls)) { leave(); return; }
-    const int4 item4 = __ldcg(reinterpret_cast<const int4*>(bp.items + (int64_t)ls * bp.cap + it));
-    const BwdItem item{item4.x, item4.y, item4.z, item4.w};
+    if (it >= bp.nitems[ls]) return;
+    const BwdItem item = bp.items[(int64_t)ls * bp.cap + it];
     Ring ring;
     ring.init(smem_raw + (size_t)warp * Ring::kBytes);
     using Entry = BwdEntry<X3, (PK > 1)>;
@@ -223,17 +218,7 @@ __global__ void __launch_bounds__(128, dkv_min_blocks<D, X3, CR, KEYS>()) bwd_dk
 #pragma unroll
         for (int n = 0; n < NT; ++n) acc[i][n][0] = acc[i][n][1] = acc[i][n][2] = acc[i][n][3] = 0.f;
 
-    auto entry = [&](int e) {
-        Entry x;
-        if constexpr (sizeof(Entry) == 8) {
-            *reinterpret_cast<uint2*>(&x) = __ldcg(reinterpret_cast<const uint2*>(entries + min(e, len - 1)));
-        } else {
-#pragma unroll
-            for (int i = 0; i < (int)sizeof(Entry) / 16; ++i) reinterpret_cast<uint4*>(&x)[i] = __ldcg(reinterpret_cast<const uint4*>(entries + min(e, len - 1)) + i);
-        }
-        return x;
-    };
-    Entry cur = entry(lane), nxt = entry(32 + lane);
+    Entry cur = entries[min(lane, len - 1)], nxt = entries[min(32 + lane, len - 1)];
     static_assert(!X3 || NSTG == 2, "a step's factors are taken when the next one is fetched");
     float fa = 0.f, fb = 0.f;                      // split-half: the factors of the visits fetched last
     bool differ = false;                           // do they differ among the 32 of `cur`?
@@ -248,7 +233,7 @@ __global__ void __launch_bounds__(128, dkv_min_blocks<D, X3, CR, KEYS>()) bwd_dk
     auto fill = [&](int s) {                       // operand, record and table row of the step's one or two visits
         const int e0 = s * VPS;
         if (e0 && (e0 & 31) == 0) {
-            cur = nxt; nxt = entry(e0 + 32 + lane);
+            cur = nxt; nxt = entries[min(e0 + 32 + lane, len - 1)];
             compare();
         }
         if constexpr (X3) {
@@ -405,7 +390,6 @@ __global__ void __launch_bounds__(128, dkv_min_blocks<D, X3, CR, KEYS>()) bwd_dk
     for (int i = 0; i < KS; ++i)
 #pragma unroll
         for (int n = 0; n < NT; ++n) red_add_v4(dst + (i * NT + n) * 128, acc[i][n][0] * post, acc[i][n][1] * post, acc[i][n][2] * post, acc[i][n][3] * post);
-    leave();
 }
 
 // Accumulators to the leaves' gradients: dK' rotated back by the child index, plus the mean-pool shares of the ancestors' gradients

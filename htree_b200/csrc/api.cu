@@ -75,7 +75,7 @@ struct BwdLayout {
     BwdParams bp;
     int64_t acc_bytes, scratch_bytes, zero_bytes;
     int64_t acck[HTREE_MAX_LEVELS], accv[HTREE_MAX_LEVELS];
-    int64_t o_qb, o_dob, o_stp, o_sts, o_fac, o_rank, o_nvis, o_cnt, o_base, o_entries, o_items, o_nitems;
+    int64_t o_qb, o_dob, o_stp, o_sts, o_fac, o_rank, o_nvis, o_xtab, o_cnt, o_base, o_entries, o_items, o_nitems;
     int total, per_launch;
 };
 
@@ -110,6 +110,8 @@ static int bwd_layout(const HtreeShape* s, int L, const int32_t* ln, int64_t bud
     const int64_t entry = x3 ? (many ? sizeof(BwdEntry<true, true>) : sizeof(BwdEntry<true, false>)) : (many ? sizeof(BwdEntry<false, true>) : sizeof(BwdEntry<false, false>));
     // A window's blocked queries (4 KB each at 16 heads of 128) should stay in the L2 while its parents gather them: 8192 queries
     // are 33 MB; longer windows mean longer visit lists and fewer reductions.
+    const int64_t xtab = x3 ? 0 : up((int64_t)TK * CR * D * 2);
+    budget -= xtab < budget / 2 ? xtab : budget / 2;
     int64_t subq = 0, ng = 0, bytes = 0;
     for (int64_t most = 8192; most >= 16; most >>= 1) {
         const int64_t nw = (Tq + most - 1) / most;
@@ -140,6 +142,7 @@ static int bwd_layout(const HtreeShape* s, int L, const int32_t* ln, int64_t bud
     y.o_qb = take(per * ng * qb); y.o_dob = take(per * ng * qb);
     y.o_stp = take(per * ng * MV * sb); y.o_sts = take(per * ng * MV * sb);
     y.o_fac = x3 ? take(per * ng * L * 8) : -1;
+    y.o_xtab = x3 ? -1 : take(xtab);
     y.o_nvis = many ? take(per * ng * L * 4) : -1;
     y.o_rank = take(per * ng * MV * (many ? 16 : 4)); y.o_entries = take(per * ng * MV * entry);
     y.o_cnt = take(cnt_words(per, NK) * 4 + 4 + units * 4); y.o_base = take(per * NK * 8);
@@ -571,6 +574,7 @@ int htree_b200_run_backward(const HtreeShape* shape, const void* q, void* const*
     bp.qb = sb + y.o_qb; bp.dob = sb + y.o_dob; bp.stp = sb + y.o_stp; bp.sts = sb + y.o_sts;
     bp.fac = y.o_fac < 0 ? nullptr : reinterpret_cast<float2*>(sb + y.o_fac);
     bp.rank = reinterpret_cast<int32_t*>(sb + y.o_rank); bp.vis = reinterpret_cast<uint4*>(sb + y.o_rank);
+    bp.xtab = y.o_xtab < 0 ? nullptr : sb + y.o_xtab;
     bp.nvis = y.o_nvis < 0 ? nullptr : reinterpret_cast<int32_t*>(sb + y.o_nvis); bp.entries = sb + y.o_entries;
     bp.cnt = reinterpret_cast<int32_t*>(sb + y.o_cnt); bp.range = reinterpret_cast<uint32_t*>(bp.cnt + cnt_words(y.per_launch, bp.NK)); bp.base = reinterpret_cast<int2*>(sb + y.o_base);
     bp.items = reinterpret_cast<BwdItem*>(sb + y.o_items); bp.nitems = reinterpret_cast<int32_t*>(sb + y.o_nitems);
@@ -578,7 +582,8 @@ int htree_b200_run_backward(const HtreeShape* shape, const void* q, void* const*
     for (int s0 = 0; s0 < y.total; s0 += y.per_launch) {
         bp.sub0 = s0; bp.nsub = y.total - s0 < y.per_launch ? y.total - s0 : y.per_launch;
         // the counters, and ahead of the first launch (which has the most windows) the words of the range behind them
-        rc = launch_bwd_clear(bp.cnt, cnt_words(bp.nsub, bp.NK) * 4 + (s0 == 0 ? (1 + (int64_t)shape->B * shape->H_kv) * 4 : 0), st);
+        rc = launch_bwd_clear(bp.cnt, cnt_words(bp.nsub, bp.NK) * 4 + (s0 == 0 ? (1 + (int64_t)shape->B * shape->H_kv) * 4 : 0), table,
+                              s0 == 0 ? const_cast<unsigned char*>(bp.xtab) : nullptr, shape->top_k * shape->compression_rate, shape->K, st);
         if (rc == 0 && s0 == 0) rc = launch_bwd_begin(bp, shape->dtype, acc, flags & HTREE_BWD_KEEP_ACCUM ? 0 : y.zero_bytes, st);
         if (rc == 0) rc = launch_bwd_dq(bp, shape->dtype, st);
         if (rc == 0) rc = launch_bwd_dkv(bp, shape->dtype, st);

@@ -208,7 +208,7 @@ __global__ void __launch_bounds__(128, dkv_min_blocks<D, X3, CR, KEYS>()) bwd_dk
     const Entry* entries = reinterpret_cast<const Entry*>(bp.entries) + (int64_t)ls * bp.ng * bp.MV + item.start;
     const unsigned char* qsrc = KEYS ? bp.qb : bp.dob;
     const unsigned char* ssrc = KEYS ? bp.sts : bp.stp;
-    const unsigned char* tab = reinterpret_cast<const unsigned char*>(p.tab);
+    const unsigned char* tab = X3 ? reinterpret_cast<const unsigned char*>(p.tab) : bp.xtab;
     constexpr int VPS = NH == 2 ? 1 : 2;                                    // visits per step
     const int len = item.len, steps = (len + VPS - 1) / VPS;
 
@@ -304,32 +304,21 @@ __global__ void __launch_bounds__(128, dkv_min_blocks<D, X3, CR, KEYS>()) bwd_dk
             }
         }
         if constexpr (KEYS && !X3) {
-            const uint32_t sel = (g & 1) ? 0x3232u : 0x1010u;
-            const uint32_t ta = slot + 2 * QB + 2 * SB + 2 * PPT * (g >> 1) + tab_of_pair, tb = VPS == 2 ? ta + PK * TAB : ta;
+            const uint32_t ta = slot + 2 * QB + 2 * SB + 2 * KS * (4 * (g & 1) + (g >> 1)) + tab_of_pair;
+            uint32_t ca[KS / 2], sa[KS / 2], cb[KS / 2], sb[KS / 2];
+            lds_x<D>(ta, ca, sa);
+            if constexpr (VPS == 2) lds_x<D>(ta + PK * TAB, cb, sb);
 #pragma unroll
-            for (int k4 = 0; k4 < KS; k4 += 4) {
-                const uint4 ca4 = lds_u4(ta + 4 * k4), sa4 = lds_u4(ta + 2 * HALF + 4 * k4);
-                const uint4 cb4 = VPS == 2 ? lds_u4(tb + 4 * k4) : ca4, sb4 = VPS == 2 ? lds_u4(tb + 2 * HALF + 4 * k4) : sa4;
-                const uint32_t ca[4] = {ca4.x, ca4.y, ca4.z, ca4.w}, sa[4] = {sa4.x, sa4.y, sa4.z, sa4.w};
-                const uint32_t cb[4] = {cb4.x, cb4.y, cb4.z, cb4.w}, sb[4] = {sb4.x, sb4.y, sb4.z, sb4.w};
+            for (int i = 0; i < KS; ++i) {
+                uint32_t la, ha, lb, hb, a[4];
+                lds64(slot + i * 256 + lane * 8, la, ha);
+                lds64(slot + QB + i * 256 + lane * 8, lb, hb);
+                const __half2 c0 = half_of(ca[i / 2], i & 1), s0 = half_of(sa[i / 2], i & 1);
+                rotate_x<false>(la, ha, c0, s0, a[0], a[1]);
+                if constexpr (VPS == 2) rotate_x<false>(lb, hb, half_of(cb[i / 2], i & 1), half_of(sb[i / 2], i & 1), a[2], a[3]);
+                else rotate_x<false>(lb, hb, c0, s0, a[2], a[3]);
 #pragma unroll
-                for (int u = 0; u < 4; ++u) {
-                    const int i = k4 + u;
-                    uint32_t la, ha, lb, hb, a[4];
-                    lds64(slot + i * 256 + lane * 8, la, ha);
-                    lds64(slot + QB + i * 256 + lane * 8, lb, hb);
-                    const uint32_t c0 = __byte_perm(ca[u], ca[u], sel), s0 = __byte_perm(sa[u], sa[u], sel);
-                    const uint32_t n0 = neg_h2(s0);
-                    rotate_h2(la, ha, c0, s0, n0, a[0], a[1]);
-                    if constexpr (VPS == 2) {
-                        const uint32_t c1 = __byte_perm(cb[u], cb[u], sel), s1 = __byte_perm(sb[u], sb[u], sel);
-                        rotate_h2(lb, hb, c1, s1, neg_h2(s1), a[2], a[3]);
-                    } else {
-                        rotate_h2(lb, hb, c0, s0, n0, a[2], a[3]);
-                    }
-#pragma unroll
-                    for (int n = 0; n < NT; ++n) mma_acc<FT>(acc[i][n], a, bw[n][0], bw[n][1]);
-                }
+                for (int n = 0; n < NT; ++n) mma_acc<FT>(acc[i][n], a, bw[n][0], bw[n][1]);
             }
         } else if constexpr (!X3) {
 #pragma unroll
@@ -540,20 +529,32 @@ static int launch_range_t(const BwdParams& bp, void* zero, int64_t zero_bytes, c
     const unsigned grid = (unsigned)(a.of_dO + units * a.of_v);
     return launch_chained(p.K == 128 ? bwd_range_kernel<T, 128> : bwd_range_kernel<T, 64>, dim3(grid), dim3(256), 0, st, a);
 }
-// Zeros, `n` 16-byte pieces (a memset node in the chain would have to end and be waited for like any launch that is not chained).
-__global__ void __launch_bounds__(256) bwd_clear_kernel(uint4* p, int64_t n) {
+// Zeros, `n` 16-byte pieces (a memset node in the chain would have to end and be waited for like any launch that is not chained), and the
+// rotary rows in lane order.
+template <int D>
+__global__ void __launch_bounds__(256) bwd_clear_kernel(uint4* p, int64_t n, const __half* tab, uint4* xtab, int rows) {
     chain_enter();
     for (int64_t i = (int64_t)blockIdx.x * 256 + threadIdx.x; i < n; i += (int64_t)gridDim.x * 256) p[i] = make_uint4(0u, 0u, 0u, 0u);
+    constexpr int PER = D / 8;                     // pieces of 8 halves per row
+    for (int i = blockIdx.x * 256 + threadIdx.x; i < rows * PER; i += gridDim.x * 256) {
+        const int row = i / PER, at = i % PER * 8, part = at / (D / 2);      // cosines, sines
+        const __half* src = tab + (int64_t)row * D + part * (D / 2);
+        alignas(16) __half x[8];
+#pragma unroll
+        for (int u = 0; u < 8; ++u) x[u] = src[x_index<D>(at % (D / 2) + u)];
+        xtab[i] = *reinterpret_cast<const uint4*>(x);
+    }
 }
-// clears whole 16-byte pieces: `bytes` rounded up
-int launch_bwd_clear(void* p, int64_t bytes, cudaStream_t st) {
-    const int64_t n = (bytes + 15) / 16, blocks = (n + 1023) / 1024;
-    return launch_chained(bwd_clear_kernel, dim3((unsigned)(blocks < 148 * 8 ? blocks : 148 * 8)), dim3(256), 0, st, static_cast<uint4*>(p), n);
+// clears whole 16-byte pieces: `bytes` rounded up; rows of the table where `xtab` is given
+int launch_bwd_clear(void* p, int64_t bytes, const void* tab, void* xtab, int rows, int D, cudaStream_t st) {
+    const int64_t n = (bytes + 15) / 16, most = xtab && (int64_t)rows * (D / 8) > n ? (int64_t)rows * (D / 8) : n, blocks = (most + 1023) / 1024;
+    return launch_chained(D == 128 ? bwd_clear_kernel<128> : bwd_clear_kernel<64>, dim3((unsigned)(blocks < 148 * 8 ? blocks : 148 * 8)), dim3(256), 0, st,
+                          static_cast<uint4*>(p), n, static_cast<const __half*>(tab), static_cast<uint4*>(xtab), xtab ? rows : 0);
 }
 // Ahead of the first pass, bp.range being zero: clears `zero_bytes` of accumulators (a multiple of 256, or none) and finds the range of
 // 16-bit operands (split ones have factors per group).
 int launch_bwd_begin(const BwdParams& bp, int dtype, void* zero, int64_t zero_bytes, cudaStream_t st) {
-    if (pack_split(dtype, bp.a.K)) return zero_bytes ? launch_bwd_clear(zero, zero_bytes, st) : 0;
+    if (pack_split(dtype, bp.a.K)) return zero_bytes ? launch_bwd_clear(zero, zero_bytes, nullptr, nullptr, 0, bp.a.K, st) : 0;
     return dtype == HTREE_BF16 ? launch_range_t<__nv_bfloat16>(bp, zero, zero_bytes, st) : launch_range_t<__half>(bp, zero, zero_bytes, st);
 }
 

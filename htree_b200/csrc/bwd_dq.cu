@@ -15,6 +15,9 @@ namespace htree {
 
 template <int D, bool X3, int PK>
 constexpr int dq_stages() { return D * (X3 ? 2 : 1) >= 128 ? 2 : PK > 1 ? 2 : 3; }     // slots of 8 KB: warps matter more than depth
+// A slot: the keys with their table rows, 16-bit: those rows in lane order too (bwd_tform.cuh), the values.
+template <int D, bool X3, int CR, int PK>
+constexpr int dq_values() { using C = TForm<D, X3, CR, PK>; return C::KSLOT + (X3 ? 0 : C::NTAB * C::TAB); }
 // Warps per block and blocks per SM: registers first.  The ring takes nearly all of the SM's L1, so anything that spills is
 // re-read from L2 in every chunk: with 180 bytes of spills, groups of 16 heads of 128 spent 4.6 of 9.4 cycles per instruction
 // waiting for it.  Those run as blocks of one warp (at most 20 bytes of spills at 12 warps per SM; the compiler keeps 150 in larger
@@ -39,7 +42,8 @@ __global__ void __launch_bounds__(dq_warps<D, X3, NH>() * 32, dq_min_blocks<D, X
     using FS = Frag<__half>;
     constexpr int KS = C::KS, PPT = C::PPT, PPC = C::PPC, HALF = C::HALF, GP = QC::GP;
     constexpr int NSTG = dq_stages<D, X3, PK>();
-    using Ring = WarpRing<NSTG, C::KSLOT + C::VSLOT>;
+    using Ring = WarpRing<NSTG, dq_values<D, X3, CR, PK>() + C::VSLOT>;
+    constexpr int VOFF = dq_values<D, X3, CR, PK>();
     extern __shared__ __align__(128) unsigned char smem_raw[];
     const AttnParams& p = bp.a;
 
@@ -236,18 +240,31 @@ __global__ void __launch_bounds__(dq_warps<D, X3, NH>() * 32, dq_min_blocks<D, X
             const uint32_t vstride = (uint32_t)p.Hkv * PB;
             if constexpr (PK == 1) p0 = par[c * PPC];
             ring.template copy<PB>(0, kblk + (uint64_t)(uint32_t)p0 * kstride, lane);
-            ring.template copy<PB>(C::KSLOT, vblk + (uint64_t)(uint32_t)p0 * vstride, lane);
+            ring.template copy<PB>(VOFF, vblk + (uint64_t)(uint32_t)p0 * vstride, lane);
             if constexpr (CR == 8) {
                 const int p1 = c * PPC + 1 < np ? par[c * PPC + 1] : p0;
                 ring.template copy<PB>(C::PB, kblk + (uint64_t)(uint32_t)p1 * kstride + 2 * C::ODD, lane);
-                ring.template copy<PB>(C::KSLOT + C::PB, vblk + (uint64_t)(uint32_t)p1 * vstride, lane);
+                ring.template copy<PB>(VOFF + C::PB, vblk + (uint64_t)(uint32_t)p1 * vstride, lane);
                 if constexpr (X3) ring.template copy<16>(C::DATA + 16, kblk + (uint64_t)(uint32_t)p1 * kstride + C::FACS_OFF, lane);
             }
             if constexpr (X3) ring.template copy<16>(C::DATA, kblk + (uint64_t)(uint32_t)p0 * kstride + C::FACS_OFF, lane);
-            if constexpr (PK > 1) { copy_tab_rows<PK, C::TAB>(ring, C::TAB_OFF, p.tab, c, lane); return; }
-            const unsigned char* row = reinterpret_cast<const unsigned char*>(p.tab) + (uint32_t)(rp - 16 * c) * C::TAB;
-            ring.template copy<C::TAB>(C::TAB_OFF, row, lane);
-            if constexpr (C::DUAL) ring.template copy<C::TAB>(C::TAB_OFF + C::TAB, rp - 16 * c >= 8 ? row - 8 * C::TAB : row, lane);
+            if constexpr (X3) {
+                if constexpr (PK > 1) copy_tab_rows<PK, C::TAB>(ring, C::TAB_OFF, p.tab, c, lane);
+                else ring.template copy<C::TAB>(C::TAB_OFF, reinterpret_cast<const unsigned char*>(p.tab) + (uint32_t)(rp - 16 * c) * C::TAB, lane);
+            } else {
+                // the rows for the scores, then those in lane order for dq, in as few instructions as they fit
+                constexpr int PER = C::TAB / 16;
+                const int d0 = PK > 1 ? c : rp - 16 * c, d1 = C::DUAL && d0 >= 8 ? d0 - 8 : d0;
+#pragma unroll
+                for (int i = 0; i < 2 * C::NTAB * PER; i += 32) {
+                    const int piece = i + lane, k = piece / PER, j = k % C::NTAB;
+                    const int row = PK > 1 ? __shfl_sync(0xffffffffu, d0, j) : j ? d1 : d0;
+                    const unsigned char* from = k < C::NTAB ? reinterpret_cast<const unsigned char*>(p.tab) : bp.xtab;
+                    if (2 * C::NTAB * PER % 32 == 0 || piece < 2 * C::NTAB * PER)
+                        asm volatile("cp.async.cg.shared.global [%0], [%1], 16;\n" ::"r"(ring.fill + C::TAB_OFF + 16 * piece),
+                                     "l"(from + (uint32_t)row * C::TAB + 16 * (piece % PER)) : "memory");
+                }
+            }
         };
         ring.start();
         // this visit's place in its parent's list
@@ -342,7 +359,7 @@ __global__ void __launch_bounds__(dq_warps<D, X3, NH>() * 32, dq_min_blocks<D, X
                 any = mask != 0u;
             }
             const uint32_t slot = ring.wait();
-            const LaneBase<D, X3, CR> lb(slot, slot + C::KSLOT, lane);
+            const LaneBase<D, X3, CR> lb(slot, slot + VOFF, lane);
             const uint32_t tabs = slot + C::TAB_OFF;
 
             uint32_t pw[NH][2], sw[NH][2], pwl[X3 ? NH : 1][2], swl[X3 ? NH : 1][2];   // P^T, dS^T: word w = child g + 8w, heads 2r, 2r+1
@@ -411,44 +428,29 @@ __global__ void __launch_bounds__(dq_warps<D, X3, NH>() * 32, dq_min_blocks<D, X
                 }
                 // dq^T += K~^T dS^T: transposed key fragments (rows x(ks, g)), rotated back by the chunk's distance
                 if constexpr (!X3) {
-                    const uint32_t sel = (g & 1) ? 0x3232u : 0x1010u;
-                    const uint32_t tb = tabs + 2 * PPT * (g >> 1) + tab_of_pair;
+                    const uint32_t tx = tabs + (C::NTAB * C::TAB + 2 * KS * (4 * (g & 1) + (g >> 1))) + tab_of_pair;
+                    uint32_t cw[KS / 2], sn[KS / 2], cv[C::DUAL ? KS / 2 : 1], sv[C::DUAL ? KS / 2 : 1];      // (cv, sv: the odd parent's distance)
+                    lds_x<D>(tx, cw, sn);
+                    if constexpr (C::DUAL) lds_x<D>(tx + C::TAB, cv, sv);
 #pragma unroll
-                    for (int k4 = 0; k4 < KS; k4 += 4) {
-                        const uint4 c4 = lds_u4(tb + 4 * k4), s4 = lds_u4(tb + 2 * HALF + 4 * k4);
-                        const uint32_t cw[4] = {c4.x, c4.y, c4.z, c4.w}, snw[4] = {s4.x, s4.y, s4.z, s4.w};
-                        uint32_t cv[4], snv[4];                  // the odd parent's distance
-                        if constexpr (C::DUAL) {
-                            const uint4 d4 = lds_u4(tb + C::TAB + 4 * k4), t4 = lds_u4(tb + C::TAB + 2 * HALF + 4 * k4);
-                            cv[0] = d4.x; cv[1] = d4.y; cv[2] = d4.z; cv[3] = d4.w;
-                            snv[0] = t4.x; snv[1] = t4.y; snv[2] = t4.z; snv[3] = t4.w;
-                        }
+                    for (int ks = 0; ks < KS; ++ks) {
+                        uint32_t m[4], a[4];
+                        key_frag_trans<D, X3, CR>(lb, 0, ks, m);
+                        const __half2 c2 = half_of(cw[ks / 2], ks & 1), s2 = half_of(sn[ks / 2], ks & 1);
+                        if constexpr (SUMS) {            // the chunk's sums are rotated, in fp32
+                            const uint32_t am[4] = {m[0], m[2], m[1], m[3]};
+                            const float cf = __low2float(c2), sf = __low2float(s2);
+                            float acc[4];
+                            mma_zero<__half>(acc, am, db[0][0], db[0][1]);
 #pragma unroll
-                        for (int u = 0; u < 4; ++u) {
-                            const int ks = k4 + u;
-                            uint32_t m[4], a[4];
-                            key_frag_trans<D, X3, CR>(lb, 0, ks, m);
-                            const uint32_t cc = __byte_perm(cw[u], cw[u], sel), ss = __byte_perm(snw[u], snw[u], sel);
-                            if constexpr (SUMS) {            // the chunk's sums are rotated, in fp32
-                                const uint32_t am[4] = {m[0], m[2], m[1], m[3]};
-                                const float cf = __low2float(as_h2(cc)), sf = __low2float(as_h2(ss));
-                                float acc[4];
-                                mma_zero<__half>(acc, am, db[0][0], db[0][1]);
-#pragma unroll
-                                for (int e = 0; e < 2; ++e) {
-                                    dq[0][ks][e] = fmaf(acc[2 + e], sf, fmaf(acc[e], cf, dq[0][ks][e]));
-                                    dq[0][ks][2 + e] = fmaf(acc[e], -sf, fmaf(acc[2 + e], cf, dq[0][ks][2 + e]));
-                                }
-                                continue;
+                            for (int e = 0; e < 2; ++e) {
+                                dq[0][ks][e] = fmaf(acc[2 + e], sf, fmaf(acc[e], cf, dq[0][ks][e]));
+                                dq[0][ks][2 + e] = fmaf(acc[e], -sf, fmaf(acc[2 + e], cf, dq[0][ks][2 + e]));
                             }
-                            const uint32_t ns = neg_h2(ss);                    // inverse rotation
-                            rotate_h2(m[0], m[2], cc, ns, ss, a[0], a[1]);
-                            if constexpr (C::DUAL) {
-                                const uint32_t c2 = __byte_perm(cv[u], cv[u], sel), s2 = __byte_perm(snv[u], snv[u], sel);
-                                rotate_h2(m[1], m[3], c2, neg_h2(s2), s2, a[2], a[3]);
-                            } else {
-                                rotate_h2(m[1], m[3], cc, ns, ss, a[2], a[3]);
-                            }
+                        } else {
+                            rotate_x<true>(m[0], m[2], c2, s2, a[0], a[1]);
+                            if constexpr (C::DUAL) rotate_x<true>(m[1], m[3], half_of(cv[ks / 2], ks & 1), half_of(sv[ks / 2], ks & 1), a[2], a[3]);
+                            else rotate_x<true>(m[1], m[3], c2, s2, a[2], a[3]);
 #pragma unroll
                             for (int h = 0; h < NH; ++h) mma_acc<__half>(dq[h][ks], a, db[h][0], db[h][1]);
                         }
@@ -580,7 +582,7 @@ __global__ void __launch_bounds__(dq_warps<D, X3, NH>() * 32, dq_min_blocks<D, X
 template <typename T, int D, bool X3, int NH, int CR, int PK, bool SUMS>
 static int launch_dq_warps(const BwdParams& bp, cudaStream_t st) {
     using C = TForm<D, X3, CR, PK>;
-    using Ring = WarpRing<dq_stages<D, X3, PK>(), C::KSLOT + C::VSLOT>;
+    using Ring = WarpRing<dq_stages<D, X3, PK>(), dq_values<D, X3, CR, PK>() + C::VSLOT>;
     const size_t per_warp = walk_warp_bytes<Ring, PK>(walk_layout(bp.a, CR));
     constexpr int max_w = dq_warps<D, X3, NH>(), max_warps = max_w * dq_min_blocks<D, X3, NH>();
     int W = 1, best = 0;

@@ -48,6 +48,7 @@ struct BwdParams {
     unsigned char* dob;                      // blocked output gradients [group][half]
     unsigned char* stp;                      // P  [group * MV + visit][half]
     unsigned char* sts;                      // dS
+    const unsigned char* xtab;               // 16-bit: the rotary table by dimensions of a lane (x_index), [distance][cos | sin]
     uint32_t* range;                         // 16-bit: bits of the largest |dO|_1 of a row, and of every unit's largest |v|; else unused
     float2* fac;                             // split-half: {dK, dV} factors of the visits of a group and level, [group * L + level]; else NULL
     int32_t* rank;                           // [group * MV + visit], or
@@ -62,6 +63,36 @@ struct BwdParams {
     float* accv[HTREE_MAX_LEVELS];
 };
 
+// Products over heads or children put dims x = PPT (g / 2) + 2 ks + (g & 1) on the rows of lane (g, *): a lane needs KS cosines and sines
+// that the table has in twice as many words, interleaved with its neighbour's.  Rows in lane order (written once per backward, a row per
+// distance) are half the shared-memory reads, and which half of a word is used is known to the compiler, whose packed multiply-adds
+// broadcast it: no permutes.
+template <int D>
+__host__ __device__ constexpr int x_index(int i) {                  // the dimension at place i of a row's cosines (or sines)
+    constexpr int KS = D / 16, PPT = D / 8;
+    return PPT * ((i / KS) & 3) + 2 * (i % KS) + i / (4 * KS);
+}
+// this lane's words: KS halves of cosines at `at`, of sines D bytes behind
+template <int D>
+__device__ __forceinline__ void lds_x(uint32_t at, uint32_t (&c)[D / 32], uint32_t (&s)[D / 32]) {
+    if constexpr (D == 128) {
+        const uint4 a = lds_u4(at), b = lds_u4(at + D);
+        c[0] = a.x; c[1] = a.y; c[2] = a.z; c[3] = a.w;
+        s[0] = b.x; s[1] = b.y; s[2] = b.z; s[3] = b.w;
+    } else {
+        static_assert(D == 64, "16-bit operands of 64 or 128 dims");
+        asm("ld.shared.v2.b32 {%0,%1}, [%2];\n" : "=r"(c[0]), "=r"(c[1]) : "r"(at));
+        asm("ld.shared.v2.b32 {%0,%1}, [%2];\n" : "=r"(s[0]), "=r"(s[1]) : "r"(at + D));
+    }
+}
+__device__ __forceinline__ __half2 half_of(uint32_t w, int odd) { return odd ? __high2half2(as_h2(w)) : __low2half2(as_h2(w)); }
+// (lo, hi) rotated by the angle (c, s) or, BACK, by its opposite; the roundings of rotate_h2
+template <bool BACK>
+__device__ __forceinline__ void rotate_x(uint32_t lo, uint32_t hi, __half2 c, __half2 s, uint32_t& x, uint32_t& y) {
+    x = as_u32(__hfma2(as_h2(lo), c, __hmul2(as_h2(hi), BACK ? s : __hneg2(s))));
+    y = as_u32(__hfma2(as_h2(hi), c, __hmul2(as_h2(lo), BACK ? __hneg2(s) : s)));
+}
+
 // The power of two that 16-bit dS is carried with, in steps of 2^4: brings |P (dP - D)| <= 2 max|dO|_1 max|v| below 2^15.
 __device__ __forceinline__ float ds_scale(uint32_t dO_l1, uint32_t v) {
     const int e = 393 - (int)(dO_l1 >> 23) - (int)(v >> 23);
@@ -72,7 +103,7 @@ int launch_bwd_begin(const BwdParams& bp, int dtype, void* zero, int64_t zero_by
 int launch_bwd_dq(const BwdParams& bp, int dtype, cudaStream_t st);
 int launch_bwd_dkv(const BwdParams& bp, int dtype, cudaStream_t st);
 int launch_bwd_fold(const BwdParams& bp, int dtype, void* dk, void* dv, bool typed, cudaStream_t st);
-int launch_bwd_clear(void* p, int64_t bytes, cudaStream_t st);
+int launch_bwd_clear(void* p, int64_t bytes, const void* tab, void* xtab, int rows, int D, cudaStream_t st);
 
 template <int D, bool X3, int NH, int CR>
 struct BForm {

@@ -239,10 +239,9 @@ __device__ __forceinline__ void load_query(Row row, int r, float scale, QueryReg
 // B fragments of k-step ks: the query rotated by the chunk's distance.  `tab` is the chunk's table row in shared memory.
 __device__ __forceinline__ __half2 as_h2(uint32_t x) { return *reinterpret_cast<const __half2*>(&x); }
 __device__ __forceinline__ uint32_t as_u32(__half2 x) { return *reinterpret_cast<const uint32_t*>(&x); }
-__device__ __forceinline__ uint32_t neg_h2(uint32_t x) { return x ^ 0x80008000u; }
-// (lo, hi) rotated by (c, s), ns = -s: lo*c - hi*s, lo*s + hi*c, four packed instructions
-__device__ __forceinline__ void rotate_h2(uint32_t lo, uint32_t hi, uint32_t c, uint32_t s, uint32_t ns, uint32_t& x, uint32_t& y) {
-    x = as_u32(__hfma2(as_h2(lo), as_h2(c), __hmul2(as_h2(hi), as_h2(ns))));
+// (lo, hi) rotated by (c, s): lo*c - hi*s, lo*s + hi*c, four packed instructions (which negate an operand for nothing)
+__device__ __forceinline__ void rotate_h2(uint32_t lo, uint32_t hi, uint32_t c, uint32_t s, uint32_t& x, uint32_t& y) {
+    x = as_u32(__hfma2(as_h2(lo), as_h2(c), __hmul2(as_h2(hi), __hneg2(as_h2(s)))));
     y = as_u32(__hfma2(as_h2(hi), as_h2(c), __hmul2(as_h2(lo), as_h2(s))));
 }
 
@@ -271,16 +270,15 @@ __device__ __forceinline__ void score16(const LaneBase<D, false, CR>& s, uint32_
             const int ks = k4 + u;
             uint32_t a[4];
             key_frag<D, false, CR>(s, 0, ks, a);
-            const uint32_t ns = neg_h2(sn[u]);
 #pragma unroll
             for (int h = 0; h < NH; ++h) {
                 uint32_t b0, b1;
-                rotate_h2(q.v[h][0][ks], q.v[h][1][ks], c[u], sn[u], ns, b0, b1);
+                rotate_h2(q.v[h][0][ks], q.v[h][1][ks], c[u], sn[u], b0, b1);
                 float (&acc)[4] = TWO && (ks & 1) ? U[TWO ? h : 0] : S[h];
                 if (ks < (TWO ? 2 : 1)) mma_zero<__half>(acc, a, b0, b1);
                 else mma_acc<__half>(acc, a, b0, b1);
                 if constexpr (DUAL) {
-                    rotate_h2(q.v[h][0][ks], q.v[h][1][ks], c2[u], sn2[u], neg_h2(sn2[u]), b0, b1);
+                    rotate_h2(q.v[h][0][ks], q.v[h][1][ks], c2[u], sn2[u], b0, b1);
                     if (ks == 0) mma_zero<__half>(U[DUAL ? h : 0], a, b0, b1);
                     else mma_acc<__half>(U[DUAL ? h : 0], a, b0, b1);
                 }

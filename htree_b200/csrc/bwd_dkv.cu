@@ -64,18 +64,15 @@ __global__ void __launch_bounds__(256) bwd_range_kernel(const __grid_constant__ 
     }
 }
 
-// One block per window: exclusive prefix sums over the parents of their visits and of their work items (pieces of at most `seg`
-// visits of one parent).  The items themselves are written by the next kernel: one block that wrote them all took 80 us where
-// parents have thousands of visits (12000 positions, 512 nodes per layer).
-__global__ void __launch_bounds__(1024) bwd_scan_kernel(const __grid_constant__ BwdParams bp) {
-    chain_enter();
-    __shared__ int2 wsum[32];
-    const int sub = blockIdx.x, tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-    const int32_t* cnt = bp.cnt + (int64_t)sub * bp.NK;
-    int2* base = bp.base + (int64_t)sub * bp.NK;
-    const int per = (bp.NK + 1023) / 1024, k0 = tid * per, k1 = min(bp.NK, k0 + per);
+// Exclusive prefix sums over a window's parents of their visits and of their work items (pieces of at most `seg` visits of one parent), by
+// the NTH threads of a block; returns the number of items.
+template <int NTH>
+__device__ __forceinline__ int scan_parents(const int32_t* cnt, int2* base, int NK, int seg) {
+    __shared__ int2 wsum[NTH / 32];
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    const int per = (NK + NTH - 1) / NTH, k0 = tid * per, k1 = min(NK, k0 + per);
     int2 s = make_int2(0, 0);
-    for (int k = k0; k < k1; ++k) { const int c = cnt[k]; s.x += c; s.y += (c + bp.seg - 1) / bp.seg; }
+    for (int k = k0; k < k1; ++k) { const int c = cnt[k]; s.x += c; s.y += (c + seg - 1) / seg; }
     int2 inc = s;
 #pragma unroll
     for (int o = 1; o < 32; o <<= 1) {
@@ -86,21 +83,42 @@ __global__ void __launch_bounds__(1024) bwd_scan_kernel(const __grid_constant__ 
     __syncthreads();
     int2 before = make_int2(inc.x - s.x, inc.y - s.y);
     int total = 0;
-    for (int w = 0; w < 32; ++w) {
+    for (int w = 0; w < NTH / 32; ++w) {
         if (w < warp) { before.x += wsum[w].x; before.y += wsum[w].y; }
         total += wsum[w].y;
     }
     for (int k = k0; k < k1; ++k) {
         const int c = cnt[k];
         base[k] = before;
-        before.x += c; before.y += (c + bp.seg - 1) / bp.seg;
+        before.x += c; before.y += (c + seg - 1) / seg;
     }
-    if (tid == 0) bp.nitems[sub] = total;
+    return total;
+}
+// One block per window.  The items themselves are written by the next kernel: one block that wrote them all took 80 us where
+// parents have thousands of visits (12000 positions, 512 nodes per layer).
+__global__ void __launch_bounds__(1024) bwd_scan_kernel(const __grid_constant__ BwdParams bp) {
+    chain_enter();
+    const int sub = blockIdx.x;
+    const int total = scan_parents<1024>(bp.cnt + (int64_t)sub * bp.NK, bp.base + (int64_t)sub * bp.NK, bp.NK, bp.seg);
+    if (threadIdx.x == 0) bp.nitems[sub] = total;
+}
+// Few parents and few blocks that need their sums: every block of the fill kernel makes them for itself, a launch less.
+constexpr int kOwnScan = 1024;
+template <bool OWN>
+__device__ __forceinline__ const int2* window_base(const BwdParams& bp) {
+    if constexpr (!OWN) return bp.base + (int64_t)blockIdx.y * bp.NK;
+    __shared__ int2 own[kOwnScan];
+    const int total = scan_parents<256>(bp.cnt + (int64_t)blockIdx.y * bp.NK, own, bp.NK, bp.seg);
+    if (blockIdx.x == 0 && threadIdx.x == 0) bp.nitems[blockIdx.y] = total;
+    __syncthreads();
+    return own;
 }
 
 // One warp per group: every visit's entry goes to its place in its parent's list; the first visit of an item writes the item.
+template <bool OWN>
 __global__ void __launch_bounds__(256) bwd_fill_kernel(const __grid_constant__ BwdParams bp) {
     chain_enter();
+    const int2* sums = window_base<OWN>(bp);
     const AttnParams& p = bp.a;
     const int lane = threadIdx.x & 31, qi = (int)((blockIdx.x * blockDim.x + threadIdx.x) >> 5);
     const int sub = bp.sub0 + blockIdx.y, unit = sub / bp.nw;
@@ -120,7 +138,7 @@ __global__ void __launch_bounds__(256) bwd_fill_kernel(const __grid_constant__ B
         np = __reduce_add_sync(0xffffffffu, np);
         const int rp = (np - 1) * CR + (int)(((int64_t)t / p.lpow[l]) % CR);
         if (np <= 0 || (l > 0 && rp + 1 <= TK)) continue;
-        const int2* base = bp.base + (int64_t)blockIdx.y * bp.NK + bp.koff[l];
+        const int2* base = sums + bp.koff[l];
         const int32_t* cnt = bp.cnt + (int64_t)blockIdx.y * bp.NK + bp.koff[l];
         for (int i = lane; i < np; i += 32) {
             int x = load_parent(p, l, qidx * TK + i);
@@ -141,8 +159,10 @@ __global__ void __launch_bounds__(256) bwd_fill_kernel(const __grid_constant__ B
 }
 
 // The same for groups of several queries, whose visits the first pass has listed.
+template <bool OWN>
 __global__ void __launch_bounds__(256) bwd_fill_many_kernel(const __grid_constant__ BwdParams bp) {
     chain_enter();
+    const int2* sums = window_base<OWN>(bp);
     const AttnParams& p = bp.a;
     const int lane = threadIdx.x & 31, gi = (int)((blockIdx.x * blockDim.x + threadIdx.x) >> 5);
     if (gi >= bp.ng || ((bp.sub0 + (int)blockIdx.y) % bp.nw) * bp.subq + gi * bp.PK >= p.Tq) return;
@@ -151,7 +171,7 @@ __global__ void __launch_bounds__(256) bwd_fill_many_kernel(const __grid_constan
     for (int l = p.L - 1; l >= 0; --l) {
         if (bp.voff[l] < 0) continue;
         const int n = bp.nvis[grp * p.L + l];
-        const int2* base = bp.base + (int64_t)blockIdx.y * bp.NK + bp.koff[l];
+        const int2* base = sums + bp.koff[l];
         const int32_t* cnt = bp.cnt + (int64_t)blockIdx.y * bp.NK + bp.koff[l];
         for (int i = lane; i < n; i += 32) {
             const int64_t v = grp * bp.MV + bp.voff[l] + i;
@@ -172,7 +192,7 @@ __global__ void __launch_bounds__(256) bwd_fill_many_kernel(const __grid_constan
 // dK' (KEYS) or dV of one item: dX^T[dims x children] += A[dims x heads] B[heads x children] over its visits, 16 rows (heads) a
 // step: one visit of up to 16 heads, or two visits of up to 8.  A = the blocked queries rotated by the visit's distance, or the
 // blocked output gradients; B = dS or P as the first pass left them.  One warp per item, operands through the warp's ring.
-// The two gradients are separate launches: each gathers from one blocked tensor only (a window of it stays in L2) and its
+// The two gradients are one after the other: each gathers from one blocked tensor only (a window of it stays in L2) and its
 // accumulator is 64 registers, which leaves room for 12 and more warps per SM.  Bound by that gather: 14 TB/s of a measured 20.
 // Ring depth: three slots; two where that lets more blocks share an SM and they are the faster choice: split-half, and the keys of
 // groups of 9 to 16 heads of 128 (65536 positions, 64 heads: 13.2 -> 12.4 ms; with 8 heads a group three slots keep a lead of 1%).
@@ -184,7 +204,7 @@ template <int D, bool X3, int CR, bool KEYS>
 constexpr int dkv_min_blocks() { return X3 ? (D == 128 ? 2 : !KEYS && (D == 32 || CR == 8) ? 6 : 3) : D == 128 ? 3 : 4; }
 
 template <typename T, int D, bool X3, int NH, int CR, bool KEYS, int PK>
-__global__ void __launch_bounds__(128, dkv_min_blocks<D, X3, CR, KEYS>()) bwd_dkv_kernel(const __grid_constant__ BwdParams bp) {
+__device__ __forceinline__ void dkv_item(const BwdParams& bp) {
     using BF = BForm<D, X3, NH, CR>;
     using C = TForm<D, X3, CR>;
     using FT = typename std::conditional<X3 || KEYS, __half, T>::type;      // operand type of the products
@@ -196,7 +216,6 @@ __global__ void __launch_bounds__(128, dkv_min_blocks<D, X3, CR, KEYS>()) bwd_dk
     constexpr int PLANE = NT * 128;                                         // bytes from the hi to the lo words of a record
     using Ring = WarpRing<NSTG, SLOT>;
     extern __shared__ __align__(128) unsigned char smem_raw[];
-    chain_enter();
     const AttnParams& p = bp.a;
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, g = lane >> 2;
     const int it = blockIdx.x * (blockDim.x >> 5) + warp, ls = blockIdx.y;
@@ -381,6 +400,19 @@ __global__ void __launch_bounds__(128, dkv_min_blocks<D, X3, CR, KEYS>()) bwd_dk
         for (int n = 0; n < NT; ++n) red_add_v4(dst + (i * NT + n) * 128, acc[i][n][0] * post, acc[i][n][1] * post, acc[i][n][2] * post, acc[i][n][3] * post);
 }
 
+template <typename T, int D, bool X3, int NH, int CR, bool KEYS, int PK>
+__global__ void __launch_bounds__(128, dkv_min_blocks<D, X3, CR, KEYS>()) bwd_dkv_kernel(const __grid_constant__ BwdParams bp) {
+    chain_enter();
+    dkv_item<T, D, X3, NH, CR, KEYS, PK>(bp);
+}
+// dK, then dV, of the 16-bit types in one launch: the same warps fit an SM for either, and the one's last blocks run beside the other's first.
+template <typename T, int D, int NH, int CR, int PK>
+__global__ void __launch_bounds__(128, dkv_min_blocks<D, false, CR, true>()) bwd_dkv_both_kernel(const __grid_constant__ BwdParams bp) {
+    chain_enter();
+    if (blockIdx.z == 0) dkv_item<T, D, false, NH, CR, true, PK>(bp);
+    else dkv_item<T, D, false, NH, CR, false, PK>(bp);
+}
+
 // Accumulators to the leaves' gradients: dK' rotated back by the child index, plus the mean-pool shares of the ancestors' gradients
 // (src/backward.py:787-841), which every block of leaves sums up for itself from the top: a row of D per level, where a launch per
 // level would wait for the one before.  blockIdx.y: 0 = dK, 1 = dV; one warp per block of leaves.
@@ -481,27 +513,41 @@ __global__ void __launch_bounds__(128) bwd_fold_kernel(const __grid_constant__ F
     }
 }
 
+template <int D, bool X3, int NH, int CR, bool KEYS, int PK>
+constexpr size_t dkv_smem() {
+    using BF = BForm<D, X3, NH, CR>;
+    return 4 * WarpRing<dkv_stages<D, X3, NH, KEYS>(), 2 * BF::QB + 2 * BF::SB + (KEYS ? 2 * PK * TForm<D, X3, CR>::TAB : 0)>::kBytes;
+}
 template <typename T, int D, bool X3, int NH, int CR, bool KEYS, int PK>
 static int launch_dkv_one(const BwdParams& bp, cudaStream_t st) {
-    using BF = BForm<D, X3, NH, CR>;
-    constexpr int SLOT = 2 * BF::QB + 2 * BF::SB + (KEYS ? 2 * PK * TForm<D, X3, CR>::TAB : 0);
-    using Ring = WarpRing<dkv_stages<D, X3, NH, KEYS>(), SLOT>;
-    const size_t smem = 4 * Ring::kBytes;
+    constexpr size_t smem = dkv_smem<D, X3, NH, CR, KEYS, PK>();
     auto* k = bwd_dkv_kernel<T, D, X3, NH, CR, KEYS, PK>;
     static SmemLimit shared;
     const cudaError_t e = shared.raise((const void*)k, smem);
     if (e != cudaSuccess) return (int)e;
     return launch_chained(k, dim3((bp.cap + 3) / 4, bp.nsub), dim3(128), smem, st, bp);
 }
+template <typename T, int D, bool X3, int NH, int CR, int PK>
+static int launch_dkv_pk(const BwdParams& bp, cudaStream_t st) {
+    if constexpr (X3) {
+        const int rc = launch_dkv_one<T, D, X3, NH, CR, true, PK>(bp, st);
+        return rc ? rc : launch_dkv_one<T, D, X3, NH, CR, false, (PK > 1 ? 2 : 1)>(bp, st);
+    } else {
+        constexpr size_t k = dkv_smem<D, X3, NH, CR, true, PK>(), v = dkv_smem<D, X3, NH, CR, false, PK>(), smem = k > v ? k : v;
+        auto* kernel = bwd_dkv_both_kernel<T, D, NH, CR, PK>;
+        static SmemLimit shared;
+        const cudaError_t e = shared.raise((const void*)kernel, smem);
+        if (e != cudaSuccess) return (int)e;
+        return launch_chained(kernel, dim3((bp.cap + 3) / 4, bp.nsub, 2), dim3(128), smem, st, bp);
+    }
+}
 template <typename T, int D, bool X3, int NH, int CR>
 static int launch_dkv_cr(const BwdParams& bp, cudaStream_t st) {
-    int rc;
     if constexpr (NH == 1 && CR == 16) {
-        if (bp.PK == 2) { rc = launch_dkv_one<T, D, X3, NH, CR, true, 2>(bp, st); return rc ? rc : launch_dkv_one<T, D, X3, NH, CR, false, 2>(bp, st); }
-        if (bp.PK == 4) { rc = launch_dkv_one<T, D, X3, NH, CR, true, 4>(bp, st); return rc ? rc : launch_dkv_one<T, D, X3, NH, CR, false, 2>(bp, st); }
+        if (bp.PK == 2) return launch_dkv_pk<T, D, X3, NH, CR, 2>(bp, st);
+        if (bp.PK == 4) return launch_dkv_pk<T, D, X3, NH, CR, 4>(bp, st);
     }
-    rc = launch_dkv_one<T, D, X3, NH, CR, true, 1>(bp, st);
-    return rc ? rc : launch_dkv_one<T, D, X3, NH, CR, false, 1>(bp, st);
+    return launch_dkv_pk<T, D, X3, NH, CR, 1>(bp, st);
 }
 template <typename T, int D, bool X3>
 static int launch_dkv_t(const BwdParams& bp, cudaStream_t st) {
@@ -559,9 +605,11 @@ int launch_bwd_begin(const BwdParams& bp, int dtype, void* zero, int64_t zero_by
 }
 
 int launch_bwd_dkv(const BwdParams& bp, int dtype, cudaStream_t st) {
-    int rc = launch_chained(bwd_scan_kernel, dim3(bp.nsub), dim3(1024), 0, st, bp);
-    if (rc == 0) rc = bp.PK > 1 ? launch_chained(bwd_fill_many_kernel, dim3((bp.ng + 7) / 8, bp.nsub), dim3(256), 0, st, bp)
-                                : launch_chained(bwd_fill_kernel, dim3((bp.subq + 7) / 8, bp.nsub), dim3(256), 0, st, bp);
+    const dim3 grid((bp.ng + 7) / 8, bp.nsub);
+    const bool own = bp.NK <= kOwnScan && (int64_t)grid.x * grid.y <= 148 * 4;
+    int rc = own ? 0 : launch_chained(bwd_scan_kernel, dim3(bp.nsub), dim3(1024), 0, st, bp);
+    if (rc == 0) rc = launch_chained(bp.PK > 1 ? (own ? bwd_fill_many_kernel<true> : bwd_fill_many_kernel<false>) : own ? bwd_fill_kernel<true> : bwd_fill_kernel<false>,
+                                     grid, dim3(256), 0, st, bp);
     if (rc) return rc;
     switch (dtype) {
         case HTREE_F32: return launch_dkv_d<float>(bp, st);

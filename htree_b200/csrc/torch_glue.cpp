@@ -30,10 +30,19 @@ HtreeShape make_shape(const at::Tensor& q, const at::Tensor& k, int64_t cr, int6
     return s;
 }
 
+// One workspace: the plan's, the softmax statistics and the parent lists behind it (an allocation and a saved tensor each cost a
+// microsecond or two of a step).
 struct Forward {
-    at::Tensor out, stats, parents, ws;
+    at::Tensor out, ws;
     HtreePlan plan;
+    int64_t stats, parents;       // where they start
 };
+int64_t up256(int64_t x) { return (x + 255) & ~int64_t(255); }
+void place(Forward& f, const HtreeShape& s, int64_t Tq) {
+    f.stats = up256(f.plan.bytes);
+    f.parents = f.stats + up256(2 * (int64_t)s.B * Tq * s.H * 4);
+}
+int64_t lists(const HtreeShape& s, int64_t Tq) { return (int64_t)s.B * Tq * s.H_kv * s.top_k; }       // entries of a level
 
 // tables: cos, sin, rows of the transposed kernels, rows of the selection kernel, status word
 bool run_forward(const HtreeShape& s, const at::Tensor& q, const at::Tensor& k, const at::Tensor& v, const std::vector<at::Tensor>& tables,
@@ -43,12 +52,12 @@ bool run_forward(const HtreeShape& s, const at::Tensor& q, const at::Tensor& k, 
     if (!save && L * B * Tq * s.H_kv * s.top_k * 4 > budget) return false;
     const auto bytes = at::TensorOptions().device(q.device()).dtype(at::kByte);
     f.out = at::empty(q.sizes(), q.options());
-    f.stats = at::empty({2, B, Tq, H}, bytes.dtype(at::kFloat));
-    f.parents = at::empty({L, B, Tq, s.H_kv, s.top_k}, bytes.dtype(at::kInt));
-    f.ws = at::empty({f.plan.bytes}, bytes);
+    place(f, s, Tq);
+    f.ws = at::empty({f.parents + L * lists(s, Tq) * 4}, bytes);
+    unsigned char* w = static_cast<unsigned char*>(f.ws.data_ptr());
     int32_t* par[HTREE_MAX_LEVELS];
-    for (int64_t l = 0; l < L; ++l) par[l] = f.parents.data_ptr<int32_t>() + l * (B * Tq * s.H_kv * s.top_k);
-    float* gmax = f.stats.data_ptr<float>();
+    for (int64_t l = 0; l < L; ++l) par[l] = reinterpret_cast<int32_t*>(w + f.parents) + l * lists(s, Tq);
+    float* gmax = reinterpret_cast<float*>(w + f.stats);
     check(htree_b200_run_forward(&s, &f.plan, q.data_ptr(), k.data_ptr(), v.data_ptr(), tables[0].data_ptr<float>(), tables[1].data_ptr<float>(),
                                  tables[2].data_ptr(), tables[3].data_ptr(), (int32_t)tables[0].size(0), (float)scale, f.ws.data_ptr(),
                                  f.out.data_ptr(), gmax, gmax + B * Tq * H, par, tables[4].data_ptr<int32_t>(), save ? 0u : HTREE_FWD_INFERENCE,
@@ -64,7 +73,7 @@ struct HTreeNode : public torch::autograd::Function<HTreeNode> {
         const HtreeShape s = make_shape(q, k, cr, mtn, tk, -1);
         Forward f;
         TORCH_CHECK(run_forward(s, q, k, v, tables, scale, true, 0, f), "htree_b200: unsupported shape");
-        ctx->save_for_backward({q, k, v, f.out, f.stats, f.parents, f.ws, tables[0], tables[1], tables[2], tables[4]});
+        ctx->save_for_backward({q, k, v, f.out, f.ws, tables[0], tables[1], tables[2], tables[4]});
         ctx->saved_data["cr"] = cr; ctx->saved_data["mtn"] = mtn; ctx->saved_data["tk"] = tk;
         ctx->saved_data["scale"] = scale; ctx->saved_data["budget"] = budget;
         return f.out;
@@ -72,14 +81,15 @@ struct HTreeNode : public torch::autograd::Function<HTreeNode> {
 
     static variable_list backward(AutogradContext* ctx, variable_list grads) {
         const auto sv = ctx->get_saved_variables();
-        const at::Tensor &q = sv[0], &k = sv[1], &out = sv[3], &stats = sv[4], &parents = sv[5], &ws = sv[6];
+        const at::Tensor &q = sv[0], &k = sv[1], &out = sv[3], &ws = sv[4];
         c10::cuda::CUDAGuard guard(q.device());
         at::Tensor dO = grads[0].to(q.scalar_type()).contiguous();
         if (!aligned(dO, 32)) dO = dO.clone();
         const double scale = ctx->saved_data["scale"].toDouble();
         const int64_t budget = ctx->saved_data["budget"].toInt();
         const HtreeShape s = make_shape(q, k, ctx->saved_data["cr"].toInt(), ctx->saved_data["mtn"].toInt(), ctx->saved_data["tk"].toInt(), -1);
-        HtreePlan plan;
+        Forward f;
+        HtreePlan& plan = f.plan;
         int64_t acc_bytes = 0, scratch_bytes = 0;
         check(htree_b200_plan(&s, HTREE_PLAN_BACKWARD, &plan), "plan");
         check(htree_b200_backward_plan(&s, budget, &acc_bytes, &scratch_bytes), "backward plan");
@@ -89,15 +99,15 @@ struct HTreeNode : public torch::autograd::Function<HTreeNode> {
         void *blk[HTREE_MAX_LEVELS], *bwd[HTREE_MAX_LEVELS];
         int32_t* par[HTREE_MAX_LEVELS];
         unsigned char *w = static_cast<unsigned char*>(ws.data_ptr()), *a = static_cast<unsigned char*>(scratch.data_ptr());
-        const int64_t step = parents.numel() / parents.size(0);
+        place(f, s, q.size(1));
         for (int l = 0; l < plan.levels; ++l) {
             blk[l] = w + plan.blocks[l]; bwd[l] = w + plan.blocks_bwd[l];
-            par[l] = parents.data_ptr<int32_t>() + l * step;
+            par[l] = reinterpret_cast<int32_t*>(w + f.parents) + l * lists(s, q.size(1));
         }
-        const float* gmax = stats.data_ptr<float>();
-        check(htree_b200_run_backward(&s, q.data_ptr(), blk, bwd, sv[7].data_ptr<float>(), sv[8].data_ptr<float>(), sv[9].data_ptr(),
-                                      (int32_t)sv[7].size(0), (float)scale, out.data_ptr(), dO.data_ptr(), gmax, gmax + stats.numel() / 2, par, a,
-                                      a + acc_bytes, budget, dq.data_ptr(), dk.data_ptr(), dv.data_ptr(), 1, sv[10].data_ptr<int32_t>(), 0u,
+        const float* gmax = reinterpret_cast<const float*>(w + f.stats);
+        check(htree_b200_run_backward(&s, q.data_ptr(), blk, bwd, sv[5].data_ptr<float>(), sv[6].data_ptr<float>(), sv[7].data_ptr(),
+                                      (int32_t)sv[5].size(0), (float)scale, out.data_ptr(), dO.data_ptr(), gmax, gmax + (int64_t)s.B * q.size(1) * s.H, par, a,
+                                      a + acc_bytes, budget, dq.data_ptr(), dk.data_ptr(), dv.data_ptr(), 1, sv[8].data_ptr<int32_t>(), 0u,
                                       at::cuda::getCurrentCUDAStream().stream()),
               "backward");
         variable_list r(13);        // q, k, v, then tables and options, which have no gradient

@@ -7,8 +7,8 @@
 // one rotary-table row into its ring in shared memory (asynchronously, NSTG - 1 chunks ahead), forms
 // S^T = K' q^ (one query rotation per chunk), P^T, and O^T += V^T P^T.
 //
-// Bound by the L2 gather of the blocks (14.6 to 17.1 of a measured 20 TB/s) and the shared-memory read pipe (63% busy with 16 heads a
-// group, 76% with 8): without its copies it would take about 80% of its time.  Measured against the kernel that gathers rows with heads on the matrix
+// Bound by the L2 gather of the blocks (14.6 to 17.1 of a measured 20 TB/s) and the shared-memory read pipe (61% busy with 16 heads a
+// group, 82% with 8): without its copies it would take about 80% of its time.  Measured against the kernel that gathers rows with heads on the matrix
 // rows: 4 x 65536 positions, 64 heads of 128: 95 -> 77 ms.  Groups of at most 4 heads leave half of the 8 columns empty: where queries
 // select many of the same parents two or four of them share a warp (tform.cuh): 12000 positions, 16 heads of 32, top_k 512: 5.06 -> 3.32 ms.
 #include "tform.cuh"

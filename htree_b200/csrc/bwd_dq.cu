@@ -6,9 +6,9 @@
 // with K~ = scale R(-distance) K', its fragments transposed by the load: rotated back into the query's frame in registers, or, split-half,
 // dq^T += R(-distance) (K'^T dS^T), which leaves the keys' planes as they are.
 //
-// Bound by the latency of those five products in a row at 12 warps per SM (issue 49%, shared-memory pipe 67%, tensor pipe 38%).
-// 4 x 65536 positions, 64 heads of 128: this pass 137 ms and the parent-stationary one 90 ms, where the single kernel with reductions
-// took 360 ms.
+// Bound by shared-memory reads (69% of the pipe with 16 heads of 128 a group, 83% with 8): values and keys once each, the keys once more
+// transposed, table rows.  4 x 65536 positions, 64 heads of 128: this pass 129 ms and the parent-stationary one 86 ms, where the single
+// kernel with reductions took 360 ms.
 #include "bwd_tform.cuh"
 
 namespace htree {

@@ -6,9 +6,9 @@
 // importance does not depend on which: every chunk is evaluated alike (the query rotated in fp32 and rounded once to half per
 // parent, two accumulation chains, the chunk's own maximum as reference, heads summed in one fixed tree) and the search is exact.
 //
-// Bound by the shared-memory read pipe (76% busy at 8 heads of 128) and latency at 12 to 16 warps per SM; of its time the copies are a
+// Bound by the shared-memory read pipe (61% busy at 8 heads of 128, 76% before the third part of the table rows was left out) and latency at 12 to 16 warps per SM; of its time the copies are a
 // third, the Top-K search and the rotation a tenth each.  Measured against the kernel that gathers rows: 4 x 65536 positions, 64 heads
-// of 128: 49 -> 43.7 ms.
+// of 128: 49 -> 42 ms.
 #include "tform.cuh"
 
 namespace htree {

@@ -600,7 +600,7 @@ static int launch_acc_cr(const AttnParams& p, cudaStream_t st) {
         const int leaf = (p.ln[0] + CR - 1) / CR, chunks = ((p.TK < leaf ? p.TK : leaf) * CR + 15) / 16;
         int CL = 1;
         while (CL < 8 && 2 * CL * groups <= 148 && 2 * CL * kAccSplitWarps * rounds <= chunks) CL *= 2;
-        return launch_chained_clusters(k, CL, dim3(p.Tq * CL, p.B * p.Hkv), dim3(kAccSplitWarps * 32), split_smem, st, p);
+        return launch_clusters(k, CL, dim3(p.Tq, p.B * p.Hkv), dim3(kAccSplitWarps * 32), split_smem, st, p);
     }
     if constexpr (NH == 1 && CR == 16) {
         const int PK = queries_per_warp(CR, p.G, p.TK, (p.ln[0] + CR - 1) / CR, groups);

@@ -111,16 +111,20 @@ static int bwd_layout(const HtreeShape* s, int L, const int32_t* ln, int64_t bud
     // A window's blocked queries (4 KB each at 16 heads of 128) should stay in the L2 while its parents gather them: 8192 queries
     // are 33 MB; longer windows mean longer visit lists and fewer reductions.
     const int64_t xtab = x3 ? 0 : up((int64_t)TK * CR * D * 2);
-    budget -= xtab < budget / 2 ? xtab : budget / 2;
     int64_t subq = 0, ng = 0, bytes = 0;
-    for (int64_t most = 8192; most >= 16; most >>= 1) {
-        const int64_t nw = (Tq + most - 1) / most;
-        subq = ((Tq + nw - 1) / nw + PK - 1) / PK * PK;
-        ng = subq / PK;
-        const int64_t visits = ng * MV;
-        bytes = up(ng * qb) * 2 + up(visits * sb) * 2 + up(visits * (many ? 16 : 4)) + up(visits * entry) + (x3 ? up(ng * L * 8) : 0) + (many ? up(ng * L * 4) : 0) +
-                2 * up(NK * 4) + up((visits / 8 + NK) * 16) + 256;
-        if (bytes <= budget && visits < (int64_t(1) << 31)) { bp.nw = (int32_t)nw; break; }
+    // the table comes out of the buffer's size, or, where no window would fit beside it, on top
+    const int64_t whole = budget;
+    for (budget -= xtab < budget ? xtab : budget;; budget = whole) {
+        for (int64_t most = 8192; most >= 16; most >>= 1) {
+            const int64_t nw = (Tq + most - 1) / most;
+            subq = ((Tq + nw - 1) / nw + PK - 1) / PK * PK;
+            ng = subq / PK;
+            const int64_t visits = ng * MV;
+            bytes = up(ng * qb) * 2 + up(visits * sb) * 2 + up(visits * (many ? 16 : 4)) + up(visits * entry) + (x3 ? up(ng * L * 8) : 0) + (many ? up(ng * L * 4) : 0) +
+                    2 * up(NK * 4) + up((visits / 8 + NK) * 16) + 256;
+            if (bytes <= budget && visits < (int64_t(1) << 31)) { bp.nw = (int32_t)nw; break; }
+        }
+        if (bp.nw || budget == whole) break;
     }
     if (bp.nw == 0) return HTREE_E_SCRATCH;
     bp.subq = (int32_t)subq; bp.ng = (int32_t)ng; bp.MV = (int32_t)MV; bp.NK = (int32_t)NK;

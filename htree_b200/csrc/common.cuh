@@ -145,6 +145,14 @@ int launch_chained_clusters(void (*kernel)(P...), int cluster, dim3 grid, dim3 b
     note_launch();
     return (int)e;
 }
+// ... of `CL` blocks a cluster along x, or, where the device has no room for such a cluster, of one
+template <typename... P>
+int launch_clusters(void (*kernel)(P...), int CL, dim3 grid, dim3 block, size_t smem, cudaStream_t st, const P&... args) {
+    const int rc = launch_chained_clusters(kernel, CL, dim3(grid.x * CL, grid.y), block, smem, st, args...);
+    if (rc == 0 || CL == 1) return rc;
+    cudaGetLastError();
+    return launch_chained_clusters(kernel, 1, grid, block, smem, st, args...);
+}
 template <typename... P>
 int launch_chained(void (*kernel)(P...), dim3 grid, dim3 block, size_t smem, cudaStream_t st, const P&... args) {
     return launch_chained_clusters(kernel, 1, grid, block, smem, st, args...);

@@ -2,12 +2,12 @@
 // selecting half of htree_select_accumulate_gqa_kernel (src/parallel.py:537-867, 1167-1399).  Products, chunks and operand blocks
 // of tform.cuh; writes the parent list that each level consumes.
 //
-// One warp per (batch, query position, KV head) group; with SPLIT the 8 warps of a block, or of up to 8 blocks, share a group's chunks.  A candidate's
-// importance does not depend on which: every chunk is evaluated alike (the query rotated in fp32 and rounded once to half per
+// One warp per (batch, query position, KV head) group; with SPLIT the 8 warps of a block, or of up to 8 blocks, share a group's chunks.
+// A candidate's importance does not depend on which: every chunk is evaluated alike (the query rotated in fp32 and rounded once to half per
 // parent, two accumulation chains, the chunk's own maximum as reference, heads summed in one fixed tree) and the search is exact.
 //
-// Bound by the shared-memory read pipe (61% busy at 8 heads of 128, 76% before the third part of the table rows was left out) and latency at 12 to 16 warps per SM; of its time the copies are a
-// third, the Top-K search and the rotation a tenth each.  Measured against the kernel that gathers rows: 4 x 65536 positions, 64 heads
+// Bound by the shared-memory read pipe (61% busy at 8 heads of 128, 76% before the third part of the table rows was left out) and latency
+// at 12 to 16 warps per SM; of its time the copies are a third, the Top-K search and the rotation a tenth each.  Measured against the kernel that gathers rows: 4 x 65536 positions, 64 heads
 // of 128: 49 -> 42 ms.
 #include "tform.cuh"
 
@@ -411,7 +411,7 @@ static int launch_select_cr(const AttnParams& in, cudaStream_t st) {
         // accumulation alone on clusters a decode call took 63.5 us, with both 60.9.
         int CL = 1;
         while (CL < 8 && 2 * CL * groups <= 148 && 2 * CL * kSelSplitWarps <= maxc / 16) CL *= 2;
-        return launch_chained_clusters(k, CL, dim3(p.Tq * CL, p.B * p.Hkv), dim3(kSelSplitWarps * 32), split_smem, st, p);
+        return launch_clusters(k, CL, dim3(p.Tq, p.B * p.Hkv), dim3(kSelSplitWarps * 32), split_smem, st, p);
     }
     const size_t per_warp = Ring::kBytes + scratch;
     constexpr int max_warps = 4 * sel_min_blocks<D, X3, NH>();

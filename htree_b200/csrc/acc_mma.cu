@@ -24,11 +24,15 @@ namespace htree {
 // heads, 32-wide heads (634 -> 689), fp32 64-wide heads with 16 children (84.5 -> 88.9).
 template <int D, bool X3, int NH, int CR>
 constexpr bool acc_single() { return (D == 128 && (NH == 1 || X3)) || (X3 && D == 64 && NH == 1 && CR == 8); }
+// Groups of up to 8 heads of 64 in 16 bits fit 20 warps, with two slots of 4 KB each: 20000 positions of 4 groups 2045 -> 1947 us, eight
+// children 2513 -> 2470 (32-wide heads, two queries a warp: no change, 385 and 387).
 template <int D, bool X3, int NH, int CR>
-constexpr int acc_stages() { return acc_single<D, X3, NH, CR>() ? 1 : D * (X3 ? 2 : 1) >= 128 ? 2 : 3; }     // slots of 8 KB: warps matter more than depth
+constexpr bool acc_twenty() { return D == 64 && !X3 && NH == 1; }
+template <int D, bool X3, int NH, int CR>
+constexpr int acc_stages() { return acc_single<D, X3, NH, CR>() ? 1 : D * (X3 ? 2 : 1) >= 128 || acc_twenty<D, X3, NH, CR>() ? 2 : 3; }     // slots of 8 KB: warps matter more than depth
 constexpr int kAccWarps = 4, kAccSplitWarps = 8;
 template <int D, bool X3, int NH, int CR>
-constexpr int acc_min_blocks() { return (X3 && D == 128) ? 2 : D == 128 ? (NH == 1 ? 4 : 3) : (X3 && D == 64 && NH == 2) ? 3 : 4; }
+constexpr int acc_min_blocks() { return (X3 && D == 128) ? 2 : D == 128 ? (NH == 1 ? 4 : 3) : (X3 && D == 64 && NH == 2) ? 3 : acc_twenty<D, X3, NH, CR>() ? 5 : 4; }
 // Slots of the warps that share a query: two of 8 KB, three of less, so that two blocks of 64- and 32-wide heads still share an SM (a third
 // slot of 8 KB gave nothing: 28.4 against 29.2 us).
 template <int D, bool X3>

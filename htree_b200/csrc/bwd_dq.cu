@@ -218,6 +218,7 @@ __global__ void __launch_bounds__(dq_warps<D, X3, NH>() * 32, dq_min_blocks<D, X
             for (int j = 0; j < PK; ++j) {
                 if (tl + j >= p.Tq) break;
                 int n = list_of(j).load(p, l, (qidx + (int64_t)j * p.Hkv) * TK, nblk, 8, lane);
+                n = list_of(j).ascending(p, n, 8, lane);
                 const int right = (n - 1) * CR + (int)(((int64_t)(p.t0 + tl + j) / p.lpow[l]) % CR);
                 if (l > 0 && right < TK) n = 0;
                 if (l > 0 && n > 0) {

@@ -443,8 +443,26 @@ struct ParentList {
         if (end > np && p.status) atomicOr(p.status, bit);
         return np;
     }
+    // For a list (of 16-bit entries) that goes into a union of several: strictly ascending from here on, entries that are not above the
+    // one before dropped and reported; returns how many are left.  A union of such lists has no more steps than the level has parents,
+    // which is what its visits' slots are sized for.  Checked once per list: passing over such entries in UnionWalk::step cost the backward 3%.
+    __device__ __forceinline__ int ascending(const AttnParams& p, int np, int bit, int lane) const {
+        uint16_t* x = reinterpret_cast<uint16_t*>(at);
+        __syncwarp();
+        bool bad = false;
+        for (int i = lane + 1; i < np; i += 32) bad |= x[i] <= x[i - 1];
+        if (!__any_sync(0xffffffffu, bad)) return np;
+        int left = 0;
+        if (lane == 0) {
+            for (int i = 0, last = -1; i < np; ++i)
+                if ((int)x[i] > last) { last = x[i]; x[left++] = (uint16_t)last; }
+            if (p.status) atomicOr(p.status, bit);
+        }
+        __syncwarp();
+        return __shfl_sync(0xffffffffu, left, 0);
+    }
 };
-// The union of PK queries' lists (of 16-bit entries), walked in ascending order.  Lane j (mod PK) holds query j's list and place in it.
+// The union of PK queries' ascending lists (of 16-bit entries), walked in that order.  Lane j (mod PK) holds query j's list and place in it.
 template <int PK>
 struct UnionWalk {
     const uint16_t* list;         // of this lane's query

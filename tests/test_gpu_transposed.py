@@ -280,3 +280,48 @@ def test_top_level_in_fp32_arithmetic(dt, D, G, T, TK, MTN, Hkv, CR, clustered):
         assert torch.equal(lists[0][l], lists[1][l]), f"level {l}"
     torch.cuda.synchronize()
     ops.check_status()
+
+
+@pytest.mark.parametrize("dt,D,G,T,TK,MTN,Hkv", [
+    (HF, 32, 4, 1601, 64, 128, 4), (FP, 64, 3, 1600, 64, 128, 4), (BF, 128, 4, 1600, 64, 1024, 2),       # two queries a warp
+    (BF, 64, 1, 1601, 64, 128, 4), (FP, 128, 2, 1603, 64, 128, 4)])                                      # four
+@pytest.mark.parametrize("compact", [False, True])
+def test_malformed_parent_lists_of_queries_that_share_a_warp(dt, D, G, T, TK, MTN, Hkv, compact, monkeypatch):
+    """The union of lists that do not ascend has no more steps than the level has parents (101, where 64 entries of one parent and a
+    neighbour's list would make 127), reports them, and leaves the other queries' gradients as they are."""
+    import htree_b200 as ht
+    from htree_b200 import ops
+    if compact:
+        monkeypatch.setattr(ops, "SELECTION_STORAGE", "uint16")
+    q, k, v, dO = _inputs(dt, 1, T, Hkv, G, D)
+    out, ctx = ht.htree_forward(q, k, v, 16, MTN, TK, _save_for_backward=True)
+    want = ht.htree_backward(dO, q, out, ctx)
+    lists = {l: x.clone() for l, x in ctx["per_layer_parents"].items()}
+    rows = torch.arange(T // 2 | 1, T, 2, device=DEV)        # every other query of the later half: each warp has one as it should be
+    same = torch.ones(T, dtype=torch.bool, device=DEV)
+    same[rows] = False
+
+    def one_parent(x): x[:, rows] = 3
+    def descending(x): x[:, rows] = x[:, rows].flip(-1)
+    def holes(x): x[:, rows, :, 1::2] = -1
+    def first_missing(x): x[:, rows, :, 0] = -1
+    def past_the_end(x): x[:, rows, :, 5] = -2 if compact else 1 << 30
+    def twice(x): x[:, rows, :, 7] = x[:, rows, :, 6]
+    for hurt in (one_parent, descending, holes, first_missing, past_the_end, twice):
+        for levels in ([0], list(range(ctx["num_layers"]))):
+            bad = {l: x.clone() for l, x in lists.items()}
+            for l in levels:
+                hurt(bad[l])
+            ctx["per_layer_parents"] = bad
+            got = ht.htree_backward(dO, q, out, ctx)
+            torch.cuda.synchronize()
+            assert all(x.isfinite().all() for x in got), hurt.__name__
+            assert torch.equal(got[0][:, same], want[0][:, same]), hurt.__name__
+            with pytest.raises(RuntimeError, match="outside its tree level"):
+                ops.check_status()
+    ctx["per_layer_parents"] = {l: x.clone() for l, x in lists.items()}
+    for l in range(ctx["num_layers"]):
+        ctx["per_layer_parents"][l][:, rows] = -1                # no parents at all: nothing to report
+    got = ht.htree_backward(dO, q, out, ctx)
+    assert torch.equal(got[0][:, same], want[0][:, same]) and not got[0][:, rows].any()
+    ops.check_status()

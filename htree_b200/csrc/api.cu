@@ -74,8 +74,8 @@ static int fill_params(AttnParams& p, const HtreeShape* s, int L, const int32_t*
 struct BwdLayout {
     BwdParams bp;
     int64_t acc_bytes, scratch_bytes, zero_bytes;
-    int64_t acck[HTREE_MAX_LEVELS], accv[HTREE_MAX_LEVELS];
-    int64_t o_qb, o_dob, o_stp, o_sts, o_fac, o_rank, o_nvis, o_xtab, o_cnt, o_base, o_entries, o_items, o_nitems;
+    int64_t acck[HTREE_MAX_LEVELS], accv[HTREE_MAX_LEVELS], xtab;      // in the accumulators' buffer; xtab < 0: none
+    int64_t o_qb, o_dob, o_stp, o_sts, o_fac, o_rank, o_nvis, o_cnt, o_base, o_entries, o_items, o_nitems;
     int total, per_launch;
 };
 
@@ -105,31 +105,30 @@ static int bwd_layout(const HtreeShape* s, int L, const int32_t* ln, int64_t bud
         y.accv[l] = at; at += up(blocks * D * CR * 4);
     }
     y.zero_bytes = at;
-    y.acc_bytes = at;
+    // The rotary rows stand behind the accumulators, whose size is no part of the budget: windows of any size of one backward find them
+    // at the same place, and a budget for little more than a window is not taken up by 2 MB of table.
+    y.xtab = x3 ? -1 : at;
+    y.acc_bytes = x3 ? at : at + up((int64_t)TK * CR * D * 2);
     const int64_t qb = (int64_t)NH * D * 16 * (x3 ? 2 : 1), sb = (int64_t)NH * (CR / 8) * 128 * (x3 ? 2 : 1);
     const int64_t entry = x3 ? (many ? sizeof(BwdEntry<true, true>) : sizeof(BwdEntry<true, false>)) : (many ? sizeof(BwdEntry<false, true>) : sizeof(BwdEntry<false, false>));
     // A window's blocked queries (4 KB each at 16 heads of 128) should stay in the L2 while its parents gather them: 8192 queries
     // are 33 MB; longer windows mean longer visit lists and fewer reductions.
-    const int64_t xtab = x3 ? 0 : up((int64_t)TK * CR * D * 2);
     int64_t subq = 0, ng = 0, bytes = 0;
-    // the table comes out of the buffer's size, or, where no window would fit beside it, on top
-    const int64_t whole = budget;
-    for (budget -= xtab < budget ? xtab : budget;; budget = whole) {
-        for (int64_t most = 8192; most >= 16; most >>= 1) {
-            const int64_t nw = (Tq + most - 1) / most;
-            subq = ((Tq + nw - 1) / nw + PK - 1) / PK * PK;
-            ng = subq / PK;
-            const int64_t visits = ng * MV;
-            bytes = up(ng * qb) * 2 + up(visits * sb) * 2 + up(visits * (many ? 16 : 4)) + up(visits * entry) + (x3 ? up(ng * L * 8) : 0) + (many ? up(ng * L * 4) : 0) +
-                    2 * up(NK * 4) + up((visits / 8 + NK) * 16) + 256;
-            if (bytes <= budget && visits < (int64_t(1) << 31)) { bp.nw = (int32_t)nw; break; }
-        }
-        if (bp.nw || budget == whole) break;
+    const int64_t fixed = up(4 + units * 4);                    // besides the windows: the words of the range
+    for (int64_t most = 8192; most >= 8; most >>= 1) {
+        const int64_t nw = (Tq + most - 1) / most;
+        subq = ((Tq + nw - 1) / nw + PK - 1) / PK * PK;
+        ng = subq / PK;
+        const int64_t visits = ng * MV;
+        // of a window; the buffers below hold no more than `per` times that and the words
+        bytes = up(ng * qb) * 2 + up(visits * sb) * 2 + up(visits * (many ? 16 : 4)) + up(visits * entry) + (x3 ? up(ng * L * 8) : 0) + (many ? up(ng * L * 4) : 0) +
+                up(NK * 4) + up(NK * 8) + up((visits / 8 + NK) * (int64_t)sizeof(BwdItem)) + up(4);
+        if (fixed + bytes <= budget && visits < (int64_t(1) << 31)) { bp.nw = (int32_t)nw; break; }
     }
     if (bp.nw == 0) return HTREE_E_SCRATCH;
     bp.subq = (int32_t)subq; bp.ng = (int32_t)ng; bp.MV = (int32_t)MV; bp.NK = (int32_t)NK;
     y.total = (int)(units * bp.nw);
-    int64_t per = budget / bytes;
+    int64_t per = (budget - fixed) / bytes;
     if (per > 32767 / ng) per = 32767 / ng;
     if (per * ng * MV >= (int64_t(1) << 31)) per = ((int64_t(1) << 31) - 1) / (ng * MV);
     if (per > y.total) per = y.total;
@@ -146,7 +145,6 @@ static int bwd_layout(const HtreeShape* s, int L, const int32_t* ln, int64_t bud
     y.o_qb = take(per * ng * qb); y.o_dob = take(per * ng * qb);
     y.o_stp = take(per * ng * MV * sb); y.o_sts = take(per * ng * MV * sb);
     y.o_fac = x3 ? take(per * ng * L * 8) : -1;
-    y.o_xtab = x3 ? -1 : take(xtab);
     y.o_nvis = many ? take(per * ng * L * 4) : -1;
     y.o_rank = take(per * ng * MV * (many ? 16 : 4)); y.o_entries = take(per * ng * MV * entry);
     y.o_cnt = take(cnt_words(per, NK) * 4 + 4 + units * 4); y.o_base = take(per * NK * 8);
@@ -578,7 +576,7 @@ int htree_b200_run_backward(const HtreeShape* shape, const void* q, void* const*
     bp.qb = sb + y.o_qb; bp.dob = sb + y.o_dob; bp.stp = sb + y.o_stp; bp.sts = sb + y.o_sts;
     bp.fac = y.o_fac < 0 ? nullptr : reinterpret_cast<float2*>(sb + y.o_fac);
     bp.rank = reinterpret_cast<int32_t*>(sb + y.o_rank); bp.vis = reinterpret_cast<uint4*>(sb + y.o_rank);
-    bp.xtab = y.o_xtab < 0 ? nullptr : sb + y.o_xtab;
+    bp.xtab = y.xtab < 0 ? nullptr : ab + y.xtab;
     bp.nvis = y.o_nvis < 0 ? nullptr : reinterpret_cast<int32_t*>(sb + y.o_nvis); bp.entries = sb + y.o_entries;
     bp.cnt = reinterpret_cast<int32_t*>(sb + y.o_cnt); bp.range = reinterpret_cast<uint32_t*>(bp.cnt + cnt_words(y.per_launch, bp.NK)); bp.base = reinterpret_cast<int2*>(sb + y.o_base);
     bp.items = reinterpret_cast<BwdItem*>(sb + y.o_items); bp.nitems = reinterpret_cast<int32_t*>(sb + y.o_nitems);

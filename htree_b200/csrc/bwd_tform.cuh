@@ -48,7 +48,7 @@ struct BwdParams {
     unsigned char* dob;                      // blocked output gradients [group][half]
     unsigned char* stp;                      // P  [group * MV + visit][half]
     unsigned char* sts;                      // dS
-    const unsigned char* xtab;               // 16-bit: the rotary table by dimensions of a lane (x_index), [distance][cos | sin]
+    const unsigned char* xtab;               // 16-bit: the rotary table by dimensions of a lane (x_index), [distance][cos | sin], behind the accumulators
     uint32_t* range;                         // 16-bit: bits of the largest |dO|_1 of a row, and of every unit's largest |v|; else unused
     float2* fac;                             // split-half: {dK, dV} factors of the visits of a group and level, [group * L + level]; else NULL
     int32_t* rank;                           // [group * MV + visit], or

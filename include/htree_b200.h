@@ -282,8 +282,8 @@ int htree_b200_backward(const HtreeShape* shape, const void* q, void* const* lay
  * P and dS of every visit (a query's visit to a parent) in `scratch`, a parent-stationary pass sums dK and dV from them.
  * Same reference kernels and results as htree_b200_backward, and the same query windows (HTREE_BWD_KEEP_ACCUM,
  * HTREE_BWD_NO_FOLD; `acc` is what the calls of one backward share).
- *   budget    bytes the scratch may take; htree_b200_backward_plan returns how many of them, and of `acc`, are used
- *             (HTREE_E_SCRATCH: too little even for the smallest launch; HTREE_E_UNSUPPORTED: not a shape of this path)
+ *   budget    bytes the scratch may take, all told; htree_b200_backward_plan returns how many of them are used, and the bytes of
+ *             `acc`, which are no part of it (HTREE_E_SCRATCH: too little even for the smallest launch; HTREE_E_UNSUPPORTED: not a shape of this path)
  *   dq, dk, dv  fp32, or with typed != 0 the storage type (dk, dv may be NULL with HTREE_BWD_NO_FOLD)
  *   q, out, dO 32-byte aligned, everything else 16-byte */
 int htree_b200_backward_plan(const HtreeShape* shape, int64_t budget, int64_t* acc_bytes, int64_t* scratch_bytes);

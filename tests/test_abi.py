@@ -68,6 +68,37 @@ def test_argument_errors_are_reported_before_any_launch():
         assert "unknown htree_b200 error" not in _lib.error_string(code)
 
 
+def _backward_plan(shape, budget):
+    a, s = ctypes.c_int64(-1), ctypes.c_int64(-1)
+    return _lib.lib().htree_b200_backward_plan(ctypes.byref(shape), budget, ctypes.byref(a), ctypes.byref(s)), a.value, s.value
+
+
+def test_backward_scratch_stays_within_its_budget():
+    """However tight the budget: the plan takes no more, or says that it is too little, and a larger budget is never refused where a
+    smaller one was not."""
+    shapes = [dict(T=235, H=1, H_kv=1, K=128, top_k=512, max_top_nodes=8192, dtype=1),
+              dict(T=1600, H=16, H_kv=4, K=32, top_k=512, max_top_nodes=8192, dtype=2),         # two queries a warp
+              dict(T=1601, H=4, H_kv=4, K=64, top_k=64, max_top_nodes=64, dtype=1),             # four
+              dict(T=1602, H=8, H_kv=4, K=128, top_k=64, max_top_nodes=64, dtype=0),
+              dict(T=9001, H=32, H_kv=2, K=128, top_k=16, max_top_nodes=64, dtype=1),           # many parents, short lists
+              dict(T=70000, H=4, H_kv=4, K=64, top_k=16, max_top_nodes=64, dtype=0, compression_rate=8),
+              dict(B=300, T=20, H=128, H_kv=128, K=64, top_k=16, max_top_nodes=64, dtype=2),    # many units of little work
+              dict(T=60000, H=16, H_kv=1, K=128, top_k=128, max_top_nodes=128, dtype=1, T_q=37, t_offset=50000)]
+    for kw in shapes:
+        shape = _shape(**dict(dict(B=1, compression_rate=16, V=kw["K"]), **kw))
+        accepted = False
+        for i in range(12 * 8, 36 * 8):
+            budget = int(2 ** (i / 8))
+            rc, acc, scratch = _backward_plan(shape, budget)
+            if rc:
+                assert rc == -11 and not accepted, (kw, budget, rc)
+            else:
+                assert 0 < scratch <= budget and acc > 0, (kw, budget, scratch)
+                accepted = True
+        assert accepted
+    assert _backward_plan(_shape(**dict(shapes[0], B=1, V=128, compression_rate=16)), 471800)[0] == 0      # one window of it fits
+
+
 def test_python_entry_points_refuse_cpu_tensors():
     import torch
     from htree_b200 import htree_forward

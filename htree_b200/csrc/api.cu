@@ -110,7 +110,7 @@ static int bwd_layout(const HtreeShape* s, int L, const int32_t* ln, int64_t bud
     y.xtab = x3 ? -1 : at;
     y.acc_bytes = x3 ? at : at + up((int64_t)TK * CR * D * 2);
     const int64_t qb = (int64_t)NH * D * 16 * (x3 ? 2 : 1), sb = (int64_t)NH * (CR / 8) * 128 * (x3 ? 2 : 1);
-    const int64_t entry = x3 ? (many ? sizeof(BwdEntry<true, true>) : sizeof(BwdEntry<true, false>)) : (many ? sizeof(BwdEntry<false, true>) : sizeof(BwdEntry<false, false>));
+    const int64_t entry = entry_bytes(x3, PK);
     // A window's blocked queries (4 KB each at 16 heads of 128) should stay in the L2 while its parents gather them: 8192 queries
     // are 33 MB; longer windows mean longer visit lists and fewer reductions.
     int64_t subq = 0, ng = 0, bytes = 0;
@@ -121,7 +121,7 @@ static int bwd_layout(const HtreeShape* s, int L, const int32_t* ln, int64_t bud
         ng = subq / PK;
         const int64_t visits = ng * MV;
         // of a window; the buffers below hold no more than `per` times that and the words
-        bytes = up(ng * qb) * 2 + up(visits * sb) * 2 + up(visits * (many ? 16 : 4)) + up(visits * entry) + (x3 ? up(ng * L * 8) : 0) + (many ? up(ng * L * 4) : 0) +
+        bytes = up(ng * qb) * 2 + up(visits * sb) * 2 + up(visits * (many ? 16 : 4)) + up(visits * entry) + (x3 ? up(ng * PK * L * 8) : 0) + (many ? up(ng * L * 4) : 0) +
                 up(NK * 4) + up(NK * 8) + up((visits / 8 + NK) * (int64_t)sizeof(BwdItem)) + up(4);
         if (fixed + bytes <= budget && visits < (int64_t(1) << 31)) { bp.nw = (int32_t)nw; break; }
     }
@@ -144,7 +144,7 @@ static int bwd_layout(const HtreeShape* s, int L, const int32_t* ln, int64_t bud
     auto take = [&](int64_t n) { const int64_t o = at; at += up(n); return o; };
     y.o_qb = take(per * ng * qb); y.o_dob = take(per * ng * qb);
     y.o_stp = take(per * ng * MV * sb); y.o_sts = take(per * ng * MV * sb);
-    y.o_fac = x3 ? take(per * ng * L * 8) : -1;
+    y.o_fac = x3 ? take(per * ng * PK * L * 8) : -1;
     y.o_nvis = many ? take(per * ng * L * 4) : -1;
     y.o_rank = take(per * ng * MV * (many ? 16 : 4)); y.o_entries = take(per * ng * MV * entry);
     y.o_cnt = take(cnt_words(per, NK) * 4 + 4 + units * 4); y.o_base = take(per * NK * 8);

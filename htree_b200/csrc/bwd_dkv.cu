@@ -149,9 +149,9 @@ __global__ void __launch_bounds__(256) bwd_fill_kernel(const __grid_constant__ B
             const uint32_t where = (uint32_t)grp | ((uint32_t)(rp - CR * i) << 15);
             if (bp.fac) {
                 const float2 f = bp.fac[grp * p.L + l];
-                reinterpret_cast<BwdEntry<true, false>*>(bp.entries)[entry0 + at.x + rank] = BwdEntry<true, false>{(uint32_t)v, where, f.x, f.y};
+                reinterpret_cast<BwdEntry<true, 1>*>(bp.entries)[entry0 + at.x + rank] = BwdEntry<true, 1>{(uint32_t)v, where, {f}};
             } else {
-                reinterpret_cast<BwdEntry<false, false>*>(bp.entries)[entry0 + at.x + rank] = BwdEntry<false, false>{(uint32_t)v, where};
+                reinterpret_cast<BwdEntry<false, 1>*>(bp.entries)[entry0 + at.x + rank] = BwdEntry<false, 1>{(uint32_t)v, where};
             }
             if (rank % bp.seg == 0) items[at.y + rank / bp.seg] = BwdItem{bp.koff[l] + x, at.x + rank, min(bp.seg, cnt[x] - rank), 0};
         }
@@ -178,11 +178,12 @@ __global__ void __launch_bounds__(256) bwd_fill_many_kernel(const __grid_constan
             const uint4 x = bp.vis[v];
             const int2 at = base[x.x];
             const int rank = (int)x.y;
+            uint4* entry = reinterpret_cast<uint4*>(static_cast<unsigned char*>(bp.entries) + (entry0 + at.x + rank) * entry_bytes(bp.fac != nullptr, bp.PK));
+            entry[0] = make_uint4((uint32_t)v, (uint32_t)grp, x.z, x.w);
             if (bp.fac) {
-                const float2 f = bp.fac[grp * p.L + l];
-                reinterpret_cast<BwdEntry<true, true>*>(bp.entries)[entry0 + at.x + rank] = BwdEntry<true, true>{(uint32_t)v, (uint32_t)grp, {x.z, x.w}, f.x, f.y, {0.f, 0.f}};
-            } else {
-                reinterpret_cast<BwdEntry<false, true>*>(bp.entries)[entry0 + at.x + rank] = BwdEntry<false, true>{(uint32_t)v, (uint32_t)grp, {x.z, x.w}};
+                const uint4* f = reinterpret_cast<const uint4*>(bp.fac + (grp * p.L + l) * bp.PK);
+                entry[1] = f[0];
+                if (bp.PK > 2) entry[2] = f[1];
             }
             if (rank % bp.seg == 0) items[at.y + rank / bp.seg] = BwdItem{bp.koff[l] + (int)x.x, at.x + rank, min(bp.seg, cnt[x.x] - rank), 0};
         }
@@ -199,9 +200,9 @@ __global__ void __launch_bounds__(256) bwd_fill_many_kernel(const __grid_constan
 template <int D, bool X3, int NH, bool KEYS>
 constexpr int dkv_stages() { return X3 || (KEYS && D == 128 && NH == 2) ? 2 : 3; }
 // Blocks per SM that the registers have to allow: six for the smallest split-half dV accumulators (80 registers; the compiler's 83 and
-// 86 left five).
+// 86 left five), five for the smallest dK (96; 99 left four).
 template <int D, bool X3, int CR, bool KEYS>
-constexpr int dkv_min_blocks() { return X3 ? (D == 128 ? 2 : !KEYS && (D == 32 || CR == 8) ? 6 : 3) : D == 128 ? 3 : 4; }
+constexpr int dkv_min_blocks() { return X3 ? (D == 128 ? 2 : !KEYS && (D == 32 || CR == 8) ? 6 : D == 32 ? 5 : 3) : D == 128 ? 3 : 4; }
 
 template <typename T, int D, bool X3, int NH, int CR, bool KEYS, int PK>
 __device__ __forceinline__ void dkv_item(const BwdParams& bp) {
@@ -223,7 +224,7 @@ __device__ __forceinline__ void dkv_item(const BwdParams& bp) {
     const BwdItem item = bp.items[(int64_t)ls * bp.cap + it];
     Ring ring;
     ring.init(smem_raw + (size_t)warp * Ring::kBytes);
-    using Entry = BwdEntry<X3, (PK > 1)>;
+    using Entry = BwdEntry<X3, PK>;
     const Entry* entries = reinterpret_cast<const Entry*>(bp.entries) + (int64_t)ls * bp.ng * bp.MV + item.start;
     const unsigned char* qsrc = KEYS ? bp.qb : bp.dob;
     const unsigned char* ssrc = KEYS ? bp.sts : bp.stp;
@@ -239,14 +240,26 @@ __device__ __forceinline__ void dkv_item(const BwdParams& bp) {
 
     Entry cur = entries[min(lane, len - 1)], nxt = entries[min(32 + lane, len - 1)];
     static_assert(!X3 || NSTG == 2, "a step's factors are taken when the next one is fetched");
-    float fa = 0.f, fb = 0.f;                      // split-half: the factors of the visits fetched last
+    float fa = 0.f, fb = 0.f;                      // split-half: the factors of the visits fetched last (of this lane's columns' query)
     bool differ = false;                           // do they differ among the 32 of `cur`?
+    auto factor = [&](int j) { if constexpr (X3) return KEYS ? cur.f[j].x : cur.f[j].y; else return 1.f; };
     auto compare = [&]() {
         if constexpr (X3) {
-            const float f = KEYS ? cur.fk : cur.fv;
-            fa = fb = __shfl_sync(0xffffffffu, f, 0);
-            differ = __any_sync(0xffffffffu, f != fa);
+            fa = fb = __shfl_sync(0xffffffffu, factor(0), 0);
+            bool off = false;
+#pragma unroll
+            for (int j = 0; j < PK; ++j) off |= factor(j) != fa;
+            differ = __any_sync(0xffffffffu, off);
         }
+    };
+    auto factor_of = [&](int e) {                  // of entry e
+        float f = __shfl_sync(0xffffffffu, factor(0), e);
+#pragma unroll
+        for (int j = 1; j < PK; ++j) {
+            const float x = __shfl_sync(0xffffffffu, factor(j), e);
+            if (Cols<PK>::of_pair(lane & 3) == j) f = x;
+        }
+        return f;
     };
     compare();
     auto fill = [&](int s) {                       // operand, record and table row of the step's one or two visits
@@ -257,9 +270,8 @@ __device__ __forceinline__ void dkv_item(const BwdParams& bp) {
         }
         if constexpr (X3) {
             if (differ) {
-                const float f = KEYS ? cur.fk : cur.fv;
-                fa = __shfl_sync(0xffffffffu, f, e0 & 31);
-                if constexpr (VPS == 2) fb = __shfl_sync(0xffffffffu, f, (e0 + 1) & 31);      // (past the end: the last entry again)
+                fa = factor_of(e0 & 31);
+                if constexpr (VPS == 2) fb = factor_of((e0 + 1) & 31);      // (past the end: the last entry again)
             }
         }
         const uint32_t ax = __shfl_sync(0xffffffffu, cur.visit, e0 & 31), ay = __shfl_sync(0xffffffffu, cur.where, e0 & 31);
@@ -293,35 +305,28 @@ __device__ __forceinline__ void dkv_item(const BwdParams& bp) {
     for (int s = 0; s < steps; ++s) {
         __syncwarp();
         const float f0 = fa, f1 = fb;              // of this step's visits
+        const bool mixed = differ;
         if (next < steps) fill(next);
         ring.commit();
         ++next;
-        const uint32_t slot = ring.wait();
+        uint32_t slot = ring.wait();
         const bool lone = VPS == 2 && 2 * s + 1 >= len;
-        const uint32_t ra = slot + 2 * QB, rb = ra + SB;
         uint32_t bw[NT][2], bl[X3 ? NT : 1][2];
         auto lds32 = [](uint32_t a) { uint32_t x; asm("ld.shared.b32 %0, [%1];" : "=r"(x) : "r"(a)); return x; };
         auto lds64 = [](uint32_t a, uint32_t& x, uint32_t& y) { asm("ld.shared.v2.b32 {%0,%1}, [%2];" : "=r"(x), "=r"(y) : "r"(a)); };
+        auto load_records = [&]() {
+            const uint32_t ra = slot + 2 * QB, rb = ra + SB;
 #pragma unroll
-        for (int pl = 0; pl < (X3 ? 2 : 1); ++pl) {
+            for (int pl = 0; pl < (X3 ? 2 : 1); ++pl) {
 #pragma unroll
-            for (int n = 0; n < NT; ++n) {
-                const uint32_t o = pl * PLANE + lane * (4 * NT) + 4 * n;
-                const uint32_t x = lds32(ra + o), y = lone ? 0u : lds32(rb + o);
-                if (pl == 0) { bw[n][0] = x; bw[n][1] = y; } else { bl[X3 ? n : 0][0] = x; bl[X3 ? n : 0][1] = y; }
+                for (int n = 0; n < NT; ++n) {
+                    const uint32_t o = pl * PLANE + lane * (4 * NT) + 4 * n;
+                    const uint32_t x = lds32(ra + o), y = lone ? 0u : lds32(rb + o);
+                    if (pl == 0) { bw[n][0] = x; bw[n][1] = y; } else { bl[X3 ? n : 0][0] = x; bl[X3 ? n : 0][1] = y; }
+                }
             }
-        }
-        float vfac = f0;                           // what brings this step's products back
-        if (X3 && VPS == 2 && f0 != f1) {          // two visits in one product: to their common factor (a product by a power of two)
-            float ratio[2];
-            vfac = common_factor(fminf(fmaxf(f0, 0x1p-126f), 0x1p126f), fminf(fmaxf(f1, 0x1p-126f), 0x1p126f), ratio);
-            const __half2 r0 = __float2half2_rn(ratio[0]), r1 = __float2half2_rn(ratio[1]);
-#pragma unroll
-            for (int n = 0; n < NT; ++n) {
-                bw[n][0] = as_u32(__hmul2(as_h2(bw[n][0]), r0)); bw[n][1] = as_u32(__hmul2(as_h2(bw[n][1]), r1));
-                bl[X3 ? n : 0][0] = as_u32(__hmul2(as_h2(bl[X3 ? n : 0][0]), r0)); bl[X3 ? n : 0][1] = as_u32(__hmul2(as_h2(bl[X3 ? n : 0][1]), r1));
-            }
-        }
+        };
+        load_records();
         if constexpr (KEYS && !X3) {
             const uint32_t ta = slot + 2 * QB + 2 * SB + 2 * KS * (4 * (g & 1) + (g >> 1)) + tab_of_pair;
             uint32_t ca[KS / 2], sa[KS / 2], cb[KS / 2], sb[KS / 2];
@@ -349,37 +354,74 @@ __device__ __forceinline__ void dkv_item(const BwdParams& bp) {
                 for (int n = 0; n < NT; ++n) mma_acc<FT>(acc[i][n], a, bw[n][0], bw[n][1]);
             }
         } else {
+            auto products = [&](float vfac) {      // vfac: what brings them back
 #pragma unroll
-            for (int i = 0; i < KS; ++i) {
-                uint32_t ah[4], al[4];
-                if constexpr (KEYS) {
+                for (int i = 0; i < KS; ++i) {
+                    uint32_t ah[4], al[4];
+                    if constexpr (KEYS) {
 #pragma unroll
-                    for (int v = 0; v < 2; ++v) {
-                        const uint4 x = lds_u4(slot + v * QB + i * 512 + lane * 16);
-                        const uint32_t t4 = slot + 2 * QB + 2 * SB + (VPS == 2 ? v : 0) * PK * TAB + tab_of_pair + 4 * (PPT * (g >> 1) + 2 * i + (g & 1));
-                        const float cs = __uint_as_float(lds32(t4)), sn = __uint_as_float(lds32(t4 + 4 * HALF));
-                        float2 u, w;
-                        rotate_pairs_f32(make_float2(__uint_as_float(x.x), __uint_as_float(x.y)), make_float2(__uint_as_float(x.z), __uint_as_float(x.w)),
-                                         make_float2(cs, cs), make_float2(sn, sn), make_float2(-sn, -sn), u, w);
-                        split_half2(u.x, u.y, ah[2 * v], al[2 * v]);
-                        split_half2(w.x, w.y, ah[2 * v + 1], al[2 * v + 1]);
+                        for (int v = 0; v < 2; ++v) {
+                            const uint4 x = lds_u4(slot + v * QB + i * 512 + lane * 16);
+                            const uint32_t t4 = slot + 2 * QB + 2 * SB + (VPS == 2 ? v : 0) * PK * TAB + tab_of_pair + 4 * (PPT * (g >> 1) + 2 * i + (g & 1));
+                            const float cs = __uint_as_float(lds32(t4)), sn = __uint_as_float(lds32(t4 + 4 * HALF));
+                            float2 u, w;
+                            rotate_pairs_f32(make_float2(__uint_as_float(x.x), __uint_as_float(x.y)), make_float2(__uint_as_float(x.z), __uint_as_float(x.w)),
+                                             make_float2(cs, cs), make_float2(sn, sn), make_float2(-sn, -sn), u, w);
+                            split_half2(u.x, u.y, ah[2 * v], al[2 * v]);
+                            split_half2(w.x, w.y, ah[2 * v + 1], al[2 * v + 1]);
+                        }
+                    } else {
+#pragma unroll
+                        for (int v = 0; v < 2; ++v) {
+                            lds64(slot + v * QB + i * 256 + lane * 8, ah[2 * v], ah[2 * v + 1]);
+                            lds64(slot + v * QB + D * 16 + i * 256 + lane * 8, al[2 * v], al[2 * v + 1]);
+                        }
                     }
-                } else {
 #pragma unroll
-                    for (int v = 0; v < 2; ++v) {
-                        lds64(slot + v * QB + i * 256 + lane * 8, ah[2 * v], ah[2 * v + 1]);
-                        lds64(slot + v * QB + D * 16 + i * 256 + lane * 8, al[2 * v], al[2 * v + 1]);
+                    for (int n = 0; n < NT; ++n) {
+                        float t[4];
+                        mma_zero<__half>(t, al, bw[n][0], bw[n][1]);
+                        mma_acc<FT>(t, ah, bl[X3 ? n : 0][0], bl[X3 ? n : 0][1]);
+                        mma_acc<FT>(t, ah, bw[n][0], bw[n][1]);
+#pragma unroll
+                        for (int u = 0; u < 4; ++u) acc[i][n][u] = fmaf(t[u], vfac, acc[i][n][u]);
                     }
                 }
-#pragma unroll
-                for (int n = 0; n < NT; ++n) {
-                    float t[4];
-                    mma_zero<__half>(t, al, bw[n][0], bw[n][1]);
-                    mma_acc<FT>(t, ah, bl[X3 ? n : 0][0], bl[X3 ? n : 0][1]);
-                    mma_acc<FT>(t, ah, bw[n][0], bw[n][1]);
-#pragma unroll
-                    for (int u = 0; u < 4; ++u) acc[i][n][u] = fmaf(t[u], vfac, acc[i][n][u]);
+            };
+            if constexpr (VPS == 1) {
+                products(f0);
+            } else {
+                // Columns of several queries in one product.  Those whose factors are within a step (2^4) of the largest go into it, times
+                // the ratio, and the others have products of their own: a half pair ends at 2^-25, so that with all of them brought to one
+                // factor a query whose gradient (or q) is 2^-20 of its neighbour's lost 3.6e-4 of a P of 1/512, and 2^-30 all of it.
+                float w0 = f0, w1 = lone ? f0 : f1, top = f0;
+                bool uneven = false;
+                if (mixed) {
+                    top = redux_max_f32(fmaxf(w0, w1), 0xffffffffu);
+                    uneven = __any_sync(0xffffffffu, w0 != top || w1 != top);
                 }
+#pragma unroll 1
+                do {
+                    if (uneven) {
+                        auto take = [&](float& w) {            // a column's ratio, 0: not in this product
+                            const bool in = top >= 0x1p-122f ? 16.f * w >= top : w == top;
+                            const float x = in ? __int_as_float(__float_as_int(1.f) + __float_as_int(w) - __float_as_int(top)) : 0.f;      // powers of two
+                            if (in) w = 0.f;
+                            return __float2half2_rn(x);
+                        };
+                        const __half2 r0 = take(w0), r1 = take(w1);
+#pragma unroll
+                        for (int n = 0; n < NT; ++n) {
+                            bw[n][0] = as_u32(__hmul2(as_h2(bw[n][0]), r0)); bw[n][1] = as_u32(__hmul2(as_h2(bw[n][1]), r1));
+                            bl[X3 ? n : 0][0] = as_u32(__hmul2(as_h2(bl[X3 ? n : 0][0]), r0)); bl[X3 ? n : 0][1] = as_u32(__hmul2(as_h2(bl[X3 ? n : 0][1]), r1));
+                        }
+                    }
+                    products(top);
+                    if (!uneven) break;
+                    top = redux_max_f32(fmaxf(w0, w1), 0xffffffffu);
+                    asm volatile("" : "+r"(slot));     // (what the products read again is not to be kept from the first of them)
+                    if (top != 0.f) load_records();
+                } while (top != 0.f);
             }
         }
 #pragma unroll
@@ -531,7 +573,7 @@ template <typename T, int D, bool X3, int NH, int CR, int PK>
 static int launch_dkv_pk(const BwdParams& bp, cudaStream_t st) {
     if constexpr (X3) {
         const int rc = launch_dkv_one<T, D, X3, NH, CR, true, PK>(bp, st);
-        return rc ? rc : launch_dkv_one<T, D, X3, NH, CR, false, (PK > 1 ? 2 : 1)>(bp, st);
+        return rc ? rc : launch_dkv_one<T, D, X3, NH, CR, false, PK>(bp, st);
     } else {
         constexpr size_t k = dkv_smem<D, X3, NH, CR, true, PK>(), v = dkv_smem<D, X3, NH, CR, false, PK>(), smem = k > v ? k : v;
         auto* kernel = bwd_dkv_both_kernel<T, D, NH, CR, PK>;

@@ -85,6 +85,7 @@ __global__ void __launch_bounds__(dq_warps<D, X3, NH>() * 32, dq_min_blocks<D, X
                                  r, p.scale, q);
     uint32_t dO[NH][2][KS], dOl[X3 ? NH : 1][2][X3 ? KS : 1];
     float Drow[NH][2], lse[NH][2], ginv[NH][2];
+    bool zero = true;                                   // is this lane's dO all zero?
     constexpr float kPScale = 16384.f;                  // split-half: P is carried times 2^14
     float dscale = 1.f, dinv = 1.f;                     // split-half: dO times dscale; dinv = 1 / (dscale kPScale), for P dO and for dS
     float bound_v = 0.f, bound_d = 0.f;                 // |P (dP - D)| as carried <= bound_v * the value block's factor + bound_d
@@ -138,6 +139,7 @@ __global__ void __launch_bounds__(dq_warps<D, X3, NH>() * 32, dq_min_blocks<D, X
         sum += __shfl_xor_sync(0xffffffffu, sum, 2);
         l1 += __shfl_xor_sync(0xffffffffu, l1, 1);
         l1 += __shfl_xor_sync(0xffffffffu, l1, 2);
+        zero = zero && l1 == 0.f;
         if constexpr (!X3) {
             bound_v = fmaxf(bound_v, QC::max_of(l1));
         } else {
@@ -156,6 +158,9 @@ __global__ void __launch_bounds__(dq_warps<D, X3, NH>() * 32, dq_min_blocks<D, X
     }
 
     bound_v = QC::for_pair(bound_v, r); bound_d = QC::for_pair(bound_d, r);
+    if constexpr (X3) {                                 // a query without a gradient: factors of zero, which no product has to be made for
+        if (QC::all_of(zero, r)) dinv = 0.f;
+    }
     float rescale = 1.f;                                // 16-bit: from dS as carried for dq to dS as carried in the records
     if constexpr (!X3) {
         const uint32_t v = __ldg(bp.range + 1 + unit);
@@ -318,7 +323,6 @@ __global__ void __launch_bounds__(dq_warps<D, X3, NH>() * 32, dq_min_blocks<D, X
                 if (QC::of_pair(r) == j) v = x;
             }
         }
-        float krat = 1.f, vrat = 1.f;                                 // several queries, split-half: to the factors that a record's columns share
         if constexpr (X3) {
             // dS's scale follows from a bound, 2^4 to 2^8 above what ordinary data reach at P = 1.  Found per level: per chunk, from the
             // largest |dS| or from the chunk's own factor, cost the pass 5 to 7% (32-wide heads)
@@ -328,13 +332,7 @@ __global__ void __launch_bounds__(dq_warps<D, X3, NH>() * 32, dq_min_blocks<D, X
 #pragma unroll
                 for (int h = 0; h < NH; ++h) { Drow[h][0] *= f; Drow[h][1] *= f; }
             }
-            float fk = back * q.inv, fv = dinv;
-            if constexpr (PK > 1) {
-                const float ck = redux_max_f32(fk, 0xffffffffu), cv = redux_max_f32(fv, 0xffffffffu);
-                krat = fk * pow2_inverse(ck); vrat = fv * pow2_inverse(cv);
-                fk = ck; fv = cv;
-            }
-            if (lane == 0) bp.fac[(int64_t)grp * L + l] = make_float2(fk, fv);
+            if (g == 0 && r * PK % 4 == 0) bp.fac[((int64_t)grp * L + l) * PK + QC::of_pair(r)] = make_float2(back * q.inv, dinv);
         }
         if (PK == 1 && l > 0) {
             for (int i = lane; i < (rp + 32) / 32; i += 32) selw[i] = 0u;
@@ -415,14 +413,6 @@ __global__ void __launch_bounds__(dq_warps<D, X3, NH>() * 32, dq_min_blocks<D, X
                         sw[h][0] = FS::pack(dS[0], dS[1]); sw[h][1] = FS::pack(dS[2], dS[3]);
                     }
                     db[h][0] = movm(sw[h][0]); db[h][1] = movm(sw[h][1]);
-                    if constexpr (X3 && PK > 1) {
-                        if (krat != 1.f) {
-                            split_half2(dS[0] * krat, dS[1] * krat, sw[h][0], swl[X3 ? h : 0][0]); split_half2(dS[2] * krat, dS[3] * krat, sw[h][1], swl[X3 ? h : 0][1]);
-                        }
-                        if (vrat != 1.f) {
-                            split_half2(P[0] * vrat, P[1] * vrat, pw[h][0], pwl[X3 ? h : 0][0]); split_half2(P[2] * vrat, P[3] * vrat, pw[h][1], pwl[X3 ? h : 0][1]);
-                        }
-                    }
                     if (!X3 && rescale != 1.f) {
                         sw[h][0] = FS::pack(dS[0] * rescale, dS[1] * rescale); sw[h][1] = FS::pack(dS[2] * rescale, dS[3] * rescale);
                     }

@@ -19,7 +19,7 @@
 //
 // Where several queries share a warp (PK > 1, tform.cuh) they are one group here: eight columns of blocked heads, one record for all who
 // visit a parent, a table row per query.  12000 positions, 16 heads of 32, top_k 512: dq 8.1 -> 6.8 ms, dK and dV 4.4 -> 2.6 ms, half the
-// records.  A query's scales are its own; a record's columns are brought to their largest factor.
+// records.  A query's scales are its own, in a record too, and the sums over visits undo each query's by itself (dkv_item).
 //
 // Work is cut into windows of `subq` queries of one (batch, KV head) unit, small enough for a window's blocked queries to stay
 // in L2 while its parents gather from them, and into launches of `nsub` windows, whose P and dS fit the caller's buffer.
@@ -28,12 +28,15 @@
 
 namespace htree {
 
-// A visit in its parent's list: visit slot, group | table row << 15, and, split-half, the factors of dK and dV.  Where several queries
-// share a warp (MANY) a group is PK queries and a visit one of any of them: the group, and a table row per query in 16 bits each.
-template <bool X3, bool MANY> struct __align__(8) BwdEntry { uint32_t visit, where; };
-template <> struct __align__(16) BwdEntry<true, false> { uint32_t visit, where; float fk, fv; };
-template <> struct __align__(16) BwdEntry<false, true> { uint32_t visit, where, rows[2]; };
-template <> struct __align__(16) BwdEntry<true, true> { uint32_t visit, where, rows[2]; float fk, fv, pad[2]; };
+// A visit in its parent's list: visit slot, group | table row << 15, and, split-half, the factors {dK, dV}.  Where PK queries share a warp a
+// group is all of them and a visit one of any of them: the group, a table row per query in 16 bits each, and factors per query.
+template <bool X3, int PK> struct __align__(16) BwdEntry { uint32_t visit, where, rows[2]; };
+template <int PK> struct __align__(16) BwdEntry<true, PK> { uint32_t visit, where, rows[2]; float2 f[PK]; };
+template <> struct __align__(8) BwdEntry<false, 1> { uint32_t visit, where; };
+template <> struct __align__(16) BwdEntry<true, 1> { uint32_t visit, where; float2 f[1]; };
+constexpr int64_t entry_bytes(bool x3, int PK) { return (PK > 1 ? 16 : 8) + (x3 ? 8 * PK : 0); }
+static_assert(sizeof(BwdEntry<true, 4>) == entry_bytes(true, 4) && sizeof(BwdEntry<true, 2>) == entry_bytes(true, 2) && sizeof(BwdEntry<true, 1>) == entry_bytes(true, 1) &&
+              sizeof(BwdEntry<false, 2>) == entry_bytes(false, 2) && sizeof(BwdEntry<false, 1>) == entry_bytes(false, 1), "");
 
 struct BwdItem { int32_t key, start, len, pad; };     // a piece of one parent's visit list
 
@@ -50,13 +53,13 @@ struct BwdParams {
     unsigned char* sts;                      // dS
     const unsigned char* xtab;               // 16-bit: the rotary table by dimensions of a lane (x_index), [distance][cos | sin], behind the accumulators
     uint32_t* range;                         // 16-bit: bits of the largest |dO|_1 of a row, and of every unit's largest |v|; else unused
-    float2* fac;                             // split-half: {dK, dV} factors of the visits of a group and level, [group * L + level]; else NULL
+    float2* fac;                             // split-half: {dK, dV} factors of a query's visits on a level, [(group * L + level) * PK + query]; else NULL
     int32_t* rank;                           // [group * MV + visit], or
-    uint4* vis;                              // MANY: {parent, rank, rows} [group * MV + visit]
-    int32_t* nvis;                           // MANY: visits [group * L + level]
+    uint4* vis;                              // PK > 1: {parent, rank, rows} [group * MV + visit]
+    int32_t* nvis;                           // PK > 1: visits [group * L + level]
     int32_t* cnt;                            // [nsub][NK]
     int2* base;                              // [nsub][NK]: first entry, first item
-    void* entries;                           // [nsub][subq * MV] Entry
+    void* entries;                           // [nsub][ng * MV] BwdEntry
     BwdItem* items;                          // [nsub][cap]
     int32_t* nitems;                         // [nsub]
     float* acck[HTREE_MAX_LEVELS];           // dK', dV of every level in accumulator order, [block][i][child tile][lane][4]

@@ -189,6 +189,11 @@ struct Cols {
     }
     // a value per query held by the lanes (g, *) of its columns, for the lanes (*, r)
     static __device__ __forceinline__ float for_pair(float x, int r) { return PK == 1 ? x : __shfl_sync(0xffffffffu, x, 4 * GP * of_pair(r)); }
+    // for the lanes (*, r): is `x` true for every lane (g, *) of the columns of their query?
+    static __device__ __forceinline__ bool all_of(bool x, int r) {
+        const uint32_t off = __ballot_sync(0xffffffffu, !x);
+        return PK == 1 ? off == 0u : (off >> (4 * GP * of_pair(r)) & ((uint32_t)((uint64_t(1) << (4 * GP)) - 1u))) == 0u;
+    }
     // the lanes (*, r) of the query of columns 2r, 2r + 1
     static __device__ __forceinline__ uint32_t lanes_of_pair(int r) {
         return PK == 1 ? 0xffffffffu : PK == 2 ? 0x33333333u << (r & 2) : 0x11111111u << r;

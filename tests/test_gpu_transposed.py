@@ -325,3 +325,21 @@ def test_malformed_parent_lists_of_queries_that_share_a_warp(dt, D, G, T, TK, MT
     got = ht.htree_backward(dO, q, out, ctx)
     assert torch.equal(got[0][:, same], want[0][:, same]) and not got[0][:, rows].any()
     ops.check_status()
+
+
+@pytest.mark.parametrize("dt,D,G,T,TK,MTN,Hkv,CR", [
+    (BF, 32, 4, 1600, 512, 8192, 4, 16), (BF, 32, 4, 1601, 512, 8192, 4, 16),       # two queries a warp; the last one beside the one before, or alone
+    (FP, 32, 1, 1600, 512, 512, 4, 16), (BF, 32, 2, 1603, 64, 512, 4, 16),          # four
+    (FP, 64, 4, 1600, 64, 64, 2, 16), (FP, 128, 3, 1602, 64, 64, 4, 16), (FP, 64, 4, 1500, 64, 64, 2, 8)])      # (eight children: one)
+@pytest.mark.parametrize("of_dO,of_q", [(2.0 ** -4, 1), (2.0 ** -12, 1), (2.0 ** -24, 2.0 ** -8), (1, 2.0 ** -20), (1e-9, 1), (0, 1)])
+def test_small_neighbours_keep_their_digits(dt, D, G, T, TK, MTN, Hkv, CR, of_dO, of_q):
+    """The newest key is read by the newest query alone, whose visit shares its products with those of queries 1 / of_dO times as
+    large: the key's gradients are as exact as if all were alike."""
+    import htree_b200 as ht
+    q, k, v, dO = _inputs(dt, 1, T, Hkv, G, D)
+    dO[:, -1] *= of_dO
+    q[:, -1] *= of_q
+    out, ctx = ht.htree_forward(q, k, v, CR, MTN, TK, _save_for_backward=True)
+    ours, want = ht.htree_backward(dO, q, out, ctx), ht.htree_backward(dO, q, out, ctx, _force_generic=True)
+    for name, a, b in zip(("dq", "dk", "dv"), ours, want):          # (one row's dq is 1.3e-5 off at every scale)
+        assert _rel(a[:, -1], b[:, -1]) < 2e-5 and _rel(a[:, :-1], b[:, :-1]) < 2e-5, name

@@ -190,6 +190,9 @@ __global__ void __launch_bounds__(256) bwd_fill_many_kernel(const __grid_constan
     }
 }
 
+// Is a factor (a power of two, or 0) near enough to the largest one of its product, that the operand can take the ratio?
+__device__ __forceinline__ bool near_factor(float f, float top) { return top >= 0x1p-122f ? 16.f * f >= top : f == top; }
+
 // dK' (KEYS) or dV of one item: dX^T[dims x children] += A[dims x heads] B[heads x children] over its visits, 16 rows (heads) a
 // step: one visit of up to 16 heads, or two visits of up to 8.  A = the blocked queries rotated by the visit's distance, or the
 // blocked output gradients; B = dS or P as the first pass left them.  One warp per item, operands through the warp's ring.
@@ -240,16 +243,28 @@ __device__ __forceinline__ void dkv_item(const BwdParams& bp) {
 
     Entry cur = entries[min(lane, len - 1)], nxt = entries[min(32 + lane, len - 1)];
     static_assert(!X3 || NSTG == 2, "a step's factors are taken when the next one is fetched");
-    float fa = 0.f, fb = 0.f;                      // split-half: the factors of the visits fetched last (of this lane's columns' query)
-    bool differ = false;                           // do they differ among the 32 of `cur`?
+    // Split-half: the factors of the visits fetched last (of this lane's columns' query), and the largest of the step's.  Most steps have one
+    // factor, `usual`; `odd` has a bit for every entry of `cur` with another one, `far` for those that are not within 2^4 of their step's largest.
+    float fa = 0.f, fb = 0.f, ft = 0.f, usual = 0.f, largest = 0.f;
+    uint32_t odd = 0u, far = 0u;
+    int kind = 0;                                  // of the step fetched last: 1 if a visit is odd, 3 if one is far
     auto factor = [&](int j) { if constexpr (X3) return KEYS ? cur.f[j].x : cur.f[j].y; else return 1.f; };
     auto compare = [&]() {
         if constexpr (X3) {
-            fa = fb = __shfl_sync(0xffffffffu, factor(0), 0);
-            bool off = false;
+            usual = __shfl_sync(0xffffffffu, factor(0), 0);
+            const uint32_t others = __ballot_sync(0xffffffffu, factor(0) != usual);
+            if (__popc(others) > 16) usual = __shfl_sync(0xffffffffu, factor(0), __ffs(others) - 1);
+            bool off = false, out = false;
+            largest = factor(0);
 #pragma unroll
-            for (int j = 0; j < PK; ++j) off |= factor(j) != fa;
-            differ = __any_sync(0xffffffffu, off);
+            for (int j = 0; j < PK; ++j) { off |= factor(j) != usual; largest = fmaxf(largest, factor(j)); }
+            odd = __ballot_sync(0xffffffffu, off);
+            if constexpr (VPS == 2) {
+                largest = fmaxf(largest, __shfl_xor_sync(0xffffffffu, largest, 1));
+#pragma unroll
+                for (int j = 0; j < PK; ++j) out |= !near_factor(factor(j), largest);
+                far = __ballot_sync(0xffffffffu, out);
+            }
         }
     };
     auto factor_of = [&](int e) {                  // of entry e
@@ -269,9 +284,16 @@ __device__ __forceinline__ void dkv_item(const BwdParams& bp) {
             compare();
         }
         if constexpr (X3) {
-            if (differ) {
+            constexpr uint32_t BITS = VPS == 2 ? 3u : 1u;
+            kind = (odd >> (e0 & 31) & BITS) != 0u;
+            fa = fb = ft = usual;
+            if (kind) {
                 fa = factor_of(e0 & 31);
-                if constexpr (VPS == 2) fb = factor_of((e0 + 1) & 31);      // (past the end: the last entry again)
+                if constexpr (VPS == 2) {
+                    fb = factor_of((e0 + 1) & 31);                          // (past the end: the last entry again)
+                    ft = __shfl_sync(0xffffffffu, largest, e0 & 31);
+                    if (far >> (e0 & 31) & BITS) kind = 3;
+                }
             }
         }
         const uint32_t ax = __shfl_sync(0xffffffffu, cur.visit, e0 & 31), ay = __shfl_sync(0xffffffffu, cur.where, e0 & 31);
@@ -304,8 +326,8 @@ __device__ __forceinline__ void dkv_item(const BwdParams& bp) {
 #pragma unroll 1
     for (int s = 0; s < steps; ++s) {
         __syncwarp();
-        const float f0 = fa, f1 = fb;              // of this step's visits
-        const bool mixed = differ;
+        const float f0 = fa, f1 = fb, f01 = ft;    // of this step's visits
+        const int mixed = kind;
         if (next < steps) fill(next);
         ring.commit();
         ++next;
@@ -394,17 +416,12 @@ __device__ __forceinline__ void dkv_item(const BwdParams& bp) {
                 // Columns of several queries in one product.  Those whose factors are within a step (2^4) of the largest go into it, times
                 // the ratio, and the others have products of their own: a half pair ends at 2^-25, so that with all of them brought to one
                 // factor a query whose gradient (or q) is 2^-20 of its neighbour's lost 3.6e-4 of a P of 1/512, and 2^-30 all of it.
-                float w0 = f0, w1 = lone ? f0 : f1, top = f0;
-                bool uneven = false;
-                if (mixed) {
-                    top = redux_max_f32(fmaxf(w0, w1), 0xffffffffu);
-                    uneven = __any_sync(0xffffffffu, w0 != top || w1 != top);
-                }
+                float w0 = f0, w1 = f1, top = f01;
 #pragma unroll 1
-                do {
-                    if (uneven) {
+                for (;;) {
+                    if (mixed) {
                         auto take = [&](float& w) {            // a column's ratio, 0: not in this product
-                            const bool in = top >= 0x1p-122f ? 16.f * w >= top : w == top;
+                            const bool in = near_factor(w, top);
                             const float x = in ? __int_as_float(__float_as_int(1.f) + __float_as_int(w) - __float_as_int(top)) : 0.f;      // powers of two
                             if (in) w = 0.f;
                             return __float2half2_rn(x);
@@ -417,11 +434,12 @@ __device__ __forceinline__ void dkv_item(const BwdParams& bp) {
                         }
                     }
                     products(top);
-                    if (!uneven) break;
+                    if (mixed < 3) break;
                     top = redux_max_f32(fmaxf(w0, w1), 0xffffffffu);
+                    if (top == 0.f) break;
                     asm volatile("" : "+r"(slot));     // (what the products read again is not to be kept from the first of them)
-                    if (top != 0.f) load_records();
-                } while (top != 0.f);
+                    load_records();
+                }
             }
         }
 #pragma unroll

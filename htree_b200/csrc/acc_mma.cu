@@ -101,7 +101,12 @@ acc_mma_kernel(const __grid_constant__ AttnParams p) {
     }, r, p.scale, q);
     const uint32_t tab_of_lane = PK == 1 ? 0 : QC::of_lane(g) * C::TAB;
 
+    // Several queries of 16 bits: a block that only a neighbour selected may hold values that are not finite, and 0 times one of them is NaN.
+    // If a sum is NaN at the end, the queries are walked once more one by one, as each would be in a warp of its own.
+    constexpr bool kAlone = PK > 1 && !X3;                            // (split-half values are clamped as they are packed)
+    int alone = -1;                                                   // the only query that is walked, or -1: all
     float O[NH][MT][4];
+walk_again:
 #pragma unroll
     for (int h = 0; h < NH; ++h)
 #pragma unroll
@@ -143,6 +148,7 @@ acc_mma_kernel(const __grid_constant__ AttnParams p) {
                 int n = list_of(j).load(p, l, (qidx + (int64_t)j * p.Hkv) * TK, nblk, 4, lane);
                 const int right = (n - 1) * CR + (int)(((int64_t)(p.t0 + tl + j) / p.lpow[l]) % CR);
                 if (l > 0 && right < TK) n = 0;                       // every candidate is kept: nothing to accumulate
+                if (kAlone && alone >= 0 && j != alone) n = 0;
                 if (l > 0 && n > 0) {
                     uint32_t* bits = bits_of(j);
                     for (int i = lane; i < (right + 32) / 32; i += 32) bits[i] = 0u;
@@ -533,12 +539,20 @@ acc_mma_kernel(const __grid_constant__ AttnParams p) {
         }
         if (CL > 1) cluster_sync();                                   // nobody leaves while others read from it
     } else {
+    if constexpr (kAlone) {
+        bool nan = false;
+#pragma unroll
+        for (int i = 0; i < MT; ++i)
+#pragma unroll
+            for (int u = 0; u < 4; ++u) nan |= O[0][i][u] != O[0][i][u];
+        if (alone < 0 && __any_sync(0xffffffffu, nan)) { alone = 0; goto walk_again; }
+    }
 #pragma unroll
     for (int h = 0; h < NH; ++h)
 #pragma unroll
         for (int e = 0; e < 2; ++e) {
             const int j = QC::of_pair(r), head = PK == 1 ? 8 * h + 2 * r + e : (2 * r + e) % GP;
-            if (head >= G || (PK > 1 && tl + j >= p.Tq)) continue;
+            if (head >= G || (PK > 1 && tl + j >= p.Tq) || (kAlone && alone >= 0 && j != alone)) continue;
             const int64_t at = hbase + (int64_t)j * p.H + head;
             const float inv = 1.f / s_run[h][e];
             T* orow = reinterpret_cast<T*>(p.out) + at * D + C::VB * g;
@@ -559,6 +573,7 @@ acc_mma_kernel(const __grid_constant__ AttnParams p) {
             }
             if (g == 0) { p.gmax[at] = m_true[h][e]; p.gsum[at] = s_run[h][e] * __expf(m_run[h][e] - m_true[h][e]); }
         }
+    if (kAlone && alone >= 0 && ++alone < PK) goto walk_again;
     }
 }
 

@@ -176,16 +176,17 @@ __global__ void __launch_bounds__(256) bwd_fill_many_kernel(const __grid_constan
         for (int i = lane; i < n; i += 32) {
             const int64_t v = grp * bp.MV + bp.voff[l] + i;
             const uint4 x = bp.vis[v];
-            const int2 at = base[x.x];
+            const uint32_t parent = x.x & 0xffffu;
+            const int2 at = base[parent];
             const int rank = (int)x.y;
             uint4* entry = reinterpret_cast<uint4*>(static_cast<unsigned char*>(bp.entries) + (entry0 + at.x + rank) * entry_bytes(bp.fac != nullptr, bp.PK));
-            entry[0] = make_uint4((uint32_t)v, (uint32_t)grp, x.z, x.w);
+            entry[0] = make_uint4((uint32_t)v, (uint32_t)grp | (x.x & ~0xffffu), x.z, x.w);
             if (bp.fac) {
                 const uint4* f = reinterpret_cast<const uint4*>(bp.fac + (grp * p.L + l) * bp.PK);
                 entry[1] = f[0];
                 if (bp.PK > 2) entry[2] = f[1];
             }
-            if (rank % bp.seg == 0) items[at.y + rank / bp.seg] = BwdItem{bp.koff[l] + (int)x.x, at.x + rank, min(bp.seg, cnt[x.x] - rank), 0};
+            if (rank % bp.seg == 0) items[at.y + rank / bp.seg] = BwdItem{bp.koff[l] + (int)parent, at.x + rank, min(bp.seg, cnt[parent] - rank), 0};
         }
     }
 }
@@ -277,7 +278,8 @@ __device__ __forceinline__ void dkv_item(const BwdParams& bp) {
         return f;
     };
     compare();
-    auto fill = [&](int s) {                       // operand, record and table row of the step's one or two visits
+    uint32_t skips = 0u;                           // PK > 1: per step on its way a byte, the queries of its two visits whose columns are left out
+    auto fill = [&](int s, int ahead) {            // operand, record and table row of the step's one or two visits
         const int e0 = s * VPS;
         if (e0 && (e0 & 31) == 0) {
             cur = nxt; nxt = entries[min(e0 + 32 + lane, len - 1)];
@@ -308,6 +310,7 @@ __device__ __forceinline__ void dkv_item(const BwdParams& bp) {
         ring.template copy<NH * SB>(2 * QB, ssrc + (int64_t)ax * (NH * SB), lane);
         if constexpr (KEYS && PK == 1) ring.template copy<TAB>(2 * QB + 2 * SB, tab + (int64_t)(ay >> 15) * C::TAB, lane);
         tab_rows(e0, 2 * QB + 2 * SB);
+        if (PK > 1 && ay >> 16) skips |= ay >> 16 << (8 * ahead);
         if constexpr (VPS == 2) {
             const int e1 = min(e0 + 1, len - 1);
             const uint32_t bx = __shfl_sync(0xffffffffu, cur.visit, e1 & 31), by = __shfl_sync(0xffffffffu, cur.where, e1 & 31);
@@ -315,12 +318,13 @@ __device__ __forceinline__ void dkv_item(const BwdParams& bp) {
             ring.template copy<SB>(2 * QB + SB, ssrc + (int64_t)bx * SB, lane);
             if constexpr (KEYS && PK == 1) ring.template copy<TAB>(2 * QB + 2 * SB + TAB, tab + (int64_t)(by >> 15) * C::TAB, lane);
             tab_rows(e1, 2 * QB + 2 * SB + PK * TAB);
+            if (PK > 1 && by >> 16) skips |= by >> 16 << (8 * ahead + 4);
         }
     };
     int next = 0;
 #pragma unroll 1
     for (; next < NSTG - 1; ++next) {
-        if (next < steps) fill(next);
+        if (next < steps) fill(next, next);
         ring.commit();
     }
 #pragma unroll 1
@@ -328,10 +332,23 @@ __device__ __forceinline__ void dkv_item(const BwdParams& bp) {
         __syncwarp();
         const float f0 = fa, f1 = fb, f01 = ft;    // of this step's visits
         const int mixed = kind;
-        if (next < steps) fill(next);
+        if (next < steps) fill(next, NSTG - 1);
         ring.commit();
         ++next;
         uint32_t slot = ring.wait();
+        if (PK > 1 && skips) {
+            const uint32_t skip = skips & 0xffu;
+            skips >>= 8;
+            constexpr int LB = KEYS && X3 ? 16 : 8;    // a lane's bytes at a time, which it alone reads
+#pragma unroll
+            for (int v = 0; v < 2; ++v) {
+                if (!(skip >> (4 * v + Cols<PK>::of_pair(lane & 3)) & 1)) continue;
+#pragma unroll
+                for (int i = 0; i < QB / 256; ++i)
+                    asm volatile("st.shared.v2.b32 [%0], {%1,%1};\n" ::"r"(slot + v * QB + i / (LB / 8) * (32 * LB) + lane * LB + i % (LB / 8) * 8), "r"(0u) : "memory");
+            }
+            asm volatile("" : "+r"(slot)::"memory");   // (what orders the reads behind these writes)
+        }
         const bool lone = VPS == 2 && 2 * s + 1 >= len;
         uint32_t bw[NT][2], bl[X3 ? NT : 1][2];
         auto lds32 = [](uint32_t a) { uint32_t x; asm("ld.shared.b32 %0, [%1];" : "=r"(x) : "r"(a)); return x; };

@@ -86,6 +86,7 @@ __global__ void __launch_bounds__(dq_warps<D, X3, NH>() * 32, dq_min_blocks<D, X
     uint32_t dO[NH][2][KS], dOl[X3 ? NH : 1][2][X3 ? KS : 1];
     float Drow[NH][2], lse[NH][2], ginv[NH][2];
     bool zero = true;                                   // is this lane's dO all zero?
+    bool finite = true;                                 // are its dO and q finite?
     constexpr float kPScale = 16384.f;                  // split-half: P is carried times 2^14
     float dscale = 1.f, dinv = 1.f;                     // split-half: dO times dscale; dinv = 1 / (dscale kPScale), for P dO and for dS
     float bound_v = 0.f, bound_d = 0.f;                 // |P (dP - D)| as carried <= bound_v * the value block's factor + bound_d
@@ -140,6 +141,7 @@ __global__ void __launch_bounds__(dq_warps<D, X3, NH>() * 32, dq_min_blocks<D, X
         l1 += __shfl_xor_sync(0xffffffffu, l1, 1);
         l1 += __shfl_xor_sync(0xffffffffu, l1, 2);
         zero = zero && l1 == 0.f;
+        finite = finite && l1 < INFINITY;               // (a sum that overflows counts as one that is not)
         if constexpr (!X3) {
             bound_v = fmaxf(bound_v, QC::max_of(l1));
         } else {
@@ -160,6 +162,21 @@ __global__ void __launch_bounds__(dq_warps<D, X3, NH>() * 32, dq_min_blocks<D, X
     bound_v = QC::for_pair(bound_v, r); bound_d = QC::for_pair(bound_d, r);
     if constexpr (X3) {                                 // a query without a gradient: factors of zero, which no product has to be made for
         if (QC::all_of(zero, r)) dinv = 0.f;
+    }
+    // Several queries: those with a dO or q that is not finite.  Their columns of the blocked operands must not meet the records of parents
+    // that only a neighbour visited: 0 times infinity is NaN.
+    uint32_t spoilt = 0u;
+    if constexpr (PK > 1) {
+#pragma unroll
+        for (int hf = 0; hf < 2; ++hf)
+#pragma unroll
+            for (int i = 0; i < QueryRegs<T, D, X3, NH>::N; ++i) {
+                const uint32_t x = q.v[0][hf][i];
+                finite = finite && (X3 ? fabsf(__uint_as_float(x)) < INFINITY : (x & 0x7c00u) != 0x7c00u && (x & 0x7c000000u) != 0x7c000000u);
+            }
+        const uint32_t off = __ballot_sync(0xffffffffu, !finite);
+#pragma unroll
+        for (int j = 0; j < PK; ++j) spoilt |= (off >> (4 * GP * j) & ((1u << (4 * GP)) - 1u)) != 0u ? 1u << j : 0u;
     }
     float rescale = 1.f;                                // 16-bit: from dS as carried for dq to dS as carried in the records
     if constexpr (!X3) {
@@ -295,9 +312,10 @@ __global__ void __launch_bounds__(dq_warps<D, X3, NH>() * 32, dq_min_blocks<D, X
                     uint32_t rows[2] = {0u, 0u};
 #pragma unroll
                     for (int j = 0; j < PK; ++j) rows[j >> 1] |= (uint32_t)__shfl_sync(0xffffffffu, row, j) << (16 * (j & 1));
+                    const uint32_t skip = spoilt ? spoilt & ~__ballot_sync(0xffffffffu, walk.rank >= 0) : 0u;
                     if (lane == 0) {
                         if (next) bp.vis[visit0 + next - 1] = placed;
-                        placed = make_uint4((uint32_t)parent, (uint32_t)atomicAdd(cnt + parent, 1), rows[0], rows[1]);
+                        placed = make_uint4((uint32_t)parent | skip << 16, (uint32_t)atomicAdd(cnt + parent, 1), rows[0], rows[1]);
                     }
                     ++next; ++pending;
                 }
@@ -403,6 +421,10 @@ __global__ void __launch_bounds__(dq_warps<D, X3, NH>() * 32, dq_min_blocks<D, X
                         P[i] = X3 ? __expf(fmaf(S[h][i], sfac[i >> 1], -lse[h][i & 1])) * ginv[h][i & 1] : ex2_approx(fmaf(S[h][i], kLog2e, -lse[h][i & 1]));
                         P[i] = (i < 2 ? c0 : c1) ? P[i] : 0.f;
                         dS[i] = P[i] * fmaf(dP[h][i], X3 ? fac[i >> 1].y : sscale, -Drow[h][i & 1]);
+                    }
+                    if (PK > 1 && (!X3 || spoilt)) {           // (dP may be infinite where the query has no part in the block)
+#pragma unroll
+                        for (int i = 0; i < 4; ++i) dS[i] = mask ? dS[i] : 0.f;
                     }
                     if constexpr (X3) {
                         split_half2(P[0], P[1], pw[h][0], pwl[X3 ? h : 0][0]); split_half2(P[2], P[3], pw[h][1], pwl[X3 ? h : 0][1]);

@@ -29,7 +29,8 @@
 namespace htree {
 
 // A visit in its parent's list: visit slot, group | table row << 15, and, split-half, the factors {dK, dV}.  Where PK queries share a warp a
-// group is all of them and a visit one of any of them: the group, a table row per query in 16 bits each, and factors per query.
+// group is all of them and a visit one of any of them: group | queries << 16 whose columns are left out, a table row per query in 16 bits
+// each, and factors per query.
 template <bool X3, int PK> struct __align__(16) BwdEntry { uint32_t visit, where, rows[2]; };
 template <int PK> struct __align__(16) BwdEntry<true, PK> { uint32_t visit, where, rows[2]; float2 f[PK]; };
 template <> struct __align__(8) BwdEntry<false, 1> { uint32_t visit, where; };
@@ -55,7 +56,7 @@ struct BwdParams {
     uint32_t* range;                         // 16-bit: bits of the largest |dO|_1 of a row, and of every unit's largest |v|; else unused
     float2* fac;                             // split-half: {dK, dV} factors of a query's visits on a level, [(group * L + level) * PK + query]; else NULL
     int32_t* rank;                           // [group * MV + visit], or
-    uint4* vis;                              // PK > 1: {parent, rank, rows} [group * MV + visit]
+    uint4* vis;                              // PK > 1: {parent | queries << 16 to leave out, rank, rows} [group * MV + visit]
     int32_t* nvis;                           // PK > 1: visits [group * L + level]
     int32_t* cnt;                            // [nsub][NK]
     int2* base;                              // [nsub][NK]: first entry, first item

@@ -343,3 +343,48 @@ def test_small_neighbours_keep_their_digits(dt, D, G, T, TK, MTN, Hkv, CR, of_dO
     ours, want = ht.htree_backward(dO, q, out, ctx), ht.htree_backward(dO, q, out, ctx, _force_generic=True)
     for name, a, b in zip(("dq", "dk", "dv"), ours, want):          # (one row's dq is 1.3e-5 off at every scale)
         assert _rel(a[:, -1], b[:, -1]) < 2e-5 and _rel(a[:, :-1], b[:, :-1]) < 2e-5, name
+
+
+# (Values of split halves and bf16 queries are clamped to half's range where they are read.)
+@pytest.mark.parametrize("dt,D,G,T,TK,MTN,Hkv,what", [c + (w,) for c in (
+    (BF, 64, 4, 2403, 64, 256, 2), (HF, 64, 1, 2401, 64, 64, 2), (BF, 128, 4, 2047, 64, 128, 2), (HF, 128, 2, 2401, 64, 128, 2),
+    (HF, 32, 4, 2401, 64, 512, 2), (FP, 64, 2, 2402, 64, 64, 2), (FP, 128, 4, 2049, 64, 64, 2), (BF, 64, 4, 2403, 256, 4096, 2))
+    for w in ("v", "q", "dO") if not (w == "v" and (c[0] == FP or c[1] == 32) or w == "q" and c[0] == BF)])
+@pytest.mark.parametrize("bad", [float("inf"), float("nan")])
+def test_what_is_not_finite_stays_with_the_queries_that_read_it(dt, D, G, T, TK, MTN, Hkv, what, bad):
+    """Queries from position 1 on, so that some warps have queries on both sides of the start of a block: an infinite value there does not
+    reach the query before it, nor that query's infinite q or dO the gradients of the block.  (NaN likewise.)"""
+    import htree_b200 as ht
+    from htree_b200 import ops
+    q, k, v, dO = _inputs(dt, 1, T, Hkv, G, D)
+    first = 1536                                 # (a block starts here on the level above too)
+    if what == "v":
+        v[:, first + 3, 0, 3] = bad
+    else:
+        (q if what == "q" else dO)[:, first - 1, G - 1, 5] = bad        # (of KV head 0)
+
+    def windows(cuts):
+        acc, outs, dqs = {}, [], []
+        for a, b in zip(cuts, cuts[1:]):
+            qw = q[:, a:b].contiguous()
+            o, c = ht.htree_forward(qw, k, v, 16, MTN, TK, _save_for_backward=True, _q_offset=a)
+            r = ht.htree_backward(dO[:, a:b].contiguous(), qw, o, c, _window=dict(t0=a, first=a == 1, last=b == T, acc=acc))
+            outs.append(o); dqs.append(r[0])
+        return torch.cat(outs, 1), torch.cat(dqs, 1), r[1], r[2]
+
+    ours, want = windows([1, T - 1, T]), windows(list(range(1, T, 501)) + [T])       # (1002 groups and fewer: a warp each)
+    assert not all(x.isfinite().all() for x in want)
+    early, late = slice(0, first - 2), slice(first, None)
+    assert all(x[:, early].isfinite().all() for x in want[:2])
+    if what != "v":
+        assert all(x[:, late].isfinite().all() for x in want[2:])
+    for name, a, b in zip(("out", "dq", "dk", "dv"), ours, want):
+        fine = b.isfinite()
+        assert torch.equal(a.isfinite(), fine), name
+        if name in ("out", "dq"):
+            fine[:, first - 2] = False                  # (the query itself: its dS is scaled by the call's largest dO, which it is left out of)
+            assert torch.equal(a[fine], b[fine]), name
+        else:
+            assert not fine.any() or _rel(a[fine], b[fine]) < 1e-5, name
+    torch.cuda.synchronize()
+    ops.check_status()

@@ -226,6 +226,10 @@ static int launch_top(const AttnParams& p, cudaStream_t st) {
     int QW = 8;
     while (QW > 1 && kTopKeyBytes + QW * per_warp > limit / 2) QW /= 2;       // two blocks per SM
     const size_t smem = kTopKeyBytes + QW * per_warp;
+    // Two warps an SM (a level of more than 5376 nodes, with more than 8 heads 5120) are too few with 32-wide heads, whose tiles are as large as
+    // those of 128 for a quarter of the products: 2400 queries, 2 x 8 heads, 6000 nodes 4.51 ms against 3.77 of a block per query; 5300 nodes,
+    // three warps, 3.22 against 3.48; 4096 nodes, four, 2.43 against 2.93.  128-wide heads: 6000 nodes 12.2 against 16.9, 7500 14.5 against 20.4.
+    if (D < 128 && 228 * 1024 / (smem + 1024) * QW < 3) return HTREE_E_UNSUPPORTED;
     if (smem > limit) return HTREE_E_UNSUPPORTED;
     auto* k = select_top_kernel<T, D, GP, FORM>;
     static SmemLimit shared;

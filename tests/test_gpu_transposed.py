@@ -388,3 +388,34 @@ def test_what_is_not_finite_stays_with_the_queries_that_read_it(dt, D, G, T, TK,
             assert not fine.any() or _rel(a[fine], b[fine]) < 1e-5, name
     torch.cuda.synchronize()
     ops.check_status()
+
+
+@pytest.mark.parametrize("dt,D,G,T,TK,MTN,Hkv,CR", [(FP, 128, 8, 4096, 32, 256, 2, 16), (HF, 32, 4, 12000, 512, 8192, 2, 16), (BF, 32, 8, 5000, 64, 512, 2, 8)])
+@pytest.mark.parametrize("bad", [float("inf"), float("nan")])
+def test_top_level_with_what_is_not_finite(dt, D, G, T, TK, MTN, Hkv, CR, bad):
+    """Lists of queries that see no infinite key are those of one block per query, whatever the queries and keys of their tile hold; the
+    others name nodes that exist, ascending."""
+    import htree_b200 as ht
+    from htree_b200 import ops
+    q, k, v, _ = _inputs(dt, 1, T, Hkv, G, D)
+    q[:, 100::7, 1, 3] = bad
+    k[:, T // 2, :, 5] = bad
+    lists = []
+    for generic in (False, True):
+        _, ctx = ht.htree_forward(q, k, v, CR, MTN, TK, _save_for_backward=True, _force_generic=generic)
+        lists.append(ctx["per_layer_parents"])
+    L = ctx["num_layers"]
+    seen = torch.arange(T, device=DEV) // CR ** (L - 1) >= T // 2 // CR ** (L - 1)        # (from the top level's node of that key on)
+    own = torch.zeros(T, Hkv, dtype=torch.bool, device=DEV)
+    own[100::7, 0] = True                                                                # (head 1 belongs to KV head 0)
+    clean = ~(seen[:, None] | own)
+    assert 0.2 < clean.float().mean().item() < 0.8
+    n = T
+    for l in range(L):
+        ours, want = lists[0][l][0], lists[1][l][0]
+        n = (n + CR - 1) // CR                                                           # the parents of level l
+        assert torch.equal(ours[clean], want[clean]), f"level {l}"
+        assert ours.min().item() >= -1 and ours.max().item() < n
+        assert ((ours[..., 1:] > ours[..., :-1]) | (ours[..., 1:] == -1)).all()
+    torch.cuda.synchronize()
+    ops.check_status()

@@ -305,7 +305,8 @@ static int attend(const HtreeShape* shape, const void* q, void* const* layers_k,
     }
     if (rc || select_only) return rc;
     if (pack_leaves) {
-        rc = launch_pack_listed(*shape, p.Tq, layers_k[0], layers_v[0], blocks[0], parents[0], cos_cache, sin_cache, (cudaStream_t)stream);
+        rc = launch_pack_listed(*shape, p.Tq, layers_k[0], layers_v[0], blocks[0], parents[0], (flags & HTREE_PARENTS_U16) != 0, cos_cache, sin_cache,
+                                (cudaStream_t)stream);
         if (rc) return rc;
     }
     p.flags = flags | ((flags & HTREE_FWD_INFERENCE) ? kFlagSplitOk : 0u);

@@ -247,8 +247,8 @@ constexpr uint32_t kFlagSplitOk = 1u << 30;   // internal: a forward whose selec
 bool pack_supported(int dtype, int K, int V, int CR);
 bool pack_split(int dtype, int D);                       // split-half operands?
 size_t pack_block_bytes(int D, bool x3, int CR);         // bytes of one forward block
-int launch_pack_listed(const HtreeShape& s, int Tq, const void* k, const void* v, void* blk, const int32_t* parents, const float* cosc,
-                       const float* sinc, cudaStream_t st);
+int launch_pack_listed(const HtreeShape& s, int Tq, const void* k, const void* v, void* blk, const void* parents, bool narrow,
+                       const float* cosc, const float* sinc, cudaStream_t st);
 int launch_pack_blocks(const HtreeShape& s, int first, int L, const int32_t* ln, void* const* lk, void* const* lv, void* const* blk,
                        void* const* vkblk, bool pool, const float* cosc, const float* sinc, cudaStream_t st);
 int64_t top_keys_bytes(const HtreeShape& s, int L, const int32_t* ln);       // select_top.cu

@@ -17,10 +17,10 @@ struct PackArgs {
     void* pv;
     const float* cosc;
     const float* sinc;
-    const int32_t* list;    // NULL, or parents [B, Tq, Hkv, TK]: only the blocks they name are packed
+    const void* list;       // NULL, or parents [B, Tq, Hkv, TK] (uint16 with `narrow`): only the blocks they name are packed
     int64_t total;      // B * NBLK * Hkv blocks, or list entries
     int32_t Tq, TK;
-    int32_t N, NBLK, Hkv;
+    int32_t N, NBLK, Hkv, narrow;
 };
 
 template <typename T> struct V16;
@@ -87,8 +87,9 @@ __global__ void __launch_bounds__(128) pack_blocks_kernel(const __grid_constant_
     if (blk >= a.total) return;
     const int lane = threadIdx.x & 31, g = lane >> 2, r = lane & 3;
     if (a.list) {
-        const int node = a.list[blk];
-        if ((unsigned)node >= (unsigned)a.NBLK) return;
+        // (HTREE_PARENTS_U16: no level has 65536 parents, and "none" is past their end like -1)
+        const uint32_t node = a.narrow ? static_cast<const uint16_t*>(a.list)[blk] : static_cast<const uint32_t*>(a.list)[blk];
+        if (node >= (uint32_t)a.NBLK) return;
         const int64_t grp = blk / a.TK;
         blk = ((grp / ((int64_t)a.Hkv * a.Tq)) * a.NBLK + node) * a.Hkv + grp % a.Hkv;
     }
@@ -324,10 +325,10 @@ int launch_pack_blocks(const HtreeShape& s, int first, int L, const int32_t* ln,
 }
 
 // The leaf blocks that the parent lists of level 0 name, [B, Tq, H_kv, top_k] (a block named twice is written twice, alike).
-int launch_pack_listed(const HtreeShape& s, int Tq, const void* k, const void* v, void* blk, const int32_t* parents, const float* cosc,
-                       const float* sinc, cudaStream_t st) {
+int launch_pack_listed(const HtreeShape& s, int Tq, const void* k, const void* v, void* blk, const void* parents, bool narrow,
+                       const float* cosc, const float* sinc, cudaStream_t st) {
     PackArgs a = pack_args(s, s.T, k, v, blk, cosc, sinc);
-    a.list = parents; a.Tq = Tq; a.TK = s.top_k;
+    a.list = parents; a.narrow = narrow; a.Tq = Tq; a.TK = s.top_k;
     a.total = (int64_t)s.B * Tq * s.H_kv * s.top_k;
     return launch_pack(a, s, st);
 }

@@ -764,3 +764,36 @@ def test_plan_with_selections_in_the_workspace(dtype, K, G):
     for l in range(plan.levels):
         n = B * T * Hkv * TK * 4
         assert torch.equal(ws[plan.parents[l]:plan.parents[l] + n].view(torch.int32).view(B, T, Hkv, TK), ctx["per_layer_parents"][l])
+
+
+@pytest.mark.parametrize("dtype,K,G,CR,Tq", [("bfloat16", 128, 16, 16, 1), ("float32", 64, 4, 8, 5), ("float16", 32, 8, 16, 2)])
+def test_window_of_few_queries_with_compact_lists(dtype, K, G, CR, Tq):
+    """htree_b200_run_forward for a window that reads at most half of the leaves' blocks packs the blocks that its lists name, whichever
+    their format.  (One head group's lists end with the buffer: nothing behind it may be read.)"""
+    from htree_b200 import _lib, ops as hops
+    import ctypes
+    ops = _ops()
+    B, T, Hkv, TK, MTN = 2, 9001, 2, 16, 64
+    q, k, v, _ = (x.to(DEV) for x in parity.make_inputs(B, T, Hkv * G, Hkv, K, K, dtype, 98))
+    q = q[:, T - Tq:].contiguous()
+    shape = _lib.HtreeShape(B, T, Hkv * G, Hkv, K, K, CR, TK, MTN, hops._DTYPES[q.dtype], Tq, T - Tq)
+    plan = _lib.HtreePlan()
+    _lib.check(_lib.lib().htree_b200_plan(shape, 0, plan), "plan")
+    assert 2 * Tq * TK <= plan.nodes[1]
+    n_pos, scale = TK * CR + 1024, K ** -0.5
+    t = hops._tables(K, n_pos, 10000.0, scale, hops._split(q.dtype, K), 0)
+    outs, lists = [], []
+    for wide in (torch.int32, torch.int16):
+        ws, out = torch.full((plan.bytes,), 0xFF, dtype=torch.uint8, device=DEV), torch.empty_like(q)      # (blocks of NaN but for what is packed)
+        stats = torch.empty(2, B, Tq, Hkv * G, dtype=torch.float32, device=DEV)
+        par = torch.empty(plan.levels, B, Tq, Hkv, TK, dtype=wide, device=DEV)
+        flags = _lib.FWD_INFERENCE | (_lib.PARENTS_U16 if wide == torch.int16 else 0)
+        pptr = _lib.address_array(par.data_ptr(), par[0].numel() * wide.itemsize, plan.levels)
+        _lib.check(_lib.lib().htree_b200_run_forward(shape, plan, q.data_ptr(), k.data_ptr(), v.data_ptr(), t[5], t[6], t[7], t[8], n_pos, scale,
+                                                     ws.data_ptr(), out.data_ptr(), stats[0].data_ptr(), stats[1].data_ptr(), pptr, t[9], flags,
+                                                     hops._stream()), "forward")
+        torch.cuda.synchronize(); ops.check_status()
+        outs.append(out); lists.append(par)
+    want = ops.htree_forward(q, k, v, CR, MTN, TK, _q_offset=T - Tq)
+    assert torch.equal(outs[0], want) and torch.equal(outs[1], want)
+    assert torch.equal(lists[1].to(torch.int32), lists[0])             # (ids below 2^15; -1 is 0xFFFF)

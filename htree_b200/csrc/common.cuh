@@ -63,6 +63,19 @@ struct AttnParams {
     uint32_t flags;
 };
 
+// The fp32 arithmetic that decides selections outside the tensor cores, one rounding each: a pair of a key or of a query rotated by
+// (cos, sin), and a term of a score.  Kernels that have to select alike use these, not expressions: which of two products is contracted
+// with their sum is up to the compiler, and it took another one for keys than for queries (kept here: the bits of earlier builds).
+__device__ __forceinline__ void rotate_key_f32(float lo, float hi, float cs, float sn, float& x, float& y) {
+    x = __fmaf_rn(lo, cs, -__fmul_rn(hi, sn));
+    y = __fmaf_rn(lo, sn, __fmul_rn(hi, cs));
+}
+__device__ __forceinline__ void rotate_query_f32(float lo, float hi, float cs, float sn, float& x, float& y) {
+    x = __fmaf_rn(lo, cs, -__fmul_rn(hi, sn));
+    y = __fmaf_rn(hi, cs, __fmul_rn(lo, sn));
+}
+__device__ __forceinline__ float score_term(float q, float k, float sum) { return __fmaf_rn(q, k, sum); }
+
 template <typename T> __device__ __forceinline__ float to_f(T x);
 template <> __device__ __forceinline__ float to_f<float>(float x) { return x; }
 template <> __device__ __forceinline__ float to_f<__nv_bfloat16>(__nv_bfloat16 x) { return __bfloat162float(x); }

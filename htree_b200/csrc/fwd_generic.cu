@@ -80,16 +80,16 @@ __device__ __forceinline__ void score_row(const float* qT, int GPAD, int g0, con
         const float cs[4] = {c4.x, c4.y, c4.z, c4.w}, sn[4] = {s4.x, s4.y, s4.z, s4.w};
 #pragma unroll
         for (int u = 0; u < 4; ++u) {
-            const float klo = lo[u] * cs[u] - hi[u] * sn[u];
-            const float khi = lo[u] * sn[u] + hi[u] * cs[u];
+            float klo, khi;
+            rotate_key_f32(lo[u], hi[u], cs[u], sn[u], klo, khi);
             const float* qa = qT + (d + u) * GPAD + g0;
             const float* qb = qT + (d + u + half) * GPAD + g0;
 #pragma unroll
             for (int g = 0; g < GP; g += 4) {
-                const float4 x = *reinterpret_cast<const float4*>(qa + g);
-                const float4 y = *reinterpret_cast<const float4*>(qb + g);
-                acc[g] += x.x * klo; acc[g + 1] += x.y * klo; acc[g + 2] += x.z * klo; acc[g + 3] += x.w * klo;
-                acc[g] += y.x * khi; acc[g + 1] += y.y * khi; acc[g + 2] += y.z * khi; acc[g + 3] += y.w * khi;
+                const float4 x4 = *reinterpret_cast<const float4*>(qa + g), y4 = *reinterpret_cast<const float4*>(qb + g);
+                const float x[4] = {x4.x, x4.y, x4.z, x4.w}, y[4] = {y4.x, y4.y, y4.z, y4.w};
+#pragma unroll
+                for (int i = 0; i < 4; ++i) acc[g + i] = score_term(y[i], khi, score_term(x[i], klo, acc[g + i]));
             }
         }
     }
@@ -179,8 +179,8 @@ __global__ void __launch_bounds__(NT) fwd_generic_kernel(const __grid_constant__
             if (g < G && !empty) {
                 const float lo = to_f(qg[(int64_t)g * K + d]), hi = to_f(qg[(int64_t)g * K + d + half]);
                 const float cs = __ldg(p.cosc + (int64_t)rp * half + d), sn = __ldg(p.sinc + (int64_t)rp * half + d);
-                a = (lo * cs - hi * sn) * p.scale;
-                c = (lo * sn + hi * cs) * p.scale;
+                rotate_query_f32(lo, hi, cs, sn, a, c);
+                a *= p.scale; c *= p.scale;
             }
             m.qT[d * GPAD + g] = a;
             m.qT[(d + half) * GPAD + g] = c;

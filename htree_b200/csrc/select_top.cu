@@ -3,9 +3,9 @@
 // rotated once (rotate_top_keys_kernel) and the scores are a dense product, eight queries against 128 nodes at a time.  Levels below
 // take their lists from here (fwd_generic.cu).
 //
-// The selections are fwd_generic_kernel's: the same expressions in the same order of dimensions (two heads per packed multiply-add, each
-// half rounded like the scalar one), its importance sums in both their forms, an exact Top-K.  The forms: a maximum and a sum per candidate
-// (kPerNode, where a level's scores exceed that kernel's shared memory), or sums relative to the level's maximum, which is known behind
+// The selections are fwd_generic_kernel's: rotate_key_f32, rotate_query_f32 and score_term in the same order of dimensions (ffma2: two
+// heads' terms, each half rounded like the scalar one), its importance sums in both their forms, an exact Top-K.  The forms: a maximum
+// and a sum per candidate (kPerNode, where a level's scores exceed that kernel's shared memory), or sums relative to the level's maximum, which is known behind
 // the last score: the scores are computed twice (kTwice; keeping them in shared memory left 8 of 24 warps an SM: 161 -> 183 us).
 //
 // One warp per query: 4 nodes a lane, all heads; keys from a tile in shared memory that the block's warps share.  Bound by the
@@ -44,8 +44,10 @@ __global__ void __launch_bounds__(128) rotate_top_keys_kernel(const __grid_const
         }
 #pragma unroll
         for (int u = 0; u < 4; ++u) {
-            out[(2 * (d + u)) * kTopTile] = lo[u] * cs[u] - hi[u] * sn[u];
-            out[(2 * (d + u) + 1) * kTopTile] = lo[u] * sn[u] + hi[u] * cs[u];
+            float x, y;
+            rotate_key_f32(lo[u], hi[u], cs[u], sn[u], x, y);
+            out[(2 * (d + u)) * kTopTile] = x;
+            out[(2 * (d + u) + 1) * kTopTile] = y;
         }
     }
 }
@@ -83,8 +85,8 @@ __global__ void __launch_bounds__(256) select_top_kernel(const __grid_constant__
                 const T* q = reinterpret_cast<const T*>(p.q) + (hbase + g) * D;
                 const float lo = to_f(q[d]), hi = to_f(q[d + HALF]);
                 const float cs = __ldg(p.cosc + (int64_t)rp * HALF + d), sn = __ldg(p.sinc + (int64_t)rp * HALF + d);
-                a = (lo * cs - hi * sn) * p.scale;
-                c = (lo * sn + hi * cs) * p.scale;
+                rotate_query_f32(lo, hi, cs, sn, a, c);
+                a *= p.scale; c *= p.scale;
             }
             qT[2 * d * GP + g] = a;
             qT[(2 * d + 1) * GP + g] = c;

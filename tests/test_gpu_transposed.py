@@ -282,6 +282,32 @@ def test_top_level_in_fp32_arithmetic(dt, D, G, T, TK, MTN, Hkv, CR, clustered):
     ops.check_status()
 
 
+@pytest.mark.parametrize("dt,D,G,T,TK,MTN,CR", [(FP, 128, 8, 2100, 16, 256, 16), (HF, 32, 4, 5000, 64, 512, 8), (FP, 32, 16, 4097, 32, 300, 16)])
+def test_top_level_of_windows_and_rebuilt_lists(dt, D, G, T, TK, MTN, CR):
+    """A window selects with the dense product from 592 groups on and with a block per query below, and a backward without saved lists
+    rebuilds them with the latter: the same nodes throughout, for every batch row."""
+    import htree_b200 as ht
+    from htree_b200 import ops
+    q, k, v, dO = _inputs(dt, 2, T, 2, G, D)
+    out, ctx = ht.htree_forward(q, k, v, CR, MTN, TK, _save_for_backward=True)
+    lists = ctx["per_layer_parents"]
+    for w in (147, 148, 700):
+        for t0 in (T - w, T // 2 + 1):
+            _, c = ht.htree_forward(q[:, t0:t0 + w].contiguous(), k, v, CR, MTN, TK, _save_for_backward=True, _q_offset=t0)
+            for l in lists:
+                assert torch.equal(c["per_layer_parents"][l], lists[l][:, t0:t0 + w]), (w, t0, l)
+    want = ht.htree_backward(dO, q, out, ctx)
+    lists = {l: x.clone() for l, x in lists.items()}
+    ctx["per_layer_parents"] = None
+    rebuilt = ops.recompute_parents(q, ctx["layers_k"], ctx["layers_v"], ctx["cos_cache"], ctx["sin_cache"], CR, TK, MTN, ctx["scale"],
+                                    layers_v_blk=ctx["layers_v_blk"], rope_base=ctx["rope_base"])
+    for l in lists:
+        assert torch.equal(rebuilt[l], lists[l]), l
+    assert torch.equal(ht.htree_backward(dO, q, out, ctx)[0], want[0])
+    torch.cuda.synchronize()
+    ops.check_status()
+
+
 @pytest.mark.parametrize("dt,D,G,T,TK,MTN,Hkv", [
     (HF, 32, 4, 1601, 64, 128, 4), (FP, 64, 3, 1600, 64, 128, 4), (BF, 128, 4, 1600, 64, 1024, 2),       # two queries a warp
     (BF, 64, 1, 1601, 64, 128, 4), (FP, 128, 2, 1603, 64, 128, 4)])                                      # four

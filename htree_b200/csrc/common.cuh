@@ -155,7 +155,7 @@ int launch_chained_clusters(void (*kernel)(P...), int cluster, dim3 grid, dim3 b
     cfg.gridDim = grid; cfg.blockDim = block; cfg.dynamicSmemBytes = smem; cfg.stream = st;
     cfg.attrs = at; cfg.numAttrs = cluster > 1 ? 2 : 1;
     const cudaError_t e = cudaLaunchKernelEx(&cfg, kernel, args...);
-    note_launch();
+    if (e == cudaSuccess) note_launch(); else cudaGetLastError();     // (returned; not left behind for an unrelated call to report)
     return (int)e;
 }
 // ... of `CL` blocks a cluster along x, or, where the device has no room for such a cluster, of one
@@ -163,7 +163,6 @@ template <typename... P>
 int launch_clusters(void (*kernel)(P...), int CL, dim3 grid, dim3 block, size_t smem, cudaStream_t st, const P&... args) {
     const int rc = launch_chained_clusters(kernel, CL, dim3(grid.x * CL, grid.y), block, smem, st, args...);
     if (rc == 0 || CL == 1) return rc;
-    cudaGetLastError();
     return launch_chained_clusters(kernel, 1, grid, block, smem, st, args...);
 }
 template <typename... P>
@@ -250,6 +249,7 @@ class SmemLimit {
         if (dev < 64 && have_[dev].load(std::memory_order_relaxed) >= bytes) return cudaSuccess;
         e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
         if (e == cudaSuccess && dev < 64) have_[dev].store(bytes, std::memory_order_release);
+        if (e != cudaSuccess) cudaGetLastError();
         return e;
     }
 };

@@ -506,7 +506,7 @@ static int launch_tt(const AttnParams& p, size_t smem, int GP, cudaStream_t st) 
     dim3 grid(p.Tq, p.B * p.Hkv);
     auto* k = GP == 4 ? fwd_generic_kernel<T, 4, TILED> : GP == 8 ? fwd_generic_kernel<T, 8, TILED> : fwd_generic_kernel<T, 16, TILED>;
     const cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    if (e != cudaSuccess) return (int)e;
+    if (e != cudaSuccess) { cudaGetLastError(); return (int)e; }
     return launch_chained(k, grid, dim3(NT), smem, st, p);
 }
 

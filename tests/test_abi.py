@@ -99,6 +99,21 @@ def test_backward_scratch_stays_within_its_budget():
     assert _backward_plan(_shape(**dict(shapes[0], B=1, V=128, compression_rate=16)), 471800)[0] == 0      # one window of it fits
 
 
+def test_launches_are_counted_where_they_happen():
+    """Without a device every launch is refused: the call says so and counts none.  (With one, the same call succeeds and counts.)"""
+    import torch
+    dev = "cuda" if torch.cuda.is_available() else "cpu"
+    sizes = [1000, 63, 4]
+    shape = _shape(B=1, T=1000, H=4, H_kv=4, K=64, V=64, top_k=16, compression_rate=16, max_top_nodes=16, dtype=1)
+    levels = [torch.zeros(2, n, 4, 64, dtype=torch.bfloat16, device=dev) for n in sizes]
+    k, v = _lib.ptr_array([x[0].data_ptr() for x in levels]), _lib.ptr_array([x[1].data_ptr() for x in levels])
+    before = _lib.launch_count()
+    rc = _lib.lib().htree_b200_build_tree(ctypes.byref(shape), k, v, None, None, None, None, None, None)
+    if dev == "cuda":
+        torch.cuda.synchronize()
+    assert (rc == 0 and _lib.launch_count() > before) if dev == "cuda" else (rc > 0 and _lib.launch_count() == before)
+
+
 def test_python_entry_points_refuse_cpu_tensors():
     import torch
     from htree_b200 import htree_forward

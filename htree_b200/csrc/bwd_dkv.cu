@@ -197,8 +197,9 @@ __device__ __forceinline__ bool near_factor(float f, float top) { return top >= 
 // dK' (KEYS) or dV of one item: dX^T[dims x children] += A[dims x heads] B[heads x children] over its visits, 16 rows (heads) a
 // step: one visit of up to 16 heads, or two visits of up to 8.  A = the blocked queries rotated by the visit's distance, or the
 // blocked output gradients; B = dS or P as the first pass left them.  One warp per item, operands through the warp's ring.
-// The two gradients are one after the other: each gathers from one blocked tensor only (a window of it stays in L2) and its
-// accumulator is 64 registers, which leaves room for 12 and more warps per SM.  Bound by that gather: 14 TB/s of a measured 20.
+// A warp makes one of the two gradients: it gathers from one blocked tensor only (a window of it stays in L2) and its accumulator is 64
+// registers, which leaves room for 12 and more warps per SM.  dK's items come first, split-half in a launch of their own, 16-bit in one
+// launch with dV's.  Bound by that gather: 16.3 TB/s of a measured 20 with 16 heads of 128.
 // Ring depth: three slots; two where that lets more blocks share an SM and they are the faster choice: split-half, and the keys of
 // groups of 9 to 16 heads of 128 (65536 positions, 64 heads: 13.2 -> 12.4 ms; with 8 heads a group three slots keep a lead of 1%).
 template <int D, bool X3, int NH, bool KEYS>

@@ -7,8 +7,8 @@
 // parent, two accumulation chains, the chunk's own maximum as reference, heads summed in one fixed tree) and the search is exact.
 //
 // Bound by the shared-memory read pipe (61% busy at 8 heads of 128, 76% before the third part of the table rows was left out) and latency
-// at 12 to 16 warps per SM; of its time the copies are a third, the Top-K search and the rotation a tenth each.  Measured against the kernel that gathers rows: 4 x 65536 positions, 64 heads
-// of 128: 49 -> 42 ms.
+// at 12 to 16 warps per SM; of its time the copies are a third, the Top-K search and the rotation a tenth each.  Measured against the
+// kernel that gathers rows: 4 x 65536 positions, 64 heads of 128: 49 -> 42 ms.
 #include "tform.cuh"
 
 namespace htree {
@@ -20,8 +20,9 @@ struct SelForm {
     static constexpr int DATA = PPC * KPART, TAB_ROW = D * 6, TAB = D * 4, SLOT = DATA + PPC * TAB;
     // a table row is [cos | sin | -sin] in fp32, each part ordered [k-step pair][r][4]: the four lanes of a quad read 64 consecutive
     // bytes (rows in natural order cost 8 wavefronts a load, a third of the kernel's shared-memory traffic).  A 16-byte load takes 4
-    // wavefronts however many lanes share its words, so the third part is not fetched but formed, one packed multiply for two values:
-    // 16 of 88 wavefronts a chunk and an eighth of the bytes.  8 heads of 128, 65536 positions: 8.08 -> 7.08 ms; 16 heads 1.43 -> 1.38.
+    // wavefronts however many lanes share its words, so the third part, which the C interface's tables have, is not fetched but formed,
+    // one packed multiply for two values: 16 of 88 wavefronts a chunk and an eighth of the bytes.  8 heads of 128, 65536 positions:
+    // 8.08 -> 7.08 ms (6.84 with the shorter Top-K loops below); 16 heads 1.43 -> 1.38.
     static constexpr int NSTG = SLOT > 4096 ? 2 : 3;
 };
 // Queries up to here take the longest walks first, so that these are not the tail of the call; in longer ones nearly all walks

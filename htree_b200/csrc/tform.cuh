@@ -35,7 +35,8 @@ namespace htree {
 // Several queries in one warp (PK > 1; groups of at most 4 heads, 16 children): consecutive positions share the 8 columns, GP = 8 / PK
 // of them each.  The warp walks the union of their parent lists; a block that several of them selected is fetched, read and multiplied
 // once, each column rotated by its own query's distance (PK table rows a chunk).  A query that did not select it has P = 0 there,
-// which changes nothing: rows are those of a walk alone, bit for bit.
+// which changes nothing while the block's values are finite (16-bit values that are not: acc_mma.cu walks again; the backward leaves out what
+// does not belong, bwd_dq.cu): rows are those of a walk alone, bit for bit.
 template <int D, bool X3, int CR, int PK = 1>
 struct TForm {
     static constexpr int KS = D / 16, HALF = D / 2, PPT = HALF / 4, VB = D / 8, MT = D / 16;
@@ -301,7 +302,6 @@ __device__ __forceinline__ void score16(const LaneBase<D, false, CR>& s, uint32_
 }
 
 // Split-half form (see mma_common.cuh for why the leading product of every k-step is summed with ordinary fp32 adds).
-// KEEP: the rotated query's hi / lo fragments are returned as well.
 template <typename T, int D, int NH, int CR>
 __device__ __forceinline__ void score_x3(const LaneBase<D, true, CR>& s, uint32_t tab, int r, const QueryRegs<T, D, true, NH>& q, float (&S)[NH][4]) {
     using FS = Frag<__half>;

@@ -136,7 +136,7 @@ def rope_rows(k_dim: int, cache_size: int, rope_base: float, scale: Optional[flo
 
 def rope_rows_select(k_dim: int, cache_size: int, rope_base: float, device) -> torch.Tensor:
     """The rotary table of the selection kernel: fp32 rows [cos | sin | -sin], each part ordered [k-step pair][r][4] over the pairs
-    (k_dim/8)*r + 4*(k-step pair) + {0..3} that lane r of a quad rotates."""
+    (k_dim/8)*r + 4*(k-step pair) + {0..3} that lane r of a quad rotates.  (The format of the C interface; the third part is not read.)"""
     key = (k_dim, cache_size, rope_base, "select", device)
     hit = _rope_rows.get(key)
     if hit is None:

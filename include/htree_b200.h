@@ -193,6 +193,7 @@ int htree_b200_forward(const HtreeShape* shape, const void* q, void* const* laye
  * accumulates; with HTREE_FWD_SELECT_ONLY it stops after the selection (out, gmax, gsum may be NULL).
  *   table          [n_pos, K] rows [cos(K/2) | sin(K/2)]: fp32 for fp32 storage and for K = 32, else IEEE half multiplied by scale
  *   table_f32      [n_pos, 3K/2] fp32 rows [cos | sin | -sin], each part ordered [i][r][4] over the pairs (K/8)*r + 4*i + {0..3}
+ *                  (the third part is not read: it is formed from the second)
  *   parents        L pointers, written by the selection and read by the accumulation (required)
  *   q              32-byte aligned */
 int64_t htree_b200_operand_block_bytes(const HtreeShape* shape, int32_t level, int32_t backward);

@@ -46,9 +46,9 @@ FALLBACK_PEAKS = {"hbm_gbs": 6650.0, "bf16_tflops": 1590.0, "bf16_tflops_sustain
 # groups; the backward's is the records of P and dS that its first pass leaves for its second (1 KB written and read back per group
 # and chunk) and grows with the accumulated chunks.
 NCU_TRAFFIC_BYTES = {"T": 16384, "B": 1,
-                     "forward": (0.2708e9 + 0.0363e9) + (0.3468e9 + 0.2333e9),                  # selection + accumulation
-                     "backward": (0.2852e9 + 0.0466e9) + (1.0510e9 + 7.0009e9) + 0.0628e9       # range, first pass, fill
-                                 + (3.7652e9 + 0.0551e9) + (3.7811e9 + 0.0570e9) + 0.0770e9,    # dK, dV, fold
+                     "forward": (0.2703e9 + 0.0362e9) + (0.3464e9 + 0.2332e9),                  # selection + accumulation
+                     "backward": (0.2852e9 + 0.0466e9) + (1.0494e9 + 6.9965e9) + 0.0624e9       # range, first pass, fill
+                                 + (7.4865e9 + 0.1239e9) + 0.0726e9,                            # dK and dV, fold
                      "capture": "profiles/operand_block_kernels_cfg3_eighth.md"}
 
 TDT = {"float32": torch.float32, "bfloat16": torch.bfloat16, "float16": torch.float16}

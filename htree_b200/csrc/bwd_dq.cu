@@ -161,7 +161,8 @@ __global__ void __launch_bounds__(dq_warps<D, X3, NH>() * 32, dq_min_blocks<D, X
 
     bound_v = QC::for_pair(bound_v, r); bound_d = QC::for_pair(bound_d, r);
     if constexpr (X3) {                                 // a query without a gradient: factors of zero, which no product has to be made for
-        if (QC::all_of(zero, r)) dinv = 0.f;
+        // (and a dS of zeros that is not scaled: the largest scale times a value factor would be infinite)
+        if (QC::all_of(zero, r)) { dinv = 0.f; bound_d = 8192.f; }
     }
     // Several queries: those with a dO or q that is not finite.  Their columns of the blocked operands must not meet the records of parents
     // that only a neighbour visited: 0 times infinity is NaN.

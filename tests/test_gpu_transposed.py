@@ -416,6 +416,23 @@ def test_what_is_not_finite_stays_with_the_queries_that_read_it(dt, D, G, T, TK,
     ops.check_status()
 
 
+@pytest.mark.parametrize("D,G,Hkv,CR", [(32, 8, 2, 16), (32, 4, 4, 16), (64, 2, 4, 16), (128, 8, 2, 8), (64, 16, 2, 8)])
+@pytest.mark.parametrize("size", [1e6, 1e20])
+def test_no_gradient_beside_large_values(D, G, Hkv, CR, size):
+    """Queries without an output gradient have dq = 0 and add nothing, however large the values (the scale of their dS, from a bound of
+    zero, was 2^124)."""
+    import htree_b200 as ht
+    q, k, v, dO = _inputs(FP, 1, 2000, Hkv, G, D)
+    v *= size
+    dO /= size
+    dO[:, 1000:1101] = 0
+    out, ctx = ht.htree_forward(q, k, v, CR, 64, 32, _save_for_backward=True)
+    ours, want = ht.htree_backward(dO, q, out, ctx), ht.htree_backward(dO, q, out, ctx, _force_generic=True)
+    assert not ours[0][:, 1000:1101].any()
+    for name, a, b in zip(("dq", "dk", "dv"), ours, want):
+        assert ((a.double() - b.double()).norm() / b.double().norm()).item() < 1e-5, name
+
+
 @pytest.mark.parametrize("dt,D,G,T,TK,MTN,Hkv,CR", [(FP, 128, 8, 4096, 32, 256, 2, 16), (HF, 32, 4, 12000, 512, 8192, 2, 16), (BF, 32, 8, 5000, 64, 512, 2, 8)])
 @pytest.mark.parametrize("bad", [float("inf"), float("nan")])
 def test_top_level_with_what_is_not_finite(dt, D, G, T, TK, MTN, Hkv, CR, bad):

@@ -86,7 +86,7 @@ __global__ void __launch_bounds__(dq_warps<D, X3, NH>() * 32, dq_min_blocks<D, X
     uint32_t dO[NH][2][KS], dOl[X3 ? NH : 1][2][X3 ? KS : 1];
     float Drow[NH][2], lse[NH][2], ginv[NH][2];
     bool zero = true;                                   // is this lane's dO all zero?
-    bool finite = true;                                 // are its dO and q finite?
+    bool finite = true;                                 // are its dO, dO . out and q finite?
     constexpr float kPScale = 16384.f;                  // split-half: P is carried times 2^14
     float dscale = 1.f, dinv = 1.f;                     // split-half: dO times dscale; dinv = 1 / (dscale kPScale), for P dO and for dS
     float bound_v = 0.f, bound_d = 0.f;                 // |P (dP - D)| as carried <= bound_v * the value block's factor + bound_d
@@ -141,7 +141,7 @@ __global__ void __launch_bounds__(dq_warps<D, X3, NH>() * 32, dq_min_blocks<D, X
         l1 += __shfl_xor_sync(0xffffffffu, l1, 1);
         l1 += __shfl_xor_sync(0xffffffffu, l1, 2);
         zero = zero && l1 == 0.f;
-        finite = finite && l1 < INFINITY;               // (a sum that overflows counts as one that is not)
+        finite = finite && l1 < INFINITY && fabsf(sum) < INFINITY;      // (a sum that overflows counts as one that is not)
         if constexpr (!X3) {
             bound_v = fmaxf(bound_v, QC::max_of(l1));
         } else {
@@ -223,6 +223,8 @@ __global__ void __launch_bounds__(dq_warps<D, X3, NH>() * 32, dq_min_blocks<D, X
         for (int i = 0; i < KS; ++i) dq[h][i][0] = dq[h][i][1] = dq[h][i][2] = dq[h][i][3] = 0.f;
 
     float back = dinv;                                                // split-half: times dS as carried = dS
+    bool select_dS = !X3;                                             // several queries: may dP be infinite where a query has no part in a block?
+    bool over = false;                                                // several queries, split-half: does the factor of this one's dK overflow?
     for (int l = L - 1; l >= 0; --l) {
         if (bp.voff[l] < 0) continue;
         const int Nl = p.ln[l];
@@ -351,7 +353,14 @@ __global__ void __launch_bounds__(dq_warps<D, X3, NH>() * 32, dq_min_blocks<D, X
 #pragma unroll
                 for (int h = 0; h < NH; ++h) { Drow[h][0] *= f; Drow[h][1] *= f; }
             }
-            if (g == 0 && r * PK % 4 == 0) bp.fac[((int64_t)grp * L + l) * PK + QC::of_pair(r)] = make_float2(back * q.inv, dinv);
+            float fk = back * q.inv;
+            if constexpr (PK > 1) {
+                // a block that only a neighbour visits may have values beyond this query's bound: an infinite dP
+                select_dS = spoilt != 0u || __any_sync(0xffffffffu, !(bound_v * sscale * redux_max_f32(v, 0xffffffffu) < INFINITY));
+                over = fk == INFINITY;                                // (0 of a query that has no part in a visit times it is NaN)
+                if (over) fk = 0x1p127f;
+            }
+            if (g == 0 && r * PK % 4 == 0) bp.fac[((int64_t)grp * L + l) * PK + QC::of_pair(r)] = make_float2(fk, dinv);
         }
         if (PK == 1 && l > 0) {
             for (int i = lane; i < (rp + 32) / 32; i += 32) selw[i] = 0u;
@@ -423,7 +432,7 @@ __global__ void __launch_bounds__(dq_warps<D, X3, NH>() * 32, dq_min_blocks<D, X
                         P[i] = (i < 2 ? c0 : c1) ? P[i] : 0.f;
                         dS[i] = P[i] * fmaf(dP[h][i], X3 ? fac[i >> 1].y : sscale, -Drow[h][i & 1]);
                     }
-                    if (PK > 1 && (!X3 || spoilt)) {           // (dP may be infinite where the query has no part in the block)
+                    if (PK > 1 && select_dS) {
 #pragma unroll
                         for (int i = 0; i < 4; ++i) dS[i] = mask ? dS[i] : 0.f;
                     }
@@ -436,6 +445,12 @@ __global__ void __launch_bounds__(dq_warps<D, X3, NH>() * 32, dq_min_blocks<D, X
                         sw[h][0] = FS::pack(dS[0], dS[1]); sw[h][1] = FS::pack(dS[2], dS[3]);
                     }
                     db[h][0] = movm(sw[h][0]); db[h][1] = movm(sw[h][1]);
+                    if (PK > 1 && X3 && over) {                // what the factor no longer says is in the record
+#pragma unroll
+                        for (int i = 0; i < 4; ++i) dS[i] = dS[i] == 0.f ? 0.f : dS[i] * INFINITY;
+                        sw[h][0] = FS::pack(dS[0], dS[1]); sw[h][1] = FS::pack(dS[2], dS[3]);
+                        swl[X3 ? h : 0][0] = swl[X3 ? h : 0][1] = 0u;
+                    }
                     if (!X3 && rescale != 1.f) {
                         sw[h][0] = FS::pack(dS[0] * rescale, dS[1] * rescale); sw[h][1] = FS::pack(dS[2] * rescale, dS[3] * rescale);
                     }
@@ -489,6 +504,7 @@ __global__ void __launch_bounds__(dq_warps<D, X3, NH>() * 32, dq_min_blocks<D, X
                         }
                     }
                     kfac *= back;
+                    if (PK > 1 && !mask) kfac = 0.f;           // (the product of another query's range may be infinite, and the sums are zero)
 #pragma unroll
                     for (int ks = 0; ks < KS; ++ks) {
                         uint32_t mh[4], ml[4];

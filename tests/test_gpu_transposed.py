@@ -433,6 +433,41 @@ def test_no_gradient_beside_large_values(D, G, Hkv, CR, size):
         assert ((a.double() - b.double()).norm() / b.double().norm()).item() < 1e-5, name
 
 
+@pytest.mark.parametrize("dt,D,G,T,TK,MTN,Hkv", [(FP, 64, 2, 2402, 64, 64, 2), (FP, 128, 4, 2049, 64, 64, 4), (FP, 32, 4, 2403, 64, 512, 2)])
+@pytest.mark.parametrize("what", ["v", "k"])
+def test_what_overflows_stays_with_the_queries_that_read_it(dt, D, G, T, TK, MTN, Hkv, what):
+    """Values and keys near the end of fp32's range, as above: their factors, times another query's, are infinite, and so are the sums of
+    the queries that read them."""
+    import htree_b200 as ht
+    q, k, v, dO = _inputs(dt, 1, T, Hkv, G, D)
+    first = 1536
+    if what == "v":
+        v[:, first + 3, 0, 3] = 3e38
+    else:
+        k[:, first + 3, 0, 3] = 3e38
+        dO *= 1e8
+
+    def windows(cuts):
+        acc, outs, dqs = {}, [], []
+        for a, b in zip(cuts, cuts[1:]):
+            qw = q[:, a:b].contiguous()
+            o, c = ht.htree_forward(qw, k, v, 16, MTN, TK, _save_for_backward=True, _q_offset=a)
+            r = ht.htree_backward(dO[:, a:b].contiguous(), qw, o, c, _window=dict(t0=a, first=a == 1, last=b == T, acc=acc))
+            outs.append(o); dqs.append(r[0])
+        return torch.cat(outs, 1), torch.cat(dqs, 1), r[1], r[2]
+
+    ours, want = windows([1, T - 1, T]), windows(list(range(1, T, 501)) + [T])       # (1002 groups and fewer: a warp each)
+    early = slice(0, first - 1)                                                       # (row 0 is position 1)
+    for name, a, b in zip(("out", "dq", "dk", "dv"), ours, want):
+        fine = b.isfinite()
+        assert torch.equal(a.isfinite(), fine), name
+        if name in ("out", "dq"):
+            assert fine[:, early].all() and torch.equal(a[:, early], b[:, early]), name
+        a, b = a[fine].double(), b[fine].double()
+        assert ((a - b).norm() / b.norm()).item() < 1e-5, name
+    torch.cuda.synchronize()
+
+
 @pytest.mark.parametrize("dt,D,G,T,TK,MTN,Hkv,CR", [(FP, 128, 8, 4096, 32, 256, 2, 16), (HF, 32, 4, 12000, 512, 8192, 2, 16), (BF, 32, 8, 5000, 64, 512, 2, 8)])
 @pytest.mark.parametrize("bad", [float("inf"), float("nan")])
 def test_top_level_with_what_is_not_finite(dt, D, G, T, TK, MTN, Hkv, CR, bad):
